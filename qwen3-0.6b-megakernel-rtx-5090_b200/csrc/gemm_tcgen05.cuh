@@ -24,6 +24,12 @@
 // row / tensor scale multiplies the accumulator in the epilogue.  The activations stay fp16 and the accumulation fp32,
 // so the products are those of the dequantised matrix: tcgen05's own narrow kinds (f8f6f4, mxf4nvf4) would need the
 // ACTIVATIONS in 8 or 4 bits as well, which a greedy decoder checked token by token cannot afford.
+//
+// Split activations (template parameter AH = 2): A is [M x 2 K], columns [0, K) the fp16 rounding hi of the fp32
+// activations and columns [K, 2 K) the fp16 rounding lo of what it left (x - hi).  A stage holds both A tiles and ONE B
+// tile, which eight MMAs read instead of four: the weights cross HBM, L2 and the copy engine once.  hi + lo keeps 22 bits
+// of x (absolute floor 2^-25, the fp16 subnormals), the products are exact and the sums fp32, so the result is the one of
+// fp32 activations - what the token-serial kernels compute - at twice the MMA work.
 #ifndef QMK_GEMM_TCGEN05_CUH_
 #define QMK_GEMM_TCGEN05_CUH_
 
@@ -38,7 +44,8 @@ namespace qmk_gemm {
 constexpr int BM = 128, BK = 64;                 // BK * 2 bytes = one 128-byte swizzle row; the N tile (128 or 64) is a template parameter
 // Ring depth per N-tile variant: as many stages as fit in ~192 KB (a skinny M = 128 problem is bound by the
 // latency of its K loop, so the whole K extent of a 1024-wide matrix is in flight at once).
-constexpr int stages_for(int bn, int wq = 0) {
+constexpr int stages_for(int bn, int wq = 0, int ah = 1) {
+  if (ah == 2) return bn == 32 ? 5 : bn == 256 ? 3 : bn == 128 && wq ? 3 : 4;
   return wq ? (bn == 32 ? 8 : bn == 64 ? 6 : bn == 128 ? 4 : 2) : (bn == 32 ? 10 : bn == 64 ? 8 : bn == 128 ? 6 : 4);
 }
 constexpr int MAX_GROUPS = 3;   // matrices sharing one A operand that one launch can multiply (q/k/v, gate/up)
@@ -48,8 +55,8 @@ constexpr int threads_for(int wq) { return wq ? THREADS_PACKED : THREADS; }
 constexpr uint32_t TILE_A_BYTES = BM * BK * 2;   // 16 KB
 // Packed K block of one B row: 64 e4m3 bytes, or 32 bytes of e2m1 pairs
 constexpr uint32_t raw_row_bytes(int wq) { return wq == 1 ? 64u : wq == 2 ? 32u : 0u; }
-constexpr uint32_t stage_bytes_for(int bn, int wq = 0) {
-  return TILE_A_BYTES + static_cast<uint32_t>(bn) * BK * 2 + static_cast<uint32_t>(bn) * raw_row_bytes(wq);
+constexpr uint32_t stage_bytes_for(int bn, int wq = 0, int ah = 1) {
+  return static_cast<uint32_t>(ah) * TILE_A_BYTES + static_cast<uint32_t>(bn) * BK * 2 + static_cast<uint32_t>(bn) * raw_row_bytes(wq);
 }
 // Per-row scales kept in shared memory for the whole tile: the fp32 row / tensor scale, and for NVFP4 the block
 // scales of the CTA's K range (one byte per 16 values; K <= 3072 -> 192 bytes, rows 196 bytes apart against bank
@@ -61,8 +68,8 @@ constexpr uint32_t scale_bytes_for(int bn, int wq) {
 }
 constexpr int MAX_STAGES = 16;
 constexpr uint32_t BARRIER_BYTES = 640;   // full[16], empty[16], acc_full, raw_full[16], a_full[16], TMEM address, abort flag
-constexpr size_t smem_bytes_for(int bn, int wq = 0) {
-  return 1024 /* alignment slack */ + static_cast<size_t>(stages_for(bn, wq)) * stage_bytes_for(bn, wq) + BARRIER_BYTES +
+constexpr size_t smem_bytes_for(int bn, int wq = 0, int ah = 1) {
+  return 1024 /* alignment slack */ + static_cast<size_t>(stages_for(bn, wq, ah)) * stage_bytes_for(bn, wq, ah) + BARRIER_BYTES +
          scale_bytes_for(bn, wq);
 }
 // Ring depth of a launch: the compile-time depth above (one CTA per SM, ~200 KB: a skinny problem wants its whole K
@@ -70,14 +77,14 @@ constexpr size_t smem_bytes_for(int bn, int wq = 0) {
 // of one (TMEM -> registers -> global) runs under the main loop of the other, which is what a multi-wave prefill GEMM
 // wants (measured on 2048 prompt tokens: 7.9 -> 6.8 ms per pass).
 struct RingGeometry { int stages; uint32_t ring_bytes; size_t smem_bytes; };
-inline RingGeometry ring_geometry(int sb, int wq, uint32_t budget_bytes) {
+inline RingGeometry ring_geometry(int sb, int wq, uint32_t budget_bytes, int ah = 1) {
   RingGeometry g;
-  g.stages = stages_for(sb, wq);
+  g.stages = stages_for(sb, wq, ah);
   if (budget_bytes > 0) {
-    const int fit = static_cast<int>(budget_bytes / stage_bytes_for(sb, wq));
+    const int fit = static_cast<int>(budget_bytes / stage_bytes_for(sb, wq, ah));
     if (fit < g.stages) g.stages = fit < 2 ? 2 : fit;
   }
-  g.ring_bytes = static_cast<uint32_t>(g.stages) * stage_bytes_for(sb, wq);
+  g.ring_bytes = static_cast<uint32_t>(g.stages) * stage_bytes_for(sb, wq, ah);
   g.smem_bytes = 1024 + static_cast<size_t>(g.ring_bytes) + BARRIER_BYTES + scale_bytes_for(sb, wq);
   return g;
 }
@@ -210,8 +217,8 @@ __device__ __forceinline__ uint32_t e4m3x2_to_half2_bits(uint32_t two_bytes) {
 
 // FUSE (BN = 32 or 64): B0 is the gate matrix and B1 the up matrix of a SwiGLU MLP; the CTA keeps two accumulators
 // (gate tile in TMEM columns [0, BN), up tile in [BN, 2 BN)) and its epilogue writes fp16 silu(gate) * up to
-// groups.C[0] (reinterpreted as __half [M x N]) instead of two fp32 matrices.
-template <int BN, bool FUSE = false, int WQ = 0>
+// groups.C[0] (reinterpreted as __half [M x N]) instead of two fp32 matrices; AH = 2: as hi and lo halves, [M x 2 N].
+template <int BN, bool FUSE = false, int WQ = 0, int AH = 1>
 __global__ void __launch_bounds__(WQ ? THREADS_PACKED : THREADS, 1)
 gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b0,
                    const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ CUtensorMap map_b2,
@@ -223,7 +230,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   constexpr int SB = FUSE ? 2 * BN : BN;          // B rows held per stage / accumulator columns
   constexpr uint32_t RAW_ROW = raw_row_bytes(WQ);
   const int STAGES = groups.stages;
-  constexpr uint32_t STAGE_BYTES = stage_bytes_for(SB, WQ);
+  constexpr uint32_t STAGE_BYTES = stage_bytes_for(SB, WQ, AH);
   // which matrix this CTA works on
   int tile = blockIdx.x, grp = 0;
   if (!FUSE && tile >= groups.N[0] / BN) { tile -= groups.N[0] / BN; grp = 1; }
@@ -260,9 +267,9 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   auto b_landed = [&](int s) { return WQ ? raw_full(s) : full(s); };
   auto a_landed = [&](int s) { return WQ ? a_full(s) : full(s); };
   constexpr uint32_t TILE_RAW_BYTES = BN * RAW_ROW;
-  const uint32_t a_tx = groups.a_box_bytes ? groups.a_box_bytes : TILE_A_BYTES;
+  const uint32_t a_tx = AH * (groups.a_box_bytes ? groups.a_box_bytes : TILE_A_BYTES);
   const uint32_t b_tx = (FUSE ? 2u : 1u) * (WQ ? TILE_RAW_BYTES : TILE_B_BYTES);
-  constexpr uint32_t TILE_A = TILE_A_BYTES;   // the B tile follows the A tile in a stage
+  constexpr uint32_t TILE_A = AH * TILE_A_BYTES;   // the B tile follows the A tile(s) in a stage
   const int kcol = WQ ? static_cast<int>(RAW_ROW) : BK;          // B-map columns (bytes for packed rows) per K block
   const uint32_t b_dst = WQ ? TILE_A + (FUSE ? 2u : 1u) * TILE_B_BYTES : TILE_A;   // where the B copies land in a stage
   const uint32_t b_dst_step = WQ ? TILE_RAW_BYTES : TILE_B_BYTES;
@@ -331,6 +338,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       for (int kb = 0; kb < prologue; ++kb) {
         if (WQ) bar_expect_tx(a_full(kb), a_tx);
         tma_load_2d(base + kb * STAGE_BYTES, &map_a, (kb0 + kb) * BK, m0, a_landed(kb));
+        if (AH == 2) tma_load_2d(base + kb * STAGE_BYTES + TILE_A_BYTES, &map_a, K + (kb0 + kb) * BK, m0, a_landed(kb));
       }
       int issued = prologue;
       // self test of the bounded waits: the loads are never issued, so the MMA thread's first wait runs out
@@ -341,6 +349,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         bar_expect_tx(b_landed(s), WQ ? b_tx : a_tx + b_tx);
         if (WQ) bar_expect_tx(a_full(s), a_tx);
         tma_load_2d(base + s * STAGE_BYTES, &map_a, (kb0 + kb) * BK, m0, a_landed(s));
+        if (AH == 2) tma_load_2d(base + s * STAGE_BYTES + TILE_A_BYTES, &map_a, K + (kb0 + kb) * BK, m0, a_landed(s));
         tma_load_2d(base + s * STAGE_BYTES + b_dst, map_b, (kb0 + kb) * kcol, n0, b_landed(s));
         if (FUSE) tma_load_2d(base + s * STAGE_BYTES + b_dst + b_dst_step, &map_b1, (kb0 + kb) * kcol, n0, b_landed(s));
         issued = kb + 1;
@@ -371,6 +380,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           // FUSE: the up tile follows the gate tile in shared memory (BN more rows of the same 8-row-group layout),
           // so one MMA of N = 2 BN covers both and leaves gate in columns [0, BN), up in [BN, 2 BN)
           mma_f16_ss(tmem_base, da + 2u * j, db + 2u * j, (kb > 0 || j > 0) ? 1u : 0u, idesc_for(SB));
+          if (AH == 2) mma_f16_ss(tmem_base, da + (TILE_A_BYTES >> 4) + 2u * j, db + 2u * j, 1u, idesc_for(SB));
         }
         mma_commit(empty(s));               // the stage is free once these MMAs have read it
       }
@@ -440,7 +450,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ok && FUSE) {
       const int row = m0 + quarter * 32 + lane;
-      __half *arow = reinterpret_cast<__half *>(C) + static_cast<size_t>(row) * N + n0;
+      __half *arow = reinterpret_cast<__half *>(C) + static_cast<size_t>(row) * (AH * N) + n0;
 #pragma unroll 1
       for (int c = 0; c < BN / 16; ++c) {     // 16 columns of the gate tile and the same 16 of the up tile per pass
         uint32_t g[16], u[16];
@@ -461,7 +471,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             : "memory");
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (row < M) {
-          uint32_t packed[8];
+          uint32_t packed[8], packed_lo[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             float g0 = __uint_as_float(g[2 * i]), g1 = __uint_as_float(g[2 * i + 1]);
@@ -470,6 +480,14 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
               g0 *= s_rowscale[c * 16 + 2 * i]; g1 *= s_rowscale[c * 16 + 2 * i + 1];
               u0 *= s_rowscale[BN + c * 16 + 2 * i]; u1 *= s_rowscale[BN + c * 16 + 2 * i + 1];
             }
+            if (AH == 2) {
+              const float a0 = g0 / (1.0f + expf(-g0)) * u0, a1 = g1 / (1.0f + expf(-g1)) * u1;
+              const __half2 hi = __floats2half2_rn(a0, a1);
+              const __half2 lo = __floats2half2_rn(a0 - __low2float(hi), a1 - __high2float(hi));
+              packed[i] = *reinterpret_cast<const uint32_t *>(&hi);
+              packed_lo[i] = *reinterpret_cast<const uint32_t *>(&lo);
+              continue;
+            }
             // (hardware exp2 and reciprocal: a few ulp, far inside the fp16 rounding of the result; the exact forms
             // cost about 25 instructions per value and made this epilogue as long as a third of the K loop)
             const __half2 h = __floats2half2_rn(__fdividef(g0, 1.0f + __expf(-g0)) * u0, __fdividef(g1, 1.0f + __expf(-g1)) * u1);
@@ -477,6 +495,10 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           }
           *reinterpret_cast<uint4 *>(arow + c * 16) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
           *reinterpret_cast<uint4 *>(arow + c * 16 + 8) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+          if (AH == 2) {
+            *reinterpret_cast<uint4 *>(arow + N + c * 16) = make_uint4(packed_lo[0], packed_lo[1], packed_lo[2], packed_lo[3]);
+            *reinterpret_cast<uint4 *>(arow + N + c * 16 + 8) = make_uint4(packed_lo[4], packed_lo[5], packed_lo[6], packed_lo[7]);
+          }
         }
       }
     } else if (ok) {

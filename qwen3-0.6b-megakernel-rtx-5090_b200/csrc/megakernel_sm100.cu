@@ -223,7 +223,7 @@ struct Engine {
 
 constexpr int MAX_DEVICES = 16;
 Engine g_engines[MAX_DEVICES];
-std::mutex g_mutex;
+std::recursive_mutex g_mutex;   // (recursive: a prefill on the tensor cores runs under it and takes its options through prefill_env)
 
 Engine *current_engine_unlocked() {
   int dev = 0;
@@ -537,7 +537,7 @@ Params base_params(const void *embed, const LDGLayerWeight *layers, const void *
 
 namespace qmk_internal {
 int prefill_env(int max_seq_len, cudaStream_t stream, PrefillEnv *out) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   clear_error(e);
@@ -556,7 +556,7 @@ int prefill_env(int max_seq_len, cudaStream_t stream, PrefillEnv *out) {
   return QMK_OK;
 }
 int report(int code, const std::string &msg) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   return fail(current_engine_unlocked(), code, msg);
 }
 }  // namespace qmk_internal
@@ -566,7 +566,7 @@ extern "C" {
 int qmk_abi_version(void) { return 2; }
 
 int qmk_configure(int vocab_size, int rope_from_table, int split_len, int max_ctas, int timeout_ms) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   if (vocab_size == 0 || split_len == 0 || timeout_ms == 0) return fail(e, QMK_ERR_BAD_ARGUMENT, "zero option value");
@@ -580,7 +580,7 @@ int qmk_configure(int vocab_size, int rope_from_table, int split_len, int max_ct
 }
 
 int qmk_set_inv_freq(const float *inv_freq64) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e || !inv_freq64) return QMK_ERR_BAD_ARGUMENT;
   // callers re-apply their options before every op: the same frequencies again cost nothing
@@ -594,7 +594,7 @@ int qmk_set_inv_freq(const float *inv_freq64) {
 }
 
 int qmk_set_logits_dump(float *logits_out) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   e->logits_out = logits_out;
@@ -602,7 +602,7 @@ int qmk_set_logits_dump(float *logits_out) {
 }
 
 int qmk_set_weight_format(int format) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   if (format < 0 || format > 2)
@@ -612,7 +612,7 @@ int qmk_set_weight_format(int format) {
 }
 
 int qmk_set_prefill_attention(int tensor_core) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   if (tensor_core >= 0) e->prefill_attn_tc = tensor_core ? 1 : 0;
@@ -620,7 +620,7 @@ int qmk_set_prefill_attention(int tensor_core) {
 }
 
 int qmk_set_decode_attention(int tensor_core) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   if (tensor_core >= 0) e->decode_attn_mma = tensor_core ? 1 : 0;
@@ -628,7 +628,7 @@ int qmk_set_decode_attention(int tensor_core) {
 }
 
 int qmk_set_step_overlap(int enabled) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   if (enabled >= 0) e->step_overlap = enabled ? 1 : 0;
@@ -636,7 +636,7 @@ int qmk_set_step_overlap(int enabled) {
 }
 
 int qmk_set_tuning2(int repl, int stream_inflight) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   if (repl == 1 || repl == 2 || repl == 4) e->repl = repl;
@@ -646,7 +646,7 @@ int qmk_set_tuning2(int repl, int stream_inflight) {
 }
 
 int qmk_set_tuning(int spin_sleep_ns, int l2_evict_first) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   if (spin_sleep_ns >= 0) e->spin_sleep_ns = e->fused_sleep_ns = spin_sleep_ns > 10000 ? 10000 : spin_sleep_ns;
@@ -655,7 +655,7 @@ int qmk_set_tuning(int spin_sleep_ns, int l2_evict_first) {
 }
 
 int qmk_set_fused(int fused, int red_copies) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   if (fused > 2) return fail(e, QMK_ERR_BAD_ARGUMENT, "fused must be 0, 1 or 2");
@@ -666,7 +666,7 @@ int qmk_set_fused(int fused, int red_copies) {
 }
 
 int qmk_invalidate_weights(void) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   for (auto &p : e->prepared) p.force = 1;
@@ -674,7 +674,7 @@ int qmk_invalidate_weights(void) {
 }
 
 int qmk_release_weights(const LDGLayerWeight *layer_weights) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   for (size_t i = 0; i < e->prepared.size();) {
@@ -690,7 +690,7 @@ int qmk_release_weights(const LDGLayerWeight *layer_weights) {
 }
 
 int qmk_set_profile_buffer(unsigned long long *timestamps) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   e->prof = timestamps;
@@ -750,7 +750,7 @@ int qmk_decode(int input_token_id, int *output_token_id, const void *embed_weigh
                void *k_cache, void *v_cache, void *hidden_buffer, void *g_normalized, void *block_max_vals,
                void *block_max_idxs, int num_layers, int position, int max_seq_len, float attn_scale,
                cudaStream_t stream) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   return decode_unlocked(input_token_id, output_token_id, embed_weight, layer_weights, final_norm_weight, lm_head_weight,
                          cos_table, sin_table, k_cache, v_cache, hidden_buffer, g_normalized, block_max_vals, block_max_idxs,
                          num_layers, position, max_seq_len, attn_scale, stream);
@@ -761,7 +761,7 @@ int qmk_generate(int first_token_id, int num_steps, const void *embed_weight, co
                  const void *sin_table, void *k_cache, void *v_cache, void *hidden_buffer, void *g_normalized,
                  void *block_max_vals, void *block_max_idxs, int *output_log, int num_layers, int start_position,
                  int max_seq_len, float attn_scale, int eos_token_id, int synchronize, cudaStream_t stream) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   return generate_unlocked(first_token_id, num_steps, embed_weight, layer_weights, final_norm_weight, lm_head_weight,
                            cos_table, sin_table, k_cache, v_cache, hidden_buffer, g_normalized, block_max_vals,
                            block_max_idxs, output_log, num_layers, start_position, max_seq_len, attn_scale, eos_token_id,
@@ -773,7 +773,7 @@ int qmk_generate_batch(int num_sequences, const int *first_token_ids, const int 
                        const void *lm_head_weight, const void *cos_table, const void *sin_table, void *const *k_caches,
                        void *const *v_caches, int *const *output_logs, int num_layers, int max_seq_len, float attn_scale,
                        int synchronize, cudaStream_t stream) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   clear_error(e);
@@ -811,6 +811,7 @@ int qmk_generate_batch(int num_sequences, const int *first_token_ids, const int 
 }  // extern "C"
 
 namespace {
+constexpr int SPLIT_PREFILL_MIN_TOKENS = 4;
 int prefill_unlocked(const int *token_ids_host, int num_tokens, const void *embed_weight,
                      const LDGLayerWeight *layer_weights, const void *final_norm_weight, const void *cos_table,
                      const void *sin_table, void *k_cache, void *v_cache, int num_layers, int start_position,
@@ -823,6 +824,13 @@ int prefill_unlocked(const int *token_ids_host, int num_tokens, const void *embe
   for (int i = 0; i < num_tokens; ++i)
     if (token_ids_host[i] < 0 || token_ids_host[i] >= e->vocab)
       return fail(e, QMK_ERR_BAD_TOKEN, "prompt token outside [0, vocab)");
+  // Prompts of more than a few tokens go through the chunked tensor-core pass with split activations (hi + lo fp16 halves of
+  // every fp32 operand: the precision of the kernels below) instead of one persistent step per token: a pass over up to
+  // a few hundred tokens takes 1.3-1.5 ms, a step without its LM head 0.42 ms.  31 tokens 13.0 -> 1.4 ms, 776 tokens
+  // 349 -> 3.4 ms.
+  if (num_tokens >= SPLIT_PREFILL_MIN_TOKENS && e->wfmt != 2)
+    return qmk_tc::prefill_split(token_ids_host, num_tokens, embed_weight, layer_weights, cos_table, sin_table, k_cache, v_cache,
+                                 num_layers, start_position, max_seq_len, attn_scale, stream);
   if (num_tokens > e->tok_cap) {  // grow-only staging, as the reference keeps (megakernel_5090.cu:1303-1307)
     if (e->tok_dev) cudaFree(e->tok_dev);
     e->tok_dev = nullptr;
@@ -893,7 +901,8 @@ int qmk_prefill(const int *token_ids_host, int num_tokens, const void *embed_wei
                 const LDGLayerWeight *layer_weights, const void *final_norm_weight, const void *cos_table,
                 const void *sin_table, void *k_cache, void *v_cache, int num_layers, int start_position,
                 int max_seq_len, float attn_scale, cudaStream_t stream) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  auto workspace = qmk_tc::prefill_lock();
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   return prefill_unlocked(token_ids_host, num_tokens, embed_weight, layer_weights, final_norm_weight, cos_table, sin_table,
                           k_cache, v_cache, num_layers, start_position, max_seq_len, attn_scale, stream);
 }
@@ -921,7 +930,7 @@ int qmk_engine_create(const qmk_engine_config *config, qmk_engine **out) {
 int qmk_engine_destroy(qmk_engine *h) {
   if (!h) return QMK_OK;
   {
-    std::lock_guard<std::mutex> lock(g_mutex);
+    std::lock_guard<std::recursive_mutex> lock(g_mutex);
     int prev = 0;
     cudaGetDevice(&prev);
     if (cudaSetDevice(h->device) == cudaSuccess) {
@@ -947,7 +956,7 @@ int qmk_engine_destroy(qmk_engine *h) {
 }
 
 int qmk_engine_apply(qmk_engine *h) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   return apply_handle_unlocked(h, nullptr);
 }
 
@@ -956,7 +965,7 @@ int qmk_engine_decode(qmk_engine *h, int input_token_id, int *output_token_id, c
                       const void *cos_table, const void *sin_table, void *k_cache, void *v_cache, void *hidden_buffer,
                       void *g_normalized, void *block_max_vals, void *block_max_idxs, int num_layers, int position,
                       int max_seq_len, float attn_scale, cudaStream_t stream) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   const int rc = apply_handle_unlocked(h, layer_weights);
   if (rc != QMK_OK) return rc;
   return decode_unlocked(input_token_id, output_token_id, embed_weight, layer_weights, final_norm_weight, lm_head_weight,
@@ -970,7 +979,7 @@ int qmk_engine_generate(qmk_engine *h, int first_token_id, int num_steps, const 
                         void *g_normalized, void *block_max_vals, void *block_max_idxs, int *output_log, int num_layers,
                         int start_position, int max_seq_len, float attn_scale, int eos_token_id, int synchronize,
                         cudaStream_t stream) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   const int rc = apply_handle_unlocked(h, layer_weights);
   if (rc != QMK_OK) return rc;
   return generate_unlocked(first_token_id, num_steps, embed_weight, layer_weights, final_norm_weight, lm_head_weight,
@@ -983,7 +992,8 @@ int qmk_engine_prefill(qmk_engine *h, const int *token_ids_host, int num_tokens,
                        const LDGLayerWeight *layer_weights, const void *final_norm_weight, const void *cos_table,
                        const void *sin_table, void *k_cache, void *v_cache, int num_layers, int start_position,
                        int max_seq_len, float attn_scale, cudaStream_t stream) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  auto workspace = qmk_tc::prefill_lock();
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   const int rc = apply_handle_unlocked(h, layer_weights);
   if (rc != QMK_OK) return rc;
   return prefill_unlocked(token_ids_host, num_tokens, embed_weight, layer_weights, final_norm_weight, cos_table, sin_table,
@@ -991,7 +1001,7 @@ int qmk_engine_prefill(qmk_engine *h, const int *token_ids_host, int num_tokens,
 }
 
 int qmk_sync_status(void) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   if (!e->ready) return e->last_status;
@@ -1009,14 +1019,14 @@ int qmk_sync_status(void) {
 const char *qmk_last_error(void) {
   // a copy per calling thread, taken under the lock: another thread's next call may rewrite the engine's string
   static thread_local std::string mine;
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   mine = e ? e->last_error : std::string("no CUDA device");
   return mine.c_str();
 }
 
 int qmk_num_ctas(void) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e || ensure_ready(e) != QMK_OK) return -1;
   return grid_for(e);
@@ -1027,7 +1037,7 @@ long long qmk_scratch_bytes(void) {
 }
 
 int qmk_selftest_wait_timeout(int budget_us) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   int rc = ensure_ready(e);
@@ -1072,7 +1082,7 @@ int qmk_generate_static(int first_token_id, int num_steps, const void *embed_wei
                         const void *lm_head_weight, void *k_cache, void *v_cache, void *g_normalized,
                         int *output_log, int num_layers, int start_position, int max_seq_len, float attn_scale,
                         int eos_token_id, cudaStream_t stream) {
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return QMK_ERR_CUDA;
   clear_error(e);

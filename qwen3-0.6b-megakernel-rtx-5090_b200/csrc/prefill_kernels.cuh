@@ -38,6 +38,23 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// Four values as fp16 at dst; SPLIT: also the fp16 rounding of what the first rounding left, `lo_off` halves further on.
+template <bool SPLIT>
+__device__ __forceinline__ void store_halves4(__half *dst, int lo_off, float4 v) {
+  const __half2 a = __floats2half2_rn(v.x, v.y), b = __floats2half2_rn(v.z, v.w);
+  uint2 out;
+  out.x = *reinterpret_cast<const uint32_t *>(&a);
+  out.y = *reinterpret_cast<const uint32_t *>(&b);
+  *reinterpret_cast<uint2 *>(dst) = out;
+  if (SPLIT) {
+    const __half2 la = __floats2half2_rn(v.x - __low2float(a), v.y - __high2float(a));
+    const __half2 lb = __floats2half2_rn(v.z - __low2float(b), v.w - __high2float(b));
+    out.x = *reinterpret_cast<const uint32_t *>(&la);
+    out.y = *reinterpret_cast<const uint32_t *>(&lb);
+    *reinterpret_cast<uint2 *>(dst + lo_off) = out;
+  }
+}
+
 // x[t][:] = embedding row of token t as fp32.  grid = T, block = 256.  `wq`: 0 fp16 rows; 1 FP8-E4M3 rows (H bytes,
 // then a 16-byte trailer with the fp32 row scale); 2 NVFP4 rows (H / 2 bytes of e2m1 pairs, low nibble first, H / 16
 // e4m3 block scales, then the trailer with the fp32 tensor scale).
@@ -71,6 +88,8 @@ __global__ void embed_rows(const int *tokens, const void *embed, int wq, float *
 // Residual add + RMSNorm: x[t] += add[t] (if add), y[t] = fp16(x[t] * rstd * w).  grid = T, block = 256.
 // `add` may come as `nparts` (<= 4) partial matrices `part_stride` floats apart (split-K GEMM output): they are
 // added in index order.
+// SPLIT: y is [T][2 x H], the fp16 rounding of the result and the fp16 rounding of what it left.
+template <bool SPLIT>
 __global__ void add_rmsnorm_rows(float *x, const float *add, int nparts, size_t part_stride, const __half *w, __half *y) {
   __shared__ float red[8];
   pdl_wait();
@@ -98,18 +117,16 @@ __global__ void add_rmsnorm_rows(float *x, const float *add, int nparts, size_t 
   const float rstd = 1.0f / sqrtf(tot * (1.0f / H) + RMS_EPS);
   if (add) *reinterpret_cast<float4 *>(xr + k0) = v;
   const __half2 w01 = *reinterpret_cast<const __half2 *>(&wraw.x), w23 = *reinterpret_cast<const __half2 *>(&wraw.y);
-  const __half2 y01 = __floats2half2_rn(v.x * rstd * __low2float(w01), v.y * rstd * __high2float(w01));
-  const __half2 y23 = __floats2half2_rn(v.z * rstd * __low2float(w23), v.w * rstd * __high2float(w23));
-  uint2 out;
-  out.x = *reinterpret_cast<const uint32_t *>(&y01);
-  out.y = *reinterpret_cast<const uint32_t *>(&y23);
-  *reinterpret_cast<uint2 *>(y + static_cast<size_t>(t) * H + k0) = out;
+  const float4 n = make_float4(v.x * rstd * __low2float(w01), v.y * rstd * __high2float(w01), v.z * rstd * __low2float(w23),
+                               v.w * rstd * __high2float(w23));
+  store_halves4<SPLIT>(y + static_cast<size_t>(t) * (SPLIT ? 2 * H : H) + k0, H, n);
 }
 
 // The same for long chunks: one WARP per row (grid = ceil(T / 8), block = 256), eight 16-byte pieces per lane, every
 // load of the lane issued before the first add.  The block-per-row form above keeps one piece per thread in flight
 // and needs two waves of blocks for 2048 rows; it spent its 7 us waiting, not copying.  (The sum of squares is added
 // in another order than above: results agree to rounding, not bit for bit.)
+template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 add_rmsnorm_rows_wide(float *x, const float *add, int nparts, size_t part_stride, const __half *w, __half *y, int T) {
   pdl_wait();
@@ -146,12 +163,9 @@ add_rmsnorm_rows_wide(float *x, const float *add, int nparts, size_t part_stride
   for (int i = 0; i < PIECES; ++i) {
     if (add) *reinterpret_cast<float4 *>(xr + 4 * (lane + 32 * i)) = v[i];
     const __half2 w01 = *reinterpret_cast<const __half2 *>(&wraw[i].x), w23 = *reinterpret_cast<const __half2 *>(&wraw[i].y);
-    const __half2 y01 = __floats2half2_rn(v[i].x * rstd * __low2float(w01), v[i].y * rstd * __high2float(w01));
-    const __half2 y23 = __floats2half2_rn(v[i].z * rstd * __low2float(w23), v[i].w * rstd * __high2float(w23));
-    uint2 out;
-    out.x = *reinterpret_cast<const uint32_t *>(&y01);
-    out.y = *reinterpret_cast<const uint32_t *>(&y23);
-    *reinterpret_cast<uint2 *>(y + static_cast<size_t>(t) * H + 4 * (lane + 32 * i)) = out;
+    const float4 n = make_float4(v[i].x * rstd * __low2float(w01), v[i].y * rstd * __high2float(w01),
+                                 v[i].z * rstd * __low2float(w23), v[i].w * rstd * __high2float(w23));
+    store_halves4<SPLIT>(y + static_cast<size_t>(t) * (SPLIT ? 2 * H : H) + 4 * (lane + 32 * i), H, n);
   }
 }
 
@@ -161,7 +175,8 @@ add_rmsnorm_rows_wide(float *x, const float *add, int nparts, size_t part_stride
 // all four issued before the first is used (the kernel is a few dependent round trips per warp: with one head per warp
 // and four blocks per token it spent 13 us on seven waves of blocks at 2048 tokens).
 // in_f16: q / k / v hold fp16 (the projection's epilogue stored halves) instead of fp32.
-// q_f16_scale != 0: the rotated queries are stored as fp16 times that factor (same [t][head][128] layout in halves).
+// q_f16_scale != 0: the rotated queries are stored as fp16 times that factor (same [t][head][128] layout in halves);
+// q_split: as hi and lo halves, [t][2][head][128].
 // Packed prompts (row_info != null): row t belongs to sequence row_info[t].x at position row_info[t].y (negative:
 // a padding row, nothing to do), whose K / V caches start at kv_ptrs[2 seq], kv_ptrs[2 seq + 1]; the layer's rows
 // begin `layer_off` halves into each.
@@ -170,7 +185,7 @@ qk_norm_rope_cache(const float *q, const float *k, const float *v, int in_f16, c
                    const __half *k_norm, const float *rope, const __half *cos_table,
                    const __half *sin_table, float *qr, __half *k_cache_layer, __half *v_cache_layer,
                    int pos0, int max_seq_len, const int2 *row_info, const unsigned long long *kv_ptrs, size_t layer_off,
-                   float q_f16_scale) {
+                   float q_f16_scale, int q_split) {
   pdl_wait();
   pdl_trigger();
   const int t = blockIdx.x, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -239,7 +254,10 @@ qk_norm_rope_cache(const float *q, const float *k, const float *v, int in_f16, c
     } else {            // high half: lo * sin + hi * cos
       r = make_float4(o.x * sn.x + a.x * cs.x, o.y * sn.y + a.y * cs.y, o.z * sn.z + a.z * cs.z, o.w * sn.w + a.w * cs.w);
     }
-    if (h < 2 && q_f16_scale != 0.f)   // fp16 queries, pre-scaled: the tcgen05 attention kernel takes them by TMA as they are
+    if (h < 2 && q_split)
+      store_halves4<true>(reinterpret_cast<__half *>(qr) + (static_cast<size_t>(t) * 2 * NQ + w + 8 * h) * D + d0, NQ * D,
+                          make_float4(r.x * q_f16_scale, r.y * q_f16_scale, r.z * q_f16_scale, r.w * q_f16_scale));
+    else if (h < 2 && q_f16_scale != 0.f)   // fp16 queries, pre-scaled: the tcgen05 attention kernel takes them by TMA as they are
       *reinterpret_cast<uint2 *>(reinterpret_cast<__half *>(qr) + (static_cast<size_t>(t) * NQ + w + 8 * h) * D + d0) =
           pack4(r.x * q_f16_scale, r.y * q_f16_scale, r.z * q_f16_scale, r.w * q_f16_scale);
     else if (h < 2)

@@ -129,6 +129,7 @@ static int sm_count() {
   }
   return sms > 0 ? sms : 148;
 }
+thread_local int t_ah = 1;                     // fp16 halves per activation (SplitActScope)
 thread_local unsigned int t_ring_budget = 0;   // shared-memory budget of the ring (0 = the compile-time depth, one CTA per SM)
 static int pick_box_n(int M, int N, int b_tiles) {
   const int sms = sm_count() * (t_ring_budget ? 2 : 1);   // CTA slots of one wave: rings sized to a budget share an SM in pairs
@@ -155,19 +156,22 @@ bool pdl_active() { return t_pdl; }
 // The kernel for an N tile, epilogue and weight format, and its dynamic shared memory.
 using GemmKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const qmk_gemm::Groups,
                             int, int, unsigned int *, unsigned long long, int);
-template <int WQ>
+template <int WQ, int AH>
 static GemmKernel gemm_kernel_wq(int bn, bool fuse) {
-  if (fuse) return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, true, WQ> : qmk_gemm::gemm_f16_tn_kernel<64, true, WQ>;
-  return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, false, WQ>
-                  : bn == 64 ? qmk_gemm::gemm_f16_tn_kernel<64, false, WQ> : qmk_gemm::gemm_f16_tn_kernel<128, false, WQ>;
+  if (fuse) return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, true, WQ, AH> : qmk_gemm::gemm_f16_tn_kernel<64, true, WQ, AH>;
+  return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, false, WQ, AH>
+                  : bn == 64 ? qmk_gemm::gemm_f16_tn_kernel<64, false, WQ, AH> : qmk_gemm::gemm_f16_tn_kernel<128, false, WQ, AH>;
 }
-// (the widest tiles - 256 B rows per stage - exist for fp16 weights only)
-static GemmKernel gemm_kernel(int bn, bool fuse, int wq) {
-  if (wq == 0 && fuse && bn == 128) return qmk_gemm::gemm_f16_tn_kernel<128, true, 0>;
-  if (wq == 0 && !fuse && bn == 256) return qmk_gemm::gemm_f16_tn_kernel<256, false, 0>;
-  return wq == 0 ? gemm_kernel_wq<0>(bn, fuse) : wq == 1 ? gemm_kernel_wq<1>(bn, fuse) : gemm_kernel_wq<2>(bn, fuse);
+// (the widest tiles - 256 B rows per stage - exist for fp16 weights only; split activations for fp16 and FP8 weights)
+static GemmKernel gemm_kernel(int bn, bool fuse, int wq, int ah) {
+  if (wq == 0 && fuse && bn == 128)
+    return ah == 2 ? qmk_gemm::gemm_f16_tn_kernel<128, true, 0, 2> : qmk_gemm::gemm_f16_tn_kernel<128, true, 0, 1>;
+  if (wq == 0 && !fuse && bn == 256)
+    return ah == 2 ? qmk_gemm::gemm_f16_tn_kernel<256, false, 0, 2> : qmk_gemm::gemm_f16_tn_kernel<256, false, 0, 1>;
+  if (ah == 2) return wq == 0 ? gemm_kernel_wq<0, 2>(bn, fuse) : gemm_kernel_wq<1, 2>(bn, fuse);
+  return wq == 0 ? gemm_kernel_wq<0, 1>(bn, fuse) : wq == 1 ? gemm_kernel_wq<1, 1>(bn, fuse) : gemm_kernel_wq<2, 1>(bn, fuse);
 }
-static size_t gemm_smem(int bn, bool fuse, int wq) { return qmk_gemm::smem_bytes_for(fuse ? 2 * bn : bn, wq); }
+static size_t gemm_smem(int bn, bool fuse, int wq, int ah) { return qmk_gemm::smem_bytes_for(fuse ? 2 * bn : bn, wq, ah); }
 
 // Opt-in shared-memory size of every tile variant, once per device (outside any stream capture).
 int ensure_gemm_attrs(std::string *err) {
@@ -176,17 +180,21 @@ int ensure_gemm_attrs(std::string *err) {
   std::lock_guard<std::mutex> lock(g_mu);
   if (dev >= 0 && dev < 16 && !g_attr_set[dev]) {
     cudaError_t e = cudaSuccess;
-    for (int wq = 0; wq < 3 && e == cudaSuccess; ++wq)
-      for (int fuse = 0; fuse < 2 && e == cudaSuccess; ++fuse)
-        for (int bn = 32; bn <= (fuse ? 64 : 128) * (wq == 0 ? 2 : 1) && e == cudaSuccess; bn *= 2)
-          e = cudaFuncSetAttribute(reinterpret_cast<const void *>(gemm_kernel(bn, fuse != 0, wq)),
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gemm_smem(bn, fuse != 0, wq)));
+    for (int ah = 1; ah < 3 && e == cudaSuccess; ++ah)
+      for (int wq = 0; wq < 4 - ah && e == cudaSuccess; ++wq)
+        for (int fuse = 0; fuse < 2 && e == cudaSuccess; ++fuse)
+          for (int bn = 32; bn <= (fuse ? 64 : 128) * (wq == 0 ? 2 : 1) && e == cudaSuccess; bn *= 2)
+            e = cudaFuncSetAttribute(reinterpret_cast<const void *>(gemm_kernel(bn, fuse != 0, wq, ah)),
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gemm_smem(bn, fuse != 0, wq, ah)));
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(qmk_pf::causal_attention_mma, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                qmk_pf::ATM_SMEM_BYTES);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(qmk_attn::SMEM_BYTES));
+      e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(qmk_attn::Layout<false>::SMEM_BYTES));
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(qmk_attn::Layout<true>::SMEM_BYTES));
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(qmk_pf::decode_attention_ring, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                qmk_pf::DAR_SMEM_BYTES);
@@ -220,7 +228,7 @@ static bool set_packed(qmk_gemm::Groups *gr, int wq, int K, int ngroups, const v
 thread_local float *t_amax_val = nullptr;   // the next single-matrix GEMM of this thread leaves (value, column) pairs here
 thread_local int *t_amax_idx = nullptr;
 static size_t set_ring(qmk_gemm::Groups *gr, int sb, int wq) {
-  const qmk_gemm::RingGeometry g = qmk_gemm::ring_geometry(sb, wq, t_ring_budget);
+  const qmk_gemm::RingGeometry g = qmk_gemm::ring_geometry(sb, wq, t_ring_budget, t_ah);
   gr->stages = g.stages;
   gr->ring_bytes = g.ring_bytes;
   return g.smem_bytes;
@@ -228,6 +236,8 @@ static size_t set_ring(qmk_gemm::Groups *gr, int sb, int wq) {
 
 RingBudgetScope::RingBudgetScope(unsigned int bytes) : prev_(t_ring_budget) { t_ring_budget = bytes; }
 RingBudgetScope::~RingBudgetScope() { t_ring_budget = prev_; }
+SplitActScope::SplitActScope(bool on) : prev_(t_ah) { t_ah = on ? 2 : 1; }
+SplitActScope::~SplitActScope() { t_ah = prev_; }
 void set_argmax_target(float *val, int *idx) { t_amax_val = val; t_amax_idx = idx; }
 thread_local bool t_out_f16 = false;        // the next grouped GEMM of this thread stores fp16
 void set_out_f16(bool on) { t_out_f16 = on; }
@@ -278,7 +288,7 @@ int launch_gemm_grouped(const CUtensorMap &map_a, int ngroups, const CUtensorMap
   int rows = live_rows > 0 ? live_rows : M;   // rows the epilogue stores (the rest of the tile is padding)
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
   const size_t smem = set_ring(&gr, box_n, wq);
-  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq), grid, dim3(qmk_gemm::threads_for(wq)), smem, stream,
+  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah), grid, dim3(qmk_gemm::threads_for(wq)), smem, stream,
                                 map_a, b0, b1, b2, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
   return QMK_OK;
@@ -310,7 +320,7 @@ int launch_gemm_swiglu(const CUtensorMap &map_a, const CUtensorMap &map_gate, co
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
   const size_t smem = set_ring(&gr, 2 * box_n, wq);
-  cudaError_t e = launch_kernel(gemm_kernel(box_n, true, wq), dim3(N / box_n, M / qmk_gemm::BM), dim3(qmk_gemm::threads_for(wq)),
+  cudaError_t e = launch_kernel(gemm_kernel(box_n, true, wq, t_ah), dim3(N / box_n, M / qmk_gemm::BM), dim3(qmk_gemm::threads_for(wq)),
                                 smem, stream, map_a, map_gate, map_up, map_up, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
   return QMK_OK;
@@ -341,7 +351,7 @@ int launch_gemm_splitk(const CUtensorMap &map_a, const CUtensorMap &map_b, float
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
   const size_t smem = set_ring(&gr, box_n, wq);
-  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq), dim3(N / box_n, M / qmk_gemm::BM, splits), dim3(qmk_gemm::threads_for(wq)),
+  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah), dim3(N / box_n, M / qmk_gemm::BM, splits), dim3(qmk_gemm::threads_for(wq)),
                                 smem, stream, map_a, map_b, map_b, map_b, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
   return QMK_OK;
@@ -373,6 +383,7 @@ struct Workspace {                  // per device, allocated on first use, never
   __half *xn = nullptr, *attn = nullptr, *act = nullptr;
   unsigned int *status = nullptr;
   CUtensorMap map_xn, map_attn, map_act, map_qh;
+  CUtensorMap map_xn2, map_attn2, map_act2, map_qh2;   // split activations: rows of hi and lo halves
   // batched decode: per-sequence state and the logits of one step
   int *positions = nullptr, *start_positions = nullptr;
   cudaStream_t gstream = nullptr;        // capture needs a non-default stream
@@ -409,7 +420,8 @@ struct Workspace {                  // per device, allocated on first use, never
 // Prefill and batched decode keep separate workspaces and locks: a serving loop prefills the next request on one
 // stream (and thread) while a decode step of the live sequences runs on another.
 Workspace g_ws[16], g_ws_decode[16];
-std::mutex g_ws_mu, g_ws_decode_mu;
+std::recursive_mutex g_ws_mu;   // (recursive: qmk_tc::prefill_split's caller holds it already, see prefill_lock)
+std::mutex g_ws_decode_mu;
 
 #define PF_CUDA(call)                                                                             \
   do {                                                                                            \
@@ -431,14 +443,15 @@ int ensure_workspace(Workspace &w, int rows) {
   PF_CUDA(cudaMalloc(&w.qr, sizeof(float) * C * QS));
   PF_CUDA(cudaMalloc(&w.o, sizeof(float) * 2 * C * H));      // (two split-K partial matrices of a prefill chunk)
   PF_CUDA(cudaMalloc(&w.down, sizeof(float) * 2 * C * H));
-  PF_CUDA(cudaMalloc(&w.xn, sizeof(__half) * C * H));
-  PF_CUDA(cudaMalloc(&w.attn, sizeof(__half) * C * QS));
-  PF_CUDA(cudaMalloc(&w.act, sizeof(__half) * C * I));
+  // (room for the hi and lo halves of split activations, [C][2 x width])
+  PF_CUDA(cudaMalloc(&w.xn, sizeof(__half) * C * 2 * H));
+  PF_CUDA(cudaMalloc(&w.attn, sizeof(__half) * C * 2 * QS));
+  PF_CUDA(cudaMalloc(&w.act, sizeof(__half) * C * 2 * I));
   PF_CUDA(cudaMalloc(&w.status, 16));
   // GEMM operand rows beyond a short chunk are read (and ignored): they must hold finite numbers
-  PF_CUDA(cudaMemset(w.xn, 0, sizeof(__half) * C * H));
-  PF_CUDA(cudaMemset(w.attn, 0, sizeof(__half) * C * QS));
-  PF_CUDA(cudaMemset(w.act, 0, sizeof(__half) * C * I));
+  PF_CUDA(cudaMemset(w.xn, 0, sizeof(__half) * C * 2 * H));
+  PF_CUDA(cudaMemset(w.attn, 0, sizeof(__half) * C * 2 * QS));
+  PF_CUDA(cudaMemset(w.act, 0, sizeof(__half) * C * 2 * I));
   PF_CUDA(cudaMemset(w.qr, 0, sizeof(float) * C * QS));
   std::string err;
   int rc = qmk_tc::make_map_f16(&w.map_xn, w.xn, C, H, qmk_gemm::BM, &err);
@@ -446,6 +459,11 @@ int ensure_workspace(Workspace &w, int rows) {
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_act, w.act, C, I, qmk_gemm::BM, &err);
   // the rotated queries as fp16 (the first half of the fp32 buffer), read by the attention kernel in 128-row boxes
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_qh, w.qr, C, QS, qmk_gemm::BM, &err);
+  // the same buffers as [C][hi | lo]
+  if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_xn2, w.xn, C, 2 * H, qmk_gemm::BM, &err);
+  if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_attn2, w.attn, C, 2 * QS, qmk_gemm::BM, &err);
+  if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_act2, w.act, C, 2 * I, qmk_gemm::BM, &err);
+  if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_qh2, w.qr, C, 2 * QS, qmk_gemm::BM, &err);
   if (rc != QMK_OK) return qmk_internal::report(rc, err);
   w.ready = true;
   return QMK_OK;
@@ -499,12 +517,13 @@ constexpr size_t PK_ROWS_OFF = 0, PK_ITEMS_OFF = 32768, PK_MAPS_OFF = 49152, PK_
 
 int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_weight, const LDGLayerWeight *layer_weights,
                  const void *cos_table, const void *sin_table, void *k_cache, void *v_cache, int num_layers,
-                 int start_position, int max_seq_len, float attn_scale, cudaStream_t stream, const PackedSeqs *pk) {
+                 int start_position, int max_seq_len, float attn_scale, cudaStream_t stream, const PackedSeqs *pk, bool split) {
   using namespace qmk_pf;
   if (num_tokens <= 0) return QMK_OK;
   qmk_internal::PrefillEnv env;
   int rc = qmk_internal::prefill_env(max_seq_len, stream, &env);
   if (rc != QMK_OK) return rc;
+  if (split) env.attn_tc = 1;   // (the mma.sync attention has no split form)
   if (!token_ids_host || !embed_weight || !layer_weights || (!pk && (!k_cache || !v_cache)))
     return qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "prefill: null pointer argument");
   const int wq = env.wfmt;   // 0 fp16, 1 FP8-E4M3 rows, 2 NVFP4 rows: packed matrices are expanded inside the GEMM
@@ -532,7 +551,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
   int dev = 0;
   PF_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 16) return qmk_internal::report(QMK_ERR_CUDA, "device index out of range");
-  std::lock_guard<std::mutex> lock(g_ws_mu);
+  std::lock_guard<std::recursive_mutex> lock(g_ws_mu);
   Workspace &w = g_ws[dev];
   rc = ensure_workspace(w, CHUNK);
   if (rc == QMK_OK) rc = ensure_weight_maps(w, layer_weights, num_layers, wq, stream);
@@ -598,11 +617,6 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
   };
   static const int rec_slot[7] = {1, 2, 3, 6, 8, 9, 10};   // q, k, v, o, gate, up, down inside a layer record
   auto wptr = [&](int l, int j) { return reinterpret_cast<const void *>(rec[static_cast<size_t>(l) * 12 + rec_slot[j]]); };
-  auto gemm = [&](const CUtensorMap &a, int l, int j, float *c, int M, int N, int K, int live) {
-    const int box_n = qmk_tc::gemm_box_n(M, N);
-    return qmk_tc::launch_gemm(a, wmap_for(l, j, box_n), c, M, N, K, box_n, w.status, env.timeout_ms, stream, &err, live, 0,
-                               wq, wptr(l, j));
-  };
   // several matrices against the same activations in one launch (q/k/v)
   auto gemm_group = [&](const CUtensorMap &a, int l, int n, const int *js, float *const *cs, const int *ns, int M, int K,
                         int live) {
@@ -629,17 +643,23 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     // halves the loop; the partial matrices are added by the residual + RMSNorm kernel that follows anyway.
     // Short chunks: four splits (M = 512: 32 tiles x 4 = 128 CTAs with K loops of 8 / 12 blocks; unsplit, the narrowest
     // tiles gave 128 CTAs with loops of 32 / 48 blocks of N = 32 MMAs and these two products were 41 % of the pass).
-    const int od_splits = wq != 0 ? 1 : M >= 1024 ? 2 : 4;
-    const size_t od_stride = od_splits > 1 ? static_cast<size_t>(M) * H : 0;
+    // Packed weights split only short chunks: a CTA expands its weight tile itself, so two CTAs with half a K loop each beat
+    // one only while there are too few tiles (93 tokens 2.06 -> 1.75 ms; 1023 tokens measured 1 % slower with two splits).
+    const int od_splits = M < 1024 ? 4 : wq == 0 ? 2 : 1;
+    const size_t od_stride = static_cast<size_t>(M) * H;
     auto gemm_od = [&](const CUtensorMap &a, int l, int j, float *c, int Mrows, int K, int live) {
-      if (od_splits == 1) return gemm(a, l, j, c, Mrows, H, K, live);
       // 256-wide tiles, one CTA per SM with the whole ring: the main loops are bound by shared-memory traffic (TMA
       // writes + MMA operand reads), and a 256-wide tile moves a quarter fewer bytes per flop than a 128-wide one
       // (2048 tokens: 4.12 -> 4.07 ms per pass, same box); shorter chunks would leave SMs without a tile
-      if (Mrows >= 2048) {
+      if (Mrows >= 2048 && wq == 0) {
         qmk_tc::RingBudgetScope whole(0);
         return qmk_tc::launch_gemm_splitk(a, wmap_for(l, j, 256), c, Mrows, H, K, od_splits, w.status, env.timeout_ms, stream, &err,
                                           256, live, 0, wq, wptr(l, j));
+      }
+      if (od_splits == 1) {
+        const int box_n = qmk_tc::gemm_box_n(Mrows, H);
+        return qmk_tc::launch_gemm(a, wmap_for(l, j, box_n), c, Mrows, H, K, box_n, w.status, env.timeout_ms, stream, &err, live, 0, wq,
+                                   wptr(l, j));
       }
       return qmk_tc::launch_gemm_splitk(a, wmap_for(l, j, 128), c, Mrows, H, K, od_splits, w.status, env.timeout_ms, stream, &err, 128,
                                         live, 0, wq, wptr(l, j));
@@ -664,6 +684,9 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     // showed it (128 prefill + decode cycles compared bit for bit, and the test that found it runs every time).
     qmk_tc::PdlScope pdl_scope(false);
     const bool pdl_gemm = env.pdl != 0;
+    qmk_tc::SplitActScope split_scope(split);
+    const CUtensorMap &map_xn = split ? w.map_xn2 : w.map_xn, &map_attn = split ? w.map_attn2 : w.map_attn,
+                      &map_act = split ? w.map_act2 : w.map_act, &map_qh = split ? w.map_qh2 : w.map_qh;
     qmk_tc::RingBudgetScope ring_scope(PREFILL_RING_BYTES);   // two GEMM CTAs per SM: one's epilogue under the other's main loop
     {
       qmk_tc::PdlScope first(false);            // (follows a copy, not a kernel)
@@ -672,9 +695,9 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     // residual add (+ split-K partials) and RMSNorm: a warp per row for long chunks, a block per row for short ones
     auto norm_rows = [&](const float *add, const __half *g) {
       if (T >= 256 && od_splits <= 2)
-        return qmk_tc::launch_kernel(add_rmsnorm_rows_wide, dim3((T + 7) / 8), dim3(256), 0, stream, w.x, add, od_splits, od_stride, g,
-                                     w.xn, T);
-      return qmk_tc::launch_kernel(add_rmsnorm_rows, dim3(T), dim3(256), 0, stream, w.x, add, od_splits, od_stride, g, w.xn);
+        return qmk_tc::launch_kernel(split ? add_rmsnorm_rows_wide<true> : add_rmsnorm_rows_wide<false>, dim3((T + 7) / 8), dim3(256), 0,
+                                     stream, w.x, add, od_splits, od_stride, g, w.xn, T);
+      return qmk_tc::launch_kernel(split ? add_rmsnorm_rows<true> : add_rmsnorm_rows<false>, dim3(T), dim3(256), 0, stream, w.x, add, od_splits, od_stride, g, w.xn);
     };
     for (int l = 0; l < num_layers; ++l) {
       const unsigned long long *r = rec.data() + static_cast<size_t>(l) * 12;
@@ -687,27 +710,30 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
         const int ns[3] = {QS, KVS, KVS};
         // fp16 q / k / v: every CTA of this launch reaches its epilogue at the same time, and the burst of stores set
         // its length (9.8 of 26 us at 2048 rows with fp32); the consumer below rounds to fp16 anyway
-        qmk_tc::set_out_f16(true);
+        // (split activations: fp32, the operands downstream are not rounded to fp16)
+        qmk_tc::set_out_f16(!split);
         {
           qmk_tc::PdlScope g(pdl_gemm);
-          rc = gemm_group(w.map_xn, l, 3, js, cs, ns, M, H, T);
+          rc = gemm_group(map_xn, l, 3, js, cs, ns, M, H, T);
         }
         qmk_tc::set_out_f16(false);
         if (rc != QMK_OK) break;
       }
       // (Folding this kernel into the q/k/v GEMM's epilogue - one 128-wide N tile is one head - was built and measured
       // slower: 128 threads per CTA walking TMEM eight columns at a time lose to 2300 x 4 fully parallel CTAs.)
-      PF_CUDA(qmk_tc::launch_kernel(qk_norm_rope_cache, dim3(T), dim3(256), 0, stream, w.q, w.k, w.v, 1,
+      PF_CUDA(qmk_tc::launch_kernel(qk_norm_rope_cache, dim3(T), dim3(256), 0, stream, w.q, w.k, w.v, split ? 0 : 1,
                                     reinterpret_cast<const __half *>(r[4]), reinterpret_cast<const __half *>(r[5]), rope, cosv, sinv,
                                     w.qr, kc, vc, pos0, max_seq_len,
                                     pk ? reinterpret_cast<const int2 *>(w.packed + PK_ROWS_OFF) : nullptr,
                                     pk ? reinterpret_cast<const unsigned long long *>(w.packed + PK_PTRS_OFF) : nullptr,
                                     static_cast<size_t>(l) * layer_stride,
-                                    env.attn_tc ? attn_scale * 1.4426950408889634f : 0.f));
+                                    env.attn_tc ? attn_scale * 1.4426950408889634f : 0.f, split ? 1 : 0));
       if (l == num_layers - 1) break;   // the cache is complete; nothing downstream of the last layer is kept
       if (env.attn_tc)
-        PF_CUDA(qmk_tc::launch_kernel(qmk_attn::causal_attention_tc, dim3(pk ? pk_items : (T + qmk_attn::TQ - 1) / qmk_attn::TQ * NQ),
-                                      dim3(qmk_attn::THREADS), qmk_attn::SMEM_BYTES, stream, w.map_qh, map_kc, map_vc, l * NKV, w.attn, T,
+        PF_CUDA(qmk_tc::launch_kernel(split ? qmk_attn::causal_attention_tc<true> : qmk_attn::causal_attention_tc<false>,
+                                      dim3(pk ? pk_items : (T + qmk_attn::TQ - 1) / qmk_attn::TQ * NQ), dim3(qmk_attn::THREADS),
+                                      split ? qmk_attn::Layout<true>::SMEM_BYTES : qmk_attn::Layout<false>::SMEM_BYTES, stream, map_qh,
+                                      map_kc, map_vc, l * NKV, w.attn, T,
                                       pos0, attn_scale, w.status, static_cast<unsigned long long>(env.timeout_ms) * 1000000ull,
                                       pk ? reinterpret_cast<const int4 *>(w.packed + PK_ITEMS_OFF) : nullptr,
                                       pk ? reinterpret_cast<const CUtensorMap *>(w.packed + PK_MAPS_OFF) : nullptr));
@@ -716,7 +742,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
                                       w.qr, kc, vc, w.attn, T, pos0, max_seq_len, attn_scale));
       {
         qmk_tc::PdlScope g(pdl_gemm);
-        rc = gemm_od(w.map_attn, l, 3, w.o, M, QS, T);
+        rc = gemm_od(map_attn, l, 3, w.o, M, QS, T);
       }
       if (rc != QMK_OK) break;
       PF_CUDA(norm_rows(w.o, reinterpret_cast<const __half *>(r[7])));
@@ -726,14 +752,14 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
         qmk_tc::RingBudgetScope gu_scope(M >= 1024 ? GATE_UP_RING_BYTES : PREFILL_RING_BYTES);
         {
           qmk_tc::PdlScope g(pdl_gemm);
-          rc = qmk_tc::launch_gemm_swiglu(w.map_xn, wmap_for(l, 4, box_gu), wmap_for(l, 5, box_gu), w.act, M, I, H, w.status,
+          rc = qmk_tc::launch_gemm_swiglu(map_xn, wmap_for(l, 4, box_gu), wmap_for(l, 5, box_gu), w.act, M, I, H, w.status,
                                           env.timeout_ms, stream, &err, box_gu, T, 0, wq, wptr(l, 4), wptr(l, 5));
         }
         if (rc != QMK_OK) break;
       }
       {
         qmk_tc::PdlScope g(pdl_gemm);
-        rc = gemm_od(w.map_act, l, 6, w.down, M, I, T);
+        rc = gemm_od(map_act, l, 6, w.down, M, I, T);
       }
       if (rc != QMK_OK) break;
     }
@@ -757,8 +783,21 @@ extern "C" int qmk_prefill_chunked(const int *token_ids_host, int num_tokens, co
                                    void *k_cache, void *v_cache, int num_layers, int start_position, int max_seq_len,
                                    float attn_scale, cudaStream_t stream) {
   return prefill_impl(token_ids_host, num_tokens, embed_weight, layer_weights, cos_table, sin_table, k_cache, v_cache, num_layers,
-                      start_position, max_seq_len, attn_scale, stream, nullptr);
+                      start_position, max_seq_len, attn_scale, stream, nullptr, false);
 }
+
+namespace qmk_tc {
+// The chunked pass with split activations, for qmk_prefill (fp32 activations at the precision of the token-serial kernels).
+// Locks: the caller takes prefill_lock() BEFORE the engine's lock and holds both - the order in which every other path
+// meets them (prefill_impl reports errors to the engine while it holds the workspace).
+std::unique_lock<std::recursive_mutex> prefill_lock() { return std::unique_lock<std::recursive_mutex>(g_ws_mu); }
+int prefill_split(const int *token_ids_host, int num_tokens, const void *embed_weight, const LDGLayerWeight *layer_weights,
+                  const void *cos_table, const void *sin_table, void *k_cache, void *v_cache, int num_layers, int start_position,
+                  int max_seq_len, float attn_scale, cudaStream_t stream) {
+  return prefill_impl(token_ids_host, num_tokens, embed_weight, layer_weights, cos_table, sin_table, k_cache, v_cache, num_layers,
+                      start_position, max_seq_len, attn_scale, stream, nullptr, true);
+}
+}  // namespace qmk_tc
 
 extern "C" int qmk_prefill_packed(const int *token_ids_host, int num_seqs, const int *seq_lens, const void *embed_weight,
                                   const LDGLayerWeight *layer_weights, const void *cos_table, const void *sin_table,
@@ -770,7 +809,7 @@ extern "C" int qmk_prefill_packed(const int *token_ids_host, int num_seqs, const
   for (int s = 0; s < num_seqs && s < MAX_PACKED_SEQS; ++s) total += seq_lens[s] > 0 ? seq_lens[s] : 0;
   const PackedSeqs pk = {num_seqs, seq_lens, k_caches, v_caches};
   return prefill_impl(token_ids_host, static_cast<int>(total), embed_weight, layer_weights, cos_table, sin_table, nullptr, nullptr,
-                      num_layers, 0, max_seq_len, attn_scale, stream, &pk);
+                      num_layers, 0, max_seq_len, attn_scale, stream, &pk, false);
 }
 
 // ----------------------------------------------------------------------------- batched decode on the GEMM path
@@ -938,7 +977,7 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
       auto wm = [&](int j) -> const CUtensorMap & { return w.wmap32[l][j]; };
       static const int rec_slot[7] = {1, 2, 3, 6, 8, 9, 10};   // q, k, v, o, gate, up, down inside a layer record
       auto wp = [&](int j) { return reinterpret_cast<const void *>(r[rec_slot[j]]); };
-      PF_CUDA(qmk_tc::launch_kernel(add_rmsnorm_rows, dim3(B), dim3(256), 0, s, w.x, l > 0 ? w.down : nullptr, DOWN_SPLITS, PART,
+      PF_CUDA(qmk_tc::launch_kernel(add_rmsnorm_rows<false>, dim3(B), dim3(256), 0, s, w.x, l > 0 ? w.down : nullptr, DOWN_SPLITS, PART,
                                     reinterpret_cast<const __half *>(r[0]), w.xn));
       {
         const CUtensorMap *maps[3] = {&wm(0), &wm(1), &wm(2)};
@@ -964,7 +1003,7 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
       if ((r2 = qmk_tc::launch_gemm_splitk(w.map_attn_b, wm(3), w.o, M, H, QS, O_SPLITS, w.status, env.timeout_ms, s, &err,
                                            TILE_N, live, a_box, wq, wp(3))) != QMK_OK)
         return r2;
-      PF_CUDA(qmk_tc::launch_kernel(add_rmsnorm_rows, dim3(B), dim3(256), 0, s, w.x, w.o, O_SPLITS, PART,
+      PF_CUDA(qmk_tc::launch_kernel(add_rmsnorm_rows<false>, dim3(B), dim3(256), 0, s, w.x, w.o, O_SPLITS, PART,
                                     reinterpret_cast<const __half *>(r[7]), w.xn));
       if ((r2 = qmk_tc::launch_gemm_swiglu(w.map_xn_b, wm(4), wm(5), w.act, M, I, H, w.status, env.timeout_ms, s, &err, TILE_N,
                                            live, a_box, wq, wp(4), wp(5))) != QMK_OK)
@@ -973,7 +1012,7 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
                                            TILE_N, live, a_box, wq, wp(6))) != QMK_OK)
         return r2;
     }
-    PF_CUDA(qmk_tc::launch_kernel(add_rmsnorm_rows, dim3(B), dim3(256), 0, s, w.x, w.down, DOWN_SPLITS, PART,
+    PF_CUDA(qmk_tc::launch_kernel(add_rmsnorm_rows<false>, dim3(B), dim3(256), 0, s, w.x, w.down, DOWN_SPLITS, PART,
                                   static_cast<const __half *>(final_norm_weight), w.xn));
     // Without a logits dump the LM head's epilogue picks the largest logit of each 128-column tile itself and the
     // rows of logits (B x 608 KB per step) are never written

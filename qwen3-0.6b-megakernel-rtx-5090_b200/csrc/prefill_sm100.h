@@ -6,7 +6,10 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <mutex>
 #include <string>
+
+struct LDGLayerWeight;
 
 namespace qmk_tc {
 // While one is alive on a thread, launch_kernel() on that thread adds the programmatic-stream-serialisation attribute.
@@ -30,6 +33,15 @@ class RingBudgetScope {
   ~RingBudgetScope();
  private:
   unsigned int prev_;
+};
+// While one is alive on a thread, GEMM launches of that thread take their A operand as hi and lo halves ([M x 2 K], the AH = 2
+// kernels of gemm_tcgen05.cuh).
+class SplitActScope {
+ public:
+  explicit SplitActScope(bool on);
+  ~SplitActScope();
+ private:
+  int prev_;
 };
 size_t selftest_ring(qmk_gemm::Groups *gr);   // ring geometry of the bounded-wait self test's one-tile launch
 template <typename... KArgs, typename... Args>
@@ -75,6 +87,10 @@ int launch_gemm_grouped(const CUtensorMap &map_a, int ngroups, const CUtensorMap
 int launch_gemm(const CUtensorMap &map_a, const CUtensorMap &map_b, float *C, int M, int N, int K, int box_n,
                 unsigned int *status, int timeout_ms, cudaStream_t stream, std::string *err, int live_rows = 0, int a_box_rows = 0,
                 int wq = 0, const void *raw = nullptr);
+std::unique_lock<std::recursive_mutex> prefill_lock();
+int prefill_split(const int *token_ids_host, int num_tokens, const void *embed_weight, const LDGLayerWeight *layer_weights,
+                  const void *cos_table, const void *sin_table, void *k_cache, void *v_cache, int num_layers, int start_position,
+                  int max_seq_len, float attn_scale, cudaStream_t stream);
 }  // namespace qmk_tc
 
 #endif  // QMK_PREFILL_SM100_H_

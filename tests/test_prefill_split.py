@@ -1,0 +1,50 @@
+"""The ``prefill`` op on the tensor cores with split activations (hi + lo fp16 halves of every fp32 operand) against the
+CPU oracle, which keeps fp32 activations.
+
+Bounds: hi + lo drops at most 2^-22 of an operand, so a first-layer row differs from the oracle's only where an fp32
+result sits within rounding error (near 1e-6) of an fp16 tie of the cache (spacing near 1e-3): one fp16 ulp, in about one
+value of a thousand, root mean square 1e-3 * sqrt(1e-3) = 3e-5.  Each such flip of a V row then moves the attention output
+of every later layer by about that rms, which flips some per cent of the rows there: 1e-3 * sqrt(3e-2) = 1.7e-4 (the
+token-serial kernel shows 0.6e-4 on three tokens), and a flip can land on a moved value: two ulps.  Operands rounded to
+fp16 once show 4e-3 to 6e-3 at the largest and fail both."""
+
+import pytest
+import torch
+
+import synthetic as S
+from oracle.decoder_ref import Decoder as OracleDecoder
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("fmt,calls", [("fp16", (3,)), ("fp16", (4,)), ("fp16", (127,)), ("fp16", (2, 129, 70)), ("fp16", (1100,)),
+                                       ("fp8", (5,)), ("fp8", (260,))])
+def test_rows_match_fp32_oracle(built_library, fmt, calls):
+    """Lengths below the op's switch to the tensor cores and at it, tile edges, a second call behind a first one, a chunk
+    long enough for the wide tiles."""
+    import qwen_megakernel_C as C
+    import quantize as Q
+    from Model.Qwen06B_architecture import Decoder
+    w = S.make_weights(seed=21, num_layers=3, vocab_size=2048, norm_std=0.1, max_seq_len=16)
+    engine_w, oracle_w = Q.quantize_weights_fp8(w) if fmt == "fp8" else (w, w)
+    n = sum(calls)
+    ids = S.make_prompt(n, seed=n, vocab_size=2048)
+    o = OracleDecoder(oracle_w, max_seq_len=1280)
+    o.prefill(ids)
+    try:
+        eng = Decoder(weights=S.weights_to(engine_w, "cuda"), verbose=False, max_seq_len=1280, weight_format=fmt)
+        at = 0
+        for c in calls:
+            eng.prefill_ids(ids[at:at + c])
+            at += c
+    finally:
+        C.set_weight_format("fp16")
+    for got, want in ((eng._k_cache, o.k_cache), (eng._v_cache, o.v_cache)):
+        want = want[:, :, :n].float()
+        diff = (got[:, :, :n].float().cpu() - want).abs()
+        print(f"{fmt} {calls}: max {float(diff.max()):.2e} rms {float(diff.square().mean().sqrt()):.2e} "
+              f"first layer {float(diff[0].max()):.2e} {float(diff[0].square().mean().sqrt()):.2e}")
+        ulp = want.abs().clamp(min=2.0) * 2.0 ** -10
+        assert bool((diff[0] <= ulp[0]).all()) and bool((diff <= 2 * ulp).all())
+        assert float(diff[0].square().mean().sqrt()) < 6e-5 and float(diff.square().mean().sqrt()) < 3.4e-4
+    assert torch.count_nonzero(eng._k_cache[:, :, n:]) == 0
