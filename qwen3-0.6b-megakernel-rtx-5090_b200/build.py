@@ -15,7 +15,7 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SOURCES = [os.path.join(HERE, "csrc", "megakernel_sm100.cu"), os.path.join(HERE, "csrc", "megakernel_batch_sm100.cu"),
-           os.path.join(HERE, "csrc", "megakernel_tc_sm100.cu"),
+           os.path.join(HERE, "csrc", "megakernel_tc_sm100.cu"), os.path.join(HERE, "csrc", "megakernel_tc_fp8_sm100.cu"),
            os.path.join(HERE, "csrc", "prefill_sm100.cu")]
 HEADERS = [os.path.join(os.path.dirname(HERE), "include", "qwen_megakernel.h"),
            os.path.join(HERE, "csrc", "megakernel_device.cuh"), os.path.join(HERE, "csrc", "megakernel_params.h"),

@@ -435,6 +435,7 @@ __device__ __forceinline__ constexpr int kind_k(int kind) { return kind == K_O ?
 // four bytes are the row's fp32 scale (the trailer keeps rows 16-byte aligned for bulk copies and brings
 // the scale into shared memory with the row).
 constexpr int FP8_TRAILER = 16;
+constexpr int FP8_PITCH = H + FP8_TRAILER;   // bytes of a row of 1024 e4m3 values, and between the rows of a K-major fp8 copy
 __device__ __forceinline__ constexpr int kind_row_bytes(int kind, int wfmt) {
   return wfmt ? kind_k(kind) + FP8_TRAILER : kind_k(kind) * 2;
 }

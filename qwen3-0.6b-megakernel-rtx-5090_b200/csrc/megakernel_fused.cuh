@@ -143,7 +143,7 @@ __device__ __noinline__ uint32_t slice_colgemv(const Params &P, Ctx c, int which
   float *prev = c.f(FF_PREV) + (which ? H : 0);
   const int g = c.warp >> 2, cb = c.warp & 3;
   const int nch = (nrows + SLICE_ROWS_PER_CHUNK - 1) / SLICE_ROWS_PER_CHUNK;
-  const int trb = wfmt ? H : 2 * H;                 // bytes of a K-major row
+  const int trb = wfmt ? FP8_PITCH : 2 * H;                 // bytes of a K-major row
   const int col8 = cb * 32 + c.lane;                // group of eight outputs this lane owns
   float acc[8];
 #pragma unroll
@@ -172,7 +172,7 @@ __device__ __noinline__ uint32_t slice_colgemv(const Params &P, Ctx c, int which
   }
   if (wfmt) {   // per-output scales of the fp8 matrix: they follow its K rows
     const float *col_scale = reinterpret_cast<const float *>(
-        reinterpret_cast<const unsigned char *>(c.layer_rec_t(layer)[which]) + static_cast<size_t>(which ? I : QS) * H);
+        reinterpret_cast<const unsigned char *>(c.layer_rec_t(layer)[which]) + static_cast<size_t>(which ? I : QS) * FP8_PITCH);
     const float4 s0 = __ldg(reinterpret_cast<const float4 *>(col_scale) + col8 * 2);
     const float4 s1 = __ldg(reinterpret_cast<const float4 *>(col_scale) + col8 * 2 + 1);
     acc[0] *= s0.x; acc[1] *= s0.y; acc[2] *= s0.z; acc[3] *= s0.w;
@@ -304,7 +304,7 @@ __device__ __noinline__ void producer_main_fused(const Params &P, const Ctx c) {
   const SegTab *t = c.segs();
   const int e0 = t->e0, ne = t->e1 - t->e0;
   const int m0 = t->nseg[K_GU] ? t->row0[K_GU][0] : 0, nm = t->nseg[K_GU] ? t->nrows[K_GU][0] : 0;
-  const int trb = P.wfmt ? H : 2 * H;
+  const int trb = P.wfmt ? FP8_PITCH : 2 * H;
   uint32_t idx = 0;
   bool ok = true;
 #pragma unroll 1

@@ -17,8 +17,8 @@ struct __align__(16) LayerW {
 // K-major copies of the two projections whose input is produced slice by slice (O: the attention output, down:
 // the MLP activations).  The library makes them from the caller's [out,in] matrices: row e of wo_t holds
 // W_o[:, e], row m of wd_t holds W_down[:, m] (1024 outputs each), so that the rows a CTA needs for ITS slice of
-// the input form one contiguous range.  fp8 format: 1024 e4m3 bytes per row, the per-output fp32 scales of the
-// matrix follow the last row.
+// the input form one contiguous range.  fp8 format: 1024 e4m3 bytes + 16 unused bytes per row (a
+// conflict-free pitch in shared memory), the per-output fp32 scales of the matrix follow the last row.
 struct __align__(16) LayerT {
   const void *wo_t, *wd_t;
 };

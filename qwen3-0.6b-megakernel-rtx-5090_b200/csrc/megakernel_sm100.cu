@@ -142,12 +142,12 @@ __global__ void __launch_bounds__(256) kmajor_prepare_kernel(const PrepArgs a) {
       for (int i = 0; i < 4; ++i) tile8[ty + 8 * i][tx] = src[static_cast<size_t>(tn * 32 + ty + 8 * i) * in_row + tk * 32 + tx];
       __syncthreads();
 #pragma unroll
-      for (int i = 0; i < 4; ++i) dst[static_cast<size_t>(tk * 32 + ty + 8 * i) * H + tn * 32 + tx] = tile8[tx][ty + 8 * i];
+      for (int i = 0; i < 4; ++i) dst[static_cast<size_t>(tk * 32 + ty + 8 * i) * FP8_PITCH + tn * 32 + tx] = tile8[tx][ty + 8 * i];
     }
     __syncthreads();
   }
   if (a.wfmt && blockIdx.x == 0) {                    // per-output scales follow the K rows
-    float *sc = reinterpret_cast<float *>(dst + static_cast<size_t>(K) * H);
+    float *sc = reinterpret_cast<float *>(dst + static_cast<size_t>(K) * FP8_PITCH);
     for (int n = t; n < H; n += 256) sc[n] = *reinterpret_cast<const float *>(src + static_cast<size_t>(n) * in_row + K);
   }
 }
@@ -202,7 +202,7 @@ struct Engine {
   bool inv_freq_set = false;
   float inv_freq[qmk::D / 2] = {};   // host copy of what c_inv_freq holds (when inv_freq_set)
   // fused single-sequence kernel (megakernel_fused.cuh)
-  int fused = 2;             // 0: always the unfused kernel; 1: fused, CUDA-core row products; 2: fused, tensor-core row products (fp16 weights)
+  int fused = 2;             // 0: always the unfused kernel; 1: fused, CUDA-core row products; 2: fused, tensor-core row products
   int red_copies = 1;
   int decode_attn_mma = 1;   // batched decode: attention on mma.sync (0: the CUDA-core ring kernel)
   int prefill_attn_tc = 1;   // chunked prefill: attention on tcgen05 (0: the mma.sync kernel)
@@ -280,8 +280,9 @@ int ensure_ready(Engine *e) {
   if (e->grid > qmk::MAX_CTAS) e->grid = qmk::MAX_CTAS;
   QMK_CUDA(e, cudaFuncSetAttribute(qmk_batch::kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(qmk_batch::smem_bytes())));
-  QMK_CUDA(e, cudaFuncSetAttribute(qmk_fused_tc::kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(qmk_fused_tc::smem_bytes())));
+  for (int wfmt = 0; wfmt < 2; ++wfmt)
+    QMK_CUDA(e, cudaFuncSetAttribute(qmk_fused_tc::build(wfmt).kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(qmk_fused_tc::build(wfmt).smem_bytes)));
   QMK_CUDA(e, cudaMalloc(&e->ll, exchange_bytes()));
   QMK_CUDA(e, cudaMemset(e->ll, 0, exchange_bytes()));
   QMK_CUDA(e, cudaMalloc(&e->status, 16));
@@ -336,11 +337,11 @@ int ensure_rope(Engine *e, int max_seq_len, cudaStream_t stream) {
 
 // Bytes of the K-major copies of one layer: O rows then down rows (fp8: each followed by 1024 fp32 scales).
 size_t kmajor_o_bytes(int wfmt) {
-  const size_t b = wfmt ? static_cast<size_t>(qmk::QS) * qmk::H + qmk::H * 4 : static_cast<size_t>(qmk::QS) * qmk::H * 2;
+  const size_t b = wfmt ? static_cast<size_t>(qmk::QS) * qmk::FP8_PITCH + qmk::H * 4 : static_cast<size_t>(qmk::QS) * qmk::H * 2;
   return (b + 255) / 256 * 256;
 }
 size_t kmajor_d_bytes(int wfmt) {
-  const size_t b = wfmt ? static_cast<size_t>(qmk::I) * qmk::H + qmk::H * 4 : static_cast<size_t>(qmk::I) * qmk::H * 2;
+  const size_t b = wfmt ? static_cast<size_t>(qmk::I) * qmk::FP8_PITCH + qmk::H * 4 : static_cast<size_t>(qmk::I) * qmk::H * 2;
   return (b + 255) / 256 * 256;
 }
 void free_prepared(Engine::Prepared &p) {
@@ -478,16 +479,19 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
     P.red_copies = e->red_copies;
     P.spin_sleep_ns = e->fused_sleep_ns;
     kernel = reinterpret_cast<const void *>(qmk::qwen3_decode_megakernel_fused);
-    // row products on the tensor cores: fp16 weights, rows owned in units of four
-    if (e->fused >= 2 && e->wfmt == 0 && P.vocab % 4 == 0 && grid >= qmk_fused_tc::min_ctas()) {
+    // row products on the tensor cores: rows owned in units of one ring chunk (four fp16 rows, eight fp8 rows).  fp8:
+    // 724 -> 533 us per token at 1024-token contexts against the CUDA-core kernel, which stays for the grids and
+    // vocabularies outside these limits.
+    const qmk_fused_tc::Build &tc = qmk_fused_tc::build(e->wfmt);
+    if (e->fused >= 2 && P.vocab % tc.rows_per_chunk == 0 && grid >= tc.min_ctas && grid <= tc.max_ctas) {
       // tiled-copy descriptors of the caller's caches (host-side encode, a few microseconds)
       std::string merr;
       const uint64_t kv_rows = static_cast<uint64_t>(P.num_layers) * qmk::NKV * static_cast<uint64_t>(P.max_seq_len);
       rc = qmk_tc::make_map_f16(reinterpret_cast<CUtensorMap *>(P.kmap), P.k_cache, kv_rows, qmk::D, 16, &merr);
       if (rc == QMK_OK) rc = qmk_tc::make_map_f16(reinterpret_cast<CUtensorMap *>(P.vmap), P.v_cache, kv_rows, qmk::D, 16, &merr);
       if (rc != QMK_OK) return fail(e, rc, "KV cache tensor map: " + merr);
-      kernel = qmk_fused_tc::kernel();
-      smem = qmk_fused_tc::smem_bytes();
+      kernel = tc.kernel;
+      smem = tc.smem_bytes;
     }
   }
   cudaError_t err =

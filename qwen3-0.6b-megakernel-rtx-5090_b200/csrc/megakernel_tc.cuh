@@ -1,4 +1,5 @@
-// Fused single-sequence decode kernel whose row products run on the tensor cores (fp16 weights).
+// Fused single-sequence decode kernel whose row products run on the tensor cores (fp16 weights; FP8-E4M3 rows with
+// QMK_TC_FP8).
 //
 // Same layer structure as megakernel_fused.cuh (four cross-CTA hand-overs per layer, integer all-reduced residual
 // sums) and the same attention items, merge and exchange code.  What changes is how a CTA multiplies its weight
@@ -20,17 +21,47 @@
 // (one bulk copy per padded 256-byte row was tried: the copy engine takes ~30 cycles per copy whatever its size,
 // and 480 copies per layer made the attention phase slower than the CUDA-core loop).
 // CTAs own whole chunks: rows of the fused q|k|v matrix, of gate/up and of the LM head are split in units of four.
+//
+// FP8 rows (QMK_TC_FP8): the four hand-overs of a layer, not bytes, are most of the time, so what the format can gain
+// over fp16 rows is the difference in bytes and no more - as long as its row products are not slower.  In the CUDA-core
+// kernel they were (one convert and one FMA per weight): 724 us per token at a 1024-token context.
+// Here the tiles take the fp16 form's few instructions: one ldmatrix.x4 brings 16 rows x 32 weights, eight
+// cvt.rn.f16x2.e4m3x2 (exact) make the A operands of two MMAs of it.  A lane's register holds four consecutive inputs,
+// an MMA fragment wants inputs 2q, 2q + 1 and 2q + 8, 2q + 9: the activations are stored in the permuted order instead
+// (xf_offset).  A packed row is 1040 bytes in memory, which is a conflict-free pitch in shared memory too: a chunk
+// is eight rows and ONE bulk copy (four 2 KB rows: four copies).  Row scales multiply the finished sums (they sit in
+// the rows' trailers); the per-output scales of the K-major O / down copies travel as one more chunk of those phases.
+// Measured after: 533 us per token (a request of 1024 + 64 tokens 48.8 -> 36.6 ms).  Against float64 the cache rows are as
+// far off as the CUDA-core kernel's (V rows of the first layer that round differently: 0.086 % and 0.084 %).
 
 namespace QMK_NS {
 #if QMK_MAX_SEQ == 1 && defined(QMK_TC_BUILD)
 
 constexpr int TC_MIN_CTAS = 96;                // smallest grid: <= 2 attention outputs per warp to merge, O / down slices of <= 32 rows
 static_assert(TC_MIN_CTAS >= FUSED_MIN_CTAS, "the tensor-core kernel shares the fused kernel's slice layout");
-static_assert(4 * ((I / 4 + TC_MIN_CTAS - 1) / TC_MIN_CTAS) <= 32, "slice_cols takes two k-steps");
-constexpr int ROW_PITCH = 2 * H + 16;          // bytes between the rows of a chunk in shared memory
-constexpr int CH_ROWS = 4;
-constexpr int ODD_SLOT_SKEW = 64;              // weight rows of chunks in odd slots start four 16-byte bank groups later
-static_assert(SLOT_BYTES >= ODD_SLOT_SKEW + CH_ROWS * ROW_PITCH, "a slot holds four padded rows");
+#ifdef QMK_TC_FP8
+constexpr bool FP8_ROWS = true;
+#else
+constexpr bool FP8_ROWS = false;
+#endif
+constexpr int ROW_BYTES = FP8_ROWS ? FP8_PITCH : 2 * H;          // bytes of a weight row in memory (fp8: scale trailer included)
+constexpr int ROW_PITCH = FP8_ROWS ? FP8_PITCH : 2 * H + 16;     // bytes between the rows of a chunk in shared memory
+constexpr int CH_ROWS = FP8_ROWS ? 8 : 4;
+constexpr int TILE_CH = 16 / CH_ROWS;          // chunks of a 16-row tile
+constexpr int SCALE_CH = FP8_ROWS ? 1 : 0;     // an O / down slice is followed by a chunk of its 1024 output scales
+// weight rows of fp16 chunks in odd slots start four 16-byte bank groups later (an ldmatrix phase reads two chunks)
+constexpr int ODD_SLOT_SKEW = FP8_ROWS ? 0 : 64;
+static_assert(SLOT_BYTES >= ODD_SLOT_SKEW + CH_ROWS * ROW_PITCH, "a slot holds a chunk of padded rows");
+static_assert(ROW_PITCH % 128 == 16, "eight consecutive rows of a chunk fall into different bank groups");
+static_assert(I % CH_ROWS == 0 && QS % CH_ROWS == 0 && KVS % CH_ROWS == 0, "a chunk lies in one matrix");
+// The norm vectors of layer L go into the buffer of layer L - 2 as soon as the ring has room for layer L's first
+// chunks, i.e. when chunk (last of L - 1) - NSLOTS was handed back.  That must be a gate/up chunk of layer L - 2 or a
+// later one: every warp is past its last use of L - 2's norm vectors (post_ln, before the gate/up rows) by then.  fp16
+// layers have over 18 chunks on every CTA; the short layers of FP8 rows bound the grid.
+constexpr int TC_MAX_CTAS = FP8_ROWS ? 160 : MAX_CTAS;
+constexpr int MIN_QKV_CH = QKV_ROWS / CH_ROWS / TC_MAX_CTAS, MIN_O_CH = (QS / TC_MAX_CTAS + CH_ROWS - 1) / CH_ROWS + SCALE_CH,
+              MIN_GU_CH = I / CH_ROWS / TC_MAX_CTAS, MIN_LAYER_CH = MIN_QKV_CH + MIN_O_CH + 3 * MIN_GU_CH + SCALE_CH;
+static_assert(MIN_LAYER_CH > NSLOTS || 2 * MIN_LAYER_CH - 1 - NSLOTS >= MIN_QKV_CH + MIN_O_CH, "norm vectors overwritten in use");
 static_assert(SLOT_BYTES % 128 == 0 && NSLOTS % 2 == 0, "swizzled boxes need 128-byte aligned slots; slot parity = chunk parity");
 static_assert(EMPTY_UNITS == 12, "1, 2, 3, 4, 6 or 12 warps share a chunk");
 constexpr float LO_SCALE = 2048.0f, LO_INV = 1.0f / 2048.0f;
@@ -41,6 +72,7 @@ constexpr int KV_V_OFF = 2 * KV_BOX;
 constexpr int KV_PITCH = 2 * D + 16;           // pitch of the four query-operand rows (plain padded rows)
 static_assert(SLOT_BYTES >= 4 * KV_BOX, "a slot holds the four boxes of a cache chunk");
 constexpr int QKV_CHUNKS = QKV_ROWS / CH_ROWS, GU_CHUNKS = I / CH_ROWS;
+static_assert(CH_ROWS * ((GU_CHUNKS + TC_MIN_CTAS - 1) / TC_MIN_CTAS) <= 32, "slice_cols takes two k-steps");
 constexpr int KPAIRS = H / 32;                 // pairs of 16-input k-steps in a row
 
 // Extra shared memory of this kernel, behind the single-sequence layout.
@@ -66,6 +98,7 @@ static_assert(OFF_XF % 128 == 0 && OFF_QF % 16 == 0, "operand rows are 16-byte a
 // Byte offset in the fragment-order array of input i's hi (lo = 0) or lo (1) half.
 __device__ __forceinline__ int xf_offset(int i, int lo) {
   const int kk = i & 31, rem = kk & 15, r8 = rem & 7;
+  if (FP8_ROWS) return (i >> 5) * 128 + lo * 64 + (rem >> 2) * 16 + (kk >> 4) * 8 + (i & 3) * 2;   // lane kq: inputs 4 kq .. 4 kq + 3
   return (i >> 5) * 128 + lo * 64 + (r8 >> 1) * 16 + ((kk >> 4) * 4 + (rem >> 3) * 2 + (r8 & 1)) * 2;
 }
 
@@ -110,6 +143,12 @@ __device__ __forceinline__ void tma_box_2d(uint32_t dst, const void *map, int c0
                ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar)) : "memory");
 }
 
+// A register of four e4m3 values as two fp16 pairs.
+__device__ __forceinline__ void e4m3x4_half2x2(uint32_t four, uint32_t &first, uint32_t &second) {
+  asm("{\n\t.reg .b16 l, u;\n\tmov.b32 {l, u}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, l;\n\tcvt.rn.f16x2.e4m3x2 %1, u;\n\t}"
+      : "=r"(first), "=r"(second) : "r"(four));
+}
+
 // One warp: rows of the 16-row tile that starts at ring chunk `first` (valid rows <= 16), k-step pairs [p0, p1).
 // Leaves the 16 row sums of that k range in part[0..15] and hands the tile's chunks back with `units` each.
 // Lanes 0..3 each wait for one of the tile's chunks (the vote that follows orders the copied bytes before every
@@ -126,25 +165,40 @@ __device__ __forceinline__ void tile_task(const Params &P, const Ctx &c, uint32_
   QMK_FINE(fslot + 1);
   int lr = (c.lane & 7) + ((c.lane >> 3) & 1) * 8;      // tile row whose address this lane supplies
   if (lr >= valid_rows) lr = 0;                         // rows past the end repeat row 0 (their sums are not used)
-  const uint32_t a_addr = weight_rows(c, first + static_cast<uint32_t>(lr >> 2)) + (lr & 3) * ROW_PITCH + (c.lane >> 4) * 16;
+  const uint32_t a_addr = weight_rows(c, first + static_cast<uint32_t>(lr / CH_ROWS)) + (lr % CH_ROWS) * ROW_PITCH + (c.lane >> 4) * 16;
   float acc0[4] = {0.f, 0.f, 0.f, 0.f}, acc1[4] = {0.f, 0.f, 0.f, 0.f};
   if (ok) {
 #pragma unroll 2
     for (int p = p0; p < p1; ++p) {
       uint32_t a0[4], a1[4];
       const uint4 b = b_pair(c, p);
-      ldsm_x4(a_addr + p * 64, a0);
-      ldsm_x4(a_addr + p * 64 + 32, a1);
+      if (FP8_ROWS) {   // r: rows 0..7 / 8..15 x inputs 0..15, then inputs 16..31; four consecutive inputs per lane
+        uint32_t r[4];
+        ldsm_x4(a_addr + p * 32, r);
+        e4m3x4_half2x2(r[0], a0[0], a0[2]);
+        e4m3x4_half2x2(r[1], a0[1], a0[3]);
+        e4m3x4_half2x2(r[2], a1[0], a1[2]);
+        e4m3x4_half2x2(r[3], a1[1], a1[3]);
+      } else {
+        ldsm_x4(a_addr + p * 64, a0);
+        ldsm_x4(a_addr + p * 64 + 32, a1);
+      }
       mma_16816(acc0, a0, b.x, b.y);
       mma_16816(acc1, a1, b.z, b.w);
     }
   }
   QMK_FINE(fslot + 5);
+  float sc_top = 1.f, sc_bot = 1.f;                     // row scales, read before the rows are handed back
+  if (FP8_ROWS && (c.lane & 3) == 0) {
+    const int r0 = c.lane >> 2, r1 = r0 + 8;
+    if (r0 < valid_rows) sc_top = *reinterpret_cast<const float *>(c.slot(first + static_cast<uint32_t>(r0 / CH_ROWS)) + (r0 % CH_ROWS) * ROW_PITCH + H);
+    if (r1 < valid_rows) sc_bot = *reinterpret_cast<const float *>(c.slot(first + static_cast<uint32_t>(r1 / CH_ROWS)) + (r1 % CH_ROWS) * ROW_PITCH + H);
+  }
   __syncwarp();
   if (c.lane < nch) mbar_arrive_n(c.empty((first + static_cast<uint32_t>(c.lane)) % NSLOTS), static_cast<uint32_t>(units));
   if ((c.lane & 3) == 0) {
-    part[c.lane >> 2] = fmaf(acc0[1] + acc1[1], LO_INV, acc0[0] + acc1[0]);
-    part[(c.lane >> 2) + 8] = fmaf(acc0[3] + acc1[3], LO_INV, acc0[2] + acc1[2]);
+    part[c.lane >> 2] = fmaf(acc0[1] + acc1[1], LO_INV, acc0[0] + acc1[0]) * sc_top;
+    part[(c.lane >> 2) + 8] = fmaf(acc0[3] + acc1[3], LO_INV, acc0[2] + acc1[2]) * sc_bot;
   }
 }
 
@@ -153,15 +207,15 @@ __device__ __forceinline__ void tile_task(const Params &P, const Ctx &c, uint32_
 // chunks, then the up rows'); tiles of 16 rows; when there are fewer tiles than warps, nkb warps share a tile's
 // 1024 inputs.  Grids of at least FUSED_MIN_CTAS CTAs have at most 6 tiles per phase: one task per warp.
 __device__ inline void build_tile_tasks(TileTask *tasks, int *nkb_out, int groups, int nch) {
-  const int tpg = (nch + 3) >> 2, T = groups * tpg;
+  const int tpg = (nch + TILE_CH - 1) / TILE_CH, T = groups * tpg;
   const int nkb = T >= CONS_WARPS ? 1 : CONS_WARPS / T;   // 12, 6, 4, 3, 2, 2, 1: divides EMPTY_UNITS
   *nkb_out = nkb;
   for (int w = 0; w < CONS_WARPS; ++w) {
     TileTask &t = tasks[w];
     t.active = w < T * nkb ? 1 : 0;
     const int tile = w / nkb, kb = w - tile * nkb, grp = tile / tpg, tt = tile - grp * tpg;
-    t.first = grp * nch + tt * 4;
-    t.valid = min(16, (nch - tt * 4) * CH_ROWS);
+    t.first = grp * nch + tt * TILE_CH;
+    t.valid = min(16, (nch - tt * TILE_CH) * CH_ROWS);
     t.p0 = (KPAIRS * kb) / nkb;
     t.p1 = (KPAIRS * (kb + 1)) / nkb;
     t.units = EMPTY_UNITS / nkb;
@@ -204,7 +258,7 @@ __device__ __noinline__ uint32_t gateup_phase(const Params &P, Ctx c) {
   QMK_FINE(12);
   cons_sync();
   if (c.tid < nch * CH_ROWS) {
-    const int r = c.tid, tpg = (nch + 3) >> 2;
+    const int r = c.tid, tpg = (nch + TILE_CH - 1) / TILE_CH;
     const float *pg = tc_part(c) + (r >> 4) * nkb * 16 + (r & 15);
     const float *pu = pg + tpg * nkb * 16;
     float g = 0.f, u = 0.f;
@@ -560,12 +614,18 @@ __device__ __noinline__ void red_wait_norm(const Params &P, const Ctx c, int whi
 // Embedding row of `token` (megakernel_5090.cu:825-830) -> residual stream, normalised with layer 0's input norm.
 __device__ __noinline__ void embed_norm(const Params &P, const Ctx c, int token, const __half *norm_w) {
   constexpr int PT = (H + CONS_THREADS - 1) / CONS_THREADS;
-  const __half *erow = P.embed + static_cast<size_t>(token) * H;
+  const unsigned char *erow = reinterpret_cast<const unsigned char *>(P.embed) + static_cast<size_t>(token) * ROW_BYTES;
+  const float escale = FP8_ROWS ? __ldg(reinterpret_cast<const float *>(erow + H)) : 1.f;
   float v[PT], ss = 0.f;
 #pragma unroll
   for (int j = 0; j < PT; ++j) {
     const int n = c.tid + j * CONS_THREADS;
-    v[j] = n < H ? __half2float(__ldg(erow + n)) : 0.f;
+    if (FP8_ROWS) {
+      const __half_raw hr = __nv_cvt_fp8_to_halfraw(static_cast<__nv_fp8_storage_t>(n < H ? __ldg(erow + n) : 0), __NV_E4M3);
+      v[j] = __half2float(*reinterpret_cast<const __half *>(&hr)) * escale;
+    } else {
+      v[j] = n < H ? __half2float(__ldg(reinterpret_cast<const __half *>(erow) + n)) : 0.f;
+    }
     ss = fmaf(v[j], v[j], ss);
   }
   const float rstd = block_rstd(c, ss);
@@ -590,7 +650,8 @@ __device__ __noinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
   const float *resid = c.f(which ? F_X1 : F_X);
   float *prev = c.f(FF_PREV) + (which ? H : 0);
   unsigned long long *mine = P.red + (which ? RED_X2 : RED_X1) + (c.cta % P.red_copies) * H;
-  const int nch = (nrows + CH_ROWS - 1) / CH_ROWS;
+  const int nch = (nrows + CH_ROWS - 1) / CH_ROWS + SCALE_CH;
+  [[maybe_unused]] const float *scales = FP8_ROWS ? reinterpret_cast<const float *>(c.slot(c.chunk + static_cast<uint32_t>(nch - 1))) : nullptr;
   const bool two = nrows > 16;
   [[maybe_unused]] const int fb = which ? 30 : 20;
   QMK_FINE(fb + 0);
@@ -604,16 +665,20 @@ __device__ __noinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
     // B: the slice's activations; row n of B^T = hi (even n) / lo (odd n) vector; one ldmatrix.x4 = two k-steps
     uint32_t bq[4];
     ldsm_x4(smem_u32(c.smem + OFF_ACT16) + (c.lane & 1) * (ACT16_PITCH * 2) + (c.lane >> 3) * 16, bq);
-    // A: this lane's row of each k-step (rows past the slice repeat row 0: their activations are zero)
+    // A: this lane's row of each k-step (rows past the slice repeat row 0: their activations are zero).  fp8: one
+    // ldmatrix.x4 takes 32 rows x 16 outputs, a lane's register holds outputs 2j, 2j + 1 of rows 2q and 2q + 1
+    // (j = lane / 4); fragment rows j, j + 8 are those two outputs.
     uint32_t arow[2];
 #pragma unroll
     for (int ks = 0; ks < 2; ++ks) {
-      int row = ks * 16 + (c.lane & 7) + 8 * (c.lane >> 4);
+      int row = FP8_ROWS ? c.lane : ks * 16 + (c.lane & 7) + 8 * (c.lane >> 4);
       if (row >= nrows) row = 0;
-      arow[ks] = weight_rows(c, c.chunk + static_cast<uint32_t>(row >> 2)) + (row & 3) * ROW_PITCH + ((c.lane >> 3) & 1) * 16;
+      arow[ks] = weight_rows(c, c.chunk + static_cast<uint32_t>(row / CH_ROWS)) + (row % CH_ROWS) * ROW_PITCH + (FP8_ROWS ? 0 : ((c.lane >> 3) & 1) * 16);
     }
     const int n0 = t->n0, n1 = t->n1;
-    const int src = (c.lane & 7) * 4;                 // lane that holds this lane's output row (fragment row = lane / 4)
+    // lane that holds this lane's output (fragment row = lane / 4), and whether it is its second row
+    const int src = FP8_ROWS ? ((c.lane & 15) >> 1) * 4 : (c.lane & 7) * 4;
+    const bool second = (c.lane & (FP8_ROWS ? 1 : 8)) != 0;
 #pragma unroll 1
     for (int t0 = c.warp; t0 < H / 16; t0 += 2 * CONS_WARPS) {
       float acc[2][4];
@@ -622,15 +687,26 @@ __device__ __noinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
       for (int u = 0; u < 2; ++u) {
         const int tile = min(t0 + u * CONS_WARPS, H / 16 - 1);   // past the end: repeat a valid tile, not added
         acc[u][0] = 0.f; acc[u][1] = 0.f; acc[u][2] = 0.f; acc[u][3] = 0.f;
-        ldsm_x4_trans(arow[0] + tile * 32, a[u]);
-        if (two) ldsm_x4_trans(arow[1] + tile * 32, a2[u]);
+        if (FP8_ROWS) {
+          uint32_t r[4];
+          ldsm_x4_trans(arow[0] + tile * 16, r);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) r[i] = __byte_perm(r[i], 0u, 0x3120);   // {row 2q, 2q + 1} of the first output, then of the second
+          e4m3x4_half2x2(r[0], a[u][0], a[u][1]);
+          e4m3x4_half2x2(r[1], a[u][2], a[u][3]);
+          e4m3x4_half2x2(r[2], a2[u][0], a2[u][1]);
+          e4m3x4_half2x2(r[3], a2[u][2], a2[u][3]);
+        } else {
+          ldsm_x4_trans(arow[0] + tile * 32, a[u]);
+          if (two) ldsm_x4_trans(arow[1] + tile * 32, a2[u]);
+        }
       }
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         mma_16816(acc[u], a[u], bq[0], bq[1]);
         if (two) mma_16816(acc[u], a2[u], bq[2], bq[3]);
       }
-      // lanes of quad 0 hold (hi, lo) sums of rows lane / 4 and lane / 4 + 8 of both tiles; lane L takes output
+      // lanes of quad 0 hold (hi, lo) sums of fragment rows lane / 4 and lane / 4 + 8 of both tiles; lane L takes output
       // L % 16 of tile L / 16
       const float s0 = __shfl_sync(0xffffffffu, fmaf(acc[0][1], LO_INV, acc[0][0]), src);
       const float s1 = __shfl_sync(0xffffffffu, fmaf(acc[0][3], LO_INV, acc[0][2]), src);
@@ -639,7 +715,8 @@ __device__ __noinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
       const int tile = t0 + (c.lane >> 4) * CONS_WARPS;
       if (tile < H / 16) {
         const int n = tile * 16 + (c.lane & 15);
-        float v = (c.lane & 16) ? ((c.lane & 8) ? s3 : s2) : ((c.lane & 8) ? s1 : s0);
+        float v = (c.lane & 16) ? (second ? s3 : s2) : (second ? s1 : s0);
+        if (FP8_ROWS) v *= scales[n];
         if (n >= n0 && n < n1) v += resid[n];
         const long long fx = __float2ll_rn(v * RED_SCALE), fx_prev = __float2ll_rn(prev[n] * RED_SCALE);
         prev[n] = v;
@@ -661,7 +738,7 @@ __device__ __noinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
 // expects in s_misc[32..43] / s_misc[48..59].
 __device__ __noinline__ uint32_t lm_head_tc(const Params &P, Ctx c, float *dump) {
   const TcTab *t = tctab(c);
-  const int nch = t->nlm, ntiles = (nch + 3) >> 2;
+  const int nch = t->nlm, ntiles = (nch + TILE_CH - 1) / TILE_CH;
   float *part = tc_part(c), *s_misc = c.f(F_MISC);
   float best = -INFINITY;
   int best_i = 0x7fffffff;
@@ -669,7 +746,7 @@ __device__ __noinline__ uint32_t lm_head_tc(const Params &P, Ctx c, float *dump)
 #pragma unroll 1
   for (int tile = 0; tile < ntiles; ++tile) {
     float *pr = part + (tile & 1) * (CONS_WARPS * 16);
-    tile_task(P, c, c.chunk + static_cast<uint32_t>(tile * 4), min(16, (nch - tile * 4) * CH_ROWS), p0, p1, pr + c.warp * 16,
+    tile_task(P, c, c.chunk + static_cast<uint32_t>(tile * TILE_CH), min(16, (nch - tile * TILE_CH) * CH_ROWS), p0, p1, pr + c.warp * 16,
               EMPTY_UNITS / CONS_WARPS);
     cons_sync();
     if (c.tid < 16) {
@@ -705,7 +782,7 @@ __device__ __noinline__ uint32_t lm_head_tc(const Params &P, Ctx c, float *dump)
 // chunk, wait + announce + copy are ~800 cycles of dependent latency; one chunk at a time capped the stream at
 // 19 GB/s per SM (LM head 2.8 TB/s), eight at a time keep that latency off the stream.
 // A layer's chunks in ring order: q|k|v rows, this CTA's old K/V rows, K-major O rows [e0, e1), gate rows, up
-// rows, K-major down rows; after the last layer the LM-head rows.
+// rows, K-major down rows (fp8: the output scales behind the O and the down rows); after the last layer the LM-head rows.
 // kv_row >= 0 marks a cache chunk: 16 rows of the K and of the V cache from that row on (rows of the caches seen as
 // [layers * 8 * max_seq_len][128]); lane r of the group copies box r (K low dims, K high dims, V low, V high).
 struct ChunkSrc { const unsigned char *src; size_t src_pitch; uint32_t rows, row_bytes, dst_pitch; int kv_row; };
@@ -727,15 +804,24 @@ __device__ __forceinline__ bool tc_issue8(const Params &P, const Ctx &c, uint32_
   }
   return true;
 }
-// Four rows of a row-major fp16 matrix with 1024 inputs, starting at `row`.
+// A chunk's rows of a row-major matrix with 1024 inputs (or of a K-major copy), starting at `row`; fp8 rows are
+// contiguous at the pitch they have in shared memory: one copy.
 __device__ __forceinline__ ChunkSrc matrix_chunk(const void *base, int row, int rows) {
   ChunkSrc d;
-  d.src = reinterpret_cast<const unsigned char *>(base) + static_cast<size_t>(row) * (2 * H);
-  d.src_pitch = 2 * H;
-  d.rows = static_cast<uint32_t>(rows);
-  d.row_bytes = 2 * H;
+  d.src = reinterpret_cast<const unsigned char *>(base) + static_cast<size_t>(row) * ROW_BYTES;
+  d.src_pitch = ROW_BYTES;
+  d.rows = static_cast<uint32_t>(FP8_ROWS ? 1 : rows);
+  d.row_bytes = static_cast<uint32_t>(FP8_ROWS ? rows * ROW_BYTES : ROW_BYTES);
   d.dst_pitch = ROW_PITCH;
   d.kv_row = -1;
+  return d;
+}
+
+// The 1024 fp32 output scales of a K-major fp8 copy with `rows` rows (they follow the last one).
+__device__ __forceinline__ ChunkSrc scale_chunk(const void *base, int rows) {
+  ChunkSrc d = matrix_chunk(base, rows, 0);
+  d.rows = 1u;
+  d.row_bytes = 4 * H;
   return d;
 }
 
@@ -750,7 +836,7 @@ __device__ __noinline__ void producer_main_tc(const Params &P, const Ctx c) {
 #pragma unroll 1
   for (int step = 0; ok && step < P.num_steps; ++step) {
     const AttnItem it = attn_item(P, c, 0, 1, CONS_WARPS, P.start_position + step);
-    const int s1 = nq, s2 = s1 + it.nchunks, s3 = s2 + no, s4 = s3 + ng, s5 = s4 + ng, per_layer = s5 + ng;
+    const int s1 = nq, s2 = s1 + it.nchunks, s3 = s2 + no + SCALE_CH, s4 = s3 + ng, s5 = s4 + ng, per_layer = s5 + ng + SCALE_CH;
 #pragma unroll 1
     for (int l = 0; ok && l < P.num_layers; ++l) {
       const unsigned long long *rec = c.layer_rec(l);
@@ -779,13 +865,16 @@ __device__ __noinline__ void producer_main_tc(const Params &P, const Ctx c) {
           d.kv_row = (l * NKV + it.g) * P.max_seq_len + it.p0 + (j - s1) * it.rpc;
         } else if (j < s3) {
           const int r = (j - s2) * CH_ROWS;
-          d = matrix_chunk(reinterpret_cast<const void *>(rect[0]), t->e0 + r, min(CH_ROWS, ne - r));
+          if (r < ne) d = matrix_chunk(reinterpret_cast<const void *>(rect[0]), t->e0 + r, min(CH_ROWS, ne - r));
+          else d = scale_chunk(reinterpret_cast<const void *>(rect[0]), QS);
         } else if (j < s4) {
           d = matrix_chunk(reinterpret_cast<const void *>(rec[REC_GATE]), (tt->g0 + j - s3) * CH_ROWS, CH_ROWS);
         } else if (j < s5) {
           d = matrix_chunk(reinterpret_cast<const void *>(rec[REC_UP]), (tt->g0 + j - s4) * CH_ROWS, CH_ROWS);
-        } else if (j < per_layer) {
+        } else if (j < s5 + ng) {
           d = matrix_chunk(reinterpret_cast<const void *>(rect[1]), (tt->g0 + j - s5) * CH_ROWS, CH_ROWS);
+        } else if (j < per_layer) {
+          d = scale_chunk(reinterpret_cast<const void *>(rect[1]), I);
         }
         ok = tc_issue8(P, c, idx + static_cast<uint32_t>(j), j < per_layer, d, pol);   // issues all eight or none
         if (ok) issued = idx + static_cast<uint32_t>(min(j0 + 8, per_layer));

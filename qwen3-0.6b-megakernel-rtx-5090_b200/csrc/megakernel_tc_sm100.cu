@@ -23,8 +23,9 @@
 #include "megakernel_tc.h"
 
 namespace qmk_fused_tc {
-const void *kernel() { return reinterpret_cast<const void *>(qmkt::qwen3_decode_megakernel_tc); }
-size_t smem_bytes() { return qmkt::TC_SMEM_BYTES; }
-int threads() { return qmkt::THREADS; }
-int min_ctas() { return qmkt::TC_MIN_CTAS; }
+const Build &build_f16() {
+  static const Build b = {reinterpret_cast<const void *>(qmkt::qwen3_decode_megakernel_tc), qmkt::TC_SMEM_BYTES, qmkt::TC_MIN_CTAS,
+                          qmkt::TC_MAX_CTAS, qmkt::CH_ROWS};
+  return b;
+}
 }  // namespace qmk_fused_tc

@@ -100,6 +100,46 @@ def test_fp8_full_model_greedy_tokens(built_library):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("ctas,prompt,vocab", [(0, 2, 4096), (0, 17, 4096), (96, 300, 4096), (107, 33, 4104), (0, 1400, 4096), (0, 40, 4100)])
+def test_fp8_tensor_core_rows_match_cuda_core_rows(built_library, ctas, prompt, vocab):
+    """FP8 rows as MMA tiles against the CUDA-core kernel and the oracle: the smallest grid of the tensor-core build (slices
+    of two k-steps), one that leaves partial tiles, contexts without old rows in the cache, with a partial cache chunk, and
+    with all splits, a vocabulary that leaves CTAs with different numbers of chunks and one that is not a multiple of
+    eight (both runs then take the CUDA-core kernel).  The two kernels differ in summation order and in the activations'
+    22 instead of 24 bits: the bound of the fp16 kernels' comparison (1e-3) holds."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import qwen_megakernel_C as C
+    from Model.Qwen06B_architecture import Decoder
+    steps, rows = 20, 1440
+    w = S.make_weights(seed=23, num_layers=3, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    ids = S.make_prompt(prompt, seed=prompt, vocab_size=vocab)
+    eng_w, ora_w = Q.quantize_weights_fp8(w)
+    want, logits = OracleDecoder(ora_w, max_seq_len=rows).generate_ids(ids, steps, keep_logits=True)
+    eng = Decoder(weights=S.weights_to(eng_w, "cuda"), verbose=False, max_seq_len=rows, weight_format="fp8")
+    dumps = []
+    try:
+        C.configure(max_ctas=ctas)
+        for fused in (2, 1, 2):
+            C.set_fused(fused=fused)
+            dump = torch.zeros(steps, vocab, device="cuda")
+            C.set_logits_dump(dump)
+            assert eng.generate_ids(ids, steps) == want, fused
+            dumps.append(dump)
+    finally:
+        C.set_logits_dump(None)
+        C.set_fused(fused=2)
+        C.configure(max_ctas=0)
+        C.set_weight_format("fp16")
+    err = [float((d.cpu() - logits).abs().max()) for d in dumps]
+    diff = float((dumps[0] - dumps[1]).abs().max())
+    print(f"ctas {ctas} prompt {prompt}: tensor vs CUDA cores {diff:.2e}; against the oracle {err[0]:.2e}, {err[1]:.2e}")
+    assert torch.equal(dumps[0], dumps[2]), "not reproducible run to run"
+    assert torch.equal(dumps[0], dumps[1]) == (vocab % 8 != 0)
+    assert diff < 1e-3 and max(err) < 3e-2
+
+
+@pytest.mark.gpu
 def test_fp8_four_sequences_per_launch(built_library):
     """FP8 weights through the multi-sequence launch (the B = 4 shape of the FP8 configuration): every
     sequence against the oracle on the dequantised weights."""
