@@ -28,8 +28,12 @@
 // Split activations (template parameter AH = 2): A is [M x 2 K], columns [0, K) the fp16 rounding hi of the fp32
 // activations and columns [K, 2 K) the fp16 rounding lo of what it left (x - hi).  A stage holds both A tiles and ONE B
 // tile, which eight MMAs read instead of four: the weights cross HBM, L2 and the copy engine once.  hi + lo keeps 22 bits
-// of x (absolute floor 2^-25, the fp16 subnormals), the products are exact and the sums fp32, so the result is the one of
-// fp32 activations - what the token-serial kernels compute - at twice the MMA work.
+// of x (absolute floor 2^-25, the fp16 subnormals) and the products are exact.  The sums need care: the tensor core
+// TRUNCATES its fp32 accumulator after every K step, so the 128 steps of a 1024-wide row in one accumulator lose 4e-6 of
+// the result, ten times what the token-serial kernels lose (share of first-layer V rows that round to another fp16 than
+// float64's: 0.93 % against 0.09 %).  So the K blocks take turns in seven accumulators, the small lo products have an
+// eighth of their own, and the epilogue adds the eight with rounded fp32 adds: at most 12 steps each, 0.12 %.
+// All 512 TMEM columns hold 64 B rows then: tiles are 64 wide (32 + 32 for gate / up), one CTA per SM with a deep ring.
 #ifndef QMK_GEMM_TCGEN05_CUH_
 #define QMK_GEMM_TCGEN05_CUH_
 
@@ -45,7 +49,7 @@ constexpr int BM = 128, BK = 64;                 // BK * 2 bytes = one 128-byte 
 // Ring depth per N-tile variant: as many stages as fit in ~192 KB (a skinny M = 128 problem is bound by the
 // latency of its K loop, so the whole K extent of a 1024-wide matrix is in flight at once).
 constexpr int stages_for(int bn, int wq = 0, int ah = 1) {
-  if (ah == 2) return bn == 32 ? 5 : bn == 256 ? 3 : bn == 128 && wq ? 3 : 4;
+  if (ah == 2) return wq ? 4 : 5;
   return wq ? (bn == 32 ? 8 : bn == 64 ? 6 : bn == 128 ? 4 : 2) : (bn == 32 ? 10 : bn == 64 ? 8 : bn == 128 ? 6 : 4);
 }
 constexpr int MAX_GROUPS = 3;   // matrices sharing one A operand that one launch can multiply (q/k/v, gate/up)
@@ -215,6 +219,35 @@ __device__ __forceinline__ uint32_t e4m3x2_to_half2_bits(uint32_t two_bytes) {
   return static_cast<uint32_t>(h.x) | (static_cast<uint32_t>(h.y) << 16);
 }
 
+// Columns [0, 16 or 32) from `addr` of this warp's 32 TMEM lanes (the caller waits for the loads).
+__device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(addr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(addr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+template <int NR>
+__device__ __forceinline__ void add_f32(uint32_t (&r)[NR], const uint32_t (&t)[NR]) {
+#pragma unroll
+  for (int i = 0; i < NR; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(t[i]));
+}
+
 // FUSE (BN = 32 or 64): B0 is the gate matrix and B1 the up matrix of a SwiGLU MLP; the CTA keeps two accumulators
 // (gate tile in TMEM columns [0, BN), up tile in [BN, 2 BN)) and its epilogue writes fp16 silu(gate) * up to
 // groups.C[0] (reinterpreted as __half [M x N]) instead of two fp32 matrices; AH = 2: as hi and lo halves, [M x 2 N].
@@ -228,6 +261,9 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   static_assert(!FUSE || BN <= 128, "the fused SwiGLU epilogue keeps two accumulators of at most 128 columns (one MMA of N = 256)");
   static_assert(WQ == 0 || (FUSE ? 2 * BN : BN) <= 128, "packed weights: at most 128 B rows per stage (scales live in shared memory)");
   constexpr int SB = FUSE ? 2 * BN : BN;          // B rows held per stage / accumulator columns
+  // accumulators: one, or with split activations the lo products' and seven that the K blocks take in turn
+  constexpr int NACC = AH == 2 ? 8 : 1;
+  static_assert(NACC * SB <= 512, "TMEM columns");
   constexpr uint32_t RAW_ROW = raw_row_bytes(WQ);
   const int STAGES = groups.stages;
   constexpr uint32_t STAGE_BYTES = stage_bytes_for(SB, WQ, AH);
@@ -253,7 +289,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   const int kblocks = groups.kblocks_per_split > 0 ? groups.kblocks_per_split : K / BK;
   const int kb0 = groups.kblocks_per_split > 0 ? static_cast<int>(blockIdx.z) * groups.kblocks_per_split : 0;
   constexpr uint32_t TILE_B_BYTES = BN * BK * 2;
-  constexpr uint32_t TMEM_COLS = SB;             // fp32 accumulator(s): 128 lanes x SB columns (a power of two >= 32)
+  constexpr uint32_t TMEM_COLS = NACC * SB;      // fp32 accumulator(s): 128 lanes x SB columns (a power of two >= 32)
   auto full = [&](int s) { return bars + 8u * s; };
   auto empty = [&](int s) { return bars + 8u * (MAX_STAGES + s); };
   const uint32_t acc_full = bars + 8u * (2 * MAX_STAGES);
@@ -379,8 +415,13 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         for (int j = 0; j < BK / 16; ++j) {  // 16 halves = 32 bytes = 2 descriptor address units per K step
           // FUSE: the up tile follows the gate tile in shared memory (BN more rows of the same 8-row-group layout),
           // so one MMA of N = 2 BN covers both and leaves gate in columns [0, BN), up in [BN, 2 BN)
-          mma_f16_ss(tmem_base, da + 2u * j, db + 2u * j, (kb > 0 || j > 0) ? 1u : 0u, idesc_for(SB));
-          if (AH == 2) mma_f16_ss(tmem_base, da + (TILE_A_BYTES >> 4) + 2u * j, db + 2u * j, 1u, idesc_for(SB));
+          const uint32_t later = (kb > 0 || j > 0) ? 1u : 0u;
+          if (AH == 2) {
+            mma_f16_ss(tmem_base, da + (TILE_A_BYTES >> 4) + 2u * j, db + 2u * j, later, idesc_for(SB));
+            mma_f16_ss(tmem_base + (1 + kb % (NACC > 1 ? NACC - 1 : 1)) * SB, da + 2u * j, db + 2u * j, (kb >= NACC - 1 || j > 0) ? 1u : 0u, idesc_for(SB));
+          } else {
+            mma_f16_ss(tmem_base, da + 2u * j, db + 2u * j, later, idesc_for(SB));
+          }
         }
         mma_commit(empty(s));               // the stage is free once these MMAs have read it
       }
@@ -448,6 +489,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     // warp-uniform outcome: the TMEM loads below are warp-wide instructions
     const bool ok = __all_sync(0xffffffffu, bar_wait(acc_full, 0, abort_flag, status, budget_ns));
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const int accs = NACC == 1 ? 1 : 1 + (kblocks < NACC - 1 ? kblocks : NACC - 1);   // accumulators in use
     if (ok && FUSE) {
       const int row = m0 + quarter * 32 + lane;
       __half *arow = reinterpret_cast<__half *>(C) + static_cast<size_t>(row) * (AH * N) + n0;
@@ -455,21 +497,17 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       for (int c = 0; c < BN / 16; ++c) {     // 16 columns of the gate tile and the same 16 of the up tile per pass
         uint32_t g[16], u[16];
         const uint32_t tg = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(c * 16);
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-            : "=r"(g[0]), "=r"(g[1]), "=r"(g[2]), "=r"(g[3]), "=r"(g[4]), "=r"(g[5]), "=r"(g[6]), "=r"(g[7]), "=r"(g[8]),
-              "=r"(g[9]), "=r"(g[10]), "=r"(g[11]), "=r"(g[12]), "=r"(g[13]), "=r"(g[14]), "=r"(g[15])
-            : "r"(tg)
-            : "memory");
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-            : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]),
-              "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
-            : "r"(tg + BN)
-            : "memory");
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        tmem_ld16(tg, g);
+        tmem_ld16(tg + BN, u);
+        tmem_ld_wait();
+        for (int a = 1; a < accs; ++a) {
+          uint32_t tg2[16], tu2[16];
+          tmem_ld16(tg + a * SB, tg2);
+          tmem_ld16(tg + a * SB + BN, tu2);
+          tmem_ld_wait();
+          add_f32(g, tg2);
+          add_f32(u, tu2);
+        }
         if (row < M) {
           uint32_t packed[8], packed_lo[8];
 #pragma unroll
@@ -513,17 +551,14 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       for (int c = 0; c < BN / 32; ++c) {
         uint32_t r[32];
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(c * 32);
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-            "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-              "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-              "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-              "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-            : "r"(taddr)
-            : "memory");
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        tmem_ld32(taddr, r);
+        tmem_ld_wait();
+        for (int a = 1; a < accs; ++a) {
+          uint32_t t[32];
+          tmem_ld32(taddr + a * SB, t);
+          tmem_ld_wait();
+          add_f32(r, t);
+        }
         if (row < M && f16) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {

@@ -135,7 +135,8 @@ static int pick_box_n(int M, int N, int b_tiles) {
   const int sms = sm_count() * (t_ring_budget ? 2 : 1);   // CTA slots of one wave: rings sized to a budget share an SM in pairs
   int best = 0;
   long best_cost = 0;
-  for (int bn = b_tiles == 2 ? 64 : 128; bn >= 32; bn /= 2) {
+  // split activations: eight accumulators in 512 TMEM columns, 64 B rows per stage
+  for (int bn = (b_tiles == 2 ? 64 : 128) / t_ah; bn >= 32; bn /= 2) {
     const long ctas = static_cast<long>(M / qmk_gemm::BM) * (N / bn);
     const long cost = ((ctas + sms - 1) / sms) * (b_tiles * bn + 320);
     if (best == 0 || cost < best_cost) { best = bn; best_cost = cost; }
@@ -156,20 +157,29 @@ bool pdl_active() { return t_pdl; }
 // The kernel for an N tile, epilogue and weight format, and its dynamic shared memory.
 using GemmKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const qmk_gemm::Groups,
                             int, int, unsigned int *, unsigned long long, int);
-template <int WQ, int AH>
+template <int WQ>
 static GemmKernel gemm_kernel_wq(int bn, bool fuse) {
-  if (fuse) return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, true, WQ, AH> : qmk_gemm::gemm_f16_tn_kernel<64, true, WQ, AH>;
-  return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, false, WQ, AH>
-                  : bn == 64 ? qmk_gemm::gemm_f16_tn_kernel<64, false, WQ, AH> : qmk_gemm::gemm_f16_tn_kernel<128, false, WQ, AH>;
+  if (fuse) return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, true, WQ> : qmk_gemm::gemm_f16_tn_kernel<64, true, WQ>;
+  return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, false, WQ>
+                  : bn == 64 ? qmk_gemm::gemm_f16_tn_kernel<64, false, WQ> : qmk_gemm::gemm_f16_tn_kernel<128, false, WQ>;
+}
+// Split activations: at most 64 B rows per stage.
+template <int WQ>
+static GemmKernel gemm_kernel_split(int bn, bool fuse) {
+  if (fuse) return qmk_gemm::gemm_f16_tn_kernel<32, true, WQ, 2>;
+  return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, false, WQ, 2> : qmk_gemm::gemm_f16_tn_kernel<64, false, WQ, 2>;
+}
+static bool box_n_ok(int box_n, bool fuse, int wq) {
+  const int rows = fuse ? 2 * box_n : box_n;
+  if (t_ah == 2) return wq < 2 && (box_n == 32 || (box_n == 64 && rows == 64));
+  return box_n == 32 || box_n == 64 || (box_n == 128 && (rows == 128 || wq == 0)) || (box_n == 256 && rows == 256 && wq == 0);
 }
 // (the widest tiles - 256 B rows per stage - exist for fp16 weights only; split activations for fp16 and FP8 weights)
 static GemmKernel gemm_kernel(int bn, bool fuse, int wq, int ah) {
-  if (wq == 0 && fuse && bn == 128)
-    return ah == 2 ? qmk_gemm::gemm_f16_tn_kernel<128, true, 0, 2> : qmk_gemm::gemm_f16_tn_kernel<128, true, 0, 1>;
-  if (wq == 0 && !fuse && bn == 256)
-    return ah == 2 ? qmk_gemm::gemm_f16_tn_kernel<256, false, 0, 2> : qmk_gemm::gemm_f16_tn_kernel<256, false, 0, 1>;
-  if (ah == 2) return wq == 0 ? gemm_kernel_wq<0, 2>(bn, fuse) : gemm_kernel_wq<1, 2>(bn, fuse);
-  return wq == 0 ? gemm_kernel_wq<0, 1>(bn, fuse) : wq == 1 ? gemm_kernel_wq<1, 1>(bn, fuse) : gemm_kernel_wq<2, 1>(bn, fuse);
+  if (ah == 2) return wq == 0 ? gemm_kernel_split<0>(bn, fuse) : gemm_kernel_split<1>(bn, fuse);
+  if (wq == 0 && fuse && bn == 128) return qmk_gemm::gemm_f16_tn_kernel<128, true>;
+  if (wq == 0 && !fuse && bn == 256) return qmk_gemm::gemm_f16_tn_kernel<256, false>;
+  return wq == 0 ? gemm_kernel_wq<0>(bn, fuse) : wq == 1 ? gemm_kernel_wq<1>(bn, fuse) : gemm_kernel_wq<2>(bn, fuse);
 }
 static size_t gemm_smem(int bn, bool fuse, int wq, int ah) { return qmk_gemm::smem_bytes_for(fuse ? 2 * bn : bn, wq, ah); }
 
@@ -183,7 +193,7 @@ int ensure_gemm_attrs(std::string *err) {
     for (int ah = 1; ah < 3 && e == cudaSuccess; ++ah)
       for (int wq = 0; wq < 4 - ah && e == cudaSuccess; ++wq)
         for (int fuse = 0; fuse < 2 && e == cudaSuccess; ++fuse)
-          for (int bn = 32; bn <= (fuse ? 64 : 128) * (wq == 0 ? 2 : 1) && e == cudaSuccess; bn *= 2)
+          for (int bn = 32; bn <= (ah == 2 ? (fuse ? 32 : 64) : (fuse ? 64 : 128) * (wq == 0 ? 2 : 1)) && e == cudaSuccess; bn *= 2)
             e = cudaFuncSetAttribute(reinterpret_cast<const void *>(gemm_kernel(bn, fuse != 0, wq, ah)),
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gemm_smem(bn, fuse != 0, wq, ah)));
     if (e == cudaSuccess)
@@ -260,8 +270,7 @@ int launch_gemm_grouped(const CUtensorMap &map_a, int ngroups, const CUtensorMap
                         const int *Ns, int M, int K, int box_n, unsigned int *status, int timeout_ms, cudaStream_t stream,
                         std::string *err, int live_rows, int a_box_rows, int wq, const void *const *raws) {
   bool bad = M <= 0 || K <= 0 || M % qmk_gemm::BM || K % qmk_gemm::BK ||
-             (box_n != 32 && box_n != 64 && box_n != 128 && !(box_n == 256 && wq == 0)) ||
-             ngroups < 1 || ngroups > qmk_gemm::MAX_GROUPS;
+             !box_n_ok(box_n, false, wq) || ngroups < 1 || ngroups > qmk_gemm::MAX_GROUPS;
   for (int g = 0; !bad && g < ngroups; ++g) bad = Ns[g] <= 0 || Ns[g] % (box_n > 128 ? box_n : 128);
   if (bad) {
     *err = "gemm: M and N must be multiples of 128 and K a multiple of 64";
@@ -300,7 +309,7 @@ int launch_gemm_swiglu(const CUtensorMap &map_a, const CUtensorMap &map_gate, co
                        int N, int K, unsigned int *status, int timeout_ms, cudaStream_t stream, std::string *err,
                        int box_n, int live_rows, int a_box_rows, int wq, const void *raw_gate, const void *raw_up) {
   if (M <= 0 || N <= 0 || K <= 0 || M % qmk_gemm::BM || N % 128 || K % qmk_gemm::BK ||
-      (box_n != 32 && box_n != 64 && !(box_n == 128 && wq == 0))) {
+      !box_n_ok(box_n, true, wq)) {
     *err = "gemm: M and N must be multiples of 128 and K a multiple of 64";
     return QMK_ERR_BAD_ARGUMENT;
   }
@@ -332,7 +341,7 @@ int launch_gemm_splitk(const CUtensorMap &map_a, const CUtensorMap &map_b, float
                        unsigned int *status, int timeout_ms, cudaStream_t stream, std::string *err, int box_n,
                        int live_rows, int a_box_rows, int wq, const void *raw) {
   if (M <= 0 || N <= 0 || K <= 0 || M % qmk_gemm::BM || N % 128 || K % qmk_gemm::BK || splits < 1 ||
-      (K / qmk_gemm::BK) % splits || (box_n != 32 && box_n != 64 && box_n != 128 && !(box_n == 256 && wq == 0 && N % 256 == 0))) {
+      (K / qmk_gemm::BK) % splits || !box_n_ok(box_n, false, wq) || N % box_n) {
     *err = "gemm: bad split-K shape";
     return QMK_ERR_BAD_ARGUMENT;
   }
@@ -625,7 +634,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     // Long chunks of fp16 weights: 256-wide tiles (one MMA of N = 256 per K step; a third fewer operand bytes per
     // flop than 128-wide ones - these GEMMs are bound by the L2 -> shared-memory feed).  Measured on the q/k/v shape at
     // 2048 rows: 28.8 -> 26.5 us.
-    const int box_n = (wq == 0 && M >= 1024 && total / 256 * (M / qmk_gemm::BM) >= qmk_tc::gemm_sm_count()) ? 256
+    const int box_n = (wq == 0 && !split && M >= 1024 && total / 256 * (M / qmk_gemm::BM) >= qmk_tc::gemm_sm_count()) ? 256
                                                                                                            : qmk_tc::gemm_box_n(M, total);
     const CUtensorMap *maps[3];
     const void *raws[3] = {nullptr, nullptr, nullptr};
@@ -651,7 +660,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
       // 256-wide tiles, one CTA per SM with the whole ring: the main loops are bound by shared-memory traffic (TMA
       // writes + MMA operand reads), and a 256-wide tile moves a quarter fewer bytes per flop than a 128-wide one
       // (2048 tokens: 4.12 -> 4.07 ms per pass, same box); shorter chunks would leave SMs without a tile
-      if (Mrows >= 2048 && wq == 0) {
+      if (Mrows >= 2048 && wq == 0 && !split) {
         qmk_tc::RingBudgetScope whole(0);
         return qmk_tc::launch_gemm_splitk(a, wmap_for(l, j, 256), c, Mrows, H, K, od_splits, w.status, env.timeout_ms, stream, &err,
                                           256, live, 0, wq, wptr(l, j));
@@ -661,7 +670,8 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
         return qmk_tc::launch_gemm(a, wmap_for(l, j, box_n), c, Mrows, H, K, box_n, w.status, env.timeout_ms, stream, &err, live, 0, wq,
                                    wptr(l, j));
       }
-      return qmk_tc::launch_gemm_splitk(a, wmap_for(l, j, 128), c, Mrows, H, K, od_splits, w.status, env.timeout_ms, stream, &err, 128,
+      const int box_n = split ? 64 : 128;
+      return qmk_tc::launch_gemm_splitk(a, wmap_for(l, j, box_n), c, Mrows, H, K, od_splits, w.status, env.timeout_ms, stream, &err, box_n,
                                         live, 0, wq, wptr(l, j));
     };
     CUtensorMap map_kc, map_vc;   // the caches up to this chunk's last position, all layers
@@ -687,7 +697,8 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     qmk_tc::SplitActScope split_scope(split);
     const CUtensorMap &map_xn = split ? w.map_xn2 : w.map_xn, &map_attn = split ? w.map_attn2 : w.map_attn,
                       &map_act = split ? w.map_act2 : w.map_act, &map_qh = split ? w.map_qh2 : w.map_qh;
-    qmk_tc::RingBudgetScope ring_scope(PREFILL_RING_BYTES);   // two GEMM CTAs per SM: one's epilogue under the other's main loop
+    // two GEMM CTAs per SM: one's epilogue under the other's main loop (split activations take the SM's whole TMEM: one CTA)
+    qmk_tc::RingBudgetScope ring_scope(split ? 0 : PREFILL_RING_BYTES);
     {
       qmk_tc::PdlScope first(false);            // (follows a copy, not a kernel)
       PF_CUDA(qmk_tc::launch_kernel(embed_rows, dim3(T), dim3(256), 0, stream, w.tokens, embed_weight, wq, w.x));
@@ -749,7 +760,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
       {
         const int box_gu = qmk_tc::gemm_box_n_fused(M, I);
         // three of these CTAs per SM instead of two: their epilogue (two TMEM reads, SiLU, fp16 pack) is the long part
-        qmk_tc::RingBudgetScope gu_scope(M >= 1024 ? GATE_UP_RING_BYTES : PREFILL_RING_BYTES);
+        qmk_tc::RingBudgetScope gu_scope(split ? 0 : M >= 1024 ? GATE_UP_RING_BYTES : PREFILL_RING_BYTES);
         {
           qmk_tc::PdlScope g(pdl_gemm);
           rc = qmk_tc::launch_gemm_swiglu(map_xn, wmap_for(l, 4, box_gu), wmap_for(l, 5, box_gu), w.act, M, I, H, w.status,
