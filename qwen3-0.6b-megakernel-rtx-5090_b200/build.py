@@ -16,11 +16,12 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 SOURCES = [os.path.join(HERE, "csrc", "megakernel_sm100.cu"), os.path.join(HERE, "csrc", "megakernel_batch_sm100.cu"),
            os.path.join(HERE, "csrc", "megakernel_tc_sm100.cu"), os.path.join(HERE, "csrc", "megakernel_tc_fp8_sm100.cu"),
+           *(os.path.join(HERE, "csrc", f"megakernel_tc_{fmt}seqs{n}_sm100.cu") for fmt in ("", "fp8_") for n in (2, 4)),
            os.path.join(HERE, "csrc", "prefill_sm100.cu")]
 HEADERS = [os.path.join(os.path.dirname(HERE), "include", "qwen_megakernel.h"),
            os.path.join(HERE, "csrc", "megakernel_device.cuh"), os.path.join(HERE, "csrc", "megakernel_params.h"),
            os.path.join(HERE, "csrc", "megakernel_batch.cuh"), os.path.join(HERE, "csrc", "megakernel_fused.cuh"),
-           os.path.join(HERE, "csrc", "megakernel_tc.cuh"), os.path.join(HERE, "csrc", "megakernel_tc.h"), os.path.join(HERE, "csrc", "megakernel_batch.h"),
+           os.path.join(HERE, "csrc", "megakernel_tc.cuh"), os.path.join(HERE, "csrc", "megakernel_tc_multi.cuh"), os.path.join(HERE, "csrc", "megakernel_tc.h"), os.path.join(HERE, "csrc", "megakernel_batch.h"),
            os.path.join(HERE, "csrc", "gemm_tcgen05.cuh"), os.path.join(HERE, "csrc", "prefill_sm100.h"),
            os.path.join(HERE, "csrc", "prefill_kernels.cuh"), os.path.join(HERE, "csrc", "engine_internal.h"),
            os.path.join(HERE, "csrc", "attention_tcgen05.cuh"), os.path.join(HERE, "csrc", "decode_attention_mma.cuh")]

@@ -258,6 +258,10 @@ size_t exchange_bytes() {
   return words * sizeof(unsigned long long);
 }
 
+// Residual sums: [x1, x2][accumulator copy][1024] of one sequence, or [x1, x2][sequence][1024].
+constexpr size_t RED_ALLOC_WORDS = 2 * qmkp::MAX_SEQ * qmk::H;
+static_assert(RED_ALLOC_WORDS >= qmk::RED_WORDS, "one allocation serves both layouts");
+
 int ensure_ready(Engine *e) {
   if (e->ready) return QMK_OK;
   cudaDeviceProp prop;
@@ -281,13 +285,13 @@ int ensure_ready(Engine *e) {
   QMK_CUDA(e, cudaFuncSetAttribute(qmk_batch::kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(qmk_batch::smem_bytes())));
   for (int wfmt = 0; wfmt < 2; ++wfmt)
-    QMK_CUDA(e, cudaFuncSetAttribute(qmk_fused_tc::build(wfmt).kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(qmk_fused_tc::build(wfmt).smem_bytes)));
+    for (const qmk_fused_tc::Build *b : {&qmk_fused_tc::build(wfmt), &qmk_fused_tc::build_seqs(wfmt, 2), &qmk_fused_tc::build_seqs(wfmt, 4)})
+      QMK_CUDA(e, cudaFuncSetAttribute(b->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(b->smem_bytes)));
   QMK_CUDA(e, cudaMalloc(&e->ll, exchange_bytes()));
   QMK_CUDA(e, cudaMemset(e->ll, 0, exchange_bytes()));
   QMK_CUDA(e, cudaMalloc(&e->status, 16));
   QMK_CUDA(e, cudaMemset(e->status, 0, 16));
-  QMK_CUDA(e, cudaMalloc(&e->red, sizeof(unsigned long long) * qmk::RED_WORDS));
+  QMK_CUDA(e, cudaMalloc(&e->red, sizeof(unsigned long long) * RED_ALLOC_WORDS));
   QMK_CUDA(e, cudaHostAlloc(&e->status_host, 16, cudaHostAllocDefault));
   memset(e->status_host, 0, 16);
   if (!e->inv_freq_set) {
@@ -353,7 +357,8 @@ void free_prepared(Engine::Prepared &p) {
 constexpr size_t MAX_PREPARED = 4;   // weight sets kept per device (a 28-layer fp16 set is 294 MB)
 
 // Finds or creates the K-major copies for the caller's layer table and enqueues the check-and-rebuild kernel.
-int ensure_prepared(Engine *e, const Params &P, int wfmt, cudaStream_t stream, Engine::Prepared **out) {
+// `optional`: where they do not fit in memory, *out stays null instead of an error.
+int ensure_prepared(Engine *e, const Params &P, int wfmt, cudaStream_t stream, Engine::Prepared **out, bool optional = false) {
   Engine::Prepared *hit = nullptr;
   for (auto &p : e->prepared)
     if (p.table == P.layers && p.num_layers == P.num_layers && p.wfmt == wfmt) hit = &p;
@@ -371,7 +376,11 @@ int ensure_prepared(Engine *e, const Params &P, int wfmt, cudaStream_t stream, E
     p.num_layers = P.num_layers;
     p.wfmt = wfmt;
     const size_t ob = kmajor_o_bytes(wfmt), db = kmajor_d_bytes(wfmt);
-    QMK_CUDA(e, cudaMalloc(&p.buf, (ob + db) * P.num_layers));
+    if (const cudaError_t err = cudaMalloc(&p.buf, (ob + db) * P.num_layers); err != cudaSuccess) {
+      cudaGetLastError();
+      if (optional && err == cudaErrorMemoryAllocation) return QMK_OK;
+      return fail(e, QMK_ERR_CUDA, std::string("cudaMalloc of the K-major copies: ") + cudaGetErrorString(err));
+    }
     QMK_CUDA(e, cudaMalloc(&p.tbl, sizeof(qmkp::LayerT) * P.num_layers));
     QMK_CUDA(e, cudaMalloc(&p.fp, sizeof(unsigned long long) * 4 * P.num_layers));
     QMK_CUDA(e, cudaMemsetAsync(p.fp, 0, sizeof(unsigned long long) * 4 * P.num_layers, stream));
@@ -410,6 +419,18 @@ void mirror_sequence0(Params &P) {
   P.k_caches[0] = P.k_cache;
   P.v_caches[0] = P.v_cache;
   P.output_logs[0] = P.output_log;
+}
+
+// Tiled-copy descriptors of the caller's caches (host-side encode, a few microseconds).
+int encode_cache_maps(Engine *e, Params &P) {
+  std::string merr;
+  const uint64_t kv_rows = static_cast<uint64_t>(P.num_layers) * qmk::NKV * static_cast<uint64_t>(P.max_seq_len);
+  for (int b = 0; b < P.nseq; ++b) {
+    int rc = qmk_tc::make_map_f16(reinterpret_cast<CUtensorMap *>(P.kmaps[b]), P.k_caches[b], kv_rows, qmk::D, 16, &merr);
+    if (rc == QMK_OK) rc = qmk_tc::make_map_f16(reinterpret_cast<CUtensorMap *>(P.vmaps[b]), P.v_caches[b], kv_rows, qmk::D, 16, &merr);
+    if (rc != QMK_OK) return fail(e, rc, "KV cache tensor map: " + merr);
+  }
+  return QMK_OK;
 }
 
 // Common launch path.  `P` arrives with the per-call fields set; `batch` selects the multi-sequence
@@ -466,7 +487,28 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
   void *args[] = {&P};
   const int grid = grid_for(e);
   const void *kernel = batch ? qmk_batch::kernel() : single_sequence_kernel(grid);
-  size_t smem = qmk::SMEM_BYTES;
+  size_t smem = batch ? qmk_batch::smem_bytes() : qmk::SMEM_BYTES;
+  int threads = batch ? qmk_batch::threads() : qmk::THREADS;
+  if (batch && e->fused >= 2) {
+    // several sequences on the tensor cores: two with 512 + 48 tokens 63.7 -> 32.9 ms.  The group-per-sequence kernel stays
+    // for the grids and vocabularies outside the limits, and where the K-major copies do not fit in memory.
+    const qmk_fused_tc::Build &tc = qmk_fused_tc::build_seqs(e->wfmt, P.nseq);
+    Engine::Prepared *prep = nullptr;
+    if (P.vocab % tc.rows_per_chunk == 0 && grid >= tc.min_ctas && grid <= tc.max_ctas) {
+      rc = ensure_prepared(e, P, e->wfmt, stream, &prep, true);
+      if (rc != QMK_OK) return rc;
+    }
+    if (prep) {
+      rc = encode_cache_maps(e, P);
+      if (rc != QMK_OK) return rc;
+      QMK_CUDA(e, cudaMemsetAsync(e->red, 0, sizeof(unsigned long long) * RED_ALLOC_WORDS, stream));
+      P.layers_t = prep->tbl;
+      P.red = e->red;
+      kernel = tc.kernel;
+      smem = tc.smem_bytes;
+      threads = qmk::THREADS;
+    }
+  }
   if (!batch && e->fused && grid >= qmk::FUSED_MIN_CTAS &&
       kernel == reinterpret_cast<const void *>(qmk::qwen3_decode_megakernel)) {
     // fused kernel: O and down projections as split-K slices of K-major copies, two all-reduced residual sums
@@ -484,20 +526,13 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
     // vocabularies outside these limits.
     const qmk_fused_tc::Build &tc = qmk_fused_tc::build(e->wfmt);
     if (e->fused >= 2 && P.vocab % tc.rows_per_chunk == 0 && grid >= tc.min_ctas && grid <= tc.max_ctas) {
-      // tiled-copy descriptors of the caller's caches (host-side encode, a few microseconds)
-      std::string merr;
-      const uint64_t kv_rows = static_cast<uint64_t>(P.num_layers) * qmk::NKV * static_cast<uint64_t>(P.max_seq_len);
-      rc = qmk_tc::make_map_f16(reinterpret_cast<CUtensorMap *>(P.kmap), P.k_cache, kv_rows, qmk::D, 16, &merr);
-      if (rc == QMK_OK) rc = qmk_tc::make_map_f16(reinterpret_cast<CUtensorMap *>(P.vmap), P.v_cache, kv_rows, qmk::D, 16, &merr);
-      if (rc != QMK_OK) return fail(e, rc, "KV cache tensor map: " + merr);
+      rc = encode_cache_maps(e, P);
+      if (rc != QMK_OK) return rc;
       kernel = tc.kernel;
       smem = tc.smem_bytes;
     }
   }
-  cudaError_t err =
-      batch ? cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(qmk_batch::threads()), args,
-                                          qmk_batch::smem_bytes(), stream)
-            : cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(qmk::THREADS), args, smem, stream);
+  const cudaError_t err = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, smem, stream);
   if (err == cudaErrorCooperativeLaunchTooLarge)
     return fail(e, QMK_ERR_NOT_RESIDENT, "persistent grid cannot be co-resident on this device");
   if (err != cudaSuccess) return fail(e, QMK_ERR_CUDA, std::string("cudaLaunchCooperativeKernel: ") + cudaGetErrorString(err));

@@ -37,7 +37,14 @@
 namespace QMK_NS {
 #if QMK_MAX_SEQ == 1 && defined(QMK_TC_BUILD)
 
-constexpr int TC_MIN_CTAS = 96;                // smallest grid: <= 2 attention outputs per warp to merge, O / down slices of <= 32 rows
+#ifndef QMK_TC_SEQS
+#define QMK_TC_SEQS 1
+#endif
+constexpr int TC_SEQS = QMK_TC_SEQS;           // sequences a launch can carry (2 and 4: megakernel_tc_multi.cuh)
+static_assert(TC_SEQS == 1 || TC_SEQS == 2 || TC_SEQS == 4, "two of the eight columns of an MMA per sequence");
+// smallest grid: <= 2 attention outputs per warp to merge, O / down slices of <= 32 rows; four sequences: phases of at
+// most as many chunks as their shorter ring has slots
+constexpr int TC_MIN_CTAS = TC_SEQS == 4 ? 112 : 96;
 static_assert(TC_MIN_CTAS >= FUSED_MIN_CTAS, "the tensor-core kernel shares the fused kernel's slice layout");
 #ifdef QMK_TC_FP8
 constexpr bool FP8_ROWS = true;
@@ -82,24 +89,37 @@ constexpr int KPAIRS = H / 32;                 // pairs of 16-input k-steps in a
 // warp fetch a pair's operand with ONE 128-byte wavefront (ldmatrix.x4 over plain hi / lo rows takes four; the row
 // products are bound by shared-memory bandwidth, where that is a third of the traffic).
 constexpr size_t OFF_XF = (SMEM_BYTES + 127) / 128 * 128;
-constexpr size_t OFF_PART = OFF_XF + 4 * H;                    // fp32 tile partials [2][12 tasks][16 rows]
-constexpr size_t OFF_QF = OFF_PART + 2 * 12 * 16 * 4;           // fp16 query operand [4: q0 hi, q0 lo, q1 hi, q1 lo][128], rows at KV_PITCH
-constexpr size_t OFF_ACT16 = OFF_QF + 4 * KV_PITCH;            // fp16 hi row, scaled-lo row of a slice's activations (merge / gate-up outputs)
-constexpr size_t OFF_TCTAB = OFF_ACT16 + ((2 * ACT16_PITCH * 2 + 15) / 16) * 16;
+constexpr int XF_PAIR = 128 * TC_SEQS;                         // bytes of a pair's operand: [sequence][hi, lo]
+constexpr int PART_TASK = 16 * TC_SEQS;                        // floats of a tile task's partials
+constexpr size_t OFF_PART = OFF_XF + 4 * H * TC_SEQS;          // fp32 tile partials [2][12 tasks][sequence][16 rows]
+constexpr size_t OFF_QF = OFF_PART + 2 * 12 * PART_TASK * 4;   // fp16 query operand [4: q0 hi, q0 lo, q1 hi, q1 lo][128], rows at KV_PITCH
+constexpr size_t OFF_ACT16 = OFF_QF + 4 * KV_PITCH;            // fp16 hi row, scaled-lo row of a slice's activations (merge / gate-up outputs), per sequence
+constexpr size_t OFF_TCTAB = OFF_ACT16 + ((TC_SEQS * 2 * ACT16_PITCH * 2 + 15) / 16) * 16;
 struct alignas(16) TileTask { int active, first, valid, p0, p1, units, pad0, pad1; };   // see build_tile_tasks
 struct alignas(16) TcTab {
   int q0, nq, g0, ng, lm0, nlm;    // first chunk / chunks of this CTA: q|k|v rows, gate (= up) rows, LM-head rows
   int nkb_qkv, nkb_gu;             // warps per tile in the two row-product phases
   TileTask qkv[12], gu[12];        // each warp's tile task in those phases
+  int s_cap, seq, local, pad;      // several sequences: most splits of one, the sequence of this CTA's attention item, the item
 };
-constexpr size_t TC_SMEM_BYTES = OFF_TCTAB + sizeof(TcTab);
+// Several sequences: previous contributions to the residual sums [x1, x2][sequence][1024] (sequences 0 and 1 where the
+// single-sequence kernel has its fp32 vectors; the pitch puts the four sequences of a fragment into different banks),
+// residuals of the outputs this CTA owns, split weights of the merge, sums of squares, tokens.
+constexpr int PREV_PITCH = H + 8, RESID_PITCH = 12;
+static_assert(4 * PREV_PITCH <= FF_SPLITW, "sequences 0 and 1 fit in front of the attention's split weights");
+constexpr size_t OFF_PREV2 = OFF_TCTAB + (sizeof(TcTab) + 15) / 16 * 16;
+constexpr size_t OFF_RESID = OFF_PREV2 + (TC_SEQS > 2 ? 4 * PREV_PITCH * 4 : 0);
+constexpr size_t OFF_SPLITW = OFF_RESID + 2 * TC_SEQS * RESID_PITCH * 4;
+constexpr size_t OFF_REDM = OFF_SPLITW + 2 * 32 * 4;
+constexpr size_t OFF_TOKENS = OFF_REDM + TC_SEQS * CONS_WARPS * 4;
+constexpr size_t TC_SMEM_BYTES = TC_SEQS > 1 ? OFF_TOKENS + TC_SEQS * 4 : OFF_TCTAB + sizeof(TcTab);
 static_assert(TC_SMEM_BYTES <= 232448, "over the 227 KB shared-memory limit of one CTA");
 static_assert(OFF_XF % 128 == 0 && OFF_QF % 16 == 0, "operand rows are 16-byte aligned, a pair's 128 bytes one wavefront");
-// Byte offset in the fragment-order array of input i's hi (lo = 0) or lo (1) half.
-__device__ __forceinline__ int xf_offset(int i, int lo) {
+// Byte offset in the fragment-order array of input i's hi (lo = 0) or lo (1) half, sequence b.
+__device__ __forceinline__ int xf_offset(int i, int lo, int b = 0) {
   const int kk = i & 31, rem = kk & 15, r8 = rem & 7;
-  if (FP8_ROWS) return (i >> 5) * 128 + lo * 64 + (rem >> 2) * 16 + (kk >> 4) * 8 + (i & 3) * 2;   // lane kq: inputs 4 kq .. 4 kq + 3
-  return (i >> 5) * 128 + lo * 64 + (r8 >> 1) * 16 + ((kk >> 4) * 4 + (rem >> 3) * 2 + (r8 & 1)) * 2;
+  if (FP8_ROWS) return (i >> 5) * XF_PAIR + b * 128 + lo * 64 + (rem >> 2) * 16 + (kk >> 4) * 8 + (i & 3) * 2;   // lane kq: inputs 4 kq .. 4 kq + 3
+  return (i >> 5) * XF_PAIR + b * 128 + lo * 64 + (r8 >> 1) * 16 + ((kk >> 4) * 4 + (rem >> 3) * 2 + (r8 & 1)) * 2;
 }
 
 __device__ __forceinline__ const TcTab *tctab(const Ctx &c) { return reinterpret_cast<const TcTab *>(c.smem + OFF_TCTAB); }
@@ -128,10 +148,10 @@ __device__ __forceinline__ uint32_t pack_half2(__half a, __half b) {
   return static_cast<uint32_t>(__half_as_ushort(a)) | (static_cast<uint32_t>(__half_as_ushort(b)) << 16);
 }
 
-// Activation operand of k-step pair p for this lane: column n = lane / 4 of B is the hi vector (n = 0), the lo vector
-// (n = 1) or zero; {x, y} = fragments of the first k-step, {z, w} of the second.
+// Activation operand of k-step pair p for this lane: column n = lane / 4 of B is the hi (even n) or the lo vector of
+// sequence n / 2, or zero; {x, y} = fragments of the first k-step, {z, w} of the second.
 __device__ __forceinline__ uint4 b_pair(const Ctx &c, int p) {
-  return c.lane < 8 ? *reinterpret_cast<const uint4 *>(c.smem + OFF_XF + p * 128 + c.lane * 16) : make_uint4(0u, 0u, 0u, 0u);
+  return c.lane < 8 * TC_SEQS ? *reinterpret_cast<const uint4 *>(c.smem + OFF_XF + p * XF_PAIR + c.lane * 16) : make_uint4(0u, 0u, 0u, 0u);
 }
 
 // Shared-window address of row 0 of the weight chunk with ring index idx.
@@ -150,7 +170,7 @@ __device__ __forceinline__ void e4m3x4_half2x2(uint32_t four, uint32_t &first, u
 }
 
 // One warp: rows of the 16-row tile that starts at ring chunk `first` (valid rows <= 16), k-step pairs [p0, p1).
-// Leaves the 16 row sums of that k range in part[0..15] and hands the tile's chunks back with `units` each.
+// Leaves the 16 row sums of that k range in part[0..15] (sequence b: part[16 b..]) and hands the tile's chunks back with `units` each.
 // Lanes 0..3 each wait for one of the tile's chunks (the vote that follows orders the copied bytes before every
 // lane's loads); two accumulators halve the chain of dependent MMAs.
 __device__ __forceinline__ void tile_task(const Params &P, const Ctx &c, uint32_t first, int valid_rows, int p0, int p1,
@@ -189,14 +209,15 @@ __device__ __forceinline__ void tile_task(const Params &P, const Ctx &c, uint32_
   }
   QMK_FINE(fslot + 5);
   float sc_top = 1.f, sc_bot = 1.f;                     // row scales, read before the rows are handed back
-  if (FP8_ROWS && (c.lane & 3) == 0) {
+  if (FP8_ROWS && (c.lane & 3) < TC_SEQS) {
     const int r0 = c.lane >> 2, r1 = r0 + 8;
     if (r0 < valid_rows) sc_top = *reinterpret_cast<const float *>(c.slot(first + static_cast<uint32_t>(r0 / CH_ROWS)) + (r0 % CH_ROWS) * ROW_PITCH + H);
     if (r1 < valid_rows) sc_bot = *reinterpret_cast<const float *>(c.slot(first + static_cast<uint32_t>(r1 / CH_ROWS)) + (r1 % CH_ROWS) * ROW_PITCH + H);
   }
   __syncwarp();
   if (c.lane < nch) mbar_arrive_n(c.empty((first + static_cast<uint32_t>(c.lane)) % NSLOTS), static_cast<uint32_t>(units));
-  if ((c.lane & 3) == 0) {
+  if ((c.lane & 3) < TC_SEQS) {   // quad b of a fragment: the hi and lo columns of sequence b
+    part += (c.lane & 3) * 16;
     part[c.lane >> 2] = fmaf(acc0[1] + acc1[1], LO_INV, acc0[0] + acc1[0]) * sc_top;
     part[(c.lane >> 2) + 8] = fmaf(acc0[3] + acc1[3], LO_INV, acc0[2] + acc1[2]) * sc_bot;
   }
@@ -225,9 +246,10 @@ __device__ inline void build_tile_tasks(TileTask *tasks, int *nkb_out, int group
 __device__ __forceinline__ void run_tile_task(const Params &P, const Ctx &c, const TileTask *tasks, int fslot) {
   const int4 a = reinterpret_cast<const int4 *>(tasks + c.warp)[0], b = reinterpret_cast<const int4 *>(tasks + c.warp)[1];
   // a = {active, first, valid, p0}, b = {p1, units, -, -}
-  if (a.x) tile_task(P, c, c.chunk + static_cast<uint32_t>(a.y), a.z, a.w, b.x, tc_part(c) + c.warp * 16, b.y, fslot);
+  if (a.x) tile_task(P, c, c.chunk + static_cast<uint32_t>(a.y), a.z, a.w, b.x, tc_part(c) + c.warp * PART_TASK, b.y, fslot);
 }
 
+#if QMK_TC_SEQS == 1
 // q|k|v rows of this CTA -> exchange words (megakernel_5090.cu:251-302).
 __device__ __noinline__ uint32_t qkv_phase(const Params &P, Ctx c, uint32_t tag) {
   const TcTab *t = tctab(c);
@@ -279,6 +301,28 @@ __device__ __noinline__ uint32_t gateup_phase(const Params &P, Ctx c) {
   return c.chunk + static_cast<uint32_t>(2 * nch);
 }
 
+#endif  // QMK_TC_SEQS == 1
+
+// The exchange area of the sequence this CTA attends for.
+__device__ __forceinline__ unsigned long long *tc_ll(const Params &P, const Ctx &c) {
+  return TC_SEQS == 1 ? P.ll : P.ll + static_cast<size_t>(tctab(c)->seq) * LL_WORDS;
+}
+// attn_item (megakernel_device.cuh); several sequences: of the sequence the CTA belongs to, with at most s_cap splits.
+__device__ __forceinline__ AttnItem tc_item(const Params &P, const Ctx &c, int pos) {
+  if (TC_SEQS == 1) return attn_item(P, c, 0, 1, CONS_WARPS, pos);
+  const int local = tctab(c)->local;
+  AttnItem it;
+  it.S = max(1, min(pos / max(1, P.split_len), tctab(c)->s_cap));
+  it.active = local < NKV * it.S;
+  it.g = local % NKV;
+  it.s = local / NKV;
+  it.p0 = it.active ? static_cast<int>(static_cast<unsigned>(pos * it.s) / static_cast<unsigned>(it.S)) : 0;
+  it.p1 = it.active ? static_cast<int>(static_cast<unsigned>(pos * (it.s + 1)) / static_cast<unsigned>(it.S)) : 0;
+  it.rpc = KV_ROWS_PER_CHUNK;
+  it.nchunks = (it.p1 - it.p0 + KV_ROWS_PER_CHUNK - 1) / KV_ROWS_PER_CHUNK;
+  return it;
+}
+
 // Attention work item (kv head g, split s) of this CTA on the tensor cores.  Same contract as attention_phase
 // (megakernel_device.cuh): old cache rows [p0, p1) arrive as ring chunks of 16 K rows + 16 V rows (272-byte pitch),
 // warp w takes chunks w, w + 12, ...; the last split also normalises, rotates and stores the new K/V row and folds
@@ -288,7 +332,7 @@ __device__ __noinline__ uint32_t gateup_phase(const Params &P, Ctx c) {
 // MMAs with V read through ldmatrix.trans and p split into hi/lo fp16 columns like q: ~75 instructions per 16
 // rows where the CUDA-core loop needs ~480.
 __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __half *nv, int layer, int pos, uint32_t tag) {
-  const AttnItem it = attn_item(P, c, 0, 1, CONS_WARPS, pos);
+  const AttnItem it = tc_item(P, c, pos);
   float *s_q = c.f(F_Q), *s_knew = c.f(F_KNEW), *s_vnew = c.f(F_VNEW), *s_wpart = c.f(F_WPART), *s_misc = c.f(F_MISC);
   const float *s_cs = c.f(F_CS);
   const unsigned long long *qkv = c.llr + LL_QKV;
@@ -479,7 +523,7 @@ __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __ha
     const float L = warp_sum(lw * scw);
     if (c.lane < 16) s_scale[h * 16 + c.lane] = scw;
     if (c.lane == 0) {
-      unsigned long long *part = P.ll + LL_PART + static_cast<size_t>((2 * g + h) * MAX_SPLITS + s) * PART_STRIDE;
+      unsigned long long *part = tc_ll(P, c) + LL_PART + static_cast<size_t>((2 * g + h) * MAX_SPLITS + s) * PART_STRIDE;
       ll_store(part + D, M, tag);
       ll_store(part + D + 1, L, tag);
     }
@@ -490,13 +534,15 @@ __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __ha
     float A = s_vnew[d] * s_scale[h * 16 + CONS_WARPS];   // 0 weight unless this CTA owns the new row
 #pragma unroll
     for (int w = 0; w < CONS_WARPS; ++w) A = fmaf(s_wpart[(w * 2 + h) * PART_STRIDE + d], s_scale[h * 16 + w], A);
-    ll_store(P.ll + LL_PART + static_cast<size_t>((2 * g + h) * MAX_SPLITS + s) * PART_STRIDE + d, A, tag);
+    ll_store(tc_ll(P, c) + LL_PART + static_cast<size_t>((2 * g + h) * MAX_SPLITS + s) * PART_STRIDE + d, A, tag);
   }
   QMK_FINE(66);
   // New K,V row -> cache (megakernel_5090.cu:392-397), off the critical path.  The fence orders the row before the
   // exchange words this CTA publishes later; readers fence once per step.
   if (owner && (c.warp == 2 || c.warp == 3)) {
-    __half *cache = ((c.warp == 2) ? P.k_cache : P.v_cache) + head_base + static_cast<size_t>(pos) * D;
+    __half *const k_cache = TC_SEQS == 1 ? P.k_cache : per_seq(P.k_caches, tctab(c)->seq);
+    __half *const v_cache = TC_SEQS == 1 ? P.v_cache : per_seq(P.v_caches, tctab(c)->seq);
+    __half *cache = ((c.warp == 2) ? k_cache : v_cache) + head_base + static_cast<size_t>(pos) * D;
     const float *snew = (c.warp == 2) ? s_knew : s_vnew;
 #pragma unroll
     for (int i = 0; i < 4; ++i) cache[c.lane + 32 * i] = __float2half_rn(snew[c.lane + 32 * i]);
@@ -505,6 +551,7 @@ __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __ha
   return c.chunk;
 }
 
+#if QMK_TC_SEQS == 1
 // 1 / sqrt(mean of squares + eps) over the 1024 values whose squares the consumer threads hold in `ss`; one barrier.
 // (rsqrt.approx: 2 ulp; the sum's order is fixed.)
 __device__ __forceinline__ float block_rstd(const Ctx &c, float ss) {
@@ -611,21 +658,27 @@ __device__ __noinline__ void red_wait_norm(const Params &P, const Ctx c, int whi
   QMK_FINE(which ? 46 : 42);
 }
 
+#endif  // QMK_TC_SEQS == 1
+
+// Element n of an embedding row.
+__device__ __forceinline__ float embed_value(const unsigned char *erow, int n) {
+  if (FP8_ROWS) {
+    const __half_raw hr = __nv_cvt_fp8_to_halfraw(static_cast<__nv_fp8_storage_t>(__ldg(erow + n)), __NV_E4M3);
+    return __half2float(*reinterpret_cast<const __half *>(&hr)) * __ldg(reinterpret_cast<const float *>(erow + H));
+  }
+  return __half2float(__ldg(reinterpret_cast<const __half *>(erow) + n));
+}
+
+#if QMK_TC_SEQS == 1
 // Embedding row of `token` (megakernel_5090.cu:825-830) -> residual stream, normalised with layer 0's input norm.
 __device__ __noinline__ void embed_norm(const Params &P, const Ctx c, int token, const __half *norm_w) {
   constexpr int PT = (H + CONS_THREADS - 1) / CONS_THREADS;
   const unsigned char *erow = reinterpret_cast<const unsigned char *>(P.embed) + static_cast<size_t>(token) * ROW_BYTES;
-  const float escale = FP8_ROWS ? __ldg(reinterpret_cast<const float *>(erow + H)) : 1.f;
   float v[PT], ss = 0.f;
 #pragma unroll
   for (int j = 0; j < PT; ++j) {
     const int n = c.tid + j * CONS_THREADS;
-    if (FP8_ROWS) {
-      const __half_raw hr = __nv_cvt_fp8_to_halfraw(static_cast<__nv_fp8_storage_t>(n < H ? __ldg(erow + n) : 0), __NV_E4M3);
-      v[j] = __half2float(*reinterpret_cast<const __half *>(&hr)) * escale;
-    } else {
-      v[j] = n < H ? __half2float(__ldg(reinterpret_cast<const __half *>(erow) + n)) : 0.f;
-    }
+    v[j] = n < H ? embed_value(erow, n) : 0.f;
     ss = fmaf(v[j], v[j], ss);
   }
   const float rstd = block_rstd(c, ss);
@@ -637,6 +690,48 @@ __device__ __noinline__ void embed_norm(const Params &P, const Ctx c, int token,
   cons_sync();
 }
 
+#endif  // QMK_TC_SEQS == 1
+
+// A operand of a slice's tiles: this lane's row of each k-step (rows past the slice repeat row 0: their activations are
+// zero).  fp8: one ldmatrix.x4 takes 32 rows x 16 outputs, a lane's register holds outputs 2j, 2j + 1 of rows 2q and
+// 2q + 1 (j = lane / 4); fragment rows j, j + 8 are those two outputs.
+__device__ __forceinline__ void slice_row_addresses(const Ctx &c, int nrows, uint32_t (&arow)[2]) {
+#pragma unroll
+  for (int ks = 0; ks < 2; ++ks) {
+    int row = FP8_ROWS ? c.lane : ks * 16 + (c.lane & 7) + 8 * (c.lane >> 4);
+    if (row >= nrows) row = 0;
+    arow[ks] = weight_rows(c, c.chunk + static_cast<uint32_t>(row / CH_ROWS)) + (row % CH_ROWS) * ROW_PITCH + (FP8_ROWS ? 0 : ((c.lane >> 3) & 1) * 16);
+  }
+}
+// Output tiles t0 and t0 + 12 of a slice (past the end: a valid tile again, for the caller to ignore).
+__device__ __forceinline__ void slice_tiles(const uint32_t (&arow)[2], const uint32_t (&bq)[4], int t0, bool two, float (&acc)[2][4]) {
+  uint32_t a[2][4], a2[2][4];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int tile = min(t0 + u * CONS_WARPS, H / 16 - 1);
+    acc[u][0] = 0.f; acc[u][1] = 0.f; acc[u][2] = 0.f; acc[u][3] = 0.f;
+    if (FP8_ROWS) {
+      uint32_t r[4];
+      ldsm_x4_trans(arow[0] + tile * 16, r);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r[i] = __byte_perm(r[i], 0u, 0x3120);   // {row 2q, 2q + 1} of the first output, then of the second
+      e4m3x4_half2x2(r[0], a[u][0], a[u][1]);
+      e4m3x4_half2x2(r[1], a[u][2], a[u][3]);
+      e4m3x4_half2x2(r[2], a2[u][0], a2[u][1]);
+      e4m3x4_half2x2(r[3], a2[u][2], a2[u][3]);
+    } else {
+      ldsm_x4_trans(arow[0] + tile * 32, a[u]);
+      if (two) ldsm_x4_trans(arow[1] + tile * 32, a2[u]);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    mma_16816(acc[u], a[u], bq[0], bq[1]);
+    if (two) mma_16816(acc[u], a2[u], bq[2], bq[3]);
+  }
+}
+
+#if QMK_TC_SEQS == 1
 // Split-K slice of the O (which = 0) or down (1) projection (see slice_colgemv of megakernel_fused.cuh) on the
 // tensor cores: partial[n] = sum_i act[i] * Wt[first + i][n] with the K-major rows as the A operand read through
 // ldmatrix.trans (tile = 16 outputs x 16 rows, at most two k-steps: slices of at most 32 rows), the slice's
@@ -665,16 +760,8 @@ __device__ __noinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
     // B: the slice's activations; row n of B^T = hi (even n) / lo (odd n) vector; one ldmatrix.x4 = two k-steps
     uint32_t bq[4];
     ldsm_x4(smem_u32(c.smem + OFF_ACT16) + (c.lane & 1) * (ACT16_PITCH * 2) + (c.lane >> 3) * 16, bq);
-    // A: this lane's row of each k-step (rows past the slice repeat row 0: their activations are zero).  fp8: one
-    // ldmatrix.x4 takes 32 rows x 16 outputs, a lane's register holds outputs 2j, 2j + 1 of rows 2q and 2q + 1
-    // (j = lane / 4); fragment rows j, j + 8 are those two outputs.
     uint32_t arow[2];
-#pragma unroll
-    for (int ks = 0; ks < 2; ++ks) {
-      int row = FP8_ROWS ? c.lane : ks * 16 + (c.lane & 7) + 8 * (c.lane >> 4);
-      if (row >= nrows) row = 0;
-      arow[ks] = weight_rows(c, c.chunk + static_cast<uint32_t>(row / CH_ROWS)) + (row % CH_ROWS) * ROW_PITCH + (FP8_ROWS ? 0 : ((c.lane >> 3) & 1) * 16);
-    }
+    slice_row_addresses(c, nrows, arow);
     const int n0 = t->n0, n1 = t->n1;
     // lane that holds this lane's output (fragment row = lane / 4), and whether it is its second row
     const int src = FP8_ROWS ? ((c.lane & 15) >> 1) * 4 : (c.lane & 7) * 4;
@@ -682,30 +769,7 @@ __device__ __noinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
 #pragma unroll 1
     for (int t0 = c.warp; t0 < H / 16; t0 += 2 * CONS_WARPS) {
       float acc[2][4];
-      uint32_t a[2][4], a2[2][4];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int tile = min(t0 + u * CONS_WARPS, H / 16 - 1);   // past the end: repeat a valid tile, not added
-        acc[u][0] = 0.f; acc[u][1] = 0.f; acc[u][2] = 0.f; acc[u][3] = 0.f;
-        if (FP8_ROWS) {
-          uint32_t r[4];
-          ldsm_x4_trans(arow[0] + tile * 16, r);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) r[i] = __byte_perm(r[i], 0u, 0x3120);   // {row 2q, 2q + 1} of the first output, then of the second
-          e4m3x4_half2x2(r[0], a[u][0], a[u][1]);
-          e4m3x4_half2x2(r[1], a[u][2], a[u][3]);
-          e4m3x4_half2x2(r[2], a2[u][0], a2[u][1]);
-          e4m3x4_half2x2(r[3], a2[u][2], a2[u][3]);
-        } else {
-          ldsm_x4_trans(arow[0] + tile * 32, a[u]);
-          if (two) ldsm_x4_trans(arow[1] + tile * 32, a2[u]);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        mma_16816(acc[u], a[u], bq[0], bq[1]);
-        if (two) mma_16816(acc[u], a2[u], bq[2], bq[3]);
-      }
+      slice_tiles(arow, bq, t0, two, acc);
       // lanes of quad 0 hold (hi, lo) sums of fragment rows lane / 4 and lane / 4 + 8 of both tiles; lane L takes output
       // L % 16 of tile L / 16
       const float s0 = __shfl_sync(0xffffffffu, fmaf(acc[0][1], LO_INV, acc[0][0]), src);
@@ -776,6 +840,8 @@ __device__ __noinline__ uint32_t lm_head_tc(const Params &P, Ctx c, float *dump)
   return c.chunk + static_cast<uint32_t>(nch);
 }
 
+#endif  // QMK_TC_SEQS == 1
+
 // ----------------------------------------------------------------------------- producer (one warp)
 // The warp issues eight chunks at a time: lanes 4g..4g+3 own chunk g of the group of eight, lane 4g waits for
 // the slot and announces the bytes, lane 4g + r copies row r (one cp.async.bulk per row, 2064-byte pitch).  Per
@@ -787,7 +853,8 @@ __device__ __noinline__ uint32_t lm_head_tc(const Params &P, Ctx c, float *dump)
 // [layers * 8 * max_seq_len][128]); lane r of the group copies box r (K low dims, K high dims, V low, V high).
 struct ChunkSrc { const unsigned char *src; size_t src_pitch; uint32_t rows, row_bytes, dst_pitch; int kv_row; };
 
-__device__ __forceinline__ bool tc_issue8(const Params &P, const Ctx &c, uint32_t ci, bool active, const ChunkSrc &d, uint64_t pol) {
+__device__ __forceinline__ bool tc_issue8(const Params &P, const Ctx &c, uint32_t ci, bool active, const ChunkSrc &d, uint64_t pol,
+                                          const void *kmap, const void *vmap) {
   if (__any_sync(0xffffffffu, (c.flags()[0] | c.flags()[1]) != 0)) return false;   // the warp leaves as a whole
   const uint32_t slot = ci % NSLOTS;
   bool ok = true;
@@ -797,7 +864,7 @@ __device__ __forceinline__ bool tc_issue8(const Params &P, const Ctx &c, uint32_
   if (active && sub == 0) mbar_arrive_expect_tx(c.full(slot), d.kv_row >= 0 ? 4u * KV_BOX : d.rows * d.row_bytes);
   __syncwarp();
   if (active && d.kv_row >= 0) {
-    tma_box_2d(smem_u32(c.slot(ci)) + sub * KV_BOX, sub < 2 ? static_cast<const void *>(P.kmap) : static_cast<const void *>(P.vmap),
+    tma_box_2d(smem_u32(c.slot(ci)) + sub * KV_BOX, sub < 2 ? kmap : vmap,
                (sub & 1) * 64, d.kv_row, c.full(slot));
   } else if (active && sub < static_cast<int>(d.rows)) {
     bulk_g2s(c.slot(ci) + (ci & 1u) * ODD_SLOT_SKEW + sub * d.dst_pitch, d.src + sub * d.src_pitch, d.row_bytes, c.full(slot), pol);
@@ -830,12 +897,21 @@ __device__ __noinline__ void producer_main_tc(const Params &P, const Ctx c) {
   const SegTab *t = c.segs();
   const TcTab *tt = tctab(c);
   const int grp = c.lane >> 2;
+  // the caches this CTA attends to
+  const int seq = TC_SEQS == 1 ? 0 : tt->seq;
+  const void *kmap = P.kmaps[0], *vmap = P.vmaps[0];
+  if (TC_SEQS > 1) {
+#pragma unroll
+    for (int b = 1; b < TC_SEQS; ++b)
+      if (seq == b) { kmap = P.kmaps[b]; vmap = P.vmaps[b]; }
+  }
+  const int start = TC_SEQS == 1 ? P.start_position : per_seq(P.start_positions, seq);
   const int nq = tt->nq, ng = tt->ng, ne = t->e1 - t->e0, no = (ne + CH_ROWS - 1) / CH_ROWS;
   uint32_t idx = 0, issued = 0;   // first chunk of the current layer / chunks issued so far
   bool ok = true;
 #pragma unroll 1
   for (int step = 0; ok && step < P.num_steps; ++step) {
-    const AttnItem it = attn_item(P, c, 0, 1, CONS_WARPS, P.start_position + step);
+    const AttnItem it = tc_item(P, c, start + step);
     const int s1 = nq, s2 = s1 + it.nchunks, s3 = s2 + no + SCALE_CH, s4 = s3 + ng, s5 = s4 + ng, per_layer = s5 + ng + SCALE_CH;
 #pragma unroll 1
     for (int l = 0; ok && l < P.num_layers; ++l) {
@@ -876,7 +952,7 @@ __device__ __noinline__ void producer_main_tc(const Params &P, const Ctx c) {
         } else if (j < per_layer) {
           d = scale_chunk(reinterpret_cast<const void *>(rect[1]), I);
         }
-        ok = tc_issue8(P, c, idx + static_cast<uint32_t>(j), j < per_layer, d, pol);   // issues all eight or none
+        ok = tc_issue8(P, c, idx + static_cast<uint32_t>(j), j < per_layer, d, pol, kmap, vmap);   // issues all eight or none
         if (ok) issued = idx + static_cast<uint32_t>(min(j0 + 8, per_layer));
       }
       idx += static_cast<uint32_t>(per_layer);
@@ -886,7 +962,7 @@ __device__ __noinline__ void producer_main_tc(const Params &P, const Ctx c) {
       for (int j0 = 0; ok && j0 < tt->nlm; j0 += 8) {
         const int j = j0 + grp;
         const ChunkSrc d = matrix_chunk(P.lm_head, (tt->lm0 + j) * CH_ROWS, CH_ROWS);
-        ok = tc_issue8(P, c, idx + static_cast<uint32_t>(j), j < tt->nlm, d, pol);
+        ok = tc_issue8(P, c, idx + static_cast<uint32_t>(j), j < tt->nlm, d, pol, kmap, vmap);
         if (ok) issued = idx + static_cast<uint32_t>(min(j0 + 8, tt->nlm));
       }
       idx += static_cast<uint32_t>(tt->nlm);
@@ -895,6 +971,62 @@ __device__ __noinline__ void producer_main_tc(const Params &P, const Ctx c) {
   if (c.lane == 0) c.flags()[2] = static_cast<int>(issued);
 }
 
+// Barriers, tables and pointer records of a CTA; the caller synchronises the block.
+__device__ __forceinline__ void tc_setup(const Params &P, const Ctx &c) {
+  if (c.tid == 0) {
+    for (int i = 0; i < NSLOTS; ++i) { mbar_init(c.full(i), 1); mbar_init(c.empty(i), EMPTY_UNITS); }
+    mbar_init(c.nfull(0), 1);
+    mbar_init(c.nfull(1), 1);
+    volatile int *fl = c.flags();
+    fl[0] = 0; fl[1] = 0; fl[2] = 0; fl[3] = 0; fl[4] = 0; fl[5] = 0; fl[6] = 0; fl[8] = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (c.tid == 32) {
+    build_segtab(reinterpret_cast<SegTab *>(c.smem + OFF_SEGS), c.cta, c.ncta, P.vocab);
+    TcTab *tt = reinterpret_cast<TcTab *>(c.smem + OFF_TCTAB);
+    int a, b;
+    split_rows(QKV_CHUNKS, c.ncta, c.cta, a, b); tt->q0 = a; tt->nq = b - a;
+    split_rows(GU_CHUNKS, c.ncta, c.cta, a, b); tt->g0 = a; tt->ng = b - a;
+    split_rows(P.vocab / CH_ROWS, c.ncta, c.cta, a, b); tt->lm0 = a; tt->nlm = b - a;
+    build_tile_tasks(tt->qkv, &tt->nkb_qkv, 1, tt->nq);
+    build_tile_tasks(tt->gu, &tt->nkb_gu, 2, tt->ng);
+  }
+  {
+    const unsigned long long *src = reinterpret_cast<const unsigned long long *>(P.layers);
+    unsigned long long *dst = reinterpret_cast<unsigned long long *>(c.smem + OFF_LAYERS);
+    for (int i = c.tid; i < P.num_layers * 12; i += THREADS) dst[i] = src[i];
+    const unsigned long long *srct = reinterpret_cast<const unsigned long long *>(P.layers_t);
+    unsigned long long *dstt = reinterpret_cast<unsigned long long *>(c.smem + OFF_LAYERS_T);
+    for (int i = c.tid; i < P.num_layers * 2; i += THREADS) dstt[i] = srct[i];
+  }
+}
+
+// Bulk copies issued but never consumed must land before the CTA exits.
+__device__ __forceinline__ void tc_drain(const Params &P, const Ctx &c) {
+  if (c.tid == CONS_THREADS) {
+    const uint32_t issued = static_cast<uint32_t>(c.flags()[2]);
+#pragma unroll 1
+    for (uint32_t i = (issued > NSLOTS ? issued - NSLOTS : 0u); i < issued; ++i) {
+      uint64_t *bar = c.full(i % NSLOTS);
+      const uint32_t parity = (i / NSLOTS) & 1u;
+      const unsigned long long t0 = now_ns();
+      while (!mbar_try_wait(bar, parity)) {
+        if (now_ns() - t0 > P.timeout_ns) { raise_error(P, c, QMK_ERR_WAIT_TIMEOUT, WHERE_DRAIN); break; }
+      }
+    }
+    for (uint32_t b = 0; b < 2; ++b) {
+      const int v = c.flags()[4 + b];
+      if (v == 0) continue;
+      const uint32_t parity = ((static_cast<uint32_t>(v) - 1u) >> 1) & 1u;
+      const unsigned long long t0 = now_ns();
+      while (!mbar_try_wait(c.nfull(b), parity)) {
+        if (now_ns() - t0 > P.timeout_ns) { raise_error(P, c, QMK_ERR_WAIT_TIMEOUT, WHERE_DRAIN); break; }
+      }
+    }
+  }
+}
+
+#if QMK_TC_SEQS == 1
 __global__ void __launch_bounds__(THREADS, 1) qwen3_decode_megakernel_tc(const __grid_constant__ Params P) {
   extern __shared__ __align__(128) unsigned char smem[];
   Ctx c;
@@ -908,34 +1040,8 @@ __global__ void __launch_bounds__(THREADS, 1) qwen3_decode_megakernel_tc(const _
   c.repl = 1;
   c.llr = P.ll;
 
-  if (c.tid == 0) {
-    for (int i = 0; i < NSLOTS; ++i) { mbar_init(c.full(i), 1); mbar_init(c.empty(i), EMPTY_UNITS); }
-    mbar_init(c.nfull(0), 1);
-    mbar_init(c.nfull(1), 1);
-    volatile int *fl = c.flags();
-    fl[0] = 0; fl[1] = 0; fl[2] = 0; fl[3] = 0; fl[4] = 0; fl[5] = 0; fl[6] = 0; fl[8] = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (c.tid == 32) {
-    build_segtab(reinterpret_cast<SegTab *>(smem + OFF_SEGS), c.cta, c.ncta, P.vocab);
-    TcTab *tt = reinterpret_cast<TcTab *>(smem + OFF_TCTAB);
-    int a, b;
-    split_rows(QKV_CHUNKS, c.ncta, c.cta, a, b); tt->q0 = a; tt->nq = b - a;
-    split_rows(GU_CHUNKS, c.ncta, c.cta, a, b); tt->g0 = a; tt->ng = b - a;
-    split_rows(P.vocab / CH_ROWS, c.ncta, c.cta, a, b); tt->lm0 = a; tt->nlm = b - a;
-    build_tile_tasks(tt->qkv, &tt->nkb_qkv, 1, tt->nq);
-    build_tile_tasks(tt->gu, &tt->nkb_gu, 2, tt->ng);
-  }
-  {
-    const unsigned long long *src = reinterpret_cast<const unsigned long long *>(P.layers);
-    unsigned long long *dst = reinterpret_cast<unsigned long long *>(smem + OFF_LAYERS);
-    for (int i = c.tid; i < P.num_layers * 12; i += THREADS) dst[i] = src[i];
-    const unsigned long long *srct = reinterpret_cast<const unsigned long long *>(P.layers_t);
-    unsigned long long *dstt = reinterpret_cast<unsigned long long *>(smem + OFF_LAYERS_T);
-    for (int i = c.tid; i < P.num_layers * 2; i += THREADS) dstt[i] = srct[i];
-    float *prev = c.f(FF_PREV);
-    for (int i = c.tid; i < 2 * H; i += THREADS) prev[i] = 0.f;
-  }
+  tc_setup(P, c);
+  for (int i = c.tid; i < 2 * H; i += THREADS) c.f(FF_PREV)[i] = 0.f;
   __syncthreads();
 
   if (c.warp == CONS_WARPS) {
@@ -1026,28 +1132,9 @@ __global__ void __launch_bounds__(THREADS, 1) qwen3_decode_megakernel_tc(const _
     if (c.tid == 0) { c.flags()[3] = static_cast<int>(c.chunk); c.flags()[1] = 1; }
   }
   __syncthreads();
-  if (c.tid == CONS_THREADS) {   // bulk copies issued but never consumed must land before the CTA exits
-    const uint32_t issued = static_cast<uint32_t>(c.flags()[2]);
-#pragma unroll 1
-    for (uint32_t i = (issued > NSLOTS ? issued - NSLOTS : 0u); i < issued; ++i) {
-      uint64_t *bar = c.full(i % NSLOTS);
-      const uint32_t parity = (i / NSLOTS) & 1u;
-      const unsigned long long t0 = now_ns();
-      while (!mbar_try_wait(bar, parity)) {
-        if (now_ns() - t0 > P.timeout_ns) { raise_error(P, c, QMK_ERR_WAIT_TIMEOUT, WHERE_DRAIN); break; }
-      }
-    }
-    for (uint32_t b = 0; b < 2; ++b) {
-      const int v = c.flags()[4 + b];
-      if (v == 0) continue;
-      const uint32_t parity = ((static_cast<uint32_t>(v) - 1u) >> 1) & 1u;
-      const unsigned long long t0 = now_ns();
-      while (!mbar_try_wait(c.nfull(b), parity)) {
-        if (now_ns() - t0 > P.timeout_ns) { raise_error(P, c, QMK_ERR_WAIT_TIMEOUT, WHERE_DRAIN); break; }
-      }
-    }
-  }
+  tc_drain(P, c);
 }
+#endif  // QMK_TC_SEQS == 1
 
 #endif  // QMK_MAX_SEQ == 1 && QMK_TC_BUILD
 }  // namespace QMK_NS

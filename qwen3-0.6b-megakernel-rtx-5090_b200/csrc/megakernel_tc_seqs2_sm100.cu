@@ -1,0 +1,31 @@
+// Tensor-core decode megakernel for up to two sequences per launch, fp16 rows (see megakernel_tc_multi.cuh).
+#include <cuda_fp16.h>
+#include <cuda_fp8.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+#include <math.h>
+
+#include "../../include/qwen_megakernel.h"
+
+#include "megakernel_params.h"
+
+#define QMK_NS qmkts2
+#define QMK_MAX_SEQ 1
+#define QMK_TC_BUILD 1
+#define QMK_TC_SEQS 2
+#define QMK_NSLOTS 18
+#define QMK_SLOT_BYTES 8832
+#define QMK_EMPTY_UNITS 12
+#include "megakernel_device.cuh"
+#include "megakernel_fused.cuh"
+#include "megakernel_tc.cuh"
+#include "megakernel_tc_multi.cuh"
+#include "megakernel_tc.h"
+
+namespace qmk_fused_tc {
+const Build &build_f16_seqs2() {
+  static const Build b = {reinterpret_cast<const void *>(qmkts2::qwen3_decode_megakernel_tc_seqs), qmkts2::TC_SMEM_BYTES, qmkts2::TC_MIN_CTAS,
+                          qmkts2::TC_MAX_CTAS, qmkts2::CH_ROWS};
+  return b;
+}
+}  // namespace qmk_fused_tc

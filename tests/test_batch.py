@@ -166,3 +166,39 @@ def test_bad_arguments_are_refused(C, tiny_cfg):
                          base.num_layers, 64, base._attn_scale)
     # still healthy
     assert len(eng.generate_ids([[1, 2, 3], [4, 5]], 3)[0]) == 3
+
+
+@pytest.mark.parametrize("fmt,ctas,lens", [("fp16", 0, [1]), ("fp16", 0, [513, 2]), ("fp16", 96, [40, 1500]), ("fp16", 112, [17, 1500, 16, 2]),
+                                           ("fp16", 0, [130, 1, 900]), ("fp8", 0, [1500, 15]), ("fp8", 112, [18, 1, 700, 256]),
+                                           ("fp16", 100, [6, 300, 9])])
+def test_tensor_core_launch_matches_group_launch(C, fmt, ctas, lens):
+    """All sequences as columns of one MMA against the launch with a group of warps per sequence (``set_fused(1)``) and the
+    oracle: one to four sequences (three leave columns idle), the smallest grids of either build and one below (both runs
+    then take the group launch, behind prompts whose prefill the switch does not touch), contexts without old rows, around
+    a 16-row cache chunk, and with every split.  Same precision, other summation order: the bound of the single-sequence
+    kernels' comparison (1e-3)."""
+    import quantize as Q
+    vocab, steps, rows = 4104, 18, 1536
+    w = S.make_weights(seed=29, num_layers=3, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    eng_w, ora_w = Q.quantize_weights_fp8(w) if fmt == "fp8" else (w, w)
+    prompts = [S.make_prompt(L, seed=200 + i, vocab_size=vocab) for i, L in enumerate(lens)]
+    want, logits = _oracle(ora_w, rows, prompts, steps)
+    dumps = []
+    try:
+        C.configure(max_ctas=ctas)
+        eng = _batch_engine(eng_w, len(lens), rows, weight_format=fmt)
+        for fused in (2, 1, 2):
+            C.set_fused(fused=fused)
+            got, dump = _run_with_dump(C, eng, prompts, steps, vocab)
+            assert got == want, fused
+            dumps.append(dump)
+    finally:
+        C.set_fused(fused=2)
+        C.configure(max_ctas=0)
+        C.set_weight_format("fp16")
+    diff = float((dumps[0] - dumps[1]).abs().max())
+    err = [max(float((d[b] - logits[b]).abs().max()) for b in range(len(lens))) for d in dumps]
+    print(f"{fmt} ctas {ctas} {lens}: columns vs groups {diff:.2e}; against the oracle {err[0]:.2e}, {err[1]:.2e}")
+    assert torch.equal(dumps[0], dumps[2]), "not reproducible run to run"
+    assert torch.equal(dumps[0], dumps[1]) == (ctas == 100)
+    assert diff < 1e-3 and max(err) < LOGIT_TOL
