@@ -47,7 +47,8 @@ constexpr int FF_ATTN = F_VEC + 2 * H;         // [<= 32]   merged attention out
 constexpr int FF_INTER = FF_ATTN + 32;         // [<= 64]   SwiGLU outputs of this CTA's gate/up rows
 constexpr int FF_SPLITW = FF_INTER + 64;       // [2][32]   weight of each split of the (at most two) heads of the slice
 constexpr int FF_COLPART = F_WPART;            // [3][1024] column partials of the three warp groups
-static_assert(FF_SPLITW + 64 <= F_VEC + I, "fused aliases exceed the activation vector");
+constexpr int FF_ATTNW = FF_SPLITW + 64;       // [2][16]   tensor-core kernel: weight of each warp's attention partial
+static_assert(FF_ATTNW + 32 <= F_VEC + I, "fused aliases exceed the activation vector");
 static_assert(3 * H <= CONS_WARPS * 2 * PART_STRIDE, "column partials exceed the attention partial area");
 static_assert(CONS_WARPS == 12, "slice_colgemv maps 12 warps to 3 row groups x 4 column blocks");
 constexpr int FUSED_MIN_CTAS = 74;             // below: a slice exceeds the aliases above / a phase exceeds the ring

@@ -106,7 +106,7 @@ struct alignas(16) TcTab {
 // single-sequence kernel has its fp32 vectors; the pitch puts the four sequences of a fragment into different banks),
 // residuals of the outputs this CTA owns, split weights of the merge, sums of squares, tokens.
 constexpr int PREV_PITCH = H + 8, RESID_PITCH = 12;
-static_assert(4 * PREV_PITCH <= FF_SPLITW, "sequences 0 and 1 fit in front of the attention's split weights");
+static_assert(4 * PREV_PITCH <= FF_SPLITW, "sequences 0 and 1 fit in front of the weight arrays");
 constexpr size_t OFF_PREV2 = OFF_TCTAB + (sizeof(TcTab) + 15) / 16 * 16;
 constexpr size_t OFF_RESID = OFF_PREV2 + (TC_SEQS > 2 ? 4 * PREV_PITCH * 4 : 0);
 constexpr size_t OFF_SPLITW = OFF_RESID + 2 * TC_SEQS * RESID_PITCH * 4;
@@ -507,7 +507,11 @@ __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __ha
   // (4) merge the warps (+ the new row).  First the 2 x 13 weights exp2(max_w - max) and the head's (max, sum), by
   // warps 0 and 1 (one head each, lane = contributing warp, lane 12 = the new row); then every (head, dim) is a
   // weighted sum of 13 independent loads (a running max + rescale per thread took 1180 cycles here).
-  float *s_scale = c.f(FF_SPLITW);                       // [2][16], free between the merges
+  // (an array of its own: the merge that follows writes its split weights without a barrier in between, and its last two
+  // warps may get there - polls included - while other warps of a CTA that is late still read these.  With one array for
+  // both, about one request in 200 right after a prefill, whose traffic leaves the first layer's instruction fetches slow,
+  // came out with a wrong first layer.)
+  float *s_scale = c.f(FF_ATTNW);                        // [2][16]
   if (c.warp < 2) {
     const int h = c.warp;
     float mw = -INFINITY, lw = 0.f;
