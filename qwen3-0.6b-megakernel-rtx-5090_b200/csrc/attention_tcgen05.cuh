@@ -268,16 +268,17 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t ts = tmem_base + 128u * static_cast<uint32_t>(p & 1);
+        // split queries: the lo products first, while the accumulator (truncated after every step) is small
 #pragma unroll
-        for (int kb = 0; kb < 2; ++kb) {                      // 64-wide halves of the head dimension, four K = 16 steps each
-          const uint64_t da = smem_desc_sw128(base + kb * (TQ * 128));
-          const uint64_t db = smem_desc_sw128(base + OFF_K + kb * (STAGES * K_HALF_BYTES) + s0 * K_HALF_BYTES);
+        for (int half = HALVES - 1; half >= 0; --half)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            mma_f16_ss(ts, da + 2u * i, db + 2u * i, (kb > 0 || i > 0) ? 1u : 0u, two ? IDESC_S2 : IDESC_S);
-            if (SPLIT) mma_f16_ss(ts, da + (Q_BYTES >> 4) + 2u * i, db + 2u * i, 1u, two ? IDESC_S2 : IDESC_S);
+          for (int kb = 0; kb < 2; ++kb) {                    // 64-wide halves of the head dimension, four K = 16 steps each
+            const uint64_t da = smem_desc_sw128(base + half * Q_BYTES + kb * (TQ * 128));
+            const uint64_t db = smem_desc_sw128(base + OFF_K + kb * (STAGES * K_HALF_BYTES) + s0 * K_HALF_BYTES);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              mma_f16_ss(ts, da + 2u * i, db + 2u * i, (half < HALVES - 1 || kb > 0 || i > 0) ? 1u : 0u, two ? IDESC_S2 : IDESC_S);
           }
-        }
         mma_commit(s_full(p & 1));
         mma_commit(k_empty(s0));             // the K slots can be refilled as soon as this product is done
         if (two) mma_commit(k_empty(s0 + 1));
@@ -297,11 +298,11 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const uint64_t dp = smem_desc_sw128(base + OFF_P + static_cast<uint32_t>(c) * (HALVES * P_BYTES));
         const uint32_t to = tmem_o0 + 128u * static_cast<uint32_t>(c);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint64_t dv = smem_desc_mn_sw128(vt + i * 16 * 128, K_HALF_BYTES);
-          mma_f16_ss(to, dp + 2u * i, dv, (n > 0 || i > 0) ? 1u : 0u, IDESC_PV);
-          if (SPLIT) mma_f16_ss(to, dp + (P_BYTES >> 4) + 2u * i, dv, 1u, IDESC_PV);
-        }
+        for (int half = HALVES - 1; half >= 0; --half)        // (split P: the lo products first, as for the scores)
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            mma_f16_ss(to, dp + static_cast<uint64_t>(half) * (P_BYTES >> 4) + 2u * i, smem_desc_mn_sw128(vt + i * 16 * 128, K_HALF_BYTES),
+                       (n > 0 || half < HALVES - 1 || i > 0) ? 1u : 0u, IDESC_PV);
         mma_commit(pv_done(c));            // O_c has taken tile j: P_c may be overwritten, O_c rescaled (or, at the end, read)
         mma_commit(v_empty(j % V_STAGES));
       }

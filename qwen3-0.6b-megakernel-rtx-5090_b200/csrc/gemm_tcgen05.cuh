@@ -31,9 +31,11 @@
 // of x (absolute floor 2^-25, the fp16 subnormals) and the products are exact.  The sums need care: the tensor core
 // TRUNCATES its fp32 accumulator after every K step, so the 128 steps of a 1024-wide row in one accumulator lose 4e-6 of
 // the result, ten times what the token-serial kernels lose (share of first-layer V rows that round to another fp16 than
-// float64's: 0.93 % against 0.09 %).  So the K blocks take turns in seven accumulators, the small lo products have an
-// eighth of their own, and the epilogue adds the eight with rounded fp32 adds: at most 12 steps each, 0.12 %.
-// All 512 TMEM columns hold 64 B rows then: tiles are 64 wide (32 + 32 for gate / up), one CTA per SM with a deep ring.
+// float64's, 109 tokens: 0.93 % against 0.093 %).  So every K block gets an accumulator of its own - the four lo products
+// first, while it is small, then the four hi products - and the epilogue warps add the finished blocks up in registers
+// with rounded fp32 adds while the next ones are multiplied (four accumulators in turn): 0.087 %.  Eight accumulators
+// that the blocks shared, added once at the end, left 0.12 % and allowed only 64-wide tiles (776 tokens: 4.9 ms, now
+// 3.9 ms).  A tile is at most 128 wide (packed weights: 64, and four more warps, since theirs expand K blocks).
 #ifndef QMK_GEMM_TCGEN05_CUH_
 #define QMK_GEMM_TCGEN05_CUH_
 
@@ -49,13 +51,13 @@ constexpr int BM = 128, BK = 64;                 // BK * 2 bytes = one 128-byte 
 // Ring depth per N-tile variant: as many stages as fit in ~192 KB (a skinny M = 128 problem is bound by the
 // latency of its K loop, so the whole K extent of a 1024-wide matrix is in flight at once).
 constexpr int stages_for(int bn, int wq = 0, int ah = 1) {
-  if (ah == 2) return wq ? 4 : 5;
+  if (ah == 2) return wq || bn == 128 ? 4 : 5;
   return wq ? (bn == 32 ? 8 : bn == 64 ? 6 : bn == 128 ? 4 : 2) : (bn == 32 ? 10 : bn == 64 ? 8 : bn == 128 ? 6 : 4);
 }
 constexpr int MAX_GROUPS = 3;   // matrices sharing one A operand that one launch can multiply (q/k/v, gate/up)
 constexpr int THREADS = 192;                     // fp16 weights: producer warp, MMA warp, four epilogue warps
 constexpr int THREADS_PACKED = 320;              // packed weights: four more warps that only expand K blocks
-constexpr int threads_for(int wq) { return wq ? THREADS_PACKED : THREADS; }
+constexpr int threads_for(int wq, int ah = 1) { return wq ? THREADS_PACKED + (ah == 2 ? 128 : 0) : THREADS; }   // split activations: four warps of their own for the sums
 constexpr uint32_t TILE_A_BYTES = BM * BK * 2;   // 16 KB
 // Packed K block of one B row: 64 e4m3 bytes, or 32 bytes of e2m1 pairs
 constexpr uint32_t raw_row_bytes(int wq) { return wq == 1 ? 64u : wq == 2 ? 32u : 0u; }
@@ -71,7 +73,7 @@ constexpr uint32_t scale_bytes_for(int bn, int wq) {
   return wq == 0 ? 0u : static_cast<uint32_t>(bn) * 4u + (wq == 2 ? static_cast<uint32_t>(bn) * BS_PITCH : 0u);
 }
 constexpr int MAX_STAGES = 16;
-constexpr uint32_t BARRIER_BYTES = 640;   // full[16], empty[16], acc_full, raw_full[16], a_full[16], TMEM address, abort flag
+constexpr uint32_t BARRIER_BYTES = 640;   // full[16], empty[16], acc_full, raw_full[16], a_full[16], TMEM address, abort flag, blk_full[4], blk_free[4]
 constexpr size_t smem_bytes_for(int bn, int wq = 0, int ah = 1) {
   return 1024 /* alignment slack */ + static_cast<size_t>(stages_for(bn, wq, ah)) * stage_bytes_for(bn, wq, ah) + BARRIER_BYTES +
          scale_bytes_for(bn, wq);
@@ -242,17 +244,8 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
       : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-template <int NR>
-__device__ __forceinline__ void add_f32(uint32_t (&r)[NR], const uint32_t (&t)[NR]) {
-#pragma unroll
-  for (int i = 0; i < NR; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(t[i]));
-}
-
-// FUSE (BN = 32 or 64): B0 is the gate matrix and B1 the up matrix of a SwiGLU MLP; the CTA keeps two accumulators
-// (gate tile in TMEM columns [0, BN), up tile in [BN, 2 BN)) and its epilogue writes fp16 silu(gate) * up to
-// groups.C[0] (reinterpreted as __half [M x N]) instead of two fp32 matrices; AH = 2: as hi and lo halves, [M x 2 N].
 template <int BN, bool FUSE = false, int WQ = 0, int AH = 1>
-__global__ void __launch_bounds__(WQ ? THREADS_PACKED : THREADS, 1)
+__global__ void __launch_bounds__(threads_for(WQ, AH), 1)
 gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b0,
                    const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ CUtensorMap map_b2,
                    const Groups groups, int M, int K, unsigned int *status, unsigned long long budget_ns,
@@ -261,8 +254,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   static_assert(!FUSE || BN <= 128, "the fused SwiGLU epilogue keeps two accumulators of at most 128 columns (one MMA of N = 256)");
   static_assert(WQ == 0 || (FUSE ? 2 * BN : BN) <= 128, "packed weights: at most 128 B rows per stage (scales live in shared memory)");
   constexpr int SB = FUSE ? 2 * BN : BN;          // B rows held per stage / accumulator columns
-  // accumulators: one, or with split activations the lo products' and seven that the K blocks take in turn
-  constexpr int NACC = AH == 2 ? 8 : 1;
+  constexpr int NACC = AH == 2 ? 4 : 1;           // accumulators: one, or with split activations four that the K blocks take in turn
   static_assert(NACC * SB <= 512, "TMEM columns");
   constexpr uint32_t RAW_ROW = raw_row_bytes(WQ);
   const int STAGES = groups.stages;
@@ -282,7 +274,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(aligned + groups.ring_bytes + 8 * (4 * MAX_STAGES + 1));
   float *s_rowscale = reinterpret_cast<float *>(aligned + groups.ring_bytes + BARRIER_BYTES);   // [SB] (WQ != 0)
   unsigned char *s_bs = reinterpret_cast<unsigned char *>(s_rowscale + SB);                // [SB][BS_PITCH] (WQ == 2)
-  static_assert(8 * (4 * MAX_STAGES + 1) + 8 <= BARRIER_BYTES, "barriers and scratch fit the bytes reserved behind the ring");
+  static_assert(8 * (4 * MAX_STAGES + 2 + 8) <= BARRIER_BYTES, "barriers and scratch fit the bytes reserved behind the ring");
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = tile * BN, m0 = blockIdx.y * BM;
@@ -295,6 +287,8 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   const uint32_t acc_full = bars + 8u * (2 * MAX_STAGES);
   auto raw_full = [&](int s) { return bars + 8u * (2 * MAX_STAGES + 1 + s); };   // packed K block landed
   auto a_full = [&](int s) { return bars + 8u * (3 * MAX_STAGES + 1 + s); };     // packed weights: the A tile landed
+  auto blk_full = [&](int a) { return bars + 8u * (4 * MAX_STAGES + 2 + a); };       // split activations: accumulator a holds a K block
+  auto blk_free = [&](int a) { return bars + 8u * (4 * MAX_STAGES + 2 + 4 + a); };   // ... and has been read
   // What the producer's copies of one stage signal.  fp16 weights: A and B complete `full` together.  Packed weights:
   // the packed K block completes `raw_full`, on which the expanding warps wait before they arrive on `full`
   // themselves (one warp per stage), and the A tile completes `a_full` - on its own barrier, because B does not
@@ -322,6 +316,8 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       if (WQ) { bar_init(raw_full(s), 1); bar_init(a_full(s), 1); }
     }
     bar_init(acc_full, 1);
+    if (AH == 2)
+      for (int a = 0; a < NACC; ++a) { bar_init(blk_full(a), 1); bar_init(blk_free(a), 4); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     // B is a weight matrix: its first tiles are requested before the wait for the preceding kernel (whose output is
@@ -406,7 +402,8 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       for (int kb = 0; kb < kblocks && ok; ++kb) {
         const int s = kb % STAGES;
         ok = bar_wait(full(s), (kb / STAGES) & 1, abort_flag, status, budget_ns) &&
-             (!WQ || bar_wait(a_full(s), (kb / STAGES) & 1, abort_flag, status, budget_ns));
+             (!WQ || bar_wait(a_full(s), (kb / STAGES) & 1, abort_flag, status, budget_ns)) &&
+             (AH == 1 || kb < NACC || bar_wait(blk_free(kb % NACC), (kb / NACC - 1) & 1, abort_flag, status, budget_ns));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint64_t da = smem_desc_sw128(base + s * STAGE_BYTES);
@@ -415,22 +412,22 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         for (int j = 0; j < BK / 16; ++j) {  // 16 halves = 32 bytes = 2 descriptor address units per K step
           // FUSE: the up tile follows the gate tile in shared memory (BN more rows of the same 8-row-group layout),
           // so one MMA of N = 2 BN covers both and leaves gate in columns [0, BN), up in [BN, 2 BN)
-          const uint32_t later = (kb > 0 || j > 0) ? 1u : 0u;
-          if (AH == 2) {
-            mma_f16_ss(tmem_base, da + (TILE_A_BYTES >> 4) + 2u * j, db + 2u * j, later, idesc_for(SB));
-            mma_f16_ss(tmem_base + (1 + kb % (NACC > 1 ? NACC - 1 : 1)) * SB, da + 2u * j, db + 2u * j, (kb >= NACC - 1 || j > 0) ? 1u : 0u, idesc_for(SB));
-          } else {
-            mma_f16_ss(tmem_base, da + 2u * j, db + 2u * j, later, idesc_for(SB));
-          }
+          if (AH == 1) mma_f16_ss(tmem_base, da + 2u * j, db + 2u * j, (kb > 0 || j > 0) ? 1u : 0u, idesc_for(SB));
+          else mma_f16_ss(tmem_base + (kb % NACC) * SB, da + (TILE_A_BYTES >> 4) + 2u * j, db + 2u * j, j > 0 ? 1u : 0u, idesc_for(SB));
+        }
+        if (AH == 2) {
+#pragma unroll
+          for (int j = 0; j < BK / 16; ++j) mma_f16_ss(tmem_base + (kb % NACC) * SB, da + 2u * j, db + 2u * j, 1u, idesc_for(SB));
+          mma_commit(blk_full(kb % NACC));
         }
         mma_commit(empty(s));               // the stage is free once these MMAs have read it
       }
-      if (ok) mma_commit(acc_full);         // accumulator complete
+      if (ok && AH == 1) mma_commit(acc_full);   // accumulator complete
     }
   } else {                                 // ---- warps 2..5: epilogue, each owns TMEM lanes 32 * (warp % 4) ..; packed
                                            //      weights: first they and warps 6..9 expand the K blocks
     const int quarter = warp & 3;
-    if (WQ) {
+    if (WQ && warp < 10) {
       // Eight warps expand: stage s belongs to the two warps whose (index mod 4) is s mod 4, each takes every other
       // 16-value chunk of it and arrives on `full` (count 2).  The chain wait -> load -> convert -> store -> fence ->
       // arrive is latency, so several chains run side by side; and a warp owns STAGES, not K blocks: it then meets
@@ -485,14 +482,67 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full(s)) : "memory");
       }
     }
-    if (warp < 6) {
+    if (AH == 2 && warp >= (WQ ? 10 : 2)) {
+      // ---- split activations: add the K blocks up in registers (row = TMEM lane), then the epilogue from there
+      float acc[SB];
+#pragma unroll
+      for (int i = 0; i < SB; ++i) acc[i] = 0.f;
+      const uint32_t lanes = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+      bool ok = true;
+      for (int kb = 0; kb < kblocks; ++kb) {
+        ok = __all_sync(0xffffffffu, bar_wait(blk_full(kb % NACC), (kb / NACC) & 1, abort_flag, status, budget_ns));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t blk = lanes + (kb % NACC) * SB;
+#pragma unroll
+        for (int c = 0; c < SB / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld32(blk + c * 32, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) acc[c * 32 + i] += __uint_as_float(r[i]);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(blk_free(kb % NACC)) : "memory");
+      }
+      const int row = m0 + quarter * 32 + lane;
+      if (ok && row < M) {
+        if (WQ) {
+#pragma unroll
+          for (int i = 0; i < SB; ++i) acc[i] *= s_rowscale[i];
+        }
+        if (FUSE) {
+          __half *arow = reinterpret_cast<__half *>(C) + static_cast<size_t>(row) * (2 * N) + n0;
+#pragma unroll
+          for (int c = 0; c < BN; c += 8) {
+            uint32_t hi4[4], lo4[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float g0 = acc[c + 2 * i], g1 = acc[c + 2 * i + 1];
+              const float a0 = g0 / (1.0f + expf(-g0)) * acc[SB - BN + c + 2 * i], a1 = g1 / (1.0f + expf(-g1)) * acc[SB - BN + c + 2 * i + 1];
+              const __half2 hi = __floats2half2_rn(a0, a1);
+              const __half2 lo = __floats2half2_rn(a0 - __low2float(hi), a1 - __high2float(hi));
+              hi4[i] = *reinterpret_cast<const uint32_t *>(&hi);
+              lo4[i] = *reinterpret_cast<const uint32_t *>(&lo);
+            }
+            *reinterpret_cast<uint4 *>(arow + c) = make_uint4(hi4[0], hi4[1], hi4[2], hi4[3]);
+            *reinterpret_cast<uint4 *>(arow + N + c) = make_uint4(lo4[0], lo4[1], lo4[2], lo4[3]);
+          }
+        } else {
+          float *crow = C + static_cast<size_t>(blockIdx.z) * groups.split_stride + static_cast<size_t>(row) * N + n0;
+#pragma unroll
+          for (int i = 0; i < SB; i += 4) *reinterpret_cast<float4 *>(crow + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+        }
+      }
+    }
+    if (AH == 1 && warp < 6) {
     // warp-uniform outcome: the TMEM loads below are warp-wide instructions
     const bool ok = __all_sync(0xffffffffu, bar_wait(acc_full, 0, abort_flag, status, budget_ns));
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int accs = NACC == 1 ? 1 : 1 + (kblocks < NACC - 1 ? kblocks : NACC - 1);   // accumulators in use
     if (ok && FUSE) {
       const int row = m0 + quarter * 32 + lane;
-      __half *arow = reinterpret_cast<__half *>(C) + static_cast<size_t>(row) * (AH * N) + n0;
+      __half *arow = reinterpret_cast<__half *>(C) + static_cast<size_t>(row) * N + n0;
 #pragma unroll 1
       for (int c = 0; c < BN / 16; ++c) {     // 16 columns of the gate tile and the same 16 of the up tile per pass
         uint32_t g[16], u[16];
@@ -500,16 +550,8 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         tmem_ld16(tg, g);
         tmem_ld16(tg + BN, u);
         tmem_ld_wait();
-        for (int a = 1; a < accs; ++a) {
-          uint32_t tg2[16], tu2[16];
-          tmem_ld16(tg + a * SB, tg2);
-          tmem_ld16(tg + a * SB + BN, tu2);
-          tmem_ld_wait();
-          add_f32(g, tg2);
-          add_f32(u, tu2);
-        }
         if (row < M) {
-          uint32_t packed[8], packed_lo[8];
+          uint32_t packed[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             float g0 = __uint_as_float(g[2 * i]), g1 = __uint_as_float(g[2 * i + 1]);
@@ -518,14 +560,6 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
               g0 *= s_rowscale[c * 16 + 2 * i]; g1 *= s_rowscale[c * 16 + 2 * i + 1];
               u0 *= s_rowscale[BN + c * 16 + 2 * i]; u1 *= s_rowscale[BN + c * 16 + 2 * i + 1];
             }
-            if (AH == 2) {
-              const float a0 = g0 / (1.0f + expf(-g0)) * u0, a1 = g1 / (1.0f + expf(-g1)) * u1;
-              const __half2 hi = __floats2half2_rn(a0, a1);
-              const __half2 lo = __floats2half2_rn(a0 - __low2float(hi), a1 - __high2float(hi));
-              packed[i] = *reinterpret_cast<const uint32_t *>(&hi);
-              packed_lo[i] = *reinterpret_cast<const uint32_t *>(&lo);
-              continue;
-            }
             // (hardware exp2 and reciprocal: a few ulp, far inside the fp16 rounding of the result; the exact forms
             // cost about 25 instructions per value and made this epilogue as long as a third of the K loop)
             const __half2 h = __floats2half2_rn(__fdividef(g0, 1.0f + __expf(-g0)) * u0, __fdividef(g1, 1.0f + __expf(-g1)) * u1);
@@ -533,10 +567,6 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           }
           *reinterpret_cast<uint4 *>(arow + c * 16) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
           *reinterpret_cast<uint4 *>(arow + c * 16 + 8) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-          if (AH == 2) {
-            *reinterpret_cast<uint4 *>(arow + N + c * 16) = make_uint4(packed_lo[0], packed_lo[1], packed_lo[2], packed_lo[3]);
-            *reinterpret_cast<uint4 *>(arow + N + c * 16 + 8) = make_uint4(packed_lo[4], packed_lo[5], packed_lo[6], packed_lo[7]);
-          }
         }
       }
     } else if (ok) {
@@ -553,12 +583,6 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(c * 32);
         tmem_ld32(taddr, r);
         tmem_ld_wait();
-        for (int a = 1; a < accs; ++a) {
-          uint32_t t[32];
-          tmem_ld32(taddr + a * SB, t);
-          tmem_ld_wait();
-          add_f32(r, t);
-        }
         if (row < M && f16) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {

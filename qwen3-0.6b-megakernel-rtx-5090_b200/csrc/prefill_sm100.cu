@@ -135,8 +135,7 @@ static int pick_box_n(int M, int N, int b_tiles) {
   const int sms = sm_count() * (t_ring_budget ? 2 : 1);   // CTA slots of one wave: rings sized to a budget share an SM in pairs
   int best = 0;
   long best_cost = 0;
-  // split activations: eight accumulators in 512 TMEM columns, 64 B rows per stage
-  for (int bn = (b_tiles == 2 ? 64 : 128) / t_ah; bn >= 32; bn /= 2) {
+  for (int bn = b_tiles == 2 ? 64 : 128; bn >= 32; bn /= 2) {
     const long ctas = static_cast<long>(M / qmk_gemm::BM) * (N / bn);
     const long cost = ((ctas + sms - 1) / sms) * (b_tiles * bn + 320);
     if (best == 0 || cost < best_cost) { best = bn; best_cost = cost; }
@@ -163,20 +162,22 @@ static GemmKernel gemm_kernel_wq(int bn, bool fuse) {
   return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, false, WQ>
                   : bn == 64 ? qmk_gemm::gemm_f16_tn_kernel<64, false, WQ> : qmk_gemm::gemm_f16_tn_kernel<128, false, WQ>;
 }
-// Split activations: at most 64 B rows per stage.
-template <int WQ>
-static GemmKernel gemm_kernel_split(int bn, bool fuse) {
-  if (fuse) return qmk_gemm::gemm_f16_tn_kernel<32, true, WQ, 2>;
-  return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, false, WQ, 2> : qmk_gemm::gemm_f16_tn_kernel<64, false, WQ, 2>;
+// Split activations: at most 128 B rows per stage, packed 64.
+static GemmKernel gemm_kernel_split(int bn, bool fuse, int wq) {
+  if (wq == 0 && bn == (fuse ? 64 : 128)) return fuse ? qmk_gemm::gemm_f16_tn_kernel<64, true, 0, 2> : qmk_gemm::gemm_f16_tn_kernel<128, false, 0, 2>;
+  if (fuse) return wq == 0 ? qmk_gemm::gemm_f16_tn_kernel<32, true, 0, 2> : qmk_gemm::gemm_f16_tn_kernel<32, true, 1, 2>;
+  if (bn == 32) return wq == 0 ? qmk_gemm::gemm_f16_tn_kernel<32, false, 0, 2> : qmk_gemm::gemm_f16_tn_kernel<32, false, 1, 2>;
+  return wq == 0 ? qmk_gemm::gemm_f16_tn_kernel<64, false, 0, 2> : qmk_gemm::gemm_f16_tn_kernel<64, false, 1, 2>;
 }
+static int split_max_rows(int wq) { return wq == 0 ? 128 : 64; }
 static bool box_n_ok(int box_n, bool fuse, int wq) {
   const int rows = fuse ? 2 * box_n : box_n;
-  if (t_ah == 2) return wq < 2 && (box_n == 32 || (box_n == 64 && rows == 64));
+  if (t_ah == 2) return wq < 2 && (box_n == 32 || box_n == 64 || box_n == 128) && rows <= split_max_rows(wq);
   return box_n == 32 || box_n == 64 || (box_n == 128 && (rows == 128 || wq == 0)) || (box_n == 256 && rows == 256 && wq == 0);
 }
 // (the widest tiles - 256 B rows per stage - exist for fp16 weights only; split activations for fp16 and FP8 weights)
 static GemmKernel gemm_kernel(int bn, bool fuse, int wq, int ah) {
-  if (ah == 2) return wq == 0 ? gemm_kernel_split<0>(bn, fuse) : gemm_kernel_split<1>(bn, fuse);
+  if (ah == 2) return gemm_kernel_split(bn, fuse, wq);
   if (wq == 0 && fuse && bn == 128) return qmk_gemm::gemm_f16_tn_kernel<128, true>;
   if (wq == 0 && !fuse && bn == 256) return qmk_gemm::gemm_f16_tn_kernel<256, false>;
   return wq == 0 ? gemm_kernel_wq<0>(bn, fuse) : wq == 1 ? gemm_kernel_wq<1>(bn, fuse) : gemm_kernel_wq<2>(bn, fuse);
@@ -193,7 +194,7 @@ int ensure_gemm_attrs(std::string *err) {
     for (int ah = 1; ah < 3 && e == cudaSuccess; ++ah)
       for (int wq = 0; wq < 4 - ah && e == cudaSuccess; ++wq)
         for (int fuse = 0; fuse < 2 && e == cudaSuccess; ++fuse)
-          for (int bn = 32; bn <= (ah == 2 ? (fuse ? 32 : 64) : (fuse ? 64 : 128) * (wq == 0 ? 2 : 1)) && e == cudaSuccess; bn *= 2)
+          for (int bn = 32; bn <= (ah == 2 ? split_max_rows(wq) / (fuse ? 2 : 1) : (fuse ? 64 : 128) * (wq == 0 ? 2 : 1)) && e == cudaSuccess; bn *= 2)
             e = cudaFuncSetAttribute(reinterpret_cast<const void *>(gemm_kernel(bn, fuse != 0, wq, ah)),
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gemm_smem(bn, fuse != 0, wq, ah)));
     if (e == cudaSuccess)
@@ -297,7 +298,7 @@ int launch_gemm_grouped(const CUtensorMap &map_a, int ngroups, const CUtensorMap
   int rows = live_rows > 0 ? live_rows : M;   // rows the epilogue stores (the rest of the tile is padding)
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
   const size_t smem = set_ring(&gr, box_n, wq);
-  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah), grid, dim3(qmk_gemm::threads_for(wq)), smem, stream,
+  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah), grid, dim3(qmk_gemm::threads_for(wq, t_ah)), smem, stream,
                                 map_a, b0, b1, b2, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
   return QMK_OK;
@@ -329,7 +330,7 @@ int launch_gemm_swiglu(const CUtensorMap &map_a, const CUtensorMap &map_gate, co
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
   const size_t smem = set_ring(&gr, 2 * box_n, wq);
-  cudaError_t e = launch_kernel(gemm_kernel(box_n, true, wq, t_ah), dim3(N / box_n, M / qmk_gemm::BM), dim3(qmk_gemm::threads_for(wq)),
+  cudaError_t e = launch_kernel(gemm_kernel(box_n, true, wq, t_ah), dim3(N / box_n, M / qmk_gemm::BM), dim3(qmk_gemm::threads_for(wq, t_ah)),
                                 smem, stream, map_a, map_gate, map_up, map_up, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
   return QMK_OK;
@@ -360,7 +361,7 @@ int launch_gemm_splitk(const CUtensorMap &map_a, const CUtensorMap &map_b, float
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
   const size_t smem = set_ring(&gr, box_n, wq);
-  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah), dim3(N / box_n, M / qmk_gemm::BM, splits), dim3(qmk_gemm::threads_for(wq)),
+  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah), dim3(N / box_n, M / qmk_gemm::BM, splits), dim3(qmk_gemm::threads_for(wq, t_ah)),
                                 smem, stream, map_a, map_b, map_b, map_b, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
   return QMK_OK;
@@ -626,6 +627,8 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
   };
   static const int rec_slot[7] = {1, 2, 3, 6, 8, 9, 10};   // q, k, v, o, gate, up, down inside a layer record
   auto wptr = [&](int l, int j) { return reinterpret_cast<const void *>(rec[static_cast<size_t>(l) * 12 + rec_slot[j]]); };
+  // packed weights with split activations take narrower tiles
+  auto split_box = [&](int box_n, int widest) { return split && wq != 0 && box_n > widest ? widest : box_n; };
   // several matrices against the same activations in one launch (q/k/v)
   auto gemm_group = [&](const CUtensorMap &a, int l, int n, const int *js, float *const *cs, const int *ns, int M, int K,
                         int live) {
@@ -635,7 +638,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     // flop than 128-wide ones - these GEMMs are bound by the L2 -> shared-memory feed).  Measured on the q/k/v shape at
     // 2048 rows: 28.8 -> 26.5 us.
     const int box_n = (wq == 0 && !split && M >= 1024 && total / 256 * (M / qmk_gemm::BM) >= qmk_tc::gemm_sm_count()) ? 256
-                                                                                                           : qmk_tc::gemm_box_n(M, total);
+                                                                                                           : split_box(qmk_tc::gemm_box_n(M, total), 64);
     const CUtensorMap *maps[3];
     const void *raws[3] = {nullptr, nullptr, nullptr};
     for (int i = 0; i < n; ++i) { maps[i] = &wmap_for(l, js[i], box_n); raws[i] = wptr(l, js[i]); }
@@ -666,11 +669,11 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
                                           256, live, 0, wq, wptr(l, j));
       }
       if (od_splits == 1) {
-        const int box_n = qmk_tc::gemm_box_n(Mrows, H);
+        const int box_n = split_box(qmk_tc::gemm_box_n(Mrows, H), 64);
         return qmk_tc::launch_gemm(a, wmap_for(l, j, box_n), c, Mrows, H, K, box_n, w.status, env.timeout_ms, stream, &err, live, 0, wq,
                                    wptr(l, j));
       }
-      const int box_n = split ? 64 : 128;
+      const int box_n = split_box(128, 64);
       return qmk_tc::launch_gemm_splitk(a, wmap_for(l, j, box_n), c, Mrows, H, K, od_splits, w.status, env.timeout_ms, stream, &err, box_n,
                                         live, 0, wq, wptr(l, j));
     };
@@ -758,7 +761,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
       if (rc != QMK_OK) break;
       PF_CUDA(norm_rows(w.o, reinterpret_cast<const __half *>(r[7])));
       {
-        const int box_gu = qmk_tc::gemm_box_n_fused(M, I);
+        const int box_gu = split_box(qmk_tc::gemm_box_n_fused(M, I), 32);
         // three of these CTAs per SM instead of two: their epilogue (two TMEM reads, SiLU, fp16 pack) is the long part
         qmk_tc::RingBudgetScope gu_scope(split ? 0 : M >= 1024 ? GATE_UP_RING_BYTES : PREFILL_RING_BYTES);
         {
