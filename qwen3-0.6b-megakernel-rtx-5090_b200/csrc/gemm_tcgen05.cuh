@@ -189,6 +189,9 @@ struct Groups {
   // (NVFP4) and of the fp32 scale (the trailer) inside a row.
   const unsigned char *braw[MAX_GROUPS];
   uint32_t raw_pitch, raw_bs_off, raw_scale_off;
+  // fp16 B matrices that hold the values of packed rows (expand_packed_rows): fp32 scale of every B row, multiplied into
+  // the accumulator like the scales of packed rows (null = none; FUSE: [0] gate, [1] up).  Single fp16 activations only.
+  const float *row_scale[MAX_GROUPS] = {nullptr, nullptr, nullptr};
   // Ring geometry (ring_geometry()): stages and bytes from the ring's start to the barriers.
   int stages;
   uint32_t ring_bytes;
@@ -559,6 +562,10 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             if (WQ) {
               g0 *= s_rowscale[c * 16 + 2 * i]; g1 *= s_rowscale[c * 16 + 2 * i + 1];
               u0 *= s_rowscale[BN + c * 16 + 2 * i]; u1 *= s_rowscale[BN + c * 16 + 2 * i + 1];
+            } else if (groups.row_scale[0]) {
+              const float2 sg = __ldg(reinterpret_cast<const float2 *>(groups.row_scale[0] + n0 + c * 16) + i);
+              const float2 su = __ldg(reinterpret_cast<const float2 *>(groups.row_scale[1] + n0 + c * 16) + i);
+              g0 *= sg.x; g1 *= sg.y; u0 *= su.x; u1 *= su.y;
             }
             // (hardware exp2 and reciprocal: a few ulp, far inside the fp16 rounding of the result; the exact forms
             // cost about 25 instructions per value and made this epilogue as long as a third of the K loop)
@@ -575,6 +582,8 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       __half *hrow = reinterpret_cast<__half *>(C) + static_cast<size_t>(row) * N + n0;   // (out_f16)
       const bool pick = groups.amax_val != nullptr;
       const bool f16 = groups.out_f16 != 0;
+      const float *rscale = grp == 0 ? groups.row_scale[0] : grp == 1 ? groups.row_scale[1] : groups.row_scale[2];
+      if (rscale) rscale += n0;
       float best = -INFINITY;
       int best_col = 0x7fffffff;
 #pragma unroll 1
@@ -583,6 +592,16 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(c * 32);
         tmem_ld32(taddr, r);
         tmem_ld_wait();
+        if (!WQ && rscale) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            const float4 sc = __ldg(reinterpret_cast<const float4 *>(rscale + c * 32 + i));
+            r[i] = __float_as_uint(__uint_as_float(r[i]) * sc.x);
+            r[i + 1] = __float_as_uint(__uint_as_float(r[i + 1]) * sc.y);
+            r[i + 2] = __float_as_uint(__uint_as_float(r[i + 2]) * sc.z);
+            r[i + 3] = __float_as_uint(__uint_as_float(r[i + 3]) * sc.w);
+          }
+        }
         if (row < M && f16) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
@@ -629,6 +648,65 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+  }
+}
+
+// Values of packed rows as fp16 matrices [rows][K] (exact: e4m3, and e2m1 x e4m3 block scale, have at most six
+// significant bits) and their fp32 row scales, for up to seven matrices in one launch: a warp per row, a lane per 16
+// values.  Bound by writing the fp16 bytes (31.5 MB a layer).
+struct ExpandArgs {
+  const unsigned char *src[7];
+  __half *dst[7];
+  float *scale[7];
+  int first_row[8];             // rows before matrix j among all rows; [7] = all rows
+  int K[7];
+  uint32_t pitch[7], bs_off[7], scale_off[7];
+};
+constexpr int EXPAND_THREADS = 256;
+template <int WQ>
+__global__ void __launch_bounds__(EXPAND_THREADS) expand_packed_rows(const __grid_constant__ ExpandArgs a) {
+  const int row = blockIdx.x * (EXPAND_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= a.first_row[7]) return;
+  const unsigned char *src = nullptr;
+  __half *dst = nullptr;
+  float *scale = nullptr;
+  int K = 0;
+  uint32_t bs = 0, so = 0;
+#pragma unroll
+  for (int j = 0; j < 7; ++j)   // (compile-time indices: a run-time index would copy the parameter to local memory)
+    if (row >= a.first_row[j] && row < a.first_row[j + 1]) {
+      const size_t r = static_cast<size_t>(row - a.first_row[j]);
+      K = a.K[j]; bs = a.bs_off[j]; so = a.scale_off[j];
+      src = a.src[j] + r * a.pitch[j];
+      dst = a.dst[j] + r * static_cast<size_t>(K);
+      scale = a.scale[j] + r;
+    }
+  if (lane == 0) *scale = *reinterpret_cast<const float *>(src + so);
+  for (int i = lane; i < K / 16; i += 32) {
+    uint32_t h[8];
+    if (WQ == 1) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(src) + i);
+      h[0] = e4m3x2_to_half2_bits(v.x); h[1] = e4m3x2_to_half2_bits(v.x >> 16);
+      h[2] = e4m3x2_to_half2_bits(v.y); h[3] = e4m3x2_to_half2_bits(v.y >> 16);
+      h[4] = e4m3x2_to_half2_bits(v.z); h[5] = e4m3x2_to_half2_bits(v.z >> 16);
+      h[6] = e4m3x2_to_half2_bits(v.w); h[7] = e4m3x2_to_half2_bits(v.w >> 16);
+    } else {
+      const uint2 v = __ldg(reinterpret_cast<const uint2 *>(src) + i);
+      const uint32_t sb2 = e4m3x2_to_half2_bits(__ldg(src + bs + i));   // low half = the block's scale
+      const __half2 sc = __half2half2(__ushort_as_half(static_cast<unsigned short>(sb2 & 0xFFFFu)));
+      uint32_t lo[4], hi[4];
+      e2m1x8_to_half2x4(v.x, lo);
+      e2m1x8_to_half2x4(v.y, hi);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const __half2 p = __hmul2(*reinterpret_cast<const __half2 *>(&lo[k]), sc), q = __hmul2(*reinterpret_cast<const __half2 *>(&hi[k]), sc);
+        h[k] = *reinterpret_cast<const uint32_t *>(&p);
+        h[4 + k] = *reinterpret_cast<const uint32_t *>(&q);
+      }
+    }
+    uint4 *out = reinterpret_cast<uint4 *>(dst + static_cast<size_t>(i) * 16);
+    out[0] = make_uint4(h[0], h[1], h[2], h[3]);
+    out[1] = make_uint4(h[4], h[5], h[6], h[7]);
   }
 }
 

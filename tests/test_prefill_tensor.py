@@ -175,3 +175,31 @@ def test_refusals(C):
         eng.prefill_ids([1, 600])
     eng.reset()
     assert len(eng.generate_ids([1, 2, 3], 2)) == 2
+
+
+@pytest.mark.parametrize("fmt,n", [("fp8", 257), ("fp8", 385), ("nvfp4", 300), ("nvfp4", 1100), ("fp8", 4200)])
+def test_packed_weights_expanded_once_per_layer(C, fmt, n):
+    """Chunks of 384 and more (padded) rows expand a packed layer's matrices once instead of inside the GEMMs: the shortest
+    such chunk (257 tokens), ragged ones, a length with the wide tiles and split K, two chunks of which the second is
+    short.  The products are the same (exact values, row scale behind the sum), so the first layer's rows equal bit for bit
+    those of calls that stay below the switch; from 1024 rows on the RMSNorm kernel adds its squares in another order, which
+    moves single operands to the neighbouring fp16 (2^-11 of one of 1024 products): one unit in the last place of a row's
+    value, 2^-8 below 8.  Later layers to the rounding of other tiles and splits, like every two passes of this path (1e-2)."""
+    import quantize as Q
+    vocab, L = 2048, 4224
+    w = S.make_weights(seed=33, num_layers=2, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    eng_w, _ = (Q.quantize_weights_fp8 if fmt == "fp8" else Q.quantize_weights_nvfp4)(w)
+    ids = S.make_prompt(n, seed=n, vocab_size=vocab)
+    try:
+        a = _engine(eng_w, L, "tensor", weight_format=fmt)
+        b = _engine(eng_w, L, "tensor", weight_format=fmt)
+        a.prefill_ids(ids)
+        for i in range(0, n, 250):
+            b.prefill_ids(ids[i:i + 250])
+    finally:
+        C.set_weight_format("fp16")
+    for x, y in ((a._k_cache[:, :, :n], b._k_cache[:, :, :n]), (a._v_cache[:, :, :n], b._v_cache[:, :, :n])):
+        first, diff = float((x[0].float() - y[0].float()).abs().max()), float((x.float() - y.float()).abs().max())
+        print(f"{fmt} {n}: max difference {diff:.2e}, first layer {first:.2e}")
+        assert first <= (2.0 ** -8 if n >= 1024 else 0.0) and float(x[0].abs().max()) < 8.0
+        assert diff < 1e-2
