@@ -508,9 +508,7 @@ __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __ha
   // warps 0 and 1 (one head each, lane = contributing warp, lane 12 = the new row); then every (head, dim) is a
   // weighted sum of 13 independent loads (a running max + rescale per thread took 1180 cycles here).
   // (an array of its own: the merge that follows writes its split weights without a barrier in between, and its last two
-  // warps may get there - polls included - while other warps of a CTA that is late still read these.  With one array for
-  // both, about one request in 200 right after a prefill, whose traffic leaves the first layer's instruction fetches slow,
-  // came out with a wrong first layer.)
+  // warps may get there while other warps of a CTA that is late still read these)
   float *s_scale = c.f(FF_ATTNW);                        // [2][16]
   if (c.warp < 2) {
     const int h = c.warp;
@@ -535,7 +533,9 @@ __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __ha
   cons_sync();
   if (c.tid < 2 * D) {
     const int h = c.tid >> 7, d = c.tid & (D - 1);
-    float A = s_vnew[d] * s_scale[h * 16 + CONS_WARPS];   // 0 weight unless this CTA owns the new row
+    // (not a zero weight: on a CTA that does not own the new row s_vnew holds what an earlier kernel left in shared memory,
+    // and 0 x NaN is NaN - which the integer sums then took for 0, a wrong first layer after some prefills)
+    float A = owner ? s_vnew[d] * s_scale[h * 16 + CONS_WARPS] : 0.f;
 #pragma unroll
     for (int w = 0; w < CONS_WARPS; ++w) A = fmaf(s_wpart[(w * 2 + h) * PART_STRIDE + d], s_scale[h * 16 + w], A);
     ll_store(tc_ll(P, c) + LL_PART + static_cast<size_t>((2 * g + h) * MAX_SPLITS + s) * PART_STRIDE + d, A, tag);
