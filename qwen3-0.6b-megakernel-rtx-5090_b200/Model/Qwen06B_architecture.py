@@ -353,7 +353,7 @@ class BatchDecoder:
         """``engine``: "persistent" (one megakernel launch, <= 4 sequences, fp32 activations), "gemm" (tcgen05
         GEMMs per step, <= 128 sequences, fp16 GEMM operands; packed FP8 / NVFP4 matrices are expanded inside the
         GEMMs) or "auto": persistent up to 4 sequences, gemm above (NVFP4: always gemm) - measured at 1024-token
-        contexts, us per step: 2 sequences 642 persistent, 4 sequences 930 against 1130 (FP8 rows 868 against 1275)."""
+        contexts, us per step: 2 sequences 613 persistent, 4 sequences 812 against 1130 (FP8 rows 805 against 1275)."""
         n = int(num_sequences)
         if engine == "auto":
             engine = "persistent" if n <= self.MAX_SEQUENCES and decoder_kw.get("weight_format", "fp16") != "nvfp4" else "gemm"

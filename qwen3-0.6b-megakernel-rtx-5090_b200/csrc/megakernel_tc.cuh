@@ -227,6 +227,11 @@ __device__ __forceinline__ void tile_task(const Params &P, const Ctx &c, uint32_
 // than the MMAs).  Phase rows = `groups` runs of `nch` consecutive chunks (q|k|v: one run; gate/up: the gate rows'
 // chunks, then the up rows'); tiles of 16 rows; when there are fewer tiles than warps, nkb warps share a tile's
 // 1024 inputs.  Grids of at least FUSED_MIN_CTAS CTAs have at most 6 tiles per phase: one task per warp.
+// fp16 rows: the tiles run on from the gate into the up rows (148 CTAs: 40 to 48 rows are three tiles, where the gate and
+// the up rows by themselves were two each, the second of them half empty; the MMAs of a sub-partition issue one at a time):
+// 523 / 535 / 568 -> 518 / 531 / 563 us per token at 64 / 1024 / 4096-token contexts.  fp8 rows gained nothing at 1024 and
+// lost 1 % at 64 and stay apart (their row conversions weigh more than the MMAs).
+constexpr bool GU_ONE_RUN = !FP8_ROWS;
 __device__ inline void build_tile_tasks(TileTask *tasks, int *nkb_out, int groups, int nch) {
   const int tpg = (nch + TILE_CH - 1) / TILE_CH, T = groups * tpg;
   const int nkb = T >= CONS_WARPS ? 1 : CONS_WARPS / T;   // 12, 6, 4, 3, 2, 2, 1: divides EMPTY_UNITS
@@ -243,6 +248,8 @@ __device__ inline void build_tile_tasks(TileTask *tasks, int *nkb_out, int group
     t.pad0 = t.pad1 = 0;
   }
 }
+// Row of the gate/up phase's tiles that holds the up row of gate row r.
+__device__ __forceinline__ int up_row(int nch, int r) { return r + (GU_ONE_RUN ? nch * CH_ROWS : (nch + TILE_CH - 1) / TILE_CH * 16); }
 __device__ __forceinline__ void run_tile_task(const Params &P, const Ctx &c, const TileTask *tasks, int fslot) {
   const int4 a = reinterpret_cast<const int4 *>(tasks + c.warp)[0], b = reinterpret_cast<const int4 *>(tasks + c.warp)[1];
   // a = {active, first, valid, p0}, b = {p1, units, -, -}
@@ -280,12 +287,12 @@ __device__ __noinline__ uint32_t gateup_phase(const Params &P, Ctx c) {
   QMK_FINE(12);
   cons_sync();
   if (c.tid < nch * CH_ROWS) {
-    const int r = c.tid, tpg = (nch + TILE_CH - 1) / TILE_CH;
+    const int r = c.tid, ru = up_row(nch, r);
     const float *pg = tc_part(c) + (r >> 4) * nkb * 16 + (r & 15);
-    const float *pu = pg + tpg * nkb * 16;
+    const float *pu = tc_part(c) + (ru >> 4) * nkb * 16 + (ru & 15);
     float g = 0.f, u = 0.f;
 #pragma unroll
-    for (int kb = 0; kb < CONS_WARPS / 2; ++kb)
+    for (int kb = 0; kb < CONS_WARPS; ++kb)
       if (kb < nkb) { g += pg[kb * 16]; u += pu[kb * 16]; }
     const float a = g / (1.0f + expf(-g)) * u;
     c.f(FF_INTER)[r] = a;
@@ -993,7 +1000,7 @@ __device__ __forceinline__ void tc_setup(const Params &P, const Ctx &c) {
     split_rows(GU_CHUNKS, c.ncta, c.cta, a, b); tt->g0 = a; tt->ng = b - a;
     split_rows(P.vocab / CH_ROWS, c.ncta, c.cta, a, b); tt->lm0 = a; tt->nlm = b - a;
     build_tile_tasks(tt->qkv, &tt->nkb_qkv, 1, tt->nq);
-    build_tile_tasks(tt->gu, &tt->nkb_gu, 2, tt->ng);
+    build_tile_tasks(tt->gu, &tt->nkb_gu, GU_ONE_RUN ? 1 : 2, GU_ONE_RUN ? 2 * tt->ng : tt->ng);
   }
   {
     const unsigned long long *src = reinterpret_cast<const unsigned long long *>(P.layers);

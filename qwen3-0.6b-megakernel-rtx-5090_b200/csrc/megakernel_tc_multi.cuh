@@ -9,8 +9,8 @@
 // words read back, cache rows.
 // The launch it replaces (megakernel_batch.cuh, which stays for grids outside this kernel's range) gives each sequence a
 // group of warps that convert and multiply every weight for themselves, and has six hand-overs per layer.
-// Measured, us per step at 64 / 1024 / 2048-token contexts: two fp16 sequences 616 / 642 / 673, three 803 / 896 / 964, four
-// 812 / 930 / 1031, four with FP8 rows 797 / 868 / 977 (the group launch: two 1137 / 1317 at 64 / 1024; four 1655 / 1942;
+// Measured, us per step at 64 / 1024 / 2048-token contexts: two fp16 sequences 581 / 613 / 635, three 683 / 750 / 847, four
+// 712 / 812 / 928, four with FP8 rows 730 / 805 / 909 (the group launch: two 1137 / 1317 at 64 / 1024; four 1655 / 1942;
 // the GEMM step: four fp16 1086 / 1130 / 1196, four FP8 1224 / 1275 / 1341, with fp16-rounded activations).  Distance from
 // float64 as before: 0.68 % of layer 1's V rows that two sequences decode round differently (0.70 % with the group launch).
 
@@ -60,12 +60,12 @@ __device__ __noinline__ uint32_t gateup_phase_seqs(const Params &P, Ctx c) {
   const int b = c.tid / TPS, r = c.tid % TPS;
   __half *act16 = reinterpret_cast<__half *>(c.smem + OFF_ACT16) + 2 * b * ACT16_PITCH;
   if (r < nch * CH_ROWS) {
-    const int tpg = (nch + TILE_CH - 1) / TILE_CH;
+    const int ru = up_row(nch, r);
     const float *pg = tc_part(c) + (r >> 4) * nkb * PART_TASK + b * 16 + (r & 15);
-    const float *pu = pg + tpg * nkb * PART_TASK;
+    const float *pu = tc_part(c) + (ru >> 4) * nkb * PART_TASK + b * 16 + (ru & 15);
     float g = 0.f, u = 0.f;
 #pragma unroll
-    for (int kb = 0; kb < CONS_WARPS / 2; ++kb)
+    for (int kb = 0; kb < CONS_WARPS; ++kb)
       if (kb < nkb) { g += pg[kb * PART_TASK]; u += pu[kb * PART_TASK]; }
     const float a = g / (1.0f + expf(-g)) * u;
     act16[r] = split_half(a, false);
@@ -96,6 +96,11 @@ __device__ __noinline__ void merge_seqs(const Params &P, const Ctx c, int step, 
     const int e = min(e0 + c.warp + q * CONS_WARPS, e1 - 1);
     wp[q] = area + static_cast<size_t>((e >> 7) * MAX_SPLITS + s) * PART_STRIDE + (e & (D - 1));
     if (mine && e0 + c.warp + q * CONS_WARPS < e1) valid |= 1u << q;
+  }
+  {   // one lane per warp watches the last split's word of the last sequence first (see merge_slice)
+    const int Sl = max(1, min((per_seq(P.start_positions, P.nseq - 1) + step) / max(1, P.split_len), tctab(c)->s_cap));
+    const int e = min(e0 + c.warp, e1 - 1);
+    ll_sentinel(P, c, P.ll + static_cast<size_t>(P.nseq - 1) * LL_WORDS + LL_PART + static_cast<size_t>((e >> 7) * MAX_SPLITS + Sl - 1) * PART_STRIDE + (e & (D - 1)), tag);
   }
   float a[NE];
   const int hw = h0 + (c.warp - (CONS_WARPS - 2));                // head whose split weights this warp makes (last two warps)
@@ -237,6 +242,10 @@ __device__ __forceinline__ void normalise_seqs(const Ctx &c, const float (&v)[TC
   cons_sync();
 }
 
+// Contributions that may still be missing from the watched word when a warp goes on to fetch all its words: with several
+// sequences the adds drain for longer, and the fetch's round trip fits into the rest of it (four sequences, us per step at
+// 64 / 1024 / 2048 tokens: 0: 812 / 932 / 1034, 16: 771 / 896 / 981, 48: 725 / 844 / 953, with the watch in front of the merge 712 / 812 / 928; 147: no better).  One sequence gains nothing.
+constexpr unsigned long long SUM_SLACK = 48;
 // red_wait_norm for all sequences: which = 0: x1, 1: x2 (kept as the residual of the next layer's O slice, x).
 __device__ __noinline__ void red_wait_norm_seqs(const Params &P, const Ctx c, int which, uint32_t use, const __half *norm_w) {
   const unsigned long long base = static_cast<unsigned long long>(use) * static_cast<unsigned long long>(c.ncta);
@@ -244,7 +253,7 @@ __device__ __noinline__ void red_wait_norm_seqs(const Params &P, const Ctx c, in
   if (c.lane == 0) {   // one lane per warp watches one word (see red_wait_norm)
     const unsigned long long *p = src + static_cast<size_t>(P.nseq - 1) * H;
     uint32_t n = 0;
-    while (((ll_load(p) - base) & RED_CNT_MASK) != 0ull) {
+    while (((base - ll_load(p)) & RED_CNT_MASK) > SUM_SLACK) {
       if ((++n & 1023u) == 0u && (c.flags()[0] || ld_relaxed_u32(P.status) != 0u)) break;   // the full wait below reports time-outs
       if (n > (1u << 22)) break;
     }
