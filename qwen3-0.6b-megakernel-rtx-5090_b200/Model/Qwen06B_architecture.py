@@ -171,9 +171,10 @@ class Decoder:
         if weight_format not in ("fp16", "fp8", "nvfp4"):
             raise ValueError("weight_format must be 'fp16', 'fp8' or 'nvfp4'")
         self.weight_format = weight_format
-        # "serial": the reference's token-by-token prefill (fp32 activations, bit-identical to decoding the
-        # prompt); "tensor": chunked prefill on the tensor cores (fp16 GEMM operands; packed matrices are expanded
-        # inside the GEMMs)
+        # "serial": the prefill op (fp32 activations: prompts of up to three tokens token by token, longer ones in one
+        # pass with every operand split into two fp16 halves, equal to decoding the prompt up to rounding);
+        # "tensor": chunked prefill on the tensor cores (fp16 GEMM operands; packed matrices are expanded inside the
+        # GEMMs or, for long chunks, once per layer)
         if prefill_mode not in ("serial", "tensor"):
             raise ValueError("prefill_mode must be 'serial' or 'tensor'")
         if prefill_mode == "serial" and weight_format == "nvfp4":

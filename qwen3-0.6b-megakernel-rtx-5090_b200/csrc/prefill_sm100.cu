@@ -752,8 +752,8 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     // tail of the kernel before them (every kernel here lasts 2-6 us longer than its CTAs run; 2048 tokens 4.11 -> 3.81
     // ms).  The row kernels and the attention kernel launch plainly: with EVERY kernel of this chain launched as a
     // programmatic dependent, a decode launched after the prefill had returned produced run-to-run different logits
-    // although every cache row compared bit-identical afterwards - unexplained; the attribute on the GEMMs alone never
-    // showed it (128 prefill + decode cycles compared bit for bit, and the test that found it runs every time).
+    // although every cache row compared bit-identical afterwards (an uninitialised read in the decode kernel, since
+    // mended: see its attention; the chain has not been measured again).
     qmk_tc::PdlScope pdl_scope(false);
     const bool pdl_gemm = env.pdl != 0;
     qmk_tc::SplitActScope split_scope(split);
