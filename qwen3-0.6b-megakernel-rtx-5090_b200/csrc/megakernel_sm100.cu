@@ -433,11 +433,8 @@ int encode_cache_maps(Engine *e, Params &P) {
   return QMK_OK;
 }
 
-// Common launch path.  `P` arrives with the per-call fields set; `batch` selects the multi-sequence
-// build (per-sequence entries filled by the caller) instead of the single-sequence kernel.
-int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool batch = false) {
-  if (P.num_steps <= 0) return QMK_OK;
-  if (!batch) mirror_sequence0(P);
+// What every call with filled per-call fields has to satisfy before anything is launched.
+int check_call(Engine *e, const Params &P) {
   if (!P.embed || !P.layers || (!P.prefill && (!P.final_norm || !P.lm_head)))
     return fail(e, QMK_ERR_BAD_ARGUMENT, "null weight or cache pointer");
   if (!aligned16(P.embed) || !aligned16(P.layers) || (P.lm_head && !aligned16(P.lm_head)))
@@ -456,7 +453,17 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
   if (e->wfmt == 2)
     return fail(e, QMK_ERR_BAD_ARGUMENT,
                 "NVFP4 rows are read by the tensor-core entry points only (qmk_prefill_chunked, qmk_decode_batched)");
-  int rc = ensure_ready(e);
+  return QMK_OK;
+}
+
+// Common launch path.  `P` arrives with the per-call fields set; `batch` selects the multi-sequence
+// build (per-sequence entries filled by the caller) instead of the single-sequence kernel.
+int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool batch = false) {
+  if (P.num_steps <= 0) return QMK_OK;
+  if (!batch) mirror_sequence0(P);
+  int rc = check_call(e, P);
+  if (rc != QMK_OK) return rc;
+  rc = ensure_ready(e);
   if (rc != QMK_OK) return rc;
 
   // Tags are (sequence number * 64 + layer); restart the sequence before it can wrap.
@@ -863,11 +870,18 @@ int prefill_unlocked(const int *token_ids_host, int num_tokens, const void *embe
   for (int i = 0; i < num_tokens; ++i)
     if (token_ids_host[i] < 0 || token_ids_host[i] >= e->vocab)
       return fail(e, QMK_ERR_BAD_TOKEN, "prompt token outside [0, vocab)");
+  Params P = base_params(embed_weight, layer_weights, final_norm_weight, nullptr, cos_table, sin_table, k_cache, v_cache,
+                         num_layers, start_position, max_seq_len, attn_scale);
+  P.prefill = 1;
+  P.num_steps = num_tokens;
+  mirror_sequence0(P);
+  const int rc = check_call(e, P);   // (both routes: the chunked pass by itself does not look at the alignment of the embedding)
+  if (rc != QMK_OK) return rc;
   // Prompts of more than a few tokens go through the chunked tensor-core pass with split activations (hi + lo fp16 halves of
   // every fp32 operand: the precision of the kernels below) instead of one persistent step per token: a pass over up to
   // a few hundred tokens takes 1.3-1.5 ms, a step without its LM head 0.42 ms.  31 tokens 13.0 -> 1.2 ms, 776 tokens
   // 349 -> 3.9 ms.
-  if (num_tokens >= SPLIT_PREFILL_MIN_TOKENS && e->wfmt != 2)
+  if (num_tokens >= SPLIT_PREFILL_MIN_TOKENS)
     return qmk_tc::prefill_split(token_ids_host, num_tokens, embed_weight, layer_weights, cos_table, sin_table, k_cache, v_cache,
                                  num_layers, start_position, max_seq_len, attn_scale, stream);
   if (num_tokens > e->tok_cap) {  // grow-only staging, as the reference keeps (megakernel_5090.cu:1303-1307)
@@ -880,10 +894,6 @@ int prefill_unlocked(const int *token_ids_host, int num_tokens, const void *embe
     e->tok_cap = cap;
   }
   QMK_CUDA(e, cudaMemcpyAsync(e->tok_dev, token_ids_host, sizeof(int) * num_tokens, cudaMemcpyHostToDevice, stream));
-  Params P = base_params(embed_weight, layer_weights, final_norm_weight, nullptr, cos_table, sin_table, k_cache, v_cache,
-                         num_layers, start_position, max_seq_len, attn_scale);
-  P.prefill = 1;
-  P.num_steps = num_tokens;
   P.token_ids = e->tok_dev;
   return launch(e, P, stream, true);
 }

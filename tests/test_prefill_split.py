@@ -48,3 +48,24 @@ def test_rows_match_fp32_oracle(built_library, fmt, calls):
         assert bool((diff[0] <= ulp[0]).all()) and bool((diff <= 2 * ulp).all())
         assert float(diff[0].square().mean().sqrt()) < 6e-5 and float(diff.square().mean().sqrt()) < 3.4e-4
     assert torch.count_nonzero(eng._k_cache[:, :, n:]) == 0
+
+
+@pytest.mark.parametrize("n", [2, 12])
+def test_misaligned_pointers_are_refused(built_library, n):
+    """The op's pointer rules hold on both of its routes (few tokens: persistent steps; more: the chunked pass, whose
+    row kernels read the embedding 16 bytes at a time)."""
+    from Model.Qwen06B_architecture import Decoder
+    w = S.make_weights(seed=1, num_layers=2, vocab_size=512, max_seq_len=16)
+    eng = Decoder(weights=S.weights_to(w, "cuda"), verbose=False, max_seq_len=32)
+    good = list(eng._common())
+
+    def shifted(t):
+        return torch.zeros(t.numel() + 8, dtype=t.dtype, device="cuda")[1:1 + t.numel()].view(t.shape)
+    ids = torch.arange(n, dtype=torch.int32)
+    for at in (0, 6, 7):      # embedding, K cache, V cache
+        args = list(good)
+        args[at] = shifted(good[at])
+        with pytest.raises(RuntimeError, match="16-byte aligned"):
+            eng._prefill_op(ids, *args, eng.num_layers, 0, eng.max_seq_len, eng._attn_scale)
+    eng.prefill_ids(ids.tolist())
+    assert torch.count_nonzero(eng._k_cache[:, :, :n]) > 0
