@@ -448,31 +448,37 @@ std::mutex g_ws_decode_mu;
       return qmk_internal::report(QMK_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(err__)); \
   } while (0)
 
-// `rows`: activation rows the buffers hold (CHUNK for prefill, one 128-row tile for the batched decode)
-int ensure_workspace(Workspace &w, int rows) {
+// `rows`: activation rows the buffers hold (CHUNK for prefill, one 128-row tile for the batched decode).  All or nothing:
+// buffers that were made are given back when a later one does not fit.  `no_room`: set (and nothing reported) where the
+// reason is memory, for callers with another way.
+int ensure_workspace(Workspace &w, int rows, bool *no_room = nullptr) {
   if (w.ready) return QMK_OK;
   using namespace qmk_pf;
   const size_t C = static_cast<size_t>(rows);
-  PF_CUDA(cudaMalloc(&w.tokens, sizeof(int) * C));
-  PF_CUDA(cudaMalloc(&w.x, sizeof(float) * C * H));
-  PF_CUDA(cudaMalloc(&w.q, sizeof(float) * C * QS));
-  PF_CUDA(cudaMalloc(&w.k, sizeof(float) * C * KVS));
-  PF_CUDA(cudaMalloc(&w.v, sizeof(float) * C * KVS));
-  PF_CUDA(cudaMalloc(&w.qr, sizeof(float) * C * QS));
-  PF_CUDA(cudaMalloc(&w.o, sizeof(float) * 2 * C * H));      // (two split-K partial matrices of a prefill chunk)
-  PF_CUDA(cudaMalloc(&w.down, sizeof(float) * 2 * C * H));
-  // (room for the hi and lo halves of split activations, [C][2 x width])
-  PF_CUDA(cudaMalloc(&w.xn, sizeof(__half) * C * 2 * H));
-  PF_CUDA(cudaMalloc(&w.attn, sizeof(__half) * C * 2 * QS));
-  PF_CUDA(cudaMalloc(&w.act, sizeof(__half) * C * 2 * I));
-  PF_CUDA(cudaMalloc(&w.status, 16));
+  struct Buffer { void **at; size_t bytes; };
+  const Buffer buffers[] = {
+      {reinterpret_cast<void **>(&w.tokens), sizeof(int) * C},
+      {reinterpret_cast<void **>(&w.x), sizeof(float) * C * H},
+      {reinterpret_cast<void **>(&w.q), sizeof(float) * C * QS},
+      {reinterpret_cast<void **>(&w.k), sizeof(float) * C * KVS},
+      {reinterpret_cast<void **>(&w.v), sizeof(float) * C * KVS},
+      {reinterpret_cast<void **>(&w.qr), sizeof(float) * C * QS},
+      {reinterpret_cast<void **>(&w.o), sizeof(float) * 2 * C * H},      // (two split-K partial matrices of a prefill chunk)
+      {reinterpret_cast<void **>(&w.down), sizeof(float) * 2 * C * H},
+      // (room for the hi and lo halves of split activations, [C][2 x width])
+      {reinterpret_cast<void **>(&w.xn), sizeof(__half) * C * 2 * H},
+      {reinterpret_cast<void **>(&w.attn), sizeof(__half) * C * 2 * QS},
+      {reinterpret_cast<void **>(&w.act), sizeof(__half) * C * 2 * I},
+      {reinterpret_cast<void **>(&w.status), 16}};
+  cudaError_t e = cudaSuccess;
   // GEMM operand rows beyond a short chunk are read (and ignored): they must hold finite numbers
-  PF_CUDA(cudaMemset(w.xn, 0, sizeof(__half) * C * 2 * H));
-  PF_CUDA(cudaMemset(w.attn, 0, sizeof(__half) * C * 2 * QS));
-  PF_CUDA(cudaMemset(w.act, 0, sizeof(__half) * C * 2 * I));
-  PF_CUDA(cudaMemset(w.qr, 0, sizeof(float) * C * QS));
+  for (const Buffer &b : buffers)
+    if (e == cudaSuccess && (e = cudaMalloc(b.at, b.bytes)) == cudaSuccess) e = cudaMemset(*b.at, 0, b.bytes);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);   // (a caller's stream may not wait for the legacy one)
   std::string err;
-  int rc = qmk_tc::make_map_f16(&w.map_xn, w.xn, C, H, qmk_gemm::BM, &err);
+  int rc = e == cudaSuccess ? QMK_OK : QMK_ERR_CUDA;
+  if (rc != QMK_OK) err = std::string("workspace of the tensor-core path: ") + cudaGetErrorString(e);
+  if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_xn, w.xn, C, H, qmk_gemm::BM, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_attn, w.attn, C, QS, qmk_gemm::BM, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_act, w.act, C, I, qmk_gemm::BM, &err);
   // the rotated queries as fp16 (the first half of the fp32 buffer), read by the attention kernel in 128-row boxes
@@ -482,7 +488,13 @@ int ensure_workspace(Workspace &w, int rows) {
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_attn2, w.attn, C, 2 * QS, qmk_gemm::BM, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_act2, w.act, C, 2 * I, qmk_gemm::BM, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_qh2, w.qr, C, 2 * QS, qmk_gemm::BM, &err);
-  if (rc != QMK_OK) return qmk_internal::report(rc, err);
+  if (rc != QMK_OK) {
+    for (const Buffer &b : buffers)
+      if (*b.at) { cudaFree(*b.at); *b.at = nullptr; }
+    cudaGetLastError();
+    if (no_room && e == cudaErrorMemoryAllocation) { *no_room = true; return rc; }
+    return qmk_internal::report(rc, err);
+  }
   w.ready = true;
   return QMK_OK;
 }
@@ -563,7 +575,8 @@ constexpr size_t PK_ROWS_OFF = 0, PK_ITEMS_OFF = 32768, PK_MAPS_OFF = 49152, PK_
 
 int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_weight, const LDGLayerWeight *layer_weights,
                  const void *cos_table, const void *sin_table, void *k_cache, void *v_cache, int num_layers,
-                 int start_position, int max_seq_len, float attn_scale, cudaStream_t stream, const PackedSeqs *pk, bool split) {
+                 int start_position, int max_seq_len, float attn_scale, cudaStream_t stream, const PackedSeqs *pk, bool split,
+                 bool *no_room = nullptr) {
   using namespace qmk_pf;
   if (num_tokens <= 0) return QMK_OK;
   qmk_internal::PrefillEnv env;
@@ -600,7 +613,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
   if (dev < 0 || dev >= 16) return qmk_internal::report(QMK_ERR_CUDA, "device index out of range");
   std::lock_guard<std::recursive_mutex> lock(g_ws_mu);
   Workspace &w = g_ws[dev];
-  rc = ensure_workspace(w, CHUNK);
+  rc = ensure_workspace(w, CHUNK, no_room);
   if (rc == QMK_OK) rc = ensure_weight_maps(w, layer_weights, num_layers, wq, stream);
   if (rc != QMK_OK) return rc;
   // ---- packed prompts: rows = the sequences one after the other, each padded to whole 128-row tiles
@@ -887,13 +900,14 @@ extern "C" int qmk_prefill_chunked(const int *token_ids_host, int num_tokens, co
 namespace qmk_tc {
 // The chunked pass with split activations, for qmk_prefill (fp32 activations at the precision of the token-serial kernels).
 // Locks: the caller takes prefill_lock() BEFORE the engine's lock and holds both - the order in which every other path
-// meets them (prefill_impl reports errors to the engine while it holds the workspace).
+// meets them (prefill_impl reports errors to the engine while it holds the workspace).  `no_room`: set, with nothing
+// launched or reported, where the workspace does not fit in memory.
 std::unique_lock<std::recursive_mutex> prefill_lock() { return std::unique_lock<std::recursive_mutex>(g_ws_mu); }
 int prefill_split(const int *token_ids_host, int num_tokens, const void *embed_weight, const LDGLayerWeight *layer_weights,
                   const void *cos_table, const void *sin_table, void *k_cache, void *v_cache, int num_layers, int start_position,
-                  int max_seq_len, float attn_scale, cudaStream_t stream) {
+                  int max_seq_len, float attn_scale, cudaStream_t stream, bool *no_room) {
   return prefill_impl(token_ids_host, num_tokens, embed_weight, layer_weights, cos_table, sin_table, k_cache, v_cache, num_layers,
-                      start_position, max_seq_len, attn_scale, stream, nullptr, true);
+                      start_position, max_seq_len, attn_scale, stream, nullptr, true, no_room);
 }
 }  // namespace qmk_tc
 

@@ -69,3 +69,49 @@ def test_misaligned_pointers_are_refused(built_library, n):
             eng._prefill_op(ids, *args, eng.num_layers, 0, eng.max_seq_len, eng._attn_scale)
     eng.prefill_ids(ids.tolist())
     assert torch.count_nonzero(eng._k_cache[:, :, :n]) > 0
+
+
+FULL_DEVICE = r"""
+import json, sys
+sys.path[:0] = [{root!r}, {pkg!r}]
+import torch
+import synthetic as S
+from Model.Qwen06B_architecture import Decoder
+w = S.make_weights(seed=3, num_layers=2, vocab_size=4096, norm_std=0.1, max_seq_len=16)
+eng = Decoder(weights=S.weights_to(w, "cuda"), verbose=False, max_seq_len=64)
+steps = [eng.step(t) for t in {ids!r}[:-1]]              # token by token: exchange words and K-major copies exist now
+rows = eng._k_cache[:, :, :eng.position].clone()
+eng._k_cache.zero_(); eng._v_cache.zero_(); eng.reset()
+torch.cuda.synchronize()
+ballast = torch.empty(torch.cuda.mem_get_info()[0] - (160 << 20), dtype=torch.uint8, device="cuda")
+free = []
+for _ in range(3):
+    tokens = eng.generate_ids({ids!r}, 6)
+    torch.cuda.synchronize()
+    free.append(torch.cuda.mem_get_info()[0])
+same = bool(torch.equal(rows, eng._k_cache[:, :, :rows.shape[2]]))
+del ballast
+torch.cuda.empty_cache()
+print(json.dumps(dict(tokens=tokens, free=free, same=same, again=eng.generate_ids({ids!r}, 6))))
+"""
+
+
+def test_prompt_is_prefilled_step_by_step_where_the_workspace_does_not_fit(built_library):
+    """A process whose device memory is given away (160 MB left; the chunked pass wants 285 MB): prompts go through the
+    persistent steps, bit for bit as decoded token by token, no call keeps memory, and once there is room again the
+    chunked pass gives the same tokens."""
+    import json
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    pkg = os.path.join(root, "qwen3-0.6b-megakernel-rtx-5090_b200")
+    ids = S.make_prompt(12, seed=5, vocab_size=4096)
+    want = OracleDecoder(S.make_weights(seed=3, num_layers=2, vocab_size=4096, norm_std=0.1, max_seq_len=16),
+                         max_seq_len=64).generate_ids(ids, 6)[0]
+    proc = subprocess.run([sys.executable, "-c", FULL_DEVICE.format(root=root, pkg=pkg, ids=ids)], capture_output=True, text=True,
+                          timeout=600)
+    assert proc.returncode == 0, proc.stdout[-2000:] + proc.stderr[-4000:]
+    res = json.loads(proc.stdout.strip().splitlines()[-1])
+    assert res["tokens"] == want and res["again"] == want and res["same"]
+    assert res["free"][0] == res["free"][-1] and res["free"][0] > 100 << 20
