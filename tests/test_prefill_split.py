@@ -115,3 +115,28 @@ def test_prompt_is_prefilled_step_by_step_where_the_workspace_does_not_fit(built
     res = json.loads(proc.stdout.strip().splitlines()[-1])
     assert res["tokens"] == want and res["again"] == want and res["same"]
     assert res["free"][0] == res["free"][-1] and res["free"][0] > 100 << 20
+
+
+def test_unfused_switch_covers_the_prefill_op(built_library):
+    """``set_fused(0)`` is the unfused kernel for every op: a prompt prefilled under it leaves the rows that decoding it
+    token by token leaves, bit for bit."""
+    import qwen_megakernel_C as C
+    from Model.Qwen06B_architecture import Decoder
+    w = S.make_weights(seed=9, num_layers=2, vocab_size=512, norm_std=0.1, max_seq_len=16)
+    ids = S.make_prompt(40, seed=2, vocab_size=512)
+    eng = Decoder(weights=S.weights_to(w, "cuda"), verbose=False, max_seq_len=64)
+    rows = []
+    try:
+        for fused in (0, 2):
+            C.set_fused(fused=fused)
+            eng.reset()
+            eng.prefill_ids(ids)
+            rows.append((eng._k_cache.clone(), eng._v_cache.clone()))
+            eng.reset()
+            for t in ids:
+                eng.step(t)
+            if fused == 0:
+                assert torch.equal(rows[-1][0], eng._k_cache) and torch.equal(rows[-1][1], eng._v_cache)
+    finally:
+        C.set_fused(fused=2)
+    assert float((rows[0][0].float() - rows[1][0].float()).abs().max()) < 8e-3
