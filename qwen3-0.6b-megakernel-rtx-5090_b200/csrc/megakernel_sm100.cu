@@ -858,6 +858,10 @@ int qmk_generate_batch(int num_sequences, const int *first_token_ids, const int 
 
 namespace {
 constexpr int SPLIT_PREFILL_MIN_TOKENS = 4;
+// A prompt that may take the chunked pass locks that pass's workspace, before the engine; a shorter one does not wait for it.
+std::unique_lock<std::recursive_mutex> chunked_pass_lock(int num_tokens) {
+  return num_tokens >= SPLIT_PREFILL_MIN_TOKENS ? qmk_tc::prefill_lock() : std::unique_lock<std::recursive_mutex>();
+}
 int prefill_unlocked(const int *token_ids_host, int num_tokens, const void *embed_weight,
                      const LDGLayerWeight *layer_weights, const void *final_norm_weight, const void *cos_table,
                      const void *sin_table, void *k_cache, void *v_cache, int num_layers, int start_position,
@@ -954,7 +958,7 @@ int qmk_prefill(const int *token_ids_host, int num_tokens, const void *embed_wei
                 const LDGLayerWeight *layer_weights, const void *final_norm_weight, const void *cos_table,
                 const void *sin_table, void *k_cache, void *v_cache, int num_layers, int start_position,
                 int max_seq_len, float attn_scale, cudaStream_t stream) {
-  auto workspace = qmk_tc::prefill_lock();
+  const auto workspace = chunked_pass_lock(num_tokens);
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   return prefill_unlocked(token_ids_host, num_tokens, embed_weight, layer_weights, final_norm_weight, cos_table, sin_table,
                           k_cache, v_cache, num_layers, start_position, max_seq_len, attn_scale, stream);
@@ -1045,7 +1049,7 @@ int qmk_engine_prefill(qmk_engine *h, const int *token_ids_host, int num_tokens,
                        const LDGLayerWeight *layer_weights, const void *final_norm_weight, const void *cos_table,
                        const void *sin_table, void *k_cache, void *v_cache, int num_layers, int start_position,
                        int max_seq_len, float attn_scale, cudaStream_t stream) {
-  auto workspace = qmk_tc::prefill_lock();
+  const auto workspace = chunked_pass_lock(num_tokens);
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   const int rc = apply_handle_unlocked(h, layer_weights);
   if (rc != QMK_OK) return rc;

@@ -140,3 +140,43 @@ def test_unfused_switch_covers_the_prefill_op(built_library):
     finally:
         C.set_fused(fused=2)
     assert float((rows[0][0].float() - rows[1][0].float()).abs().max()) < 8e-3
+
+
+def test_short_prompts_do_not_wait_for_a_chunked_pass(built_library):
+    """The workspace of the chunked pass is held for a whole pass (some 20 ms here).  A call of the op that does not use it -
+    measured on one that is refused before any GPU work - returns meanwhile."""
+    import threading
+    import time
+    from Model.Qwen06B_architecture import Decoder
+    w = S.weights_to(S.make_weights(seed=9, num_layers=28, vocab_size=512, max_seq_len=16), "cuda")
+    long = Decoder(weights=w, verbose=False, max_seq_len=8192, prefill_mode="tensor")
+    short = Decoder(weights=w, verbose=False, max_seq_len=64)
+    ids = S.make_prompt(8191, seed=1, vocab_size=512)
+    passes, stop = [], threading.Event()
+
+    def prefill():
+        with torch.cuda.stream(torch.cuda.Stream()):
+            while not stop.is_set():
+                t0 = time.perf_counter()
+                long.reset()
+                long.prefill_ids(ids)
+                passes.append(time.perf_counter() - t0)
+    short.prefill_ids([1, 2])
+    thread = threading.Thread(target=prefill)
+    thread.start()
+    try:
+        while len(passes) < 2:
+            time.sleep(0.005)
+        waits = []
+        for _ in range(40):
+            t0 = time.perf_counter()
+            with pytest.raises(RuntimeError, match="vocab"):
+                short.prefill_ids([600])
+            waits.append(time.perf_counter() - t0)
+            time.sleep(0.003)
+    finally:
+        stop.set()
+        thread.join()
+    waits.sort()
+    print(f"pass {sorted(passes)[len(passes) // 2] * 1e3:.1f} ms, refused short call {waits[20] * 1e3:.3f} / {waits[-1] * 1e3:.3f} ms")
+    assert waits[20] < 0.1 * sorted(passes)[len(passes) // 2]
