@@ -35,7 +35,17 @@ constexpr unsigned long long RED_CNT_MASK = (1ull << RED_CNT_BITS) - 1ull;
 constexpr float RED_SCALE = 268435456.0f;             // 2^28
 constexpr float RED_INV_SCALE = 1.0f / 268435456.0f;
 constexpr int RED_MAX_COPIES = 2;
-constexpr int RED_BUF_STRIDE = RED_MAX_COPIES * H;    // words of one sum: [copy][1024]
+// Eight words (64 bytes) to a 128-byte line.  Which L2 slice serves a line is a hash of its address, and a slice adds the
+// 148 contributions to its lines one after the other: with full lines, 64 for a sum, a layer waited for whichever slice
+// had drawn three or four of them, and that depended on where the allocation fell (36 places, us per token at 64 tokens of
+// context: 497 to 535, median 502; 4096 tokens 545 at the best).  128 half lines spread better: 491 to 498, median 494;
+// 535.  Quarter lines cost more requests per warp than they spread (495 to 497; 539), eighths more still (512).
+constexpr int RED_GROUP = 8, RED_LINE = 16;
+__device__ __forceinline__ constexpr int red_index(int n) { return n / RED_GROUP * RED_LINE + n % RED_GROUP; }   // word of output n
+constexpr int RED_SUM_WORDS = H / RED_GROUP * RED_LINE;
+constexpr int RED_STEP = CONS_THREADS / RED_GROUP * RED_LINE;   // from output n to n + CONS_THREADS
+static_assert(CONS_THREADS % RED_GROUP == 0 && H % RED_GROUP == 0, "RED_STEP, whole lines");
+constexpr int RED_BUF_STRIDE = RED_MAX_COPIES * RED_SUM_WORDS;    // words of one sum: [copy][1024 outputs]
 constexpr int RED_X1 = 0, RED_X2 = RED_BUF_STRIDE;
 constexpr int RED_WORDS = 2 * RED_BUF_STRIDE;
 static_assert(MAX_CTAS < (1 << RED_CNT_BITS), "the contribution count of one use must fit the count field");
@@ -83,11 +93,11 @@ __device__ __noinline__ float red_wait_vec(const Params &P, const Ctx c, int whi
 #pragma unroll 1
   for (int r = 0; r < R; ++r) {
     const unsigned long long base = static_cast<unsigned long long>(use) * red_contributors(c.ncta, R, r);
-    const unsigned long long *src = buf + r * H + c.tid;
+    const unsigned long long *src = buf + r * RED_SUM_WORDS + red_index(c.tid);
     unsigned long long w[PT];
 #pragma unroll
     for (int j = 0; j < PT; ++j)
-      if (valid & (1u << j)) w[j] = ll_load(src + j * CONS_THREADS);
+      if (valid & (1u << j)) w[j] = ll_load(src + j * RED_STEP);
     uint32_t pending = valid;
     unsigned long long t0 = 0;
     uint32_t it = 0;
@@ -99,7 +109,7 @@ __device__ __noinline__ float red_wait_vec(const Params &P, const Ctx c, int whi
       if (P.spin_sleep_ns) __nanosleep(P.spin_sleep_ns);
 #pragma unroll
       for (int j = 0; j < PT; ++j)
-        if (pending & (1u << j)) w[j] = ll_load(src + j * CONS_THREADS);
+        if (pending & (1u << j)) w[j] = ll_load(src + j * RED_STEP);
       if ((++it & 255u) == 0u) {
         if (c.flags()[0]) break;
         if (ld_relaxed_u32(P.status) != 0u) { c.flags()[0] = 1; break; }
@@ -189,7 +199,7 @@ __device__ __noinline__ uint32_t slice_colgemv(const Params &P, Ctx c, int which
   cons_sync();
   QMK_FINE(fb + 2);
   const int n0 = t->n0, n1 = t->n1;
-  unsigned long long *mine = buf + (c.cta % P.red_copies) * H;
+  unsigned long long *mine = buf + (c.cta % P.red_copies) * RED_SUM_WORDS;
 #pragma unroll
   for (int j = 0; j < (H + CONS_THREADS - 1) / CONS_THREADS; ++j) {
     const int n = c.tid + j * CONS_THREADS;
@@ -198,7 +208,7 @@ __device__ __noinline__ uint32_t slice_colgemv(const Params &P, Ctx c, int which
       if (n >= n0 && n < n1) v += resid[n];
       const long long fx = __float2ll_rn(v * RED_SCALE), fx_prev = __float2ll_rn(prev[n] * RED_SCALE);
       prev[n] = v;
-      red_add_u64(mine + n, (static_cast<unsigned long long>(fx - fx_prev) << RED_CNT_BITS) + 1ull);
+      red_add_u64(mine + red_index(n), (static_cast<unsigned long long>(fx - fx_prev) << RED_CNT_BITS) + 1ull);
     }
   }
   QMK_FINE(fb + 3);

@@ -258,8 +258,8 @@ size_t exchange_bytes() {
   return words * sizeof(unsigned long long);
 }
 
-// Residual sums: [x1, x2][accumulator copy][1024] of one sequence, or [x1, x2][sequence][1024].
-constexpr size_t RED_ALLOC_WORDS = 2 * qmkp::MAX_SEQ * qmk::H;
+// Residual sums: [x1, x2][accumulator copy] of one sequence, or [x1, x2][sequence].
+constexpr size_t RED_ALLOC_WORDS = 2 * qmkp::MAX_SEQ * qmk::RED_SUM_WORDS;
 static_assert(RED_ALLOC_WORDS >= qmk::RED_WORDS, "one allocation serves both layouts");
 
 int ensure_ready(Engine *e) {

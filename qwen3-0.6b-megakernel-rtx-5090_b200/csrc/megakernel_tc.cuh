@@ -614,7 +614,7 @@ __device__ __noinline__ void red_wait_norm(const Params &P, const Ctx c, int whi
 #pragma unroll 1
   for (int r = 0; r < R; ++r) {
     const unsigned long long base = static_cast<unsigned long long>(use) * red_contributors(c.ncta, R, r);
-    const unsigned long long *src = buf + r * H + c.tid;
+    const unsigned long long *src = buf + r * RED_SUM_WORDS + red_index(c.tid);
     {
       // one lane per warp watches one word until it is complete, then the warp fetches its words: 32x fewer polls
       // hitting the lines the adds are draining into, at the price of one more L2 round trip at the end (measured at
@@ -631,7 +631,7 @@ __device__ __noinline__ void red_wait_norm(const Params &P, const Ctx c, int whi
     unsigned long long w[PT];
 #pragma unroll
     for (int j = 0; j < PT; ++j)
-      if (valid & (1u << j)) w[j] = ll_load(src + j * CONS_THREADS);
+      if (valid & (1u << j)) w[j] = ll_load(src + j * RED_STEP);
     uint32_t pending = valid;
     unsigned long long t0 = 0;
     uint32_t it = 0;
@@ -643,7 +643,7 @@ __device__ __noinline__ void red_wait_norm(const Params &P, const Ctx c, int whi
       if (P.spin_sleep_ns) __nanosleep(P.spin_sleep_ns);
 #pragma unroll
       for (int j = 0; j < PT; ++j)
-        if (pending & (1u << j)) w[j] = ll_load(src + j * CONS_THREADS);
+        if (pending & (1u << j)) w[j] = ll_load(src + j * RED_STEP);
       if ((++it & 255u) == 0u) {
         if (c.flags()[0]) break;
         if (ld_relaxed_u32(P.status) != 0u) { c.flags()[0] = 1; break; }
@@ -765,7 +765,7 @@ __device__ __noinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
   const int nrows = which ? tctab(c)->ng * CH_ROWS : t->e1 - t->e0;
   const float *resid = c.f(which ? F_X1 : F_X);
   float *prev = c.f(FF_PREV) + (which ? H : 0);
-  unsigned long long *mine = P.red + (which ? RED_X2 : RED_X1) + (c.cta % P.red_copies) * H;
+  unsigned long long *mine = P.red + (which ? RED_X2 : RED_X1) + (c.cta % P.red_copies) * RED_SUM_WORDS;
   const int nch = (nrows + CH_ROWS - 1) / CH_ROWS + SCALE_CH;
   [[maybe_unused]] const float *scales = FP8_ROWS ? reinterpret_cast<const float *>(c.slot(c.chunk + static_cast<uint32_t>(nch - 1))) : nullptr;
   const bool two = nrows > 16;
@@ -805,7 +805,7 @@ __device__ __noinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
         if (n >= n0 && n < n1) v += resid[n];
         const long long fx = __float2ll_rn(v * RED_SCALE), fx_prev = __float2ll_rn(prev[n] * RED_SCALE);
         prev[n] = v;
-        red_add_u64(mine + n, (static_cast<unsigned long long>(fx - fx_prev) << RED_CNT_BITS) + 1ull);
+        red_add_u64(mine + red_index(n), (static_cast<unsigned long long>(fx - fx_prev) << RED_CNT_BITS) + 1ull);
       }
     }
   }

@@ -173,7 +173,7 @@ __device__ __noinline__ uint32_t slice_cols_seqs(const Params &P, Ctx c, int whi
     const int n0 = t->n0, n1 = t->n1;
     const float *resid = tc_resid(c, which ^ 1, live ? b : 0);   // O slice: x, down slice: x1
     float *prev = tc_prev(c, which, live ? b : 0);
-    unsigned long long *sum = P.red + (which * TC_SEQS + (live ? b : 0)) * H;
+    unsigned long long *sum = P.red + (which * TC_SEQS + (live ? b : 0)) * RED_SUM_WORDS;
 #pragma unroll 1
     for (int t0 = c.warp; t0 < H / 16; t0 += 2 * CONS_WARPS) {
       float acc[2][4];
@@ -190,7 +190,7 @@ __device__ __noinline__ uint32_t slice_cols_seqs(const Params &P, Ctx c, int whi
             if (n >= n0 && n < n1) v += resid[n - n0];
             const long long fx = __float2ll_rn(v * RED_SCALE), fx_prev = __float2ll_rn(prev[n] * RED_SCALE);
             prev[n] = v;
-            red_add_u64(sum + n, (static_cast<unsigned long long>(fx - fx_prev) << RED_CNT_BITS) + 1ull);
+            red_add_u64(sum + red_index(n), (static_cast<unsigned long long>(fx - fx_prev) << RED_CNT_BITS) + 1ull);
           }
         }
       }
@@ -249,9 +249,9 @@ constexpr unsigned long long SUM_SLACK = 48;
 // red_wait_norm for all sequences: which = 0: x1, 1: x2 (kept as the residual of the next layer's O slice, x).
 __device__ __noinline__ void red_wait_norm_seqs(const Params &P, const Ctx c, int which, uint32_t use, const __half *norm_w) {
   const unsigned long long base = static_cast<unsigned long long>(use) * static_cast<unsigned long long>(c.ncta);
-  const unsigned long long *src = P.red + static_cast<size_t>(which) * TC_SEQS * H + c.tid;
+  const unsigned long long *src = P.red + static_cast<size_t>(which) * TC_SEQS * RED_SUM_WORDS + red_index(c.tid);
   if (c.lane == 0) {   // one lane per warp watches one word (see red_wait_norm)
-    const unsigned long long *p = src + static_cast<size_t>(P.nseq - 1) * H;
+    const unsigned long long *p = src + static_cast<size_t>(P.nseq - 1) * RED_SUM_WORDS;
     uint32_t n = 0;
     while (((base - ll_load(p)) & RED_CNT_MASK) > SUM_SLACK) {
       if ((++n & 1023u) == 0u && (c.flags()[0] || ld_relaxed_u32(P.status) != 0u)) break;   // the full wait below reports time-outs
@@ -267,7 +267,7 @@ __device__ __noinline__ void red_wait_norm_seqs(const Params &P, const Ctx c, in
     for (int j = 0; j < VPT; ++j) {
       const int i = b * VPT + j;
       w[i] = base;
-      if (b < P.nseq && c.tid + j * CONS_THREADS < H) { valid |= 1u << i; w[i] = ll_load(src + b * H + j * CONS_THREADS); }
+      if (b < P.nseq && c.tid + j * CONS_THREADS < H) { valid |= 1u << i; w[i] = ll_load(src + b * RED_SUM_WORDS + j * RED_STEP); }
     }
   uint32_t pending = valid, it = 0;
   unsigned long long t0 = 0;
@@ -280,7 +280,7 @@ __device__ __noinline__ void red_wait_norm_seqs(const Params &P, const Ctx c, in
     for (int b = 0; b < TC_SEQS; ++b)
 #pragma unroll
       for (int j = 0; j < VPT; ++j)
-        if (pending & (1u << (b * VPT + j))) w[b * VPT + j] = ll_load(src + b * H + j * CONS_THREADS);
+        if (pending & (1u << (b * VPT + j))) w[b * VPT + j] = ll_load(src + b * RED_SUM_WORDS + j * RED_STEP);
     if ((++it & 255u) == 0u) {
       if (c.flags()[0]) break;
       if (ld_relaxed_u32(P.status) != 0u) { c.flags()[0] = 1; break; }
