@@ -154,6 +154,21 @@ __device__ __forceinline__ __half split_half(float x, bool lo) {
   const __half h = __float2half_rn(x);
   return lo ? __float2half_rn((x - __half2float(h)) * LO_SCALE) : h;
 }
+// Range: a half ends at 65504, the fp32 values do not.  Operands that may lie above are divided by a power of two first and
+// the finished sums multiplied by it (both exact; 1 for everything a usual model holds, and then nothing changes):
+//   * SwiGLU outputs: by the largest of the CTA's slice (at most 32 rows: one warp holds them all);
+//   * rotated queries: by the largest of the head;
+//   * RMS-normalised activations, which stay below 32 x |norm weight|: by 64 where a weight of the vector exceeds 2040.
+// Attention outputs need none: they are averages of fp16 cache rows.
+constexpr int M_XSCALE = 24, M_QSCALE = 26, M_ASCALE = 20;   // words of F_MISC: activations, query heads [2], SwiGLU slice [sequence]
+constexpr float NORM_W_LIMIT = 2040.0f, NORM_DOWN = 1.0f / 64.0f, NORM_UP = 64.0f;
+// Exponent k >= 0 with |v| * 2^-k < 2^15 in every lane of the warp (infinities and NaN stay what they are).
+__device__ __forceinline__ uint32_t operand_exponent(float v) {
+  const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(v) & 0x7fffffffu) >> 23;
+  return top > 141u ? top - 141u : 0u;
+}
+__device__ __forceinline__ float exp2_down(uint32_t k) { return __uint_as_float((127u - k) << 23); }
+__device__ __forceinline__ float exp2_up(uint32_t k) { return __uint_as_float((127u + k) << 23); }
 __device__ __forceinline__ uint32_t pack_half2(__half a, __half b) {
   return static_cast<uint32_t>(__half_as_ushort(a)) | (static_cast<uint32_t>(__half_as_ushort(b)) << 16);
 }
@@ -282,7 +297,7 @@ __device__ __noinline__ uint32_t qkv_phase(const Params &P, Ctx c, uint32_t tag)
 #pragma unroll
     for (int kb = 0; kb < CONS_WARPS; ++kb)
       if (kb < nkb) v += p[kb * 16];
-    ll_store(P.ll + LL_QKV + t->q0 * CH_ROWS + r, v, tag);
+    ll_store(P.ll + LL_QKV + t->q0 * CH_ROWS + r, v * c.f(F_MISC)[M_XSCALE], tag);
   }
   QMK_FINE(4);
   return c.chunk + static_cast<uint32_t>(nch);
@@ -296,23 +311,26 @@ __device__ __noinline__ uint32_t gateup_phase(const Params &P, Ctx c) {
   run_tile_task(P, c, t->gu, 10);
   QMK_FINE(12);
   cons_sync();
-  if (c.tid < nch * CH_ROWS) {
+  if (c.warp < 2) {          // warp 0 holds the slice; rows past it multiply stale bytes: zero activations
     const int r = c.tid, ru = up_row(nch, r);
-    const float *pg = tc_part(c) + (r >> 4) * nkb * 16 + (r & 15);
-    const float *pu = tc_part(c) + (ru >> 4) * nkb * 16 + (ru & 15);
-    float g = 0.f, u = 0.f;
+    float a = 0.f;
+    if (r < nch * CH_ROWS) {
+      const float *pg = tc_part(c) + (r >> 4) * nkb * 16 + (r & 15);
+      const float *pu = tc_part(c) + (ru >> 4) * nkb * 16 + (ru & 15);
+      float g = 0.f, u = 0.f;
 #pragma unroll
-    for (int kb = 0; kb < CONS_WARPS; ++kb)
-      if (kb < nkb) { g += pg[kb * 16]; u += pu[kb * 16]; }
-    const float a = g / (1.0f + expf(-g)) * u;
-    c.f(FF_INTER)[r] = a;
+      for (int kb = 0; kb < CONS_WARPS; ++kb)
+        if (kb < nkb) { g += pg[kb * 16]; u += pu[kb * 16]; }
+      const float up = c.f(F_MISC)[M_XSCALE];
+      g *= up;
+      a = g / (1.0f + expf(-g)) * (u * up);
+    }
+    const uint32_t k = operand_exponent(a);
+    if (c.tid == 0) c.f(F_MISC)[M_ASCALE] = exp2_up(k);
+    a *= exp2_down(k);
     __half *act16 = reinterpret_cast<__half *>(c.smem + OFF_ACT16);
     act16[r] = split_half(a, false);
     act16[ACT16_PITCH + r] = split_half(a, true);
-  } else if (c.tid < 64) {   // rows past the slice multiply stale bytes: zero activations
-    __half *act16 = reinterpret_cast<__half *>(c.smem + OFF_ACT16);
-    act16[c.tid] = __float2half_rn(0.f);
-    act16[ACT16_PITCH + c.tid] = __float2half_rn(0.f);
   }
   QMK_FINE(14);
   return c.chunk + static_cast<uint32_t>(2 * nch);
@@ -392,11 +410,14 @@ __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __ha
     if (w < 2) {
       __half *qh = reinterpret_cast<__half *>(c.smem + OFF_QF + (2 * w) * KV_PITCH);
       __half *ql = reinterpret_cast<__half *>(c.smem + OFF_QF + (2 * w + 1) * KV_PITCH);
+      const uint32_t k = operand_exponent(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
+      if (lane == 0) s_misc[M_QSCALE + w] = exp2_up(k);
+      const float down = exp2_down(k);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         s_q[w * D + lane + 32 * i] = v[i];
-        qh[lane + 32 * i] = split_half(v[i], false);
-        ql[lane + 32 * i] = split_half(v[i], true);
+        qh[lane + 32 * i] = split_half(v[i] * down, false);
+        ql[lane + 32 * i] = split_half(v[i] * down, true);
       }
     } else {
       // the new row takes part in this step's attention as the fp16 value the cache will hold
@@ -420,6 +441,7 @@ __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __ha
 
   // (2) stream the old rows
   const int quad = c.lane & 3, rowq = c.lane >> 2;     // accumulator fragment: rows rowq, rowq + 8; columns 2 quad, 2 quad + 1
+  const float sc_quad = sc_log2 * s_misc[M_QSCALE + (quad & 1)];
   float acc[8][4];
 #pragma unroll
   for (int t = 0; t < 8; ++t) { acc[t][0] = 0.f; acc[t][1] = 0.f; acc[t][2] = 0.f; acc[t][3] = 0.f; }
@@ -463,7 +485,7 @@ __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __ha
         mma_16816(sc, a0, qf[p][0], qf[p][1]);
         mma_16816(sc2, a1, qf[p][2], qf[p][3]);
       }
-      float s_top = fmaf(sc[1] + sc2[1], LO_INV, sc[0] + sc2[0]) * sc_log2, s_bot = fmaf(sc[3] + sc2[3], LO_INV, sc[2] + sc2[2]) * sc_log2;
+      float s_top = fmaf(sc[1] + sc2[1], LO_INV, sc[0] + sc2[0]) * sc_quad, s_bot = fmaf(sc[3] + sc2[3], LO_INV, sc[2] + sc2[2]) * sc_quad;
       if (rowq >= nrow) s_top = -INFINITY;
       if (rowq + 8 >= nrow) s_bot = -INFINITY;
       float cm = fmaxf(s_top, s_bot);
@@ -573,23 +595,23 @@ __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __ha
 }
 
 #if QMK_TC_SEQS == 1
-// 1 / sqrt(mean of squares + eps) over the 1024 values whose squares the consumer threads hold in `ss`; one barrier.
-// (rsqrt.approx: 2 ulp; the sum's order is fixed.)
-__device__ __forceinline__ float block_rstd(const Ctx &c, float ss) {
+// 1 / sqrt(mean of squares + eps) over the 1024 values whose squares the consumer threads hold in `ss`; one barrier, which
+// also tells whether `big` holds in any thread.  (rsqrt.approx: 2 ulp; the sum's order is fixed.)
+__device__ __forceinline__ float block_rstd(const Ctx &c, float ss, bool &big) {
   ss = warp_sum(ss);
   float *red = c.f(F_RED);
   if (c.lane == 0) red[c.warp] = ss;
-  cons_sync();
+  big = cons_any(big);
   const float4 r0 = reinterpret_cast<const float4 *>(red)[0], r1 = reinterpret_cast<const float4 *>(red)[1],
                r2 = reinterpret_cast<const float4 *>(red)[2];
   const float tot = (((r0.x + r0.y) + (r0.z + r0.w)) + ((r1.x + r1.y) + (r1.z + r1.w))) + ((r2.x + r2.y) + (r2.z + r2.w));
   return rsqrtf(tot * (1.0f / H) + RMS_EPS);
 }
 
-// fp32 vector value -> residual stream (fp32) and the hi/lo fp16 halves of its RMS-normalised form.
-__device__ __forceinline__ void store_normalised(const Ctx &c, int n, float v, float rstd, float w, float *dst) {
+// fp32 vector value -> residual stream (fp32) and the hi/lo fp16 halves of its RMS-normalised form times `down`.
+__device__ __forceinline__ void store_normalised(const Ctx &c, int n, float v, float rstd, float w, float down, float *dst) {
   dst[n] = v;
-  const float xn = v * rstd * w;
+  const float xn = v * rstd * w * down;
   *reinterpret_cast<__half *>(c.smem + OFF_XF + xf_offset(n, 0)) = split_half(xn, false);
   *reinterpret_cast<__half *>(c.smem + OFF_XF + xf_offset(n, 1)) = split_half(xn, true);
 }
@@ -657,21 +679,24 @@ __device__ __noinline__ void red_wait_norm(const Params &P, const Ctx c, int whi
       if (valid & (1u << j)) vi[j] += static_cast<long long>(w[j] - base) >> RED_CNT_BITS;   // exact
   }
   QMK_FINE(which ? 45 : 41);
-  float v[PT], ss = 0.f;
+  float v[PT], w[PT], ss = 0.f;
+  bool big = false;
 #pragma unroll
   for (int j = 0; j < PT; ++j) {
     v[j] = (valid & (1u << j)) ? static_cast<float>(vi[j]) * RED_INV_SCALE : 0.f;
+    w[j] = (valid & (1u << j)) ? __half2float(norm_w[c.tid + j * CONS_THREADS]) : 0.f;
     ss = fmaf(v[j], v[j], ss);
+    big |= fabsf(w[j]) > NORM_W_LIMIT;
   }
-  const float rstd = block_rstd(c, ss);
+  const float rstd = block_rstd(c, ss, big), down = big ? NORM_DOWN : 1.f;
+  if (c.tid == 0) c.f(F_MISC)[M_XSCALE] = big ? NORM_UP : 1.f;
 #pragma unroll
   for (int j = 0; j < PT; ++j)
     if (valid & (1u << j)) {
       const int n = c.tid + j * CONS_THREADS;
-      const float w = __half2float(norm_w[n]);
-      store_normalised(c, n, v[j], rstd, w, dst);
+      store_normalised(c, n, v[j], rstd, w[j], down, dst);
       if (emit && c.cta == 0) {
-        if (P.normalized_out) P.normalized_out[n] = v[j] * rstd * w;
+        if (P.normalized_out) P.normalized_out[n] = v[j] * rstd * w[j];
         if (P.hidden_out) P.hidden_out[n] = __float2half_rn(v[j]);
       }
     }
@@ -695,18 +720,22 @@ __device__ __forceinline__ float embed_value(const unsigned char *erow, int n) {
 __device__ __noinline__ void embed_norm(const Params &P, const Ctx c, int token, const __half *norm_w) {
   constexpr int PT = (H + CONS_THREADS - 1) / CONS_THREADS;
   const unsigned char *erow = reinterpret_cast<const unsigned char *>(P.embed) + static_cast<size_t>(token) * ROW_BYTES;
-  float v[PT], ss = 0.f;
+  float v[PT], w[PT], ss = 0.f;
+  bool big = false;
 #pragma unroll
   for (int j = 0; j < PT; ++j) {
     const int n = c.tid + j * CONS_THREADS;
     v[j] = n < H ? embed_value(erow, n) : 0.f;
+    w[j] = n < H ? __half2float(norm_w[n]) : 0.f;
     ss = fmaf(v[j], v[j], ss);
+    big |= fabsf(w[j]) > NORM_W_LIMIT;
   }
-  const float rstd = block_rstd(c, ss);
+  const float rstd = block_rstd(c, ss, big), down = big ? NORM_DOWN : 1.f;
+  if (c.tid == 0) c.f(F_MISC)[M_XSCALE] = big ? NORM_UP : 1.f;
 #pragma unroll
   for (int j = 0; j < PT; ++j) {
     const int n = c.tid + j * CONS_THREADS;
-    if (n < H) store_normalised(c, n, v[j], rstd, __half2float(norm_w[n]), c.f(F_X));
+    if (n < H) store_normalised(c, n, v[j], rstd, w[j], down, c.f(F_X));
   }
   cons_sync();
 }
@@ -784,6 +813,7 @@ __device__ __noinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
     uint32_t arow[2];
     slice_row_addresses(c, nrows, arow);
     const int n0 = t->n0, n1 = t->n1;
+    const float up = which ? c.f(F_MISC)[M_ASCALE] : 1.f;
     // lane that holds this lane's output (fragment row = lane / 4), and whether it is its second row
     const int src = FP8_ROWS ? ((c.lane & 15) >> 1) * 4 : (c.lane & 7) * 4;
     const bool second = (c.lane & (FP8_ROWS ? 1 : 8)) != 0;
@@ -800,7 +830,7 @@ __device__ __noinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
       const int tile = t0 + (c.lane >> 4) * CONS_WARPS;
       if (tile < H / 16) {
         const int n = tile * 16 + (c.lane & 15);
-        float v = (c.lane & 16) ? (second ? s3 : s2) : (second ? s1 : s0);
+        float v = ((c.lane & 16) ? (second ? s3 : s2) : (second ? s1 : s0)) * up;
         if (FP8_ROWS) v *= scales[n];
         if (n >= n0 && n < n1) v += resid[n];
         const long long fx = __float2ll_rn(v * RED_SCALE), fx_prev = __float2ll_rn(prev[n] * RED_SCALE);
@@ -828,6 +858,7 @@ __device__ __noinline__ uint32_t lm_head_tc(const Params &P, Ctx c, float *dump)
   float best = -INFINITY;
   int best_i = 0x7fffffff;
   const int p0 = (KPAIRS * c.warp) / CONS_WARPS, p1 = (KPAIRS * (c.warp + 1)) / CONS_WARPS;
+  const float up = s_misc[M_XSCALE];
 #pragma unroll 1
   for (int tile = 0; tile < ntiles; ++tile) {
     float *pr = part + (tile & 1) * (CONS_WARPS * 16);
@@ -840,6 +871,7 @@ __device__ __noinline__ uint32_t lm_head_tc(const Params &P, Ctx c, float *dump)
         float v = 0.f;
 #pragma unroll
         for (int w = 0; w < CONS_WARPS; ++w) v += pr[w * 16 + c.tid];
+        v *= up;
         const int o = t->lm0 * CH_ROWS + row;
         if (v > best) { best = v; best_i = o; }     // rows ascend per thread: strict > keeps the lowest index
         if (dump) dump[o] = v;

@@ -47,7 +47,7 @@ __device__ __noinline__ uint32_t qkv_phase_seqs(const Params &P, Ctx c, uint32_t
 #pragma unroll
     for (int kb = 0; kb < CONS_WARPS; ++kb)
       if (kb < nkb) v += p[kb * PART_TASK];
-    ll_store(P.ll + static_cast<size_t>(b) * LL_WORDS + LL_QKV + t->q0 * CH_ROWS + r, v, tag);
+    ll_store(P.ll + static_cast<size_t>(b) * LL_WORDS + LL_QKV + t->q0 * CH_ROWS + r, v * c.f(F_MISC)[M_XSCALE], tag);
   }
   return c.chunk + static_cast<uint32_t>(nch);
 }
@@ -59,20 +59,25 @@ __device__ __noinline__ uint32_t gateup_phase_seqs(const Params &P, Ctx c) {
   cons_sync();
   const int b = c.tid / TPS, r = c.tid % TPS;
   __half *act16 = reinterpret_cast<__half *>(c.smem + OFF_ACT16) + 2 * b * ACT16_PITCH;
-  if (r < nch * CH_ROWS) {
-    const int ru = up_row(nch, r);
-    const float *pg = tc_part(c) + (r >> 4) * nkb * PART_TASK + b * 16 + (r & 15);
-    const float *pu = tc_part(c) + (ru >> 4) * nkb * PART_TASK + b * 16 + (ru & 15);
-    float g = 0.f, u = 0.f;
+  if (r < 64) {          // a sequence's first warp holds its slice; rows past it multiply stale bytes: zero activations
+    float a = 0.f;
+    if (r < nch * CH_ROWS) {
+      const int ru = up_row(nch, r);
+      const float *pg = tc_part(c) + (r >> 4) * nkb * PART_TASK + b * 16 + (r & 15);
+      const float *pu = tc_part(c) + (ru >> 4) * nkb * PART_TASK + b * 16 + (ru & 15);
+      float g = 0.f, u = 0.f;
 #pragma unroll
-    for (int kb = 0; kb < CONS_WARPS; ++kb)
-      if (kb < nkb) { g += pg[kb * PART_TASK]; u += pu[kb * PART_TASK]; }
-    const float a = g / (1.0f + expf(-g)) * u;
+      for (int kb = 0; kb < CONS_WARPS; ++kb)
+        if (kb < nkb) { g += pg[kb * PART_TASK]; u += pu[kb * PART_TASK]; }
+      const float up = c.f(F_MISC)[M_XSCALE];
+      g *= up;
+      a = g / (1.0f + expf(-g)) * (u * up);
+    }
+    const uint32_t k = operand_exponent(a);
+    if (r == 0) c.f(F_MISC)[M_ASCALE + b] = exp2_up(k);
+    a *= exp2_down(k);
     act16[r] = split_half(a, false);
     act16[ACT16_PITCH + r] = split_half(a, true);
-  } else if (r < 64) {   // rows past the slice multiply stale bytes: zero activations
-    act16[r] = __float2half_rn(0.f);
-    act16[ACT16_PITCH + r] = __float2half_rn(0.f);
   }
   return c.chunk + static_cast<uint32_t>(2 * nch);
 }
@@ -171,6 +176,7 @@ __device__ __noinline__ uint32_t slice_cols_seqs(const Params &P, Ctx c, int whi
     const int b = c.lane & 3, j = c.lane >> 2;
     const bool live = b < P.nseq;
     const int n0 = t->n0, n1 = t->n1;
+    const float up = which ? c.f(F_MISC)[M_ASCALE + (live ? b : 0)] : 1.f;
     const float *resid = tc_resid(c, which ^ 1, live ? b : 0);   // O slice: x, down slice: x1
     float *prev = tc_prev(c, which, live ? b : 0);
     unsigned long long *sum = P.red + (which * TC_SEQS + (live ? b : 0)) * RED_SUM_WORDS;
@@ -185,7 +191,7 @@ __device__ __noinline__ uint32_t slice_cols_seqs(const Params &P, Ctx c, int whi
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
             const int n = tile * 16 + (FP8_ROWS ? 2 * j + k : j + 8 * k);
-            float v = fmaf(acc[u][2 * k + 1], LO_INV, acc[u][2 * k]);
+            float v = fmaf(acc[u][2 * k + 1], LO_INV, acc[u][2 * k]) * up;
             if (FP8_ROWS) v *= scales[n];
             if (n >= n0 && n < n1) v += resid[n - n0];
             const long long fx = __float2ll_rn(v * RED_SCALE), fx_prev = __float2ll_rn(prev[n] * RED_SCALE);
@@ -214,14 +220,19 @@ __device__ __forceinline__ void normalise_seqs(const Ctx &c, const float (&v)[TC
     ss = warp_sum(ss);
     if (c.lane == 0) red[b * CONS_WARPS + c.warp] = ss;
   }
-  cons_sync();
   const int n0 = c.segs()->n0, n1 = c.segs()->n1;
   float w[VPT];
+  bool big = false;
 #pragma unroll
   for (int j = 0; j < VPT; ++j) {
     const int n = c.tid + j * CONS_THREADS;
     w[j] = n < H ? __half2float(norm_w[n]) : 0.f;
+    big |= fabsf(w[j]) > NORM_W_LIMIT;
   }
+  big = cons_any(big);
+  if (c.tid == 0) c.f(F_MISC)[M_XSCALE] = big ? NORM_UP : 1.f;
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) w[j] *= big ? NORM_DOWN : 1.f;
 #pragma unroll
   for (int b = 0; b < TC_SEQS; ++b) {
     const float4 *r = reinterpret_cast<const float4 *>(red + b * CONS_WARPS);
@@ -322,6 +333,7 @@ __device__ __noinline__ uint32_t lm_head_seqs(const Params &P, Ctx c, int step, 
   int best_i = 0x7fffffff;
   const int p0 = (KPAIRS * c.warp) / CONS_WARPS, p1 = (KPAIRS * (c.warp + 1)) / CONS_WARPS;
   const int b = c.tid >> 4, r = c.tid & 15;
+  const float up = c.f(F_MISC)[M_XSCALE];
   float *dump = (P.logits_out && b < P.nseq) ? P.logits_out + (static_cast<size_t>(b) * P.num_steps + step) * P.vocab : nullptr;
 #pragma unroll 1
   for (int tile = 0; tile < ntiles; ++tile) {
@@ -335,6 +347,7 @@ __device__ __noinline__ uint32_t lm_head_seqs(const Params &P, Ctx c, int step, 
         float v = 0.f;
 #pragma unroll
         for (int w = 0; w < CONS_WARPS; ++w) v += pr[w * PART_TASK + c.tid];
+        v *= up;
         const int o = t->lm0 * CH_ROWS + row;
         if (v > best) { best = v; best_i = o; }     // rows ascend per thread: strict > keeps the lowest index
         if (dump) dump[o] = v;
