@@ -277,7 +277,8 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             const uint64_t db = smem_desc_sw128(base + OFF_K + kb * (STAGES * K_HALF_BYTES) + s0 * K_HALF_BYTES);
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-              mma_f16_ss(ts, da + 2u * i, db + 2u * i, (half < HALVES - 1 || kb > 0 || i > 0) ? 1u : 0u, two ? IDESC_S2 : IDESC_S);
+              if (SPLIT && half == 0 && kb == 0 && i == 0) mma_f16_ss_onto_lo(ts, da, db, two ? IDESC_S2 : IDESC_S);
+              else mma_f16_ss(ts, da + 2u * i, db + 2u * i, (half < HALVES - 1 || kb > 0 || i > 0) ? 1u : 0u, two ? IDESC_S2 : IDESC_S);
           }
         mma_commit(s_full(p & 1));
         mma_commit(k_empty(s0));             // the K slots can be refilled as soon as this product is done
@@ -444,7 +445,7 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
               const __half2 h = __floats2half2_rn(v0, v1);
               packed[k] = *reinterpret_cast<const uint32_t *>(&h);
               if (SPLIT) {
-                const __half2 lo = __floats2half2_rn(v0 - __low2float(h), v1 - __high2float(h));
+                const __half2 lo = __floats2half2_rn((v0 - __low2float(h)) * LO_SCALE, (v1 - __high2float(h)) * LO_SCALE);
                 packed_lo[k] = *reinterpret_cast<const uint32_t *>(&lo);
               }
             }

@@ -26,16 +26,17 @@
 // ACTIVATIONS in 8 or 4 bits as well, which a greedy decoder checked token by token cannot afford.
 //
 // Split activations (template parameter AH = 2): A is [M x 2 K], columns [0, K) the fp16 rounding hi of the fp32
-// activations and columns [K, 2 K) the fp16 rounding lo of what it left (x - hi).  A stage holds both A tiles and ONE B
-// tile, which eight MMAs read instead of four: the weights cross HBM, L2 and the copy engine once.  hi + lo keeps 22 bits
-// of x (absolute floor 2^-25, the fp16 subnormals) and the products are exact.  The sums need care: the tensor core
-// TRUNCATES its fp32 accumulator after every K step, so the 128 steps of a 1024-wide row in one accumulator lose 4e-6 of
-// the result, ten times what the token-serial kernels lose (share of first-layer V rows that round to another fp16 than
-// float64's, 109 tokens: 0.93 % against 0.093 %).  So every K block gets an accumulator of its own - the four lo products
-// first, while it is small, then the four hi products - and the epilogue warps add the finished blocks up in registers
-// with rounded fp32 adds while the next ones are multiplied (four accumulators in turn): 0.087 %.  Eight accumulators
-// that the blocks shared, added once at the end, left 0.12 % and allowed only 64-wide tiles (776 tokens: 4.9 ms, now
-// 3.9 ms).  A tile is at most 128 wide (packed weights: 64, and four more warps, since theirs expand K blocks).
+// activations and columns [K, 2 K) the fp16 rounding of 2^11 times what it left, lo = (x - hi) * 2048.  A stage holds both A
+// tiles and ONE B tile, which eight MMAs read instead of four: the weights cross HBM, L2 and the copy engine once.  The
+// pair keeps 22 bits of x for every |x| from 2^-14 to 65504, and to 2^-36 below (unscaled, lo itself met the fp16
+// subnormals: activations near 1e-3 kept 15 bits, and 3.3 % of the cache values behind them rounded differently from
+// float64's, against 0.23 % now).  The products are exact.  The sums need care: the tensor core TRUNCATES its fp32
+// accumulator after every K step, so the 128 steps of a 1024-wide row in one accumulator lose 4e-6 of the result, ten times
+// what the token-serial kernels lose.  So every K block gets an accumulator of its own - the four lo products first, then
+// the four hi products, the first of which scales the accumulator back by 2^-11 - and the epilogue warps add the finished
+// blocks up in registers with rounded fp32 adds while the next ones are multiplied (four accumulators in turn).  Two
+// accumulators per block lost no less (FP8 rows) or 5 to 10 % less (fp16 rows) and made a pass 10 % longer.  A tile is at
+// most 128 wide (packed weights: 64, and four more warps, since theirs expand K blocks).
 #ifndef QMK_GEMM_TCGEN05_CUH_
 #define QMK_GEMM_TCGEN05_CUH_
 
@@ -163,6 +164,19 @@ __device__ __forceinline__ void mma_f16_ss(uint32_t tmem_d, uint64_t desc_a, uin
       ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(IDESC), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
       : "memory");
 }
+// D = A . B + D * 2^-11: the first product of hi halves on an accumulator that holds the products of the lo halves, which
+// are stored times 2^11 (LO_SCALE).
+__device__ __forceinline__ void mma_f16_ss_onto_lo(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t IDESC) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, 1, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%4, %5, %6, %7}, p, 11;\n\t"
+      "}\n"
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(IDESC), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+      : "memory");
+}
+constexpr float LO_SCALE = 2048.0f;
 // Programmatic dependent launch (see prefill_kernels.cuh): no-ops unless the launch carries the attribute.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -411,16 +425,18 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint64_t da = smem_desc_sw128(base + s * STAGE_BYTES);
         const uint64_t db = smem_desc_sw128(base + s * STAGE_BYTES + TILE_A);
+        // 16 halves = 32 bytes = 2 descriptor address units per K step
+        // FUSE: the up tile follows the gate tile in shared memory (BN more rows of the same 8-row-group layout),
+        // so one MMA of N = 2 BN covers both and leaves gate in columns [0, BN), up in [BN, 2 BN)
+        if (AH == 1) {
 #pragma unroll
-        for (int j = 0; j < BK / 16; ++j) {  // 16 halves = 32 bytes = 2 descriptor address units per K step
-          // FUSE: the up tile follows the gate tile in shared memory (BN more rows of the same 8-row-group layout),
-          // so one MMA of N = 2 BN covers both and leaves gate in columns [0, BN), up in [BN, 2 BN)
-          if (AH == 1) mma_f16_ss(tmem_base, da + 2u * j, db + 2u * j, (kb > 0 || j > 0) ? 1u : 0u, idesc_for(SB));
-          else mma_f16_ss(tmem_base + (kb % NACC) * SB, da + (TILE_A_BYTES >> 4) + 2u * j, db + 2u * j, j > 0 ? 1u : 0u, idesc_for(SB));
-        }
-        if (AH == 2) {
+          for (int j = 0; j < BK / 16; ++j) mma_f16_ss(tmem_base, da + 2u * j, db + 2u * j, (kb > 0 || j > 0) ? 1u : 0u, idesc_for(SB));
+        } else {
 #pragma unroll
-          for (int j = 0; j < BK / 16; ++j) mma_f16_ss(tmem_base + (kb % NACC) * SB, da + 2u * j, db + 2u * j, 1u, idesc_for(SB));
+          for (int j = 0; j < BK / 16; ++j) mma_f16_ss(tmem_base + (kb % NACC) * SB, da + (TILE_A_BYTES >> 4) + 2u * j, db + 2u * j, j > 0 ? 1u : 0u, idesc_for(SB));
+          mma_f16_ss_onto_lo(tmem_base + (kb % NACC) * SB, da, db, idesc_for(SB));
+#pragma unroll
+          for (int j = 1; j < BK / 16; ++j) mma_f16_ss(tmem_base + (kb % NACC) * SB, da + 2u * j, db + 2u * j, 1u, idesc_for(SB));
           mma_commit(blk_full(kb % NACC));
         }
         mma_commit(empty(s));               // the stage is free once these MMAs have read it
@@ -525,7 +541,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
               const float g0 = acc[c + 2 * i], g1 = acc[c + 2 * i + 1];
               const float a0 = g0 / (1.0f + expf(-g0)) * acc[SB - BN + c + 2 * i], a1 = g1 / (1.0f + expf(-g1)) * acc[SB - BN + c + 2 * i + 1];
               const __half2 hi = __floats2half2_rn(a0, a1);
-              const __half2 lo = __floats2half2_rn(a0 - __low2float(hi), a1 - __high2float(hi));
+              const __half2 lo = __floats2half2_rn((a0 - __low2float(hi)) * LO_SCALE, (a1 - __high2float(hi)) * LO_SCALE);
               hi4[i] = *reinterpret_cast<const uint32_t *>(&hi);
               lo4[i] = *reinterpret_cast<const uint32_t *>(&lo);
             }

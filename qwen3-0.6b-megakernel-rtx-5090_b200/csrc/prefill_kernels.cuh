@@ -38,7 +38,8 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-// Four values as fp16 at dst; SPLIT: also the fp16 rounding of what the first rounding left, `lo_off` halves further on.
+// Four values as fp16 at dst; SPLIT: also the fp16 rounding of LO_SCALE times what the first rounding left, `lo_off` halves
+// further on.
 template <bool SPLIT>
 __device__ __forceinline__ void store_halves4(__half *dst, int lo_off, float4 v) {
   const __half2 a = __floats2half2_rn(v.x, v.y), b = __floats2half2_rn(v.z, v.w);
@@ -47,8 +48,9 @@ __device__ __forceinline__ void store_halves4(__half *dst, int lo_off, float4 v)
   out.y = *reinterpret_cast<const uint32_t *>(&b);
   *reinterpret_cast<uint2 *>(dst) = out;
   if (SPLIT) {
-    const __half2 la = __floats2half2_rn(v.x - __low2float(a), v.y - __high2float(a));
-    const __half2 lb = __floats2half2_rn(v.z - __low2float(b), v.w - __high2float(b));
+    constexpr float S = qmk_gemm::LO_SCALE;
+    const __half2 la = __floats2half2_rn((v.x - __low2float(a)) * S, (v.y - __high2float(a)) * S);
+    const __half2 lb = __floats2half2_rn((v.z - __low2float(b)) * S, (v.w - __high2float(b)) * S);
     out.x = *reinterpret_cast<const uint32_t *>(&la);
     out.y = *reinterpret_cast<const uint32_t *>(&lb);
     *reinterpret_cast<uint2 *>(dst + lo_off) = out;

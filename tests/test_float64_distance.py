@@ -110,3 +110,22 @@ def test_decoded_rows(C, fmt, sequences, bound):
         share[fused] = wrong / total
     print(f"{fmt} x {sequences}: tensor cores {100 * share[2]:.4f} %, CUDA cores {100 * share[1]:.4f} %")
     assert 0 < share[2] < bound * share[1]
+
+
+@pytest.mark.parametrize("fmt,kind,tokens,bound", [("fp16", "small", 1024, 2.0), ("fp8", "small", 1024, 2.0)])
+def test_prefilled_rows(C, fmt, kind, tokens, bound):
+    """The ``prefill`` op in one pass against the same op as persistent steps on the CUDA cores (``set_fused(0)``).  SwiGLU
+    outputs near 1e-3 are where lo halves stored as they are meet the fp16 subnormals (ratio above 10 then)."""
+    from Model.Qwen06B_architecture import Decoder
+    engine_w, oracle_w = _model(fmt, kind)
+    ids = S.make_prompt(tokens, seed=tokens, vocab_size=VOCAB)
+    share = {}
+    for fused in (2, 0):
+        C.set_fused(fused=fused)
+        eng = Decoder(weights=engine_w, verbose=False, max_seq_len=(tokens + 63) // 64 * 64, weight_format=fmt)
+        eng.prefill_ids(ids)
+        wrong, total = flips(oracle_w, ids, eng._k_cache, eng._v_cache, 0)
+        share[fused] = wrong / total
+    C.set_fused(fused=2)
+    print(f"{fmt} {kind} {tokens}: one pass {100 * share[2]:.4f} %, steps {100 * share[0]:.4f} %")
+    assert 0 < share[2] < bound * share[0]
