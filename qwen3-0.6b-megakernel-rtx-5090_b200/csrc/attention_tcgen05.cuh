@@ -42,24 +42,16 @@ constexpr int TQ = 128, TK = 64;                 // queries per CTA, keys per ti
 constexpr int CHAINS = 2;                        // even / odd key tiles
 constexpr int THREADS = 64 + 128 * CHAINS + 64;  // warp 0 loads K, warp 1 issues the score MMAs, warps 2..5 / 6..9 own the 128 query rows of chain 0 / 1, warp 10 issues P . V, warp 11 loads V
 constexpr uint32_t Q_BYTES = TQ * D * 2;         // two [128 x 64] swizzled tiles
+constexpr uint32_t KV_STAGE_BYTES = 2 * TK * D * 2;   // K tile (two [64 x 64] halves of the head dimension), then the V tile
 constexpr uint32_t P_BYTES = TQ * TK * 2;
 constexpr int STAGES = 4;
 constexpr uint32_t K_HALF_BYTES = TK * 128;      // one [64 keys x 64 dims] swizzled tile
 // K: one ring per 64-wide half of the head dimension, slots adjacent (slots 2 q and 2 q + 1 form one 128-key operand);
 // V: slots of two [64 keys x 64 dims] tiles
-// Split operands (template parameter SPLIT; prefill with fp32 activations): the query tile and P come as an fp16 rounding
-// and the fp16 rounding of what it left, two MMA operands against the same K / V tile, so scores and outputs keep 22 bits
-// of q and P (K and V are fp16 by the cache's definition).  The second query tile and the second P tiles take 64 KB, for
-// which the V ring gives up two of its four stages.
-constexpr int V_STAGES_SPLIT = 2;
-template <bool SPLIT>
-struct Layout {
-  static constexpr int HALVES = SPLIT ? 2 : 1, V_STAGES = SPLIT ? V_STAGES_SPLIT : STAGES;
-  static constexpr uint32_t OFF_K = HALVES * Q_BYTES, OFF_V = OFF_K + 2 * STAGES * K_HALF_BYTES,
-                            OFF_P = OFF_V + V_STAGES * 2 * K_HALF_BYTES, OFF_BARS = OFF_P + HALVES * CHAINS * P_BYTES;
-  static constexpr size_t SMEM_BYTES = OFF_BARS + 256;
-  static_assert(SMEM_BYTES <= 232448, "227 KB per CTA");
-};
+constexpr uint32_t OFF_K = Q_BYTES, OFF_V = OFF_K + 2 * STAGES * K_HALF_BYTES, OFF_P = OFF_V + STAGES * 2 * K_HALF_BYTES,
+                   OFF_BARS = OFF_P + CHAINS * P_BYTES;
+static_assert(OFF_P == Q_BYTES + STAGES * KV_STAGE_BYTES, "ring sizes");
+constexpr size_t SMEM_BYTES = OFF_BARS + 256;
 constexpr uint32_t TMEM_COLS = 512;              // scores of pair p in columns [128 (p mod 2), +128) (chain c: +64 c), O of chain c in [256 + 128 c, +128)
 constexpr float RESCALE_THRESHOLD = 8.0f;        // log2 units
 
@@ -119,17 +111,11 @@ __device__ __forceinline__ float fast_exp2(float x) {
 // items[i] = {sequence, first row of the query tile, its position within the sequence, head | length << 8} (sorted
 // from the heaviest down by the host) and reads that sequence's caches through maps_dev[2 seq], maps_dev[2 seq + 1]
 // in device memory; T and pos0 are then not used.
-//
-// SPLIT: map_q covers [rows][2 x 2048] (hi, then lo), out is fp16 [T][2 x 2048] (hi, then lo).
-template <bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1)
 causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                     int layer_head0, __half *out, int T, int pos0, float scale, unsigned int *status,
                     unsigned long long budget_ns, const int4 *items, const CUtensorMap *maps_dev) {
   using namespace qmk_gemm;
-  using L = Layout<SPLIT>;
-  constexpr int HALVES = L::HALVES, V_STAGES = L::V_STAGES;
-  constexpr uint32_t OFF_K = L::OFF_K, OFF_V = L::OFF_V, OFF_P = L::OFF_P, OFF_BARS = L::OFF_BARS;
   extern __shared__ __align__(1024) unsigned char attn_smem[];
   const uint32_t base = s32(attn_smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -199,7 +185,7 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   // the query tile and the K ring's first fill go out at once (thread 0 is the K producer and has just initialised
   // the barriers itself); a CTA's fixed costs weigh as much as its first key tiles
   auto load_tile = [&](bool is_v, int j) {
-    const int s = is_v ? j % V_STAGES : j % STAGES;
+    const int s = j % STAGES;
     const uint32_t full = is_v ? v_full(s) : k_full(s);
     const uint32_t d0 = base + (is_v ? OFF_V + s * 2 * K_HALF_BYTES : OFF_K + s * K_HALF_BYTES);
     const uint32_t d1 = d0 + (is_v ? K_HALF_BYTES : STAGES * K_HALF_BYTES);
@@ -217,13 +203,9 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // the query tile: fp16, already times scale * log2 e (the softmax is an exp2), as two [128 x 64] boxes in the
     // K-major 128-byte-swizzled layout the score MMAs read; rows past the live ones hold other tokens' or stale
     // finite values and are never stored
-    bar_expect_tx(q_full, HALVES * Q_BYTES);
+    bar_expect_tx(q_full, Q_BYTES);
     tma_load_2d(base, &map_q, head * D, q0, q_full);
     tma_load_2d(base + TQ * 128, &map_q, head * D + 64, q0, q_full);
-    if (SPLIT) {
-      tma_load_2d(base + Q_BYTES, &map_q, NQ * D + head * D, q0, q_full);
-      tma_load_2d(base + Q_BYTES + TQ * 128, &map_q, NQ * D + head * D + 64, q0, q_full);
-    }
     for (; k_prefilled < STAGES && k_prefilled < ntiles; ++k_prefilled) load_tile(false, k_prefilled);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -235,20 +217,19 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   if (warp == 0 || warp == 3 + 4 * CHAINS) {
     if (lane == 0) {                       // ---- producers: the K ring (warp 0) and the V ring, tiles of 64 rows
       const bool is_v = warp != 0;
-      const int stages = is_v ? V_STAGES : STAGES;
       int issued = is_v ? 0 : k_prefilled;
       for (int j = issued; j < ntiles; ++j) {
-        const int s = j % stages;
-        if (j >= stages && !bar_wait(is_v ? v_empty(s) : k_empty(s), ((j / stages) - 1) & 1, abort_flag, status, budget_ns)) break;
+        const int s = j % STAGES;
+        if (j >= STAGES && !bar_wait(is_v ? v_empty(s) : k_empty(s), ((j / STAGES) - 1) & 1, abort_flag, status, budget_ns)) break;
         if (*abort_flag) break;
         load_tile(is_v, j);
         issued = j + 1;
       }
       if (*abort_flag) {                   // copies already issued must land before the CTA may exit
-        for (int jj = (issued > stages ? issued - stages : 0); jj < issued; ++jj) {
-          const uint32_t bar = is_v ? v_full(jj % stages) : k_full(jj % stages);
+        for (int jj = (issued > STAGES ? issued - STAGES : 0); jj < issued; ++jj) {
+          const uint32_t bar = is_v ? v_full(jj % STAGES) : k_full(jj % STAGES);
           const unsigned long long t0 = gtime();
-          while (!bar_try(bar, (jj / stages) & 1)) {
+          while (!bar_try(bar, (jj / STAGES) & 1)) {
             if (gtime() - t0 > (budget_ns > 2000000ull ? budget_ns : 2000000ull)) break;
           }
         }
@@ -268,18 +249,13 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t ts = tmem_base + 128u * static_cast<uint32_t>(p & 1);
-        // split queries: the lo products first, while the accumulator (truncated after every step) is small
 #pragma unroll
-        for (int half = HALVES - 1; half >= 0; --half)
+        for (int kb = 0; kb < 2; ++kb) {                      // 64-wide halves of the head dimension, four K = 16 steps each
+          const uint64_t da = smem_desc_sw128(base + kb * (TQ * 128));
+          const uint64_t db = smem_desc_sw128(base + OFF_K + kb * (STAGES * K_HALF_BYTES) + s0 * K_HALF_BYTES);
 #pragma unroll
-          for (int kb = 0; kb < 2; ++kb) {                    // 64-wide halves of the head dimension, four K = 16 steps each
-            const uint64_t da = smem_desc_sw128(base + half * Q_BYTES + kb * (TQ * 128));
-            const uint64_t db = smem_desc_sw128(base + OFF_K + kb * (STAGES * K_HALF_BYTES) + s0 * K_HALF_BYTES);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              if (SPLIT && half == 0 && kb == 0 && i == 0) mma_f16_ss_onto_lo(ts, da, db, two ? IDESC_S2 : IDESC_S);
-              else mma_f16_ss(ts, da + 2u * i, db + 2u * i, (half < HALVES - 1 || kb > 0 || i > 0) ? 1u : 0u, two ? IDESC_S2 : IDESC_S);
-          }
+          for (int i = 0; i < 4; ++i) mma_f16_ss(ts, da + 2u * i, db + 2u * i, (kb > 0 || i > 0) ? 1u : 0u, two ? IDESC_S2 : IDESC_S);
+        }
         mma_commit(s_full(p & 1));
         mma_commit(k_empty(s0));             // the K slots can be refilled as soon as this product is done
         if (two) mma_commit(k_empty(s0 + 1));
@@ -291,21 +267,18 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       for (int j = 0; j < ntiles && ok; ++j) {
         const int c = j & 1, n = j >> 1;   // chain, and the tile's index within it
         ok = bar_wait(p_ready(c), n & 1, abort_flag, status, budget_ns) &&
-             bar_wait(v_full(j % V_STAGES), (j / V_STAGES) & 1, abort_flag, status, budget_ns);
+             bar_wait(v_full(j % STAGES), (j / STAGES) & 1, abort_flag, status, budget_ns);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // O_c += P_c . V_j: four steps of 16 keys; V rows are [key][dim], i.e. MN-major for the B operand
-        const uint32_t vt = base + OFF_V + (j % V_STAGES) * 2 * K_HALF_BYTES;
-        const uint64_t dp = smem_desc_sw128(base + OFF_P + static_cast<uint32_t>(c) * (HALVES * P_BYTES));
+        const uint32_t vt = base + OFF_V + (j % STAGES) * 2 * K_HALF_BYTES;
+        const uint64_t dp = smem_desc_sw128(base + OFF_P + static_cast<uint32_t>(c) * P_BYTES);
         const uint32_t to = tmem_o0 + 128u * static_cast<uint32_t>(c);
 #pragma unroll
-        for (int half = HALVES - 1; half >= 0; --half)        // (split P: the lo products first, as for the scores)
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            mma_f16_ss(to, dp + static_cast<uint64_t>(half) * (P_BYTES >> 4) + 2u * i, smem_desc_mn_sw128(vt + i * 16 * 128, K_HALF_BYTES),
-                       (n > 0 || half < HALVES - 1 || i > 0) ? 1u : 0u, IDESC_PV);
+        for (int i = 0; i < 4; ++i)
+          mma_f16_ss(to, dp + 2u * i, smem_desc_mn_sw128(vt + i * 16 * 128, K_HALF_BYTES), (n > 0 || i > 0) ? 1u : 0u, IDESC_PV);
         mma_commit(pv_done(c));            // O_c has taken tile j: P_c may be overwritten, O_c rescaled (or, at the end, read)
-        mma_commit(v_empty(j % V_STAGES));
+        mma_commit(v_empty(j % STAGES));
       }
     }
   } else {                                 // ---- softmax: chain = warp group, thread = query row = TMEM lane
@@ -314,7 +287,7 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const int qpos = pbase + row;          // (rows past T compute on zeros and are not stored)
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t tmem_o = tmem_o0 + 128u * static_cast<uint32_t>(chain);
-    const uint32_t p_tile = base + OFF_P + static_cast<uint32_t>(chain) * (HALVES * P_BYTES);
+    const uint32_t p_tile = base + OFF_P + static_cast<uint32_t>(chain) * P_BYTES;
     float m_used = -INFINITY, l = 0.f;     // (m_used stays -inf while every key the chain has seen is masked for this row)
     bool ok = true;
     for (int j = chain; j < ntiles && ok; j += CHAINS) {
@@ -374,7 +347,7 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       float sum4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int seg = 0; seg < 8; ++seg) {
-        uint32_t packed[4], packed_lo[4];
+        uint32_t packed[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int c = seg * 8 + 2 * i;
@@ -383,16 +356,9 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           sum4[i] += a + b;
           const __half2 h = __floats2half2_rn(a, b);
           packed[i] = *reinterpret_cast<const uint32_t *>(&h);
-          if (SPLIT) {
-            const __half2 lo = __floats2half2_rn(a - __low2float(h), b - __high2float(h));
-            packed_lo[i] = *reinterpret_cast<const uint32_t *>(&lo);
-          }
         }
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(prow + ((static_cast<uint32_t>(seg) ^ x) << 4)),
                      "r"(packed[0]), "r"(packed[1]), "r"(packed[2]), "r"(packed[3]) : "memory");
-        if (SPLIT)
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(prow + P_BYTES + ((static_cast<uint32_t>(seg) ^ x) << 4)),
-                       "r"(packed_lo[0]), "r"(packed_lo[1]), "r"(packed_lo[2]), "r"(packed_lo[3]) : "memory");
       }
       l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // P before the MMA's async-proxy reads
@@ -410,7 +376,7 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     float m_other, l_other;
     asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(m_other), "=f"(l_other)
-                 : "r"(base + OFF_P + static_cast<uint32_t>(chain ^ 1) * (HALVES * P_BYTES) + static_cast<uint32_t>(row) * 8u) : "memory");
+                 : "r"(base + OFF_P + static_cast<uint32_t>(chain ^ 1) * P_BYTES + static_cast<uint32_t>(row) * 8u) : "memory");
     ok = ok && !*abort_flag;
     if (ok) {
       // chain 0 always holds key 0, which every query sees: the common maximum is finite
@@ -423,7 +389,7 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       const float fa = f_a * inv, fb = f_b * inv;
       const int t = q0 + row;
       // this warp group writes dims [64 chain, +64) of the row from both accumulators
-      __half *orow = out + static_cast<size_t>(t < T ? t : 0) * (HALVES * NQ * D) + head * D + 64 * chain;
+      __half *orow = out + static_cast<size_t>(t < T ? t : 0) * (NQ * D) + head * D + 64 * chain;
 #pragma unroll 1
       for (int c = 0; c < 2; ++c) {
         const uint32_t col = static_cast<uint32_t>(64 * chain + 32 * c);
@@ -434,7 +400,7 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (t < T) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
-            uint32_t packed[4], packed_lo[4];
+            uint32_t packed[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               float v0 = __uint_as_float(oa[i + 2 * k]) * fa, v1 = __uint_as_float(oa[i + 2 * k + 1]) * fa;
@@ -444,14 +410,8 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
               }
               const __half2 h = __floats2half2_rn(v0, v1);
               packed[k] = *reinterpret_cast<const uint32_t *>(&h);
-              if (SPLIT) {
-                const __half2 lo = __floats2half2_rn((v0 - __low2float(h)) * LO_SCALE, (v1 - __high2float(h)) * LO_SCALE);
-                packed_lo[k] = *reinterpret_cast<const uint32_t *>(&lo);
-              }
             }
             *reinterpret_cast<uint4 *>(orow + c * 32 + i) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-            if (SPLIT)
-              *reinterpret_cast<uint4 *>(orow + NQ * D + c * 32 + i) = make_uint4(packed_lo[0], packed_lo[1], packed_lo[2], packed_lo[3]);
           }
         }
       }

@@ -177,8 +177,7 @@ add_rmsnorm_rows_wide(float *x, const float *add, int nparts, size_t part_stride
 // all four issued before the first is used (the kernel is a few dependent round trips per warp: with one head per warp
 // and four blocks per token it spent 13 us on seven waves of blocks at 2048 tokens).
 // in_f16: q / k / v hold fp16 (the projection's epilogue stored halves) instead of fp32.
-// q_f16_scale != 0: the rotated queries are stored as fp16 times that factor (same [t][head][128] layout in halves);
-// q_split: as hi and lo halves, [t][2][head][128].
+// q_f16_scale != 0: the rotated queries are stored as fp16 times that factor (same [t][head][128] layout in halves).
 // Packed prompts (row_info != null): row t belongs to sequence row_info[t].x at position row_info[t].y (negative:
 // a padding row, nothing to do), whose K / V caches start at kv_ptrs[2 seq], kv_ptrs[2 seq + 1]; the layer's rows
 // begin `layer_off` halves into each.
@@ -187,7 +186,7 @@ qk_norm_rope_cache(const float *q, const float *k, const float *v, int in_f16, c
                    const __half *k_norm, const float *rope, const __half *cos_table,
                    const __half *sin_table, float *qr, __half *k_cache_layer, __half *v_cache_layer,
                    int pos0, int max_seq_len, const int2 *row_info, const unsigned long long *kv_ptrs, size_t layer_off,
-                   float q_f16_scale, int q_split) {
+                   float q_f16_scale) {
   pdl_wait();
   pdl_trigger();
   const int t = blockIdx.x, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -256,10 +255,7 @@ qk_norm_rope_cache(const float *q, const float *k, const float *v, int in_f16, c
     } else {            // high half: lo * sin + hi * cos
       r = make_float4(o.x * sn.x + a.x * cs.x, o.y * sn.y + a.y * cs.y, o.z * sn.z + a.z * cs.z, o.w * sn.w + a.w * cs.w);
     }
-    if (h < 2 && q_split)
-      store_halves4<true>(reinterpret_cast<__half *>(qr) + (static_cast<size_t>(t) * 2 * NQ + w + 8 * h) * D + d0, NQ * D,
-                          make_float4(r.x * q_f16_scale, r.y * q_f16_scale, r.z * q_f16_scale, r.w * q_f16_scale));
-    else if (h < 2 && q_f16_scale != 0.f)   // fp16 queries, pre-scaled: the tcgen05 attention kernel takes them by TMA as they are
+    if (h < 2 && q_f16_scale != 0.f)   // fp16 queries, pre-scaled: the tcgen05 attention kernel takes them by TMA as they are
       *reinterpret_cast<uint2 *>(reinterpret_cast<__half *>(qr) + (static_cast<size_t>(t) * NQ + w + 8 * h) * D + d0) =
           pack4(r.x * q_f16_scale, r.y * q_f16_scale, r.z * q_f16_scale, r.w * q_f16_scale);
     else if (h < 2)
@@ -450,6 +446,253 @@ __global__ void __launch_bounds__(ATM_THREADS) causal_attention_mma(const float 
         *reinterpret_cast<__half2 *>(out + static_cast<size_t>(tok_hi) * QS + d) = __floats2half2_rn(o[dt][2] * inv_hi, o[dt][3] * inv_hi);
     }
   }
+}
+
+// The same with split operands, for the prefill op (fp32 activations): queries and softmax weights go to the MMAs as an
+// fp16 rounding and the fp16 rounding of LO_SCALE times what it left (K and V are fp16 by the cache's definition), four MMAs
+// where the kernel above takes two.  The tensor core truncates the accumulator it is handed, so no accumulator sees more
+// than four hi products (64 dimensions of a score, 64 keys of an output); the sums are added in registers (UNSHRINK).  Share
+// of cache values that round differently from float64 in the fourth layer, attention on few keys, behind 1024 / 4096 / 8000
+// tokens: 0.47 / 0.52 / 0.54 %.  (The token-serial kernel this pass replaced: 0.57 / 0.60 / 0.60; one tcgen05 accumulator for
+// all dimensions and one for all keys: 0.77 / 1.4 / 2.1.)  Bound by the issue of mma.sync, 256 per warp and 64 keys: the whole
+// pass takes 5.1 ms at 776 tokens (tcgen05 4.3), 26 at 4096 (16), 72 at 8000 (40).
+// A row of queries is divided by a power of two where it exceeds 2^15 (see operand_exponent of the decode kernels).
+// grid = (ceil(T / 32), 8 kv heads, key splits): with few query tiles - a short prompt behind a long context - the key tiles
+// are divided among gridDim.z CTAs, which leave (unnormalised output, maximum, sum) per row and head in `part`
+// [split][T][16][130]; merge_attention_splits adds them up.  out: [T][hi 2048 | lo 2048].
+constexpr int ATS_MAX_SPLITS = 16, ATS_PART = D + 2;
+__device__ __forceinline__ void mma_16816_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// Two values as a pair of hi halves and a pair of scaled lo halves.
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t &hi, uint32_t &lo) {
+  const __half2 h = __floats2half2_rn(x, y);
+  hi = *reinterpret_cast<const uint32_t *>(&h);
+  lo = pack_half2((x - __low2float(h)) * qmk_gemm::LO_SCALE, (y - __high2float(h)) * qmk_gemm::LO_SCALE);
+}
+__global__ void __launch_bounds__(ATM_THREADS, 2) causal_attention_split(const float *qr, const __half *k_cache_layer,
+                                                            const __half *v_cache_layer, __half *out, float *part, int T, int pos0,
+                                                            int max_seq_len, float scale) {
+  constexpr float LO_INV = 1.0f / qmk_gemm::LO_SCALE;
+  pdl_wait();
+  pdl_trigger();
+  extern __shared__ __align__(16) unsigned char atm_smem[];
+  __half *const tiles = reinterpret_cast<__half *>(atm_smem);
+  const int g = blockIdx.y, t0 = (gridDim.x - 1 - blockIdx.x) * ATM_Q;   // longest tiles first
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int h = warp & 1, tw = t0 + 16 * (warp >> 1);     // this warp's head and first token
+  const int gr = lane >> 2, qd = lane & 3;                // fragment row within 8, quad lane
+  const int tok_lo = tw + gr, tok_hi = tw + gr + 8;       // the two query rows this lane holds
+  const float sc = scale * 1.4426950408889634f;
+
+  uint32_t qh[8][4], ql[8][4];   // query fragments (A operand), 8 k-steps of 16 dims
+  float up_lo, up_hi;
+  {
+    const float *q_lo = qr + (static_cast<size_t>(min(tok_lo, T - 1)) * NQ + 2 * g + h) * D;
+    const float *q_hi = qr + (static_cast<size_t>(min(tok_hi, T - 1)) * NQ + 2 * g + h) * D;
+    float m_lo = 0.f, m_hi = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < 16; ++ks) {
+      const float2 a = *reinterpret_cast<const float2 *>(q_lo + ks * 8 + qd * 2), b = *reinterpret_cast<const float2 *>(q_hi + ks * 8 + qd * 2);
+      m_lo = fmaxf(m_lo, fmaxf(fabsf(a.x), fabsf(a.y)));
+      m_hi = fmaxf(m_hi, fmaxf(fabsf(b.x), fabsf(b.y)));
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      m_lo = fmaxf(m_lo, __shfl_xor_sync(0xffffffffu, m_lo, o));
+      m_hi = fmaxf(m_hi, __shfl_xor_sync(0xffffffffu, m_hi, o));
+    }
+    const int e_lo = static_cast<int>(__float_as_uint(m_lo * fabsf(sc)) >> 23) - 141, e_hi = static_cast<int>(__float_as_uint(m_hi * fabsf(sc)) >> 23) - 141;
+    const int x_lo = max(e_lo, 0), x_hi = max(e_hi, 0);
+    up_lo = __uint_as_float(static_cast<uint32_t>(127 + x_lo) << 23);
+    up_hi = __uint_as_float(static_cast<uint32_t>(127 + x_hi) << 23);
+    const float s_lo = sc * __uint_as_float(static_cast<uint32_t>(127 - x_lo) << 23), s_hi = sc * __uint_as_float(static_cast<uint32_t>(127 - x_hi) << 23);
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      const int d = ks * 16 + qd * 2;
+      const float2 l0 = *reinterpret_cast<const float2 *>(q_lo + d), l1 = *reinterpret_cast<const float2 *>(q_lo + d + 8);
+      const float2 h0 = *reinterpret_cast<const float2 *>(q_hi + d), h1 = *reinterpret_cast<const float2 *>(q_hi + d + 8);
+      split_pair(l0.x * s_lo, l0.y * s_lo, qh[ks][0], ql[ks][0]);
+      split_pair(h0.x * s_hi, h0.y * s_hi, qh[ks][1], ql[ks][1]);
+      split_pair(l1.x * s_lo, l1.y * s_lo, qh[ks][2], ql[ks][2]);
+      split_pair(h1.x * s_hi, h1.y * s_hi, qh[ks][3], ql[ks][3]);
+    }
+  }
+  float o[16][4];
+#pragma unroll
+  for (int dt = 0; dt < 16; ++dt) { o[dt][0] = 0.f; o[dt][1] = 0.f; o[dt][2] = 0.f; o[dt][3] = 0.f; }
+  float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;
+  // rows beyond the chunk see no key at all
+  const int lim_lo = tok_lo < T ? pos0 + tok_lo : -1, lim_hi = tok_hi < T ? pos0 + tok_hi : -1;
+  const int warp_last = pos0 + min(tw + 15, T - 1);                   // highest key this warp needs (tw < T or unused)
+  const int cta_last = pos0 + min(t0 + ATM_Q - 1, T - 1);
+  const int ntiles = cta_last / ATM_KEYS + 1, splits = static_cast<int>(gridDim.z), z = static_cast<int>(blockIdx.z);
+  const int first = ntiles * z / splits * ATM_KEYS, end = ntiles * (z + 1) / splits * ATM_KEYS;   // this CTA's keys
+  const __half *kbase = k_cache_layer + static_cast<size_t>(g) * max_seq_len * D;
+  const __half *vbase = v_cache_layer + static_cast<size_t>(g) * max_seq_len * D;
+
+  auto fetch_tile = [&](int k0, int stage) {   // rows past the last key this CTA needs are zero-filled
+    __half *dk = tiles + stage * ATM_STAGE_HALVES, *dv = dk + ATM_KEYS * ATM_PITCH;
+    for (int i = threadIdx.x; i < ATM_KEYS * (D / 8); i += ATM_THREADS) {
+      const int j = i >> 4, c = i & 15;
+      const bool in = k0 + j <= cta_last;
+      const size_t off = static_cast<size_t>(in ? k0 + j : 0) * D + c * 8;
+      const uint32_t bytes = in ? 16u : 0u;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dk + j * ATM_PITCH + c * 8))),
+                   "l"(kbase + off), "r"(bytes) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dv + j * ATM_PITCH + c * 8))),
+                   "l"(vbase + off), "r"(bytes) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if (first < end) fetch_tile(first, 0);
+  int stage = 0;
+  for (int k0 = first; k0 < end; k0 += ATM_KEYS, stage ^= 1) {
+    // the other stage was last read in the previous iteration, which ended with a barrier
+    if (k0 + ATM_KEYS < end) {
+      fetch_tile(k0 + ATM_KEYS, stage ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const __half *sk = tiles + stage * ATM_STAGE_HALVES, *sv = sk + ATM_KEYS * ATM_PITCH;
+    if (tw >= T || k0 > warp_last) {   // warp-uniform: nothing (more) to do for this warp in this tile
+      __syncthreads();
+      continue;
+    }
+    // S = Q K^T for 64 keys: 8 n-tiles of 8 keys
+    float sacc[8][4];
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+      float lo[4] = {0.f, 0.f, 0.f, 0.f}, d[4], e[4];
+      const __half *krow = sk + (nt * 8 + gr) * ATM_PITCH + qd * 2;
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks) {
+        const uint32_t b0 = *reinterpret_cast<const uint32_t *>(krow + ks * 16);
+        const uint32_t b1 = *reinterpret_cast<const uint32_t *>(krow + ks * 16 + 8);
+        mma_16816(lo, ql[ks], b0, b1);
+        if (ks == 0) mma_16816_zero(d, qh[ks], b0, b1);
+        else if (ks < 4) mma_16816(d, qh[ks], b0, b1);
+        else if (ks == 4) mma_16816_zero(e, qh[ks], b0, b1);
+        else mma_16816(e, qh[ks], b0, b1);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sacc[nt][i] = fmaf(d[i] + e[i], qmk_gemm::UNSHRINK, lo[i] * LO_INV) * (i < 2 ? up_lo : up_hi);
+    }
+    // causal mask + row maxima (a row lives in the 4 lanes of a quad)
+    float mx_lo = -INFINITY, mx_hi = -INFINITY;
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+      const int key = k0 + nt * 8 + qd * 2;
+      if (key > lim_lo) sacc[nt][0] = -INFINITY;
+      if (key + 1 > lim_lo) sacc[nt][1] = -INFINITY;
+      if (key > lim_hi) sacc[nt][2] = -INFINITY;
+      if (key + 1 > lim_hi) sacc[nt][3] = -INFINITY;
+      mx_lo = fmaxf(mx_lo, fmaxf(sacc[nt][0], sacc[nt][1]));
+      mx_hi = fmaxf(mx_hi, fmaxf(sacc[nt][2], sacc[nt][3]));
+    }
+    mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 1));
+    mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
+    mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
+    mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
+    const float mn_lo = fmaxf(m_lo, mx_lo), mn_hi = fmaxf(m_hi, mx_hi);
+    const float ref_lo = (mn_lo == -INFINITY) ? 0.f : mn_lo, ref_hi = (mn_hi == -INFINITY) ? 0.f : mn_hi;   // fully masked rows
+    const float c_lo = exp2f(m_lo - ref_lo), c_hi = exp2f(m_hi - ref_hi);
+    m_lo = mn_lo; m_hi = mn_hi;
+    float sum_lo = 0.f, sum_hi = 0.f;
+    uint32_t ph[4][4], pl[4][4];   // P as A fragments: 4 key-steps of 16 keys
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+      const float p0 = exp2f(sacc[nt][0] - ref_lo), p1 = exp2f(sacc[nt][1] - ref_lo);
+      const float p2 = exp2f(sacc[nt][2] - ref_hi), p3 = exp2f(sacc[nt][3] - ref_hi);
+      sum_lo += p0 + p1;
+      sum_hi += p2 + p3;
+      split_pair(p0, p1, ph[nt >> 1][(nt & 1) * 2 + 0], pl[nt >> 1][(nt & 1) * 2 + 0]);
+      split_pair(p2, p3, ph[nt >> 1][(nt & 1) * 2 + 1], pl[nt >> 1][(nt & 1) * 2 + 1]);
+    }
+    sum_lo += __shfl_xor_sync(0xffffffffu, sum_lo, 1);
+    sum_lo += __shfl_xor_sync(0xffffffffu, sum_lo, 2);
+    sum_hi += __shfl_xor_sync(0xffffffffu, sum_hi, 1);
+    sum_hi += __shfl_xor_sync(0xffffffffu, sum_hi, 2);
+    l_lo = l_lo * c_lo + sum_lo;
+    l_hi = l_hi * c_hi + sum_hi;
+#pragma unroll
+    for (int dt = 0; dt < 16; ++dt) { o[dt][0] *= c_lo; o[dt][1] *= c_lo; o[dt][2] *= c_hi; o[dt][3] *= c_hi; }
+    // O += P V: B fragments of V through ldmatrix.trans (4 8x8 matrices: keys 0-7 / 8-15 of the step x two dim tiles)
+    const int mi = lane >> 3;
+    const __half *vrow = sv + ((mi & 1) * 8 + (lane & 7)) * ATM_PITCH + (mi >> 1) * 8;
+#pragma unroll
+    for (int dp = 0; dp < 8; ++dp) {
+      float lo0[4] = {0.f, 0.f, 0.f, 0.f}, lo1[4] = {0.f, 0.f, 0.f, 0.f}, d0[4], d1[4];
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        uint32_t b0, b1, b2, b3;
+        const uint32_t addr = static_cast<uint32_t>(__cvta_generic_to_shared(vrow + kk * 16 * ATM_PITCH + dp * 16));
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3)
+                     : "r"(addr));
+        if (kk == 0) { mma_16816_zero(d0, ph[kk], b0, b1); mma_16816_zero(d1, ph[kk], b2, b3); }
+        else { mma_16816(d0, ph[kk], b0, b1); mma_16816(d1, ph[kk], b2, b3); }
+        mma_16816(lo0, pl[kk], b0, b1);
+        mma_16816(lo1, pl[kk], b2, b3);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { o[2 * dp][i] = fmaf(d0[i], qmk_gemm::UNSHRINK, o[2 * dp][i]); o[2 * dp + 1][i] = fmaf(d1[i], qmk_gemm::UNSHRINK, o[2 * dp + 1][i]); }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { o[2 * dp][i] = fmaf(lo0[i], LO_INV, o[2 * dp][i]); o[2 * dp + 1][i] = fmaf(lo1[i], LO_INV, o[2 * dp + 1][i]); }
+    }
+    __syncthreads();   // this stage is free for the fetch of the iteration after next
+  }
+  if (tw >= T) return;
+  if (splits > 1) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int t = r ? tok_hi : tok_lo;
+      if (t >= T) continue;
+      float *p = part + ((static_cast<size_t>(z) * T + t) * NQ + 2 * g + h) * ATS_PART;
+#pragma unroll
+      for (int dt = 0; dt < 16; ++dt) *reinterpret_cast<float2 *>(p + dt * 8 + qd * 2) = make_float2(o[dt][2 * r], o[dt][2 * r + 1]);
+      if (qd == 0) *reinterpret_cast<float2 *>(p + D) = make_float2(r ? m_hi : m_lo, r ? l_hi : l_lo);
+    }
+    return;
+  }
+  const float inv_lo = 1.0f / l_lo, inv_hi = l_hi > 0.f ? 1.0f / l_hi : 0.f;   // (every live row sees its own key)
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int t = r ? tok_hi : tok_lo;
+    const float inv = r ? inv_hi : inv_lo;
+    if (t >= T) continue;
+    __half *row = out + static_cast<size_t>(t) * 2 * QS + (2 * g + h) * D + qd * 2;
+#pragma unroll
+    for (int dt = 0; dt < 16; ++dt) {
+      uint32_t hi, lo;
+      split_pair(o[dt][2 * r] * inv, o[dt][2 * r + 1] * inv, hi, lo);
+      *reinterpret_cast<uint32_t *>(row + dt * 8) = hi;
+      *reinterpret_cast<uint32_t *>(row + QS + dt * 8) = lo;
+    }
+  }
+}
+
+// out = the splits of causal_attention_split added up.  grid = T, block = 512: a warp per head, four dims per lane.
+__global__ void __launch_bounds__(512) merge_attention_splits(const float *part, int splits, __half *out, int T) {
+  pdl_wait();
+  pdl_trigger();
+  const int t = blockIdx.x, head = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float *p = part + (static_cast<size_t>(t) * NQ + head) * ATS_PART;
+  const size_t stride = static_cast<size_t>(T) * NQ * ATS_PART;
+  const float m = lane < splits ? p[lane * stride + D] : -INFINITY, l = lane < splits ? p[lane * stride + D + 1] : 0.f;
+  const float w = exp2f(m - warp_max(m));          // (split 0 holds key 0: the maximum is finite)
+  const float inv = 1.0f / warp_sum(l * w);
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s = 0; s < splits; ++s) {
+    const float ws = __shfl_sync(0xffffffffu, w, s);
+    const float2 x = *reinterpret_cast<const float2 *>(p + s * stride + 4 * lane), y = *reinterpret_cast<const float2 *>(p + s * stride + 4 * lane + 2);
+    a.x = fmaf(x.x, ws, a.x); a.y = fmaf(x.y, ws, a.y); a.z = fmaf(y.x, ws, a.z); a.w = fmaf(y.y, ws, a.w);
+  }
+  store_halves4<true>(out + static_cast<size_t>(t) * 2 * QS + head * D + 4 * lane, QS, make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv));
 }
 
 // Decode-step attention for a batch of sequences, with the per-head preparation fused in.  grid = (B, 8 kv

@@ -202,11 +202,10 @@ int ensure_gemm_attrs(std::string *err) {
       e = cudaFuncSetAttribute(qmk_pf::causal_attention_mma, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                qmk_pf::ATM_SMEM_BYTES);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(qmk_attn::Layout<false>::SMEM_BYTES));
+      e = cudaFuncSetAttribute(qmk_pf::causal_attention_split, cudaFuncAttributeMaxDynamicSharedMemorySize, qmk_pf::ATM_SMEM_BYTES);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(qmk_attn::Layout<true>::SMEM_BYTES));
+      e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(qmk_attn::SMEM_BYTES));
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(qmk_pf::decode_attention_ring, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                qmk_pf::DAR_SMEM_BYTES);
@@ -396,7 +395,7 @@ struct Workspace {                  // per device, allocated on first use, never
   __half *xn = nullptr, *attn = nullptr, *act = nullptr;
   unsigned int *status = nullptr;
   CUtensorMap map_xn, map_attn, map_act, map_qh;
-  CUtensorMap map_xn2, map_attn2, map_act2, map_qh2;   // split activations: rows of hi and lo halves
+  CUtensorMap map_xn2, map_attn2, map_act2;   // split activations: rows of hi and lo halves
   // batched decode: per-sequence state and the logits of one step
   int *positions = nullptr, *start_positions = nullptr;
   cudaStream_t gstream = nullptr;        // capture needs a non-default stream
@@ -487,7 +486,6 @@ int ensure_workspace(Workspace &w, int rows, bool *no_room = nullptr) {
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_xn2, w.xn, C, 2 * H, qmk_gemm::BM, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_attn2, w.attn, C, 2 * QS, qmk_gemm::BM, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_act2, w.act, C, 2 * I, qmk_gemm::BM, &err);
-  if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_qh2, w.qr, C, 2 * QS, qmk_gemm::BM, &err);
   if (rc != QMK_OK) {
     for (const Buffer &b : buffers)
       if (*b.at) { cudaFree(*b.at); *b.at = nullptr; }
@@ -582,7 +580,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
   qmk_internal::PrefillEnv env;
   int rc = qmk_internal::prefill_env(max_seq_len, stream, &env);
   if (rc != QMK_OK) return rc;
-  if (split) env.attn_tc = 1;   // (the mma.sync attention has no split form)
+  if (split) env.attn_tc = 0;   // (split operands have an attention kernel of their own)
   if (!token_ids_host || !embed_weight || !layer_weights || (!pk && (!k_cache || !v_cache)))
     return qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "prefill: null pointer argument");
   const int wfmt = env.wfmt;   // 0 fp16, 1 FP8-E4M3 rows, 2 NVFP4 rows
@@ -772,7 +770,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     const bool pdl_gemm = env.pdl != 0;
     qmk_tc::SplitActScope split_scope(split);
     const CUtensorMap &map_xn = split ? w.map_xn2 : w.map_xn, &map_attn = split ? w.map_attn2 : w.map_attn,
-                      &map_act = split ? w.map_act2 : w.map_act, &map_qh = split ? w.map_qh2 : w.map_qh;
+                      &map_act = split ? w.map_act2 : w.map_act;
     // two GEMM CTAs per SM: one's epilogue under the other's main loop (split activations take the SM's whole TMEM: one CTA)
     qmk_tc::RingBudgetScope ring_scope(split ? 0 : PREFILL_RING_BYTES);
     {
@@ -836,17 +834,27 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
                                     pk ? reinterpret_cast<const int2 *>(w.packed + PK_ROWS_OFF) : nullptr,
                                     pk ? reinterpret_cast<const unsigned long long *>(w.packed + PK_PTRS_OFF) : nullptr,
                                     static_cast<size_t>(l) * layer_stride,
-                                    env.attn_tc ? attn_scale * 1.4426950408889634f : 0.f, split ? 1 : 0));
+                                    env.attn_tc ? attn_scale * 1.4426950408889634f : 0.f));
       if (l == num_layers - 1) break;   // the cache is complete; nothing downstream of the last layer is kept
       if (env.attn_tc)
-        PF_CUDA(qmk_tc::launch_kernel(split ? qmk_attn::causal_attention_tc<true> : qmk_attn::causal_attention_tc<false>,
-                                      dim3(pk ? pk_items : (T + qmk_attn::TQ - 1) / qmk_attn::TQ * NQ), dim3(qmk_attn::THREADS),
-                                      split ? qmk_attn::Layout<true>::SMEM_BYTES : qmk_attn::Layout<false>::SMEM_BYTES, stream, map_qh,
-                                      map_kc, map_vc, l * NKV, w.attn, T,
+        PF_CUDA(qmk_tc::launch_kernel(qmk_attn::causal_attention_tc, dim3(pk ? pk_items : (T + qmk_attn::TQ - 1) / qmk_attn::TQ * NQ),
+                                      dim3(qmk_attn::THREADS), qmk_attn::SMEM_BYTES, stream, w.map_qh, map_kc, map_vc, l * NKV, w.attn, T,
                                       pos0, attn_scale, w.status, static_cast<unsigned long long>(env.timeout_ms) * 1000000ull,
                                       pk ? reinterpret_cast<const int4 *>(w.packed + PK_ITEMS_OFF) : nullptr,
                                       pk ? reinterpret_cast<const CUtensorMap *>(w.packed + PK_MAPS_OFF) : nullptr));
-      else
+      else if (split) {
+        const int qtiles = (T + ATM_Q - 1) / ATM_Q, ktiles = (pos0 + T + ATM_KEYS - 1) / ATM_KEYS;
+        // Two CTAs fit on an SM: fewer query tiles than that share out their keys, down to four key tiles each.  The partial
+        // outputs go where q, k and v were (their values are in the cache and in qr by now).
+        int splits = 2 * qmk_tc::gemm_sm_count() / (qtiles * NKV);
+        if (splits > ktiles / 4) splits = ktiles / 4;
+        if (splits > ATS_MAX_SPLITS) splits = ATS_MAX_SPLITS;
+        if (splits < 1 || static_cast<size_t>(splits) * T * NQ * ATS_PART > static_cast<size_t>(CHUNK) * QS) splits = 1;
+        PF_CUDA(qmk_tc::launch_kernel(causal_attention_split, dim3(qtiles, NKV, splits), dim3(ATM_THREADS), ATM_SMEM_BYTES, stream, w.qr,
+                                      kc, vc, w.attn, w.q, T, pos0, max_seq_len, attn_scale));
+        if (splits > 1)
+          PF_CUDA(qmk_tc::launch_kernel(merge_attention_splits, dim3(T), dim3(512), 0, stream, w.q, splits, w.attn, T));
+      } else
         PF_CUDA(qmk_tc::launch_kernel(causal_attention_mma, dim3((T + ATM_Q - 1) / ATM_Q, NKV), dim3(ATM_THREADS), ATM_SMEM_BYTES, stream,
                                       w.qr, kc, vc, w.attn, T, pos0, max_seq_len, attn_scale));
       {

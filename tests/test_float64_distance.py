@@ -112,10 +112,13 @@ def test_decoded_rows(C, fmt, sequences, bound):
     assert 0 < share[2] < bound * share[1]
 
 
-@pytest.mark.parametrize("fmt,kind,tokens,bound", [("fp16", "small", 1024, 2.0), ("fp8", "small", 1024, 2.0)])
+@pytest.mark.parametrize("fmt,kind,tokens,bound", [("fp16", "small", 1024, 1.3), ("fp8", "small", 1024, 1.3), ("fp16", "plain", 100, 1.4),
+                                                   ("fp16", "plain", 4096, 1.3), ("fp16", "peaky", 4096, 1.3), ("fp8", "plain", 4096, 1.3),
+                                                   ("fp8", "peaky", 4096, 1.3)])
 def test_prefilled_rows(C, fmt, kind, tokens, bound):
     """The ``prefill`` op in one pass against the same op as persistent steps on the CUDA cores (``set_fused(0)``).  SwiGLU
-    outputs near 1e-3 are where lo halves stored as they are meet the fp16 subnormals (ratio above 10 then)."""
+    outputs near 1e-3 are where lo halves stored as they are meet the fp16 subnormals (ratio above 10 then); attention on few
+    of many keys is where truncated sums of scores and outputs show (ratios of 2 and 3 at 4096 tokens)."""
     from Model.Qwen06B_architecture import Decoder
     engine_w, oracle_w = _model(fmt, kind)
     ids = S.make_prompt(tokens, seed=tokens, vocab_size=VOCAB)

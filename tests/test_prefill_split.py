@@ -180,3 +180,23 @@ def test_short_prompts_do_not_wait_for_a_chunked_pass(built_library):
     waits.sort()
     print(f"pass {sorted(passes)[len(passes) // 2] * 1e3:.1f} ms, refused short call {waits[20] * 1e3:.3f} / {waits[-1] * 1e3:.3f} ms")
     assert waits[20] < 0.1 * sorted(passes)[len(passes) // 2]
+
+
+@pytest.mark.parametrize("before,n", [(900, 5), (2300, 33), (700, 140), (64, 64)])
+def test_short_prompt_behind_a_long_context(built_library, before, n):
+    """Few query tiles share out their keys among CTAs and the partial outputs are added up: against the oracle, with the
+    bounds of the other rows here."""
+    from Model.Qwen06B_architecture import Decoder
+    w = S.make_weights(seed=22, num_layers=3, vocab_size=2048, norm_std=0.1, max_seq_len=16)
+    ids = S.make_prompt(before + n, seed=n, vocab_size=2048)
+    o = OracleDecoder(w, max_seq_len=2560)
+    o.prefill(ids)
+    eng = Decoder(weights=S.weights_to(w, "cuda"), verbose=False, max_seq_len=2560)
+    eng.prefill_ids(ids[:before])
+    eng.prefill_ids(ids[before:])
+    for got, want in ((eng._k_cache, o.k_cache), (eng._v_cache, o.v_cache)):
+        want = want[:, :, before:before + n].float()
+        diff = (got[:, :, before:before + n].float().cpu() - want).abs()
+        print(f"{before} + {n}: max {float(diff.max()):.2e} rms {float(diff.square().mean().sqrt()):.2e}")
+        ulp = want.abs().clamp(min=2.0) * 2.0 ** -10
+        assert bool((diff <= 2 * ulp).all()) and float(diff.square().mean().sqrt()) < 3.4e-4
