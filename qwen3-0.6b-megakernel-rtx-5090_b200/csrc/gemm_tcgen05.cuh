@@ -177,6 +177,7 @@ __device__ __forceinline__ void mma_f16_ss_onto_lo(uint32_t tmem_d, uint64_t des
       : "memory");
 }
 constexpr float LO_SCALE = 2048.0f;
+constexpr int STATUS_BEYOND = 3;   // status word: a split activation exceeded the range of a half
 // The truncation of a chain of four MMAs (64 products) takes 0.75 * 2^-23 off its sum on average, always towards zero
 // (measured on random fp16 operands; a chain of one 0.32, of eight 1.3; the scatter around it is 0.5).  Whoever adds such
 // sums up multiplies them by 1 + 2^-23 in the same rounded FMA: what is left is scatter, which averages out over the chains.
@@ -546,6 +547,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
               const float a0 = g0 / (1.0f + expf(-g0)) * acc[SB - BN + c + 2 * i], a1 = g1 / (1.0f + expf(-g1)) * acc[SB - BN + c + 2 * i + 1];
               const __half2 hi = __floats2half2_rn(a0, a1);
               const __half2 lo = __floats2half2_rn((a0 - __low2float(hi)) * LO_SCALE, (a1 - __high2float(hi)) * LO_SCALE);
+              if (!(fabsf(a0) <= 65504.0f && fabsf(a1) <= 65504.0f)) status[STATUS_BEYOND] = 1u;   // (the caller then takes another way)
               hi4[i] = *reinterpret_cast<const uint32_t *>(&hi);
               lo4[i] = *reinterpret_cast<const uint32_t *>(&lo);
             }

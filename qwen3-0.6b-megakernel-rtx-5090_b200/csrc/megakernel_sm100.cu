@@ -885,12 +885,13 @@ int prefill_unlocked(const int *token_ids_host, int num_tokens, const void *embe
   // every fp32 operand: the precision of the kernels below) instead of one persistent step per token: a pass over up to
   // a few hundred tokens takes 1.3-1.5 ms, a step without its LM head 0.42 ms.  31 tokens 13.0 -> 1.2 ms, 776 tokens
   // 349 -> 3.9 ms.  The pass works in 285 MB of its own: a process that has given its memory away takes the steps,
-  // and so does one that asked for the unfused kernel.
+  // and so do one that asked for the unfused kernel and a prompt with an activation above 65504, whose halves the pass
+  // cannot scale (an operand's largest value is known only when its kernel is done; the steps can, see operand_exponent).
   if (num_tokens >= SPLIT_PREFILL_MIN_TOKENS && e->fused > 0) {
-    bool no_room = false;
+    bool take_steps = false;
     rc = qmk_tc::prefill_split(token_ids_host, num_tokens, embed_weight, layer_weights, cos_table, sin_table, k_cache, v_cache,
-                               num_layers, start_position, max_seq_len, attn_scale, stream, &no_room);
-    if (!no_room) return rc;
+                               num_layers, start_position, max_seq_len, attn_scale, stream, &take_steps);
+    if (!take_steps) return rc;
   }
   if (num_tokens > e->tok_cap) {  // grow-only staging, as the reference keeps (megakernel_5090.cu:1303-1307)
     if (e->tok_dev) cudaFree(e->tok_dev);

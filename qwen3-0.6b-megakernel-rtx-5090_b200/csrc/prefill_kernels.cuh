@@ -57,6 +57,11 @@ __device__ __forceinline__ void store_halves4(__half *dst, int lo_off, float4 v)
   }
 }
 
+// Some value does not round to a finite half (or is none itself).
+__device__ __forceinline__ bool beyond_half4(float4 v) {
+  return !(fabsf(v.x) <= 65504.0f && fabsf(v.y) <= 65504.0f && fabsf(v.z) <= 65504.0f && fabsf(v.w) <= 65504.0f);
+}
+
 // x[t][:] = embedding row of token t as fp32.  grid = T, block = 256.  `wq`: 0 fp16 rows; 1 FP8-E4M3 rows (H bytes,
 // then a 16-byte trailer with the fp32 row scale); 2 NVFP4 rows (H / 2 bytes of e2m1 pairs, low nibble first, H / 16
 // e4m3 block scales, then the trailer with the fp32 tensor scale).
@@ -90,9 +95,11 @@ __global__ void embed_rows(const int *tokens, const void *embed, int wq, float *
 // Residual add + RMSNorm: x[t] += add[t] (if add), y[t] = fp16(x[t] * rstd * w).  grid = T, block = 256.
 // `add` may come as `nparts` (<= 4) partial matrices `part_stride` floats apart (split-K GEMM output): they are
 // added in index order.
-// SPLIT: y is [T][2 x H], the fp16 rounding of the result and the fp16 rounding of what it left.
+// SPLIT: y is [T][2 x H], the fp16 rounding of the result and the fp16 rounding of what it left (times LO_SCALE); `beyond` is
+// set where a result exceeds the halves' range.
 template <bool SPLIT>
-__global__ void add_rmsnorm_rows(float *x, const float *add, int nparts, size_t part_stride, const __half *w, __half *y) {
+__global__ void add_rmsnorm_rows(float *x, const float *add, int nparts, size_t part_stride, const __half *w, __half *y,
+                                 unsigned int *beyond) {
   __shared__ float red[8];
   pdl_wait();
   pdl_trigger();
@@ -122,6 +129,7 @@ __global__ void add_rmsnorm_rows(float *x, const float *add, int nparts, size_t 
   const float4 n = make_float4(v.x * rstd * __low2float(w01), v.y * rstd * __high2float(w01), v.z * rstd * __low2float(w23),
                                v.w * rstd * __high2float(w23));
   store_halves4<SPLIT>(y + static_cast<size_t>(t) * (SPLIT ? 2 * H : H) + k0, H, n);
+  if (SPLIT && beyond_half4(n)) *beyond = 1u;
 }
 
 // The same for long chunks: one WARP per row (grid = ceil(T / 8), block = 256), eight 16-byte pieces per lane, every
@@ -130,7 +138,8 @@ __global__ void add_rmsnorm_rows(float *x, const float *add, int nparts, size_t 
 // in another order than above: results agree to rounding, not bit for bit.)
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
-add_rmsnorm_rows_wide(float *x, const float *add, int nparts, size_t part_stride, const __half *w, __half *y, int T) {
+add_rmsnorm_rows_wide(float *x, const float *add, int nparts, size_t part_stride, const __half *w, __half *y, int T,
+                      unsigned int *beyond) {
   pdl_wait();
   pdl_trigger();
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -168,6 +177,7 @@ add_rmsnorm_rows_wide(float *x, const float *add, int nparts, size_t part_stride
     const float4 n = make_float4(v[i].x * rstd * __low2float(w01), v[i].y * rstd * __high2float(w01),
                                  v[i].z * rstd * __low2float(w23), v[i].w * rstd * __high2float(w23));
     store_halves4<SPLIT>(y + static_cast<size_t>(t) * (SPLIT ? 2 * H : H) + 4 * (lane + 32 * i), H, n);
+    if (SPLIT && beyond_half4(n)) *beyond = 1u;
   }
 }
 

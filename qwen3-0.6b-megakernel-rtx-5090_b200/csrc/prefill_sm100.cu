@@ -574,7 +574,7 @@ constexpr size_t PK_ROWS_OFF = 0, PK_ITEMS_OFF = 32768, PK_MAPS_OFF = 49152, PK_
 int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_weight, const LDGLayerWeight *layer_weights,
                  const void *cos_table, const void *sin_table, void *k_cache, void *v_cache, int num_layers,
                  int start_position, int max_seq_len, float attn_scale, cudaStream_t stream, const PackedSeqs *pk, bool split,
-                 bool *no_room = nullptr) {
+                 bool *take_steps = nullptr) {
   using namespace qmk_pf;
   if (num_tokens <= 0) return QMK_OK;
   qmk_internal::PrefillEnv env;
@@ -611,7 +611,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
   if (dev < 0 || dev >= 16) return qmk_internal::report(QMK_ERR_CUDA, "device index out of range");
   std::lock_guard<std::recursive_mutex> lock(g_ws_mu);
   Workspace &w = g_ws[dev];
-  rc = ensure_workspace(w, CHUNK, no_room);
+  rc = ensure_workspace(w, CHUNK, take_steps);
   if (rc == QMK_OK) rc = ensure_weight_maps(w, layer_weights, num_layers, wq, stream);
   if (rc != QMK_OK) return rc;
   // ---- packed prompts: rows = the sequences one after the other, each padded to whole 128-row tiles
@@ -781,8 +781,9 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     auto norm_rows = [&](const float *add, const __half *g) {
       if (T >= 256 && od_splits <= 2)
         return qmk_tc::launch_kernel(split ? add_rmsnorm_rows_wide<true> : add_rmsnorm_rows_wide<false>, dim3((T + 7) / 8), dim3(256), 0,
-                                     stream, w.x, add, od_splits, od_stride, g, w.xn, T);
-      return qmk_tc::launch_kernel(split ? add_rmsnorm_rows<true> : add_rmsnorm_rows<false>, dim3(T), dim3(256), 0, stream, w.x, add, od_splits, od_stride, g, w.xn);
+                                     stream, w.x, add, od_splits, od_stride, g, w.xn, T, w.status + qmk_gemm::STATUS_BEYOND);
+      return qmk_tc::launch_kernel(split ? add_rmsnorm_rows<true> : add_rmsnorm_rows<false>, dim3(T), dim3(256), 0, stream, w.x, add, od_splits, od_stride, g, w.xn,
+                                   w.status + qmk_gemm::STATUS_BEYOND);
     };
     for (int l = 0; l < num_layers; ++l) {
       const unsigned long long *r = rec.data() + static_cast<size_t>(l) * 12;
@@ -893,6 +894,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     return qmk_internal::report(static_cast<int>(host_status[0]) == 5 ? QMK_ERR_CUDA : static_cast<int>(host_status[0]),
                                 host_status[0] == 5 ? "prefill: dynamic shared memory of the attention kernel is not 1024-byte aligned"
                                                     : "prefill: a bounded device wait ran out");
+  if (split && host_status[qmk_gemm::STATUS_BEYOND] != 0) *take_steps = true;
   return QMK_OK;
 }
 }  // namespace
@@ -908,14 +910,15 @@ extern "C" int qmk_prefill_chunked(const int *token_ids_host, int num_tokens, co
 namespace qmk_tc {
 // The chunked pass with split activations, for qmk_prefill (fp32 activations at the precision of the token-serial kernels).
 // Locks: the caller takes prefill_lock() BEFORE the engine's lock and holds both - the order in which every other path
-// meets them (prefill_impl reports errors to the engine while it holds the workspace).  `no_room`: set, with nothing
-// launched or reported, where the workspace does not fit in memory.
+// meets them (prefill_impl reports errors to the engine while it holds the workspace).  `take_steps`: set, with
+// nothing reported, where the pass is not the way: the workspace does not fit in memory, or an activation exceeded the range
+// of its halves (65504; the cache rows are then to be written again).
 std::unique_lock<std::recursive_mutex> prefill_lock() { return std::unique_lock<std::recursive_mutex>(g_ws_mu); }
 int prefill_split(const int *token_ids_host, int num_tokens, const void *embed_weight, const LDGLayerWeight *layer_weights,
                   const void *cos_table, const void *sin_table, void *k_cache, void *v_cache, int num_layers, int start_position,
-                  int max_seq_len, float attn_scale, cudaStream_t stream, bool *no_room) {
+                  int max_seq_len, float attn_scale, cudaStream_t stream, bool *take_steps) {
   return prefill_impl(token_ids_host, num_tokens, embed_weight, layer_weights, cos_table, sin_table, k_cache, v_cache, num_layers,
-                      start_position, max_seq_len, attn_scale, stream, nullptr, true, no_room);
+                      start_position, max_seq_len, attn_scale, stream, nullptr, true, take_steps);
 }
 }  // namespace qmk_tc
 
@@ -1098,7 +1101,7 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
       static const int rec_slot[7] = {1, 2, 3, 6, 8, 9, 10};   // q, k, v, o, gate, up, down inside a layer record
       auto wp = [&](int j) { return reinterpret_cast<const void *>(r[rec_slot[j]]); };
       PF_CUDA(qmk_tc::launch_kernel(add_rmsnorm_rows<false>, dim3(B), dim3(256), 0, s, w.x, l > 0 ? w.down : nullptr, DOWN_SPLITS, PART,
-                                    reinterpret_cast<const __half *>(r[0]), w.xn));
+                                    reinterpret_cast<const __half *>(r[0]), w.xn, nullptr));
       {
         const CUtensorMap *maps[3] = {&wm(0), &wm(1), &wm(2)};
         float *const cs[3] = {w.q, w.k, w.v};
@@ -1124,7 +1127,7 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
                                            TILE_N, live, a_box, wq, wp(3))) != QMK_OK)
         return r2;
       PF_CUDA(qmk_tc::launch_kernel(add_rmsnorm_rows<false>, dim3(B), dim3(256), 0, s, w.x, w.o, O_SPLITS, PART,
-                                    reinterpret_cast<const __half *>(r[7]), w.xn));
+                                    reinterpret_cast<const __half *>(r[7]), w.xn, nullptr));
       if ((r2 = qmk_tc::launch_gemm_swiglu(w.map_xn_b, wm(4), wm(5), w.act, M, I, H, w.status, env.timeout_ms, s, &err, TILE_N,
                                            live, a_box, wq, wp(4), wp(5))) != QMK_OK)
         return r2;
@@ -1133,7 +1136,7 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
         return r2;
     }
     PF_CUDA(qmk_tc::launch_kernel(add_rmsnorm_rows<false>, dim3(B), dim3(256), 0, s, w.x, w.down, DOWN_SPLITS, PART,
-                                  static_cast<const __half *>(final_norm_weight), w.xn));
+                                  static_cast<const __half *>(final_norm_weight), w.xn, nullptr));
     // Without a logits dump the LM head's epilogue picks the largest logit of each 128-column tile itself and the
     // rows of logits (B x 608 KB per step) are never written
     const bool fused_pick = env.logits_out == nullptr;

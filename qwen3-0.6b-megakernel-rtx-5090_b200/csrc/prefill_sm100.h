@@ -90,7 +90,7 @@ int launch_gemm(const CUtensorMap &map_a, const CUtensorMap &map_b, float *C, in
 std::unique_lock<std::recursive_mutex> prefill_lock();
 int prefill_split(const int *token_ids_host, int num_tokens, const void *embed_weight, const LDGLayerWeight *layer_weights,
                   const void *cos_table, const void *sin_table, void *k_cache, void *v_cache, int num_layers, int start_position,
-                  int max_seq_len, float attn_scale, cudaStream_t stream, bool *no_room);
+                  int max_seq_len, float attn_scale, cudaStream_t stream, bool *take_steps);
 }  // namespace qmk_tc
 
 #endif  // QMK_PREFILL_SM100_H_

@@ -96,3 +96,25 @@ def test_decode(C, kind, fmt, sequences):
         o = OracleDecoder(oracle_w, max_seq_len=64)
         want, logits = o.generate_ids([first[b]], steps, keep_logits=True)
         _compare(f"{kind} {fmt} x {sequences}, sequence {b}", caches[b], (o.k_cache, o.v_cache), dump[b], logits, got[b], want, steps)
+
+
+@pytest.mark.parametrize("kind", ["swiglu", "norm", "query"])
+@pytest.mark.parametrize("fmt,tokens", [("fp16", 40), ("fp8", 40), ("fp16", 300)])
+def test_prefill(C, kind, fmt, tokens):
+    """The ``prefill`` op: queries are scaled by its attention kernel; the other two kinds send the prompt through the
+    persistent steps, which rewrite every row."""
+    from Model.Qwen06B_architecture import Decoder
+    engine_w, oracle_w = _model(kind, fmt)
+    ids, steps = S.make_prompt(tokens + 1, seed=tokens, vocab_size=VOCAB), 6
+    _check_reach(kind, oracle_w, ids[0])
+    eng = Decoder(weights=engine_w, tokenizer=S.StubTokenizer(-1, VOCAB), verbose=False, max_seq_len=320, weight_format=fmt)
+    dump = torch.zeros(steps, VOCAB, device="cuda")
+    C.set_logits_dump(dump)
+    try:
+        got = eng.generate_ids(ids, steps)
+    finally:
+        C.set_logits_dump(None)
+    o = OracleDecoder(oracle_w, max_seq_len=320)
+    want, logits = o.generate_ids(ids, steps, keep_logits=True)
+    _compare(f"{kind} {fmt}, prompt of {tokens}", (eng._k_cache, eng._v_cache), (o.k_cache, o.v_cache), dump, logits, got, want,
+             tokens + steps)
