@@ -209,7 +209,7 @@ struct Groups {
   const unsigned char *braw[MAX_GROUPS];
   uint32_t raw_pitch, raw_bs_off, raw_scale_off;
   // fp16 B matrices that hold the values of packed rows (expand_packed_rows): fp32 scale of every B row, multiplied into
-  // the accumulator like the scales of packed rows (null = none; FUSE: [0] gate, [1] up).  Single fp16 activations only.
+  // the accumulator like the scales of packed rows (RS kernels; FUSE: [0] gate, [1] up).  Single fp16 activations only.
   const float *row_scale[MAX_GROUPS] = {nullptr, nullptr, nullptr};
   // Ring geometry (ring_geometry()): stages and bytes from the ring's start to the barriers.
   int stages;
@@ -266,7 +266,9 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
       : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-template <int BN, bool FUSE = false, int WQ = 0, int AH = 1>
+// RS: fp16 B matrices with row scales (Groups::row_scale).  A kernel of its own: a run-time test of the pointers in the
+// epilogues of every fp16 GEMM cost a prefill pass 0.6 to 1 %.
+template <int BN, bool FUSE = false, int WQ = 0, int AH = 1, bool RS = false>
 __global__ void __launch_bounds__(threads_for(WQ, AH), 1)
 gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b0,
                    const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ CUtensorMap map_b2,
@@ -274,6 +276,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                    int selftest_no_loads) {
   static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 256, "N tiles of 32, 64, 128 or 256 columns");
   static_assert(!FUSE || BN <= 128, "the fused SwiGLU epilogue keeps two accumulators of at most 128 columns (one MMA of N = 256)");
+  static_assert(!RS || (WQ == 0 && AH == 1), "row scales belong to expanded matrices");
   static_assert(WQ == 0 || (FUSE ? 2 * BN : BN) <= 128, "packed weights: at most 128 B rows per stage (scales live in shared memory)");
   constexpr int SB = FUSE ? 2 * BN : BN;          // B rows held per stage / accumulator columns
   constexpr int NACC = AH == 2 ? 4 : 1;           // accumulators: one, or with split activations four that the K blocks take in turn
@@ -595,7 +598,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             if (WQ) {
               g0 *= s_rowscale[c * 16 + 2 * i]; g1 *= s_rowscale[c * 16 + 2 * i + 1];
               u0 *= s_rowscale[BN + c * 16 + 2 * i]; u1 *= s_rowscale[BN + c * 16 + 2 * i + 1];
-            } else if (groups.row_scale[0]) {
+            } else if (RS) {
               const float2 sg = __ldg(reinterpret_cast<const float2 *>(groups.row_scale[0] + n0 + c * 16) + i);
               const float2 su = __ldg(reinterpret_cast<const float2 *>(groups.row_scale[1] + n0 + c * 16) + i);
               g0 *= sg.x; g1 *= sg.y; u0 *= su.x; u1 *= su.y;
@@ -615,8 +618,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       __half *hrow = reinterpret_cast<__half *>(C) + static_cast<size_t>(row) * N + n0;   // (out_f16)
       const bool pick = groups.amax_val != nullptr;
       const bool f16 = groups.out_f16 != 0;
-      const float *rscale = grp == 0 ? groups.row_scale[0] : grp == 1 ? groups.row_scale[1] : groups.row_scale[2];
-      if (rscale) rscale += n0;
+      const float *rscale = RS ? (grp == 0 ? groups.row_scale[0] : grp == 1 ? groups.row_scale[1] : groups.row_scale[2]) + n0 : nullptr;
       float best = -INFINITY;
       int best_col = 0x7fffffff;
 #pragma unroll 1
@@ -625,7 +627,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(c * 32);
         tmem_ld32(taddr, r);
         tmem_ld_wait();
-        if (!WQ && rscale) {
+        if (RS) {
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
             const float4 sc = __ldg(reinterpret_cast<const float4 *>(rscale + c * 32 + i));

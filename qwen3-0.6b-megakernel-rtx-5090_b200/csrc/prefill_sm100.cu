@@ -157,11 +157,18 @@ bool pdl_active() { return t_pdl; }
 // The kernel for an N tile, epilogue and weight format, and its dynamic shared memory.
 using GemmKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const qmk_gemm::Groups,
                             int, int, unsigned int *, unsigned long long, int);
-template <int WQ>
+template <int WQ, bool RS = false>
 static GemmKernel gemm_kernel_wq(int bn, bool fuse) {
-  if (fuse) return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, true, WQ> : qmk_gemm::gemm_f16_tn_kernel<64, true, WQ>;
-  return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, false, WQ>
-                  : bn == 64 ? qmk_gemm::gemm_f16_tn_kernel<64, false, WQ> : qmk_gemm::gemm_f16_tn_kernel<128, false, WQ>;
+  if (fuse) return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, true, WQ, 1, RS> : qmk_gemm::gemm_f16_tn_kernel<64, true, WQ, 1, RS>;
+  return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, false, WQ, 1, RS>
+                  : bn == 64 ? qmk_gemm::gemm_f16_tn_kernel<64, false, WQ, 1, RS> : qmk_gemm::gemm_f16_tn_kernel<128, false, WQ, 1, RS>;
+}
+// (the widest tiles - 256 B rows per stage - exist for fp16 weights only)
+template <bool RS>
+static GemmKernel gemm_kernel_f16(int bn, bool fuse) {
+  if (fuse && bn == 128) return qmk_gemm::gemm_f16_tn_kernel<128, true, 0, 1, RS>;
+  if (!fuse && bn == 256) return qmk_gemm::gemm_f16_tn_kernel<256, false, 0, 1, RS>;
+  return gemm_kernel_wq<0, RS>(bn, fuse);
 }
 // Split activations: at most 128 B rows per stage, packed 64.
 static GemmKernel gemm_kernel_split(int bn, bool fuse, int wq) {
@@ -176,12 +183,11 @@ static bool box_n_ok(int box_n, bool fuse, int wq) {
   if (t_ah == 2) return wq < 2 && (box_n == 32 || box_n == 64 || box_n == 128) && rows <= split_max_rows(wq);
   return box_n == 32 || box_n == 64 || (box_n == 128 && (rows == 128 || wq == 0)) || (box_n == 256 && rows == 256 && wq == 0);
 }
-// (the widest tiles - 256 B rows per stage - exist for fp16 weights only; split activations for fp16 and FP8 weights)
-static GemmKernel gemm_kernel(int bn, bool fuse, int wq, int ah) {
+// (split activations exist for fp16 and FP8 weights; `scaled`: fp16 matrices with row scales)
+static GemmKernel gemm_kernel(int bn, bool fuse, int wq, int ah, bool scaled) {
   if (ah == 2) return gemm_kernel_split(bn, fuse, wq);
-  if (wq == 0 && fuse && bn == 128) return qmk_gemm::gemm_f16_tn_kernel<128, true>;
-  if (wq == 0 && !fuse && bn == 256) return qmk_gemm::gemm_f16_tn_kernel<256, false>;
-  return wq == 0 ? gemm_kernel_wq<0>(bn, fuse) : wq == 1 ? gemm_kernel_wq<1>(bn, fuse) : gemm_kernel_wq<2>(bn, fuse);
+  if (wq == 0) return scaled ? gemm_kernel_f16<true>(bn, fuse) : gemm_kernel_f16<false>(bn, fuse);
+  return wq == 1 ? gemm_kernel_wq<1>(bn, fuse) : gemm_kernel_wq<2>(bn, fuse);
 }
 static size_t gemm_smem(int bn, bool fuse, int wq, int ah) { return qmk_gemm::smem_bytes_for(fuse ? 2 * bn : bn, wq, ah); }
 
@@ -196,8 +202,9 @@ int ensure_gemm_attrs(std::string *err) {
       for (int wq = 0; wq < 4 - ah && e == cudaSuccess; ++wq)
         for (int fuse = 0; fuse < 2 && e == cudaSuccess; ++fuse)
           for (int bn = 32; bn <= (ah == 2 ? split_max_rows(wq) / (fuse ? 2 : 1) : (fuse ? 64 : 128) * (wq == 0 ? 2 : 1)) && e == cudaSuccess; bn *= 2)
-            e = cudaFuncSetAttribute(reinterpret_cast<const void *>(gemm_kernel(bn, fuse != 0, wq, ah)),
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gemm_smem(bn, fuse != 0, wq, ah)));
+            for (int scaled = 0; scaled < (wq == 0 && ah == 1 ? 2 : 1) && e == cudaSuccess; ++scaled)
+              e = cudaFuncSetAttribute(reinterpret_cast<const void *>(gemm_kernel(bn, fuse != 0, wq, ah, scaled != 0)),
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gemm_smem(bn, fuse != 0, wq, ah)));
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(qmk_pf::causal_attention_mma, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                qmk_pf::ATM_SMEM_BYTES);
@@ -299,7 +306,7 @@ int launch_gemm_grouped(const CUtensorMap &map_a, int ngroups, const CUtensorMap
   int rows = live_rows > 0 ? live_rows : M;   // rows the epilogue stores (the rest of the tile is padding)
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
   const size_t smem = set_ring(&gr, box_n, wq);
-  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah), grid, dim3(qmk_gemm::threads_for(wq, t_ah)), smem, stream,
+  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah, gr.row_scale[0] != nullptr), grid, dim3(qmk_gemm::threads_for(wq, t_ah)), smem, stream,
                                 map_a, b0, b1, b2, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
   return QMK_OK;
@@ -331,7 +338,7 @@ int launch_gemm_swiglu(const CUtensorMap &map_a, const CUtensorMap &map_gate, co
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
   const size_t smem = set_ring(&gr, 2 * box_n, wq);
-  cudaError_t e = launch_kernel(gemm_kernel(box_n, true, wq, t_ah), dim3(N / box_n, M / qmk_gemm::BM), dim3(qmk_gemm::threads_for(wq, t_ah)),
+  cudaError_t e = launch_kernel(gemm_kernel(box_n, true, wq, t_ah, gr.row_scale[0] != nullptr), dim3(N / box_n, M / qmk_gemm::BM), dim3(qmk_gemm::threads_for(wq, t_ah)),
                                 smem, stream, map_a, map_gate, map_up, map_up, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
   return QMK_OK;
@@ -362,7 +369,7 @@ int launch_gemm_splitk(const CUtensorMap &map_a, const CUtensorMap &map_b, float
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
   const size_t smem = set_ring(&gr, box_n, wq);
-  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah), dim3(N / box_n, M / qmk_gemm::BM, splits), dim3(qmk_gemm::threads_for(wq, t_ah)),
+  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah, gr.row_scale[0] != nullptr), dim3(N / box_n, M / qmk_gemm::BM, splits), dim3(qmk_gemm::threads_for(wq, t_ah)),
                                 smem, stream, map_a, map_b, map_b, map_b, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
   return QMK_OK;
