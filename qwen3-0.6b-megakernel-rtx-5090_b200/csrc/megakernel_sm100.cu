@@ -87,13 +87,42 @@ __global__ void wait_timeout_probe(const __grid_constant__ Params P, unsigned lo
 // arrays used in turn (read `parity`, write `parity ^ 1`), so that the CTA that stores the new hash cannot change
 // what the other CTAs of its group compare against.  A change confined to unsampled elements goes unnoticed:
 // callers that edit weights in place call qmk_invalidate_weights().
+// Launches of several sequences read the caller's matrices themselves before they had these copies, and notice every edit
+// still: kmajor_hash_kernel hashes all of the matrices in front of the check (294 MB of a 28-layer fp16 table, about 50 us per
+// launch beside 0.57 ms per step; every single-sequence step would pay a tenth).
 constexpr int PREP_SUB = 16;      // CTAs per matrix
 struct PrepArgs {
   const LayerW *layers;           // the caller's table (device)
   const qmkp::LayerT *out;        // destinations (device)
-  unsigned long long *fp;         // [2][2 * num_layers] hashes
+  unsigned long long *fp;         // [2][2 * num_layers] hashes of the samples, [2][2 * num_layers] of all bytes, [2 * num_layers] sums being formed
   int num_layers, wfmt, parity, force;
+  int all, all_parity;            // compare the hashes of all bytes too (kmajor_hash_kernel ran before)
 };
+__device__ __forceinline__ const unsigned char *prep_matrix(const PrepArgs &a, int m) {
+  return reinterpret_cast<const unsigned char *>((m & 1) ? a.layers[m >> 1].w_down : a.layers[m >> 1].wo);
+}
+__device__ __forceinline__ size_t prep_row_bytes(const PrepArgs &a, int m) {
+  const size_t K = (m & 1) ? I : QS;
+  return a.wfmt ? K + FP8_TRAILER : K * 2;
+}
+__global__ void __launch_bounds__(256) kmajor_hash_kernel(const PrepArgs a) {
+  const int m = blockIdx.y;
+  const uint4 *src = reinterpret_cast<const uint4 *>(prep_matrix(a, m));
+  const size_t n16 = prep_row_bytes(a, m) * H / 16;
+  unsigned long long sum = 0;
+#pragma unroll 4
+  for (size_t i = static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x; i < n16; i += static_cast<size_t>(PREP_SUB) * 256) {
+    const uint4 v = __ldg(src + i);
+    unsigned long long h = (static_cast<unsigned long long>(v.x) << 32 | v.y) * 0xD6E8FEB86659FD93ull;
+    h ^= (static_cast<unsigned long long>(v.z) << 32 | v.w) * 0xA0761D6478BD642Full;
+    h ^= (i + 1) * 0x9E3779B97F4A7C15ull;
+    h = (h ^ (h >> 29)) * 0xBF58476D1CE4E5B9ull;
+    sum += h ^ (h >> 32);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) atomicAdd(a.fp + 8 * a.num_layers + m, sum);
+}
 __global__ void __launch_bounds__(256) kmajor_prepare_kernel(const PrepArgs a) {
   __shared__ unsigned long long s_hash;
   __shared__ int s_redo;
@@ -101,9 +130,9 @@ __global__ void __launch_bounds__(256) kmajor_prepare_kernel(const PrepArgs a) {
   __shared__ unsigned char tile8[32][33];
   const int m = blockIdx.y, l = m >> 1, which = m & 1, t = threadIdx.x;
   const int K = which ? I : QS;                       // inputs of the projection = rows of the K-major copy
-  const unsigned char *src = reinterpret_cast<const unsigned char *>(which ? a.layers[l].w_down : a.layers[l].wo);
+  const unsigned char *src = prep_matrix(a, m);
   unsigned char *dst = reinterpret_cast<unsigned char *>(const_cast<void *>(which ? a.out[l].wd_t : a.out[l].wo_t));
-  const size_t in_row = a.wfmt ? static_cast<size_t>(K) + FP8_TRAILER : static_cast<size_t>(K) * 2;
+  const size_t in_row = prep_row_bytes(a, m);
   const size_t n16 = in_row * H / 16;
   if (t == 0) s_hash = reinterpret_cast<unsigned long long>(src) * 0x9E3779B97F4A7C15ull;
   __syncthreads();
@@ -120,8 +149,16 @@ __global__ void __launch_bounds__(256) kmajor_prepare_kernel(const PrepArgs a) {
   const unsigned long long hash = s_hash;
   const int M = 2 * a.num_layers;
   if (t == 0) {
-    s_redo = (a.force || a.fp[static_cast<size_t>(a.parity) * M + m] != hash) ? 1 : 0;
-    if (blockIdx.x == 0) a.fp[static_cast<size_t>(a.parity ^ 1) * M + m] = hash;
+    bool redo = a.force || a.fp[static_cast<size_t>(a.parity) * M + m] != hash;
+    unsigned long long *all = a.fp + 2 * M;
+    const unsigned long long now = a.all ? all[2 * M + m] : 0ull;
+    if (a.all) redo |= all[static_cast<size_t>(a.all_parity) * M + m] != now;
+    s_redo = redo ? 1 : 0;
+    if (blockIdx.x == 0) {
+      a.fp[static_cast<size_t>(a.parity ^ 1) * M + m] = hash;
+      if (a.all) all[static_cast<size_t>(a.all_parity ^ 1) * M + m] = now;
+      else if (redo) all[m] = all[M + m] = ~0ull;     // the copy is about to be one whose bytes nobody has hashed
+    }
   }
   __syncthreads();
   if (!s_redo) return;
@@ -211,7 +248,7 @@ struct Engine {
   unsigned long long *red = nullptr;   // the two residual sums
   struct Prepared {          // K-major copies of W_o / W_down of one caller table
     const void *table = nullptr;
-    int num_layers = 0, wfmt = 0, parity = 0, force = 1;
+    int num_layers = 0, wfmt = 0, parity = 0, all_parity = 0, force = 1;
     unsigned char *buf = nullptr;
     qmkp::LayerT *tbl = nullptr;
     unsigned long long *fp = nullptr;
@@ -357,8 +394,9 @@ void free_prepared(Engine::Prepared &p) {
 constexpr size_t MAX_PREPARED = 4;   // weight sets kept per device (a 28-layer fp16 set is 294 MB)
 
 // Finds or creates the K-major copies for the caller's layer table and enqueues the check-and-rebuild kernel.
-// `optional`: where they do not fit in memory, *out stays null instead of an error.
-int ensure_prepared(Engine *e, const Params &P, int wfmt, cudaStream_t stream, Engine::Prepared **out, bool optional = false) {
+// `several` (sequences): every byte of the matrices is checked, and where the copies do not fit in memory *out stays null
+// instead of an error.
+int ensure_prepared(Engine *e, const Params &P, int wfmt, cudaStream_t stream, Engine::Prepared **out, bool several = false) {
   Engine::Prepared *hit = nullptr;
   for (auto &p : e->prepared)
     if (p.table == P.layers && p.num_layers == P.num_layers && p.wfmt == wfmt) hit = &p;
@@ -378,12 +416,12 @@ int ensure_prepared(Engine *e, const Params &P, int wfmt, cudaStream_t stream, E
     const size_t ob = kmajor_o_bytes(wfmt), db = kmajor_d_bytes(wfmt);
     if (const cudaError_t err = cudaMalloc(&p.buf, (ob + db) * P.num_layers); err != cudaSuccess) {
       cudaGetLastError();
-      if (optional && err == cudaErrorMemoryAllocation) return QMK_OK;
+      if (several && err == cudaErrorMemoryAllocation) return QMK_OK;
       return fail(e, QMK_ERR_CUDA, std::string("cudaMalloc of the K-major copies: ") + cudaGetErrorString(err));
     }
     QMK_CUDA(e, cudaMalloc(&p.tbl, sizeof(qmkp::LayerT) * P.num_layers));
-    QMK_CUDA(e, cudaMalloc(&p.fp, sizeof(unsigned long long) * 4 * P.num_layers));
-    QMK_CUDA(e, cudaMemsetAsync(p.fp, 0, sizeof(unsigned long long) * 4 * P.num_layers, stream));
+    QMK_CUDA(e, cudaMalloc(&p.fp, sizeof(unsigned long long) * 10 * P.num_layers));
+    QMK_CUDA(e, cudaMemsetAsync(p.fp, 0, sizeof(unsigned long long) * 10 * P.num_layers, stream));
     std::vector<qmkp::LayerT> host(P.num_layers);
     for (int l = 0; l < P.num_layers; ++l) {
       host[l].wo_t = p.buf + (ob + db) * l;
@@ -403,6 +441,13 @@ int ensure_prepared(Engine *e, const Params &P, int wfmt, cudaStream_t stream, E
   a.wfmt = wfmt;
   a.parity = hit->parity;
   a.force = hit->force;
+  a.all = several ? 1 : 0;
+  a.all_parity = hit->all_parity;
+  if (several) {
+    QMK_CUDA(e, cudaMemsetAsync(hit->fp + 8 * P.num_layers, 0, sizeof(unsigned long long) * 2 * P.num_layers, stream));
+    qmk::kmajor_hash_kernel<<<dim3(qmk::PREP_SUB, 2 * P.num_layers), 256, 0, stream>>>(a);
+    hit->all_parity ^= 1;
+  }
   qmk::kmajor_prepare_kernel<<<dim3(qmk::PREP_SUB, 2 * P.num_layers), 256, 0, stream>>>(a);
   QMK_CUDA(e, cudaGetLastError());
   hit->parity ^= 1;

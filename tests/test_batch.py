@@ -202,3 +202,46 @@ def test_tensor_core_launch_matches_group_launch(C, fmt, ctas, lens):
     assert torch.equal(dumps[0], dumps[2]), "not reproducible run to run"
     assert torch.equal(dumps[0], dumps[1]) == (ctas == 100)
     assert diff < 1e-3 and max(err) < LOGIT_TOL
+
+
+@pytest.mark.parametrize("fmt", ["fp16", "fp8"])
+def test_every_in_place_edit_of_the_weights_is_noticed(C, fmt):
+    """A launch of several sequences multiplies K-major copies of W_o and W_down and checks all bytes of the caller's
+    matrices first: an edit that none of the sampled hashes of the single-sequence calls covers, the edit taken back behind a
+    single-sequence call, and one in the last row of W_down."""
+    import quantize as Q
+    vocab, steps = 2048, 6
+    w = S.make_weights(seed=51, num_layers=2, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    eng_w, ora_w = Q.quantize_weights_fp8(w) if fmt == "fp8" else (w, w)
+    dev = S.weights_to(eng_w, "cuda")
+    prompts = [[5], [900]]
+    try:
+        eng = _batch_engine(dict(dev), 2, 64, weight_format=fmt)
+        live = eng._base._weights["layer_weights"]
+
+        def rows():
+            eng.generate_ids(prompts, steps)
+            return [k[:, :, :steps].clone() for k in eng._k_caches]
+
+        def fresh():
+            other = _batch_engine({k: ([t.clone() for t in v] if isinstance(v, list) else v.clone()) for k, v in eng._base._weights.items()},
+                                  2, 64, weight_format=fmt)
+            other.generate_ids(prompts, steps)
+            return [k[:, :, :steps].clone() for k in other._k_caches]
+
+        def same(a, b):
+            return all(torch.equal(x, y) for x, y in zip(a, b))
+        first = rows()
+        wo, wd = live[6].view(torch.uint8), live[10].view(torch.uint8)
+        keep = wo[0, 80:96].clone()
+        wo[0, 80:96] = wo[1, 160:176]           # sixteen bytes between the first two samples of the first layer's W_o
+        edited = rows()
+        assert not same(first, edited) and same(edited, fresh())
+        eng._base.generate_ids([7], 3)
+        wo[0, 80:96] = keep
+        assert same(rows(), first)
+        wd[1023, 3040:3056] = wd[5, 64:80]
+        last = rows()
+        assert not same(last, first) and same(last, fresh())
+    finally:
+        C.set_weight_format("fp16")
