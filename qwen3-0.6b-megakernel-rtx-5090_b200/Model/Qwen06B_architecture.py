@@ -351,23 +351,24 @@ class BatchDecoder:
 
     def __init__(self, weights=None, tokenizer=None, num_sequences: int = 4, max_seq_len: int = MAX_SEQ_LEN,
                  verbose: bool = False, engine: str = "auto", **decoder_kw):
-        """``engine``: "persistent" (one megakernel launch, <= 4 sequences, fp32 activations), "gemm" (tcgen05
-        GEMMs per step, <= 128 sequences, fp16 GEMM operands; packed FP8 / NVFP4 matrices are expanded inside the
-        GEMMs) or "auto": persistent up to 4 sequences, gemm above (NVFP4: always gemm) - measured at 1024-token
-        contexts, us per step: 2 sequences 613 persistent, 4 sequences 812 against 1130 (FP8 rows 805 against 1275)."""
+        """``engine``: "persistent" (one megakernel launch, <= 4 sequences, activations as pairs of fp16 halves), "gemm"
+        (tcgen05 GEMMs per step, <= 128 sequences, fp16 GEMM operands; packed FP8 / NVFP4 matrices are expanded inside the
+        GEMMs) or "auto" (``auto_engine``)."""
         n = int(num_sequences)
-        if engine == "auto":
-            engine = "persistent" if n <= self.MAX_SEQUENCES and decoder_kw.get("weight_format", "fp16") != "nvfp4" else "gemm"
-        if engine not in ("persistent", "gemm"):
+        if engine not in ("auto", "persistent", "gemm"):
             raise ValueError("engine must be 'auto', 'persistent' or 'gemm'")
         limit = self.MAX_SEQUENCES if engine == "persistent" else self.MAX_GEMM_SEQUENCES
         if not 1 <= n <= limit:
             raise ValueError(f"num_sequences must be 1..{limit} for the {engine} engine")
-        self.engine = engine
         self.num_sequences = n
         # slot 0 owns the weights, tables and the first cache; the other slots only add caches
         self._base = Decoder(weights=weights, tokenizer=tokenizer, max_seq_len=max_seq_len, verbose=verbose,
                              **decoder_kw)
+        if engine == "auto":
+            engine = self.auto_engine(n, self._base.weight_format, self._base.vocab_size, self._base.max_seq_len,
+                                      qwen_megakernel_C.num_ctas() if n == self.MAX_SEQUENCES else 0,
+                                      torch.cuda.mem_get_info()[0])
+        self.engine = engine
         self.tokenizer = self._base.tokenizer
         self.max_seq_len = self._base.max_seq_len
         dev = self._base._embed_weight.device
@@ -388,6 +389,24 @@ class BatchDecoder:
         # Decode rounds of an overlapping scheduler must stay off the legacy default stream: work queued there
         # (this op's event wait lasts a whole round) orders itself against every blocking stream of the process.
         self._decode_stream = torch.cuda.Stream(device=dev) if self.supports_overlap else None
+
+    @classmethod
+    def auto_engine(cls, n: int, weight_format: str, vocab_size: int, max_seq_len: int, ctas: int, free_bytes: int) -> str:
+        """Persistent up to three sequences, gemm from five on (NVFP4 rows: always gemm).  Four: persistent where the launch
+        runs on the tensor cores - a grid of at least 112 CTAs, whole ring chunks of vocabulary, room for the K-major
+        copies; its group-per-sequence form takes 1.9 ms a step - and contexts end before the GEMM step overtakes it.
+        Measured, us per step of four fp16 sequences at 1024 / 4096 / 8000 tokens: 779 / 1129 / 1546 persistent, 1127 / 1331 /
+        1583 gemm (slopes 106 and 63 per 1000 tokens); FP8 rows 818 / 1117 / 1499 and 1281 / 1478 / 1727 (one long context
+        among short ones costs either less).  A four-slot serving job of prompts of 64 to 2048 tokens, 128 new ones each,
+        tensor-core prefill: 0.96 s persistent, prefills between the rounds; 1.36 s gemm with prefills beside them."""
+        if weight_format == "nvfp4" or n > cls.MAX_SEQUENCES:
+            return "gemm"
+        if n < cls.MAX_SEQUENCES or vocab_size % 128:      # (the GEMM step reads vocabularies of whole tiles only)
+            return "persistent"
+        fp8 = weight_format == "fp8"
+        tensor_cores = (112 <= ctas <= (160 if fp8 else 256) and vocab_size % (8 if fp8 else 4) == 0
+                        and free_bytes >= (160 if fp8 else 300) << 20)
+        return "persistent" if tensor_cores and max_seq_len <= (12288 if fp8 else 8192) else "gemm"
 
     def prefill_slot(self, b: int, ids: Sequence[int]) -> None:
         """Fill slot ``b``'s KV cache with ``ids`` from position 0 (the ``prefill`` op)."""

@@ -107,3 +107,20 @@ def test_build_rejects_a_stack_frame_in_a_decode_megakernel():
     bad = ok.replace("    8 bytes stack frame", "    408 bytes stack frame")
     with pytest.raises(RuntimeError, match="stack frame"):
         build.check_stack_frames(bad)
+
+
+def test_engine_choice_for_four_sequences():
+    """``BatchDecoder(engine="auto")`` with four sequences takes the persistent engine only where its launch runs on the
+    tensor cores and contexts stay below the crossover; three and five do not depend on any of it."""
+    from Model.Qwen06B_architecture import BatchDecoder
+    auto, room = BatchDecoder.auto_engine, 1 << 34
+    for fmt in ("fp16", "fp8"):
+        assert auto(4, fmt, 151936, 2048, 148, room) == "persistent"
+        assert auto(4, fmt, 151936, 2048, 111, room) == "gemm"           # smaller grid than the launch is built for
+        assert auto(4, fmt, 151936, 2048, 148, 100 << 20) == "gemm"      # no room for the K-major copies
+        assert auto(4, fmt, 151936, 16384, 148, room) == "gemm"
+        assert auto(4, fmt, 4104, 16384, 100, 0) == "persistent"         # the GEMM step does not read this vocabulary
+        assert auto(3, fmt, 151936, 32768, 0, 0) == "persistent" and auto(5, fmt, 151936, 64, 148, room) == "gemm"
+    assert auto(4, "fp16", 151936, 8320, 148, room) == "gemm" and auto(4, "fp8", 151936, 8320, 148, room) == "persistent"
+    assert auto(4, "fp8", 151936, 2048, 200, room) == "gemm" and auto(4, "fp16", 151936, 2048, 200, room) == "persistent"
+    assert [auto(n, "nvfp4", 151936, 2048, 148, room) for n in (1, 4, 9)] == ["gemm"] * 3

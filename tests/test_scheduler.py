@@ -329,3 +329,27 @@ def test_gpu_overlapped_prefill_matches_serial_scheduling(built_library, tiny_cf
         outs.append([f.result(timeout=0).tokens for f in futs])
         assert all(len(t) == n for t, (_, n) in zip(outs[-1], reqs))
     assert outs[0] == outs[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("overlap", [False, True])
+def test_gpu_four_slots_with_tensor_prefill(built_library, overlap):
+    """What a four-slot server runs: the persistent engine with prefills on the tensor cores between its rounds.  It offers no
+    overlap; a caller that asks for it all the same gets the same answers.  Each request's tokens equal those of the
+    single-sequence engine behind the same prefill."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from Model.Qwen06B_architecture import BatchDecoder, Decoder
+    vocab = 2048
+    w = S.weights_to(S.make_weights(seed=5, num_layers=2, vocab_size=vocab, norm_std=0.1, max_seq_len=16), "cuda")
+    tok = S.StubTokenizer(-1, vocab)
+    reqs = [(S.make_prompt(3 + (i * 37) % 300, seed=200 + i, vocab_size=vocab), 4 + (i * 5) % 23) for i in range(12)]
+    single = Decoder(weights=w, tokenizer=tok, verbose=False, max_seq_len=384, prefill_mode="tensor")
+    want = [single.generate_ids(ids, n) for ids, n in reqs]
+    eng = BatchDecoder(weights=w, tokenizer=tok, num_sequences=4, max_seq_len=384, prefill_mode="tensor")
+    assert eng.engine == "persistent" and not eng.supports_overlap
+    sch = ContinuousBatcher(eng, eos_token_id=None, quantum=8, overlap_prefill=overlap, packed_prefill=False)
+    futs = [sch.submit(ids, n) for ids, n in reqs]
+    sch.run_until_idle()
+    sch.stop()
+    assert [f.result(timeout=0).tokens for f in futs] == want
