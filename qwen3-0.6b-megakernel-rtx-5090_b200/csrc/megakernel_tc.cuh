@@ -135,15 +135,24 @@ __device__ __forceinline__ void mma_16816_zero(float (&d)[4], const uint32_t (&a
                : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
-// c += A . B.  The tensor core truncates the accumulator it is given after every step, always towards zero: a chain of
-// MMAs loses more of a sum than rounded fp32 adds of the same products do.  So every product starts from zero and is added
-// in registers.
+// c += A . B in the tensor core.  It truncates the accumulator it is given after every step, always towards zero: a long
+// chain of MMAs loses more of a sum than rounded fp32 adds of the same products do.  So a chain is at most four MMAs long (64
+// products), and the chains are added up in registers.  Four MMAs of 11-bit operands take 0.75 * 2^-23 off their sum on
+// average (one 0.32, eight 1.3; measured on random operands, the scatter around it is 0.5): the adds multiply by
+// UNSHRINK_F16.  e4m3 weights (0.06 per MMA) are best off with one product per add.
 __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// c += A . B in registers.
+__device__ __forceinline__ void mma_add_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   float d[4];
   mma_16816_zero(d, a, b0, b1);
 #pragma unroll
   for (int i = 0; i < 4; ++i) c[i] += d[i];
 }
+constexpr float UNSHRINK_F16 = 1.0f + 1.0f / 8388608.0f;
 
 __device__ __forceinline__ void ldsm_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
@@ -197,7 +206,7 @@ __device__ __forceinline__ void e4m3x4_half2x2(uint32_t four, uint32_t &first, u
 // One warp: rows of the 16-row tile that starts at ring chunk `first` (valid rows <= 16), k-step pairs [p0, p1).
 // Leaves the 16 row sums of that k range in part[0..15] (sequence b: part[16 b..]) and hands the tile's chunks back with `units` each.
 // Lanes 0..3 each wait for one of the tile's chunks (the vote that follows orders the copied bytes before every
-// lane's loads); two accumulators halve the chain of dependent MMAs.
+// lane's loads).
 __device__ __forceinline__ void tile_task(const Params &P, const Ctx &c, uint32_t first, int valid_rows, int p0, int p1,
                                           float *part, int units, int fslot = 70) {
   const int nch = (valid_rows + CH_ROWS - 1) / CH_ROWS;
@@ -211,25 +220,39 @@ __device__ __forceinline__ void tile_task(const Params &P, const Ctx &c, uint32_
   int lr = (c.lane & 7) + ((c.lane >> 3) & 1) * 8;      // tile row whose address this lane supplies
   if (lr >= valid_rows) lr = 0;                         // rows past the end repeat row 0 (their sums are not used)
   const uint32_t a_addr = weight_rows(c, first + static_cast<uint32_t>(lr / CH_ROWS)) + (lr % CH_ROWS) * ROW_PITCH + (c.lane >> 4) * 16;
-  float acc0[4] = {0.f, 0.f, 0.f, 0.f}, acc1[4] = {0.f, 0.f, 0.f, 0.f};
-  if (ok) {
+  float sum[4] = {0.f, 0.f, 0.f, 0.f};
+  if (ok && FP8_ROWS) {   // r: rows 0..7 / 8..15 x inputs 0..15, then inputs 16..31; four consecutive inputs per lane
+    float odd[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 2
     for (int p = p0; p < p1; ++p) {
-      uint32_t a0[4], a1[4];
+      uint32_t a0[4], a1[4], r[4];
       const uint4 b = b_pair(c, p);
-      if (FP8_ROWS) {   // r: rows 0..7 / 8..15 x inputs 0..15, then inputs 16..31; four consecutive inputs per lane
-        uint32_t r[4];
-        ldsm_x4(a_addr + p * 32, r);
-        e4m3x4_half2x2(r[0], a0[0], a0[2]);
-        e4m3x4_half2x2(r[1], a0[1], a0[3]);
-        e4m3x4_half2x2(r[2], a1[0], a1[2]);
-        e4m3x4_half2x2(r[3], a1[1], a1[3]);
-      } else {
-        ldsm_x4(a_addr + p * 64, a0);
-        ldsm_x4(a_addr + p * 64 + 32, a1);
+      ldsm_x4(a_addr + p * 32, r);
+      e4m3x4_half2x2(r[0], a0[0], a0[2]);
+      e4m3x4_half2x2(r[1], a0[1], a0[3]);
+      e4m3x4_half2x2(r[2], a1[0], a1[2]);
+      e4m3x4_half2x2(r[3], a1[1], a1[3]);
+      mma_add_16816(sum, a0, b.x, b.y);
+      mma_add_16816(odd, a1, b.z, b.w);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum[i] += odd[i];
+  } else if (ok) {
+    for (int p = p0; p < p1; p += 2) {
+      float acc[4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (u == 1 && p + 1 == p1) break;
+        uint32_t a0[4], a1[4];
+        const uint4 b = b_pair(c, p + u);
+        ldsm_x4(a_addr + (p + u) * 64, a0);
+        ldsm_x4(a_addr + (p + u) * 64 + 32, a1);
+        if (u == 0) mma_16816_zero(acc, a0, b.x, b.y);
+        else mma_16816(acc, a0, b.x, b.y);
+        mma_16816(acc, a1, b.z, b.w);
       }
-      mma_16816(acc0, a0, b.x, b.y);
-      mma_16816(acc1, a1, b.z, b.w);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sum[i] = fmaf(acc[i], UNSHRINK_F16, sum[i]);
     }
   }
   QMK_FINE(fslot + 5);
@@ -243,8 +266,8 @@ __device__ __forceinline__ void tile_task(const Params &P, const Ctx &c, uint32_
   if (c.lane < nch) mbar_arrive_n(c.empty((first + static_cast<uint32_t>(c.lane)) % NSLOTS), static_cast<uint32_t>(units));
   if ((c.lane & 3) < TC_SEQS) {   // quad b of a fragment: the hi and lo columns of sequence b
     part += (c.lane & 3) * 16;
-    part[c.lane >> 2] = fmaf(acc0[1] + acc1[1], LO_INV, acc0[0] + acc1[0]) * sc_top;
-    part[(c.lane >> 2) + 8] = fmaf(acc0[3] + acc1[3], LO_INV, acc0[2] + acc1[2]) * sc_bot;
+    part[c.lane >> 2] = fmaf(sum[1], LO_INV, sum[0]) * sc_top;
+    part[(c.lane >> 2) + 8] = fmaf(sum[3], LO_INV, sum[2]) * sc_bot;
   }
 }
 
@@ -485,7 +508,8 @@ __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __ha
         mma_16816(sc, a0, qf[p][0], qf[p][1]);
         mma_16816(sc2, a1, qf[p][2], qf[p][3]);
       }
-      float s_top = fmaf(sc[1] + sc2[1], LO_INV, sc[0] + sc2[0]) * sc_quad, s_bot = fmaf(sc[3] + sc2[3], LO_INV, sc[2] + sc2[2]) * sc_quad;
+      float s_top = fmaf(sc[0] + sc2[0], UNSHRINK_F16, (sc[1] + sc2[1]) * LO_INV) * sc_quad,
+            s_bot = fmaf(sc[2] + sc2[2], UNSHRINK_F16, (sc[3] + sc2[3]) * LO_INV) * sc_quad;
       if (rowq >= nrow) s_top = -INFINITY;
       if (rowq + 8 >= nrow) s_bot = -INFINITY;
       float cm = fmaxf(s_top, s_bot);
@@ -521,7 +545,7 @@ __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __ha
       for (int t = 0; t < 8; ++t) {
         uint32_t a[4];
         ldsm_x4_trans(v_row + (t >> 2) * KV_BOX + ((((t & 3) * 32) + v_off) ^ v_xor), a);
-        mma_16816(acc[t], a, b0, b1);
+        mma_add_16816(acc[t], a, b0, b1);
       }
     }
     __syncwarp();
@@ -776,8 +800,8 @@ __device__ __forceinline__ void slice_tiles(const uint32_t (&arow)[2], const uin
   }
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
-    mma_16816(acc[u], a[u], bq[0], bq[1]);
-    if (two) mma_16816(acc[u], a2[u], bq[2], bq[3]);
+    mma_add_16816(acc[u], a[u], bq[0], bq[1]);
+    if (two) mma_add_16816(acc[u], a2[u], bq[2], bq[3]);
   }
 }
 

@@ -83,12 +83,12 @@ def flips(weights, ids, k_rows, v_rows, first):
         x = x + (g * torch.sigmoid(g) * (h @ w[9].T)) @ w[10].T
 
 
-@pytest.mark.parametrize("fmt,sequences,bound", [("fp8", 1, 1.1), ("fp8", 2, 1.1), ("fp16", 1, 1.3), ("fp16", 2, 1.3), ("fp16", 4, 1.3)])
+@pytest.mark.parametrize("fmt,sequences,bound", [("fp8", 1, 1.1), ("fp8", 2, 1.1), ("fp16", 1, 1.2), ("fp16", 2, 1.2), ("fp16", 4, 1.2)])
 def test_decoded_rows(C, fmt, sequences, bound):
     """Tensor-core decode against the CUDA-core launches.  About 2400 flips of 1.5 million values a sequence on either side,
     2 % of counting noise each: 1.1 is above four sigma of it.  fp16 weights: the products of 11-bit operands lose a little
-    inside the MMA itself (16 of them aligned and truncated to its internal width), measured 1.1 to 1.2.  With accumulators
-    handed from MMA to MMA these ratios were 1.2 (FP8 rows) and 1.6 (fp16 rows)."""
+    inside the MMA itself (16 of them aligned and truncated to its internal width), measured 1.00 to 1.08.  With accumulators
+    handed from MMA to MMA over whole rows these ratios were 1.13 to 1.26 (FP8 rows) and 1.6 to 1.7 (fp16 rows)."""
     from Model.Qwen06B_architecture import BatchDecoder, Decoder
     engine_w, oracle_w = _model(fmt)
     prompts = [S.make_prompt(1024 - 7 * b, seed=b, vocab_size=VOCAB) for b in range(sequences)]
