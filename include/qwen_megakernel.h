@@ -210,16 +210,20 @@ int qmk_set_decode_attention(int tensor_core);
  * plainly).  Same results either way; negative keeps. */
 int qmk_set_step_overlap(int enabled);
 
-/* Kernel choice for one sequence (qmk_decode / qmk_generate / qmk_prefill); negative keeps a value.
+/* Kernel choice of qmk_decode / qmk_generate / qmk_prefill and qmk_generate_batch; negative keeps a value.
  *  fused  2 (default) or 1: the fused kernel - the O and down projections run as split-K slices on the CTAs that
  *         produced their inputs, and the two residual sums of a layer are all-reduced in 64-bit integer
  *         accumulators (four cross-CTA hand-overs per layer).  It reads K-major copies of W_o and W_down that
  *         the library makes from the caller's matrices (294 MB for 28 fp16 layers) on the first call with a
  *         layer table and re-checks by sampled hashes on every call.  Grids below 74 CTAs and
- *         qmk_generate_static use the unfused kernel (six hand-overs, no copies).  0: always unfused.
+ *         qmk_generate_static use the unfused kernel (six hand-overs, no copies).  0: always unfused, for
+ *         prompts of qmk_prefill too.
  *         2 multiplies weight rows on the tensor cores (mma.sync tiles of 16 rows, the fp32 activation vector
- *         split into two fp16 columns); it needs fp16 weights and a vocabulary that is a multiple of 4, and falls
- *         back to 1 (CUDA-core row products, any format) otherwise.
+ *         split into two fp16 columns; sums in fp32 registers): fp16 rows with a vocabulary that is a multiple of 4
+ *         on grids of 96 to 256 CTAs, FP8 rows with a multiple of 8 on 96 to 160; falls back to 1 (CUDA-core row
+ *         products, any format) otherwise.  qmk_generate_batch: see there.
+ *  Numbers: residual sums are fixed point, exact to 2^-28 and good for |x| < 3.3e7; other activations have the
+ *  range of fp32 (an operand above 65504, the end of fp16, is scaled by a power of two for the MMAs).
  *  red_copies  1 or 2 accumulator copies per sum (2 halves the same-address add queue, doubles the words read).
  * The reference has neither (its layer is eight grid barriers, megakernel_5090.cu:879-915). */
 int qmk_set_fused(int fused, int red_copies);
@@ -254,6 +258,11 @@ int qmk_generate(
     void *block_max_vals, void *block_max_idxs, int *output_log, int num_layers,
     int start_position, int max_seq_len, float attn_scale, int eos_token_id,
     int synchronize, cudaStream_t stream);
+/* Prompts of up to three tokens run as persistent decode steps.  Longer ones run as one chunked pass (the kernels of
+ * qmk_prefill_chunked, with every fp32 operand split into two fp16 halves): cache rows equal those of the steps up to
+ * rounding, not bit for bit.  The pass needs 285 MB of scratch, allocated on the first such call per device; where that
+ * does not fit, where an activation exceeds 65504 and under qmk_set_fused(0) the prompt runs as steps, which need 8 MB.
+ * max_ctas and the row products chosen with qmk_set_fused(1) concern the steps only.  Blocks until done. */
 int qmk_prefill(
     const int *token_ids_host, int num_tokens, const void *embed_weight,
     const struct LDGLayerWeight *layer_weights, const void *final_norm_weight,
@@ -263,7 +272,15 @@ int qmk_prefill(
 
 /* Greedy decode of up to four independent sequences in ONE persistent launch:
  * every weight row is streamed from HBM once per step and used by all
- * sequences; the math warps of each CTA are split into one group per sequence.
+ * sequences, which are columns of the same tensor-core products.  That launch
+ * reads the K-major copies described at qmk_set_fused (every byte of the
+ * caller's W_o and W_down is checked on each call, so edits in place need no
+ * qmk_invalidate_weights here) and its residual sums are fixed point, for
+ * |x| < 3.3e7.  Grids below 96 CTAs (three and four sequences: 112) or above 256
+ * (FP8 rows: 160), vocabularies that are no multiple of 4 (FP8: 8),
+ * qmk_set_fused(0 / 1) and a device without room for the copies take a launch
+ * without either, in which the math warps of a CTA are split into one group per
+ * sequence (about twice the time).
  * The reference decodes one sequence per launch (megakernel_5090.cu:1216-1260
  * launch_ldg_generate_nosync); this is its multi-sequence form, the building
  * block for the batched configurations.  Host arrays of num_sequences entries:
@@ -316,9 +333,11 @@ int qmk_generate_static(
  * of once per token, megakernel_5090.cu:1324-1350), with row-wise kernels for RMSNorm, per-head QK-norm +
  * RoPE + cache write, causal attention over the cache, and SwiGLU between them.  Same arguments, cache
  * layout, position rule and blocking behaviour as qmk_prefill; all three weight formats (packed FP8 / NVFP4 matrices
- * stay packed in HBM and are expanded to fp16 tiles inside the GEMM, see qmk_gemm_packed_tn).  GEMM operands are rounded to fp16 (the
- * decode kernel keeps fp32 activations), so cache rows agree with qmk_prefill's to fp16 rounding, not
- * bit for bit.  Scratch (about 230 MB) is allocated on the first call per device. */
+ * stay packed in HBM and are expanded to fp16 tiles inside the GEMM, see qmk_gemm_packed_tn, or once per layer in chunks
+ * of 384 rows and more).  GEMM operands are rounded to fp16 (the
+ * decode kernels keep 22 bits of fp32 activations), so cache rows agree with qmk_prefill's to fp16 rounding, not
+ * bit for bit.  Scratch (285 MB, shared with qmk_prefill; 32 MB more for expanded layers where they fit) is allocated on
+ * the first call per device. */
 int qmk_prefill_chunked(
     const int *token_ids_host, int num_tokens, const void *embed_weight,
     const struct LDGLayerWeight *layer_weights, const void *cos_table, const void *sin_table,

@@ -172,7 +172,8 @@ class Decoder:
             raise ValueError("weight_format must be 'fp16', 'fp8' or 'nvfp4'")
         self.weight_format = weight_format
         # "serial": the prefill op (fp32 activations: prompts of up to three tokens token by token, longer ones in one
-        # pass with every operand split into two fp16 halves, equal to decoding the prompt up to rounding);
+        # pass with every operand split into two fp16 halves, equal to decoding the prompt up to rounding; token by token
+        # too where the pass has no room or an activation exceeds the halves' range);
         # "tensor": chunked prefill on the tensor cores (fp16 GEMM operands; packed matrices are expanded inside the
         # GEMMs or, for long chunks, once per layer)
         if prefill_mode not in ("serial", "tensor"):
@@ -337,7 +338,7 @@ class Decoder:
 
 
 class BatchDecoder:
-    """Greedy decode of up to four independent sequences per launch.
+    """Greedy decode of several independent sequences: up to four per persistent launch, up to 128 on the GEMM path.
 
     The reference decodes one sequence per persistent launch
     (Model/Qwen06B_architecture.py:398-448); this wraps the multi-sequence form of the same kernel

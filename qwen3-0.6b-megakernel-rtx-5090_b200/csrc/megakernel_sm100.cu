@@ -574,7 +574,7 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
     P.spin_sleep_ns = e->fused_sleep_ns;
     kernel = reinterpret_cast<const void *>(qmk::qwen3_decode_megakernel_fused);
     // row products on the tensor cores: rows owned in units of one ring chunk (four fp16 rows, eight fp8 rows).  fp8:
-    // 724 -> 533 us per token at 1024-token contexts against the CUDA-core kernel, which stays for the grids and
+    // 724 -> 493 us per token at 1024-token contexts against the CUDA-core kernel, which stays for the grids and
     // vocabularies outside these limits.
     const qmk_fused_tc::Build &tc = qmk_fused_tc::build(e->wfmt);
     if (e->fused >= 2 && P.vocab % tc.rows_per_chunk == 0 && grid >= tc.min_ctas && grid <= tc.max_ctas) {
@@ -928,8 +928,8 @@ int prefill_unlocked(const int *token_ids_host, int num_tokens, const void *embe
   if (rc != QMK_OK) return rc;
   // Prompts of more than a few tokens go through the chunked tensor-core pass with split activations (hi + lo fp16 halves of
   // every fp32 operand: the precision of the kernels below) instead of one persistent step per token: a pass over up to
-  // a few hundred tokens takes 1.3-1.5 ms, a step without its LM head 0.42 ms.  31 tokens 13.0 -> 1.2 ms, 776 tokens
-  // 349 -> 3.9 ms.  The pass works in 285 MB of its own: a process that has given its memory away takes the steps,
+  // a hundred tokens takes 1.7-1.8 ms, a step without its LM head 0.42 ms.  31 tokens 13.0 -> 1.7 ms, 776 tokens
+  // 349 -> 5.1 ms.  The pass works in 285 MB of its own: a process that has given its memory away takes the steps,
   // and so do one that asked for the unfused kernel and a prompt with an activation above 65504, whose halves the pass
   // cannot scale (an operand's largest value is known only when its kernel is done; the steps can, see operand_exponent).
   if (num_tokens >= SPLIT_PREFILL_MIN_TOKENS && e->fused > 0) {

@@ -31,8 +31,8 @@
 // (xf_offset).  A packed row is 1040 bytes in memory, which is a conflict-free pitch in shared memory too: a chunk
 // is eight rows and ONE bulk copy (four 2 KB rows: four copies).  Row scales multiply the finished sums (they sit in
 // the rows' trailers); the per-output scales of the K-major O / down copies travel as one more chunk of those phases.
-// Measured after: 533 us per token (a request of 1024 + 64 tokens 48.8 -> 36.6 ms).  Against float64 the cache rows are as
-// far off as the CUDA-core kernel's (V rows of the first layer that round differently: 0.086 % and 0.084 %).
+// Measured after: 493 us per token (128 tokens from a 1024-token context).  Against float64 the cache rows are nearer than the
+// CUDA-core kernel's (later layers' values that round differently: 0.154 % and 0.167 %).
 
 namespace QMK_NS {
 #if QMK_MAX_SEQ == 1 && defined(QMK_TC_BUILD)
@@ -277,8 +277,9 @@ __device__ __forceinline__ void tile_task(const Params &P, const Ctx &c, uint32_
 // 1024 inputs.  Grids of at least FUSED_MIN_CTAS CTAs have at most 6 tiles per phase: one task per warp.
 // fp16 rows: the tiles run on from the gate into the up rows (148 CTAs: 40 to 48 rows are three tiles, where the gate and
 // the up rows by themselves were two each, the second of them half empty; the MMAs of a sub-partition issue one at a time):
-// 523 / 535 / 568 -> 518 / 531 / 563 us per token at 64 / 1024 / 4096-token contexts.  fp8 rows gained nothing at 1024 and
-// lost 1 % at 64 and stay apart (their row conversions weigh more than the MMAs).
+// 523 / 535 / 568 -> 518 / 531 / 563 us per token at 64 / 1024 / 4096-token contexts (both with full lines of sums, see
+// RED_GROUP).  fp8 rows gained nothing at 1024 and lost 1 % at 64 and stay apart (their row conversions weigh more than the
+// MMAs).
 constexpr bool GU_ONE_RUN = !FP8_ROWS;
 __device__ inline void build_tile_tasks(TileTask *tasks, int *nkb_out, int groups, int nch) {
   const int tpg = (nch + TILE_CH - 1) / TILE_CH, T = groups * tpg;

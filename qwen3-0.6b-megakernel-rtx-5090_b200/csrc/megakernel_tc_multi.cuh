@@ -9,10 +9,11 @@
 // words read back, cache rows.
 // The launch it replaces (megakernel_batch.cuh, which stays for grids outside this kernel's range) gives each sequence a
 // group of warps that convert and multiply every weight for themselves, and has six hand-overs per layer.
-// Measured, us per step at 64 / 1024 / 2048-token contexts: two fp16 sequences 581 / 613 / 635, three 683 / 750 / 847, four
-// 712 / 812 / 928, four with FP8 rows 730 / 805 / 909 (the group launch: two 1137 / 1317 at 64 / 1024; four 1655 / 1942;
-// the GEMM step: four fp16 1086 / 1130 / 1196, four FP8 1224 / 1275 / 1341, with fp16-rounded activations).  Distance from
-// float64 as before: 0.68 % of layer 1's V rows that two sequences decode round differently (0.70 % with the group launch).
+// Measured, us per step at 64 / 1024 / 2048-token contexts: two fp16 sequences 565 / 582 / 614, four 693 / 770 / 904, four
+// with FP8 rows 656 / 740 / 863 (the group launch: two 1137 / 1317 at 64 / 1024; four 1655 / 1942; the GEMM step: four fp16
+// 1080 / 1126 / 1189, four FP8 1230 / 1281 / 1345, with fp16-rounded activations).  Share of later layers' cache values
+// that round to another fp16 than float64's, 1024 tokens: two and four fp16 sequences 0.156 and 0.161 % (group launch 0.147
+// and 0.150), two with FP8 rows 0.152 (0.151).
 
 namespace QMK_NS {
 #if QMK_MAX_SEQ == 1 && defined(QMK_TC_BUILD) && QMK_TC_SEQS > 1
@@ -255,7 +256,8 @@ __device__ __forceinline__ void normalise_seqs(const Ctx &c, const float (&v)[TC
 
 // Contributions that may still be missing from the watched word when a warp goes on to fetch all its words: with several
 // sequences the adds drain for longer, and the fetch's round trip fits into the rest of it (four sequences, us per step at
-// 64 / 1024 / 2048 tokens: 0: 812 / 932 / 1034, 16: 771 / 896 / 981, 48: 725 / 844 / 953, with the watch in front of the merge 712 / 812 / 928; 147: no better).  One sequence gains nothing.
+// 64 / 1024 / 2048 tokens: 0: 812 / 932 / 1034, 16: 771 / 896 / 981, 48: 725 / 844 / 953, with the watch in front of the merge 712 / 812 / 928; 147: no better; all with full lines of sums, see RED_GROUP).
+// One sequence gains nothing.
 constexpr unsigned long long SUM_SLACK = 48;
 // red_wait_norm for all sequences: which = 0: x1, 1: x2 (kept as the residual of the next layer's O slice, x).
 __device__ __noinline__ void red_wait_norm_seqs(const Params &P, const Ctx c, int which, uint32_t use, const __half *norm_w) {

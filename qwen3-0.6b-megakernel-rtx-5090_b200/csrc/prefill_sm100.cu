@@ -772,7 +772,9 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     // programmatic dependent, a decode launched after the prefill had returned produced run-to-run different logits
     // although every cache row compared bit-identical afterwards (an uninitialised read in the decode kernel, since
     // mended: see its attention).  With the mend fp16 prefills are right with every kernel dependent (109 tokens 1.48 ->
-    // 1.30 ms), packed prompts of expanded layers are not (rel 0.16): a hazard not yet found.
+    // 1.30 ms), packed prompts of expanded layers are not (rel 0.16): expand_packed_rows has no wait of its own.  As a
+    // dependent it would overwrite the expanded matrices under the GEMMs of the layer before, and the row kernel behind it
+    // would wait for it alone and not for the sums it adds.  Launched plainly, as here, both are in order.
     qmk_tc::PdlScope pdl_scope(false);
     const bool pdl_gemm = env.pdl != 0;
     qmk_tc::SplitActScope split_scope(split);

@@ -249,7 +249,7 @@ def _golden_ctx4096():
 def test_benchmark_configuration_matches_golden(C, prefill_mode):
     """The configuration bench.py times (full model, seed 0, make_prompt(4096, seed 0), max_seq_len 4352):
     first 8 greedy tokens identical to the oracle's golden file, their top-8 logits within 3e-2.  Both prefill
-    paths: the token-serial op (fp32 activations) and the chunked tensor-core prefill (fp16 GEMM operands)."""
+    paths: the prefill op (fp32 activations, in one pass of split operands) and the chunked tensor-core prefill (fp16 GEMM operands)."""
     g = _golden_ctx4096()
     cfg = g["config"]
     ids = S.make_prompt(cfg["prompt_len"], seed=cfg["prompt_seed"])

@@ -1,4 +1,4 @@
-"""Tensor-core chunked prefill against the CPU oracle and against the token-serial prefill.
+"""Tensor-core chunked prefill against the CPU oracle and against the ``prefill`` op.
 
 The chunked path rounds GEMM operands to fp16 (the decode kernel and the oracle keep fp32 activations), so
 the bar is a tolerance, stated here: KV cache rows within 2e-2 max-abs of the oracle's (values are O(1),
@@ -79,7 +79,8 @@ def test_packed_fp8_weights_prefill_on_the_tensor_cores(C):
 
 
 def test_appends_at_a_start_position_and_agrees_with_serial_prefill(C):
-    """Prefill in two calls (the second starts at position 300) and compare with the token-serial op."""
+    """Prefill in two calls (the second starts at position 300) and compare with the ``prefill`` op in one call, and with the
+    same op as persistent steps (``set_fused(0)``), which share no kernel with either."""
     vocab, L = 2048, 1024
     w = S.make_weights(seed=13, num_layers=2, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
     ids = S.make_prompt(900, seed=3, vocab_size=vocab)
@@ -93,6 +94,14 @@ def test_appends_at_a_start_position_and_agrees_with_serial_prefill(C):
     verr = float((a._v_cache[:, :, :900].float() - b._v_cache[:, :, :900].float()).abs().max())
     print(f"two-call tensor prefill vs serial prefill: K {kerr:.2e} V {verr:.2e}")
     assert kerr < CACHE_TOL and verr < CACHE_TOL
+    b.reset()
+    C.set_fused(fused=0)
+    try:
+        b.prefill_ids(ids)
+    finally:
+        C.set_fused(fused=2)
+    for mine, steps in ((a._k_cache, b._k_cache), (a._v_cache, b._v_cache)):
+        assert float((mine[:, :, :900].float() - steps[:, :, :900].float()).abs().max()) < CACHE_TOL
 
 
 @pytest.mark.parametrize("n_prompt", [150, 900])
