@@ -182,8 +182,8 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   }
   pdl_wait();   // queries and this chunk's cache rows come from the kernel launched just before
   pdl_trigger();
-  // the query tile and the K ring's first fill go out at once (thread 0 is the K producer and has just initialised
-  // the barriers itself); a CTA's fixed costs weigh as much as its first key tiles
+  // the query tile and the K ring's first fill go out at once (warp 0 has just initialised the barriers); a CTA's fixed costs weigh as much as its first key tiles
+  if (warp == 0) __syncwarp();
   auto load_tile = [&](bool is_v, int j) {
     const int s = j % STAGES;
     const uint32_t full = is_v ? v_full(s) : k_full(s);
@@ -193,20 +193,21 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     tma_load_3d(d0, is_v ? mv : mk, 0, j * TK, layer_head0 + g, full);
     tma_load_3d(d1, is_v ? mv : mk, 64, j * TK, layer_head0 + g, full);
   };
-  int k_prefilled = 0;
-  if (items != nullptr && lane == 0 && (warp == 0 || warp == 3 + 4 * CHAINS)) {
+  const int k_prefilled = ntiles < STAGES ? ntiles : STAGES;
+  // (the same thread of a warp every time: the election is deterministic)
+  if (items != nullptr && (warp == 0 || warp == 3 + 4 * CHAINS) && elect_one()) {
     // descriptors written by a copy before this launch: the loading threads make them visible to their TMA unit
     asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(reinterpret_cast<uint64_t>(mk)) : "memory");
     asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(reinterpret_cast<uint64_t>(mv)) : "memory");
   }
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
     // the query tile: fp16, already times scale * log2 e (the softmax is an exp2), as two [128 x 64] boxes in the
     // K-major 128-byte-swizzled layout the score MMAs read; rows past the live ones hold other tokens' or stale
     // finite values and are never stored
     bar_expect_tx(q_full, Q_BYTES);
     tma_load_2d(base, &map_q, head * D, q0, q_full);
     tma_load_2d(base + TQ * 128, &map_q, head * D + 64, q0, q_full);
-    for (; k_prefilled < STAGES && k_prefilled < ntiles; ++k_prefilled) load_tile(false, k_prefilled);
+    for (int j = 0; j < k_prefilled; ++j) load_tile(false, j);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -215,7 +216,7 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   const uint32_t tmem_o0 = tmem_base + 256u;  // S buffer b at tmem_base + 64 b, O of chain c at tmem_o0 + 128 c
 
   if (warp == 0 || warp == 3 + 4 * CHAINS) {
-    if (lane == 0) {                       // ---- producers: the K ring (warp 0) and the V ring, tiles of 64 rows
+    if (elect_one()) {                     // ---- producers: the K ring (warp 0) and the V ring, tiles of 64 rows
       const bool is_v = warp != 0;
       int issued = is_v ? 0 : k_prefilled;
       for (int j = issued; j < ntiles; ++j) {
@@ -236,7 +237,7 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {                       // ---- score MMAs: S of tiles 2 p and 2 p + 1 as one N = 128 product
+    if (elect_one()) {                     // ---- score MMAs: S of tiles 2 p and 2 p + 1 as one N = 128 product
       bool ok = true;
       const int npairs = (ntiles + 1) >> 1;
       for (int p = 0; p < npairs && ok; ++p) {
@@ -262,7 +263,7 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       }
     }
   } else if (warp == 2 + 4 * CHAINS) {
-    if (lane == 0) {                       // ---- P . V MMAs, tiles in order (chains alternate)
+    if (elect_one()) {                     // ---- P . V MMAs, tiles in order (chains alternate)
       bool ok = true;
       for (int j = 0; j < ntiles && ok; ++j) {
         const int c = j & 1, n = j >> 1;   // chain, and the tile's index within it

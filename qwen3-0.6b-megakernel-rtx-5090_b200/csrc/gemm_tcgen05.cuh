@@ -102,6 +102,16 @@ __device__ __forceinline__ unsigned long long gtime() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
+// One thread of a converged warp.  tcgen05.mma, tcgen05.commit and the TMA copies take their operands from uniform registers:
+// in a region entered through elect.sync the compiler knows that one thread is active, under `lane == 0` it does not and
+// wraps every such instruction in a loop over the active lanes.  K loop of the decode step's q/k/v GEMM (64 MMAs of
+// 128 x 32 x 16, all operands resident): 5.5 us under `lane == 0`, 3.65 elected, 2.4 with the ring's slot and parity counted
+// instead of divided.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+  return ok != 0;
+}
 __device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
@@ -122,14 +132,14 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
 // Bounded wait: false when the budget ran out or another role already gave up.
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, unsigned int *status,
                                          unsigned long long budget_ns) {
-  if (bar_try(bar, parity)) return true;
-  const unsigned long long t0 = gtime();
-  uint32_t it = 0;
-  for (;;) {
+  unsigned long long t0 = 0;   // (the clock is read from the 64th try on: most waits end before)
+  for (uint32_t it = 1;; ++it) {
     if (bar_try(bar, parity)) return true;
-    if ((++it & 63u) == 0u) {
+    if ((it & 63u) == 0u) {
       if (*abort_flag) return false;
-      if (gtime() - t0 > budget_ns) {
+      const unsigned long long t = gtime();
+      if (t0 == 0) t0 = t;
+      if (t - t0 > budget_ns) {
         *abort_flag = 1;
         atomicCAS(status, 0u, 4u);
         return false;
@@ -159,9 +169,9 @@ __device__ __forceinline__ void mma_f16_ss(uint32_t tmem_d, uint64_t desc_a, uin
       "{\n\t"
       ".reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
       "}\n"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(IDESC), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(IDESC), "r"(accumulate)
       : "memory");
 }
 // D = A . B + D * 2^-11: the first product of hi halves on an accumulator that holds the products of the lo halves, which
@@ -328,10 +338,10 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   const int kcol = WQ ? static_cast<int>(RAW_ROW) : BK;          // B-map columns (bytes for packed rows) per K block
   const uint32_t b_dst = WQ ? TILE_A + (FUSE ? 2u : 1u) * TILE_B_BYTES : TILE_A;   // where the B copies land in a stage
   const uint32_t b_dst_step = WQ ? TILE_RAW_BYTES : TILE_B_BYTES;
-  // the first fill of the ring needs no free-slot wait: thread 0 issues it before the CTA-wide barrier below, so
+  // the first fill of the ring needs no free-slot wait: it is issued before the CTA-wide barrier below, so
   // that the first TMA round trip overlaps the TMEM allocation
   const int prologue = selftest_no_loads ? 0 : (kblocks < STAGES ? kblocks : STAGES);
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map_b)) : "memory");
     if (FUSE) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_b1)) : "memory");
@@ -386,7 +396,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {                       // ---- producer
+    if (elect_one()) {                     // ---- producer
       pdl_wait();                          // A is the preceding kernel's output
       // Only now may the NEXT kernel of the chain be scheduled (to set itself up and request its weight tiles behind
       // this one): a kernel that let its dependents go before its own predecessor had completed put three kernels in
@@ -397,11 +407,12 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         tma_load_2d(base + kb * STAGE_BYTES, &map_a, (kb0 + kb) * BK, m0, a_landed(kb));
         if (AH == 2) tma_load_2d(base + kb * STAGE_BYTES + TILE_A_BYTES, &map_a, K + (kb0 + kb) * BK, m0, a_landed(kb));
       }
-      int issued = prologue;
+      int issued = prologue, s = prologue == STAGES ? 0 : prologue;   // slot of K block kb
+      uint32_t parity = 0;                                            // of the use before it, whose MMAs free the slot
       // self test of the bounded waits: the loads are never issued, so the MMA thread's first wait runs out
       for (int kb = prologue; kb < (selftest_no_loads ? 0 : kblocks); ++kb) {
-        const int s = kb % STAGES;
-        if (kb >= STAGES && !bar_wait(empty(s), ((kb / STAGES) - 1) & 1, abort_flag, status, budget_ns)) break;
+        // (past the prologue the ring is full: kb >= STAGES)
+        if (!bar_wait(empty(s), parity, abort_flag, status, budget_ns)) break;
         if (*abort_flag) break;
         bar_expect_tx(b_landed(s), WQ ? b_tx : a_tx + b_tx);
         if (WQ) bar_expect_tx(a_full(s), a_tx);
@@ -410,6 +421,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         tma_load_2d(base + s * STAGE_BYTES + b_dst, map_b, (kb0 + kb) * kcol, n0, b_landed(s));
         if (FUSE) tma_load_2d(base + s * STAGE_BYTES + b_dst + b_dst_step, &map_b1, (kb0 + kb) * kcol, n0, b_landed(s));
         issued = kb + 1;
+        if (++s == STAGES) { s = 0; parity ^= 1u; }
       }
       // after an abort the copies already issued must land before the CTA can exit
       if (*abort_flag) {
@@ -422,17 +434,18 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {                       // ---- MMA issuer
+    if (elect_one()) {                     // ---- MMA issuer
       bool ok = true;
-      for (int kb = 0; kb < kblocks && ok; ++kb) {
-        const int s = kb % STAGES;
-        ok = bar_wait(full(s), (kb / STAGES) & 1, abort_flag, status, budget_ns) &&
-             (!WQ || bar_wait(a_full(s), (kb / STAGES) & 1, abort_flag, status, budget_ns)) &&
+      int s = 0;                           // slot and parity of K block kb
+      uint32_t parity = 0;
+      const uint64_t da0 = smem_desc_sw128(base), db0 = smem_desc_sw128(base + TILE_A);
+      uint64_t da = da0, db = db0;         // (a ring ends below 2^18 bytes: the slot's offset does not leave the address field)
+      for (int kb = 0; kb < kblocks; ++kb) {
+        ok = bar_wait(full(s), parity, abort_flag, status, budget_ns) &&
+             (!WQ || bar_wait(a_full(s), parity, abort_flag, status, budget_ns)) &&
              (AH == 1 || kb < NACC || bar_wait(blk_free(kb % NACC), (kb / NACC - 1) & 1, abort_flag, status, budget_ns));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint64_t da = smem_desc_sw128(base + s * STAGE_BYTES);
-        const uint64_t db = smem_desc_sw128(base + s * STAGE_BYTES + TILE_A);
         // 16 halves = 32 bytes = 2 descriptor address units per K step
         // FUSE: the up tile follows the gate tile in shared memory (BN more rows of the same 8-row-group layout),
         // so one MMA of N = 2 BN covers both and leaves gate in columns [0, BN), up in [BN, 2 BN)
@@ -448,6 +461,9 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           mma_commit(blk_full(kb % NACC));
         }
         mma_commit(empty(s));               // the stage is free once these MMAs have read it
+        da += STAGE_BYTES >> 4;
+        db += STAGE_BYTES >> 4;
+        if (++s == STAGES) { s = 0; parity ^= 1u; da = da0; db = db0; }
       }
       if (ok && AH == 1) mma_commit(acc_full);   // accumulator complete
     }
@@ -462,10 +478,12 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       // reached use u of a stage before anyone had waited for use u - 1 would run ahead on stale data.
       const int cw = warp - 2, part = cw >> 2;
       bool live = !selftest_no_loads;
+      int s = -1;
+      uint32_t parity = 0;
       for (int kb = 0; kb < kblocks && live; ++kb) {
-        const int s = kb % STAGES;
+        if (++s == STAGES) { s = 0; parity ^= 1u; }
         if ((s & 3) != (cw & 3)) continue;
-        live = __all_sync(0xffffffffu, bar_wait(raw_full(s), (kb / STAGES) & 1, abort_flag, status, budget_ns));
+        live = __all_sync(0xffffffffu, bar_wait(raw_full(s), parity, abort_flag, status, budget_ns));
         if (!live) break;
         const uint32_t btile = base + s * STAGE_BYTES + TILE_A;
         const uint32_t rawt = base + s * STAGE_BYTES + b_dst;
