@@ -181,7 +181,6 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   pdl_wait();   // queries and this chunk's cache rows come from the kernel launched just before
-  pdl_trigger();
   // the query tile and the K ring's first fill go out at once (warp 0 has just initialised the barriers); a CTA's fixed costs weigh as much as its first key tiles
   if (warp == 0) __syncwarp();
   auto load_tile = [&](bool is_v, int j) {
@@ -212,6 +211,8 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  // behind the TMEM allocation: the next kernel's CTAs allocate too, and hold what they have while they wait for this kernel
+  pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_o0 = tmem_base + 256u;  // S buffer b at tmem_base + 64 b, O of chain c at tmem_o0 + 128 c
 

@@ -718,6 +718,8 @@ struct ExpandArgs {
 constexpr int EXPAND_THREADS = 256;
 template <int WQ>
 __global__ void __launch_bounds__(EXPAND_THREADS) expand_packed_rows(const __grid_constant__ ExpandArgs a) {
+  pdl_wait();      // (the layer before has multiplied the matrices this overwrites, and has made the sums the next kernel adds)
+  pdl_trigger();
   const int row = blockIdx.x * (EXPAND_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= a.first_row[7]) return;
   const unsigned char *src = nullptr;

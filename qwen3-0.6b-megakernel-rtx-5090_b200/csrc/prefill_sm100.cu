@@ -246,8 +246,11 @@ static bool set_packed(qmk_gemm::Groups *gr, int wq, int K, int ngroups, const v
 // Ring depth of a launch (see qmk_gemm::ring_geometry): `sb` = B rows per stage; returns the dynamic shared memory.
 thread_local float *t_amax_val = nullptr;   // the next single-matrix GEMM of this thread leaves (value, column) pairs here
 thread_local int *t_amax_idx = nullptr;
-static size_t set_ring(qmk_gemm::Groups *gr, int sb, int wq) {
-  const qmk_gemm::RingGeometry g = qmk_gemm::ring_geometry(sb, wq, t_ring_budget, t_ah);
+// A launch of at most one CTA per SM takes the full depth whatever the budget: nothing of its own shares the SM, and with the
+// three stages of a 128-wide tile that fit 96 KB its K loop waits for L2.  Prompts of 31 / 109 / 500 / 1000 tokens with every
+// kernel of the chain a programmatic dependent 1.07 / 1.24 / 1.79 / 2.42 -> 0.91 / 1.06 / 1.56 / 2.10 ms (2000: no such launch).
+static size_t set_ring(qmk_gemm::Groups *gr, int sb, int wq, long ctas = 0) {
+  const qmk_gemm::RingGeometry g = qmk_gemm::ring_geometry(sb, wq, ctas > sm_count() ? t_ring_budget : 0, t_ah);
   gr->stages = g.stages;
   gr->ring_bytes = g.ring_bytes;
   return g.smem_bytes;
@@ -305,7 +308,7 @@ int launch_gemm_grouped(const CUtensorMap &map_a, int ngroups, const CUtensorMap
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
   int rows = live_rows > 0 ? live_rows : M;   // rows the epilogue stores (the rest of the tile is padding)
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
-  const size_t smem = set_ring(&gr, box_n, wq);
+  const size_t smem = set_ring(&gr, box_n, wq, static_cast<long>(grid.x) * grid.y);
   cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah, gr.row_scale[0] != nullptr), grid, dim3(qmk_gemm::threads_for(wq, t_ah)), smem, stream,
                                 map_a, b0, b1, b2, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
@@ -337,7 +340,7 @@ int launch_gemm_swiglu(const CUtensorMap &map_a, const CUtensorMap &map_gate, co
   int rows = live_rows > 0 ? live_rows : M;
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
-  const size_t smem = set_ring(&gr, 2 * box_n, wq);
+  const size_t smem = set_ring(&gr, 2 * box_n, wq, static_cast<long>(N / box_n) * (M / qmk_gemm::BM));
   cudaError_t e = launch_kernel(gemm_kernel(box_n, true, wq, t_ah, gr.row_scale[0] != nullptr), dim3(N / box_n, M / qmk_gemm::BM), dim3(qmk_gemm::threads_for(wq, t_ah)),
                                 smem, stream, map_a, map_gate, map_up, map_up, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
@@ -368,7 +371,7 @@ int launch_gemm_splitk(const CUtensorMap &map_a, const CUtensorMap &map_b, float
   int rows = live_rows > 0 ? live_rows : M;
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
-  const size_t smem = set_ring(&gr, box_n, wq);
+  const size_t smem = set_ring(&gr, box_n, wq, static_cast<long>(N / box_n) * (M / qmk_gemm::BM) * splits);
   cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah, gr.row_scale[0] != nullptr), dim3(N / box_n, M / qmk_gemm::BM, splits), dim3(qmk_gemm::threads_for(wq, t_ah)),
                                 smem, stream, map_a, map_b, map_b, map_b, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
@@ -750,7 +753,10 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
         return qmk_tc::launch_gemm(a, wmap_for(l, j, box_n), c, Mrows, H, K, box_n, w.status, env.timeout_ms, stream, &err, live, 0, wq,
                                    wptr(l, j));
       }
-      const int box_n = split_box(128, 64);
+      // the narrowest tile whose CTAs fit on the SMs at once: a 128-row chunk has 32 CTAs of 128 columns, whose epilogues alone
+      // took 2.1 us (31 / 109 / 250 tokens 0.91 / 1.06 / 1.27 -> 0.85 / 0.94 / 1.21 ms; from 500 tokens on the tile is the same)
+      int box_n = 32;
+      while (box_n < split_box(128, 64) && static_cast<long>(Mrows / qmk_gemm::BM) * (H / box_n) * od_splits > qmk_tc::gemm_sm_count()) box_n *= 2;
       return qmk_tc::launch_gemm_splitk(a, wmap_for(l, j, box_n), c, Mrows, H, K, od_splits, w.status, env.timeout_ms, stream, &err, box_n,
                                         live, 0, wq, wptr(l, j));
     };
@@ -766,17 +772,13 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
       if (rc != QMK_OK) break;
     }
     PF_CUDA(cudaMemcpyAsync(w.tokens, token_ids_host + c0, sizeof(int) * T, cudaMemcpyHostToDevice, stream));
-    // Programmatic dependent launch for the GEMMs only: their set-up and first ring fill of WEIGHT tiles run under the
-    // tail of the kernel before them (every kernel here lasts 2-6 us longer than its CTAs run; 2048 tokens 4.11 -> 3.81
-    // ms).  The row kernels and the attention kernel launch plainly: with EVERY kernel of this chain launched as a
-    // programmatic dependent, a decode launched after the prefill had returned produced run-to-run different logits
-    // although every cache row compared bit-identical afterwards (an uninitialised read in the decode kernel, since
-    // mended: see its attention).  With the mend fp16 prefills are right with every kernel dependent (109 tokens 1.48 ->
-    // 1.30 ms), packed prompts of expanded layers are not (rel 0.16): expand_packed_rows has no wait of its own.  As a
-    // dependent it would overwrite the expanded matrices under the GEMMs of the layer before, and the row kernel behind it
-    // would wait for it alone and not for the sums it adds.  Launched plainly, as here, both are in order.
-    qmk_tc::PdlScope pdl_scope(false);
-    const bool pdl_gemm = env.pdl != 0;
+    // Every kernel behind the first launches as a programmatic dependent: its set-up (and a GEMM's first ring fill of WEIGHT
+    // tiles) runs under the tail of the kernel before it.  In order are, with each kernel waiting for its predecessor before
+    // its first dependent read and any write: the residual rows and sums; the expanded matrices of a packed layer
+    // (expand_packed_rows waits for the last GEMM that multiplies them, and the first GEMM that requests tiles of them ahead
+    // of its own wait is launched after the row kernel between has seen the expansion complete).  109 / 1000 / 2000 tokens,
+    // GEMMs alone dependent -> all: 1.41 / 2.59 / 3.80 -> 1.24 / 2.42 / 3.74 ms.
+    qmk_tc::PdlScope pdl_scope(env.pdl != 0);
     qmk_tc::SplitActScope split_scope(split);
     const CUtensorMap &map_xn = split ? w.map_xn2 : w.map_xn, &map_attn = split ? w.map_attn2 : w.map_attn,
                       &map_act = split ? w.map_act2 : w.map_act;
@@ -799,8 +801,6 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
       __half *kc = pk ? nullptr : static_cast<__half *>(k_cache) + l * layer_stride;
       __half *vc = pk ? nullptr : static_cast<__half *>(v_cache) + l * layer_stride;
       if (wq != wfmt) {
-        // (launched plainly, and so is the row kernel behind it: it runs after the layer before has read the buffers, and
-        // the GEMMs, which request weight tiles before they wait for their predecessor, start after it)
         qmk_gemm::ExpandArgs a;
         size_t at = 0;
         a.first_row[0] = 0;
@@ -829,10 +829,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
         // its length (9.8 of 26 us at 2048 rows with fp32); the consumer below rounds to fp16 anyway
         // (split activations: fp32, the operands downstream are not rounded to fp16)
         qmk_tc::set_out_f16(!split);
-        {
-          qmk_tc::PdlScope g(pdl_gemm);
-          rc = gemm_group(map_xn, l, 3, js, cs, ns, M, H, T);
-        }
+        rc = gemm_group(map_xn, l, 3, js, cs, ns, M, H, T);
         qmk_tc::set_out_f16(false);
         if (rc != QMK_OK) break;
       }
@@ -867,29 +864,20 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
       } else
         PF_CUDA(qmk_tc::launch_kernel(causal_attention_mma, dim3((T + ATM_Q - 1) / ATM_Q, NKV), dim3(ATM_THREADS), ATM_SMEM_BYTES, stream,
                                       w.qr, kc, vc, w.attn, T, pos0, max_seq_len, attn_scale));
-      {
-        qmk_tc::PdlScope g(pdl_gemm);
-        rc = gemm_od(map_attn, l, 3, w.o, M, QS, T);
-      }
+      rc = gemm_od(map_attn, l, 3, w.o, M, QS, T);
       if (rc != QMK_OK) break;
       PF_CUDA(norm_rows(w.o, reinterpret_cast<const __half *>(r[7])));
       {
         const int box_gu = split_box(qmk_tc::gemm_box_n_fused(M, I), 32);
         // three of these CTAs per SM instead of two: their epilogue (two TMEM reads, SiLU, fp16 pack) is the long part
         qmk_tc::RingBudgetScope gu_scope(split ? 0 : M >= 1024 ? GATE_UP_RING_BYTES : PREFILL_RING_BYTES);
-        {
-          qmk_tc::PdlScope g(pdl_gemm);
-          const int js[2] = {4, 5};
-          row_scales(js, 2);
-          rc = qmk_tc::launch_gemm_swiglu(map_xn, wmap_for(l, 4, box_gu), wmap_for(l, 5, box_gu), w.act, M, I, H, w.status,
-                                          env.timeout_ms, stream, &err, box_gu, T, 0, wq, wptr(l, 4), wptr(l, 5));
-        }
+        const int js[2] = {4, 5};
+        row_scales(js, 2);
+        rc = qmk_tc::launch_gemm_swiglu(map_xn, wmap_for(l, 4, box_gu), wmap_for(l, 5, box_gu), w.act, M, I, H, w.status,
+                                        env.timeout_ms, stream, &err, box_gu, T, 0, wq, wptr(l, 4), wptr(l, 5));
         if (rc != QMK_OK) break;
       }
-      {
-        qmk_tc::PdlScope g(pdl_gemm);
-        rc = gemm_od(map_act, l, 6, w.down, M, I, T);
-      }
+      rc = gemm_od(map_act, l, 6, w.down, M, I, T);
       if (rc != QMK_OK) break;
     }
     if (rc != QMK_OK) break;

@@ -378,7 +378,8 @@ def set_decode_attention(tensor_core: bool) -> None:
 
 
 def set_step_overlap(enabled: bool) -> None:
-    """Batched decode: launch the kernels of a step as programmatic dependents of one another (default on)."""
+    """Launch the kernels of a batched decode step, and of a tensor-core prefill, as programmatic dependents of one another
+    (default on)."""
     _check(_lib.qmk_set_step_overlap(int(bool(enabled))) == 0, "set_step_overlap failed")
 
 

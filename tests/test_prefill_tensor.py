@@ -212,3 +212,42 @@ def test_packed_weights_expanded_once_per_layer(C, fmt, n):
         print(f"{fmt} {n}: max difference {diff:.2e}, first layer {first:.2e}")
         assert first <= (2.0 ** -8 if n >= 1024 else 0.0) and float(x[0].abs().max()) < 8.0
         assert diff < 1e-2
+
+
+@pytest.mark.parametrize("fmt,lens", [("fp16", [31]), ("fp16", [129]), ("fp16", [513]), ("fp16", [4225]), ("fp8", [129]), ("fp8", [257]),
+                                      ("nvfp4", [128]), ("nvfp4", [1025]), ("fp16", [1, 37, 300, 1000]), ("nvfp4", [128, 700, 64]), ("fp8", [200, 3])])
+def test_launch_overlap_changes_nothing_but_time(C, fmt, lens):
+    """The kernels of a pass start under the tails of their predecessors (``set_step_overlap``); launched one after the other
+    they leave the same cache rows, bit for bit.  One chunk of each of the launch rules - one tile, K split four ways with each
+    tile width, two chunks - packed matrices inside the GEMMs and expanded per layer, several prompts in a pass."""
+    import quantize as Q
+    from Model.Qwen06B_architecture import BatchDecoder
+    vocab, L = 2048, 4352 if max(lens) > 2048 else 1152
+    w = S.make_weights(seed=41, num_layers=3, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    if fmt != "fp16":
+        w, _ = (Q.quantize_weights_fp8 if fmt == "fp8" else Q.quantize_weights_nvfp4)(w)
+    prompts = [S.make_prompt(n, seed=n, vocab_size=vocab) for n in lens]
+    try:
+        if len(lens) == 1:
+            one = _engine(w, L, "tensor", weight_format=fmt)
+            caches = [one._k_cache, one._v_cache]
+        else:
+            many = BatchDecoder(weights=S.weights_to(w, "cuda"), tokenizer=S.StubTokenizer(-1, vocab), num_sequences=len(lens),
+                                max_seq_len=L, engine="gemm", prefill_mode="tensor", weight_format=fmt)
+            caches = list(many._k_caches) + list(many._v_caches)
+        rows = {}
+        for overlap in (True, False, True, True):
+            C.set_step_overlap(overlap)
+            for c in caches:
+                c.zero_()
+            if len(lens) == 1:
+                one.reset()
+                one.prefill_ids(prompts[0])
+            else:
+                many.prefill_slots(list(range(len(lens))), prompts)
+            got = [c.clone() for c in caches]
+            assert all(torch.equal(a, b) for a, b in zip(got, rows.setdefault(0, got)))
+        assert all(bool(torch.isfinite(c.float()).all()) and float(c.float().abs().max()) > 0.1 for c in rows[0])
+    finally:
+        C.set_step_overlap(True)
+        C.set_weight_format("fp16")
