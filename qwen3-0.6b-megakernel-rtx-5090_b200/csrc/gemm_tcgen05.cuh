@@ -284,8 +284,8 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                    const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ CUtensorMap map_b2,
                    const Groups groups, int M, int K, unsigned int *status, unsigned long long budget_ns,
                    int selftest_no_loads) {
-  static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 256, "N tiles of 32, 64, 128 or 256 columns");
-  static_assert(!FUSE || BN <= 128, "the fused SwiGLU epilogue keeps two accumulators of at most 128 columns (one MMA of N = 256)");
+  static_assert(BN == 32 || BN == 64 || BN == 128, "N tiles of 32, 64 or 128 columns");
+  static_assert(!FUSE || BN <= 64, "the fused SwiGLU epilogue keeps two accumulators of at most 64 columns (one MMA of N = 128)");
   static_assert(!RS || (WQ == 0 && AH == 1), "row scales belong to expanded matrices");
   static_assert(WQ == 0 || (FUSE ? 2 * BN : BN) <= 128, "packed weights: at most 128 B rows per stage (scales live in shared memory)");
   constexpr int SB = FUSE ? 2 * BN : BN;          // B rows held per stage / accumulator columns

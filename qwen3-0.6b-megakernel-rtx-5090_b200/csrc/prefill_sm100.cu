@@ -12,6 +12,7 @@
 
 #include "../../include/qwen_megakernel.h"
 #include "gemm_tcgen05.cuh"
+#include "gemm_pair_tcgen05.cuh"
 #include "prefill_sm100.h"
 #include "prefill_kernels.cuh"
 #include "attention_tcgen05.cuh"
@@ -93,6 +94,22 @@ int make_map_packed(CUtensorMap *map, const void *ptr, uint64_t rows, int K, uin
   if (r != CUDA_SUCCESS) { *err = "cuTensorMapEncodeTiled failed with code " + std::to_string(static_cast<int>(r)); return QMK_ERR_CUDA; }
   return QMK_OK;
 }
+// Output matrix of the pair kernel [rows x cols], fp32 or fp16: blocks of 32 rows x 128 bytes, 128-byte swizzle.
+int make_map_c(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t cols, bool f16, std::string *err) {
+  EncodeTiledFn enc = encoder();
+  if (!enc) { *err = "cuTensorMapEncodeTiled is not available from this driver"; return QMK_ERR_CUDA; }
+  const cuuint64_t size = f16 ? 2 : 4;
+  if ((reinterpret_cast<uintptr_t>(ptr) & 15u) || (cols * size) % 16) { *err = "matrix not 16-byte aligned"; return QMK_ERR_BAD_ARGUMENT; }
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {cols * size};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(128 / size), 32};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult r = enc(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(ptr), dims, strides,
+                         box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) { *err = "cuTensorMapEncodeTiled (output) failed with code " + std::to_string(static_cast<int>(r)); return QMK_ERR_CUDA; }
+  return QMK_OK;
+}
 int make_map_b(CUtensorMap *map, const void *ptr, uint64_t rows, int K, uint32_t box_rows, int wq, std::string *err) {
   return wq ? make_map_packed(map, ptr, rows, K, box_rows, wq, err) : make_map_f16(map, ptr, rows, static_cast<uint64_t>(K), box_rows, err);
 }
@@ -163,11 +180,8 @@ static GemmKernel gemm_kernel_wq(int bn, bool fuse) {
   return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, false, WQ, 1, RS>
                   : bn == 64 ? qmk_gemm::gemm_f16_tn_kernel<64, false, WQ, 1, RS> : qmk_gemm::gemm_f16_tn_kernel<128, false, WQ, 1, RS>;
 }
-// (the widest tiles - 256 B rows per stage - exist for fp16 weights only)
 template <bool RS>
 static GemmKernel gemm_kernel_f16(int bn, bool fuse) {
-  if (fuse && bn == 128) return qmk_gemm::gemm_f16_tn_kernel<128, true, 0, 1, RS>;
-  if (!fuse && bn == 256) return qmk_gemm::gemm_f16_tn_kernel<256, false, 0, 1, RS>;
   return gemm_kernel_wq<0, RS>(bn, fuse);
 }
 // Split activations: at most 128 B rows per stage, packed 64.
@@ -181,7 +195,7 @@ static int split_max_rows(int wq) { return wq == 0 ? 128 : 64; }
 static bool box_n_ok(int box_n, bool fuse, int wq) {
   const int rows = fuse ? 2 * box_n : box_n;
   if (t_ah == 2) return wq < 2 && (box_n == 32 || box_n == 64 || box_n == 128) && rows <= split_max_rows(wq);
-  return box_n == 32 || box_n == 64 || (box_n == 128 && (rows == 128 || wq == 0)) || (box_n == 256 && rows == 256 && wq == 0);
+  return box_n == 32 || box_n == 64 || (box_n == 128 && rows == 128);
 }
 // (split activations exist for fp16 and FP8 weights; `scaled`: fp16 matrices with row scales)
 static GemmKernel gemm_kernel(int bn, bool fuse, int wq, int ah, bool scaled) {
@@ -190,6 +204,16 @@ static GemmKernel gemm_kernel(int bn, bool fuse, int wq, int ah, bool scaled) {
   return wq == 1 ? gemm_kernel_wq<1>(bn, fuse) : gemm_kernel_wq<2>(bn, fuse);
 }
 static size_t gemm_smem(int bn, bool fuse, int wq, int ah) { return qmk_gemm::smem_bytes_for(fuse ? 2 * bn : bn, wq, ah); }
+
+// Pairs of CTAs (gemm_pair_tcgen05.cuh): C matrices fp32 or fp16, or the SwiGLU of a gate and an up matrix.
+using PairKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
+                            const CUtensorMap, const qmk_pair::Args,
+                            unsigned int *, unsigned long long);
+static PairKernel pair_kernel(int mode, bool scaled) {
+  if (mode == 0) return scaled ? qmk_pair::gemm_pair_kernel<0, true> : qmk_pair::gemm_pair_kernel<0, false>;
+  if (mode == 1) return scaled ? qmk_pair::gemm_pair_kernel<1, true> : qmk_pair::gemm_pair_kernel<1, false>;
+  return scaled ? qmk_pair::gemm_pair_kernel<2, true> : qmk_pair::gemm_pair_kernel<2, false>;
+}
 
 // Opt-in shared-memory size of every tile variant, once per device (outside any stream capture).
 int ensure_gemm_attrs(std::string *err) {
@@ -201,10 +225,14 @@ int ensure_gemm_attrs(std::string *err) {
     for (int ah = 1; ah < 3 && e == cudaSuccess; ++ah)
       for (int wq = 0; wq < 4 - ah && e == cudaSuccess; ++wq)
         for (int fuse = 0; fuse < 2 && e == cudaSuccess; ++fuse)
-          for (int bn = 32; bn <= (ah == 2 ? split_max_rows(wq) / (fuse ? 2 : 1) : (fuse ? 64 : 128) * (wq == 0 ? 2 : 1)) && e == cudaSuccess; bn *= 2)
+          for (int bn = 32; bn <= (ah == 2 ? split_max_rows(wq) / (fuse ? 2 : 1) : fuse ? 64 : 128) && e == cudaSuccess; bn *= 2)
             for (int scaled = 0; scaled < (wq == 0 && ah == 1 ? 2 : 1) && e == cudaSuccess; ++scaled)
               e = cudaFuncSetAttribute(reinterpret_cast<const void *>(gemm_kernel(bn, fuse != 0, wq, ah, scaled != 0)),
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gemm_smem(bn, fuse != 0, wq, ah)));
+    for (int mode = 0; mode < 3 && e == cudaSuccess; ++mode)
+      for (int scaled = 0; scaled < 2 && e == cudaSuccess; ++scaled)
+        e = cudaFuncSetAttribute(reinterpret_cast<const void *>(pair_kernel(mode, scaled != 0)), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(qmk_pair::SMEM_BYTES));
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(qmk_pf::causal_attention_mma, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                qmk_pf::ATM_SMEM_BYTES);
@@ -283,7 +311,7 @@ int launch_gemm_grouped(const CUtensorMap &map_a, int ngroups, const CUtensorMap
                         std::string *err, int live_rows, int a_box_rows, int wq, const void *const *raws) {
   bool bad = M <= 0 || K <= 0 || M % qmk_gemm::BM || K % qmk_gemm::BK ||
              !box_n_ok(box_n, false, wq) || ngroups < 1 || ngroups > qmk_gemm::MAX_GROUPS;
-  for (int g = 0; !bad && g < ngroups; ++g) bad = Ns[g] <= 0 || Ns[g] % (box_n > 128 ? box_n : 128);
+  for (int g = 0; !bad && g < ngroups; ++g) bad = Ns[g] <= 0 || Ns[g] % 128;
   if (bad) {
     *err = "gemm: M and N must be multiples of 128 and K a multiple of 64";
     return QMK_ERR_BAD_ARGUMENT;
@@ -378,6 +406,38 @@ int launch_gemm_splitk(const CUtensorMap &map_a, const CUtensorMap &map_b, float
   return QMK_OK;
 }
 
+// The pair kernel: up to three matrices B_g (maps with 128 rows per box) against A, mode 0 fp32 (K split in `splits` parts, the
+// partial matrices pair_rows(M) rows apart), 1 fp16, 2 SwiGLU of maps_b[0] (gate) and maps_b[1] (up) with N = Ns[0] outputs.
+// maps_c: make_map_c.  M a multiple of 128; the last tile may reach 128 rows past it, as far as the C maps go.
+int launch_gemm_pair(int mode, const CUtensorMap &map_a, int ngroups, const CUtensorMap *const *maps_b, const CUtensorMap *const *maps_c,
+                     const int *Ns, int M, int K, int splits, unsigned int *status, int timeout_ms, cudaStream_t stream, std::string *err) {
+  const int columns = mode == 2 ? qmk_pair::TN / 2 : qmk_pair::TN, matrices = mode == 2 ? 1 : ngroups;
+  bool bad = mode < 0 || mode > 2 || M <= 0 || M % 128 || K <= 0 || splits < 1 || K % (qmk_pair::BK * splits) || ngroups < 1 || ngroups > 3 ||
+             (mode == 2 && ngroups != 2) || (splits > 1 && (mode != 0 || ngroups != 1));
+  for (int g = 0; !bad && g < matrices; ++g) bad = Ns[g] <= 0 || Ns[g] % columns;
+  for (int g = 0; !bad && g < ngroups; ++g) bad = (t_row_scale[g] == nullptr) != (t_row_scale[0] == nullptr);   // scales for all or for none
+  if (bad) { *err = "gemm: bad shape for pairs of CTAs"; return QMK_ERR_BAD_ARGUMENT; }
+  const int arc = ensure_gemm_attrs(err);
+  if (arc != QMK_OK) return arc;
+  qmk_pair::Args a;
+  a.n_tiles = 0;
+  for (int g = 0; g < 3; ++g) {
+    a.N[g] = g < matrices ? Ns[g] : 0;
+    a.row_scale[g] = g < ngroups ? t_row_scale[g] : nullptr;
+    a.n_tiles += a.N[g] / columns;
+  }
+  a.m_tiles = (M + qmk_pair::TM - 1) / qmk_pair::TM;
+  a.splits = splits;
+  a.kblocks = K / qmk_pair::BK / splits;
+  const int tiles = a.m_tiles * a.n_tiles * splits, pairs = std::min(tiles, sm_count() / 2);
+  const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
+  const cudaError_t e = launch_kernel(pair_kernel(mode, a.row_scale[0] != nullptr), dim3(2 * pairs), dim3(qmk_pair::THREADS), qmk_pair::SMEM_BYTES, stream,
+                                      map_a, *maps_b[0], *maps_b[ngroups > 1 ? 1 : 0], *maps_b[ngroups > 2 ? 2 : 0], *maps_c[0], *maps_c[matrices > 1 ? 1 : 0], *maps_c[matrices > 2 ? 2 : 0],
+                                      a, status, budget);
+  if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
+  return QMK_OK;
+}
+
 int launch_gemm(const CUtensorMap &map_a, const CUtensorMap &map_b, float *C, int M, int N, int K, int box_n,
                 unsigned int *status, int timeout_ms, cudaStream_t stream, std::string *err, int live_rows, int a_box_rows,
                 int wq, const void *raw) {
@@ -393,7 +453,8 @@ int launch_gemm(const CUtensorMap &map_a, const CUtensorMap &map_b, float *C, in
 // ----------------------------------------------------------------------------- chunked prefill
 namespace {
 
-constexpr unsigned int PREFILL_RING_BYTES = 96 * 1024, GATE_UP_RING_BYTES = 64 * 1024;
+constexpr unsigned int PREFILL_RING_BYTES = 96 * 1024;
+constexpr int PAIR_MIN_ROWS = 512;
 constexpr int EXPAND_MIN_ROWS = 384;
 constexpr int CHUNK = 4096;         // prompt tokens per pass over the weights (a multiple of the GEMM's 128)
 constexpr int MAX_LAYERS = 48;
@@ -405,6 +466,7 @@ struct Workspace {                  // per device, allocated on first use, never
   __half *xn = nullptr, *attn = nullptr, *act = nullptr;
   unsigned int *status = nullptr;
   CUtensorMap map_xn, map_attn, map_act, map_qh;
+  CUtensorMap map_cq, map_ck, map_cv, map_cact, map_co, map_cdown;   // outputs of the pair GEMMs
   CUtensorMap map_xn2, map_attn2, map_act2;   // split activations: rows of hi and lo halves
   // batched decode: per-sequence state and the logits of one step
   int *positions = nullptr, *start_positions = nullptr;
@@ -438,10 +500,10 @@ struct Workspace {                  // per device, allocated on first use, never
   // packed weights, long prefill chunks: one layer's matrices as fp16 values, their row scales and maps
   __half *expanded = nullptr;
   float *expanded_scale = nullptr;
-  CUtensorMap emap[7][3];              // boxes of 64, 128 and 256 rows
+  CUtensorMap emap[7][2];              // boxes of 64 and 128 rows
   CUtensorMap emap32[7];
   int table_wq = 0;                    // weight format the maps below were made for
-  CUtensorMap wmap[MAX_LAYERS][7][3];  // q, k, v, o, gate, up, down; boxes of 64, 128 and (fp16 weights) 256 rows
+  CUtensorMap wmap[MAX_LAYERS][7][2];  // q, k, v, o, gate, up, down; boxes of 64 and 128 rows
   CUtensorMap wmap32[MAX_LAYERS][7];   // the same matrices in boxes of 32 rows (decode steps: more, smaller tiles)
 };
 // Prefill and batched decode keep separate workspaces and locks: a serving loop prefills the next request on one
@@ -496,6 +558,13 @@ int ensure_workspace(Workspace &w, int rows, bool *no_room = nullptr) {
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_xn2, w.xn, C, 2 * H, qmk_gemm::BM, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_attn2, w.attn, C, 2 * QS, qmk_gemm::BM, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_act2, w.act, C, 2 * I, qmk_gemm::BM, &err);
+  // outputs of the pair GEMMs: q, k, v as fp16, the SwiGLU, fp32 sums (or partial matrices)
+  if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_cq, w.q, C, QS, true, &err);
+  if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_ck, w.k, C, KVS, true, &err);
+  if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_cv, w.v, C, KVS, true, &err);
+  if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_cact, w.act, C, I, true, &err);
+  if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_co, w.o, 2 * C, H, false, &err);
+  if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_cdown, w.down, 2 * C, H, false, &err);
   if (rc != QMK_OK) {
     for (const Buffer &b : buffers)
       if (*b.at) { cudaFree(*b.at); *b.at = nullptr; }
@@ -528,7 +597,7 @@ int ensure_expanded(Workspace &w) {
   size_t at = 0;
   for (int j = 0; j < 7 && rc == QMK_OK; ++j) {
     rc = qmk_tc::make_map_f16(&w.emap32[j], buf + at, MAT_ROWS[j], MAT_COLS[j], 32, &err);
-    for (int b = 0; b < 3 && rc == QMK_OK; ++b) rc = qmk_tc::make_map_f16(&w.emap[j][b], buf + at, MAT_ROWS[j], MAT_COLS[j], 64 << b, &err);
+    for (int b = 0; b < 2 && rc == QMK_OK; ++b) rc = qmk_tc::make_map_f16(&w.emap[j][b], buf + at, MAT_ROWS[j], MAT_COLS[j], 64 << b, &err);
     at += static_cast<size_t>(MAT_ROWS[j]) * MAT_COLS[j];
   }
   if (rc != QMK_OK) { cudaFree(buf); cudaFree(scale); return qmk_internal::report(rc, err); }
@@ -556,7 +625,7 @@ int ensure_weight_maps(Workspace &w, const LDGLayerWeight *layers_dev, int num_l
         const int rc = qmk_tc::make_map_b(&w.wmap32[l][j], ptr, MAT_ROWS[j], MAT_COLS[j], 32, wq, &err);
         if (rc != QMK_OK) return qmk_internal::report(rc, err);
       }
-      for (int b = 0; b < (wq == 0 ? 3 : 2); ++b) {
+      for (int b = 0; b < 2; ++b) {
         const int rc = qmk_tc::make_map_b(&w.wmap[l][j][b], ptr, MAT_ROWS[j], MAT_COLS[j], 64 << b, wq, &err);
         if (rc != QMK_OK) return qmk_internal::report(rc, err);
       }
@@ -681,8 +750,8 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
   std::string err;
   // weight matrix j of layer l in boxes of `box_n` rows
   auto wmap_for = [&](int l, int j, int box_n) -> const CUtensorMap & {
-    if (wq != wfmt) return box_n == 32 ? w.emap32[j] : w.emap[j][box_n == 64 ? 0 : box_n == 128 ? 1 : 2];
-    return box_n == 32 ? w.wmap32[l][j] : w.wmap[l][j][box_n == 64 ? 0 : box_n == 128 ? 1 : 2];
+    if (wq != wfmt) return box_n == 32 ? w.emap32[j] : w.emap[j][box_n == 64 ? 0 : 1];
+    return box_n == 32 ? w.wmap32[l][j] : w.wmap[l][j][box_n == 64 ? 0 : 1];
   };
   static const int rec_slot[7] = {1, 2, 3, 6, 8, 9, 10};   // q, k, v, o, gate, up, down inside a layer record
   auto wptr = [&](int l, int j) { return reinterpret_cast<const void *>(rec[static_cast<size_t>(l) * 12 + rec_slot[j]]); };
@@ -699,16 +768,20 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
   struct ClearScales { ~ClearScales() { for (int i = 0; i < 3; ++i) qmk_tc::t_row_scale[i] = nullptr; } } clear_scales;   // on every way out
   // packed weights with split activations take narrower tiles
   auto split_box = [&](int box_n, int widest) { return split && wq != 0 && box_n > widest ? widest : box_n; };
+  bool by_pairs = false;   // this chunk's GEMMs run on pairs of CTAs
   // several matrices against the same activations in one launch (q/k/v)
   auto gemm_group = [&](const CUtensorMap &a, int l, int n, const int *js, float *const *cs, const int *ns, int M, int K,
                         int live) {
     int total = 0;
     for (int i = 0; i < n; ++i) total += ns[i];
-    // Long chunks of fp16 weights: 256-wide tiles (one MMA of N = 256 per K step; a third fewer operand bytes per
-    // flop than 128-wide ones - these GEMMs are bound by the L2 -> shared-memory feed).  Measured on the q/k/v shape at
-    // 2048 rows: 28.8 -> 26.5 us.
-    const int box_n = (wq == 0 && !split && M >= 1024 && total / 256 * (M / qmk_gemm::BM) >= qmk_tc::gemm_sm_count()) ? 256
-                                                                                                           : split_box(qmk_tc::gemm_box_n(M, total), 64);
+    if (by_pairs) {
+      const CUtensorMap *maps[3];
+      for (int i = 0; i < n; ++i) maps[i] = &wmap_for(l, js[i], 128);
+      const CUtensorMap *const out[3] = {&w.map_cq, &w.map_ck, &w.map_cv};
+      row_scales(js, n);
+      return qmk_tc::launch_gemm_pair(1, a, n, maps, out, ns, M, K, 1, w.status, env.timeout_ms, stream, &err);
+    }
+    const int box_n = split_box(qmk_tc::gemm_box_n(M, total), 64);
     const CUtensorMap *maps[3];
     const void *raws[3] = {nullptr, nullptr, nullptr};
     for (int i = 0; i < n; ++i) { maps[i] = &wmap_for(l, js[i], box_n); raws[i] = wptr(l, js[i]); }
@@ -729,24 +802,27 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
       if (rc != QMK_OK) return rc;
       if (w.expanded) wq = 0;
     }
-    // The O and down projections have only 1024 output columns: with 128-wide tiles a long chunk gives 128 CTAs for
-    // 148 SMs (296 slots with two CTAs per SM) and a K loop of 32 / 48 blocks.  K split in two doubles the CTAs and
-    // halves the loop; the partial matrices are added by the residual + RMSNorm kernel that follows anyway.
-    // Short chunks: four splits (M = 512: 32 tiles x 4 = 128 CTAs with K loops of 8 / 12 blocks; unsplit, the narrowest
-    // tiles gave 128 CTAs with loops of 32 / 48 blocks of N = 32 MMAs and these two products were 41 % of the pass).
+    // Chunks of more than four row tiles run on pairs of CTAs (fp16 weights, expanded packed ones).  760 / 1000 / 1500 / 2000 /
+    // 4000 / 8191 tokens, single CTAs -> pairs: 2.01 / 2.10 / 3.17 / 3.74 / 8.10 / 20.4 -> 1.79 / 2.03 / 2.55 / 3.28 / 6.77 /
+    // 17.6 ms; 500 tokens 1.56 -> 1.61, 250 tokens 1.21 -> 1.40 (a 256 x 256 tile for each pair leaves most pairs idle).
+    by_pairs = wq == 0 && !split && M > PAIR_MIN_ROWS;
+    // The O and down projections have only 1024 output columns.  K is split so that their tiles fill the SMs; the partial
+    // matrices are added by the residual + RMSNorm kernel that follows anyway.  Pairs: as many parts (1, 2 or 4) as give every
+    // pair at most one tile.  Single CTAs: four (M = 512: 32 tiles x 4 = 128 CTAs with K loops of 8 / 12 blocks; unsplit, the
+    // narrowest tiles gave 128 CTAs with loops of 32 / 48 blocks of N = 32 MMAs and these two products were 41 % of the pass),
+    // long chunks of split activations two.
     // Packed weights split only short chunks: a CTA expands its weight tile itself, so two CTAs with half a K loop each beat
     // one only while there are too few tiles (93 tokens 2.06 -> 1.75 ms; 1023 tokens measured 1 % slower with two splits).
-    const int od_splits = M < 1024 ? 4 : wq == 0 ? 2 : 1;
-    const size_t od_stride = static_cast<size_t>(M) * H;
+    const int row_tiles = (M + qmk_pair::TM - 1) / qmk_pair::TM, od_tiles = row_tiles * (H / qmk_pair::TN), od_pairs = qmk_tc::gemm_sm_count() / 2;
+    const int od_splits = by_pairs ? (4 * od_tiles <= od_pairs ? 4 : 2 * od_tiles <= od_pairs ? 2 : 1) : M < 1024 ? 4 : wq == 0 ? 2 : 1;
+    const size_t od_stride = static_cast<size_t>(by_pairs ? row_tiles * qmk_pair::TM : M) * H;
     auto gemm_od = [&](const CUtensorMap &a, int l, int j, float *c, int Mrows, int K, int live) {
       row_scales(&j, 1);
-      // 256-wide tiles, one CTA per SM with the whole ring: the main loops are bound by shared-memory traffic (TMA
-      // writes + MMA operand reads), and a 256-wide tile moves a quarter fewer bytes per flop than a 128-wide one
-      // (2048 tokens: 4.12 -> 4.07 ms per pass, same box); shorter chunks would leave SMs without a tile
-      if (Mrows >= 2048 && wq == 0 && !split) {
-        qmk_tc::RingBudgetScope whole(0);
-        return qmk_tc::launch_gemm_splitk(a, wmap_for(l, j, 256), c, Mrows, H, K, od_splits, w.status, env.timeout_ms, stream, &err,
-                                          256, live, 0, wq, wptr(l, j));
+      if (by_pairs) {
+        const CUtensorMap *const map = &wmap_for(l, j, 128);
+        const CUtensorMap *const out = c == w.o ? &w.map_co : &w.map_cdown;
+        const int n = H;
+        return qmk_tc::launch_gemm_pair(0, a, 1, &map, &out, &n, Mrows, K, od_splits, w.status, env.timeout_ms, stream, &err);
       }
       if (od_splits == 1) {
         const int box_n = split_box(qmk_tc::gemm_box_n(Mrows, H), 64);
@@ -869,12 +945,17 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
       PF_CUDA(norm_rows(w.o, reinterpret_cast<const __half *>(r[7])));
       {
         const int box_gu = split_box(qmk_tc::gemm_box_n_fused(M, I), 32);
-        // three of these CTAs per SM instead of two: their epilogue (two TMEM reads, SiLU, fp16 pack) is the long part
-        qmk_tc::RingBudgetScope gu_scope(split ? 0 : M >= 1024 ? GATE_UP_RING_BYTES : PREFILL_RING_BYTES);
         const int js[2] = {4, 5};
         row_scales(js, 2);
-        rc = qmk_tc::launch_gemm_swiglu(map_xn, wmap_for(l, 4, box_gu), wmap_for(l, 5, box_gu), w.act, M, I, H, w.status,
-                                        env.timeout_ms, stream, &err, box_gu, T, 0, wq, wptr(l, 4), wptr(l, 5));
+        if (by_pairs) {
+          const CUtensorMap *const maps[2] = {&wmap_for(l, 4, 128), &wmap_for(l, 5, 128)};
+          const CUtensorMap *const out = &w.map_cact;
+          const int n = I;
+          rc = qmk_tc::launch_gemm_pair(2, map_xn, 2, maps, &out, &n, M, H, 1, w.status, env.timeout_ms, stream, &err);
+        } else {
+          rc = qmk_tc::launch_gemm_swiglu(map_xn, wmap_for(l, 4, box_gu), wmap_for(l, 5, box_gu), w.act, M, I, H, w.status,
+                                          env.timeout_ms, stream, &err, box_gu, T, 0, wq, wptr(l, 4), wptr(l, 5));
+        }
         if (rc != QMK_OK) break;
       }
       rc = gemm_od(map_act, l, 6, w.down, M, I, T);
@@ -1235,7 +1316,6 @@ extern "C" int qmk_selftest_gemm_wait_timeout(int budget_us) {
     gr.raw_pitch = gr.raw_bs_off = gr.raw_scale_off = 0;
     gr.amax_val = nullptr;
     gr.out_f16 = 0;
-  gr.out_f16 = 0;
     gr.amax_idx = nullptr;
     const size_t smem = qmk_tc::selftest_ring(&gr);
     qmk_gemm::gemm_f16_tn_kernel<128><<<dim3(1, 1), qmk_gemm::THREADS, smem>>>(
@@ -1257,12 +1337,20 @@ extern "C" int qmk_gemm_f16_tn(const void *a, const void *b, float *c, int m, in
   CUtensorMap ma, mb;
   unsigned int *status = nullptr;
   int rc = qmk_tc::make_map_f16(&ma, a, m, k, qmk_gemm::BM, &err);
-  const int box_n = (m > 0 && n > 0 && m % 128 == 0 && n % 128 == 0) ? qmk_tc::gemm_box_n(m, n) : 128;
+  const bool by_pairs = m > PAIR_MIN_ROWS && n > 0 && n % qmk_pair::TN == 0;
+  const int box_n = (!by_pairs && m > 0 && n > 0 && m % 128 == 0 && n % 128 == 0) ? qmk_tc::gemm_box_n(m, n) : 128;
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&mb, b, n, k, box_n, &err);
   if (rc == QMK_OK && cudaMalloc(&status, 16) != cudaSuccess) { rc = QMK_ERR_CUDA; err = "cudaMalloc failed"; }
   if (rc == QMK_OK) {
     cudaMemsetAsync(status, 0, 16, stream);
-    rc = qmk_tc::launch_gemm(ma, mb, c, m, n, k, box_n, status, 2000, stream, &err);
+    if (by_pairs) {
+      CUtensorMap mc;
+      const CUtensorMap *const maps_b[1] = {&mb}, *const maps_c[1] = {&mc};
+      rc = qmk_tc::make_map_c(&mc, c, m, n, false, &err);
+      if (rc == QMK_OK) rc = qmk_tc::launch_gemm_pair(0, ma, 1, maps_b, maps_c, &n, m, k, 1, status, 2000, stream, &err);
+    } else {
+      rc = qmk_tc::launch_gemm(ma, mb, c, m, n, k, box_n, status, 2000, stream, &err);
+    }
   }
   if (rc == QMK_OK) {
     unsigned int host[4] = {0, 0, 0, 0};

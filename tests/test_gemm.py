@@ -29,6 +29,18 @@ def test_matches_torch(C, m, n, k):
     assert err < 1e-3 * (k ** 0.5) * 4
 
 
+@pytest.mark.parametrize("m,n,k", [(640, 256, 64), (640, 2304, 128), (896, 512, 448), (1024, 1024, 384), (1152, 4096, 1024), (4096, 1024, 3072)])
+def test_pairs_of_ctas_match_torch(C, m, n, k):
+    """More than 512 rows run on pairs of CTAs with 256 x 256 tiles: K of one block, of fewer blocks than the ring has stages, of
+    a full ring and one block over; an odd number of 128-row tiles (the last pair's second half lies past the matrix); fewer
+    tiles than pairs, and several per pair (the two accumulator buffers in turn).  A and B are small integers, so every sum
+    is exact and each element is compared for equality."""
+    g = torch.Generator("cpu").manual_seed(m + n + k)
+    a = torch.randint(-3, 4, (m, k), generator=g).to(torch.float16).cuda()
+    b = torch.randint(-3, 4, (n, k), generator=g).to(torch.float16).cuda()
+    assert torch.equal(C.gemm_f16_tn(a, b), a.float() @ b.float().T)
+
+
 def test_every_element_lands_in_its_place(C):
     """Operands that make every output element distinct: A row i = one-hot at column i (scaled), so C row i is
     a scaled copy of B's column i; any swizzle or tile mix-up moves values."""

@@ -214,7 +214,7 @@ def test_packed_weights_expanded_once_per_layer(C, fmt, n):
         assert diff < 1e-2
 
 
-@pytest.mark.parametrize("fmt,lens", [("fp16", [31]), ("fp16", [129]), ("fp16", [513]), ("fp16", [4225]), ("fp8", [129]), ("fp8", [257]),
+@pytest.mark.parametrize("fmt,lens", [("fp16", [31]), ("fp16", [129]), ("fp16", [513]), ("fp16", [1409]), ("fp16", [4225]), ("fp8", [129]), ("fp8", [257]),
                                       ("nvfp4", [128]), ("nvfp4", [1025]), ("fp16", [1, 37, 300, 1000]), ("nvfp4", [128, 700, 64]), ("fp8", [200, 3])])
 def test_launch_overlap_changes_nothing_but_time(C, fmt, lens):
     """The kernels of a pass start under the tails of their predecessors (``set_step_overlap``); launched one after the other
@@ -222,7 +222,7 @@ def test_launch_overlap_changes_nothing_but_time(C, fmt, lens):
     tile width, two chunks - packed matrices inside the GEMMs and expanded per layer, several prompts in a pass."""
     import quantize as Q
     from Model.Qwen06B_architecture import BatchDecoder
-    vocab, L = 2048, 4352 if max(lens) > 2048 else 1152
+    vocab, L = 2048, 4352 if max(lens) > 2048 else 1536
     w = S.make_weights(seed=41, num_layers=3, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
     if fmt != "fp16":
         w, _ = (Q.quantize_weights_fp8 if fmt == "fp8" else Q.quantize_weights_nvfp4)(w)
