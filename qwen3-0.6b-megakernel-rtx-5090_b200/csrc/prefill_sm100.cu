@@ -115,14 +115,14 @@ int make_map_b(CUtensorMap *map, const void *ptr, uint64_t rows, int K, uint32_t
 }
 
 // 3-D tensor map of an fp16 KV cache [heads][max_seq_len][128] of which the first `rows` positions of every head are
-// valid: boxes of 64 dims x 64 positions of one head, 128-byte swizzle; positions >= rows read as zeros.
+// valid: boxes of 64 dims x 128 positions of one head, 128-byte swizzle; positions >= rows read as zeros.
 int make_map_kv(CUtensorMap *map, const void *cache, uint64_t rows, uint64_t max_seq_len, uint64_t heads, std::string *err) {
   EncodeTiledFn enc = encoder();
   if (!enc) { *err = "cuTensorMapEncodeTiled is not available from this driver"; return QMK_ERR_CUDA; }
   if (reinterpret_cast<uintptr_t>(cache) & 15u) { *err = "cache not 16-byte aligned"; return QMK_ERR_BAD_ARGUMENT; }
   const cuuint64_t dims[3] = {128, rows, heads};
   const cuuint64_t strides[2] = {256, max_seq_len * 256};
-  const cuuint32_t box[3] = {64, 64, 1};
+  const cuuint32_t box[3] = {64, 128, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void *>(cache), dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -239,7 +239,10 @@ int ensure_gemm_attrs(std::string *err) {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(qmk_pf::causal_attention_split, cudaFuncAttributeMaxDynamicSharedMemorySize, qmk_pf::ATM_SMEM_BYTES);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(qmk_attn::SMEM_BYTES));
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(qmk_attn::SMEM_BYTES));
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(qmk_pf::decode_attention_ring, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -456,6 +459,13 @@ namespace {
 constexpr unsigned int PREFILL_RING_BYTES = 96 * 1024;
 constexpr int PAIR_MIN_ROWS = 512;
 constexpr int EXPAND_MIN_ROWS = 384;
+// The prefill attention's CTAs: a pair of heads for each query tile, or one head whose keys go to two chains - twice the CTAs with
+// half the key tiles each, for twice the key and value copies.  Pairs once there are a third more of them than SMs.  Pairs /
+// chains, 1000 / 2000 / 2500 / 3000 / 4000 / 8191 tokens: 2.20 / 3.34 / 4.26 / 4.95 / 6.52 / 16.7, 2.01 / 3.20 / 4.16 / 4.93 / 6.66 /
+// 17.0 ms.
+bool attention_by_chains(int rows) {
+  return (rows + qmk_attn::TQ - 1) / qmk_attn::TQ * qmk_attn::NKV * 3 < 4 * qmk_tc::gemm_sm_count();
+}
 constexpr int CHUNK = 4096;         // prompt tokens per pass over the weights (a multiple of the GEMM's 128)
 constexpr int MAX_LAYERS = 48;
 
@@ -466,7 +476,7 @@ struct Workspace {                  // per device, allocated on first use, never
   __half *xn = nullptr, *attn = nullptr, *act = nullptr;
   unsigned int *status = nullptr;
   CUtensorMap map_xn, map_attn, map_act, map_qh;
-  CUtensorMap map_cq, map_ck, map_cv, map_cact, map_co, map_cdown;   // outputs of the pair GEMMs
+  CUtensorMap map_cq, map_ck, map_cv, map_cact, map_co, map_cdown, map_cattn;   // outputs of the pair GEMMs and of the attention
   CUtensorMap map_xn2, map_attn2, map_act2;   // split activations: rows of hi and lo halves
   // batched decode: per-sequence state and the logits of one step
   int *positions = nullptr, *start_positions = nullptr;
@@ -558,7 +568,8 @@ int ensure_workspace(Workspace &w, int rows, bool *no_room = nullptr) {
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_xn2, w.xn, C, 2 * H, qmk_gemm::BM, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_attn2, w.attn, C, 2 * QS, qmk_gemm::BM, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_act2, w.act, C, 2 * I, qmk_gemm::BM, &err);
-  // outputs of the pair GEMMs: q, k, v as fp16, the SwiGLU, fp32 sums (or partial matrices)
+  // outputs of the pair GEMMs: q, k, v as fp16, the SwiGLU, fp32 sums (or partial matrices); of the attention
+  if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_cattn, w.attn, C, QS, true, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_cq, w.q, C, QS, true, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_ck, w.k, C, KVS, true, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_cv, w.v, C, KVS, true, &err);
@@ -727,10 +738,11 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
         mrc = qmk_tc::make_map_kv(&maps[2 * s + 1], pk->v_caches[s], static_cast<uint64_t>(len), static_cast<uint64_t>(max_seq_len),
                                   static_cast<uint64_t>(num_layers) * NKV, &merr);
       if (mrc != QMK_OK) return qmk_internal::report(mrc, merr);
+      const bool attn_chains = attention_by_chains(total_rows);
       for (int qt = 0; qt * qmk_attn::TQ < len; ++qt) {
         const int last = (qt + 1) * qmk_attn::TQ < len ? (qt + 1) * qmk_attn::TQ - 1 : len - 1;
-        for (int h = 0; h < NQ; ++h)
-          order.push_back({last / qmk_attn::TK + 1, make_int4(s, row0 + qt * qmk_attn::TQ, qt * qmk_attn::TQ, h | (len << 8))});
+        for (int unit = 0; unit < (attn_chains ? NQ : NKV); ++unit)
+          order.push_back({last / qmk_attn::TK + 1, make_int4(s, row0 + qt * qmk_attn::TQ, qt * qmk_attn::TQ, unit | (len << 8))});
       }
       row0 += (len + qmk_gemm::BM - 1) / qmk_gemm::BM * qmk_gemm::BM;
       tok0 += len;
@@ -919,10 +931,12 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
                                     static_cast<size_t>(l) * layer_stride,
                                     env.attn_tc ? attn_scale * 1.4426950408889634f : 0.f));
       if (l == num_layers - 1) break;   // the cache is complete; nothing downstream of the last layer is kept
+      const bool attn_chains = attention_by_chains(T);   // (packed prompts: T = all their rows, one chunk)
       if (env.attn_tc)
-        PF_CUDA(qmk_tc::launch_kernel(qmk_attn::causal_attention_tc, dim3(pk ? pk_items : (T + qmk_attn::TQ - 1) / qmk_attn::TQ * NQ),
-                                      dim3(qmk_attn::THREADS), qmk_attn::SMEM_BYTES, stream, w.map_qh, map_kc, map_vc, l * NKV, w.attn, T,
-                                      pos0, attn_scale, w.status, static_cast<unsigned long long>(env.timeout_ms) * 1000000ull,
+        PF_CUDA(qmk_tc::launch_kernel(attn_chains ? qmk_attn::causal_attention_tc<true> : qmk_attn::causal_attention_tc<false>,
+                                      dim3(pk ? pk_items : (T + qmk_attn::TQ - 1) / qmk_attn::TQ * (attn_chains ? NQ : NKV)),
+                                      dim3(qmk_attn::THREADS), qmk_attn::SMEM_BYTES, stream, w.map_qh, map_kc, map_vc, w.map_cattn, l * NKV, T,
+                                      pos0, w.status, static_cast<unsigned long long>(env.timeout_ms) * 1000000ull,
                                       pk ? reinterpret_cast<const int4 *>(w.packed + PK_ITEMS_OFF) : nullptr,
                                       pk ? reinterpret_cast<const CUtensorMap *>(w.packed + PK_MAPS_OFF) : nullptr));
       else if (split) {

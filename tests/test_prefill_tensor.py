@@ -251,3 +251,31 @@ def test_launch_overlap_changes_nothing_but_time(C, fmt, lens):
     finally:
         C.set_step_overlap(True)
         C.set_weight_format("fp16")
+
+
+@pytest.mark.parametrize("before,n", [(0, 64), (0, 65), (0, 129), (0, 320), (77, 51), (63, 1), (1000, 200), (130, 1500), (0, 4225)])
+def test_attention_kernels_agree(C, before, n):
+    """The tcgen05 attention against the mma.sync kernel on the same chunk: less than a key tile, one key over, an odd and an even
+    number of key tiles, prompts that continue at a position inside a tile (so that the diagonal crosses it), chunks whose
+    query tiles run as chains of one head and as pairs of heads.  Both round queries, keys and softmax weights to fp16 and
+    add in fp32; what differs is the order of sums: 1e-2 on cache values, as between any two passes of this path."""
+    vocab, L = 2048, 4352 if n > 2048 else 2048
+    w = S.make_weights(seed=51, num_layers=3, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    ids = S.make_prompt(before + n, seed=n, vocab_size=vocab)
+    eng = _engine(w, L, "tensor")
+    rows = []
+    try:
+        for kernel in (1, 0, 1):
+            C.set_prefill_attention(kernel)
+            eng.reset()
+            for cache in (eng._k_cache, eng._v_cache):
+                cache.fill_(float("nan") if kernel else 0.0)      # (rows behind the prompt do not reach the tcgen05 kernel)
+            if before:
+                eng.prefill_ids(ids[:before])
+            eng.prefill_ids(ids[before:])
+            rows.append((eng._k_cache[:, :, :before + n].float().clone(), eng._v_cache[:, :, :before + n].float().clone()))
+    finally:
+        C.set_prefill_attention(1)
+    for a, b, again in zip(*rows):
+        assert bool(torch.isfinite(a).all()) and torch.equal(a, again)
+        assert float((a - b).abs().max()) < 1e-2
