@@ -16,6 +16,7 @@
 #include "prefill_sm100.h"
 #include "prefill_kernels.cuh"
 #include "attention_tcgen05.cuh"
+#include "attention_pairs_tcgen05.cuh"
 #include "decode_attention_mma.cuh"
 #include "engine_internal.h"
 #include <vector>
@@ -115,14 +116,15 @@ int make_map_b(CUtensorMap *map, const void *ptr, uint64_t rows, int K, uint32_t
 }
 
 // 3-D tensor map of an fp16 KV cache [heads][max_seq_len][128] of which the first `rows` positions of every head are
-// valid: boxes of 64 dims x 128 positions of one head, 128-byte swizzle; positions >= rows read as zeros.
-int make_map_kv(CUtensorMap *map, const void *cache, uint64_t rows, uint64_t max_seq_len, uint64_t heads, std::string *err) {
+// valid: boxes of 64 dims x `box_rows` positions of one head, 128-byte swizzle; positions >= rows read as zeros.
+int make_map_kv(CUtensorMap *map, const void *cache, uint64_t rows, uint64_t max_seq_len, uint64_t heads, uint32_t box_rows,
+                std::string *err) {
   EncodeTiledFn enc = encoder();
   if (!enc) { *err = "cuTensorMapEncodeTiled is not available from this driver"; return QMK_ERR_CUDA; }
   if (reinterpret_cast<uintptr_t>(cache) & 15u) { *err = "cache not 16-byte aligned"; return QMK_ERR_BAD_ARGUMENT; }
   const cuuint64_t dims[3] = {128, rows, heads};
   const cuuint64_t strides[2] = {256, max_seq_len * 256};
-  const cuuint32_t box[3] = {64, 128, 1};
+  const cuuint32_t box[3] = {64, box_rows, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void *>(cache), dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -239,11 +241,11 @@ int ensure_gemm_attrs(std::string *err) {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(qmk_pf::causal_attention_split, cudaFuncAttributeMaxDynamicSharedMemorySize, qmk_pf::ATM_SMEM_BYTES);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(qmk_attn::SMEM_BYTES));
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(qmk_attn::SMEM_BYTES));
+      e = cudaFuncSetAttribute(qmk_attn_pairs::causal_attention_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(qmk_attn_pairs::SMEM_BYTES));
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(qmk_pf::decode_attention_ring, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                qmk_pf::DAR_SMEM_BYTES);
@@ -459,12 +461,12 @@ namespace {
 constexpr unsigned int PREFILL_RING_BYTES = 96 * 1024;
 constexpr int PAIR_MIN_ROWS = 512;
 constexpr int EXPAND_MIN_ROWS = 384;
-// The prefill attention's CTAs: a pair of heads for each query tile, or one head whose keys go to two chains - twice the CTAs with
-// half the key tiles each, for twice the key and value copies.  Pairs once there are a third more of them than SMs.  Pairs /
-// chains, 1000 / 2000 / 2500 / 3000 / 4000 / 8191 tokens: 2.20 / 3.34 / 4.26 / 4.95 / 6.52 / 16.7, 2.01 / 3.20 / 4.16 / 4.93 / 6.66 /
-// 17.0 ms.
-bool attention_by_chains(int rows) {
-  return (rows + qmk_attn::TQ - 1) / qmk_attn::TQ * qmk_attn::NKV * 3 < 4 * qmk_tc::gemm_sm_count();
+// Chunks of one prompt take the attention kernel with both heads of a kv head per CTA once it has a third more CTAs than SMs: with
+// fewer, the kernel with one head per CTA and two chains of key tiles fills the SMs better (2000 / 2500 / 3000 / 4000 / 8191
+// tokens 3.20 / 4.16 / 4.93 / 6.77 / 17.6 ms by one head, 3.34 / 4.26 / 4.95 / 6.59 / 16.8 by two).  Packed prompts, whose
+// sequences are a fraction of a chunk, keep the former.
+bool attention_by_pairs(int rows) {
+  return (rows + qmk_attn_pairs::TQ - 1) / qmk_attn_pairs::TQ * qmk_attn_pairs::NKV * 3 >= 4 * qmk_tc::gemm_sm_count();
 }
 constexpr int CHUNK = 4096;         // prompt tokens per pass over the weights (a multiple of the GEMM's 128)
 constexpr int MAX_LAYERS = 48;
@@ -733,16 +735,15 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
       ptrs[2 * s] = reinterpret_cast<unsigned long long>(pk->k_caches[s]);
       ptrs[2 * s + 1] = reinterpret_cast<unsigned long long>(pk->v_caches[s]);
       int mrc = qmk_tc::make_map_kv(&maps[2 * s], pk->k_caches[s], static_cast<uint64_t>(len), static_cast<uint64_t>(max_seq_len),
-                                    static_cast<uint64_t>(num_layers) * NKV, &merr);
+                                    static_cast<uint64_t>(num_layers) * NKV, qmk_attn::TK, &merr);
       if (mrc == QMK_OK)
         mrc = qmk_tc::make_map_kv(&maps[2 * s + 1], pk->v_caches[s], static_cast<uint64_t>(len), static_cast<uint64_t>(max_seq_len),
-                                  static_cast<uint64_t>(num_layers) * NKV, &merr);
+                                  static_cast<uint64_t>(num_layers) * NKV, qmk_attn::TK, &merr);
       if (mrc != QMK_OK) return qmk_internal::report(mrc, merr);
-      const bool attn_chains = attention_by_chains(total_rows);
       for (int qt = 0; qt * qmk_attn::TQ < len; ++qt) {
         const int last = (qt + 1) * qmk_attn::TQ < len ? (qt + 1) * qmk_attn::TQ - 1 : len - 1;
-        for (int unit = 0; unit < (attn_chains ? NQ : NKV); ++unit)
-          order.push_back({last / qmk_attn::TK + 1, make_int4(s, row0 + qt * qmk_attn::TQ, qt * qmk_attn::TQ, unit | (len << 8))});
+        for (int h = 0; h < NQ; ++h)
+          order.push_back({last / qmk_attn::TK + 1, make_int4(s, row0 + qt * qmk_attn::TQ, qt * qmk_attn::TQ, h | (len << 8))});
       }
       row0 += (len + qmk_gemm::BM - 1) / qmk_gemm::BM * qmk_gemm::BM;
       tok0 += len;
@@ -819,18 +820,21 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     // 17.6 ms; 500 tokens 1.56 -> 1.61, 250 tokens 1.21 -> 1.40 (a 256 x 256 tile for each pair leaves most pairs idle).
     by_pairs = wq == 0 && !split && M > PAIR_MIN_ROWS;
     // The O and down projections have only 1024 output columns.  K is split so that their tiles fill the SMs; the partial
-    // matrices are added by the residual + RMSNorm kernel that follows anyway.  Pairs: as many parts (1, 2 or 4) as give every
-    // pair at most one tile.  Single CTAs: four (M = 512: 32 tiles x 4 = 128 CTAs with K loops of 8 / 12 blocks; unsplit, the
-    // narrowest tiles gave 128 CTAs with loops of 32 / 48 blocks of N = 32 MMAs and these two products were 41 % of the pass),
-    // long chunks of split activations two.
+    // matrices are added by the residual + RMSNorm kernel that follows anyway.  Four parts below 1024 rows (M = 512: 32 tiles x
+    // 4 = 128 CTAs with K loops of 8 / 12 blocks; unsplit, the narrowest tiles gave 128 CTAs with loops of 32 / 48 blocks of N =
+    // 32 MMAs and these two products were 41 % of the pass), two above: the sums, and with them the last bits of every row behind,
+    // do not depend on which kernel made them.  (One part where the pairs would fill the SMs without
+    // a split: 4000 tokens 6.59 -> 6.50 ms, and NVFP4 batches whose picks were ties to 1e-3 went another way.)
     // Packed weights split only short chunks: a CTA expands its weight tile itself, so two CTAs with half a K loop each beat
     // one only while there are too few tiles (93 tokens 2.06 -> 1.75 ms; 1023 tokens measured 1 % slower with two splits).
-    const int row_tiles = (M + qmk_pair::TM - 1) / qmk_pair::TM, od_tiles = row_tiles * (H / qmk_pair::TN), od_pairs = qmk_tc::gemm_sm_count() / 2;
-    const int od_splits = by_pairs ? (4 * od_tiles <= od_pairs ? 4 : 2 * od_tiles <= od_pairs ? 2 : 1) : M < 1024 ? 4 : wq == 0 ? 2 : 1;
-    const size_t od_stride = static_cast<size_t>(by_pairs ? row_tiles * qmk_pair::TM : M) * H;
+    const int od_splits = M < 1024 ? 4 : wq == 0 ? 2 : 1;
+    // Two parts whose 128-wide tiles all find an SM of their own (1024 and 1152 rows) stay with single CTAs: 32 or 40 tiles of
+    // 256 x 256 leave half of the pairs idle (1000 tokens, with four parts to fill them, 2.03 ms; here 2.02).
+    const bool od_pairs = by_pairs && (M < 1024 || static_cast<long>(M / qmk_gemm::BM) * (H / 128) * od_splits > qmk_tc::gemm_sm_count());
+    const size_t od_stride = static_cast<size_t>(od_pairs ? (M + qmk_pair::TM - 1) / qmk_pair::TM * qmk_pair::TM : M) * H;
     auto gemm_od = [&](const CUtensorMap &a, int l, int j, float *c, int Mrows, int K, int live) {
       row_scales(&j, 1);
-      if (by_pairs) {
+      if (od_pairs) {
         const CUtensorMap *const map = &wmap_for(l, j, 128);
         const CUtensorMap *const out = c == w.o ? &w.map_co : &w.map_cdown;
         const int n = H;
@@ -851,12 +855,14 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     CUtensorMap map_kc, map_vc;   // the caches up to this chunk's last position, all layers
     memset(&map_kc, 0, sizeof(map_kc));
     memset(&map_vc, 0, sizeof(map_vc));
+    const bool attn_pairs = env.attn_tc && !pk && attention_by_pairs(T);
+    const uint32_t kv_box = attn_pairs ? qmk_attn_pairs::TK : qmk_attn::TK;
     if (env.attn_tc && !pk) {
       rc = qmk_tc::make_map_kv(&map_kc, k_cache, static_cast<uint64_t>(pos0 + T), static_cast<uint64_t>(max_seq_len),
-                               static_cast<uint64_t>(num_layers) * NKV, &err);
+                               static_cast<uint64_t>(num_layers) * NKV, kv_box, &err);
       if (rc == QMK_OK)
         rc = qmk_tc::make_map_kv(&map_vc, v_cache, static_cast<uint64_t>(pos0 + T), static_cast<uint64_t>(max_seq_len),
-                                 static_cast<uint64_t>(num_layers) * NKV, &err);
+                                 static_cast<uint64_t>(num_layers) * NKV, kv_box, &err);
       if (rc != QMK_OK) break;
     }
     PF_CUDA(cudaMemcpyAsync(w.tokens, token_ids_host + c0, sizeof(int) * T, cudaMemcpyHostToDevice, stream));
@@ -931,12 +937,14 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
                                     static_cast<size_t>(l) * layer_stride,
                                     env.attn_tc ? attn_scale * 1.4426950408889634f : 0.f));
       if (l == num_layers - 1) break;   // the cache is complete; nothing downstream of the last layer is kept
-      const bool attn_chains = attention_by_chains(T);   // (packed prompts: T = all their rows, one chunk)
-      if (env.attn_tc)
-        PF_CUDA(qmk_tc::launch_kernel(attn_chains ? qmk_attn::causal_attention_tc<true> : qmk_attn::causal_attention_tc<false>,
-                                      dim3(pk ? pk_items : (T + qmk_attn::TQ - 1) / qmk_attn::TQ * (attn_chains ? NQ : NKV)),
-                                      dim3(qmk_attn::THREADS), qmk_attn::SMEM_BYTES, stream, w.map_qh, map_kc, map_vc, w.map_cattn, l * NKV, T,
-                                      pos0, w.status, static_cast<unsigned long long>(env.timeout_ms) * 1000000ull,
+      if (attn_pairs)
+        PF_CUDA(qmk_tc::launch_kernel(qmk_attn_pairs::causal_attention_pairs, dim3((T + qmk_attn_pairs::TQ - 1) / qmk_attn_pairs::TQ * NKV),
+                                      dim3(qmk_attn_pairs::THREADS), qmk_attn_pairs::SMEM_BYTES, stream, w.map_qh, map_kc, map_vc,
+                                      w.map_cattn, l * NKV, T, pos0, w.status, static_cast<unsigned long long>(env.timeout_ms) * 1000000ull));
+      else if (env.attn_tc)
+        PF_CUDA(qmk_tc::launch_kernel(qmk_attn::causal_attention_tc, dim3(pk ? pk_items : (T + qmk_attn::TQ - 1) / qmk_attn::TQ * NQ),
+                                      dim3(qmk_attn::THREADS), qmk_attn::SMEM_BYTES, stream, w.map_qh, map_kc, map_vc, l * NKV, w.attn, T,
+                                      pos0, attn_scale, w.status, static_cast<unsigned long long>(env.timeout_ms) * 1000000ull,
                                       pk ? reinterpret_cast<const int4 *>(w.packed + PK_ITEMS_OFF) : nullptr,
                                       pk ? reinterpret_cast<const CUtensorMap *>(w.packed + PK_MAPS_OFF) : nullptr));
       else if (split) {

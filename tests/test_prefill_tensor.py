@@ -257,7 +257,7 @@ def test_launch_overlap_changes_nothing_but_time(C, fmt, lens):
 def test_attention_kernels_agree(C, before, n):
     """The tcgen05 attention against the mma.sync kernel on the same chunk: less than a key tile, one key over, an odd and an even
     number of key tiles, prompts that continue at a position inside a tile (so that the diagonal crosses it), chunks whose
-    query tiles run as chains of one head and as pairs of heads.  Both round queries, keys and softmax weights to fp16 and
+    query tiles run by one head and by two.  Both round queries, keys and softmax weights to fp16 and
     add in fp32; what differs is the order of sums: 1e-2 on cache values, as between any two passes of this path."""
     vocab, L = 2048, 4352 if n > 2048 else 2048
     w = S.make_weights(seed=51, num_layers=3, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
