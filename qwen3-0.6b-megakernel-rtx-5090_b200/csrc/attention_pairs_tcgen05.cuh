@@ -2,8 +2,7 @@
 //
 // A CTA works on two SLOTS of 128 query rows: one 128-query tile of the two heads that share a kv head, and so every key and value
 // tile.  Keys and values come from the fp16 cache in tiles of 128 rows through two-stage rings fed by 3-D tiled TMA loads (no
-// multicast; rows past the end of the
-// sequence are outside the tensor map's extent and arrive as zeros).  Per slot h and key tile u
+// multicast; rows past the end of the sequence are outside the tensor map's extent and arrive as zeros).  Per slot h and tile u
 //   S_h[128 x 128]  = Q_h . K_u^T    tcgen05.mma from shared memory, fp32 scores in 128 TMEM columns
 //   P_h             = exp2(S_h - m)  four warps, one query row per thread: tcgen05.ld, causal mask, row maximum, exp2; P as
 //                                    fp16 pairs back into the first 64 of the slot's score columns (tcgen05.st)
