@@ -16,7 +16,6 @@
 #include "prefill_sm100.h"
 #include "prefill_kernels.cuh"
 #include "attention_tcgen05.cuh"
-#include "attention_pairs_tcgen05.cuh"
 #include "decode_attention_mma.cuh"
 #include "engine_internal.h"
 #include <vector>
@@ -116,15 +115,14 @@ int make_map_b(CUtensorMap *map, const void *ptr, uint64_t rows, int K, uint32_t
 }
 
 // 3-D tensor map of an fp16 KV cache [heads][max_seq_len][128] of which the first `rows` positions of every head are
-// valid: boxes of 64 dims x `box_rows` positions of one head, 128-byte swizzle; positions >= rows read as zeros.
-int make_map_kv(CUtensorMap *map, const void *cache, uint64_t rows, uint64_t max_seq_len, uint64_t heads, uint32_t box_rows,
-                std::string *err) {
+// valid: boxes of 64 dims x 64 positions of one head, 128-byte swizzle; positions >= rows read as zeros.
+int make_map_kv(CUtensorMap *map, const void *cache, uint64_t rows, uint64_t max_seq_len, uint64_t heads, std::string *err) {
   EncodeTiledFn enc = encoder();
   if (!enc) { *err = "cuTensorMapEncodeTiled is not available from this driver"; return QMK_ERR_CUDA; }
   if (reinterpret_cast<uintptr_t>(cache) & 15u) { *err = "cache not 16-byte aligned"; return QMK_ERR_BAD_ARGUMENT; }
   const cuuint64_t dims[3] = {128, rows, heads};
   const cuuint64_t strides[2] = {256, max_seq_len * 256};
-  const cuuint32_t box[3] = {64, box_rows, 1};
+  const cuuint32_t box[3] = {64, 64, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void *>(cache), dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -243,9 +241,6 @@ int ensure_gemm_attrs(std::string *err) {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(qmk_attn::SMEM_BYTES));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(qmk_attn_pairs::causal_attention_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(qmk_attn_pairs::SMEM_BYTES));
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(qmk_pf::decode_attention_ring, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                qmk_pf::DAR_SMEM_BYTES);
@@ -461,13 +456,6 @@ namespace {
 constexpr unsigned int PREFILL_RING_BYTES = 96 * 1024;
 constexpr int PAIR_MIN_ROWS = 512;
 constexpr int EXPAND_MIN_ROWS = 384;
-// Chunks of one prompt take the attention kernel with both heads of a kv head per CTA once it has a third more CTAs than SMs: with
-// fewer, the kernel with one head per CTA and two chains of key tiles fills the SMs better (2000 / 2500 / 3000 / 4000 / 8191
-// tokens 3.20 / 4.16 / 4.93 / 6.77 / 17.6 ms by one head, 3.34 / 4.26 / 4.95 / 6.59 / 16.8 by two).  Packed prompts, whose
-// sequences are a fraction of a chunk, keep the former.
-bool attention_by_pairs(int rows) {
-  return (rows + qmk_attn_pairs::TQ - 1) / qmk_attn_pairs::TQ * qmk_attn_pairs::NKV * 3 >= 4 * qmk_tc::gemm_sm_count();
-}
 constexpr int CHUNK = 4096;         // prompt tokens per pass over the weights (a multiple of the GEMM's 128)
 constexpr int MAX_LAYERS = 48;
 
@@ -478,7 +466,7 @@ struct Workspace {                  // per device, allocated on first use, never
   __half *xn = nullptr, *attn = nullptr, *act = nullptr;
   unsigned int *status = nullptr;
   CUtensorMap map_xn, map_attn, map_act, map_qh;
-  CUtensorMap map_cq, map_ck, map_cv, map_cact, map_co, map_cdown, map_cattn;   // outputs of the pair GEMMs and of the attention
+  CUtensorMap map_cq, map_ck, map_cv, map_cact, map_co, map_cdown;   // outputs of the pair GEMMs
   CUtensorMap map_xn2, map_attn2, map_act2;   // split activations: rows of hi and lo halves
   // batched decode: per-sequence state and the logits of one step
   int *positions = nullptr, *start_positions = nullptr;
@@ -570,8 +558,7 @@ int ensure_workspace(Workspace &w, int rows, bool *no_room = nullptr) {
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_xn2, w.xn, C, 2 * H, qmk_gemm::BM, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_attn2, w.attn, C, 2 * QS, qmk_gemm::BM, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&w.map_act2, w.act, C, 2 * I, qmk_gemm::BM, &err);
-  // outputs of the pair GEMMs: q, k, v as fp16, the SwiGLU, fp32 sums (or partial matrices); of the attention
-  if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_cattn, w.attn, C, QS, true, &err);
+  // outputs of the pair GEMMs: q, k, v as fp16, the SwiGLU, fp32 sums (or partial matrices)
   if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_cq, w.q, C, QS, true, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_ck, w.k, C, KVS, true, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_cv, w.v, C, KVS, true, &err);
@@ -735,10 +722,10 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
       ptrs[2 * s] = reinterpret_cast<unsigned long long>(pk->k_caches[s]);
       ptrs[2 * s + 1] = reinterpret_cast<unsigned long long>(pk->v_caches[s]);
       int mrc = qmk_tc::make_map_kv(&maps[2 * s], pk->k_caches[s], static_cast<uint64_t>(len), static_cast<uint64_t>(max_seq_len),
-                                    static_cast<uint64_t>(num_layers) * NKV, qmk_attn::TK, &merr);
+                                    static_cast<uint64_t>(num_layers) * NKV, &merr);
       if (mrc == QMK_OK)
         mrc = qmk_tc::make_map_kv(&maps[2 * s + 1], pk->v_caches[s], static_cast<uint64_t>(len), static_cast<uint64_t>(max_seq_len),
-                                  static_cast<uint64_t>(num_layers) * NKV, qmk_attn::TK, &merr);
+                                  static_cast<uint64_t>(num_layers) * NKV, &merr);
       if (mrc != QMK_OK) return qmk_internal::report(mrc, merr);
       for (int qt = 0; qt * qmk_attn::TQ < len; ++qt) {
         const int last = (qt + 1) * qmk_attn::TQ < len ? (qt + 1) * qmk_attn::TQ - 1 : len - 1;
@@ -855,14 +842,12 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     CUtensorMap map_kc, map_vc;   // the caches up to this chunk's last position, all layers
     memset(&map_kc, 0, sizeof(map_kc));
     memset(&map_vc, 0, sizeof(map_vc));
-    const bool attn_pairs = env.attn_tc && !pk && attention_by_pairs(T);
-    const uint32_t kv_box = attn_pairs ? qmk_attn_pairs::TK : qmk_attn::TK;
     if (env.attn_tc && !pk) {
       rc = qmk_tc::make_map_kv(&map_kc, k_cache, static_cast<uint64_t>(pos0 + T), static_cast<uint64_t>(max_seq_len),
-                               static_cast<uint64_t>(num_layers) * NKV, kv_box, &err);
+                               static_cast<uint64_t>(num_layers) * NKV, &err);
       if (rc == QMK_OK)
         rc = qmk_tc::make_map_kv(&map_vc, v_cache, static_cast<uint64_t>(pos0 + T), static_cast<uint64_t>(max_seq_len),
-                                 static_cast<uint64_t>(num_layers) * NKV, kv_box, &err);
+                                 static_cast<uint64_t>(num_layers) * NKV, &err);
       if (rc != QMK_OK) break;
     }
     PF_CUDA(cudaMemcpyAsync(w.tokens, token_ids_host + c0, sizeof(int) * T, cudaMemcpyHostToDevice, stream));
@@ -937,11 +922,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
                                     static_cast<size_t>(l) * layer_stride,
                                     env.attn_tc ? attn_scale * 1.4426950408889634f : 0.f));
       if (l == num_layers - 1) break;   // the cache is complete; nothing downstream of the last layer is kept
-      if (attn_pairs)
-        PF_CUDA(qmk_tc::launch_kernel(qmk_attn_pairs::causal_attention_pairs, dim3((T + qmk_attn_pairs::TQ - 1) / qmk_attn_pairs::TQ * NKV),
-                                      dim3(qmk_attn_pairs::THREADS), qmk_attn_pairs::SMEM_BYTES, stream, w.map_qh, map_kc, map_vc,
-                                      w.map_cattn, l * NKV, T, pos0, w.status, static_cast<unsigned long long>(env.timeout_ms) * 1000000ull));
-      else if (env.attn_tc)
+      if (env.attn_tc)
         PF_CUDA(qmk_tc::launch_kernel(qmk_attn::causal_attention_tc, dim3(pk ? pk_items : (T + qmk_attn::TQ - 1) / qmk_attn::TQ * NQ),
                                       dim3(qmk_attn::THREADS), qmk_attn::SMEM_BYTES, stream, w.map_qh, map_kc, map_vc, l * NKV, w.attn, T,
                                       pos0, attn_scale, w.status, static_cast<unsigned long long>(env.timeout_ms) * 1000000ull,

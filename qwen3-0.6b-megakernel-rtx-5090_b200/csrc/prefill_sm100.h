@@ -68,7 +68,7 @@ struct PackedRow { uint32_t data_bytes, bs_off, scale_off, pitch; };
 PackedRow packed_row(int wq, int K);
 int make_map_packed(CUtensorMap *map, const void *ptr, uint64_t rows, int K, uint32_t box_rows, int wq, std::string *err);
 int make_map_b(CUtensorMap *map, const void *ptr, uint64_t rows, int K, uint32_t box_rows, int wq, std::string *err);
-int make_map_kv(CUtensorMap *map, const void *cache, uint64_t rows, uint64_t max_seq_len, uint64_t heads, uint32_t box_rows, std::string *err);
+int make_map_kv(CUtensorMap *map, const void *cache, uint64_t rows, uint64_t max_seq_len, uint64_t heads, std::string *err);
 int make_map_f16(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, std::string *err);
 int gemm_sm_count();
 int gemm_box_n(int M, int N);

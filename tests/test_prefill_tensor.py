@@ -256,8 +256,8 @@ def test_launch_overlap_changes_nothing_but_time(C, fmt, lens):
 @pytest.mark.parametrize("before,n", [(0, 64), (0, 65), (0, 129), (0, 320), (77, 51), (63, 1), (1000, 200), (130, 1500), (0, 4225)])
 def test_attention_kernels_agree(C, before, n):
     """The tcgen05 attention against the mma.sync kernel on the same chunk: less than a key tile, one key over, an odd and an even
-    number of key tiles, prompts that continue at a position inside a tile (so that the diagonal crosses it), chunks whose
-    query tiles run by one head and by two.  Both round queries, keys and softmax weights to fp16 and
+    number of key tiles, prompts that continue at a position inside a tile (so that the diagonal crosses it), two
+    chunks.  Both round queries, keys and softmax weights to fp16 and
     add in fp32; what differs is the order of sums: 1e-2 on cache values, as between any two passes of this path."""
     vocab, L = 2048, 4352 if n > 2048 else 2048
     w = S.make_weights(seed=51, num_layers=3, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
@@ -279,3 +279,19 @@ def test_attention_kernels_agree(C, before, n):
     for a, b, again in zip(*rows):
         assert bool(torch.isfinite(a).all()) and torch.equal(a, again)
         assert float((a - b).abs().max()) < 1e-2
+
+
+@pytest.mark.parametrize("cuts", [(1100, 4000), (1500, 3000, 4096), (2900, 4000)])
+def test_rows_do_not_depend_on_how_a_prompt_is_cut(C, cuts):
+    """A prompt in one call and in calls of 1024 tokens and more: every product then adds in the same order (K of the O and
+    down products in two parts, the keys of a query in the same tiles and chains), so the cache rows are equal bit for bit."""
+    vocab, L = 2048, 4352
+    w = S.make_weights(seed=61, num_layers=3, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    ids = S.make_prompt(cuts[-1], seed=len(cuts), vocab_size=vocab)
+    one, parts = _engine(w, L, "tensor"), _engine(w, L, "tensor")
+    one.prefill_ids(ids)
+    for a, b in zip((0,) + cuts, cuts):
+        parts.prefill_ids(ids[a:b])
+    for x, y in ((one._k_cache, parts._k_cache), (one._v_cache, parts._v_cache)):
+        assert float(x[:, :, :cuts[-1]].float().abs().max()) > 0.1
+        assert torch.equal(x[:, :, :cuts[-1]], y[:, :, :cuts[-1]])
