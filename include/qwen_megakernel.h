@@ -410,6 +410,10 @@ int qmk_selftest_wait_timeout(int budget_us);
  * budget_us, all roles leave, TMEM is freed; returns QMK_ERR_WAIT_TIMEOUT when that happened as designed. */
 int qmk_selftest_gemm_wait_timeout(int budget_us);
 
+/* The same for the pairs of CTAs that multiply more than 512 rows.  what = 1: no loads; 2: the issuing thread gives up behind its
+ * first tile, with a ring of copies in flight; 3: the second CTA of the pair loads nothing. */
+int qmk_selftest_gemm_pair_wait_timeout(int budget_us, int what);
+
 #ifdef __cplusplus
 }
 #endif

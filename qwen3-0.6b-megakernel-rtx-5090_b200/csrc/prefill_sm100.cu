@@ -429,6 +429,7 @@ int launch_gemm_pair(int mode, const CUtensorMap &map_a, int ngroups, const CUte
   a.m_tiles = (M + qmk_pair::TM - 1) / qmk_pair::TM;
   a.splits = splits;
   a.kblocks = K / qmk_pair::BK / splits;
+  a.selftest = 0;
   const int tiles = a.m_tiles * a.n_tiles * splits, pairs = std::min(tiles, sm_count() / 2);
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
   const cudaError_t e = launch_kernel(pair_kernel(mode, a.row_scale[0] != nullptr), dim3(2 * pairs), dim3(qmk_pair::THREADS), qmk_pair::SMEM_BYTES, stream,
@@ -1331,6 +1332,43 @@ extern "C" int qmk_selftest_gemm_wait_timeout(int budget_us) {
   cudaFree(ab);
   cudaFree(c);
   cudaFree(status);
+  if (rc != QMK_OK && rc != QMK_ERR_WAIT_TIMEOUT) return qmk_internal::report(rc, err);
+  return rc;
+}
+
+// The same of the pair kernel: one pair, two 256 x 256 tiles of eight K blocks.  Beside loads that are never issued: the second CTA's
+// alone (the first has a ring of copies in flight whose barriers cannot complete), and an issuer that gives up behind the first
+// tile (MMAs and a ring of copies in flight).  All end in status 4 with the pair's copies and MMAs drained.
+extern "C" int qmk_selftest_gemm_pair_wait_timeout(int budget_us, int what) {
+  std::string err;
+  if (budget_us < 1 || budget_us > 1000000 || what < qmk_pair::NO_LOADS || what > qmk_pair::SECOND_CTA_NO_LOADS)
+    return qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "budget_us must be in [1, 1e6], what in [1, 3]");
+  int rc = qmk_tc::ensure_gemm_attrs(&err);
+  if (rc != QMK_OK) return qmk_internal::report(rc, err);
+  constexpr int M = 2 * qmk_pair::TM, N = qmk_pair::TN, K = 8 * qmk_pair::BK;
+  unsigned char *buf = nullptr;            // A, B, C, status
+  constexpr size_t at_b = sizeof(__half) * M * K, at_c = at_b + sizeof(__half) * N * K, at_status = at_c + sizeof(float) * M * N;
+  PF_CUDA(cudaMalloc(&buf, at_status + 16));
+  cudaError_t e = cudaMemset(buf, 0, at_status + 16);
+  CUtensorMap ma, mb, mc;
+  rc = qmk_tc::make_map_f16(&ma, buf, M, K, 128, &err);
+  if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&mb, buf + at_b, N, K, 128, &err);
+  if (rc == QMK_OK) rc = qmk_tc::make_map_c(&mc, buf + at_c, M, N, false, &err);
+  if (rc == QMK_OK && e == cudaSuccess) {
+    qmk_pair::Args a;
+    for (int g = 0; g < 3; ++g) { a.N[g] = g == 0 ? N : 0; a.row_scale[g] = nullptr; }
+    a.m_tiles = 2; a.n_tiles = 1; a.splits = 1;
+    a.kblocks = K / qmk_pair::BK;
+    a.selftest = what;
+    qmk_pair::gemm_pair_kernel<0, false><<<dim3(2), qmk_pair::THREADS, qmk_pair::SMEM_BYTES>>>(
+        ma, mb, mb, mb, mc, mc, mc, a, reinterpret_cast<unsigned int *>(buf + at_status), static_cast<unsigned long long>(budget_us) * 1000ull);
+    unsigned int host[4] = {0, 0, 0, 0};
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpy(host, buf + at_status, 16, cudaMemcpyDeviceToHost);
+    rc = static_cast<int>(host[0]);
+  }
+  if (e != cudaSuccess) { rc = QMK_ERR_CUDA; err = std::string("gemm self test: ") + cudaGetErrorString(e); }
+  cudaFree(buf);
   if (rc != QMK_OK && rc != QMK_ERR_WAIT_TIMEOUT) return qmk_internal::report(rc, err);
   return rc;
 }

@@ -136,3 +136,17 @@ def test_bounded_wait_reports_timeout_and_frees_tmem(C):
         assert C.selftest_gemm_wait_timeout(300) == 4
     a = torch.ones(128, 64, dtype=torch.float16, device="cuda")
     assert torch.equal(C.gemm_f16_tn(a, a), torch.full((128, 128), 64.0, device="cuda"))
+
+
+@pytest.mark.parametrize("what", [1, 2, 3])
+def test_bounded_waits_of_a_pair_drain_both_ctas(C, what):
+    """Pairs of CTAs: no loads, an issuer that stops behind a tile (MMAs and a ring of copies in flight), a second CTA without loads
+    (the first one's copies wait on barriers that its partner completes).  Status 4, and pairs after it are exact: they find
+    all 512 TMEM columns and shared memory that no late copy writes."""
+    g = torch.Generator("cpu").manual_seed(what)
+    a = torch.randint(-3, 4, (1152, 512), generator=g).to(torch.float16).cuda()
+    b = torch.randint(-3, 4, (4096, 512), generator=g).to(torch.float16).cuda()
+    want = a.float() @ b.float().T
+    for _ in range(3):
+        assert C.selftest_gemm_pair_wait_timeout(300, what) == 4
+        assert torch.equal(C.gemm_f16_tn(a, b), want)
