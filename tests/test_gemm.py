@@ -17,7 +17,8 @@ def C(built_library):
 
 
 @pytest.mark.parametrize("m,n,k", [(128, 128, 64), (128, 128, 256), (256, 1024, 1024), (512, 3072, 1024), (128, 1024, 3072),
-                                   (1024, 2048, 512), (512, 2048, 256)])   # N tiles of 32, 32, 32, 128, 32, 128 and 64 columns on 148 SMs
+                                   (1024, 2048, 512), (512, 2048, 256), (384, 6144, 512)])
+# N tiles of 32, 32, 32, 128 and 32 columns on 148 SMs, pairs of CTAs, 64 and 128 columns
 def test_matches_torch(C, m, n, k):
     g = torch.Generator("cpu").manual_seed(m + n + k)
     a = torch.randn(m, k, generator=g).to(torch.float16).cuda()
@@ -29,12 +30,13 @@ def test_matches_torch(C, m, n, k):
     assert err < 1e-3 * (k ** 0.5) * 4
 
 
-@pytest.mark.parametrize("m,n,k", [(640, 256, 64), (640, 2304, 128), (896, 512, 448), (1024, 1024, 384), (1152, 4096, 1024), (4096, 1024, 3072)])
+@pytest.mark.parametrize("m,n,k", [(640, 256, 64), (640, 2304, 128), (896, 512, 448), (1024, 1024, 384), (1152, 4096, 1024), (4096, 1024, 3072),
+                                   (4096, 4096, 128), (3968, 4096, 448)])
 def test_pairs_of_ctas_match_torch(C, m, n, k):
     """More than 512 rows run on pairs of CTAs with 256 x 256 tiles: K of one block, of fewer blocks than the ring has stages, of
     a full ring and one block over; an odd number of 128-row tiles (the last pair's second half lies past the matrix); fewer
-    tiles than pairs, and several per pair (the two accumulator buffers in turn).  A and B are small integers, so every sum
-    is exact and each element is compared for equality."""
+    tiles than pairs, and two to four per pair (from the third on an accumulator buffer is used again, which both CTAs'
+    epilogues have to give back).  A and B are small integers, so every sum is exact and each element is compared for equality."""
     g = torch.Generator("cpu").manual_seed(m + n + k)
     a = torch.randint(-3, 4, (m, k), generator=g).to(torch.float16).cuda()
     b = torch.randint(-3, 4, (n, k), generator=g).to(torch.float16).cuda()

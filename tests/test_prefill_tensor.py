@@ -30,10 +30,10 @@ def _engine(w, max_seq_len, mode, **kw):
                    verbose=False, max_seq_len=max_seq_len, prefill_mode=mode, **kw)
 
 
-@pytest.mark.parametrize("n_prompt", [1, 37, 128, 700, 2300])
+@pytest.mark.parametrize("n_prompt", [1, 37, 128, 513, 700, 800, 2300])
 def test_cache_and_next_tokens_match_oracle(C, n_prompt):
-    """Prompt lengths below a tile, one tile exactly, several tiles with a ragged tail, and two chunks
-    (2048 + 252)."""
+    """Prompt lengths below a tile, one tile exactly, several tiles with a ragged tail (an odd and an even number of row tiles with K
+    of the O and down products in four parts on pairs of CTAs), and many."""
     vocab, steps, L = 2048, 4, 2560
     w = S.make_weights(seed=12, num_layers=3, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
     ids = S.make_prompt(n_prompt + 1, seed=n_prompt, vocab_size=vocab)
@@ -281,17 +281,27 @@ def test_attention_kernels_agree(C, before, n):
         assert float((a - b).abs().max()) < 1e-2
 
 
-@pytest.mark.parametrize("cuts", [(1100, 4000), (1500, 3000, 4096), (2900, 4000)])
-def test_rows_do_not_depend_on_how_a_prompt_is_cut(C, cuts):
+@pytest.mark.parametrize("fmt,cuts", [("fp16", (1100, 4000)), ("fp16", (1500, 3000, 4096)), ("fp16", (2900, 4000)), ("fp16", (4096, 7500)),
+                                      ("nvfp4", (1100, 2300)), ("fp16", (400, 800)), ("fp16", (400, 513)), ("fp16", (130, 640)), ("fp8", (400, 800)),
+                                      ("nvfp4", (385, 770))])
+def test_rows_do_not_depend_on_how_a_prompt_is_cut(C, fmt, cuts):
     """A prompt in one call and in calls of 1024 tokens and more: every product then adds in the same order (K of the O and
-    down products in two parts, the keys of a query in the same tiles and chains), so the cache rows are equal bit for bit."""
-    vocab, L = 2048, 4352
+    down products in two parts, the keys of a query in the same tiles and chains), so the cache rows are equal bit for bit.  So
+    are those of a prompt below 1024 tokens on pairs of CTAs and its pieces of at most 512 on single ones (K in four parts,
+    one RMSNorm kernel): every epilogue of either kernel, with row scales too."""
+    import quantize as Q
+    vocab, L = 2048, 7680 if cuts[-1] > 4300 else 4352
     w = S.make_weights(seed=61, num_layers=3, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    if fmt != "fp16":
+        w, _ = (Q.quantize_weights_fp8 if fmt == "fp8" else Q.quantize_weights_nvfp4)(w)
     ids = S.make_prompt(cuts[-1], seed=len(cuts), vocab_size=vocab)
-    one, parts = _engine(w, L, "tensor"), _engine(w, L, "tensor")
-    one.prefill_ids(ids)
-    for a, b in zip((0,) + cuts, cuts):
-        parts.prefill_ids(ids[a:b])
+    try:
+        one, parts = (_engine(w, L, "tensor", weight_format=fmt) for _ in range(2))
+        one.prefill_ids(ids)
+        for a, b in zip((0,) + cuts, cuts):
+            parts.prefill_ids(ids[a:b])
+    finally:
+        C.set_weight_format("fp16")
     for x, y in ((one._k_cache, parts._k_cache), (one._v_cache, parts._v_cache)):
         assert float(x[:, :, :cuts[-1]].float().abs().max()) > 0.1
         assert torch.equal(x[:, :, :cuts[-1]], y[:, :, :cuts[-1]])
