@@ -395,11 +395,13 @@ class BatchDecoder:
     def auto_engine(cls, n: int, weight_format: str, vocab_size: int, max_seq_len: int, ctas: int, free_bytes: int) -> str:
         """Persistent up to three sequences, gemm from five on (NVFP4 rows: always gemm).  Four: persistent where the launch
         runs on the tensor cores - a grid of at least 112 CTAs, whole ring chunks of vocabulary, room for the K-major
-        copies; its group-per-sequence form takes 1.9 ms a step - and contexts end before the GEMM step overtakes it.
-        Measured, us per step of four fp16 sequences at 1024 / 4096 / 8000 tokens: 779 / 1129 / 1546 persistent, 1127 / 1331 /
-        1583 gemm (slopes 106 and 63 per 1000 tokens); FP8 rows 818 / 1117 / 1499 and 1281 / 1478 / 1727 (one long context
-        among short ones costs either less).  A four-slot serving job of prompts of 64 to 2048 tokens, 128 new ones each,
-        tensor-core prefill: 0.96 s persistent, prefills between the rounds; 1.36 s gemm with prefills beside them."""
+        copies; its group-per-sequence form takes 1.9 ms a step - and the cache has room for 8192 rows at most (FP8 12288).
+        Measured, us per step of four fp16 sequences at 64 / 1024 / 2048 / 4096 / 8000 tokens: 711 / 799 / 913 / 1141 / 1543
+        persistent, 808 / 856 / 925 / 1060 / 1309 gemm; FP8 rows 746 / 822 / 925 / 1118 / 1495 and 977 / 1025 / 1081 / 1215 / 1456
+        (one long context among short ones costs either less).  So the GEMM step is the faster one behind about 2200 tokens
+        (FP8 6500); the bound on the rows dates from a GEMM step of 1127 / 1331 / 1583 us at 1024 / 4096 / 8000.  A four-slot
+        serving job, 32 prompts of 64 to 2048 tokens, 128 new ones each, tensor-core prefill: 0.95 s persistent, prefills
+        between the rounds; 0.99 s gemm with prefills beside them."""
         if weight_format == "nvfp4" or n > cls.MAX_SEQUENCES:
             return "gemm"
         if n < cls.MAX_SEQUENCES or vocab_size % 128:      # (the GEMM step reads vocabularies of whole tiles only)

@@ -9,8 +9,8 @@
 //   P            = exp2(S_j - m) with the causal mask four warps, one query row per thread (tcgen05.ld), P rounded to
 //                                                    fp16 and stored to shared memory as the next A operand
 //   O[128 x 128] += P[128 x 64] . V_j[64 x 128]      tcgen05.mma, B read MN-major straight from the [key][dim] rows
-// An MMA of 128 rows occupies the tensor pipe for about 70 cycles whatever its N (measured: eight N = 64 score MMAs
-// and four N = 128 P . V MMAs per tile took 1150 cycles of issue time), so the scores are issued 128 keys wide.
+// Fewer and wider MMAs: the scores are issued 128 keys wide.  (Eight N = 64 score MMAs and four N = 128 P . V MMAs per tile took
+// 1150 cycles of issue, about 70 each whatever their N, when a `lane == 0` thread issued them; see elect_one.)
 // TWO CHAINS per CTA: even key tiles belong to chain 0, odd ones to chain 1, each with its own four softmax warps, P
 // tile, running (maximum, sum) and O accumulator; at the end the two partial results are merged per row like two
 // splits of the key range.  One tile's chain - scores committed, TMEM read, P stored and fenced, P . V issued and
@@ -181,8 +181,8 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   pdl_wait();   // queries and this chunk's cache rows come from the kernel launched just before
-  // the query tile and the K ring's first fill go out at once (warp 0 has just initialised the barriers); a CTA's fixed costs weigh as much as its first key tiles
-  if (warp == 0) __syncwarp();
+  // the query tile and the K ring's first fill go out at once; a CTA's fixed costs weigh as much as its first key tiles
+  if (warp == 0) __syncwarp();   // (thread 0 has initialised the barriers, the elected thread uses them)
   auto load_tile = [&](bool is_v, int j) {
     const int s = j % STAGES;
     const uint32_t full = is_v ? v_full(s) : k_full(s);
@@ -202,7 +202,7 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   if (warp == 0 && elect_one()) {
     // the query tile: fp16, already times scale * log2 e (the softmax is an exp2), as two [128 x 64] boxes in the
     // K-major 128-byte-swizzled layout the score MMAs read; rows past the live ones hold other tokens' or stale
-    // finite values and are never stored
+    // values, stay in their own rows of every product and are never stored
     bar_expect_tx(q_full, Q_BYTES);
     tma_load_2d(base, &map_q, head * D, q0, q_full);
     tma_load_2d(base + TQ * 128, &map_q, head * D + 64, q0, q_full);

@@ -1,9 +1,13 @@
 // C[M x N] = A[M x K] * B[N x K]^T (fp16 operands, fp32 accumulation) for long chunks: pairs of CTAs on one 256 x 256 tile.
 //
-// What bounds a prefill GEMM here is the 64 bytes per cycle that an SM takes in from L2.  A 128 x 256 tile of one CTA
-// (gemm_f16_tn_kernel) brings in 48 KB per 64-wide K block, 768 cycles, for 512 cycles of tensor arithmetic (752 measured);
-// its 128 x 128 gate/up tile 32 KB, 512 cycles, for 256.  With tcgen05.mma.cta_group::2 each CTA of a pair brings its own 128
-// rows of A and HALF of the 256 rows of B, and both halves feed both tensor cores: 32 KB for 512 cycles of arithmetic.
+// With tcgen05.mma.cta_group::2 each CTA of a pair brings its own 128 rows of A and HALF of the 256 rows of B, and both halves feed
+// both tensor cores: 32 KB for 512 cycles of arithmetic per 64-wide K block.  Measured per K block, from the cycles of 4096 x 4096
+// products of K = 1536 and 3072: 525 (operands zero) to 555 (random).  A launch's remaining time is its start, its last
+// epilogue and the pairs without a tile in the last round (2048 rows: tensor pipe 57 and 64 % active in the q/k/v and gate/up
+// products, 40 and 51 % in O and down, whose 64 tiles are one for each of 64 pairs).
+// What single-CTA tiles of 128 x 256 lose is not their main loop: stand-alone, with every SM at work on operands in L2, loads of
+// 48 KB take 458 cycles (107 bytes per cycle and SM; 32 KB 367; one SM alone 125 bytes per cycle), N = 256 MMAs of resident
+// operands 512, and both together 513.  What is left is that they start and end a CTA once per tile.
 //
 // Persistent: a pair takes tiles pair, pair + pairs, ... (m fastest), and the accumulator has two buffers of 256 TMEM columns,
 // so the epilogue of one tile runs under the main loop of the next.  Roles per CTA: warp 0 loads (one thread), warp 1 of

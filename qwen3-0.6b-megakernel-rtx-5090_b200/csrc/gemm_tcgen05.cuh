@@ -1,9 +1,9 @@
 // C[M x N] (fp32) = A[M x K] (fp16, row-major) * B[N x K]^T (fp16, row-major) on the sm_100a tensor cores.
 //
-// One CTA per 128 x BN output tile (BN = 128, or 64 when 128-wide tiles would leave most SMs idle),
+// One CTA per 128 x BN output tile (BN = 128, or 64 or 32 when wider tiles would leave SMs idle),
 // warp-specialised:
 //   warp 0   : one thread streams 128 x 64 tiles of A and BN x 64 tiles of B with tiled TMA loads (128-byte
-//              swizzle) into a 4-stage shared-memory ring (full/empty mbarriers);
+//              swizzle) into a ring of 2 to 10 stages in shared memory (full/empty mbarriers);
 //   warp 1   : allocates BN TMEM columns, then one thread issues tcgen05.mma (M 128, N BN, K 16; four per
 //              64-wide K block) with shared-memory matrix descriptors, commits each stage back to the
 //              producer and finally commits the accumulator to the epilogue;
@@ -53,7 +53,7 @@ constexpr int BM = 128, BK = 64;                 // BK * 2 bytes = one 128-byte 
 // latency of its K loop, so the whole K extent of a 1024-wide matrix is in flight at once).
 constexpr int stages_for(int bn, int wq = 0, int ah = 1) {
   if (ah == 2) return wq || bn == 128 ? 4 : 5;
-  return wq ? (bn == 32 ? 8 : bn == 64 ? 6 : bn == 128 ? 4 : 2) : (bn == 32 ? 10 : bn == 64 ? 8 : bn == 128 ? 6 : 4);
+  return wq ? (bn == 32 ? 8 : bn == 64 ? 6 : 4) : (bn == 32 ? 10 : bn == 64 ? 8 : 6);
 }
 constexpr int MAX_GROUPS = 3;   // matrices sharing one A operand that one launch can multiply (q/k/v, gate/up)
 constexpr int THREADS = 192;                     // fp16 weights: producer warp, MMA warp, four epilogue warps

@@ -12,8 +12,8 @@
 
 namespace qmk_pf {
 
-// Programmatic dependent launch: the kernels of a decode step are launched with the stream-serialisation attribute,
-// so kernel n + 1 may be scheduled as soon as every CTA of kernel n has executed pdl_trigger(); pdl_wait() then blocks
+// Programmatic dependent launch: the kernels of a batched decode step, and those of a prefill pass behind its first, are
+// launched with the stream-serialisation attribute, so kernel n + 1 may be scheduled as soon as every CTA of kernel n has executed pdl_trigger(); pdl_wait() then blocks
 // until kernel n has COMPLETED and its writes are visible.  Whatever a kernel does before pdl_wait() - barrier and
 // TMEM set-up, tensor-map prefetch, streaming weights or cache rows no kernel of the step writes - overlaps its
 // predecessor.  Every kernel of the chain waits before its first dependent read and before any global write, and

@@ -164,8 +164,8 @@ int gemm_sm_count() { return sm_count(); }
 int gemm_box_n(int M, int N) { return pick_box_n(M, N, 1); }
 int gemm_box_n_fused(int M, int N) { return pick_box_n(M, N, 2); }
 
-// Launches of a decode step carry the programmatic-stream-serialisation attribute (see pdl_wait in
-// prefill_kernels.cuh); the step builder switches it on for the calling thread, everything else launches plainly.
+// Launches of a decode step, and of a prefill chunk behind its first kernel, carry the programmatic-stream-serialisation
+// attribute (see pdl_wait in prefill_kernels.cuh): who builds the chain switches it on for the calling thread.
 thread_local bool t_pdl = false;
 PdlScope::PdlScope(bool on) : prev_(t_pdl) { t_pdl = on; }
 PdlScope::~PdlScope() { t_pdl = prev_; }
@@ -179,10 +179,6 @@ static GemmKernel gemm_kernel_wq(int bn, bool fuse) {
   if (fuse) return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, true, WQ, 1, RS> : qmk_gemm::gemm_f16_tn_kernel<64, true, WQ, 1, RS>;
   return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, false, WQ, 1, RS>
                   : bn == 64 ? qmk_gemm::gemm_f16_tn_kernel<64, false, WQ, 1, RS> : qmk_gemm::gemm_f16_tn_kernel<128, false, WQ, 1, RS>;
-}
-template <bool RS>
-static GemmKernel gemm_kernel_f16(int bn, bool fuse) {
-  return gemm_kernel_wq<0, RS>(bn, fuse);
 }
 // Split activations: at most 128 B rows per stage, packed 64.
 static GemmKernel gemm_kernel_split(int bn, bool fuse, int wq) {
@@ -200,7 +196,7 @@ static bool box_n_ok(int box_n, bool fuse, int wq) {
 // (split activations exist for fp16 and FP8 weights; `scaled`: fp16 matrices with row scales)
 static GemmKernel gemm_kernel(int bn, bool fuse, int wq, int ah, bool scaled) {
   if (ah == 2) return gemm_kernel_split(bn, fuse, wq);
-  if (wq == 0) return scaled ? gemm_kernel_f16<true>(bn, fuse) : gemm_kernel_f16<false>(bn, fuse);
+  if (wq == 0) return scaled ? gemm_kernel_wq<0, true>(bn, fuse) : gemm_kernel_wq<0, false>(bn, fuse);
   return wq == 1 ? gemm_kernel_wq<1>(bn, fuse) : gemm_kernel_wq<2>(bn, fuse);
 }
 static size_t gemm_smem(int bn, bool fuse, int wq, int ah) { return qmk_gemm::smem_bytes_for(fuse ? 2 * bn : bn, wq, ah); }
@@ -375,8 +371,8 @@ int launch_gemm_swiglu(const CUtensorMap &map_a, const CUtensorMap &map_gate, co
   return QMK_OK;
 }
 
-// Split-K form for skinny problems (one 128-row tile, long K): `splits` CTAs per output tile, partial matrices
-// C + z * M * N.  K / 64 must be a multiple of `splits`.  `map_b` made with `box_n` (64 or 32) rows per box.
+// Split-K form for problems with few output tiles and a long K (decode steps, O and down of a prefill): `splits` CTAs per
+// tile, partial matrices C + z * M * N.  K / 64 must be a multiple of `splits`.  `map_b` made with `box_n` rows per box.
 int launch_gemm_splitk(const CUtensorMap &map_a, const CUtensorMap &map_b, float *C, int M, int N, int K, int splits,
                        unsigned int *status, int timeout_ms, cudaStream_t stream, std::string *err, int box_n,
                        int live_rows, int a_box_rows, int wq, const void *raw) {
@@ -407,7 +403,7 @@ int launch_gemm_splitk(const CUtensorMap &map_a, const CUtensorMap &map_b, float
 }
 
 // The pair kernel: up to three matrices B_g (maps with 128 rows per box) against A, mode 0 fp32 (K split in `splits` parts, the
-// partial matrices pair_rows(M) rows apart), 1 fp16, 2 SwiGLU of maps_b[0] (gate) and maps_b[1] (up) with N = Ns[0] outputs.
+// partial matrices M rounded up to 256 rows apart), 1 fp16, 2 SwiGLU of maps_b[0] (gate) and maps_b[1] (up) with N = Ns[0] outputs.
 // maps_c: make_map_c.  M a multiple of 128; the last tile may reach 128 rows past it, as far as the C maps go.
 int launch_gemm_pair(int mode, const CUtensorMap &map_a, int ngroups, const CUtensorMap *const *maps_b, const CUtensorMap *const *maps_c,
                      const int *Ns, int M, int K, int splits, unsigned int *status, int timeout_ms, cudaStream_t stream, std::string *err) {
@@ -543,7 +539,8 @@ int ensure_workspace(Workspace &w, int rows, bool *no_room = nullptr) {
       {reinterpret_cast<void **>(&w.act), sizeof(__half) * C * 2 * I},
       {reinterpret_cast<void **>(&w.status), 16}};
   cudaError_t e = cudaSuccess;
-  // GEMM operand rows beyond a short chunk are read (and ignored): they must hold finite numbers
+  // GEMM operand rows beyond a short chunk are read: zeros at first, later what earlier passes left there (any bits: a pass with
+  // split activations uses the same memory in another layout).  They reach their own rows of a product only, which nobody uses.
   for (const Buffer &b : buffers)
     if (e == cudaSuccess && (e = cudaMalloc(b.at, b.bytes)) == cudaSuccess) e = cudaMemset(*b.at, 0, b.bytes);
   if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);   // (a caller's stream may not wait for the legacy one)
@@ -796,7 +793,10 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     const int M = (T + qmk_gemm::BM - 1) / qmk_gemm::BM * qmk_gemm::BM;
     const int pos0 = start_position + c0;
     // Packed weights, long chunks: a GEMM expands its weight tile once per 128 rows; from EXPAND_MIN_ROWS rows on it is
-    // cheaper to expand the layer's matrices once (4000 tokens, FP8 11.3 -> 8.6 ms, NVFP4 10.8 -> 8.5; 1000: 3.9 -> 3.2; 380: 2.40 -> 2.31; 250: 2.06 -> 2.12) and run the fp16 form, with its wider tiles.
+    // cheaper to expand the layer's matrices once and run the fp16 form, on pairs of CTAs above 512 rows.  FP8 / NVFP4, in the
+    // GEMMs -> expanded: 250 tokens 1.42 / 1.44 -> 1.60 / 1.57 ms, 500: 2.02 / 1.98 -> 2.00 / 1.97, 1000: 3.35 / 3.19 -> 2.49 / 2.47,
+    // 4000: 10.6 / 10.1 -> 7.1 / 7.1.  The line was drawn when 380 tokens gained (2.40 -> 2.31); with overlapped launches they
+    // lose 1.75 / 1.76 -> 1.84 / 1.81, and 512 rows would be the better line.
     wq = wfmt;
     if (wfmt != 0 && !split && M >= EXPAND_MIN_ROWS) {
       rc = ensure_expanded(w);
