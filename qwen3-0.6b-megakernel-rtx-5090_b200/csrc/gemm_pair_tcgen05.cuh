@@ -18,8 +18,10 @@
 //
 // MODE 0: C fp32; 1: C fp16; 2: fp16 silu(gate) * up, where the pair's first CTA brings 128 gate rows and the second the 128 up
 // rows of the same columns.  RS: every B row has an fp32 scale (expanded packed matrices).
-// Every wait is bounded (status 4).  A time-out of any role of either CTA sends both through `drain`, behind the barriers where all
-// roles have met: the MMAs issued so far and every copy in flight end before a CTA leaves or frees its TMEM.
+// Every wait is bounded (status 4).  After a time-out of whatever role the issuing thread gives up too, or is through: it then waits
+// for the MMAs issued and the copies of both CTAs in flight, which complete on its barriers (`drain`), or its readers wait for the
+// accumulator it has completed, before both CTAs meet at the cluster barrier, free TMEM and leave.  All of it in the roles' cold
+// exits: a look at a flag behind the barriers, with a second meeting for the drain, made prompts of 513 to 760 tokens 1.2 % longer.
 #ifndef QMK_GEMM_PAIR_TCGEN05_CUH_
 #define QMK_GEMM_PAIR_TCGEN05_CUH_
 
@@ -45,10 +47,9 @@ struct Args {
   const float *row_scale[3];     // RS: scales of the groups' B rows (MODE 2: [0] gate, [1] up)
   int m_tiles, n_tiles, splits;  // tiles of 256 rows / 256 columns (MODE 2: 128 outputs) over all groups, parts of K
   int kblocks;                   // K blocks of 64 of a part; the partial matrices (MODE 0) are m_tiles * 256 rows apart
-  int selftest;                  // 0; of the bounded waits: NO_LOADS, SECOND_CTA_NO_LOADS, ISSUER_STOPS (behind a pair's first tile)
 };
 
-enum SelfTest { NO_LOADS = 1, ISSUER_STOPS = 2, SECOND_CTA_NO_LOADS = 3 };
+enum SelfTest { NO_LOADS = 1, ISSUER_STOPS = 2, SECOND_CTA_NO_LOADS = 3 };   // of the bounded waits (the issuer: behind a pair's first tile)
 
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
@@ -90,40 +91,20 @@ __device__ __forceinline__ void commit_pair(uint32_t bar) {   // arrives on this
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(bar), "h"(static_cast<unsigned short>(3)) : "memory");
 }
-// After a time-out (both CTAs, all threads, behind a cluster barrier; `issued`: K blocks whose copies this CTA has asked for).  The
-// full barrier of a slot completes when BOTH CTAs' copies have landed, and the one that gave up first may have asked for fewer: it
-// counts what it will not ask for as arrived, then the first CTA waits for the last use of every slot.  The issuing thread commits
-// once more and both CTAs wait for that, so no MMA reads or writes either of them any longer.  Both waits have a limit.
-__device__ __noinline__ void drain(uint32_t full0, uint32_t stopped, uint32_t issued, uint32_t rank, unsigned long long budget_ns) {
-  using namespace qmk_gemm;
-  const unsigned long long limit = budget_ns > 2000000ull ? budget_ns : 2000000ull;   // (both take microseconds)
-  auto ended = [&](uint32_t bar, uint32_t parity) {
-    const unsigned long long t0 = gtime();
-    while (!bar_try(bar, parity))
-      if (gtime() - t0 > limit) break;
-  };
-  const int warp = threadIdx.x >> 5;
-  cluster_sync();                          // both counts are written
-  if (warp == 0 && elect_one()) {
-    uint32_t peer, mine_u, other_u;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(issued), "r"(rank ^ 1u));
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(mine_u) : "r"(issued) : "memory");
-    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(other_u) : "r"(peer) : "memory");
-    const int mine = static_cast<int>(mine_u), other = static_cast<int>(other_u), last = mine > other ? mine : other;
-    for (int i = mine; i < last; ++i) {    // (at most one lap of the ring: a slot is asked for again when both uses of it were multiplied)
-      const uint32_t bar = full0 + 8u * static_cast<uint32_t>(i % STAGES);
-      if (rank == 0) bar_expect_tx(bar, 2 * STAGE_BYTES);
-      asm volatile("mbarrier.complete_tx.relaxed.cluster.shared::cluster.b64 [%0], %1;" ::"r"(in_first_cta(bar)), "r"(STAGE_BYTES) : "memory");
-    }
-    if (rank == 0)
-      for (int i = last > STAGES ? last - STAGES : 0; i < last; ++i) ended(full0 + 8u * static_cast<uint32_t>(i % STAGES), static_cast<uint32_t>(i / STAGES) & 1u);
-  }
-  if (warp == 1 && elect_one()) {
-    if (rank == 0) commit_pair(stopped);
-    ended(stopped, 0);
-  }
-  __syncwarp();
-  cluster_sync();
+// Behind a time-out: waits for a phase that copies or MMAs under way complete (microseconds; 2 ms at most, or the budget).
+__device__ __forceinline__ void bar_drain(uint32_t bar, uint32_t parity, unsigned long long budget_ns) {
+  const unsigned long long t0 = qmk_gemm::gtime(), limit = budget_ns > 2000000ull ? budget_ns : 2000000ull;
+  while (!qmk_gemm::bar_try(bar, parity))
+    if (qmk_gemm::gtime() - t0 > limit) break;
+}
+// The issuing thread's way out after a time-out: the MMAs issued so far end, and so do the copies of the ring of K blocks
+// [next, next + STAGES) below `end` that either loader may have asked for.  (Where one CTA has asked for its half of a block and
+// the other has not, the barrier does not complete and the wait takes its whole limit.)
+__device__ __noinline__ void drain(uint32_t full0, uint32_t stopped, int next, int end, unsigned long long budget_ns) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(stopped) : "memory");
+  bar_drain(stopped, 0, budget_ns);
+  for (int i = next; i < end && i < next + STAGES; ++i)
+    bar_drain(full0 + 8u * static_cast<uint32_t>(i % STAGES), static_cast<uint32_t>(i / STAGES) & 1u, budget_ns);
 }
 // One row of 128 bytes of a warp's 32 x 128-byte block, in the 128-byte swizzle its store expects (conflict-free).
 __device__ __forceinline__ void stage_row(uint32_t block, int lane, const uint32_t (&v)[32]) {
@@ -152,7 +133,7 @@ __device__ __forceinline__ uint32_t half2_bits(float a, float b) {
   return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-template <int MODE, bool RS>
+template <int MODE, bool RS, int TEST = 0>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b0,
                  const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ CUtensorMap map_c0,
@@ -168,9 +149,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   auto acc_full = [&](int b) { return bars + 8u * (2 * STAGES + b); };
   auto acc_empty = [&](int b) { return bars + 8u * (2 * STAGES + 2 + b); };   // (in the first CTA)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(pair_smem_raw + (base - raw) + OFF_BARS + 8 * (2 * STAGES + 4));
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1), *issued_slot = abort_flag + 1;
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const uint32_t stopped = bars + 8u * (2 * STAGES + 6);                     // after a time-out: the MMAs issued have ended
-  static_assert(8 * (2 * STAGES + 7) <= 256, "barriers, TMEM address, flag and count fit behind the ring");
+  static_assert(8 * (2 * STAGES + 7) <= 256, "barriers, TMEM address and flag fit behind the ring");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
@@ -185,7 +166,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     for (int b = 0; b < 2; ++b) { bar_init(acc_full(b), 1); bar_init(acc_empty(b), 16); }   // eight warps of either CTA
     bar_init(stopped, 1);
     *abort_flag = 0;
-    *issued_slot = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -215,8 +195,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     if (elect_one()) {                     // ---- producer: this CTA's rows of A and its half of B
       int s = 0;
       uint32_t parity = 1;                 // (the first pass over the ring finds it empty)
-      int issued = 0;
-      bool ok = !(args.selftest == NO_LOADS || (args.selftest == SECOND_CTA_NO_LOADS && rank == 1)), waited = false;
+      bool ok = !(TEST == NO_LOADS || (TEST == SECOND_CTA_NO_LOADS && rank == 1)), waited = false;
       for (int tile = pair; tile < tiles && ok; tile += pairs) {
         int grp, mt, nt, z;
         locate(tile, grp, mt, nt, z);
@@ -244,27 +223,26 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             tma_load_pair(dst + TILE_BYTES, map_b, kcol, brow, fbar);
           }
           tma_load_pair(dst, &map_a, kcol, arow, fbar);
-          ++issued;
           if (++s == STAGES) { s = 0; parity ^= 1u; }
         }
       }
-      *issued_slot = issued;
     }
   } else if (warp == 1) {
     if (rank == 0 && elect_one()) {        // ---- MMA issuer of the pair
       int s = 0, n = 0;
       uint32_t parity = 0;
       bool ok = true;
+      auto give_up = [&](int next) { drain(full(0), stopped, next, (tiles - pair + pairs - 1) / pairs * kblocks, budget_ns); };
       for (int tile = pair; tile < tiles && ok; tile += pairs, ++n) {
         const int buf = n & 1;
         ok = n < 2 || bar_wait(acc_empty(buf), ((n >> 1) - 1) & 1, abort_flag, status, budget_ns);
-        if (args.selftest == ISSUER_STOPS && n == 1) ok = bar_wait(stopped, 0, abort_flag, status, budget_ns);   // (nothing arrives)
-        if (!ok) break;
+        if (TEST == ISSUER_STOPS && n == 1) ok = bar_wait(stopped, 0, abort_flag, status, budget_ns);   // (nothing arrives)
+        if (!ok) { give_up(n * kblocks); break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d = tmem_base + static_cast<uint32_t>(buf) * TN;
         for (int kb = 0; kb < kblocks; ++kb) {
           ok = bar_wait(full(s), parity, abort_flag, status, budget_ns);
-          if (!ok) break;
+          if (!ok) { give_up(n * kblocks + kb); break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint64_t da = smem_desc_sw128(base + s * STAGE_BYTES), db = smem_desc_sw128(base + s * STAGE_BYTES + TILE_BYTES);
 #pragma unroll
@@ -284,7 +262,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       int grp, mt, nt, z;
       locate(tile, grp, mt, nt, z);
       const bool ok = __all_sync(0xffffffffu, bar_wait(acc_full(buf), (n >> 1) & 1, abort_flag, status, budget_ns));
-      if (!ok) break;
+      if (!ok) {
+        bar_drain(acc_full(buf), (n >> 1) & 1, budget_ns);
+        if (tile + pairs < tiles) bar_drain(acc_full(buf ^ 1), ((n + 1) >> 1) & 1, budget_ns);
+        break;
+      }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem_base + static_cast<uint32_t>(buf) * TN + (static_cast<uint32_t>(quarter * 32) << 16);
       const int row = z * args.m_tiles * TM + mt * TM + static_cast<int>(rank) * 128 + quarter * 32;   // first of the warp's 32
@@ -360,15 +342,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (threadIdx.x == 0 && *abort_flag) {   // the other CTA is told
-    uint32_t peer;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(s32(const_cast<int *>(abort_flag))), "r"(rank ^ 1u));
-    asm volatile("st.shared::cluster.u32 [%0], %1;\n\tfence.acq_rel.cluster;" ::"r"(peer), "r"(1u) : "memory");
-  }
-  __syncwarp();
   cluster_leave();                         // neither CTA leaves while the other's copies, MMAs or arrivals reach into it (the
                                            // arrivals are waited for: a buffer's last read is not announced)
-  if (*abort_flag) drain(full(0), stopped, s32(const_cast<int *>(issued_slot)), rank, budget_ns);
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");

@@ -425,7 +425,6 @@ int launch_gemm_pair(int mode, const CUtensorMap &map_a, int ngroups, const CUte
   a.m_tiles = (M + qmk_pair::TM - 1) / qmk_pair::TM;
   a.splits = splits;
   a.kblocks = K / qmk_pair::BK / splits;
-  a.selftest = 0;
   const int tiles = a.m_tiles * a.n_tiles * splits, pairs = std::min(tiles, sm_count() / 2);
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
   const cudaError_t e = launch_kernel(pair_kernel(mode, a.row_scale[0] != nullptr), dim3(2 * pairs), dim3(qmk_pair::THREADS), qmk_pair::SMEM_BYTES, stream,
@@ -1359,11 +1358,14 @@ extern "C" int qmk_selftest_gemm_pair_wait_timeout(int budget_us, int what) {
     for (int g = 0; g < 3; ++g) { a.N[g] = g == 0 ? N : 0; a.row_scale[g] = nullptr; }
     a.m_tiles = 2; a.n_tiles = 1; a.splits = 1;
     a.kblocks = K / qmk_pair::BK;
-    a.selftest = what;
-    qmk_pair::gemm_pair_kernel<0, false><<<dim3(2), qmk_pair::THREADS, qmk_pair::SMEM_BYTES>>>(
+    auto *const kernel = what == qmk_pair::NO_LOADS       ? qmk_pair::gemm_pair_kernel<0, false, qmk_pair::NO_LOADS>
+                         : what == qmk_pair::ISSUER_STOPS ? qmk_pair::gemm_pair_kernel<0, false, qmk_pair::ISSUER_STOPS>
+                                                          : qmk_pair::gemm_pair_kernel<0, false, qmk_pair::SECOND_CTA_NO_LOADS>;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(qmk_pair::SMEM_BYTES));
+    kernel<<<dim3(2), qmk_pair::THREADS, qmk_pair::SMEM_BYTES>>>(
         ma, mb, mb, mb, mc, mc, mc, a, reinterpret_cast<unsigned int *>(buf + at_status), static_cast<unsigned long long>(budget_us) * 1000ull);
     unsigned int host[4] = {0, 0, 0, 0};
-    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpy(host, buf + at_status, 16, cudaMemcpyDeviceToHost);
     rc = static_cast<int>(host[0]);
   }

@@ -143,7 +143,7 @@ def test_bounded_wait_reports_timeout_and_frees_tmem(C):
 @pytest.mark.parametrize("what", [1, 2, 3])
 def test_bounded_waits_of_a_pair_drain_both_ctas(C, what):
     """Pairs of CTAs: no loads, an issuer that stops behind a tile (MMAs and a ring of copies in flight), a second CTA without loads
-    (the first one's copies wait on barriers that its partner completes).  Status 4, and pairs after it are exact: they find
+    (the first one's copies land on barriers that never complete).  Status 4, and pairs after it are exact: they find
     all 512 TMEM columns and shared memory that no late copy writes."""
     g = torch.Generator("cpu").manual_seed(what)
     a = torch.randint(-3, 4, (1152, 512), generator=g).to(torch.float16).cuda()
