@@ -409,6 +409,8 @@ int qmk_selftest_wait_timeout(int budget_us);
 /* The same for the tcgen05 GEMM: one tile whose loads are never issued; the MMA thread's wait runs out after
  * budget_us, all roles leave, TMEM is freed; returns QMK_ERR_WAIT_TIMEOUT when that happened as designed. */
 int qmk_selftest_gemm_wait_timeout(int budget_us);
+/* The same for the tcgen05 attention of a prefill: score products that stop behind the first, keys and values in flight. */
+int qmk_selftest_attention_wait_timeout(int budget_us);
 
 /* The same for the pairs of CTAs that multiply more than 512 rows.  what = 1: no loads; 2: the issuing thread gives up behind its
  * first tile, with a ring of copies in flight; 3: the second CTA of the pair loads nothing. */

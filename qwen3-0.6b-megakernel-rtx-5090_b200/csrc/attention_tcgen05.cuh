@@ -24,7 +24,8 @@
 // as both chains have read it into registers, so the scores run a pair ahead and the softmax warps only wait (for
 // "O has taken the chain's previous tile", one commit) before they overwrite P or rescale O.  The query tile arrives
 // by TMA as fp16 (the kernel before this one stores the rotated queries that way, pre-scaled).  One CTA per SM
-// (193 KB of shared memory, all 512 TMEM columns).  Every wait is bounded (status 4).
+// (193 KB of shared memory, all 512 TMEM columns).  Every wait is bounded (status 4); on their way out the loaders, the issuers
+// and the softmax warps wait for the copies and products that are under way.
 #ifndef QMK_ATTENTION_TCGEN05_CUH_
 #define QMK_ATTENTION_TCGEN05_CUH_
 
@@ -101,6 +102,15 @@ __device__ __forceinline__ float fast_exp2(float x) {
         "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])                                                    \
       : "memory")
 
+// An issuing thread's way out after a time-out: the products it has issued end, and so do the copies of the tiles [next, next + STAGES)
+// below `end`, which its loader may have asked for before it left.
+__device__ __noinline__ void issuer_drain(uint32_t stopped, uint32_t full0, int next, int end, unsigned long long budget_ns) {
+  qmk_gemm::mma_commit(stopped);
+  qmk_gemm::bar_drain(stopped, 0, budget_ns);
+  for (int j = next; j < end && j < next + STAGES; ++j)
+    qmk_gemm::bar_drain(full0 + 8u * static_cast<uint32_t>(j % STAGES), static_cast<uint32_t>(j / STAGES) & 1u, budget_ns);
+}
+
 // map_q: 2-D map of the fp16 queries [rows][16 heads x 128] (normalised, rotated, times scale * log2 e), boxes of
 // {64, 128}, 128-byte swizzle; query t sits at position pos0 + t and sees
 // cache rows 0 .. pos0 + t).  map_k / map_v: 3-D maps {128 dims, pos0 + T rows, layers x 8 kv heads} of the fp16
@@ -110,7 +120,8 @@ __device__ __forceinline__ float fast_exp2(float x) {
 // Packed prompts (items != null): the rows hold several sequences, each padded to whole query tiles.  CTA i takes
 // items[i] = {sequence, first row of the query tile, its position within the sequence, head | length << 8} (sorted
 // from the heaviest down by the host) and reads that sequence's caches through maps_dev[2 seq], maps_dev[2 seq + 1]
-// in device memory; T and pos0 are then not used.
+// in device memory; T and pos0 are then not used.  TEST: the self test's score issuer that stops behind its first product.
+template <bool TEST = false>
 __global__ void __launch_bounds__(THREADS, 1)
 causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                     int layer_head0, __half *out, int T, int pos0, float scale, unsigned int *status,
@@ -149,6 +160,7 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(attn_smem + OFF_BARS + 8 * 25);
   static_assert(STAGES == 4 && CHAINS == 2, "barrier layout above");
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  const uint32_t s_stopped = bars + 8u * 26, pv_stopped = bars + 8u * 27;   // after a time-out: the products issued have ended
 
   if ((base & 1023u) != 0u) {   // the swizzled tiles need a 1024-byte aligned window: report instead of computing garbage
     if (threadIdx.x == 0) atomicCAS(status, 0u, 5u);
@@ -172,6 +184,8 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       bar_init(pv_done(c), 1);
     }
     bar_init(q_full, 1);
+    bar_init(s_stopped, 1);
+    bar_init(pv_stopped, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -248,7 +262,12 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
              bar_wait(k_full(s0), (j0 / STAGES) & 1, abort_flag, status, budget_ns) &&
              (!two || bar_wait(k_full(s0 + 1), (j0 / STAGES) & 1, abort_flag, status, budget_ns)) &&
              (p < 2 || bar_wait(s_free(p & 1), ((p >> 1) - 1) & 1, abort_flag, status, budget_ns));   // both chains have read pair p - 2
-        if (!ok) break;
+        if (TEST && p == 1) ok = bar_wait(s_stopped, 0, abort_flag, status, budget_ns);   // (nothing arrives)
+        if (!ok) {
+          bar_drain(q_full, 0, budget_ns);
+          issuer_drain(s_stopped, k_full(0), j0, ntiles, budget_ns);
+          break;
+        }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t ts = tmem_base + 128u * static_cast<uint32_t>(p & 1);
 #pragma unroll
@@ -270,7 +289,10 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const int c = j & 1, n = j >> 1;   // chain, and the tile's index within it
         ok = bar_wait(p_ready(c), n & 1, abort_flag, status, budget_ns) &&
              bar_wait(v_full(j % STAGES), (j / STAGES) & 1, abort_flag, status, budget_ns);
-        if (!ok) break;
+        if (!ok) {
+          issuer_drain(pv_stopped, v_full(0), j, ntiles, budget_ns);
+          break;
+        }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // O_c += P_c . V_j: four steps of 16 keys; V rows are [key][dim], i.e. MN-major for the B operand
         const uint32_t vt = base + OFF_V + (j % STAGES) * 2 * K_HALF_BYTES;
@@ -370,6 +392,7 @@ causal_attention_tc(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     }
     const int my_tiles = (ntiles - chain + 1) / CHAINS;
     if (ok && my_tiles > 0) ok = __all_sync(0xffffffffu, bar_wait(pv_done(chain), (my_tiles - 1) & 1, abort_flag, status, budget_ns));
+    if (!ok) bar_drain(pv_done(chain), (my_tiles - 1) & 1, budget_ns);   // (issuers that are through leave the last products to their readers)
     // ---- merge of the two chains.  (m, l) of this chain's row go through its own P tile, which its last product has
     // finished reading; every softmax warp reaches the barrier whatever its waits returned.
     asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(p_tile + static_cast<uint32_t>(row) * 8u), "f"(m_used), "f"(l) : "memory");

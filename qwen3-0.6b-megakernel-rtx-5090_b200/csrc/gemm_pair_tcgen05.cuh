@@ -91,20 +91,14 @@ __device__ __forceinline__ void commit_pair(uint32_t bar) {   // arrives on this
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(bar), "h"(static_cast<unsigned short>(3)) : "memory");
 }
-// Behind a time-out: waits for a phase that copies or MMAs under way complete (microseconds; 2 ms at most, or the budget).
-__device__ __forceinline__ void bar_drain(uint32_t bar, uint32_t parity, unsigned long long budget_ns) {
-  const unsigned long long t0 = qmk_gemm::gtime(), limit = budget_ns > 2000000ull ? budget_ns : 2000000ull;
-  while (!qmk_gemm::bar_try(bar, parity))
-    if (qmk_gemm::gtime() - t0 > limit) break;
-}
 // The issuing thread's way out after a time-out: the MMAs issued so far end, and so do the copies of the ring of K blocks
 // [next, next + STAGES) below `end` that either loader may have asked for.  (Where one CTA has asked for its half of a block and
 // the other has not, the barrier does not complete and the wait takes its whole limit.)
 __device__ __noinline__ void drain(uint32_t full0, uint32_t stopped, int next, int end, unsigned long long budget_ns) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(stopped) : "memory");
-  bar_drain(stopped, 0, budget_ns);
+  qmk_gemm::bar_drain(stopped, 0, budget_ns);
   for (int i = next; i < end && i < next + STAGES; ++i)
-    bar_drain(full0 + 8u * static_cast<uint32_t>(i % STAGES), static_cast<uint32_t>(i / STAGES) & 1u, budget_ns);
+    qmk_gemm::bar_drain(full0 + 8u * static_cast<uint32_t>(i % STAGES), static_cast<uint32_t>(i / STAGES) & 1u, budget_ns);
 }
 // One row of 128 bytes of a warp's 32 x 128-byte block, in the 128-byte swizzle its store expects (conflict-free).
 __device__ __forceinline__ void stage_row(uint32_t block, int lane, const uint32_t (&v)[32]) {

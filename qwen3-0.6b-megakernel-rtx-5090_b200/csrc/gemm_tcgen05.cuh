@@ -200,6 +200,13 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// Behind a time-out: waits for a phase that copies or MMAs under way complete (microseconds; 2 ms at most, or the budget).
+__device__ __noinline__ void bar_drain(uint32_t bar, uint32_t parity, unsigned long long budget_ns) {
+  const unsigned long long t0 = gtime(), limit = budget_ns > 2000000ull ? budget_ns : 2000000ull;
+  while (!bar_try(bar, parity))
+    if (gtime() - t0 > limit) break;
+}
+
 // Up to three B matrices (same K) against one A in one launch: blockIdx.x counts the N tiles of group 0, then of
 // group 1, then of group 2; C_g is [M x N_g].
 struct Groups {

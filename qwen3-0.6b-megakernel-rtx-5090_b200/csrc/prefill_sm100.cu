@@ -235,7 +235,7 @@ int ensure_gemm_attrs(std::string *err) {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(qmk_pf::causal_attention_split, cudaFuncAttributeMaxDynamicSharedMemorySize, qmk_pf::ATM_SMEM_BYTES);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc<>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(qmk_attn::SMEM_BYTES));
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(qmk_pf::decode_attention_ring, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -923,7 +923,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
                                     env.attn_tc ? attn_scale * 1.4426950408889634f : 0.f));
       if (l == num_layers - 1) break;   // the cache is complete; nothing downstream of the last layer is kept
       if (env.attn_tc)
-        PF_CUDA(qmk_tc::launch_kernel(qmk_attn::causal_attention_tc, dim3(pk ? pk_items : (T + qmk_attn::TQ - 1) / qmk_attn::TQ * NQ),
+        PF_CUDA(qmk_tc::launch_kernel(qmk_attn::causal_attention_tc<>, dim3(pk ? pk_items : (T + qmk_attn::TQ - 1) / qmk_attn::TQ * NQ),
                                       dim3(qmk_attn::THREADS), qmk_attn::SMEM_BYTES, stream, w.map_qh, map_kc, map_vc, l * NKV, w.attn, T,
                                       pos0, attn_scale, w.status, static_cast<unsigned long long>(env.timeout_ms) * 1000000ull,
                                       pk ? reinterpret_cast<const int4 *>(w.packed + PK_ITEMS_OFF) : nullptr,
@@ -1331,6 +1331,40 @@ extern "C" int qmk_selftest_gemm_wait_timeout(int budget_us) {
   cudaFree(ab);
   cudaFree(c);
   cudaFree(status);
+  if (rc != QMK_OK && rc != QMK_ERR_WAIT_TIMEOUT) return qmk_internal::report(rc, err);
+  return rc;
+}
+
+// The same of the attention kernel: a query tile at position 512 whose score products stop behind the first, with keys and values
+// in flight.
+extern "C" int qmk_selftest_attention_wait_timeout(int budget_us) {
+  using qmk_pf::QS;
+  using qmk_pf::NKV;
+  std::string err;
+  if (budget_us < 1 || budget_us > 1000000) return qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "budget_us must be in [1, 1e6]");
+  int rc = QMK_OK;
+  constexpr int T = qmk_attn::TQ, POS = 512, ROWS = POS + T;
+  constexpr size_t q_bytes = sizeof(__half) * T * QS, kv_bytes = sizeof(__half) * NKV * ROWS * 128;
+  unsigned char *buf = nullptr;            // queries, keys, values, outputs, status
+  PF_CUDA(cudaMalloc(&buf, 2 * q_bytes + 2 * kv_bytes + 16));
+  cudaError_t e = cudaMemset(buf, 0, 2 * q_bytes + 2 * kv_bytes + 16);
+  unsigned char *const k = buf + q_bytes, *const v = k + kv_bytes, *const out = v + kv_bytes, *const status = out + q_bytes;
+  CUtensorMap mq, mk, mv;
+  rc = qmk_tc::make_map_f16(&mq, buf, T, QS, qmk_gemm::BM, &err);
+  if (rc == QMK_OK) rc = qmk_tc::make_map_kv(&mk, k, ROWS, ROWS, NKV, &err);
+  if (rc == QMK_OK) rc = qmk_tc::make_map_kv(&mv, v, ROWS, ROWS, NKV, &err);
+  if (rc == QMK_OK && e == cudaSuccess) {
+    e = cudaFuncSetAttribute(qmk_attn::causal_attention_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(qmk_attn::SMEM_BYTES));
+    qmk_attn::causal_attention_tc<true><<<dim3(qmk_pf::NQ), qmk_attn::THREADS, qmk_attn::SMEM_BYTES>>>(
+        mq, mk, mv, 0, reinterpret_cast<__half *>(out), T, POS, 1.0f, reinterpret_cast<unsigned int *>(status),
+        static_cast<unsigned long long>(budget_us) * 1000ull, nullptr, nullptr);
+    unsigned int host[4] = {0, 0, 0, 0};
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpy(host, status, 16, cudaMemcpyDeviceToHost);
+    rc = static_cast<int>(host[0]);
+  }
+  if (e != cudaSuccess) { rc = QMK_ERR_CUDA; err = std::string("attention self test: ") + cudaGetErrorString(e); }
+  cudaFree(buf);
   if (rc != QMK_OK && rc != QMK_ERR_WAIT_TIMEOUT) return qmk_internal::report(rc, err);
   return rc;
 }

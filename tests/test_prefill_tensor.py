@@ -305,3 +305,18 @@ def test_rows_do_not_depend_on_how_a_prompt_is_cut(C, fmt, cuts):
     for x, y in ((one._k_cache, parts._k_cache), (one._v_cache, parts._v_cache)):
         assert float(x[:, :, :cuts[-1]].float().abs().max()) > 0.1
         assert torch.equal(x[:, :, :cuts[-1]], y[:, :, :cuts[-1]])
+
+
+def test_attention_waits_run_out_and_leave_the_device_usable(C):
+    """Score products that stop behind the first, with keys and values in flight: status 4 after the budget, copies landed and TMEM
+    freed (the prefill behind it allocates all of it on every SM), rows as before."""
+    w = S.make_weights(seed=71, num_layers=2, vocab_size=2048, norm_std=0.1, max_seq_len=16)
+    ids = S.make_prompt(1300, seed=1, vocab_size=2048)
+    eng = _engine(w, 1536, "tensor")
+    eng.prefill_ids(ids)
+    before = eng._k_cache.clone(), eng._v_cache.clone()
+    for _ in range(3):
+        assert C.selftest_attention_wait_timeout(300) == 4
+        eng.reset()
+        eng.prefill_ids(ids)
+        assert torch.equal(eng._k_cache, before[0]) and torch.equal(eng._v_cache, before[1])
