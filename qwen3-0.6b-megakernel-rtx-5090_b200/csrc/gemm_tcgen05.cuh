@@ -51,19 +51,32 @@ namespace qmk_gemm {
 constexpr int BM = 128, BK = 64;                 // BK * 2 bytes = one 128-byte swizzle row; the N tile (128 or 64) is a template parameter
 // Ring depth per N-tile variant: as many stages as fit in ~192 KB (a skinny M = 128 problem is bound by the
 // latency of its K loop, so the whole K extent of a 1024-wide matrix is in flight at once).
-constexpr int stages_for(int bn, int wq = 0, int ah = 1) {
+// `am` = rows of A that a stage holds (below): with 64 the stages are smaller and a ring holds all 16 K blocks of a 1024-wide
+// matrix against 32 columns.
+constexpr int stages_for(int bn, int wq = 0, int ah = 1, int am = 128) {
+  if (am == 64) return wq == 0 ? (bn == 32 ? 16 : bn == 64 ? 12 : 8) : wq == 1 ? (bn == 32 ? 14 : bn == 64 ? 10 : 6) : (bn == 32 ? 15 : bn == 64 ? 11 : 6);
   if (ah == 2) return wq || bn == 128 ? 4 : 5;
   return wq ? (bn == 32 ? 8 : bn == 64 ? 6 : 4) : (bn == 32 ? 10 : bn == 64 ? 8 : 6);
 }
 constexpr int MAX_GROUPS = 3;   // matrices sharing one A operand that one launch can multiply (q/k/v, gate/up)
+constexpr int MAX_PREFETCH = 3;
 constexpr int THREADS = 192;                     // fp16 weights: producer warp, MMA warp, four epilogue warps
 constexpr int THREADS_PACKED = 320;              // packed weights: four more warps that only expand K blocks
-constexpr int threads_for(int wq, int ah = 1) { return wq ? THREADS_PACKED + (ah == 2 ? 128 : 0) : THREADS; }   // split activations: four warps of their own for the sums
+// Threads that issue products: two for fp16 weights against at most 64 rows and 64 columns.  A wait costs an issuing thread 125 cycles
+// whatever it finds, and in a loop with waits it issues a product every 66, so one thread takes 263 to 390 cycles for a K block that
+// the tensor core does in 99 (64 rows x 32 columns).  Each has an accumulator of its own, added in the epilogue.  Decode step of 8 /
+// 16 / 64 sequences, 64-token contexts: 767 / 776 / 894 -> 742 / 753 / 853 us.  (128 rows: nothing gained, and a prompt's rows must not
+// depend on the tile that made them; packed weights: the second thread takes issue slots from the expanding warps, 1 to 4 % lost.)
+constexpr int issuers_for(int sb, int wq, int am) { return am == 64 && wq == 0 && sb <= 64 ? 2 : 1; }
+// split activations of packed weights: four warps of their own for the sums; two issuers: a warp for the second
+constexpr int threads_for(int sb, int wq, int ah = 1, int am = 128) {
+  return (wq ? THREADS_PACKED + (ah == 2 ? 128 : 0) : THREADS) + (issuers_for(sb, wq, am) == 2 ? 32 : 0);
+}
 constexpr uint32_t TILE_A_BYTES = BM * BK * 2;   // 16 KB
 // Packed K block of one B row: 64 e4m3 bytes, or 32 bytes of e2m1 pairs
 constexpr uint32_t raw_row_bytes(int wq) { return wq == 1 ? 64u : wq == 2 ? 32u : 0u; }
-constexpr uint32_t stage_bytes_for(int bn, int wq = 0, int ah = 1) {
-  return static_cast<uint32_t>(ah) * TILE_A_BYTES + static_cast<uint32_t>(bn) * BK * 2 + static_cast<uint32_t>(bn) * raw_row_bytes(wq);
+constexpr uint32_t stage_bytes_for(int bn, int wq = 0, int ah = 1, int am = 128) {
+  return static_cast<uint32_t>(ah) * am * BK * 2 + static_cast<uint32_t>(bn) * BK * 2 + static_cast<uint32_t>(bn) * raw_row_bytes(wq);
 }
 // Per-row scales kept in shared memory for the whole tile: the fp32 row / tensor scale, and for NVFP4 the block
 // scales of the CTA's K range (one byte per 16 values; K <= 3072 -> 192 bytes, rows 196 bytes apart against bank
@@ -75,8 +88,8 @@ constexpr uint32_t scale_bytes_for(int bn, int wq) {
 }
 constexpr int MAX_STAGES = 16;
 constexpr uint32_t BARRIER_BYTES = 640;   // full[16], empty[16], acc_full, raw_full[16], a_full[16], TMEM address, abort flag, blk_full[4], blk_free[4]
-constexpr size_t smem_bytes_for(int bn, int wq = 0, int ah = 1) {
-  return 1024 /* alignment slack */ + static_cast<size_t>(stages_for(bn, wq, ah)) * stage_bytes_for(bn, wq, ah) + BARRIER_BYTES +
+constexpr size_t smem_bytes_for(int bn, int wq = 0, int ah = 1, int am = 128) {
+  return 1024 /* alignment slack */ + static_cast<size_t>(stages_for(bn, wq, ah, am)) * stage_bytes_for(bn, wq, ah, am) + BARRIER_BYTES +
          scale_bytes_for(bn, wq);
 }
 // Ring depth of a launch: the compile-time depth above (one CTA per SM, ~200 KB: a skinny problem wants its whole K
@@ -84,14 +97,15 @@ constexpr size_t smem_bytes_for(int bn, int wq = 0, int ah = 1) {
 // of one (TMEM -> registers -> global) runs under the main loop of the other, which is what a multi-wave prefill GEMM
 // wants (measured on 2048 prompt tokens: 7.9 -> 6.8 ms per pass).
 struct RingGeometry { int stages; uint32_t ring_bytes; size_t smem_bytes; };
-inline RingGeometry ring_geometry(int sb, int wq, uint32_t budget_bytes, int ah = 1) {
+inline RingGeometry ring_geometry(int sb, int wq, uint32_t budget_bytes, int ah, int am, int kblocks) {
   RingGeometry g;
-  g.stages = stages_for(sb, wq, ah);
+  g.stages = stages_for(sb, wq, ah, am);
   if (budget_bytes > 0) {
-    const int fit = static_cast<int>(budget_bytes / stage_bytes_for(sb, wq, ah));
+    const int fit = static_cast<int>(budget_bytes / stage_bytes_for(sb, wq, ah, am));
     if (fit < g.stages) g.stages = fit < 2 ? 2 : fit;
   }
-  g.ring_bytes = static_cast<uint32_t>(g.stages) * stage_bytes_for(sb, wq, ah);
+  if (kblocks < g.stages) g.stages = kblocks;
+  g.ring_bytes = static_cast<uint32_t>(g.stages) * stage_bytes_for(sb, wq, ah, am);
   g.smem_bytes = 1024 + static_cast<size_t>(g.ring_bytes) + BARRIER_BYTES + scale_bytes_for(sb, wq);
   return g;
 }
@@ -153,14 +167,17 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
       ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar)
       : "memory");
 }
+__device__ __forceinline__ void prefetch_l2(const void *src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 // Shared-memory matrix descriptor of a K-major tile stored as rows of 128 bytes with the 128-byte swizzle:
 // 8-row groups are 1024 bytes apart (stride byte offset), version 1 (sm_100), layout type 2 (SWIZZLE_128B).
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
   return static_cast<uint64_t>((addr & 0x3FFFFu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 // Instruction descriptor: fp32 accumulator, fp16 A and B, both K-major, N >> 3 at bit 17, M >> 4 at bit 24.
-constexpr uint32_t idesc_for(int bn) {
-  return (1u << 4) | (static_cast<uint32_t>(bn >> 3) << 17) | (static_cast<uint32_t>(BM >> 4) << 24);
+constexpr uint32_t idesc_for(int bn, int am = BM) {
+  return (1u << 4) | (static_cast<uint32_t>(bn >> 3) << 17) | (static_cast<uint32_t>(am >> 4) << 24);
 }
 
 __device__ __forceinline__ void mma_f16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t accumulate,
@@ -237,6 +254,12 @@ struct Groups {
   // reading the whole row of logits, which is never written.
   float *amax_val;
   int *amax_idx;
+  // Weights a later kernel of the chain will read, brought into L2 meanwhile: CTA i of the launch asks for the i-th `prefetch_piece`
+  // bytes of each matrix (up to prefetch_bytes; all multiples of 16).  The chain is bound by latency, DRAM idles for most of it, and
+  // a kernel sees its weights' addresses only a microsecond before its activations are there.  Decode step of 5 sequences 786 -> 771 us,
+  // prompts of 31 / 109 / 500 tokens 857 / 947 / 1555 -> 827 / 931 / 1525 us.
+  const unsigned char *prefetch[MAX_PREFETCH] = {nullptr, nullptr, nullptr};
+  uint32_t prefetch_bytes[MAX_PREFETCH] = {0, 0, 0}, prefetch_piece[MAX_PREFETCH] = {0, 0, 0};
   // Plain epilogue, no split-K: 1 = the C matrices are fp16 [M x N_g] (the pointers are reinterpreted), half the
   // store burst of a launch whose CTAs all reach their epilogue together.
   int out_f16;
@@ -285,8 +308,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // RS: fp16 B matrices with row scales (Groups::row_scale).  A kernel of its own: a run-time test of the pointers in the
 // epilogues of every fp16 GEMM cost a prefill pass 0.6 to 1 %.
-template <int BN, bool FUSE = false, int WQ = 0, int AH = 1, bool RS = false>
-__global__ void __launch_bounds__(threads_for(WQ, AH), 1)
+//
+// AM: rows of the MMA, 128 or, for launches of one row tile with at most 64 live rows (decode steps), 64.  With every operand in
+// place the four products of a K block take 162 cycles against 32 columns at 128 rows and 99 at 64 (the tensor core reads A from
+// shared memory, 4 KB a product against 2 KB), and a stage is 8 KB smaller, so that the ring holds more of the K loop
+// (packed weights: decode step of 64 NVFP4 sequences 1198 -> 1150 us, of 16 FP8 ones 978 -> 925).  An
+// accumulator of 64 rows lies in lanes 0 .. 15 of each warp's 32: row r in lane 32 * (r / 16) + r % 16.
+template <int BN, bool FUSE = false, int WQ = 0, int AH = 1, bool RS = false, int AM = BM>
+__global__ void __launch_bounds__(threads_for(FUSE ? 2 * BN : BN, WQ, AH, AM), 1)
 gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b0,
                    const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ CUtensorMap map_b2,
                    const Groups groups, int M, int K, unsigned int *status, unsigned long long budget_ns,
@@ -294,13 +323,18 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   static_assert(BN == 32 || BN == 64 || BN == 128, "N tiles of 32, 64 or 128 columns");
   static_assert(!FUSE || BN <= 64, "the fused SwiGLU epilogue keeps two accumulators of at most 64 columns (one MMA of N = 128)");
   static_assert(!RS || (WQ == 0 && AH == 1), "row scales belong to expanded matrices");
+  static_assert(AM == BM || (AM == 64 && AH == 1), "64 rows: single fp16 activations");
+  constexpr uint32_t HALF_A = AM * BK * 2;        // one A tile (split activations: hi, then lo)
+  constexpr int WARP_ROWS = AM / 4;               // rows of a warp's 32 TMEM lanes
   static_assert(WQ == 0 || (FUSE ? 2 * BN : BN) <= 128, "packed weights: at most 128 B rows per stage (scales live in shared memory)");
   constexpr int SB = FUSE ? 2 * BN : BN;          // B rows held per stage / accumulator columns
-  constexpr int NACC = AH == 2 ? 4 : 1;           // accumulators: one, or with split activations four that the K blocks take in turn
+  constexpr int ISSUERS = issuers_for(SB, WQ, AM);
+  constexpr int ISSUER_B = ISSUERS == 2 ? threads_for(SB, WQ, AH, AM) / 32 - 1 : 1;   // the second issuer's warp
+  constexpr int NACC = AH == 2 ? 4 : ISSUERS;     // accumulators: one per issuer, or with split activations four that the K blocks take in turn
   static_assert(NACC * SB <= 512, "TMEM columns");
   constexpr uint32_t RAW_ROW = raw_row_bytes(WQ);
   const int STAGES = groups.stages;
-  constexpr uint32_t STAGE_BYTES = stage_bytes_for(SB, WQ, AH);
+  constexpr uint32_t STAGE_BYTES = stage_bytes_for(SB, WQ, AH, AM);
   // which matrix this CTA works on
   int tile = blockIdx.x, grp = 0;
   if (!FUSE && tile >= groups.N[0] / BN) { tile -= groups.N[0] / BN; grp = 1; }
@@ -339,9 +373,9 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   auto b_landed = [&](int s) { return WQ ? raw_full(s) : full(s); };
   auto a_landed = [&](int s) { return WQ ? a_full(s) : full(s); };
   constexpr uint32_t TILE_RAW_BYTES = BN * RAW_ROW;
-  const uint32_t a_tx = AH * (groups.a_box_bytes ? groups.a_box_bytes : TILE_A_BYTES);
+  const uint32_t a_tx = AH * (groups.a_box_bytes ? groups.a_box_bytes : HALF_A);
   const uint32_t b_tx = (FUSE ? 2u : 1u) * (WQ ? TILE_RAW_BYTES : TILE_B_BYTES);
-  constexpr uint32_t TILE_A = AH * TILE_A_BYTES;   // the B tile follows the A tile(s) in a stage
+  constexpr uint32_t TILE_A = AH * HALF_A;   // the B tile follows the A tile(s) in a stage
   const int kcol = WQ ? static_cast<int>(RAW_ROW) : BK;          // B-map columns (bytes for packed rows) per K block
   const uint32_t b_dst = WQ ? TILE_A + (FUSE ? 2u : 1u) * TILE_B_BYTES : TILE_A;   // where the B copies land in a stage
   const uint32_t b_dst_step = WQ ? TILE_RAW_BYTES : TILE_B_BYTES;
@@ -357,7 +391,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       bar_init(empty(s), 1);
       if (WQ) { bar_init(raw_full(s), 1); bar_init(a_full(s), 1); }
     }
-    bar_init(acc_full, 1);
+    bar_init(acc_full, ISSUERS);
     if (AH == 2)
       for (int a = 0; a < NACC; ++a) { bar_init(blk_full(a), 1); bar_init(blk_free(a), 4); }
     *abort_flag = 0;
@@ -368,6 +402,13 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       bar_expect_tx(b_landed(kb), WQ ? b_tx : a_tx + b_tx);
       tma_load_2d(base + kb * STAGE_BYTES + b_dst, map_b, (kb0 + kb) * kcol, n0, b_landed(kb));
       if (FUSE) tma_load_2d(base + kb * STAGE_BYTES + b_dst + b_dst_step, &map_b1, (kb0 + kb) * kcol, n0, b_landed(kb));
+    }
+    const uint32_t cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+#pragma unroll
+    for (int i = 0; i < MAX_PREFETCH; ++i) {
+      const uint32_t first = cta * groups.prefetch_piece[i];
+      if (first < groups.prefetch_bytes[i])
+        prefetch_l2(groups.prefetch[i] + first, min(groups.prefetch_piece[i], groups.prefetch_bytes[i] - first));
     }
   }
   if (WQ != 0 && warp >= 2 && warp < 6) {
@@ -412,7 +453,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       for (int kb = 0; kb < prologue; ++kb) {
         if (WQ) bar_expect_tx(a_full(kb), a_tx);
         tma_load_2d(base + kb * STAGE_BYTES, &map_a, (kb0 + kb) * BK, m0, a_landed(kb));
-        if (AH == 2) tma_load_2d(base + kb * STAGE_BYTES + TILE_A_BYTES, &map_a, K + (kb0 + kb) * BK, m0, a_landed(kb));
+        if (AH == 2) tma_load_2d(base + kb * STAGE_BYTES + HALF_A, &map_a, K + (kb0 + kb) * BK, m0, a_landed(kb));
       }
       int issued = prologue, s = prologue == STAGES ? 0 : prologue;   // slot of K block kb
       uint32_t parity = 0;                                            // of the use before it, whose MMAs free the slot
@@ -424,7 +465,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         bar_expect_tx(b_landed(s), WQ ? b_tx : a_tx + b_tx);
         if (WQ) bar_expect_tx(a_full(s), a_tx);
         tma_load_2d(base + s * STAGE_BYTES, &map_a, (kb0 + kb) * BK, m0, a_landed(s));
-        if (AH == 2) tma_load_2d(base + s * STAGE_BYTES + TILE_A_BYTES, &map_a, K + (kb0 + kb) * BK, m0, a_landed(s));
+        if (AH == 2) tma_load_2d(base + s * STAGE_BYTES + HALF_A, &map_a, K + (kb0 + kb) * BK, m0, a_landed(s));
         tma_load_2d(base + s * STAGE_BYTES + b_dst, map_b, (kb0 + kb) * kcol, n0, b_landed(s));
         if (FUSE) tma_load_2d(base + s * STAGE_BYTES + b_dst + b_dst_step, &map_b1, (kb0 + kb) * kcol, n0, b_landed(s));
         issued = kb + 1;
@@ -440,7 +481,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         }
       }
     }
-  } else if (warp == 1) {
+  } else if (ISSUERS == 1 && warp == 1) {
     if (elect_one()) {                     // ---- MMA issuer
       bool ok = true;
       int s = 0;                           // slot and parity of K block kb
@@ -458,21 +499,47 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         // so one MMA of N = 2 BN covers both and leaves gate in columns [0, BN), up in [BN, 2 BN)
         if (AH == 1) {
 #pragma unroll
-          for (int j = 0; j < BK / 16; ++j) mma_f16_ss(tmem_base, da + 2u * j, db + 2u * j, (kb > 0 || j > 0) ? 1u : 0u, idesc_for(SB));
+          for (int j = 0; j < BK / 16; ++j) mma_f16_ss(tmem_base, da + 2u * j, db + 2u * j, (kb > 0 || j > 0) ? 1u : 0u, idesc_for(SB, AM));
         } else {
 #pragma unroll
-          for (int j = 0; j < BK / 16; ++j) mma_f16_ss(tmem_base + (kb % NACC) * SB, da + (TILE_A_BYTES >> 4) + 2u * j, db + 2u * j, j > 0 ? 1u : 0u, idesc_for(SB));
+          for (int j = 0; j < BK / 16; ++j) mma_f16_ss(tmem_base + (kb % NACC) * SB, da + (HALF_A >> 4) + 2u * j, db + 2u * j, j > 0 ? 1u : 0u, idesc_for(SB));
           mma_f16_ss_onto_lo(tmem_base + (kb % NACC) * SB, da, db, idesc_for(SB));
 #pragma unroll
           for (int j = 1; j < BK / 16; ++j) mma_f16_ss(tmem_base + (kb % NACC) * SB, da + 2u * j, db + 2u * j, 1u, idesc_for(SB));
           mma_commit(blk_full(kb % NACC));
         }
-        mma_commit(empty(s));               // the stage is free once these MMAs have read it
+        // the stage is free once these MMAs have read it (asked only where something is loaded into it again)
+        if (kb + STAGES < kblocks) mma_commit(empty(s));
         da += STAGE_BYTES >> 4;
         db += STAGE_BYTES >> 4;
         if (++s == STAGES) { s = 0; parity ^= 1u; da = da0; db = db0; }
       }
       if (ok && AH == 1) mma_commit(acc_full);   // accumulator complete
+    }
+  } else if (ISSUERS == 2 && (warp == 1 || warp == ISSUER_B)) {
+    if (elect_one()) {                     // ---- two MMA issuers: one takes the stages of even number, one those of odd (so that each
+                                           //      meets the uses of a stage in order)
+      const int s0 = warp == ISSUER_B ? 1 : 0;
+      bool ok = true;
+      int s = s0, lap = 0;                 // K block lap + s is in stage s
+      uint32_t parity = 0, accumulate = 0;
+      const uint64_t da0 = smem_desc_sw128(base) + s0 * (STAGE_BYTES >> 4), db0 = smem_desc_sw128(base + TILE_A) + s0 * (STAGE_BYTES >> 4);
+      uint64_t da = da0, db = db0;
+      const uint32_t acc = tmem_base + s0 * SB;
+      for (int kb = s0; kb < kblocks && s0 < STAGES; kb = lap + s) {
+        ok = bar_wait(full(s), parity, abort_flag, status, budget_ns);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < BK / 16; ++j) mma_f16_ss(acc, da + 2u * j, db + 2u * j, j > 0 ? 1u : accumulate, idesc_for(SB, AM));
+        accumulate = 1;
+        if (kb + STAGES < kblocks) mma_commit(empty(s));
+        da += 2 * (STAGE_BYTES >> 4);
+        db += 2 * (STAGE_BYTES >> 4);
+        s += 2;
+        if (s >= STAGES) { s = s0; lap += STAGES; parity ^= 1u; da = da0; db = db0; }
+      }
+      if (ok) mma_commit(acc_full);        // this issuer's accumulator complete (or not begun: `both`)
     }
   } else {                                 // ---- warps 2..5: epilogue, each owns TMEM lanes 32 * (warp % 4) ..; packed
                                            //      weights: first they and warps 6..9 expand the K blocks
@@ -601,11 +668,12 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       }
     }
     if (AH == 1 && warp < 6) {
+    const bool both = ISSUERS == 2 && kblocks > 1 && STAGES > 1;     // the second accumulator holds a part of the sums
     // warp-uniform outcome: the TMEM loads below are warp-wide instructions
     const bool ok = __all_sync(0xffffffffu, bar_wait(acc_full, 0, abort_flag, status, budget_ns));
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ok && FUSE) {
-      const int row = m0 + quarter * 32 + lane;
+      const int row = lane < WARP_ROWS ? m0 + quarter * WARP_ROWS + lane : M;   // (64 rows: the upper lanes hold none)
       __half *arow = reinterpret_cast<__half *>(C) + static_cast<size_t>(row) * N + n0;
 #pragma unroll 1
       for (int c = 0; c < BN / 16; ++c) {     // 16 columns of the gate tile and the same 16 of the up tile per pass
@@ -613,7 +681,19 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const uint32_t tg = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(c * 16);
         tmem_ld16(tg, g);
         tmem_ld16(tg + BN, u);
-        tmem_ld_wait();
+        if (both) {
+          uint32_t g2[16], u2[16];
+          tmem_ld16(tg + SB, g2);
+          tmem_ld16(tg + SB + BN, u2);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            g[i] = __float_as_uint(__uint_as_float(g[i]) + __uint_as_float(g2[i]));
+            u[i] = __float_as_uint(__uint_as_float(u[i]) + __uint_as_float(u2[i]));
+          }
+        } else {
+          tmem_ld_wait();
+        }
         if (row < M) {
           uint32_t packed[8];
 #pragma unroll
@@ -638,7 +718,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         }
       }
     } else if (ok) {
-      const int row = m0 + quarter * 32 + lane;
+      const int row = lane < WARP_ROWS ? m0 + quarter * WARP_ROWS + lane : M;
       float *crow = C + static_cast<size_t>(blockIdx.z) * groups.split_stride + static_cast<size_t>(row) * N + n0;
       __half *hrow = reinterpret_cast<__half *>(C) + static_cast<size_t>(row) * N + n0;   // (out_f16)
       const bool pick = groups.amax_val != nullptr;
@@ -651,7 +731,15 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         uint32_t r[32];
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(c * 32);
         tmem_ld32(taddr, r);
-        tmem_ld_wait();
+        if (both) {
+          uint32_t r2[32];
+          tmem_ld32(taddr + SB, r2);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(r2[i]));
+        } else {
+          tmem_ld_wait();
+        }
         if (RS) {
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {

@@ -174,6 +174,15 @@ bool pdl_active() { return t_pdl; }
 // The kernel for an N tile, epilogue and weight format, and its dynamic shared memory.
 using GemmKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const qmk_gemm::Groups,
                             int, int, unsigned int *, unsigned long long, int);
+// One row tile of at most 64 rows (short A boxes): the tiles decode steps take.
+template <int WQ>
+static GemmKernel gemm_kernel_64(int bn, bool fuse) {
+  if (fuse) return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, true, WQ, 1, false, 64> : nullptr;
+  return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, false, WQ, 1, false, 64> : bn == 128 ? qmk_gemm::gemm_f16_tn_kernel<128, false, WQ, 1, false, 64> : nullptr;
+}
+static GemmKernel gemm_kernel_64(int bn, bool fuse, int wq) {
+  return wq == 0 ? gemm_kernel_64<0>(bn, fuse) : wq == 1 ? gemm_kernel_64<1>(bn, fuse) : gemm_kernel_64<2>(bn, fuse);
+}
 template <int WQ, bool RS = false>
 static GemmKernel gemm_kernel_wq(int bn, bool fuse) {
   if (fuse) return bn == 32 ? qmk_gemm::gemm_f16_tn_kernel<32, true, WQ, 1, RS> : qmk_gemm::gemm_f16_tn_kernel<64, true, WQ, 1, RS>;
@@ -194,7 +203,8 @@ static bool box_n_ok(int box_n, bool fuse, int wq) {
   return box_n == 32 || box_n == 64 || (box_n == 128 && rows == 128);
 }
 // (split activations exist for fp16 and FP8 weights; `scaled`: fp16 matrices with row scales)
-static GemmKernel gemm_kernel(int bn, bool fuse, int wq, int ah, bool scaled) {
+static GemmKernel gemm_kernel(int bn, bool fuse, int wq, int ah, bool scaled, int am = 128) {
+  if (am == 64) return gemm_kernel_64(bn, fuse, wq);
   if (ah == 2) return gemm_kernel_split(bn, fuse, wq);
   if (wq == 0) return scaled ? gemm_kernel_wq<0, true>(bn, fuse) : gemm_kernel_wq<0, false>(bn, fuse);
   return wq == 1 ? gemm_kernel_wq<1>(bn, fuse) : gemm_kernel_wq<2>(bn, fuse);
@@ -225,6 +235,12 @@ int ensure_gemm_attrs(std::string *err) {
             for (int scaled = 0; scaled < (wq == 0 && ah == 1 ? 2 : 1) && e == cudaSuccess; ++scaled)
               e = cudaFuncSetAttribute(reinterpret_cast<const void *>(gemm_kernel(bn, fuse != 0, wq, ah, scaled != 0)),
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gemm_smem(bn, fuse != 0, wq, ah)));
+    for (int wq = 0; wq < 3 && e == cudaSuccess; ++wq)
+      for (int fuse = 0; fuse < 2 && e == cudaSuccess; ++fuse)
+        for (int bn = 32; bn <= 128 && e == cudaSuccess; bn *= 2)
+          if (gemm_kernel_64(bn, fuse != 0, wq))
+            e = cudaFuncSetAttribute(reinterpret_cast<const void *>(gemm_kernel_64(bn, fuse != 0, wq)), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(qmk_gemm::smem_bytes_for(fuse ? 2 * bn : bn, wq, 1, 64)));
     for (int mode = 0; mode < 3 && e == cudaSuccess; ++mode)
       for (int scaled = 0; scaled < 2 && e == cudaSuccess; ++scaled)
         e = cudaFuncSetAttribute(reinterpret_cast<const void *>(pair_kernel(mode, scaled != 0)), cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -273,8 +289,9 @@ thread_local int *t_amax_idx = nullptr;
 // A launch of at most one CTA per SM takes the full depth whatever the budget: nothing of its own shares the SM, and with the
 // three stages of a 128-wide tile that fit 96 KB its K loop waits for L2.  Prompts of 31 / 109 / 500 / 1000 tokens with every
 // kernel of the chain a programmatic dependent 1.07 / 1.24 / 1.79 / 2.42 -> 0.91 / 1.06 / 1.56 / 2.10 ms (2000: no such launch).
-static size_t set_ring(qmk_gemm::Groups *gr, int sb, int wq, long ctas = 0) {
-  const qmk_gemm::RingGeometry g = qmk_gemm::ring_geometry(sb, wq, ctas > sm_count() ? t_ring_budget : 0, t_ah);
+// `kblocks`: no more stages than that.
+static size_t set_ring(qmk_gemm::Groups *gr, int sb, int wq, long ctas, int am, int kblocks) {
+  const qmk_gemm::RingGeometry g = qmk_gemm::ring_geometry(sb, wq, ctas > sm_count() ? t_ring_budget : 0, t_ah, am, kblocks);
   gr->stages = g.stages;
   gr->ring_bytes = g.ring_bytes;
   return g.smem_bytes;
@@ -287,7 +304,19 @@ SplitActScope::~SplitActScope() { t_ah = prev_; }
 void set_argmax_target(float *val, int *idx) { t_amax_val = val; t_amax_idx = idx; }
 thread_local bool t_out_f16 = false;        // the next grouped GEMM of this thread stores fp16
 void set_out_f16(bool on) { t_out_f16 = on; }
-size_t selftest_ring(qmk_gemm::Groups *gr) { return set_ring(gr, 128, 0); }
+size_t selftest_ring(qmk_gemm::Groups *gr) { return set_ring(gr, 128, 0, 1, 128, 1); }
+
+// Weights for the next launches of this thread to bring into L2 (see PrefetchScope).
+thread_local PrefetchList t_prefetch;
+PrefetchScope::PrefetchScope(const PrefetchList &list) : prev_(t_prefetch) { t_prefetch = list; }
+PrefetchScope::~PrefetchScope() { t_prefetch = prev_; }
+static void set_prefetch(qmk_gemm::Groups *gr, long ctas) {
+  for (int i = 0; i < qmk_gemm::MAX_PREFETCH; ++i) {
+    gr->prefetch[i] = static_cast<const unsigned char *>(t_prefetch.ptr[i]);
+    gr->prefetch_bytes[i] = t_prefetch.ptr[i] ? static_cast<uint32_t>(t_prefetch.bytes[i]) : 0u;
+    gr->prefetch_piece[i] = static_cast<uint32_t>(((t_prefetch.bytes[i] + ctas - 1) / ctas + 15) / 16 * 16);
+  }
+}
 
 // A maps with short boxes (`a_box_rows` < 128 rows per box, a multiple of 8; decode steps with few live rows): one
 // row tile only, and the epilogue must stay inside the box.
@@ -298,6 +327,11 @@ static bool a_box_ok(int a_box_rows, int M, int *rows, uint32_t *a_box_bytes, st
   if (*rows > a_box_rows) *rows = a_box_rows;
   *a_box_bytes = static_cast<uint32_t>(a_box_rows) * qmk_gemm::BK * 2;
   return true;
+}
+
+// Rows of the MMA for a launch: 64 where its only row tile has a short A box of at most that many and the tile has such a kernel.
+static int mma_rows(const qmk_gemm::Groups &gr, int box_n, bool fuse, int wq) {
+  return gr.a_box_bytes > 0 && gr.a_box_bytes <= 64u * qmk_gemm::BK * 2 && t_ah == 1 && gr.row_scale[0] == nullptr && gemm_kernel_64(box_n, fuse, wq) ? 64 : qmk_gemm::BM;
 }
 
 // C_g[M x N_g] fp32 = A[M x K] * B_g[N_g x K]^T for up to three matrices B_g in one launch.  M, N_g multiples of
@@ -332,8 +366,10 @@ int launch_gemm_grouped(const CUtensorMap &map_a, int ngroups, const CUtensorMap
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
   int rows = live_rows > 0 ? live_rows : M;   // rows the epilogue stores (the rest of the tile is padding)
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
-  const size_t smem = set_ring(&gr, box_n, wq, static_cast<long>(grid.x) * grid.y);
-  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah, gr.row_scale[0] != nullptr), grid, dim3(qmk_gemm::threads_for(wq, t_ah)), smem, stream,
+  const int am = mma_rows(gr, box_n, false, wq);
+  set_prefetch(&gr, static_cast<long>(grid.x) * grid.y);
+  const size_t smem = set_ring(&gr, box_n, wq, static_cast<long>(grid.x) * grid.y, am, K / qmk_gemm::BK);
+  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah, gr.row_scale[0] != nullptr, am), grid, dim3(qmk_gemm::threads_for(box_n, wq, t_ah, am)), smem, stream,
                                 map_a, b0, b1, b2, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
   return QMK_OK;
@@ -364,8 +400,10 @@ int launch_gemm_swiglu(const CUtensorMap &map_a, const CUtensorMap &map_gate, co
   int rows = live_rows > 0 ? live_rows : M;
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
-  const size_t smem = set_ring(&gr, 2 * box_n, wq, static_cast<long>(N / box_n) * (M / qmk_gemm::BM));
-  cudaError_t e = launch_kernel(gemm_kernel(box_n, true, wq, t_ah, gr.row_scale[0] != nullptr), dim3(N / box_n, M / qmk_gemm::BM), dim3(qmk_gemm::threads_for(wq, t_ah)),
+  const int am = mma_rows(gr, box_n, true, wq);
+  set_prefetch(&gr, static_cast<long>(N / box_n) * (M / qmk_gemm::BM));
+  const size_t smem = set_ring(&gr, 2 * box_n, wq, static_cast<long>(N / box_n) * (M / qmk_gemm::BM), am, K / qmk_gemm::BK);
+  cudaError_t e = launch_kernel(gemm_kernel(box_n, true, wq, t_ah, gr.row_scale[0] != nullptr, am), dim3(N / box_n, M / qmk_gemm::BM), dim3(qmk_gemm::threads_for(2 * box_n, wq, t_ah, am)),
                                 smem, stream, map_a, map_gate, map_up, map_up, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
   return QMK_OK;
@@ -395,8 +433,10 @@ int launch_gemm_splitk(const CUtensorMap &map_a, const CUtensorMap &map_b, float
   int rows = live_rows > 0 ? live_rows : M;
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
-  const size_t smem = set_ring(&gr, box_n, wq, static_cast<long>(N / box_n) * (M / qmk_gemm::BM) * splits);
-  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah, gr.row_scale[0] != nullptr), dim3(N / box_n, M / qmk_gemm::BM, splits), dim3(qmk_gemm::threads_for(wq, t_ah)),
+  const int am = mma_rows(gr, box_n, false, wq);
+  set_prefetch(&gr, static_cast<long>(N / box_n) * (M / qmk_gemm::BM) * splits);
+  const size_t smem = set_ring(&gr, box_n, wq, static_cast<long>(N / box_n) * (M / qmk_gemm::BM) * splits, am, gr.kblocks_per_split);
+  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah, gr.row_scale[0] != nullptr, am), dim3(N / box_n, M / qmk_gemm::BM, splits), dim3(qmk_gemm::threads_for(box_n, wq, t_ah, am)),
                                 smem, stream, map_a, map_b, map_b, map_b, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
   return QMK_OK;
@@ -576,6 +616,8 @@ int ensure_workspace(Workspace &w, int rows, bool *no_room = nullptr) {
 // q, k, v, o, gate, up, down of a layer
 constexpr int MAT_ROWS[7] = {qmk_pf::QS, qmk_pf::KVS, qmk_pf::KVS, qmk_pf::H, qmk_pf::I, qmk_pf::I, qmk_pf::H};
 constexpr int MAT_COLS[7] = {qmk_pf::H, qmk_pf::H, qmk_pf::H, qmk_pf::QS, qmk_pf::H, qmk_pf::H, qmk_pf::I};
+
+size_t weight_bytes(int j, int wq) { return static_cast<size_t>(MAT_ROWS[j]) * (wq ? qmk_tc::packed_row(wq, MAT_COLS[j]).pitch : 2u * MAT_COLS[j]); }
 
 // Buffers of the expanded layer (32 MB), on first use.  Where they do not fit in memory `expanded` stays null.
 int ensure_expanded(Workspace &w) {
@@ -839,6 +881,17 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
       return qmk_tc::launch_gemm_splitk(a, wmap_for(l, j, box_n), c, Mrows, H, K, od_splits, w.status, env.timeout_ms, stream, &err, box_n,
                                         live, 0, wq, wptr(l, j));
     };
+    // Weights for the launches of this chunk to bring into L2 (single CTAs multiplying a layer's matrices as they are).
+    auto ahead_of = [&](int l, std::initializer_list<int> js) {
+      qmk_tc::PrefetchList list;
+      int i = 0;
+      for (int j : js)
+        if (!by_pairs && wq == wfmt && l < num_layers) {
+          list.ptr[i] = wptr(l, j);
+          list.bytes[i++] = weight_bytes(j, wq);
+        }
+      return list;
+    };
     CUtensorMap map_kc, map_vc;   // the caches up to this chunk's last position, all layers
     memset(&map_kc, 0, sizeof(map_kc));
     memset(&map_vc, 0, sizeof(map_vc));
@@ -908,6 +961,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
         // its length (9.8 of 26 us at 2048 rows with fp32); the consumer below rounds to fp16 anyway
         // (split activations: fp32, the operands downstream are not rounded to fp16)
         qmk_tc::set_out_f16(!split);
+        const qmk_tc::PrefetchScope ahead(ahead_of(l, {3}));
         rc = gemm_group(map_xn, l, 3, js, cs, ns, M, H, T);
         qmk_tc::set_out_f16(false);
         if (rc != QMK_OK) break;
@@ -943,7 +997,10 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
       } else
         PF_CUDA(qmk_tc::launch_kernel(causal_attention_mma, dim3((T + ATM_Q - 1) / ATM_Q, NKV), dim3(ATM_THREADS), ATM_SMEM_BYTES, stream,
                                       w.qr, kc, vc, w.attn, T, pos0, max_seq_len, attn_scale));
-      rc = gemm_od(map_attn, l, 3, w.o, M, QS, T);
+      {
+        const qmk_tc::PrefetchScope ahead(ahead_of(l, {4, 5, 6}));
+        rc = gemm_od(map_attn, l, 3, w.o, M, QS, T);
+      }
       if (rc != QMK_OK) break;
       PF_CUDA(norm_rows(w.o, reinterpret_cast<const __half *>(r[7])));
       {
@@ -961,6 +1018,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
         }
         if (rc != QMK_OK) break;
       }
+      const qmk_tc::PrefetchScope ahead(ahead_of(l + 1, {0, 1, 2}));
       rc = gemm_od(map_act, l, 6, w.down, M, I, T);
       if (rc != QMK_OK) break;
     }
@@ -1181,6 +1239,16 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
       auto wm = [&](int j) -> const CUtensorMap & { return w.wmap32[l][j]; };
       static const int rec_slot[7] = {1, 2, 3, 6, 8, 9, 10};   // q, k, v, o, gate, up, down inside a layer record
       auto wp = [&](int j) { return reinterpret_cast<const void *>(r[rec_slot[j]]); };
+      auto ahead_of = [&](int layer, std::initializer_list<int> js) {
+        qmk_tc::PrefetchList list;
+        int i = 0;
+        for (int j : js)
+          if (layer < num_layers) {
+            list.ptr[i] = reinterpret_cast<const void *>(rec[static_cast<size_t>(layer) * 12 + rec_slot[j]]);
+            list.bytes[i++] = weight_bytes(j, wq);
+          }
+        return list;
+      };
       PF_CUDA(qmk_tc::launch_kernel(add_rmsnorm_rows<false>, dim3(B), dim3(256), 0, s, w.x, l > 0 ? w.down : nullptr, DOWN_SPLITS, PART,
                                     reinterpret_cast<const __half *>(r[0]), w.xn, nullptr));
       {
@@ -1188,6 +1256,7 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
         float *const cs[3] = {w.q, w.k, w.v};
         const int ns[3] = {QS, KVS, KVS};
         const void *raws[3] = {wp(0), wp(1), wp(2)};
+        const qmk_tc::PrefetchScope ahead(ahead_of(l, {3}));
         if ((r2 = qmk_tc::launch_gemm_grouped(w.map_xn_b, 3, maps, cs, ns, M, H, TILE_N, w.status, env.timeout_ms, s, &err,
                                               live, a_box, wq, raws)) != QMK_OK)
           return r2;
@@ -1204,14 +1273,18 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
                                       rope, cosv, sinv, w.k_ptrs, w.v_ptrs, layer_off, w.positions, w.attn, max_seq_len, attn_scale,
                                       w.status, static_cast<unsigned long long>(env.timeout_ms) * 1000000ull, w.split_part,
                                       w.split_count));
-      if ((r2 = qmk_tc::launch_gemm_splitk(w.map_attn_b, wm(3), w.o, M, H, QS, O_SPLITS, w.status, env.timeout_ms, s, &err,
-                                           TILE_N, live, a_box, wq, wp(3))) != QMK_OK)
-        return r2;
+      {
+        const qmk_tc::PrefetchScope ahead(ahead_of(l, {4, 5, 6}));
+        if ((r2 = qmk_tc::launch_gemm_splitk(w.map_attn_b, wm(3), w.o, M, H, QS, O_SPLITS, w.status, env.timeout_ms, s, &err,
+                                             TILE_N, live, a_box, wq, wp(3))) != QMK_OK)
+          return r2;
+      }
       PF_CUDA(qmk_tc::launch_kernel(add_rmsnorm_rows<false>, dim3(B), dim3(256), 0, s, w.x, w.o, O_SPLITS, PART,
                                     reinterpret_cast<const __half *>(r[7]), w.xn, nullptr));
       if ((r2 = qmk_tc::launch_gemm_swiglu(w.map_xn_b, wm(4), wm(5), w.act, M, I, H, w.status, env.timeout_ms, s, &err, TILE_N,
                                            live, a_box, wq, wp(4), wp(5))) != QMK_OK)
         return r2;
+      const qmk_tc::PrefetchScope ahead(ahead_of(l + 1, {0, 1, 2}));
       if ((r2 = qmk_tc::launch_gemm_splitk(w.map_act_b, wm(6), w.down, M, H, I, DOWN_SPLITS, w.status, env.timeout_ms, s, &err,
                                            TILE_N, live, a_box, wq, wp(6))) != QMK_OK)
         return r2;

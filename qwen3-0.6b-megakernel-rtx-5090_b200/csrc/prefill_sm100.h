@@ -43,6 +43,19 @@ class SplitActScope {
  private:
   int prev_;
 };
+// Weight matrices (up to three, sizes in bytes, multiples of 16) that the single-CTA GEMM launches of this thread bring into L2
+// for the launches behind them.
+struct PrefetchList {
+  const void *ptr[3] = {nullptr, nullptr, nullptr};
+  size_t bytes[3] = {0, 0, 0};
+};
+class PrefetchScope {
+ public:
+  explicit PrefetchScope(const PrefetchList &list);
+  ~PrefetchScope();
+ private:
+  PrefetchList prev_;
+};
 size_t selftest_ring(qmk_gemm::Groups *gr);   // ring geometry of the bounded-wait self test's one-tile launch
 template <typename... KArgs, typename... Args>
 cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args) {

@@ -58,6 +58,26 @@ def test_tiny_model_against_oracle(C, n):
     assert eng.positions[:n] == [Ln - 1 + steps for Ln in lens]
 
 
+@pytest.mark.parametrize("n", [17, 64, 65, 128])
+def test_row_tile_edges(C, n):
+    """Up to 64 live rows the GEMMs multiply 64-row tiles (a quarter of the rows in each warp's lanes), above that 128-row ones:
+    sequences either side of the quarters' and the tile's edges against the oracle, one step each (same bar as above)."""
+    vocab, steps, L = 2048, 1, 64
+    w = S.make_weights(seed=29, num_layers=2, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    prompts = [S.make_prompt(1 + i % 5, seed=1200 + i, vocab_size=vocab) for i in range(n)]
+    eng = _engine(w, n, L, engine="gemm", prefill_mode="tensor")
+    dump = torch.zeros(n, steps, vocab, device="cuda")
+    C.set_logits_dump(dump)
+    try:
+        got = eng.generate_ids(prompts, steps)
+    finally:
+        C.set_logits_dump(None)
+    for b in sorted({0, 7, 15, 16, 17, 31, 32, 47, 48, 63, 64, 65, 95, 96, n - 1}):
+        if b < n:
+            want, logits = OracleDecoder(w, max_seq_len=L).generate_ids(prompts[b], steps, keep_logits=True)
+            assert got[b] == want and float((dump[b].cpu() - logits).abs().max()) < LOGIT_TOL, f"sequence {b} of {n}"
+
+
 def test_long_contexts_split_over_several_ctas(C):
     """Two sequences: the attention kernel divides each sequence's cache rows among eight CTAs (nine ring chunks
     per CTA at 2300 tokens, more than the ring has slots) and the last CTA to arrive adds the partial states."""
