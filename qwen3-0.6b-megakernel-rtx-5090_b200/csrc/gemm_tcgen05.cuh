@@ -59,19 +59,10 @@ constexpr int stages_for(int bn, int wq = 0, int ah = 1, int am = 128) {
   return wq ? (bn == 32 ? 8 : bn == 64 ? 6 : 4) : (bn == 32 ? 10 : bn == 64 ? 8 : 6);
 }
 constexpr int MAX_GROUPS = 3;   // matrices sharing one A operand that one launch can multiply (q/k/v, gate/up)
-constexpr int MAX_PREFETCH = 3;
+constexpr int MAX_PREFETCH = 3;                  // (below: Groups::prefetch)
 constexpr int THREADS = 192;                     // fp16 weights: producer warp, MMA warp, four epilogue warps
 constexpr int THREADS_PACKED = 320;              // packed weights: four more warps that only expand K blocks
-// Threads that issue products: two for fp16 weights against at most 64 rows and 64 columns.  A wait costs an issuing thread 125 cycles
-// whatever it finds, and in a loop with waits it issues a product every 66, so one thread takes 263 to 390 cycles for a K block that
-// the tensor core does in 99 (64 rows x 32 columns).  Each has an accumulator of its own, added in the epilogue.  Decode step of 8 /
-// 16 / 64 sequences, 64-token contexts: 767 / 776 / 894 -> 742 / 753 / 853 us.  (128 rows: nothing gained, and a prompt's rows must not
-// depend on the tile that made them; packed weights: the second thread takes issue slots from the expanding warps, 1 to 4 % lost.)
-constexpr int issuers_for(int sb, int wq, int am) { return am == 64 && wq == 0 && sb <= 64 ? 2 : 1; }
-// split activations of packed weights: four warps of their own for the sums; two issuers: a warp for the second
-constexpr int threads_for(int sb, int wq, int ah = 1, int am = 128) {
-  return (wq ? THREADS_PACKED + (ah == 2 ? 128 : 0) : THREADS) + (issuers_for(sb, wq, am) == 2 ? 32 : 0);
-}
+constexpr int threads_for(int wq, int ah = 1) { return wq ? THREADS_PACKED + (ah == 2 ? 128 : 0) : THREADS; }   // split activations: four warps of their own for the sums
 constexpr uint32_t TILE_A_BYTES = BM * BK * 2;   // 16 KB
 // Packed K block of one B row: 64 e4m3 bytes, or 32 bytes of e2m1 pairs
 constexpr uint32_t raw_row_bytes(int wq) { return wq == 1 ? 64u : wq == 2 ? 32u : 0u; }
@@ -160,6 +151,16 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile
       }
     }
   }
+}
+// The same with the waiting out of line: what surrounds the products in the issuing thread's loop costs more than the try itself
+// (16 K blocks in place, 64 rows x 32 columns: 3600 cycles with the loop above inlined, 3200 so, 1600 with no wait between them).
+__device__ __noinline__ bool bar_wait_slow(uint32_t bar, uint32_t parity, volatile int *abort_flag, unsigned int *status,
+                                           unsigned long long budget_ns) {
+  return bar_wait(bar, parity, abort_flag, status, budget_ns);
+}
+__device__ __forceinline__ bool bar_wait_cold(uint32_t bar, uint32_t parity, volatile int *abort_flag, unsigned int *status,
+                                              unsigned long long budget_ns) {
+  return bar_try(bar, parity) || bar_wait_slow(bar, parity, abort_flag, status, budget_ns);
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t bar) {
   asm volatile(
@@ -315,7 +316,7 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 // (packed weights: decode step of 64 NVFP4 sequences 1198 -> 1150 us, of 16 FP8 ones 978 -> 925).  An
 // accumulator of 64 rows lies in lanes 0 .. 15 of each warp's 32: row r in lane 32 * (r / 16) + r % 16.
 template <int BN, bool FUSE = false, int WQ = 0, int AH = 1, bool RS = false, int AM = BM>
-__global__ void __launch_bounds__(threads_for(FUSE ? 2 * BN : BN, WQ, AH, AM), 1)
+__global__ void __launch_bounds__(threads_for(WQ, AH), 1)
 gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b0,
                    const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ CUtensorMap map_b2,
                    const Groups groups, int M, int K, unsigned int *status, unsigned long long budget_ns,
@@ -328,9 +329,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   constexpr int WARP_ROWS = AM / 4;               // rows of a warp's 32 TMEM lanes
   static_assert(WQ == 0 || (FUSE ? 2 * BN : BN) <= 128, "packed weights: at most 128 B rows per stage (scales live in shared memory)");
   constexpr int SB = FUSE ? 2 * BN : BN;          // B rows held per stage / accumulator columns
-  constexpr int ISSUERS = issuers_for(SB, WQ, AM);
-  constexpr int ISSUER_B = ISSUERS == 2 ? threads_for(SB, WQ, AH, AM) / 32 - 1 : 1;   // the second issuer's warp
-  constexpr int NACC = AH == 2 ? 4 : ISSUERS;     // accumulators: one per issuer, or with split activations four that the K blocks take in turn
+  constexpr int NACC = AH == 2 ? 4 : 1;           // accumulators: one, or with split activations four that the K blocks take in turn
   static_assert(NACC * SB <= 512, "TMEM columns");
   constexpr uint32_t RAW_ROW = raw_row_bytes(WQ);
   const int STAGES = groups.stages;
@@ -391,7 +390,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       bar_init(empty(s), 1);
       if (WQ) { bar_init(raw_full(s), 1); bar_init(a_full(s), 1); }
     }
-    bar_init(acc_full, ISSUERS);
+    bar_init(acc_full, 1);
     if (AH == 2)
       for (int a = 0; a < NACC; ++a) { bar_init(blk_full(a), 1); bar_init(blk_free(a), 4); }
     *abort_flag = 0;
@@ -481,7 +480,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         }
       }
     }
-  } else if (ISSUERS == 1 && warp == 1) {
+  } else if (warp == 1) {
     if (elect_one()) {                     // ---- MMA issuer
       bool ok = true;
       int s = 0;                           // slot and parity of K block kb
@@ -489,8 +488,8 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       const uint64_t da0 = smem_desc_sw128(base), db0 = smem_desc_sw128(base + TILE_A);
       uint64_t da = da0, db = db0;         // (a ring ends below 2^18 bytes: the slot's offset does not leave the address field)
       for (int kb = 0; kb < kblocks; ++kb) {
-        ok = bar_wait(full(s), parity, abort_flag, status, budget_ns) &&
-             (!WQ || bar_wait(a_full(s), parity, abort_flag, status, budget_ns)) &&
+        ok = bar_wait_cold(full(s), parity, abort_flag, status, budget_ns) &&
+             (!WQ || bar_wait_cold(a_full(s), parity, abort_flag, status, budget_ns)) &&
              (AH == 1 || kb < NACC || bar_wait(blk_free(kb % NACC), (kb / NACC - 1) & 1, abort_flag, status, budget_ns));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -515,31 +514,6 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         if (++s == STAGES) { s = 0; parity ^= 1u; da = da0; db = db0; }
       }
       if (ok && AH == 1) mma_commit(acc_full);   // accumulator complete
-    }
-  } else if (ISSUERS == 2 && (warp == 1 || warp == ISSUER_B)) {
-    if (elect_one()) {                     // ---- two MMA issuers: one takes the stages of even number, one those of odd (so that each
-                                           //      meets the uses of a stage in order)
-      const int s0 = warp == ISSUER_B ? 1 : 0;
-      bool ok = true;
-      int s = s0, lap = 0;                 // K block lap + s is in stage s
-      uint32_t parity = 0, accumulate = 0;
-      const uint64_t da0 = smem_desc_sw128(base) + s0 * (STAGE_BYTES >> 4), db0 = smem_desc_sw128(base + TILE_A) + s0 * (STAGE_BYTES >> 4);
-      uint64_t da = da0, db = db0;
-      const uint32_t acc = tmem_base + s0 * SB;
-      for (int kb = s0; kb < kblocks && s0 < STAGES; kb = lap + s) {
-        ok = bar_wait(full(s), parity, abort_flag, status, budget_ns);
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-        for (int j = 0; j < BK / 16; ++j) mma_f16_ss(acc, da + 2u * j, db + 2u * j, j > 0 ? 1u : accumulate, idesc_for(SB, AM));
-        accumulate = 1;
-        if (kb + STAGES < kblocks) mma_commit(empty(s));
-        da += 2 * (STAGE_BYTES >> 4);
-        db += 2 * (STAGE_BYTES >> 4);
-        s += 2;
-        if (s >= STAGES) { s = s0; lap += STAGES; parity ^= 1u; da = da0; db = db0; }
-      }
-      if (ok) mma_commit(acc_full);        // this issuer's accumulator complete (or not begun: `both`)
     }
   } else {                                 // ---- warps 2..5: epilogue, each owns TMEM lanes 32 * (warp % 4) ..; packed
                                            //      weights: first they and warps 6..9 expand the K blocks
@@ -668,7 +642,6 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       }
     }
     if (AH == 1 && warp < 6) {
-    const bool both = ISSUERS == 2 && kblocks > 1 && STAGES > 1;     // the second accumulator holds a part of the sums
     // warp-uniform outcome: the TMEM loads below are warp-wide instructions
     const bool ok = __all_sync(0xffffffffu, bar_wait(acc_full, 0, abort_flag, status, budget_ns));
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -681,19 +654,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const uint32_t tg = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(c * 16);
         tmem_ld16(tg, g);
         tmem_ld16(tg + BN, u);
-        if (both) {
-          uint32_t g2[16], u2[16];
-          tmem_ld16(tg + SB, g2);
-          tmem_ld16(tg + SB + BN, u2);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            g[i] = __float_as_uint(__uint_as_float(g[i]) + __uint_as_float(g2[i]));
-            u[i] = __float_as_uint(__uint_as_float(u[i]) + __uint_as_float(u2[i]));
-          }
-        } else {
-          tmem_ld_wait();
-        }
+        tmem_ld_wait();
         if (row < M) {
           uint32_t packed[8];
 #pragma unroll
@@ -731,15 +692,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         uint32_t r[32];
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(c * 32);
         tmem_ld32(taddr, r);
-        if (both) {
-          uint32_t r2[32];
-          tmem_ld32(taddr + SB, r2);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(r2[i]));
-        } else {
-          tmem_ld_wait();
-        }
+        tmem_ld_wait();
         if (RS) {
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {

@@ -369,7 +369,7 @@ int launch_gemm_grouped(const CUtensorMap &map_a, int ngroups, const CUtensorMap
   const int am = mma_rows(gr, box_n, false, wq);
   set_prefetch(&gr, static_cast<long>(grid.x) * grid.y);
   const size_t smem = set_ring(&gr, box_n, wq, static_cast<long>(grid.x) * grid.y, am, K / qmk_gemm::BK);
-  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah, gr.row_scale[0] != nullptr, am), grid, dim3(qmk_gemm::threads_for(box_n, wq, t_ah, am)), smem, stream,
+  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah, gr.row_scale[0] != nullptr, am), grid, dim3(qmk_gemm::threads_for(wq, t_ah)), smem, stream,
                                 map_a, b0, b1, b2, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
   return QMK_OK;
@@ -403,7 +403,7 @@ int launch_gemm_swiglu(const CUtensorMap &map_a, const CUtensorMap &map_gate, co
   const int am = mma_rows(gr, box_n, true, wq);
   set_prefetch(&gr, static_cast<long>(N / box_n) * (M / qmk_gemm::BM));
   const size_t smem = set_ring(&gr, 2 * box_n, wq, static_cast<long>(N / box_n) * (M / qmk_gemm::BM), am, K / qmk_gemm::BK);
-  cudaError_t e = launch_kernel(gemm_kernel(box_n, true, wq, t_ah, gr.row_scale[0] != nullptr, am), dim3(N / box_n, M / qmk_gemm::BM), dim3(qmk_gemm::threads_for(2 * box_n, wq, t_ah, am)),
+  cudaError_t e = launch_kernel(gemm_kernel(box_n, true, wq, t_ah, gr.row_scale[0] != nullptr, am), dim3(N / box_n, M / qmk_gemm::BM), dim3(qmk_gemm::threads_for(wq, t_ah)),
                                 smem, stream, map_a, map_gate, map_up, map_up, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
   return QMK_OK;
@@ -436,7 +436,7 @@ int launch_gemm_splitk(const CUtensorMap &map_a, const CUtensorMap &map_b, float
   const int am = mma_rows(gr, box_n, false, wq);
   set_prefetch(&gr, static_cast<long>(N / box_n) * (M / qmk_gemm::BM) * splits);
   const size_t smem = set_ring(&gr, box_n, wq, static_cast<long>(N / box_n) * (M / qmk_gemm::BM) * splits, am, gr.kblocks_per_split);
-  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah, gr.row_scale[0] != nullptr, am), dim3(N / box_n, M / qmk_gemm::BM, splits), dim3(qmk_gemm::threads_for(box_n, wq, t_ah, am)),
+  cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah, gr.row_scale[0] != nullptr, am), dim3(N / box_n, M / qmk_gemm::BM, splits), dim3(qmk_gemm::threads_for(wq, t_ah)),
                                 smem, stream, map_a, map_b, map_b, map_b, gr, rows, K, status, budget, 0);
   if (e != cudaSuccess) { *err = std::string("gemm launch: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
   return QMK_OK;
