@@ -65,10 +65,7 @@ __device__ __forceinline__ bool beyond_half4(float4 v) {
 // x[t][:] = embedding row of token t as fp32.  grid = T, block = 256.  `wq`: 0 fp16 rows; 1 FP8-E4M3 rows (H bytes,
 // then a 16-byte trailer with the fp32 row scale); 2 NVFP4 rows (H / 2 bytes of e2m1 pairs, low nibble first, H / 16
 // e4m3 block scales, then the trailer with the fp32 tensor scale).
-__global__ void embed_rows(const int *tokens, const void *embed, int wq, float *x) {
-  pdl_wait();
-  pdl_trigger();
-  const int t = blockIdx.x;
+__device__ __forceinline__ void embed_row(const int *tokens, const void *embed, int wq, float *x, int t) {
   float *out = x + static_cast<size_t>(t) * H;
   if (wq == 0) {
     const __half *row = static_cast<const __half *>(embed) + static_cast<size_t>(tokens[t]) * H;
@@ -90,6 +87,11 @@ __global__ void embed_rows(const int *tokens, const void *embed, int wq, float *
       out[k] = scale * bs * ((code & 8u) ? -mag : mag);
     }
   }
+}
+__global__ void embed_rows(const int *tokens, const void *embed, int wq, float *x) {
+  pdl_wait();
+  pdl_trigger();
+  embed_row(tokens, embed, wq, x, blockIdx.x);
 }
 
 // Residual add + RMSNorm: x[t] += add[t] (if add), y[t] = fp16(x[t] * rstd * w).  grid = T, block = 256.

@@ -518,6 +518,7 @@ struct Workspace {                  // per device, allocated on first use, never
   unsigned char *packed = nullptr;       // tables of a packed prefill (row info, attention items, per-sequence descriptors and cache pointers)
   int **log_ptrs = nullptr;
   float *split_part = nullptr;            // partial attention states of split sequences (decode_attention_ring)
+  qmk_pf::DamPlan *attn_plan = nullptr;   // the step's list of attention pieces (decode_attention_mma)
   unsigned int *split_count = nullptr;    // arrival counters, one per (sequence, kv head); zero between launches
   float *logits = nullptr;
   int logits_vocab = 0;
@@ -1085,6 +1086,10 @@ unsigned int __float_as_uint_host(float f) {
 constexpr int MAX_BATCH = 128;      // one 128-row GEMM tile of sequences
 
 constexpr int MAX_ATTN_SPLITS = 8;
+constexpr size_t SPLIT_PART_FLOATS = static_cast<size_t>(MAX_BATCH) * qmk_pf::NKV * MAX_ATTN_SPLITS * 2 * (qmk_pf::D + 2);
+constexpr int MAX_ATTN_CTAS = 1024;
+static_assert(qmk_pf::dam_max_states(MAX_BATCH, MAX_ATTN_CTAS) * qmk_pf::DAM_PART <= SPLIT_PART_FLOATS &&
+                  MAX_BATCH <= qmk_pf::DAM_MAX_BATCH && MAX_LAYERS <= qmk_pf::DAM_MAX_LAYERS, "partial states of decode_attention_mma");
 int ensure_decode_workspace(Workspace &w, const void *lm_head, int vocab, int wq) {
   if (!w.positions) {
     PF_CUDA(cudaMalloc(&w.positions, sizeof(int) * MAX_BATCH));
@@ -1096,7 +1101,8 @@ int ensure_decode_workspace(Workspace &w, const void *lm_head, int vocab, int wq
     PF_CUDA(cudaMalloc(&w.v_ptrs, sizeof(void *) * MAX_BATCH));
     PF_CUDA(cudaMalloc(&w.log_ptrs, sizeof(void *) * MAX_BATCH));
     PF_CUDA(cudaMalloc(&w.kv_maps, sizeof(CUtensorMap) * 2 * MAX_BATCH));
-    PF_CUDA(cudaMalloc(&w.split_part, sizeof(float) * MAX_BATCH * qmk_pf::NKV * MAX_ATTN_SPLITS * 2 * (qmk_pf::D + 2)));
+    PF_CUDA(cudaMalloc(&w.split_part, sizeof(float) * SPLIT_PART_FLOATS));
+    PF_CUDA(cudaMalloc(&w.attn_plan, sizeof(qmk_pf::DamPlan) + sizeof(qmk_pf::DamPiece) * qmk_pf::dam_max_pieces(MAX_BATCH, MAX_ATTN_CTAS)));
     PF_CUDA(cudaMalloc(&w.split_count, sizeof(unsigned int) * MAX_BATCH * qmk_pf::NKV));
     PF_CUDA(cudaMemset(w.split_count, 0, sizeof(unsigned int) * MAX_BATCH * qmk_pf::NKV));
   }
@@ -1221,7 +1227,9 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
   // 78 MB of padding logits per step).  Measured: 6.5 k -> 7.5 k tok/s at B = 16, 18.3 k -> 21.0 k at B = 64.
   constexpr int TILE_N = 32, O_SPLITS = 4, DOWN_SPLITS = 4;
   const int live = B, a_box = w.a_rows;
-  // Few sequences: split every sequence's cache rows over several CTAs so that the attention fills the device
+  // decode_attention_mma shares all cache rows out among two CTAs per SM.
+  const int attn_ctas = std::min(2 * qmk_tc::g_sms[dev], MAX_ATTN_CTAS);
+  // decode_attention_ring, few sequences: split every sequence's cache rows over several CTAs so that the attention fills the device
   // (two CTAs fit on an SM): 8 B CTAs otherwise, each streaming a whole sequence through one ring.
   int attn_splits = (2 * qmk_tc::g_sms[dev]) / (B * NKV);   // (gemm_box_n above cached the SM count of this device)
   attn_splits = attn_splits < 1 ? 1 : attn_splits > MAX_ATTN_SPLITS ? MAX_ATTN_SPLITS : attn_splits;
@@ -1231,7 +1239,7 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
     qmk_tc::PdlScope pdl_scope(env.pdl != 0);   // every launch below may start behind its predecessor's tail
     {
       qmk_tc::PdlScope first(false);            // (the first kernel of a step has no predecessor inside the step)
-      PF_CUDA(qmk_tc::launch_kernel(embed_rows, dim3(B), dim3(256), 0, s, w.tokens, embed_weight, wq, w.x));
+      PF_CUDA(qmk_tc::launch_kernel(embed_rows_and_plan, dim3(B + 1), dim3(256), 0, s, w.tokens, embed_weight, wq, w.x, w.positions, attn_ctas, w.attn_plan));
     }
     for (int l = 0; l < num_layers; ++l) {
       const unsigned long long *r = rec.data() + static_cast<size_t>(l) * 12;
@@ -1262,11 +1270,11 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
           return r2;
       }
       if (env.attn_mma)
-        PF_CUDA(qmk_tc::launch_kernel(decode_attention_mma, dim3(B, NKV, attn_splits), dim3((DAM_WARPS + 1) * 32), DAM_SMEM_BYTES, s,
+        PF_CUDA(qmk_tc::launch_kernel(decode_attention_mma, dim3(attn_ctas), dim3((DAM_WARPS + 1) * 32), DAM_SMEM_BYTES, s,
                                       w.q, w.k, w.v, reinterpret_cast<const __half *>(r[4]), reinterpret_cast<const __half *>(r[5]),
-                                      rope, cosv, sinv, w.k_ptrs, w.v_ptrs, layer_off, w.positions, w.attn, max_seq_len, attn_scale,
+                                      rope, cosv, sinv, w.k_ptrs, w.v_ptrs, layer_off, w.attn_plan, l, w.attn, max_seq_len, attn_scale,
                                       w.status, static_cast<unsigned long long>(env.timeout_ms) * 1000000ull, w.split_part,
-                                      w.split_count, w.kv_maps, l * NKV * max_seq_len));
+                                      w.split_count, w.kv_maps));
       else
         PF_CUDA(qmk_tc::launch_kernel(decode_attention_ring, dim3(B, NKV, attn_splits), dim3((DAR_WARPS + 1) * 32), DAR_SMEM_BYTES, s,
                                       w.q, w.k, w.v, reinterpret_cast<const __half *>(r[4]), reinterpret_cast<const __half *>(r[5]),

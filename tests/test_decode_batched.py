@@ -210,6 +210,34 @@ def test_both_decode_attention_kernels(C, mma):
     assert worst < LOGIT_TOL
 
 
+@pytest.mark.parametrize("lens", [[1], [700, 20, 1], [13 * 16 + 1, 13 * 16, 12 * 16 + 1, 12 * 16, 1, 2],
+                                  [700] + [16 * i for i in range(1, 23)], [1 + (53 * i) % 300 for i in range(37)],
+                                  [1 + (101 * i) % 400 for i in range(64)], [40] * 128],
+                         ids=["one", "split", "edges", "cut", "37", "64", "128"])
+def test_attention_pieces(C, lens):
+    """The attention's list of pieces: items of one range and of several, ranges whole and cut in two or four, fewer pieces than
+    CTAs and more (64 and 128 sequences: CTAs take further pieces), against the CUDA-core kernel with a CTA per item and range.  Both
+    round the same fp32 result to fp16, so logits differ by roundings of one output and what they do downstream: the bar of
+    this file.  Who takes which piece does not show: a second run is the same bit for bit."""
+    vocab, steps, L, n = 2048, 2, 768, len(lens)
+    w = S.make_weights(seed=31, num_layers=2, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    prompts = [S.make_prompt(Ln, seed=1500 + i, vocab_size=vocab) for i, Ln in enumerate(lens)]
+    eng = _engine(w, n, L, engine="gemm", prefill_mode="tensor")
+    runs = []
+    for mma in (1, 1, 0):
+        dump = torch.zeros(n, steps, vocab, device="cuda")
+        C.set_decode_attention(mma)
+        C.set_logits_dump(dump)
+        try:
+            eng.generate_ids(prompts, steps)
+        finally:
+            C.set_logits_dump(None)
+            C.set_decode_attention(1)
+        runs.append((dump.cpu(), [k[:, :, :Ln + steps - 1].cpu() for k, Ln in zip(eng._k_caches, lens)]))
+    assert torch.equal(runs[0][0], runs[1][0]) and all(torch.equal(a, b) for a, b in zip(runs[0][1], runs[1][1]))
+    assert float((runs[0][0][:, 0] - runs[2][0][:, 0]).abs().max()) < LOGIT_TOL
+
+
 def test_refusals(C):
     vocab = 2048
     w = S.make_weights(seed=1, num_layers=2, vocab_size=vocab, max_seq_len=16)
