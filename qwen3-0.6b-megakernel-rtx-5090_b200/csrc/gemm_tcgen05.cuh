@@ -753,8 +753,9 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 }
 
 // Values of packed rows as fp16 matrices [rows][K] (exact: e4m3, and e2m1 x e4m3 block scale, have at most six
-// significant bits) and their fp32 row scales, for up to seven matrices in one launch: a warp per row, a lane per 16
-// values.  Bound by writing the fp16 bytes (31.5 MB a layer).
+// significant bits) and their fp32 row scales, for up to seven matrices in one launch: a warp per row.
+// Bound by writing the fp16 bytes (31.5 MB a layer): 13.6 us of a 4096-row layer with 16 values, two half-filled stores, a lane, 11.9 with
+// eight; prompts of 500 / 1000 NVFP4 tokens 1.99 / 2.48 -> 1.92 / 2.41 ms.
 struct ExpandArgs {
   const unsigned char *src[7];
   __half *dst[7];
@@ -785,31 +786,35 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_packed_rows(const __gri
       scale = a.scale[j] + r;
     }
   if (lane == 0) *scale = *reinterpret_cast<const float *>(src + so);
-  for (int i = lane; i < K / 16; i += 32) {
-    uint32_t h[8];
-    if (WQ == 1) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(src) + i);
-      h[0] = e4m3x2_to_half2_bits(v.x); h[1] = e4m3x2_to_half2_bits(v.x >> 16);
-      h[2] = e4m3x2_to_half2_bits(v.y); h[3] = e4m3x2_to_half2_bits(v.y >> 16);
-      h[4] = e4m3x2_to_half2_bits(v.z); h[5] = e4m3x2_to_half2_bits(v.z >> 16);
-      h[6] = e4m3x2_to_half2_bits(v.w); h[7] = e4m3x2_to_half2_bits(v.w >> 16);
-    } else {
-      const uint2 v = __ldg(reinterpret_cast<const uint2 *>(src) + i);
-      const uint32_t sb2 = e4m3x2_to_half2_bits(__ldg(src + bs + i));   // low half = the block's scale
-      const __half2 sc = __half2half2(__ushort_as_half(static_cast<unsigned short>(sb2 & 0xFFFFu)));
-      uint32_t lo[4], hi[4];
-      e2m1x8_to_half2x4(v.x, lo);
-      e2m1x8_to_half2x4(v.y, hi);
+  // eight values a lane, so that a warp's store is 512 bytes in a row, and four such pieces at a time (K is a multiple of 1024)
+  for (int i0 = lane; i0 < K / 8; i0 += 128) {
+    uint2 v[4];
+    uint32_t bscale[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const __half2 p = __hmul2(*reinterpret_cast<const __half2 *>(&lo[k]), sc), q = __hmul2(*reinterpret_cast<const __half2 *>(&hi[k]), sc);
-        h[k] = *reinterpret_cast<const uint32_t *>(&p);
-        h[4 + k] = *reinterpret_cast<const uint32_t *>(&q);
-      }
+    for (int p = 0; p < 4; ++p) {
+      const int i = i0 + 32 * p;
+      if (WQ == 1) v[p] = __ldg(reinterpret_cast<const uint2 *>(src) + i);
+      else { v[p].x = __ldg(reinterpret_cast<const uint32_t *>(src) + i); bscale[p] = __ldg(src + bs + (i >> 1)); }
     }
-    uint4 *out = reinterpret_cast<uint4 *>(dst + static_cast<size_t>(i) * 16);
-    out[0] = make_uint4(h[0], h[1], h[2], h[3]);
-    out[1] = make_uint4(h[4], h[5], h[6], h[7]);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      uint32_t h[4];
+      if (WQ == 1) {
+        h[0] = e4m3x2_to_half2_bits(v[p].x); h[1] = e4m3x2_to_half2_bits(v[p].x >> 16);
+        h[2] = e4m3x2_to_half2_bits(v[p].y); h[3] = e4m3x2_to_half2_bits(v[p].y >> 16);
+      } else {
+        const uint32_t sb2 = e4m3x2_to_half2_bits(bscale[p]);           // low half = the block's scale
+        const __half2 sc = __half2half2(__ushort_as_half(static_cast<unsigned short>(sb2 & 0xFFFFu)));
+        uint32_t e[4];
+        e2m1x8_to_half2x4(v[p].x, e);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const __half2 q = __hmul2(*reinterpret_cast<const __half2 *>(&e[k]), sc);
+          h[k] = *reinterpret_cast<const uint32_t *>(&q);
+        }
+      }
+      *reinterpret_cast<uint4 *>(dst + static_cast<size_t>(i0 + 32 * p) * 8) = make_uint4(h[0], h[1], h[2], h[3]);
+    }
   }
 }
 
