@@ -491,7 +491,7 @@ namespace {
 
 constexpr unsigned int PREFILL_RING_BYTES = 96 * 1024;
 constexpr int PAIR_MIN_ROWS = 512;
-constexpr int EXPAND_MIN_ROWS = 384;
+constexpr int EXPAND_MIN_ROWS = 512;
 constexpr int CHUNK = 4096;         // prompt tokens per pass over the weights (a multiple of the GEMM's 128)
 constexpr int MAX_LAYERS = 48;
 
@@ -836,9 +836,8 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     const int pos0 = start_position + c0;
     // Packed weights, long chunks: a GEMM expands its weight tile once per 128 rows; from EXPAND_MIN_ROWS rows on it is
     // cheaper to expand the layer's matrices once and run the fp16 form, on pairs of CTAs above 512 rows.  FP8 / NVFP4, in the
-    // GEMMs -> expanded: 250 tokens 1.42 / 1.44 -> 1.60 / 1.57 ms, 500: 2.02 / 1.98 -> 2.00 / 1.97, 1000: 3.35 / 3.19 -> 2.49 / 2.47,
-    // 4000: 10.6 / 10.1 -> 7.1 / 7.1.  The line was drawn when 380 tokens gained (2.40 -> 2.31); with overlapped launches they
-    // lose 1.75 / 1.76 -> 1.84 / 1.81, and 512 rows would be the better line.
+    // GEMMs -> expanded: 250 tokens 1.42 / 1.44 -> 1.60 / 1.57 ms, 380: 1.73 / 1.72 -> 1.85 / 1.82, 500: 2.02 / 1.98 -> 1.92 (NVFP4),
+    // 1000: 3.35 / 3.19 -> 2.40 / 2.41, 4000: 10.6 / 10.1 -> 7.1 / 7.1.
     wq = wfmt;
     if (wfmt != 0 && !split && M >= EXPAND_MIN_ROWS) {
       rc = ensure_expanded(w);
