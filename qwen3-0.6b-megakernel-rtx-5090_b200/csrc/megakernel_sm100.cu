@@ -279,12 +279,16 @@ Engine *current_engine_unlocked() {
   return e;
 }
 
+thread_local std::string t_error;   // of the calling thread's last call, if that failed: another thread's call may clear the engine's
+
 void clear_error(Engine *e) {
   e->last_status = QMK_OK;
   e->last_error.clear();
+  t_error.clear();
 }
 
 int fail(Engine *e, int code, const std::string &msg) {
+  t_error = msg;
   if (e) { e->last_status = code; e->last_error = msg; }
   fprintf(stderr, "[qwen_megakernel] error %d: %s\n", code, msg.c_str());
   return code;
@@ -597,8 +601,7 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
   if (err == cudaErrorCooperativeLaunchTooLarge)
     return fail(e, QMK_ERR_NOT_RESIDENT, "persistent grid cannot be co-resident on this device");
   if (err != cudaSuccess) return fail(e, QMK_ERR_CUDA, std::string("cudaLaunchCooperativeKernel: ") + cudaGetErrorString(err));
-  e->last_status = QMK_OK;
-  e->last_error.clear();
+  clear_error(e);
   if (synchronize) {
     QMK_CUDA(e, cudaMemcpyAsync(e->status_host, e->status, 16, cudaMemcpyDeviceToHost, stream));
     QMK_CUDA(e, cudaStreamSynchronize(stream));
@@ -1133,7 +1136,7 @@ const char *qmk_last_error(void) {
   static thread_local std::string mine;
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  mine = e ? e->last_error : std::string("no CUDA device");
+  mine = !t_error.empty() ? t_error : e ? e->last_error : std::string("no CUDA device");
   return mine.c_str();
 }
 

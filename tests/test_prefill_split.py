@@ -142,6 +142,25 @@ def test_unfused_switch_covers_the_prefill_op(built_library):
     assert float((rows[0][0].float() - rows[1][0].float()).abs().max()) < 8e-3
 
 
+def test_error_text_survives_another_threads_call(built_library):
+    """The text of a failed call is the failing thread's until its next call: a pass that another thread runs in between (and
+    that clears the device's error) does not take it away; the thread's own next call does."""
+    import threading
+    import qwen_megakernel_C as C
+    from Model.Qwen06B_architecture import Decoder
+    w = S.weights_to(S.make_weights(seed=9, num_layers=2, vocab_size=512, max_seq_len=16), "cuda")
+    eng = Decoder(weights=w, verbose=False, max_seq_len=64)
+    eng.prefill_ids([1, 2, 3, 4, 5])
+    assert C._lib.qmk_selftest_gemm_wait_timeout(0) != 0
+    thread = threading.Thread(target=lambda: (eng.reset(), eng.generate_ids([1, 2, 3, 4, 5, 6], 2)))
+    thread.start()
+    thread.join()
+    assert b"budget_us" in C._lib.qmk_last_error()
+    eng.reset()
+    eng.generate_ids([1, 2, 3, 4, 5, 6], 2)
+    assert b"budget_us" not in C._lib.qmk_last_error()
+
+
 def test_short_prompts_do_not_wait_for_a_chunked_pass(built_library):
     """The workspace of the chunked pass is held for a whole pass (some 20 ms here).  A call of the op that does not use it -
     measured on one that is refused before any GPU work - returns meanwhile."""
