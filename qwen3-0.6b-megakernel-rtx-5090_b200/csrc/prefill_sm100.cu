@@ -961,7 +961,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
         // its length (9.8 of 26 us at 2048 rows with fp32); the consumer below rounds to fp16 anyway
         // (split activations: fp32, the operands downstream are not rounded to fp16)
         qmk_tc::set_out_f16(!split);
-        const qmk_tc::PrefetchScope ahead(ahead_of(l, {3}));
+        const qmk_tc::PrefetchScope ahead(l + 1 < num_layers ? ahead_of(l, {3}) : qmk_tc::PrefetchList());   // (the last layer ends here)
         rc = gemm_group(map_xn, l, 3, js, cs, ns, M, H, T);
         qmk_tc::set_out_f16(false);
         if (rc != QMK_OK) break;
