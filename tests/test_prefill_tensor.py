@@ -186,10 +186,10 @@ def test_refusals(C):
     assert len(eng.generate_ids([1, 2, 3], 2)) == 2
 
 
-@pytest.mark.parametrize("fmt,n", [("fp8", 257), ("fp8", 385), ("nvfp4", 300), ("nvfp4", 1100), ("fp8", 4200)])
+@pytest.mark.parametrize("fmt,n", [("fp8", 257), ("fp8", 385), ("nvfp4", 300), ("nvfp4", 385), ("nvfp4", 1100), ("fp8", 4200)])
 def test_packed_weights_expanded_once_per_layer(C, fmt, n):
-    """Chunks of 384 and more (padded) rows expand a packed layer's matrices once instead of inside the GEMMs: the shortest
-    such chunk (257 tokens), ragged ones, a length with the wide tiles and split K, two chunks of which the second is
+    """Chunks of 512 and more (padded) rows expand a packed layer's matrices once instead of inside the GEMMs: the shortest
+    such chunk (385 tokens), ones below it, ragged ones, a length with the wide tiles and split K, two chunks of which the second is
     short.  The products are the same (exact values, row scale behind the sum), so the first layer's rows equal bit for bit
     those of calls that stay below the switch; from 1024 rows on the RMSNorm kernel adds its squares in another order, which
     moves single operands to the neighbouring fp16 (2^-11 of one of 1024 products): one unit in the last place of a row's
