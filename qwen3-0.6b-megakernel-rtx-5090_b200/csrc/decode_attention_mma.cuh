@@ -513,7 +513,8 @@ __global__ void __launch_bounds__((DAM_WARPS + 1) * 32, 2) decode_attention_mma(
       if (!ok) break;
     }
     ring += (nchunks >> 3) * chains + min(max((nchunks & (DAM_CHAINS - 1)) - chain0, 0), chains);
-    fetched = s_taken > j + 1;           // (a broadcast read: the same for the warp)
+    fetched = s_taken > j + 1;
+    asm volatile("" ::: "memory");       // (the piece is read behind the counter that says it is there)
     if (fetched && s_piece[(j + 1) % DAM_AHEAD].chunks >= 0) fetch_heads(s_piece[(j + 1) % DAM_AHEAD]);
     // this chain's partial state: lanes of quad h hold head h (columns hi, lo of the accumulator fragments)
     float *const item_states = split_part + static_cast<size_t>((b * NKV + g) * splits) * DAM_CHAINS * DAM_PART;
