@@ -165,13 +165,20 @@ __device__ inline void plan_pieces(const int *positions, int batch, int grid, Da
   }
 }
 // Block b < batch: embedding row of sequence b's token (embed_row); the last block: the step's attention pieces.
-__global__ void __launch_bounds__(256) embed_rows_and_plan(const int *tokens, const void *embed, int wq, float *x, const int *positions, int grid,
-                                                          DamPlan *plan) {
+// A row of logits without a largest value (all NaN, or all -inf) leaves 0x7fffffff as its pick.  As in the persistent kernels such a
+// token is an error of the step that reads it (*status = 5, which the call returns), and no address is made of it.
+__global__ void __launch_bounds__(256) embed_rows_and_plan(const int *tokens, const void *embed, int wq, int vocab, float *x, const int *positions,
+                                                          int grid, DamPlan *plan, unsigned int *status) {
   pdl_wait();
   pdl_trigger();
   const int batch = static_cast<int>(gridDim.x) - 1;
-  if (static_cast<int>(blockIdx.x) < batch) embed_row(tokens, embed, wq, x, blockIdx.x);
-  else plan_pieces(positions, batch, grid, plan);
+  if (static_cast<int>(blockIdx.x) >= batch) { plan_pieces(positions, batch, grid, plan); return; }
+  int token = tokens[blockIdx.x];
+  if (token < 0 || token >= vocab) {
+    if (threadIdx.x == 0) atomicCAS(status, 0u, 5u);
+    token = 0;
+  }
+  embed_row(token, embed, wq, x, blockIdx.x);
 }
 
 __global__ void __launch_bounds__((DAM_WARPS + 1) * 32, 2) decode_attention_mma(

@@ -62,22 +62,22 @@ __device__ __forceinline__ bool beyond_half4(float4 v) {
   return !(fabsf(v.x) <= 65504.0f && fabsf(v.y) <= 65504.0f && fabsf(v.z) <= 65504.0f && fabsf(v.w) <= 65504.0f);
 }
 
-// x[t][:] = embedding row of token t as fp32.  grid = T, block = 256.  `wq`: 0 fp16 rows; 1 FP8-E4M3 rows (H bytes,
+// x[t][:] = embedding row of `token` as fp32.  grid = T, block = 256.  `wq`: 0 fp16 rows; 1 FP8-E4M3 rows (H bytes,
 // then a 16-byte trailer with the fp32 row scale); 2 NVFP4 rows (H / 2 bytes of e2m1 pairs, low nibble first, H / 16
 // e4m3 block scales, then the trailer with the fp32 tensor scale).
-__device__ __forceinline__ void embed_row(const int *tokens, const void *embed, int wq, float *x, int t) {
+__device__ __forceinline__ void embed_row(int token, const void *embed, int wq, float *x, int t) {
   float *out = x + static_cast<size_t>(t) * H;
   if (wq == 0) {
-    const __half *row = static_cast<const __half *>(embed) + static_cast<size_t>(tokens[t]) * H;
+    const __half *row = static_cast<const __half *>(embed) + static_cast<size_t>(token) * H;
     for (int k = threadIdx.x; k < H; k += blockDim.x) out[k] = __half2float(row[k]);
   } else if (wq == 1) {
-    const unsigned char *row = static_cast<const unsigned char *>(embed) + static_cast<size_t>(tokens[t]) * (H + 16);
+    const unsigned char *row = static_cast<const unsigned char *>(embed) + static_cast<size_t>(token) * (H + 16);
     const float scale = *reinterpret_cast<const float *>(row + H);
     for (int k = threadIdx.x; k < H; k += blockDim.x)
       out[k] = scale * __half2float(__half(__nv_cvt_fp8_to_halfraw(row[k], __NV_E4M3)));
   } else {
     constexpr int PITCH = H / 2 + H / 16 + 16;
-    const unsigned char *row = static_cast<const unsigned char *>(embed) + static_cast<size_t>(tokens[t]) * PITCH;
+    const unsigned char *row = static_cast<const unsigned char *>(embed) + static_cast<size_t>(token) * PITCH;
     const float scale = *reinterpret_cast<const float *>(row + H / 2 + H / 16);
     for (int k = threadIdx.x; k < H; k += blockDim.x) {
       const unsigned int code = (row[k >> 1] >> ((k & 1) * 4)) & 0xFu;
@@ -91,7 +91,7 @@ __device__ __forceinline__ void embed_row(const int *tokens, const void *embed, 
 __global__ void embed_rows(const int *tokens, const void *embed, int wq, float *x) {
   pdl_wait();
   pdl_trigger();
-  embed_row(tokens, embed, wq, x, blockIdx.x);
+  embed_row(tokens[blockIdx.x], embed, wq, x, blockIdx.x);   // (prompt tokens: the host has looked at each)
 }
 
 // Residual add + RMSNorm: x[t] += add[t] (if add), y[t] = fp16(x[t] * rstd * w).  grid = T, block = 256.

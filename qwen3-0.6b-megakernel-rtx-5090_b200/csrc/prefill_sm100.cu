@@ -1238,7 +1238,8 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
     qmk_tc::PdlScope pdl_scope(env.pdl != 0);   // every launch below may start behind its predecessor's tail
     {
       qmk_tc::PdlScope first(false);            // (the first kernel of a step has no predecessor inside the step)
-      PF_CUDA(qmk_tc::launch_kernel(embed_rows_and_plan, dim3(B + 1), dim3(256), 0, s, w.tokens, embed_weight, wq, w.x, w.positions, attn_ctas, w.attn_plan));
+      PF_CUDA(qmk_tc::launch_kernel(embed_rows_and_plan, dim3(B + 1), dim3(256), 0, s, w.tokens, embed_weight, wq, env.vocab, w.x, w.positions,
+                                    attn_ctas, w.attn_plan, w.status));
     }
     for (int l = 0; l < num_layers; ++l) {
       const unsigned long long *r = rec.data() + static_cast<size_t>(l) * 12;
@@ -1366,7 +1367,9 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
   PF_CUDA(cudaMemcpyAsync(host_status, w.status, 16, cudaMemcpyDeviceToHost, stream));
   PF_CUDA(cudaStreamSynchronize(stream));
   if (host_status[0] != 0)
-    return qmk_internal::report(static_cast<int>(host_status[0]), "decode_batched: a bounded device wait ran out");
+    return qmk_internal::report(static_cast<int>(host_status[0]),
+                                host_status[0] == QMK_ERR_BAD_TOKEN ? "decode_batched: a pick outside [0, vocab) (logits without a largest value)"
+                                                                    : "decode_batched: a bounded device wait ran out");
   return QMK_OK;
 }
 

@@ -238,6 +238,34 @@ def test_attention_pieces(C, lens):
     assert float((runs[0][0][:, 0] - runs[2][0][:, 0]).abs().max()) < LOGIT_TOL
 
 
+@pytest.mark.parametrize("fmt", ["fp16", "fp8", "nvfp4"])
+@pytest.mark.parametrize("dumped", [False, True], ids=["graph", "dump"])
+def test_logits_without_a_largest_value_are_an_error(C, fmt, dumped):
+    """A sequence whose logits are all NaN has no pick; what stands in its place (2^31 - 1) is an error of the step that would read its
+    embedding row, as in the persistent kernels, through the LM head's own pick (graph) and the pick from stored logits (dump).
+    The call before and the call behind it are sound."""
+    import quantize as Q
+    vocab, n = 2048, 20
+    w = S.make_weights(seed=41, num_layers=2, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    pack = {"fp16": lambda x: x, "fp8": lambda x: Q.quantize_weights_fp8(x)[0], "nvfp4": lambda x: Q.quantize_weights_nvfp4(x)[0]}[fmt]
+    prompts = [S.make_prompt(1 + i % 4, seed=1700 + i, vocab_size=vocab) for i in range(n)]
+    eng = _engine(pack(w), n, 64, engine="gemm", prefill_mode="tensor", weight_format=fmt)
+    dump = torch.zeros(n, 3, vocab, device="cuda")
+    norm = eng._base._final_norm_weight
+    kept = norm.clone()
+    try:
+        want = eng.generate_ids(prompts, 3)
+        C.set_logits_dump(dump if dumped else None)
+        norm.fill_(float("nan"))
+        with pytest.raises(RuntimeError, match=r"outside \[0, vocab\).*status 5"):
+            eng.generate_ids(prompts, 3)
+        norm.copy_(kept)
+        assert eng.generate_ids(prompts, 3) == want
+    finally:
+        C.set_logits_dump(None)
+        C.set_weight_format("fp16")
+
+
 def test_refusals(C):
     vocab = 2048
     w = S.make_weights(seed=1, num_layers=2, vocab_size=vocab, max_seq_len=16)
