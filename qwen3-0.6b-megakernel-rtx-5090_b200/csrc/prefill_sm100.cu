@@ -17,6 +17,7 @@
 #include "prefill_kernels.cuh"
 #include "attention_tcgen05.cuh"
 #include "decode_attention_mma.cuh"
+#include "buffer_group.h"
 #include "engine_internal.h"
 #include <vector>
 
@@ -505,6 +506,7 @@ struct Workspace {                  // per device, allocated on first use, never
   CUtensorMap map_cq, map_ck, map_cv, map_cact, map_co, map_cdown;   // outputs of the pair GEMMs
   CUtensorMap map_xn2, map_attn2, map_act2;   // split activations: rows of hi and lo halves
   // batched decode: per-sequence state and the logits of one step
+  bool decode_ready = false;
   int *positions = nullptr, *start_positions = nullptr;
   cudaStream_t gstream = nullptr;        // capture needs a non-default stream
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
@@ -517,7 +519,7 @@ struct Workspace {                  // per device, allocated on first use, never
   CUtensorMap *kv_maps = nullptr;        // [128][2]: tiled-copy descriptors of every sequence's K and V cache (decode_attention_mma)
   unsigned char *packed = nullptr;       // tables of a packed prefill (row info, attention items, per-sequence descriptors and cache pointers)
   int **log_ptrs = nullptr;
-  float *split_part = nullptr;            // partial attention states of split sequences (decode_attention_ring)
+  float *split_part = nullptr;            // partial attention states of split sequences (both decode attention kernels)
   qmk_pf::DamPlan *attn_plan = nullptr;   // the step's list of attention pieces (decode_attention_mma)
   unsigned int *split_count = nullptr;    // arrival counters, one per (sequence, kv head); zero between launches
   float *logits = nullptr;
@@ -556,6 +558,8 @@ std::mutex g_ws_decode_mu;
       return qmk_internal::report(QMK_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(err__)); \
   } while (0)
 
+cudaError_t device_memory(void **at, size_t bytes) { return cudaMalloc(at, bytes); }
+
 // `rows`: activation rows the buffers hold (CHUNK for prefill, one 128-row tile for the batched decode).  All or nothing:
 // buffers that were made are given back when a later one does not fit.  `no_room`: set (and nothing reported) where the
 // reason is memory, for callers with another way.
@@ -563,8 +567,7 @@ int ensure_workspace(Workspace &w, int rows, bool *no_room = nullptr) {
   if (w.ready) return QMK_OK;
   using namespace qmk_pf;
   const size_t C = static_cast<size_t>(rows);
-  struct Buffer { void **at; size_t bytes; };
-  const Buffer buffers[] = {
+  const qmk_tc::Buffer buffers[] = {
       {reinterpret_cast<void **>(&w.tokens), sizeof(int) * C},
       {reinterpret_cast<void **>(&w.x), sizeof(float) * C * H},
       {reinterpret_cast<void **>(&w.q), sizeof(float) * C * QS},
@@ -578,11 +581,11 @@ int ensure_workspace(Workspace &w, int rows, bool *no_room = nullptr) {
       {reinterpret_cast<void **>(&w.attn), sizeof(__half) * C * 2 * QS},
       {reinterpret_cast<void **>(&w.act), sizeof(__half) * C * 2 * I},
       {reinterpret_cast<void **>(&w.status), 16}};
-  cudaError_t e = cudaSuccess;
+  cudaError_t e = qmk_tc::make_all(buffers, cudaSuccess, device_memory, cudaFree);
   // GEMM operand rows beyond a short chunk are read: zeros at first, later what earlier passes left there (any bits: a pass with
   // split activations uses the same memory in another layout).  They reach their own rows of a product only, which nobody uses.
-  for (const Buffer &b : buffers)
-    if (e == cudaSuccess && (e = cudaMalloc(b.at, b.bytes)) == cudaSuccess) e = cudaMemset(*b.at, 0, b.bytes);
+  for (const qmk_tc::Buffer &b : buffers)
+    if (e == cudaSuccess) e = cudaMemset(*b.at, 0, b.bytes);
   if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);   // (a caller's stream may not wait for the legacy one)
   std::string err;
   int rc = e == cudaSuccess ? QMK_OK : QMK_ERR_CUDA;
@@ -604,8 +607,7 @@ int ensure_workspace(Workspace &w, int rows, bool *no_room = nullptr) {
   if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_co, w.o, 2 * C, H, false, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_cdown, w.down, 2 * C, H, false, &err);
   if (rc != QMK_OK) {
-    for (const Buffer &b : buffers)
-      if (*b.at) { cudaFree(*b.at); *b.at = nullptr; }
+    qmk_tc::drop_all(buffers, cudaFree);
     cudaGetLastError();
     if (no_room && e == cudaErrorMemoryAllocation) { *no_room = true; return rc; }
     return qmk_internal::report(rc, err);
@@ -1090,20 +1092,26 @@ constexpr int MAX_ATTN_CTAS = 1024;
 static_assert(qmk_pf::dam_max_states(MAX_BATCH, MAX_ATTN_CTAS) * qmk_pf::DAM_PART <= SPLIT_PART_FLOATS &&
                   MAX_BATCH <= qmk_pf::DAM_MAX_BATCH && MAX_LAYERS <= qmk_pf::DAM_MAX_LAYERS, "partial states of decode_attention_mma");
 int ensure_decode_workspace(Workspace &w, const void *lm_head, int vocab, int wq) {
-  if (!w.positions) {
-    PF_CUDA(cudaMalloc(&w.positions, sizeof(int) * MAX_BATCH));
-    PF_CUDA(cudaMalloc(&w.start_positions, sizeof(int) * MAX_BATCH));
-    PF_CUDA(cudaStreamCreateWithFlags(&w.gstream, cudaStreamNonBlocking));
-    PF_CUDA(cudaEventCreateWithFlags(&w.ev_in, cudaEventDisableTiming));
-    PF_CUDA(cudaEventCreateWithFlags(&w.ev_out, cudaEventDisableTiming));
-    PF_CUDA(cudaMalloc(&w.k_ptrs, sizeof(void *) * MAX_BATCH));
-    PF_CUDA(cudaMalloc(&w.v_ptrs, sizeof(void *) * MAX_BATCH));
-    PF_CUDA(cudaMalloc(&w.log_ptrs, sizeof(void *) * MAX_BATCH));
-    PF_CUDA(cudaMalloc(&w.kv_maps, sizeof(CUtensorMap) * 2 * MAX_BATCH));
-    PF_CUDA(cudaMalloc(&w.split_part, sizeof(float) * SPLIT_PART_FLOATS));
-    PF_CUDA(cudaMalloc(&w.attn_plan, sizeof(qmk_pf::DamPlan) + sizeof(qmk_pf::DamPiece) * qmk_pf::dam_max_pieces(MAX_BATCH, MAX_ATTN_CTAS)));
-    PF_CUDA(cudaMalloc(&w.split_count, sizeof(unsigned int) * MAX_BATCH * qmk_pf::NKV));
-    PF_CUDA(cudaMemset(w.split_count, 0, sizeof(unsigned int) * MAX_BATCH * qmk_pf::NKV));
+  if (!w.decode_ready) {
+    const qmk_tc::Buffer buffers[] = {
+        {reinterpret_cast<void **>(&w.positions), sizeof(int) * MAX_BATCH},
+        {reinterpret_cast<void **>(&w.start_positions), sizeof(int) * MAX_BATCH},
+        {reinterpret_cast<void **>(&w.k_ptrs), sizeof(void *) * MAX_BATCH},
+        {reinterpret_cast<void **>(&w.v_ptrs), sizeof(void *) * MAX_BATCH},
+        {reinterpret_cast<void **>(&w.log_ptrs), sizeof(void *) * MAX_BATCH},
+        {reinterpret_cast<void **>(&w.kv_maps), sizeof(CUtensorMap) * 2 * MAX_BATCH},
+        {reinterpret_cast<void **>(&w.split_part), sizeof(float) * SPLIT_PART_FLOATS},
+        {reinterpret_cast<void **>(&w.attn_plan), sizeof(qmk_pf::DamPlan) + sizeof(qmk_pf::DamPiece) * qmk_pf::dam_max_pieces(MAX_BATCH, MAX_ATTN_CTAS)},
+        {reinterpret_cast<void **>(&w.split_count), sizeof(unsigned int) * MAX_BATCH * qmk_pf::NKV}};
+    if (!w.gstream) PF_CUDA(cudaStreamCreateWithFlags(&w.gstream, cudaStreamNonBlocking));
+    if (!w.ev_in) PF_CUDA(cudaEventCreateWithFlags(&w.ev_in, cudaEventDisableTiming));
+    if (!w.ev_out) PF_CUDA(cudaEventCreateWithFlags(&w.ev_out, cudaEventDisableTiming));
+    const cudaError_t e = qmk_tc::make_all(buffers, cudaSuccess, device_memory, cudaFree);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return qmk_internal::report(QMK_ERR_CUDA, std::string("workspace of the batched decode: ") + cudaGetErrorString(e));
+    }
+    w.decode_ready = true;
   }
   if (w.logits_vocab < vocab) {
     if (w.logits) cudaFree(w.logits);

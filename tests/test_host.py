@@ -124,3 +124,55 @@ def test_engine_choice_for_four_sequences():
     assert auto(4, "fp16", 151936, 8320, 148, room) == "gemm" and auto(4, "fp8", 151936, 8320, 148, room) == "persistent"
     assert auto(4, "fp8", 151936, 2048, 200, room) == "gemm" and auto(4, "fp16", 151936, 2048, 200, room) == "persistent"
     assert [auto(n, "nvfp4", 151936, 2048, 148, room) for n in (1, 4, 9)] == ["gemm"] * 3
+
+
+BUFFER_GROUP = r"""
+#include "buffer_group.h"
+#include <cstdio>
+#include <cstdlib>
+#include <set>
+int main() {
+  // five buffers; call 0 .. 4 of the allocator is the one that is refused (5: none)
+  for (int refused = 0; refused <= 5; ++refused) {
+    void *p[5] = {};
+    const qmk_tc::Buffer group[] = {{&p[0], 8}, {&p[1], 16}, {&p[2], 24}, {&p[3], 32}, {&p[4], 40}};
+    std::set<void *> live;
+    int calls = 0;
+    auto make = [&](void **at, std::size_t bytes) {
+      if (calls++ == refused) { *at = &calls; return 2; }        // (an allocator may leave anything behind)
+      if (bytes != 8u * static_cast<unsigned>(calls)) std::exit(10);
+      live.insert(*at = std::malloc(bytes));
+      return 0;
+    };
+    auto drop = [&](void *q) { if (live.erase(q) != 1) std::exit(11); std::free(q); };
+    const int first = qmk_tc::make_all(group, 0, make, drop);
+    if (first != (refused < 5 ? 2 : 0)) return 12;
+    for (void *q : p)
+      if ((q != nullptr) != (refused == 5)) return 13;           // all or none
+    if (live.size() != (refused == 5 ? 5u : 0u)) return 14;
+    if (refused == 5) continue;
+    calls = 0;
+    refused = refused + 100;                                     // there is room again
+    if (qmk_tc::make_all(group, 0, make, drop) != 0 || live.size() != 5) return 15;
+    refused -= 100;
+    qmk_tc::drop_all(group, drop);
+    if (!live.empty()) return 16;
+  }
+  return 0;
+}
+"""
+
+
+def test_workspace_buffers_come_all_or_none(tmp_path):
+    """The workspaces of the tensor-core paths are groups of buffers.  Whichever of them is refused, none is left: a later call
+    finds no part of a group that it would take for the whole, and makes it once there is room."""
+    import subprocess
+    src = tmp_path / "group.cpp"
+    src.write_text(BUFFER_GROUP)
+    csrc = os.path.join(ROOT, "qwen3-0.6b-megakernel-rtx-5090_b200", "csrc")
+    subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-I", csrc, "-o", str(tmp_path / "group"), str(src)], check=True)
+    assert subprocess.run([str(tmp_path / "group")]).returncode == 0
+    # and no buffer of the batched decode is made beside the group
+    code = open(os.path.join(csrc, "prefill_sm100.cu")).read()
+    body = code[code.index("int ensure_decode_workspace("):code.index("if (w.logits_vocab < vocab)")]
+    assert "make_all" in body and "cudaMalloc" not in body
