@@ -659,6 +659,7 @@ int ensure_weight_maps(Workspace &w, const LDGLayerWeight *layers_dev, int num_l
   // record order: in_ln, wq, wk, wv, q_norm, k_norm, wo, post_ln, gate, up, down, pad
   static const int slot[7] = {1, 2, 3, 6, 8, 9, 10};
   std::string err;
+  w.table_layers = 0;   // (until all maps are made: a table that is refused below has replaced some)
   for (int l = 0; l < num_layers; ++l)
     for (int j = 0; j < 7; ++j) {
       const void *ptr = reinterpret_cast<const void *>(host[static_cast<size_t>(l) * 12 + slot[j]]);

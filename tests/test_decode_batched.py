@@ -266,6 +266,30 @@ def test_logits_without_a_largest_value_are_an_error(C, fmt, dumped):
         C.set_weight_format("fp16")
 
 
+def test_a_refused_layer_table_changes_no_later_call(C):
+    """Layer tables are read back and their matrices' tensor maps kept until another table comes.  A table that is refused half-way
+    (its second layer has a null pointer) has replaced the maps of its first: a call on the table before it makes them anew."""
+    vocab, n = 2048, 6
+    engines = [_engine(S.make_weights(seed=seed, num_layers=2, vocab_size=vocab, norm_std=0.1, max_seq_len=16), n, 64, engine="gemm",
+                       prefill_mode="tensor") for seed in (51, 52)]
+    prompts = [S.make_prompt(2 + i, seed=1800 + i, vocab_size=vocab) for i in range(n)]
+    want = engines[0].generate_ids(prompts, 3)
+    rows = [k.clone() for k in engines[0]._k_caches[:n]]
+    base = engines[1]._base
+    table = base._layer_weights_packed.clone()
+    table.view(torch.int64)[12 + 6] = 0
+    common = (base._cos_table, base._sin_table)
+    with pytest.raises(RuntimeError, match="null weight pointer"):
+        C.decode_batched([1], [0], 1, base._embed_weight, table, base._final_norm_weight, base._lm_head_weight, *common,
+                         engines[1]._k_caches[:1], engines[1]._v_caches[:1], [torch.zeros(1, dtype=torch.int32, device="cuda")],
+                         base.num_layers, 64, base._attn_scale)
+    with pytest.raises(RuntimeError, match="null weight pointer"):
+        C.prefill_chunked(torch.tensor([1, 2], dtype=torch.int32), base._embed_weight, table, *common, engines[1]._k_caches[0],
+                          engines[1]._v_caches[0], base.num_layers, 0, 64, base._attn_scale)
+    assert engines[0].generate_ids(prompts, 3) == want
+    assert all(torch.equal(a, b) for a, b in zip(rows, engines[0]._k_caches))
+
+
 def test_refusals(C):
     vocab = 2048
     w = S.make_weights(seed=1, num_layers=2, vocab_size=vocab, max_seq_len=16)
