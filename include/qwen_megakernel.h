@@ -411,6 +411,9 @@ int qmk_selftest_wait_timeout(int budget_us);
 int qmk_selftest_gemm_wait_timeout(int budget_us);
 /* The same for the tcgen05 attention of a prefill: score products that stop behind the first, keys and values in flight. */
 int qmk_selftest_attention_wait_timeout(int budget_us);
+/* The same for the attention of a step of qmk_decode_batched.  what = 1: nothing is loaded; 2: one chunk of cache rows never comes while
+ * others are in flight. */
+int qmk_selftest_decode_attention_wait_timeout(int budget_us, int what);
 
 /* The same for the pairs of CTAs that multiply more than 512 rows.  what = 1: no loads; 2: the issuing thread gives up behind its
  * first tile, with a ring of copies in flight; 3: the second CTA of the pair loads nothing. */

@@ -34,8 +34,12 @@ namespace qmk_pf {
 // in device memory, and a warp handles it with 16 mma.sync.m16n8k16: scores = K[16 x 128] . q[128 x 4] (columns: head 0
 // hi / lo, head 1 hi / lo of the fp32 query split into two fp16 numbers), online softmax on the accumulator fragments
 // (log2 domain), then out[128 x 4] += V^T[128 x 16] . p[16 x 4] with V read through ldmatrix.trans and p split like q -
-// about 75 instructions per 16 rows.  Waits are bounded: on a time-out the CTA sets *status = 4, goes through the rest
-// of its items without waiting and leaves after its copies have landed.
+// about 75 instructions per 16 rows.
+//
+// Waits are bounded.  On a time-out the CTA sets *status = 4, which the call returns: what it has written is then not valid.  It goes
+// on through the pieces at hand without waiting and leaves at the first one it is not handed; pieces that it had taken from the list stay
+// undone and their items' counters behind (the next call clears them).  A slot whose copy was given up is not loaded again, and the
+// CTA stays until its copies have landed (whoever gives up waits for them, and the producer if it is still there).
 constexpr int DAM_WARPS = 8, DAM_SLOTS = 9, DAM_ROWS = 16;
 constexpr int DAM_BOX = DAM_ROWS * 128;                // one box: 16 rows x 64 dims
 constexpr int DAM_SLOT_BYTES = 4 * DAM_BOX;            // 8 KB: K dims 0..63, K dims 64..127, V dims 0..63, V dims 64..127
@@ -181,6 +185,9 @@ __global__ void __launch_bounds__(256) embed_rows_and_plan(const int *tokens, co
   embed_row(token, embed, wq, x, blockIdx.x);
 }
 
+// TEST (bounded waits only): 1: nothing is loaded or announced; 2: the third chunk's copies are not issued, those around it are.
+enum { DAM_NO_LOADS = 1, DAM_LOST_COPY = 2 };
+template <int TEST = 0>
 __global__ void __launch_bounds__((DAM_WARPS + 1) * 32, 2) decode_attention_mma(
     const float *q, const float *k, const float *v, const __half *q_norm, const __half *k_norm, const float *rope,
     const __half *cos_table, const __half *sin_table, __half *const *k_ptrs, __half *const *v_ptrs, size_t layer_off,
@@ -262,6 +269,17 @@ __global__ void __launch_bounds__((DAM_WARPS + 1) * 32, 2) decode_attention_mma(
     }
     return true;
   };
+  // after a time-out: the copies of the `issued` chunks must land before the CTA may exit
+  auto drain = [&](int issued) {
+    for (int c = (issued > DAM_SLOTS ? issued - DAM_SLOTS : 0); c < issued; ++c) {
+      unsigned long long t0, t;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+      while (!try_wait(full + c % DAM_SLOTS, (c / DAM_SLOTS) & 1)) {
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        if (t - t0 > (budget_ns > 2000000ull ? budget_ns : 2000000ull)) break;
+      }
+    }
+  };
   if (warp == DAM_WARPS) {            // ---- producer: takes pieces, streams their old rows in chunks of 16
     if (qmk_gemm::elect_one()) {      // (a thread picked by `lane == 0` takes 500 cycles to issue a chunk's copies: 8 sequences 653 -> 676 us a step)
       int issued = 0, slot = 0, mapped = -1;
@@ -281,13 +299,13 @@ __global__ void __launch_bounds__((DAM_WARPS + 1) * 32, 2) decode_attention_mma(
         const int row0 = layer * NKV * max_seq_len + (p1.x & 255) * max_seq_len + p0.z * DAM_ROWS;   // in the sequence's [layer][head][pos] cache
         const int chains = DAM_CHAINS / (p1.w >> 8), chain0 = p1.z * chains;
         for (int c = 0; c < p0.w; ++c) {
-          if (static_cast<unsigned int>((c & (DAM_CHAINS - 1)) - chain0) >= static_cast<unsigned int>(chains)) continue;
+          if (static_cast<unsigned int>((c & (DAM_CHAINS - 1)) - chain0) >= static_cast<unsigned int>(chains) || TEST == DAM_NO_LOADS) continue;
           const int row = row0 + c * DAM_ROWS;
           if (issued >= DAM_SLOTS && !wait(empty + slot, parity)) { ok = false; break; }
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(s32(full + slot)), "r"(DAM_SLOT_BYTES) : "memory");
           const uint32_t dst = s32(dam_smem + slot * DAM_SLOT_BYTES);
 #pragma unroll
-          for (int sub = 0; sub < 4; ++sub)
+          for (int sub = TEST == DAM_LOST_COPY && issued == 2 ? 4 : 0; sub < 4; ++sub)
             asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                          ::"r"(dst + sub * DAM_BOX), "l"(sub < 2 ? kmap : vmap), "r"((sub & 1) * 64), "r"(row), "r"(s32(full + slot))
                          : "memory");
@@ -310,15 +328,9 @@ __global__ void __launch_bounds__((DAM_WARPS + 1) * 32, 2) decode_attention_mma(
         __threadfence_block();
         s_taken = taken + 1;
       }
-      if (*abort_flag)   // copies already issued must land before the CTA may exit
-        for (int c = (issued > DAM_SLOTS ? issued - DAM_SLOTS : 0); c < issued; ++c) {
-          unsigned long long t0, t;
-          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-          while (!try_wait(full + c % DAM_SLOTS, (c / DAM_SLOTS) & 1)) {
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            if (t - t0 > (budget_ns > 2000000ull ? budget_ns : 2000000ull)) break;
-          }
-        }
+      // (either this look finds the flag, or whoever sets it later finds the last chunk announced)
+      __threadfence_block();
+      if (*abort_flag) drain(issued);
     }
     return;
   }
@@ -516,8 +528,8 @@ __global__ void __launch_bounds__((DAM_WARPS + 1) * 32, 2) decode_attention_mma(
         }
       }
       __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s32(empty + slot)) : "memory");
       if (!ok) break;
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s32(empty + slot)) : "memory");
     }
     ring += (nchunks >> 3) * chains + min(max((nchunks & (DAM_CHAINS - 1)) - chain0, 0), chains);
     fetched = s_taken > j + 1;
@@ -625,6 +637,10 @@ __global__ void __launch_bounds__((DAM_WARPS + 1) * 32, 2) decode_attention_mma(
     if (threadIdx.x == 0) split_count[b * NKV + g] = 0u;   // ready for the next launch (stream order)
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
+  if (*abort_flag) {
+    __threadfence_block();
+    drain(*issued_ctr);
+  }
 }
 
 }  // namespace qmk_pf

@@ -258,7 +258,7 @@ int ensure_gemm_attrs(std::string *err) {
       e = cudaFuncSetAttribute(qmk_pf::decode_attention_ring, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                qmk_pf::DAR_SMEM_BYTES);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(qmk_pf::decode_attention_mma, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      e = cudaFuncSetAttribute(qmk_pf::decode_attention_mma<>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                qmk_pf::DAM_SMEM_BYTES);
     if (e != cudaSuccess) { *err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e); return QMK_ERR_CUDA; }
     g_attr_set[dev] = true;
@@ -1279,7 +1279,7 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
           return r2;
       }
       if (env.attn_mma)
-        PF_CUDA(qmk_tc::launch_kernel(decode_attention_mma, dim3(attn_ctas), dim3((DAM_WARPS + 1) * 32), DAM_SMEM_BYTES, s,
+        PF_CUDA(qmk_tc::launch_kernel(decode_attention_mma<>, dim3(attn_ctas), dim3((DAM_WARPS + 1) * 32), DAM_SMEM_BYTES, s,
                                       w.q, w.k, w.v, reinterpret_cast<const __half *>(r[4]), reinterpret_cast<const __half *>(r[5]),
                                       rope, cosv, sinv, w.k_ptrs, w.v_ptrs, layer_off, w.attn_plan, l, w.attn, max_seq_len, attn_scale,
                                       w.status, static_cast<unsigned long long>(env.timeout_ms) * 1000000ull, w.split_part,
@@ -1454,6 +1454,60 @@ extern "C" int qmk_selftest_attention_wait_timeout(int budget_us) {
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpy(host, status, 16, cudaMemcpyDeviceToHost);
     rc = static_cast<int>(host[0]);
+  }
+  if (e != cudaSuccess) { rc = QMK_ERR_CUDA; err = std::string("attention self test: ") + cudaGetErrorString(e); }
+  cudaFree(buf);
+  if (rc != QMK_OK && rc != QMK_ERR_WAIT_TIMEOUT) return qmk_internal::report(rc, err);
+  return rc;
+}
+
+// The same of a decode step's attention: one CTA, one sequence at position 900, the chains of each kv head in two pieces (16 pieces, more
+// than the producer may be ahead).  what = 1: nothing is loaded, so that consumers wait for chunks, then for pieces, and the
+// producer for finished ones; 2: one chunk's copies are missing among a ring of others in flight.
+extern "C" int qmk_selftest_decode_attention_wait_timeout(int budget_us, int what) {
+  using namespace qmk_pf;
+  std::string err;
+  if (budget_us < 1 || budget_us > 1000000 || what < DAM_NO_LOADS || what > DAM_LOST_COPY)
+    return qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "budget_us must be in [1, 1e6], what in [1, 2]");
+  constexpr int ROWS = 1024, POS = 900, CHUNKS = (POS + DAM_ROWS - 1) / DAM_ROWS, PARTS = 2, PIECES = NKV * PARTS;
+  constexpr size_t kv_bytes = sizeof(__half) * NKV * ROWS * D, plan_bytes = sizeof(DamPlan) + sizeof(DamPiece) * PIECES;
+  constexpr size_t at_v = kv_bytes, at_q = 2 * kv_bytes, at_new = at_q + sizeof(float) * QS, at_norm = at_new + 2 * sizeof(float) * KVS,
+                   at_rope = at_norm + sizeof(__half) * D, at_out = at_rope + sizeof(float) * ROWS * D, at_maps = at_out + sizeof(__half) * QS,
+                   at_plan = at_maps + 2 * sizeof(CUtensorMap), at_part = at_plan + (plan_bytes + 127) / 128 * 128,
+                   at_count = at_part + sizeof(float) * NKV * DAM_CHAINS * DAM_PART, at_ptrs = at_count + sizeof(unsigned int) * NKV,
+                   at_status = at_ptrs + 2 * sizeof(void *), total = at_status + 16;
+  static_assert(at_maps % 128 == 0 && at_plan % 128 == 0 && at_ptrs % 8 == 0, "alignment of the self test's buffers");
+  unsigned char *buf = nullptr;
+  PF_CUDA(cudaMalloc(&buf, total));
+  cudaError_t e = cudaMemset(buf, 0, total);
+  CUtensorMap maps[2];
+  int rc = qmk_tc::make_map_f16(&maps[0], buf, NKV * ROWS, D, DAM_ROWS, &err);
+  if (rc == QMK_OK) rc = qmk_tc::make_map_f16(&maps[1], buf + at_v, NKV * ROWS, D, DAM_ROWS, &err);
+  std::vector<unsigned char> plan_bytes_host(plan_bytes, 0);
+  DamPlan *const plan = reinterpret_cast<DamPlan *>(plan_bytes_host.data());
+  plan->total = PIECES;
+  for (int i = 0; i < PIECES; ++i) plan->pieces[i] = {0, POS, 0, CHUNKS, i / PARTS, 0, i % PARTS, 1 | (PARTS << 8)};
+  const void *const ptrs[2] = {buf, buf + at_v};
+  if (rc == QMK_OK && e == cudaSuccess) {
+    e = cudaMemcpy(buf + at_maps, maps, sizeof(maps), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(buf + at_plan, plan, plan_bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(buf + at_ptrs, ptrs, sizeof(ptrs), cudaMemcpyHostToDevice);
+    auto *const kernel = what == DAM_NO_LOADS ? decode_attention_mma<DAM_NO_LOADS> : decode_attention_mma<DAM_LOST_COPY>;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DAM_SMEM_BYTES);
+    unsigned int host[4] = {0, 0, 0, 0};
+    if (e == cudaSuccess) {
+      const __half *const norm = reinterpret_cast<const __half *>(buf + at_norm);
+      const float *const q = reinterpret_cast<const float *>(buf + at_q), *const fresh = reinterpret_cast<const float *>(buf + at_new);
+      __half *const *const caches = reinterpret_cast<__half *const *>(buf + at_ptrs);
+      kernel<<<dim3(1), (DAM_WARPS + 1) * 32, DAM_SMEM_BYTES>>>(
+          q, fresh, fresh + KVS, norm, norm, reinterpret_cast<const float *>(buf + at_rope), nullptr, nullptr, caches, caches + 1, 0,
+          reinterpret_cast<DamPlan *>(buf + at_plan), 0, reinterpret_cast<__half *>(buf + at_out), ROWS, 1.0f,
+          reinterpret_cast<unsigned int *>(buf + at_status), static_cast<unsigned long long>(budget_us) * 1000ull,
+          reinterpret_cast<float *>(buf + at_part), reinterpret_cast<unsigned int *>(buf + at_count), reinterpret_cast<const CUtensorMap *>(buf + at_maps));
+      e = cudaGetLastError();
+      if (e == cudaSuccess) e = cudaMemcpy(host, buf + at_status, 16, cudaMemcpyDeviceToHost);
+      rc = static_cast<int>(host[0]);
+    }
   }
   if (e != cudaSuccess) { rc = QMK_ERR_CUDA; err = std::string("attention self test: ") + cudaGetErrorString(e); }
   cudaFree(buf);

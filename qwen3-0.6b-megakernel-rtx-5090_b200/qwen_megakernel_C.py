@@ -116,6 +116,8 @@ _lib.qmk_selftest_gemm_wait_timeout.argtypes = [_I]
 _lib.qmk_selftest_gemm_wait_timeout.restype = _I
 _lib.qmk_selftest_attention_wait_timeout.argtypes = [_I]
 _lib.qmk_selftest_attention_wait_timeout.restype = _I
+_lib.qmk_selftest_decode_attention_wait_timeout.argtypes = [_I, _I]
+_lib.qmk_selftest_decode_attention_wait_timeout.restype = _I
 _lib.qmk_selftest_gemm_pair_wait_timeout.argtypes = [_I, _I]
 _lib.qmk_selftest_gemm_pair_wait_timeout.restype = _I
 
@@ -123,7 +125,7 @@ EXPORTED_SYMBOLS = (
     "launch_ldg_decode_direct", "launch_ldg_decode_persistent", "launch_ldg_generate_nosync",
     "launch_ldg_prefill", "qmk_abi_version", "qmk_configure", "qmk_set_inv_freq", "qmk_set_logits_dump",
     "qmk_set_weight_format", "qmk_set_tuning", "qmk_set_tuning2", "qmk_set_profile_buffer", "qmk_set_fused", "qmk_set_step_overlap", "qmk_set_prefill_attention", "qmk_set_decode_attention", "qmk_invalidate_weights", "qmk_release_weights", "qmk_decode", "qmk_generate", "qmk_generate_static", "qmk_generate_batch", "qmk_gemm_f16_tn", "qmk_gemm_packed_tn", "qmk_decode_batched", "qmk_prefill_chunked", "qmk_prefill_packed", "qmk_prefill", "qmk_engine_create", "qmk_engine_destroy", "qmk_engine_apply", "qmk_engine_decode", "qmk_engine_generate", "qmk_engine_prefill", "qmk_sync_status", "qmk_last_error", "qmk_num_ctas",
-    "qmk_scratch_bytes", "qmk_selftest_wait_timeout", "qmk_selftest_gemm_wait_timeout", "qmk_selftest_attention_wait_timeout", "qmk_selftest_gemm_pair_wait_timeout",
+    "qmk_scratch_bytes", "qmk_selftest_wait_timeout", "qmk_selftest_gemm_wait_timeout", "qmk_selftest_attention_wait_timeout", "qmk_selftest_gemm_pair_wait_timeout", "qmk_selftest_decode_attention_wait_timeout",
 )
 
 
@@ -610,6 +612,12 @@ def selftest_attention_wait_timeout(budget_us: int = 300) -> int:
     """The same for the tcgen05 attention of a prefill."""
     _require_cuda()
     return int(_lib.qmk_selftest_attention_wait_timeout(int(budget_us)))
+
+
+def selftest_decode_attention_wait_timeout(budget_us: int = 300, what: int = 1) -> int:
+    """The bounded waits of a decode step's attention: nothing loaded (1), or one chunk of cache rows that never comes (2); 4 is the
+    designed answer."""
+    return int(_lib.qmk_selftest_decode_attention_wait_timeout(int(budget_us), int(what)))
 
 
 def selftest_gemm_pair_wait_timeout(budget_us: int = 300, what: int = 1) -> int:

@@ -290,6 +290,22 @@ def test_a_refused_layer_table_changes_no_later_call(C):
     assert all(torch.equal(a, b) for a, b in zip(rows, engines[0]._k_caches))
 
 
+@pytest.mark.parametrize("what", [1, 2])
+def test_attention_waits_run_out_and_leave_the_device_usable(C, what):
+    """Cache rows that never come: all of them (every wait of consumers and producer runs out), or one chunk among others in flight.
+    Status 4 after the budget, and steps behind it are as before: nothing lands in their shared memory."""
+    vocab, n, L = 2048, 37, 768
+    w = S.make_weights(seed=43, num_layers=2, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    prompts = [S.make_prompt(1 + (131 * i) % 700, seed=1900 + i, vocab_size=vocab) for i in range(n)]
+    eng = _engine(w, n, L, engine="gemm", prefill_mode="tensor")
+    want = eng.generate_ids(prompts, 3)
+    rows = [k.clone() for k in eng._k_caches]
+    for _ in range(3):
+        assert C.selftest_decode_attention_wait_timeout(300, what) == 4
+        assert eng.generate_ids(prompts, 3) == want
+        assert all(torch.equal(a, b) for a, b in zip(rows, eng._k_caches))
+
+
 def test_refusals(C):
     vocab = 2048
     w = S.make_weights(seed=1, num_layers=2, vocab_size=vocab, max_seq_len=16)
