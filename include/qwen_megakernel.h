@@ -397,7 +397,9 @@ int qmk_gemm_packed_tn(const void *a, const void *b, const void *b2, void *c, in
 /* Synchronises the device and returns the status word of the last launch
  * (QMK_OK, or the first error a CTA recorded). */
 int qmk_sync_status(void);
-/* Text of the last error on this thread's device ("" if none). */
+/* Why the calling thread's last call failed ("" if it did not): calls of other threads in between neither clear this text nor put
+ * theirs in its place.  Every function that returns a status counts as a call, qmk_engine_destroy excepted.  On a thread that has made
+ * none: the last error on its device.  The pointer is good until the thread asks again. */
 const char *qmk_last_error(void);
 /* Persistent grid size (CTAs) and bytes of library-owned device scratch. */
 int qmk_num_ctas(void);

@@ -20,7 +20,11 @@ struct PrefillEnv {
 };
 // Engine of the current device, created on first use; clears its last error.
 int prefill_env(int max_seq_len, cudaStream_t stream, PrefillEnv *out);
-// Records an error on the current device's engine (qmk_last_error) and returns `code`.
+// Start of an entry point that returns a status: from here on qmk_last_error on this thread speaks of this call.
+void begin_call();
+// Text for qmk_last_error on this thread, and nothing else.
+void note_error(const std::string &msg);
+// Records an error on the current device's engine (qmk_last_error, qmk_sync_status) and returns `code`.
 int report(int code, const std::string &msg);
 }  // namespace qmk_internal
 

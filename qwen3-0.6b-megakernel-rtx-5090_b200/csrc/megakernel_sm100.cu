@@ -279,13 +279,23 @@ Engine *current_engine_unlocked() {
   return e;
 }
 
-thread_local std::string t_error;   // of the calling thread's last call, if that failed: another thread's call may clear the engine's
+// Of the calling thread's last call, if that failed.  What other threads do in between changes the engine's text, not this one; every
+// entry point that returns a status begins with begin_call().
+thread_local std::string t_error;
+thread_local bool t_called = false;
 
 void clear_error(Engine *e) {
   e->last_status = QMK_OK;
   e->last_error.clear();
   t_error.clear();
 }
+
+// A refusal that is no error of a device's engine.
+int refuse(int code, const char *msg) {
+  t_error = msg;
+  return code;
+}
+int no_device() { return refuse(QMK_ERR_CUDA, "no CUDA device"); }
 
 int fail(Engine *e, int code, const std::string &msg) {
   t_error = msg;
@@ -642,7 +652,7 @@ namespace qmk_internal {
 int prefill_env(int max_seq_len, cudaStream_t stream, PrefillEnv *out) {
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   clear_error(e);
   int rc = ensure_ready(e);
   if (rc == QMK_OK) rc = ensure_rope(e, max_seq_len, stream);
@@ -658,6 +668,11 @@ int prefill_env(int max_seq_len, cudaStream_t stream, PrefillEnv *out) {
   out->attn_mma = e->decode_attn_mma;
   return QMK_OK;
 }
+void begin_call() {
+  t_error.clear();
+  t_called = true;
+}
+void note_error(const std::string &msg) { t_error = msg; }
 int report(int code, const std::string &msg) {
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   return fail(current_engine_unlocked(), code, msg);
@@ -669,9 +684,10 @@ extern "C" {
 int qmk_abi_version(void) { return 2; }
 
 int qmk_configure(int vocab_size, int rope_from_table, int split_len, int max_ctas, int timeout_ms) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   if (vocab_size == 0 || split_len == 0 || timeout_ms == 0) return fail(e, QMK_ERR_BAD_ARGUMENT, "zero option value");
   if (vocab_size > 0) e->vocab = vocab_size;
   if (rope_from_table >= 0) e->rope_from_table = rope_from_table ? 1 : 0;
@@ -683,9 +699,10 @@ int qmk_configure(int vocab_size, int rope_from_table, int split_len, int max_ct
 }
 
 int qmk_set_inv_freq(const float *inv_freq64) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e || !inv_freq64) return QMK_ERR_BAD_ARGUMENT;
+  if (!e || !inv_freq64) return refuse(QMK_ERR_BAD_ARGUMENT, e ? "inv_freq64 is null" : "no CUDA device");
   // callers re-apply their options before every op: the same frequencies again cost nothing
   if (e->inv_freq_set && memcmp(e->inv_freq, inv_freq64, sizeof(e->inv_freq)) == 0) return QMK_OK;
   QMK_CUDA(e, cudaDeviceSynchronize());   // no launch may still be reading the old table
@@ -697,17 +714,19 @@ int qmk_set_inv_freq(const float *inv_freq64) {
 }
 
 int qmk_set_logits_dump(float *logits_out) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   e->logits_out = logits_out;
   return QMK_OK;
 }
 
 int qmk_set_weight_format(int format) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   if (format < 0 || format > 2)
     return fail(e, QMK_ERR_BAD_ARGUMENT, "weight format must be 0 (fp16), 1 (fp8-e4m3 rows) or 2 (nvfp4 rows)");
   e->wfmt = format;
@@ -715,33 +734,37 @@ int qmk_set_weight_format(int format) {
 }
 
 int qmk_set_prefill_attention(int tensor_core) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   if (tensor_core >= 0) e->prefill_attn_tc = tensor_core ? 1 : 0;
   return QMK_OK;
 }
 
 int qmk_set_decode_attention(int tensor_core) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   if (tensor_core >= 0) e->decode_attn_mma = tensor_core ? 1 : 0;
   return QMK_OK;
 }
 
 int qmk_set_step_overlap(int enabled) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   if (enabled >= 0) e->step_overlap = enabled ? 1 : 0;
   return QMK_OK;
 }
 
 int qmk_set_tuning2(int repl, int stream_inflight) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   if (repl == 1 || repl == 2 || repl == 4) e->repl = repl;
   else if (repl >= 0) return fail(e, QMK_ERR_BAD_ARGUMENT, "repl must be 1, 2 or 4");
   if (stream_inflight >= 0) e->stream_inflight = stream_inflight > qmk::NSLOTS ? qmk::NSLOTS : stream_inflight;
@@ -749,18 +772,20 @@ int qmk_set_tuning2(int repl, int stream_inflight) {
 }
 
 int qmk_set_tuning(int spin_sleep_ns, int l2_evict_first) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   if (spin_sleep_ns >= 0) e->spin_sleep_ns = e->fused_sleep_ns = spin_sleep_ns > 10000 ? 10000 : spin_sleep_ns;
   if (l2_evict_first >= 0) e->l2_evict_first = l2_evict_first ? 1 : 0;
   return QMK_OK;
 }
 
 int qmk_set_fused(int fused, int red_copies) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   if (fused > 2) return fail(e, QMK_ERR_BAD_ARGUMENT, "fused must be 0, 1 or 2");
   if (fused >= 0) e->fused = fused;
   if (red_copies == 1 || red_copies == 2) e->red_copies = red_copies;
@@ -769,17 +794,19 @@ int qmk_set_fused(int fused, int red_copies) {
 }
 
 int qmk_invalidate_weights(void) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   for (auto &p : e->prepared) p.force = 1;
   return QMK_OK;
 }
 
 int qmk_release_weights(const LDGLayerWeight *layer_weights) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   for (size_t i = 0; i < e->prepared.size();) {
     if (layer_weights == nullptr || e->prepared[i].table == layer_weights) {
       QMK_CUDA(e, cudaDeviceSynchronize());
@@ -793,9 +820,10 @@ int qmk_release_weights(const LDGLayerWeight *layer_weights) {
 }
 
 int qmk_set_profile_buffer(unsigned long long *timestamps) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   e->prof = timestamps;
   return QMK_OK;
 }
@@ -809,7 +837,7 @@ int decode_unlocked(int input_token_id, int *output_token_id, const void *embed_
                     void *block_max_idxs, int num_layers, int position, int max_seq_len, float attn_scale,
                     cudaStream_t stream) {
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   clear_error(e);
   Params P = base_params(embed_weight, layer_weights, final_norm_weight, lm_head_weight, cos_table, sin_table, k_cache,
                          v_cache, num_layers, position, max_seq_len, attn_scale);
@@ -829,7 +857,7 @@ int generate_unlocked(int first_token_id, int num_steps, const void *embed_weigh
                       void *block_max_vals, void *block_max_idxs, int *output_log, int num_layers, int start_position,
                       int max_seq_len, float attn_scale, int eos_token_id, int synchronize, cudaStream_t stream) {
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   clear_error(e);
   if (num_steps > 0 && !output_log) return fail(e, QMK_ERR_BAD_ARGUMENT, "output_log is null");
   Params P = base_params(embed_weight, layer_weights, final_norm_weight, lm_head_weight, cos_table, sin_table, k_cache,
@@ -853,6 +881,7 @@ int qmk_decode(int input_token_id, int *output_token_id, const void *embed_weigh
                void *k_cache, void *v_cache, void *hidden_buffer, void *g_normalized, void *block_max_vals,
                void *block_max_idxs, int num_layers, int position, int max_seq_len, float attn_scale,
                cudaStream_t stream) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   return decode_unlocked(input_token_id, output_token_id, embed_weight, layer_weights, final_norm_weight, lm_head_weight,
                          cos_table, sin_table, k_cache, v_cache, hidden_buffer, g_normalized, block_max_vals, block_max_idxs,
@@ -864,6 +893,7 @@ int qmk_generate(int first_token_id, int num_steps, const void *embed_weight, co
                  const void *sin_table, void *k_cache, void *v_cache, void *hidden_buffer, void *g_normalized,
                  void *block_max_vals, void *block_max_idxs, int *output_log, int num_layers, int start_position,
                  int max_seq_len, float attn_scale, int eos_token_id, int synchronize, cudaStream_t stream) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   return generate_unlocked(first_token_id, num_steps, embed_weight, layer_weights, final_norm_weight, lm_head_weight,
                            cos_table, sin_table, k_cache, v_cache, hidden_buffer, g_normalized, block_max_vals,
@@ -876,9 +906,10 @@ int qmk_generate_batch(int num_sequences, const int *first_token_ids, const int 
                        const void *lm_head_weight, const void *cos_table, const void *sin_table, void *const *k_caches,
                        void *const *v_caches, int *const *output_logs, int num_layers, int max_seq_len, float attn_scale,
                        int synchronize, cudaStream_t stream) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   clear_error(e);
   if (num_sequences < 1 || num_sequences > qmkp::MAX_SEQ)
     return fail(e, QMK_ERR_BAD_ARGUMENT, "qmk_generate_batch: num_sequences must be 1, 2, 3 or 4");
@@ -924,7 +955,7 @@ int prefill_unlocked(const int *token_ids_host, int num_tokens, const void *embe
                      const void *sin_table, void *k_cache, void *v_cache, int num_layers, int start_position,
                      int max_seq_len, float attn_scale, cudaStream_t stream) {
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   clear_error(e);
   if (num_tokens <= 0) return QMK_OK;
   if (!token_ids_host) return fail(e, QMK_ERR_BAD_ARGUMENT, "token_ids is null");
@@ -980,12 +1011,12 @@ struct qmk_engine {
 
 namespace {
 int apply_handle_unlocked(qmk_engine *h, const void *table) {
-  if (!h) return QMK_ERR_BAD_ARGUMENT;
+  if (!h) return refuse(QMK_ERR_BAD_ARGUMENT, "null engine handle");
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return QMK_ERR_CUDA;
-  if (dev != h->device && cudaSetDevice(h->device) != cudaSuccess) return QMK_ERR_CUDA;
+  if (cudaGetDevice(&dev) != cudaSuccess) return no_device();
+  if (dev != h->device && cudaSetDevice(h->device) != cudaSuccess) return refuse(QMK_ERR_CUDA, "the engine handle's device cannot be made current");
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   const qmk_engine_config &c = h->cfg;
   e->vocab = c.vocab_size > 0 ? c.vocab_size : 151936;   // a handle never inherits another client's values
   e->rope_from_table = c.rope_from_table ? 1 : 0;
@@ -1016,6 +1047,7 @@ int qmk_prefill(const int *token_ids_host, int num_tokens, const void *embed_wei
                 const LDGLayerWeight *layer_weights, const void *final_norm_weight, const void *cos_table,
                 const void *sin_table, void *k_cache, void *v_cache, int num_layers, int start_position,
                 int max_seq_len, float attn_scale, cudaStream_t stream) {
+  qmk_internal::begin_call();
   const auto workspace = chunked_pass_lock(num_tokens);
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   return prefill_unlocked(token_ids_host, num_tokens, embed_weight, layer_weights, final_norm_weight, cos_table, sin_table,
@@ -1023,12 +1055,14 @@ int qmk_prefill(const int *token_ids_host, int num_tokens, const void *embed_wei
 }
 
 int qmk_engine_create(const qmk_engine_config *config, qmk_engine **out) {
-  if (!config || !out) return QMK_ERR_BAD_ARGUMENT;
-  if (config->weight_format < 0 || config->weight_format > 2) return QMK_ERR_BAD_ARGUMENT;
-  if (config->fused > 2 || (config->max_ctas > 0 && config->max_ctas < qmk::NKV)) return QMK_ERR_BAD_ARGUMENT;
+  qmk_internal::begin_call();
+  if (!config || !out) return refuse(QMK_ERR_BAD_ARGUMENT, "null engine options or result");
+  if (config->weight_format < 0 || config->weight_format > 2) return refuse(QMK_ERR_BAD_ARGUMENT, "unknown weight format");
+  if (config->fused > 2 || (config->max_ctas > 0 && config->max_ctas < qmk::NKV))
+    return refuse(QMK_ERR_BAD_ARGUMENT, "fused must be 0, 1 or 2, max_ctas 0 or >= 8");
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || config->device < 0 || config->device >= ndev || config->device >= MAX_DEVICES)
-    return QMK_ERR_CUDA;
+    return refuse(QMK_ERR_CUDA, "no such CUDA device");
   qmk_engine *h = new qmk_engine();
   h->device = config->device;
   h->cfg = *config;
@@ -1071,6 +1105,7 @@ int qmk_engine_destroy(qmk_engine *h) {
 }
 
 int qmk_engine_apply(qmk_engine *h) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   return apply_handle_unlocked(h, nullptr);
 }
@@ -1080,6 +1115,7 @@ int qmk_engine_decode(qmk_engine *h, int input_token_id, int *output_token_id, c
                       const void *cos_table, const void *sin_table, void *k_cache, void *v_cache, void *hidden_buffer,
                       void *g_normalized, void *block_max_vals, void *block_max_idxs, int num_layers, int position,
                       int max_seq_len, float attn_scale, cudaStream_t stream) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   const int rc = apply_handle_unlocked(h, layer_weights);
   if (rc != QMK_OK) return rc;
@@ -1094,6 +1130,7 @@ int qmk_engine_generate(qmk_engine *h, int first_token_id, int num_steps, const 
                         void *g_normalized, void *block_max_vals, void *block_max_idxs, int *output_log, int num_layers,
                         int start_position, int max_seq_len, float attn_scale, int eos_token_id, int synchronize,
                         cudaStream_t stream) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   const int rc = apply_handle_unlocked(h, layer_weights);
   if (rc != QMK_OK) return rc;
@@ -1107,6 +1144,7 @@ int qmk_engine_prefill(qmk_engine *h, const int *token_ids_host, int num_tokens,
                        const LDGLayerWeight *layer_weights, const void *final_norm_weight, const void *cos_table,
                        const void *sin_table, void *k_cache, void *v_cache, int num_layers, int start_position,
                        int max_seq_len, float attn_scale, cudaStream_t stream) {
+  qmk_internal::begin_call();
   const auto workspace = chunked_pass_lock(num_tokens);
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   const int rc = apply_handle_unlocked(h, layer_weights);
@@ -1116,10 +1154,11 @@ int qmk_engine_prefill(qmk_engine *h, const int *token_ids_host, int num_tokens,
 }
 
 int qmk_sync_status(void) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
-  if (!e->ready) return e->last_status;
+  if (!e) return no_device();
+  if (!e->ready) return refuse(e->last_status, e->last_error.c_str());
   QMK_CUDA(e, cudaDeviceSynchronize());
   QMK_CUDA(e, cudaMemcpy(e->status_host, e->status, 16, cudaMemcpyDeviceToHost));
   if (e->status_host[0] != 0) {
@@ -1128,19 +1167,21 @@ int qmk_sync_status(void) {
              e->status_host[2]);
     return fail(e, static_cast<int>(e->status_host[0]), buf);
   }
-  return e->last_status;
+  return refuse(e->last_status, e->last_error.c_str());   // (no text where that is QMK_OK)
 }
 
 const char *qmk_last_error(void) {
-  // a copy per calling thread, taken under the lock: another thread's next call may rewrite the engine's string
+  // a copy per calling thread, taken under the lock: another thread's next call may rewrite the engine's string, which is the answer
+  // for a thread that has made no call itself
   static thread_local std::string mine;
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  mine = !t_error.empty() ? t_error : e ? e->last_error : std::string("no CUDA device");
+  mine = t_called ? t_error : e ? e->last_error : std::string("no CUDA device");
   return mine.c_str();
 }
 
 int qmk_num_ctas(void) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e || ensure_ready(e) != QMK_OK) return -1;
@@ -1152,9 +1193,10 @@ long long qmk_scratch_bytes(void) {
 }
 
 int qmk_selftest_wait_timeout(int budget_us) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   int rc = ensure_ready(e);
   if (rc != QMK_OK) return rc;
   if (budget_us < 1 || budget_us > 1000000) return fail(e, QMK_ERR_BAD_ARGUMENT, "budget_us must be in [1, 1e6]");
@@ -1197,9 +1239,10 @@ int qmk_generate_static(int first_token_id, int num_steps, const void *embed_wei
                         const void *lm_head_weight, void *k_cache, void *v_cache, void *g_normalized,
                         int *output_log, int num_layers, int start_position, int max_seq_len, float attn_scale,
                         int eos_token_id, cudaStream_t stream) {
+  qmk_internal::begin_call();
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
-  if (!e) return QMK_ERR_CUDA;
+  if (!e) return no_device();
   clear_error(e);
   if (num_steps <= 0) return QMK_OK;
   if (!output_log || !embed_weight || !layer_weights || !final_norm_weight || !lm_head_weight || !k_cache || !v_cache)

@@ -1045,6 +1045,7 @@ extern "C" int qmk_prefill_chunked(const int *token_ids_host, int num_tokens, co
                                    const LDGLayerWeight *layer_weights, const void *cos_table, const void *sin_table,
                                    void *k_cache, void *v_cache, int num_layers, int start_position, int max_seq_len,
                                    float attn_scale, cudaStream_t stream) {
+  qmk_internal::begin_call();
   return prefill_impl(token_ids_host, num_tokens, embed_weight, layer_weights, cos_table, sin_table, k_cache, v_cache, num_layers,
                       start_position, max_seq_len, attn_scale, stream, nullptr, false);
 }
@@ -1068,6 +1069,7 @@ extern "C" int qmk_prefill_packed(const int *token_ids_host, int num_seqs, const
                                   const LDGLayerWeight *layer_weights, const void *cos_table, const void *sin_table,
                                   void *const *k_caches, void *const *v_caches, int num_layers, int max_seq_len, float attn_scale,
                                   cudaStream_t stream) {
+  qmk_internal::begin_call();
   if (num_seqs <= 0) return QMK_OK;
   if (!seq_lens) return qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "packed prefill: null lengths");
   long total = 0;
@@ -1146,6 +1148,7 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
                                   const void *sin_table, void *const *k_caches, void *const *v_caches,
                                   int *const *output_logs, int num_layers, int max_seq_len, float attn_scale,
                                   cudaStream_t stream) {
+  qmk_internal::begin_call();
   using namespace qmk_pf;
   if (num_steps <= 0) return QMK_OK;
   qmk_internal::PrefillEnv env;
@@ -1386,6 +1389,7 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
 // wait on the first stage runs out after budget_us, every role leaves its loop, TMEM is freed and the kernel
 // returns status 4 with the context intact.
 extern "C" int qmk_selftest_gemm_wait_timeout(int budget_us) {
+  qmk_internal::begin_call();
   std::string err;
   if (budget_us < 1 || budget_us > 1000000) return qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "budget_us must be in [1, 1e6]");
   int rc = qmk_tc::ensure_gemm_attrs(&err);
@@ -1430,6 +1434,7 @@ extern "C" int qmk_selftest_gemm_wait_timeout(int budget_us) {
 // The same of the attention kernel: a query tile at position 512 whose score products stop behind the first, with keys and values
 // in flight.
 extern "C" int qmk_selftest_attention_wait_timeout(int budget_us) {
+  qmk_internal::begin_call();
   using qmk_pf::QS;
   using qmk_pf::NKV;
   std::string err;
@@ -1465,6 +1470,7 @@ extern "C" int qmk_selftest_attention_wait_timeout(int budget_us) {
 // than the producer may be ahead).  what = 1: nothing is loaded, so that consumers wait for chunks, then for pieces, and the
 // producer for finished ones; 2: one chunk's copies are missing among a ring of others in flight.
 extern "C" int qmk_selftest_decode_attention_wait_timeout(int budget_us, int what) {
+  qmk_internal::begin_call();
   using namespace qmk_pf;
   std::string err;
   if (budget_us < 1 || budget_us > 1000000 || what < DAM_NO_LOADS || what > DAM_LOST_COPY)
@@ -1519,6 +1525,7 @@ extern "C" int qmk_selftest_decode_attention_wait_timeout(int budget_us, int wha
 // alone (the first has a ring of copies in flight whose barriers cannot complete), and an issuer that gives up behind the first
 // tile (MMAs and a ring of copies in flight).  All end in status 4 with the pair's copies and MMAs drained.
 extern "C" int qmk_selftest_gemm_pair_wait_timeout(int budget_us, int what) {
+  qmk_internal::begin_call();
   std::string err;
   if (budget_us < 1 || budget_us > 1000000 || what < qmk_pair::NO_LOADS || what > qmk_pair::SECOND_CTA_NO_LOADS)
     return qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "budget_us must be in [1, 1e6], what in [1, 3]");
@@ -1556,6 +1563,7 @@ extern "C" int qmk_selftest_gemm_pair_wait_timeout(int budget_us, int what) {
 }
 
 extern "C" int qmk_gemm_f16_tn(const void *a, const void *b, float *c, int m, int n, int k, cudaStream_t stream) {
+  qmk_internal::begin_call();
   std::string err;
   CUtensorMap ma, mb;
   unsigned int *status = nullptr;
@@ -1583,7 +1591,10 @@ extern "C" int qmk_gemm_f16_tn(const void *a, const void *b, float *c, int m, in
     else if (host[0] != 0) { rc = static_cast<int>(host[0]); err = "gemm: a bounded device wait ran out"; }
   }
   if (status) cudaFree(status);
-  if (rc != QMK_OK) fprintf(stderr, "[qwen_megakernel] error %d: %s\n", rc, err.c_str());
+  if (rc != QMK_OK) {
+    qmk_internal::note_error(err);
+    fprintf(stderr, "[qwen_megakernel] error %d: %s\n", rc, err.c_str());
+  }
   return rc;
 }
 
@@ -1592,11 +1603,13 @@ extern "C" int qmk_gemm_f16_tn(const void *a, const void *b, float *c, int m, in
 // matrix, C receives fp16 silu(A gate^T) * (A up^T) - the three forms the decode step uses.
 extern "C" int qmk_gemm_packed_tn(const void *a, const void *b, const void *b2, void *c, int m, int n, int k, int weight_format,
                                   int mode, int box_n, cudaStream_t stream) {
+  qmk_internal::begin_call();
   std::string err;
   CUtensorMap ma, mb, mb2;
   unsigned int *status = nullptr;
   if (weight_format < 1 || weight_format > 2 || mode < 0 || mode > 2 || m <= 0 || n <= 0 || m % 128 || n % 128 ||
       (mode == 2 && !b2) || !a || !b || !c) {
+    qmk_internal::note_error("qmk_gemm_packed_tn: bad argument");
     fprintf(stderr, "[qwen_megakernel] error %d: qmk_gemm_packed_tn: bad argument\n", QMK_ERR_BAD_ARGUMENT);
     return QMK_ERR_BAD_ARGUMENT;
   }
@@ -1624,6 +1637,9 @@ extern "C" int qmk_gemm_packed_tn(const void *a, const void *b, const void *b2, 
     else if (host[0] != 0) { rc = static_cast<int>(host[0]); err = "gemm: a bounded device wait ran out"; }
   }
   if (status) cudaFree(status);
-  if (rc != QMK_OK) fprintf(stderr, "[qwen_megakernel] error %d: %s\n", rc, err.c_str());
+  if (rc != QMK_OK) {
+    qmk_internal::note_error(err);
+    fprintf(stderr, "[qwen_megakernel] error %d: %s\n", rc, err.c_str());
+  }
   return rc;
 }

@@ -36,6 +36,20 @@ def test_engine_handle_argument_checks(built_library):
     assert lib.qmk_engine_apply(None) != 0
 
 
+def test_refusals_without_an_engine_have_a_text(built_library):
+    """Calls that fail before there is an engine to keep the error: the text is theirs, not an older one."""
+    import qwen_megakernel_C as C
+    lib = C._lib
+    handle = ctypes.c_void_p()
+    cfg = C._EngineConfig(0, 151936, 5, 0, -1, -1, -1, -1, None)
+    assert lib.qmk_engine_create(ctypes.byref(cfg), ctypes.byref(handle)) != 0 and b"weight format" in lib.qmk_last_error()
+    assert lib.qmk_engine_apply(None) != 0 and b"handle" in lib.qmk_last_error()
+    if not torch.cuda.is_available():
+        assert lib.qmk_set_fused(1, 1) != 0 and lib.qmk_last_error() == b"no CUDA device"
+        assert lib.qmk_decode_batched(1, None, None, 1, *[None] * 9, 1, 1, 1.0, None) != 0 and lib.qmk_last_error() == b"no CUDA device"
+    assert lib.qmk_engine_destroy(None) == 0
+
+
 def test_abi_version_handshake(built_library):
     import qwen_megakernel_C as C
     from Model import Qwen06B_architecture as A

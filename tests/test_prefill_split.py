@@ -161,6 +161,42 @@ def test_error_text_survives_another_threads_call(built_library):
     assert b"budget_us" not in C._lib.qmk_last_error()
 
 
+def test_error_text_is_of_the_threads_own_last_call(built_library):
+    """The other direction: a call that succeeded has no text, whatever another thread failed at since (the void ops tell by the
+    text).  A later call that returns a status clears the text, also where it does no work; a thread without a call of its own
+    sees the device's last error."""
+    import threading
+    import qwen_megakernel_C as C
+    from Model.Qwen06B_architecture import Decoder
+    w = S.weights_to(S.make_weights(seed=9, num_layers=2, vocab_size=512, max_seq_len=16), "cuda")
+    eng = Decoder(weights=w, verbose=False, max_seq_len=64)
+    seen = []
+
+    def elsewhere(*calls):
+        thread = threading.Thread(target=lambda: seen.extend(call() for call in calls))
+        thread.start()
+        thread.join()
+
+    def text():
+        return C._lib.qmk_last_error().decode()
+
+    eng.prefill_ids([1, 2, 3, 4, 5])
+    elsewhere(lambda: C._lib.qmk_selftest_gemm_wait_timeout(0), text)
+    assert seen[0] == 2 and "budget_us" in seen[1] and text() == ""
+    elsewhere(text)
+    assert "budget_us" in seen[2]                      # (no call of its own: the device's last error)
+    assert C._lib.qmk_sync_status() == 2 and "budget_us" in text()      # asked for: the device's status and its text
+    elsewhere(lambda: eng.prefill_ids([6]))
+    assert C._lib.qmk_sync_status() == 0 and text() == ""
+    for quiet in (lambda: C._lib.qmk_set_step_overlap(-1), lambda: C._lib.qmk_configure(-1, -1, -1, -1, -1), C._lib.qmk_num_ctas,
+                  lambda: C._lib.qmk_selftest_wait_timeout(300), lambda: C._lib.qmk_decode_batched(1, *[None] * 2, 0, *[None] * 9, 1, 1, 1.0, None)):
+        assert C._lib.qmk_selftest_gemm_wait_timeout(0) == 2 and "budget_us" in text()
+        quiet()
+        assert text() == ""
+    assert C._lib.qmk_gemm_f16_tn(None, None, None, 100, 64, 64, None) != 0 and text() not in ("", "budget_us must be in [1, 1e6]")
+    assert C._lib.qmk_engine_apply(None) != 0 and "handle" in text()
+
+
 def test_short_prompts_do_not_wait_for_a_chunked_pass(built_library):
     """The workspace of the chunked pass is held for a whole pass (some 20 ms here).  A call of the op that does not use it -
     measured on one that is refused before any GPU work - returns meanwhile."""
