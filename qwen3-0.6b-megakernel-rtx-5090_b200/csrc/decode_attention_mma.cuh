@@ -26,9 +26,9 @@ namespace qmk_pf {
 // go over the chunks, a chain a warp, and merge.  An item of several pieces is finished by whichever CTA arrives last (a counter
 // per item, nobody waits).
 //
-// Decode steps, a CTA per item and range -> pieces: 64 NVFP4 sequences of 128 to 2048 tokens 2710 -> 2120 us, 16 fp16 ones of 64 to
-// 1024 (with the GEMMs' 64-row tiles) 1023 -> 947, 32 of 64 to 2048 1775 -> 1425, 128 of 1024 3530 -> 3370; 16 and 32 of 1024, which
-// were even before, 1048 -> 1062 and 1322 -> 1330.
+// Decode steps, a CTA per item and range -> pieces (with the GEMMs' 64-row tiles and prefetch): 64 NVFP4 sequences of 128 to 2048
+// tokens 2710 -> 2120 us, 16 fp16 ones of 64 to 1024 1026 -> 932, 32 of 64 to 2048 1771 -> 1400; 16 and 32 of 1024, which were even
+// before, 1053 -> 1042 and 1285 -> 1288, 30 of 300 to 320 887 -> 877.
 //
 // A chunk is four tiled TMA boxes of 16 rows x 128 bytes with the 128-byte swizzle, through per-sequence tensor maps kept
 // in device memory, and a warp handles it with 16 mma.sync.m16n8k16: scores = K[16 x 128] . q[128 x 4] (columns: head 0

@@ -257,10 +257,14 @@ struct Groups {
   int *amax_idx;
   // Weights a later kernel of the chain will read, brought into L2 meanwhile: CTA i of the launch asks for the i-th `prefetch_piece`
   // bytes of each matrix (up to prefetch_bytes; all multiples of 16).  The chain is bound by latency, DRAM idles for most of it, and
-  // a kernel sees its weights' addresses only a microsecond before its activations are there.  Decode step of 5 sequences 786 -> 771 us,
-  // prompts of 31 / 109 / 500 tokens 857 / 947 / 1555 -> 827 / 931 / 1525 us.
+  // a kernel sees its weights' addresses only a microsecond before its activations are there.  Prompts ask as soon as a CTA is up:
+  // 31 / 109 / 500 tokens 866 / 963 / 1563 us without, 830 / 938 / 1532 so, 834 / 940 / 1585 behind the wait for the kernel before.
+  // Decode steps ask behind that wait: the O GEMM starts under the attention, which reads the caches at the DRAM rate, and 19 MB asked
+  // for there cost it 1.5 us a layer.  Without / at once / behind the wait: 8 fp16 sequences of 64 tokens 791 / 769 / 762 us a step, 30 of
+  // 300 to 320 906 / 929 / 877, 16 of 1024 1069 / 1073 / 1042.
   const unsigned char *prefetch[MAX_PREFETCH] = {nullptr, nullptr, nullptr};
   uint32_t prefetch_bytes[MAX_PREFETCH] = {0, 0, 0}, prefetch_piece[MAX_PREFETCH] = {0, 0, 0};
+  bool prefetch_behind = false;
   // Plain epilogue, no split-K: 1 = the C matrices are fp16 [M x N_g] (the pointers are reinterpreted), half the
   // store burst of a launch whose CTAs all reach their epilogue together.
   int out_f16;
@@ -381,6 +385,15 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   // the first fill of the ring needs no free-slot wait: it is issued before the CTA-wide barrier below, so
   // that the first TMA round trip overlaps the TMEM allocation
   const int prologue = selftest_no_loads ? 0 : (kblocks < STAGES ? kblocks : STAGES);
+  auto prefetch_ahead = [&]() {
+    const uint32_t cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+#pragma unroll
+    for (int i = 0; i < MAX_PREFETCH; ++i) {
+      const uint32_t first = cta * groups.prefetch_piece[i];
+      if (first < groups.prefetch_bytes[i])
+        prefetch_l2(groups.prefetch[i] + first, min(groups.prefetch_piece[i], groups.prefetch_bytes[i] - first));
+    }
+  };
   if (warp == 0 && elect_one()) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map_b)) : "memory");
@@ -402,13 +415,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       tma_load_2d(base + kb * STAGE_BYTES + b_dst, map_b, (kb0 + kb) * kcol, n0, b_landed(kb));
       if (FUSE) tma_load_2d(base + kb * STAGE_BYTES + b_dst + b_dst_step, &map_b1, (kb0 + kb) * kcol, n0, b_landed(kb));
     }
-    const uint32_t cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-#pragma unroll
-    for (int i = 0; i < MAX_PREFETCH; ++i) {
-      const uint32_t first = cta * groups.prefetch_piece[i];
-      if (first < groups.prefetch_bytes[i])
-        prefetch_l2(groups.prefetch[i] + first, min(groups.prefetch_piece[i], groups.prefetch_bytes[i] - first));
-    }
+    if (!groups.prefetch_behind) prefetch_ahead();
   }
   if (WQ != 0 && warp >= 2 && warp < 6) {
     // scales of this CTA's B rows into shared memory while the first copies are in flight (the CTA-wide barrier below
@@ -454,6 +461,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         tma_load_2d(base + kb * STAGE_BYTES, &map_a, (kb0 + kb) * BK, m0, a_landed(kb));
         if (AH == 2) tma_load_2d(base + kb * STAGE_BYTES + HALF_A, &map_a, K + (kb0 + kb) * BK, m0, a_landed(kb));
       }
+      if (groups.prefetch_behind) prefetch_ahead();
       int issued = prologue, s = prologue == STAGES ? 0 : prologue;   // slot of K block kb
       uint32_t parity = 0;                                            // of the use before it, whose MMAs free the slot
       // self test of the bounded waits: the loads are never issued, so the MMA thread's first wait runs out

@@ -312,6 +312,7 @@ thread_local PrefetchList t_prefetch;
 PrefetchScope::PrefetchScope(const PrefetchList &list) : prev_(t_prefetch) { t_prefetch = list; }
 PrefetchScope::~PrefetchScope() { t_prefetch = prev_; }
 static void set_prefetch(qmk_gemm::Groups *gr, long ctas) {
+  gr->prefetch_behind = t_prefetch.behind;
   for (int i = 0; i < qmk_gemm::MAX_PREFETCH; ++i) {
     gr->prefetch[i] = static_cast<const unsigned char *>(t_prefetch.ptr[i]);
     gr->prefetch_bytes[i] = t_prefetch.ptr[i] ? static_cast<uint32_t>(t_prefetch.bytes[i]) : 0u;
@@ -1261,6 +1262,7 @@ extern "C" int qmk_decode_batched(int num_sequences, const int *first_token_ids,
       auto wp = [&](int j) { return reinterpret_cast<const void *>(r[rec_slot[j]]); };
       auto ahead_of = [&](int layer, std::initializer_list<int> js) {
         qmk_tc::PrefetchList list;
+        list.behind = true;
         int i = 0;
         for (int j : js)
           if (layer < num_layers) {

@@ -48,6 +48,7 @@ class SplitActScope {
 struct PrefetchList {
   const void *ptr[3] = {nullptr, nullptr, nullptr};
   size_t bytes[3] = {0, 0, 0};
+  bool behind = false;               // asked for behind the wait for the kernel before (Groups::prefetch_behind)
 };
 class PrefetchScope {
  public:
