@@ -210,19 +210,38 @@ def test_both_decode_attention_kernels(C, mma):
     assert worst < LOGIT_TOL
 
 
-@pytest.mark.parametrize("lens", [[1], [700, 20, 1], [13 * 16 + 1, 13 * 16, 12 * 16 + 1, 12 * 16, 1, 2],
-                                  [700] + [16 * i for i in range(1, 23)], [1 + (53 * i) % 300 for i in range(37)],
-                                  [1 + (101 * i) % 400 for i in range(64)], [40] * 128],
-                         ids=["one", "split", "edges", "cut", "37", "64", "128"])
-def test_attention_pieces(C, lens):
+def _pieces(rows, ctas):
+    """The rule by which a step's attention is cut, restated: ranges per item, pieces of each sequence's ranges, number of pieces."""
+    n, kv_heads = len(rows), 8
+    splits = min(max(ctas // (n * kv_heads), 1), 8)
+    chunks = [-(-r // 16) for r in rows]
+    longest = max(16, kv_heads * sum(chunks) // 4 * (7 if splits == 1 else 12) // ctas)
+    parts = [1 if -(-c // splits) <= longest else 2 if -(-c // splits) <= 2 * longest else 4 for c in chunks]
+    return splits, parts, kv_heads * splits * sum(parts)
+
+
+@pytest.mark.parametrize("lens,splits,cut,several_each", [
+    ([1], 8, 1, False), ([700, 20, 1], 8, 1, False), ([13 * 16 + 1, 13 * 16, 12 * 16 + 1, 12 * 16, 1, 2], 6, 1, False),
+    ([700] + [16 * i for i in range(1, 23)], 1, 4, False), ([1 + (53 * i) % 300 for i in range(37)], 1, 2, True),
+    ([1 + (101 * i) % 400 for i in range(64)], 1, 1, True), ([40] * 128, 1, 1, True), ([1100] + [20] * 17, 2, 4, True),
+    ([64] * 5 + [2048], 6, 2, True), ([50] * 6 + [2000] + [50] * 5, 3, 4, True), ([200, 2300], 8, 2, False)],
+    ids=["one", "split", "edges", "cut", "37", "64", "128", "split-cut4", "split-cut2", "split3-cut4", "two"])
+def test_attention_pieces(C, lens, splits, cut, several_each):
     """The attention's list of pieces: items of one range and of several, ranges whole and cut in two or four, fewer pieces than
-    CTAs and more (64 and 128 sequences: CTAs take further pieces), against the CUDA-core kernel with a CTA per item and range.  Both
-    round the same fp32 result to fp16, so logits differ by roundings of one output and what they do downstream: the bar of
-    this file.  Who takes which piece does not show: a second run is the same bit for bit."""
-    vocab, steps, L, n = 2048, 2, 768, len(lens)
-    w = S.make_weights(seed=31, num_layers=2, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    CTAs and more (CTAs take further pieces), every other batch with table RoPE, against the CUDA-core kernel with a CTA per item and range.
+    Both round the same fp32 result to fp16, so they differ by roundings of one output and what they do downstream: 1.5e-3 of a logit
+    and one fp16 step (2^-9) of layer 1's new K row at most, a quarter of the bars; in the oracle a chunk of 16 rows left out of one head of
+    2048, or taken twice, moves them by 6e-2 and 8e-2.  Who takes which piece does not show: a second run is the same bit for bit."""
+    vocab, steps, n = 2048, 2, len(lens)
+    table = len(lens) % 2 == 0
+    L = (max(lens) + 64) // 64 * 64
+    ctas = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    if ctas == 296:
+        got_splits, parts, total = _pieces([Ln - 1 for Ln in lens], ctas)
+        assert (got_splits, max(parts), total > ctas) == (splits, cut, several_each), (got_splits, parts, total)
+    w = S.make_weights(seed=31, num_layers=2, vocab_size=vocab, norm_std=0.1, max_seq_len=L if table else 16)
     prompts = [S.make_prompt(Ln, seed=1500 + i, vocab_size=vocab) for i, Ln in enumerate(lens)]
-    eng = _engine(w, n, L, engine="gemm", prefill_mode="tensor")
+    eng = _engine(w, n, L, engine="gemm", prefill_mode="tensor", rope_from_table=table)
     runs = []
     for mma in (1, 1, 0):
         dump = torch.zeros(n, steps, vocab, device="cuda")
@@ -233,9 +252,40 @@ def test_attention_pieces(C, lens):
         finally:
             C.set_logits_dump(None)
             C.set_decode_attention(1)
+            C.configure(rope_from_table=0)
         runs.append((dump.cpu(), [k[:, :, :Ln + steps - 1].cpu() for k, Ln in zip(eng._k_caches, lens)]))
     assert torch.equal(runs[0][0], runs[1][0]) and all(torch.equal(a, b) for a, b in zip(runs[0][1], runs[1][1]))
-    assert float((runs[0][0][:, 0] - runs[2][0][:, 0]).abs().max()) < LOGIT_TOL
+    logit = float((runs[0][0][:, 0] - runs[2][0][:, 0]).abs().max())
+    # the first step's row of layer 1: what layer 0's attention gave, through one layer
+    row = max(float((a[1, :, Ln - 1].float() - b[1, :, Ln - 1].float()).abs().max()) for a, b, Ln in zip(runs[0][1], runs[2][1], lens))
+    print(f"pieces, {n} sequences: logits {logit:.2e}, layer-1 row {row:.2e}")
+    assert logit < 6e-3 and row < 8e-3
+
+
+@pytest.mark.parametrize("n,fmt", [(17, "fp16"), (64, "fp16"), (65, "fp16"), (128, "fp16"), (64, "fp8"), (64, "nvfp4"), (65, "nvfp4")])
+def test_graph_steps_match_dumped_steps(C, n, fmt):
+    """What a caller without a logits dump runs - a captured step, replayed, whose LM head picks from its accumulator rows - against plain
+    launches that store the logits: the same tokens and cache rows bit for bit, in every quarter of the 64- and 128-row tiles, over
+    steps that each make the attention's list anew and take it from the start."""
+    import quantize as Q
+    vocab, steps, L = 2048, 4, 512
+    w = S.make_weights(seed=33, num_layers=2, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    pack = {"fp16": lambda x: x, "fp8": lambda x: Q.quantize_weights_fp8(x)[0], "nvfp4": lambda x: Q.quantize_weights_nvfp4(x)[0]}[fmt]
+    prompts = [S.make_prompt(1 + (101 * i) % 400, seed=1600 + i, vocab_size=vocab) for i in range(n)]
+    eng = _engine(pack(w), n, L, engine="gemm", prefill_mode="tensor", weight_format=fmt)
+    dump = torch.zeros(n, steps, vocab, device="cuda")
+    runs = []
+    try:
+        for target in (None, dump, None):
+            C.set_logits_dump(target)
+            runs.append((eng.generate_ids(prompts, steps), [(k.clone(), v.clone()) for k, v in zip(eng._k_caches, eng._v_caches)]))
+    finally:
+        C.set_logits_dump(None)
+        C.set_weight_format("fp16")
+    assert [dump[b].argmax(1).tolist() for b in range(n)] == runs[1][0]
+    for tokens, rows in (runs[0], runs[2]):
+        assert tokens == runs[1][0]
+        assert all(torch.equal(a, b) and torch.equal(c, d) for (a, c), (b, d) in zip(rows, runs[1][1]))
 
 
 @pytest.mark.parametrize("fmt", ["fp16", "fp8", "nvfp4"])
