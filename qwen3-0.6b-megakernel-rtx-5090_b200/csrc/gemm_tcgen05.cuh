@@ -334,7 +334,7 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   // Split activations with packed weights are at the 128 registers that 448 threads leave: their loop keeps its waits inline (a call costs
   // spills), and 64-wide tiles, which longer prompts take, ask for nothing ahead.  FP8 prefill op of 60 / 400 / 777 tokens 1390 / 3720 /
   // 6292 us with called waits and prefetch everywhere, 1371 / 3663 / 6162 so; without any prefetch the 60 tokens take 1431.
-  constexpr bool PREFETCH = AH == 1 || WQ == 0 || BN == 32;
+  constexpr bool FULL = AH == 2 && WQ != 0, PREFETCH = !FULL || BN == 32;
   static_assert(WQ == 0 || (FUSE ? 2 * BN : BN) <= 128, "packed weights: at most 128 B rows per stage (scales live in shared memory)");
   constexpr int SB = FUSE ? 2 * BN : BN;          // B rows held per stage / accumulator columns
   constexpr int NACC = AH == 2 ? 4 : 1;           // accumulators: one, or with split activations four that the K blocks take in turn
@@ -500,9 +500,8 @@ gemm_f16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       const uint64_t da0 = smem_desc_sw128(base), db0 = smem_desc_sw128(base + TILE_A);
       uint64_t da = da0, db = db0;         // (a ring ends below 2^18 bytes: the slot's offset does not leave the address field)
       for (int kb = 0; kb < kblocks; ++kb) {
-        ok = (AH == 2 ? bar_wait(full(s), parity, abort_flag, status, budget_ns) : bar_wait_cold(full(s), parity, abort_flag, status, budget_ns)) &&
-             (!WQ || (AH == 2 ? bar_wait(a_full(s), parity, abort_flag, status, budget_ns)
-                              : bar_wait_cold(a_full(s), parity, abort_flag, status, budget_ns))) &&
+        ok = (FULL ? bar_wait(full(s), parity, abort_flag, status, budget_ns) : bar_wait_cold(full(s), parity, abort_flag, status, budget_ns)) &&
+             (!WQ || (FULL ? bar_wait(a_full(s), parity, abort_flag, status, budget_ns) : bar_wait_cold(a_full(s), parity, abort_flag, status, budget_ns))) &&
              (AH == 1 || kb < NACC || bar_wait(blk_free(kb % NACC), (kb / NACC - 1) & 1, abort_flag, status, budget_ns));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
