@@ -333,7 +333,7 @@ int qmk_generate_static(
  * RoPE + cache write, causal attention over the cache, and SwiGLU between them.  Same arguments, cache
  * layout, position rule and blocking behaviour as qmk_prefill; all three weight formats (packed FP8 / NVFP4 matrices
  * stay packed in HBM and are expanded to fp16 tiles inside the GEMM, see qmk_gemm_packed_tn, or once per layer in chunks
- * of 384 rows and more).  GEMM operands are rounded to fp16 (the
+ * of 512 rows and more).  GEMM operands are rounded to fp16 (the
  * decode kernels keep 22 bits of fp32 activations), so cache rows agree with qmk_prefill's to fp16 rounding, not
  * bit for bit.  Scratch (285 MB, shared with qmk_prefill; 32 MB more for expanded layers where they fit) is allocated on
  * the first call per device. */
@@ -358,14 +358,16 @@ int qmk_prefill_packed(
     float attn_scale, cudaStream_t stream);
 
 /* Greedy decode of up to 128 sequences on the tensor-core path (the batched configurations): each step runs
- * the seven projections and the LM head as tcgen05 GEMMs over one 128-row tile of sequences, with row kernels
+ * the seven projections and the LM head as tcgen05 GEMMs over one row tile of sequences (64 or 128 rows), with row kernels
  * for the norms, per-head QK-norm + RoPE + cache write (each sequence at its own position in its own cache),
  * per-sequence attention over the cache, SwiGLU and the argmax.  Same arguments as qmk_generate_batch (host
  * arrays of num_sequences entries; no EOS stop; logits dump [sequence][step][vocab]); all three weight formats
  * (packed matrices are expanded inside the GEMMs, which halves / quarters the weight bytes of a step), vocab
- * a multiple of 128; blocks until done.  One step costs about 400 kernel launches, so it pays from roughly
- * eight sequences on; below that qmk_generate_batch (one persistent launch) is faster.  Numerics as
- * qmk_prefill_chunked (GEMM operands rounded to fp16). */
+ * a multiple of 128; blocks until done.  A step is about 200 kernels, captured once as a graph and replayed; up to three
+ * sequences (four where contexts are short) qmk_generate_batch, one persistent launch, is faster.  Numerics as
+ * qmk_prefill_chunked (GEMM operands rounded to fp16).  A row of logits without a largest value (all NaN) has no pick: the
+ * step that would read it ends the call with QMK_ERR_BAD_TOKEN, as in qmk_generate_batch; in the last step the log
+ * holds 2^31 - 1. */
 int qmk_decode_batched(
     int num_sequences, const int *first_token_ids, const int *start_positions,
     int num_steps, const void *embed_weight,

@@ -316,8 +316,9 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 //
 // AM: rows of the MMA, 128 or, for launches of one row tile with at most 64 live rows (decode steps), 64.  With every operand in
 // place the four products of a K block take 162 cycles against 32 columns at 128 rows and 99 at 64 (the tensor core reads A from
-// shared memory, 4 KB a product against 2 KB), and a stage is 8 KB smaller, so that the ring holds more of the K loop
-// (packed weights: decode step of 64 NVFP4 sequences 1198 -> 1150 us, of 16 FP8 ones 978 -> 925).  An
+// shared memory, 4 KB a product against 2 KB), and a stage is 8 KB smaller, so that the ring holds more of the K loop.  Decode
+// steps at 64-token contexts, 128 rows everywhere -> so: 5 / 16 / 64 fp16 sequences 774 / 780 / 878 -> 759 / 773 / 894 us (the last of
+// them loses), 16 FP8 940 -> 911, 64 NVFP4 1093 -> 1060.  An
 // accumulator of 64 rows lies in lanes 0 .. 15 of each warp's 32: row r in lane 32 * (r / 16) + r % 16.
 template <int BN, bool FUSE = false, int WQ = 0, int AH = 1, bool RS = false, int AM = BM>
 __global__ void __launch_bounds__(threads_for(WQ, AH), 1)

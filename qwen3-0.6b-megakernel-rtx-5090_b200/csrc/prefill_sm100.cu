@@ -561,7 +561,7 @@ std::mutex g_ws_decode_mu;
 
 cudaError_t device_memory(void **at, size_t bytes) { return cudaMalloc(at, bytes); }
 
-// `rows`: activation rows the buffers hold (CHUNK for prefill, one 128-row tile for the batched decode).  All or nothing:
+// `rows`: activation rows the buffers hold (CHUNK for prefill, four 128-row tiles of partial sums for the batched decode).  All or nothing:
 // buffers that were made are given back when a later one does not fit.  `no_room`: set (and nothing reported) where the
 // reason is memory, for callers with another way.
 int ensure_workspace(Workspace &w, int rows, bool *no_room = nullptr) {

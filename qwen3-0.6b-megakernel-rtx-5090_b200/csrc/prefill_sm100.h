@@ -74,7 +74,7 @@ cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
 }
 
 // `box_n`: rows per box the B maps were made with (= the N tile: 32, 64 or 128).  `live_rows` (0 = all M): rows of
-// the output the epilogue stores; a decode step of B sequences pads its rows to one 128-row tile and needs only
+// the output the epilogue stores; a decode step of B sequences pads its rows to one tile and needs only
 // the first B.  `a_box_rows` (0 = 128): rows per box of the A map when it is shorter than the tile.
 // `wq`: weight format of B - 0 fp16 (maps from make_map_f16), 1 FP8-E4M3 rows, 2 NVFP4 rows (maps from make_map_packed;
 // the launch also needs the matrices' base pointers, `raw...`, for the scales inside the rows).
