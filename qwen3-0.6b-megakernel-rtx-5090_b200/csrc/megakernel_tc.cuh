@@ -204,6 +204,12 @@ __device__ __forceinline__ void e4m3x4_half2x2(uint32_t four, uint32_t &first, u
 }
 
 // One warp: rows of the 16-row tile that starts at ring chunk `first` (valid rows <= 16), k-step pairs [p0, p1).
+// Operands come in front of the products they feed.  An MMA takes 8.5 cycles of a sub-partition (stand-alone, 4 to 12 warps;
+// 21 from one to the next that depends on it), a ldmatrix 48 cycles until its data can be used and four of the SM's
+// shared-memory port: asked for one after the other, in between the MMAs, a tile waited for its operands (26 cycles per MMA).
+// With the attention's and the slices' operands ahead too: two fp16 sequences 570 -> 549 us per step, four 796 -> 780 (1024
+// tokens), one 490 -> 486, one with FP8 rows 491 -> 482.  What bounds the phase now is the port: 48 rows of gate and up are
+// 768 cycles of it.
 // Leaves the 16 row sums of that k range in part[0..15] (sequence b: part[16 b..]) and hands the tile's chunks back with `units` each.
 // Lanes 0..3 each wait for one of the tile's chunks (the vote that follows orders the copied bytes before every
 // lane's loads).
@@ -238,19 +244,17 @@ __device__ __forceinline__ void tile_task(const Params &P, const Ctx &c, uint32_
 #pragma unroll
     for (int i = 0; i < 4; ++i) sum[i] += odd[i];
   } else if (ok) {
-    for (int p = p0; p < p1; p += 2) {
-      float acc[4];
+#pragma unroll 1
+    for (int p = p0; p < p1; p += 2) {     // all operands of a chain before its first MMA
+      uint32_t a[4][4];
+      const uint4 b0 = b_pair(c, p), b1 = b_pair(c, p + 1);
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        if (u == 1 && p + 1 == p1) break;
-        uint32_t a0[4], a1[4];
-        const uint4 b = b_pair(c, p + u);
-        ldsm_x4(a_addr + (p + u) * 64, a0);
-        ldsm_x4(a_addr + (p + u) * 64 + 32, a1);
-        if (u == 0) mma_16816_zero(acc, a0, b.x, b.y);
-        else mma_16816(acc, a0, b.x, b.y);
-        mma_16816(acc, a1, b.z, b.w);
-      }
+      for (int u = 0; u < 4; ++u) ldsm_x4(a_addr + p * 64 + u * 32, a[u]);
+      float acc[4];
+      mma_16816_zero(acc, a[0], b0.x, b0.y);
+      mma_16816(acc, a[1], b0.z, b0.w);
+      mma_16816(acc, a[2], b1.x, b1.y);
+      mma_16816(acc, a[3], b1.z, b1.w);
 #pragma unroll
       for (int i = 0; i < 4; ++i) sum[i] = fmaf(acc[i], UNSHRINK_F16, sum[i]);
     }
@@ -271,12 +275,16 @@ __device__ __forceinline__ void tile_task(const Params &P, const Ctx &c, uint32_
   }
 }
 
+// First k-step pair of part i of n of a row.  fp16: whole chains of four MMAs (two pairs), so that tile_task has no odd pair to
+// look out for (the branches cost the kernel 120 bytes of spills).
+__device__ __forceinline__ int k_split(int i, int n) { return FP8_ROWS ? KPAIRS * i / n : KPAIRS / 2 * i / n * 2; }
+
 // Per-warp work of a layer phase, fixed for the launch (computed once: the integer divisions behind it cost more
 // than the MMAs).  Phase rows = `groups` runs of `nch` consecutive chunks (q|k|v: one run; gate/up: the gate rows'
 // chunks, then the up rows'); tiles of 16 rows; when there are fewer tiles than warps, nkb warps share a tile's
 // 1024 inputs.  Grids of at least FUSED_MIN_CTAS CTAs have at most 6 tiles per phase: one task per warp.
 // fp16 rows: the tiles run on from the gate into the up rows (148 CTAs: 40 to 48 rows are three tiles, where the gate and
-// the up rows by themselves were two each, the second of them half empty; the MMAs of a sub-partition issue one at a time):
+// the up rows by themselves were two each, the second of them half empty; shared memory hands out a padded tile like a full one):
 // 523 / 535 / 568 -> 518 / 531 / 563 us per token at 64 / 1024 / 4096-token contexts (both with full lines of sums, see
 // RED_GROUP).  fp8 rows gained nothing at 1024 and lost 1 % at 64 and stay apart (their row conversions weigh more than the
 // MMAs).
@@ -291,8 +299,8 @@ __device__ inline void build_tile_tasks(TileTask *tasks, int *nkb_out, int group
     const int tile = w / nkb, kb = w - tile * nkb, grp = tile / tpg, tt = tile - grp * tpg;
     t.first = grp * nch + tt * TILE_CH;
     t.valid = min(16, (nch - tt * TILE_CH) * CH_ROWS);
-    t.p0 = (KPAIRS * kb) / nkb;
-    t.p1 = (KPAIRS * (kb + 1)) / nkb;
+    t.p0 = k_split(kb, nkb);
+    t.p1 = k_split(kb + 1, nkb);
     t.units = EMPTY_UNITS / nkb;
     t.pad0 = t.pad1 = 0;
   }
@@ -470,12 +478,7 @@ __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __ha
 #pragma unroll
   for (int t = 0; t < 8; ++t) { acc[t][0] = 0.f; acc[t][1] = 0.f; acc[t][2] = 0.f; acc[t][3] = 0.f; }
   float m = -INFINITY, l = 0.f;                        // running max / sum of this lane's head (quad = head, quads 2, 3 idle)
-  uint32_t qf[4][4];                                   // query operand fragments of the four 32-input pairs
-  {
-    const uint32_t q_addr = smem_u32(c.smem + OFF_QF + (c.lane & 3) * KV_PITCH) + (c.lane >> 3) * 16;   // rows 4..7 repeat 0..3
-#pragma unroll
-    for (int p = 0; p < 4; ++p) ldsm_x4(q_addr + p * 64, qf[p]);
-  }
+  const uint32_t q_addr = smem_u32(c.smem + OFF_QF + (c.lane & 3) * KV_PITCH) + (c.lane >> 3) * 16;   // rows 4..7 repeat 0..3
   const int lr = (c.lane & 7) + ((c.lane >> 3) & 1) * 8;
   const bool pass_gate = it.nchunks > NSLOTS;   // see attention_phase
 #pragma unroll 1
@@ -502,13 +505,27 @@ __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __ha
       const uint32_t k_xor = ((k_row >> 7) & 7u) << 4;               // swizzle of that row (the same in box 1: boxes are 2048 bytes)
       const uint32_t k_off = (c.lane >> 4) * 16;
 #pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        uint32_t a0[4], a1[4];
-        ldsm_x4(k_row + (p >> 1) * KV_BOX + ((((p & 1) * 64) + k_off) ^ k_xor), a0);
-        ldsm_x4(k_row + (p >> 1) * KV_BOX + ((((p & 1) * 64) + 32 + k_off) ^ k_xor), a1);
-        mma_16816(sc, a0, qf[p][0], qf[p][1]);
-        mma_16816(sc2, a1, qf[p][2], qf[p][3]);
+      for (int h = 0; h < 2; ++h) {       // a half's operands (the query's too: kept across chunks they cost 16 registers behind the softmax), then its products
+        uint32_t qf[2][4], ka[2][2][4];
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          ldsm_x4(q_addr + (2 * h + p) * 64, qf[p]);
+          ldsm_x4(k_row + h * KV_BOX + ((p * 64 + k_off) ^ k_xor), ka[p][0]);
+          ldsm_x4(k_row + h * KV_BOX + ((p * 64 + 32 + k_off) ^ k_xor), ka[p][1]);
+        }
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          mma_16816(sc, ka[p][0], qf[p][0], qf[p][1]);
+          mma_16816(sc2, ka[p][1], qf[p][2], qf[p][3]);
+        }
       }
+      // V operand of the first half: requested here, needed behind the softmax
+      const uint32_t v_row = base + KV_V_OFF + ((c.lane & 7) + 8 * (c.lane >> 4)) * 128;
+      const uint32_t v_xor = ((v_row >> 7) & 7u) << 4;
+      const uint32_t v_off = ((c.lane >> 3) & 1) * 16;
+      uint32_t va[4][4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) ldsm_x4_trans(v_row + ((t * 32 + v_off) ^ v_xor), va[t]);
       float s_top = fmaf(sc[0] + sc2[0], UNSHRINK_F16, (sc[1] + sc2[1]) * LO_INV) * sc_quad,
             s_bot = fmaf(sc[2] + sc2[2], UNSHRINK_F16, (sc[3] + sc2[3]) * LO_INV) * sc_quad;
       if (rowq >= nrow) s_top = -INFINITY;
@@ -539,14 +556,19 @@ __device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __ha
         b0 = pack_half2(split_half(pta, lo), split_half(ptb, lo));
         b1 = pack_half2(split_half(pba, lo), split_half(pbb, lo));
       }
-      const uint32_t v_row = base + KV_V_OFF + ((c.lane & 7) + 8 * (c.lane >> 4)) * 128;
-      const uint32_t v_xor = ((v_row >> 7) & 7u) << 4;
-      const uint32_t v_off = ((c.lane >> 3) & 1) * 16;
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        uint32_t a[4];
-        ldsm_x4_trans(v_row + (t >> 2) * KV_BOX + ((((t & 3) * 32) + v_off) ^ v_xor), a);
-        mma_add_16816(acc[t], a, b0, b1);
+      for (int t0 = 0; t0 < 8; t0 += 4) {   // four products in flight, then their adds
+        float d[4][4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) mma_16816_zero(d[t], va[t], b0, b1);
+        if (t0 == 0) {
+#pragma unroll
+          for (int t = 0; t < 4; ++t) ldsm_x4_trans(v_row + KV_BOX + ((t * 32 + v_off) ^ v_xor), va[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc[t0 + t][i] += d[t][i];
       }
     }
     __syncwarp();
@@ -778,31 +800,48 @@ __device__ __forceinline__ void slice_row_addresses(const Ctx &c, int nrows, uin
     arow[ks] = weight_rows(c, c.chunk + static_cast<uint32_t>(row / CH_ROWS)) + (row % CH_ROWS) * ROW_PITCH + (FP8_ROWS ? 0 : ((c.lane >> 3) & 1) * 16);
   }
 }
-// Output tiles t0 and t0 + 12 of a slice (past the end: a valid tile again, for the caller to ignore).
-__device__ __forceinline__ void slice_tiles(const uint32_t (&arow)[2], const uint32_t (&bq)[4], int t0, bool two, float (&acc)[2][4]) {
-  uint32_t a[2][4], a2[2][4];
+// Output tiles t0, t0 + 12, ... of a slice (past the end: the last tile again, for the caller to ignore): all operands
+// first, then all products, then the sums.
+constexpr int SLICE_TILES = (H / 16 + CONS_WARPS - 1) / CONS_WARPS;
+__device__ __forceinline__ void slice_tiles(const uint32_t (&arow)[2], const uint32_t (&bq)[4], int t0, bool two, float (&acc)[SLICE_TILES][4]) {
+  uint32_t a[SLICE_TILES][4];
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
+  for (int u = 0; u < SLICE_TILES; ++u) {
     const int tile = min(t0 + u * CONS_WARPS, H / 16 - 1);
-    acc[u][0] = 0.f; acc[u][1] = 0.f; acc[u][2] = 0.f; acc[u][3] = 0.f;
-    if (FP8_ROWS) {
-      uint32_t r[4];
-      ldsm_x4_trans(arow[0] + tile * 16, r);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) r[i] = __byte_perm(r[i], 0u, 0x3120);   // {row 2q, 2q + 1} of the first output, then of the second
-      e4m3x4_half2x2(r[0], a[u][0], a[u][1]);
-      e4m3x4_half2x2(r[1], a[u][2], a[u][3]);
-      e4m3x4_half2x2(r[2], a2[u][0], a2[u][1]);
-      e4m3x4_half2x2(r[3], a2[u][2], a2[u][3]);
-    } else {
-      ldsm_x4_trans(arow[0] + tile * 32, a[u]);
-      if (two) ldsm_x4_trans(arow[1] + tile * 32, a2[u]);
-    }
+    ldsm_x4_trans(arow[0] + tile * (FP8_ROWS ? 16 : 32), a[u]);
   }
+  if (FP8_ROWS) {
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    mma_add_16816(acc[u], a[u], bq[0], bq[1]);
-    if (two) mma_add_16816(acc[u], a2[u], bq[2], bq[3]);
+    for (int u = 0; u < SLICE_TILES; ++u) {
+      uint32_t r[4], a0[4], a1[4];
+      float d[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r[i] = __byte_perm(a[u][i], 0u, 0x3120);   // {row 2q, 2q + 1} of the first output, then of the second
+      e4m3x4_half2x2(r[0], a0[0], a0[1]);
+      e4m3x4_half2x2(r[1], a0[2], a0[3]);
+      e4m3x4_half2x2(r[2], a1[0], a1[1]);
+      e4m3x4_half2x2(r[3], a1[2], a1[3]);
+      mma_16816_zero(acc[u], a0, bq[0], bq[1]);
+      if (two) {
+        mma_16816_zero(d, a1, bq[2], bq[3]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[u][i] += d[i];
+      }
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < SLICE_TILES; ++u) mma_16816_zero(acc[u], a[u], bq[0], bq[1]);
+    if (two) {
+#pragma unroll
+      for (int u = 0; u < SLICE_TILES; ++u) ldsm_x4_trans(arow[1] + min(t0 + u * CONS_WARPS, H / 16 - 1) * 32, a[u]);
+      float d[SLICE_TILES][4];
+#pragma unroll
+      for (int u = 0; u < SLICE_TILES; ++u) mma_16816_zero(d[u], a[u], bq[2], bq[3]);
+#pragma unroll
+      for (int u = 0; u < SLICE_TILES; ++u)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[u][i] += d[u][i];
+    }
   }
 }
 
@@ -842,17 +881,18 @@ __device__ __noinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
     // lane that holds this lane's output (fragment row = lane / 4), and whether it is its second row
     const int src = FP8_ROWS ? ((c.lane & 15) >> 1) * 4 : (c.lane & 7) * 4;
     const bool second = (c.lane & (FP8_ROWS ? 1 : 8)) != 0;
-#pragma unroll 1
-    for (int t0 = c.warp; t0 < H / 16; t0 += 2 * CONS_WARPS) {
-      float acc[2][4];
-      slice_tiles(arow, bq, t0, two, acc);
+    float acc[SLICE_TILES][4];
+    slice_tiles(arow, bq, c.warp, two, acc);
+    static_assert(SLICE_TILES % 2 == 0, "tiles leave in pairs");
+#pragma unroll
+    for (int u = 0; u < SLICE_TILES; u += 2) {
       // lanes of quad 0 hold (hi, lo) sums of fragment rows lane / 4 and lane / 4 + 8 of both tiles; lane L takes output
       // L % 16 of tile L / 16
-      const float s0 = __shfl_sync(0xffffffffu, fmaf(acc[0][1], LO_INV, acc[0][0]), src);
-      const float s1 = __shfl_sync(0xffffffffu, fmaf(acc[0][3], LO_INV, acc[0][2]), src);
-      const float s2 = __shfl_sync(0xffffffffu, fmaf(acc[1][1], LO_INV, acc[1][0]), src);
-      const float s3 = __shfl_sync(0xffffffffu, fmaf(acc[1][3], LO_INV, acc[1][2]), src);
-      const int tile = t0 + (c.lane >> 4) * CONS_WARPS;
+      const float s0 = __shfl_sync(0xffffffffu, fmaf(acc[u][1], LO_INV, acc[u][0]), src);
+      const float s1 = __shfl_sync(0xffffffffu, fmaf(acc[u][3], LO_INV, acc[u][2]), src);
+      const float s2 = __shfl_sync(0xffffffffu, fmaf(acc[u + 1][1], LO_INV, acc[u + 1][0]), src);
+      const float s3 = __shfl_sync(0xffffffffu, fmaf(acc[u + 1][3], LO_INV, acc[u + 1][2]), src);
+      const int tile = c.warp + (u + (c.lane >> 4)) * CONS_WARPS;
       if (tile < H / 16) {
         const int n = tile * 16 + (c.lane & 15);
         float v = ((c.lane & 16) ? (second ? s3 : s2) : (second ? s1 : s0)) * up;
@@ -882,7 +922,7 @@ __device__ __noinline__ uint32_t lm_head_tc(const Params &P, Ctx c, float *dump)
   float *part = tc_part(c), *s_misc = c.f(F_MISC);
   float best = -INFINITY;
   int best_i = 0x7fffffff;
-  const int p0 = (KPAIRS * c.warp) / CONS_WARPS, p1 = (KPAIRS * (c.warp + 1)) / CONS_WARPS;
+  const int p0 = k_split(c.warp, CONS_WARPS), p1 = k_split(c.warp + 1, CONS_WARPS);
   const float up = s_misc[M_XSCALE];
 #pragma unroll 1
   for (int tile = 0; tile < ntiles; ++tile) {

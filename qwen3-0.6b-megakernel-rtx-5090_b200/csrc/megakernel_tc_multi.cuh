@@ -181,24 +181,21 @@ __device__ __noinline__ uint32_t slice_cols_seqs(const Params &P, Ctx c, int whi
     const float *resid = tc_resid(c, which ^ 1, live ? b : 0);   // O slice: x, down slice: x1
     float *prev = tc_prev(c, which, live ? b : 0);
     unsigned long long *sum = P.red + (which * TC_SEQS + (live ? b : 0)) * RED_SUM_WORDS;
-#pragma unroll 1
-    for (int t0 = c.warp; t0 < H / 16; t0 += 2 * CONS_WARPS) {
-      float acc[2][4];
-      slice_tiles(arow, bq, t0, two, acc);
+    float acc[SLICE_TILES][4];
+    slice_tiles(arow, bq, c.warp, two, acc);
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int tile = t0 + u * CONS_WARPS;
-        if (live && tile < H / 16) {
+    for (int u = 0; u < SLICE_TILES; ++u) {
+      const int tile = c.warp + u * CONS_WARPS;
+      if (live && tile < H / 16) {
 #pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const int n = tile * 16 + (FP8_ROWS ? 2 * j + k : j + 8 * k);
-            float v = fmaf(acc[u][2 * k + 1], LO_INV, acc[u][2 * k]) * up;
-            if (FP8_ROWS) v *= scales[n];
-            if (n >= n0 && n < n1) v += resid[n - n0];
-            const long long fx = __float2ll_rn(v * RED_SCALE), fx_prev = __float2ll_rn(prev[n] * RED_SCALE);
-            prev[n] = v;
-            red_add_u64(sum + red_index(n), (static_cast<unsigned long long>(fx - fx_prev) << RED_CNT_BITS) + 1ull);
-          }
+        for (int k = 0; k < 2; ++k) {
+          const int n = tile * 16 + (FP8_ROWS ? 2 * j + k : j + 8 * k);
+          float v = fmaf(acc[u][2 * k + 1], LO_INV, acc[u][2 * k]) * up;
+          if (FP8_ROWS) v *= scales[n];
+          if (n >= n0 && n < n1) v += resid[n - n0];
+          const long long fx = __float2ll_rn(v * RED_SCALE), fx_prev = __float2ll_rn(prev[n] * RED_SCALE);
+          prev[n] = v;
+          red_add_u64(sum + red_index(n), (static_cast<unsigned long long>(fx - fx_prev) << RED_CNT_BITS) + 1ull);
         }
       }
     }
@@ -333,7 +330,7 @@ __device__ __noinline__ uint32_t lm_head_seqs(const Params &P, Ctx c, int step, 
   float *part = tc_part(c);
   float best = -INFINITY;
   int best_i = 0x7fffffff;
-  const int p0 = (KPAIRS * c.warp) / CONS_WARPS, p1 = (KPAIRS * (c.warp + 1)) / CONS_WARPS;
+  const int p0 = k_split(c.warp, CONS_WARPS), p1 = k_split(c.warp + 1, CONS_WARPS);
   const int b = c.tid >> 4, r = c.tid & 15;
   const float up = c.f(F_MISC)[M_XSCALE];
   float *dump = (P.logits_out && b < P.nseq) ? P.logits_out + (static_cast<size_t>(b) * P.num_steps + step) * P.vocab : nullptr;
