@@ -225,7 +225,7 @@ __device__ __noinline__ uint32_t slice_colgemv(const Params &P, Ctx c, int which
 // act16 (tensor-core build): also leave the outputs as fp16 hi / scaled-lo halves at act16[i] / act16[ACT16_PITCH + i],
 // zero from the slice's end up to 32.
 constexpr int ACT16_PITCH = 72;                // halves between the hi and the lo row (64 + 8: other banks)
-__device__ __noinline__ void merge_slice(const Params &P, const Ctx c, int S, uint32_t tag, __half *act16 = nullptr) {
+__device__ __forceinline__ void merge_slice(const Params &P, const Ctx c, int S, uint32_t tag, __half *act16 = nullptr) {
   float *s_attn = c.f(FF_ATTN), *s_wt = c.f(FF_SPLITW);
   const int e0 = c.segs()->e0, e1 = c.segs()->e1;
   const int h0 = e0 >> 7;
@@ -386,7 +386,7 @@ __device__ __noinline__ float embed_row(const Params &P, const Ctx c, int token)
 // Argmax across the grid (megakernel_5090.cu:1137-1167): every CTA publishes the best (value, row) of its LM-head
 // rows (left per warp in s_misc[32..], s_misc[48..]), reads all CTAs' pairs and leaves the winning row, lowest
 // index on ties, in s_misc[16].  Entered after a consumer barrier.
-__device__ __noinline__ void argmax_exchange(const Params &P, const Ctx c, uint32_t atag) {
+__device__ __forceinline__ void argmax_exchange(const Params &P, const Ctx c, uint32_t atag) {
   float *s_misc = c.f(F_MISC), *s_amax = c.f(F_AMAX);
   if (c.tid == 0) {
     float best = s_misc[32];

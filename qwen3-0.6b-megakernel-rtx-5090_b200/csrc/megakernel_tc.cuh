@@ -313,9 +313,14 @@ __device__ __forceinline__ void run_tile_task(const Params &P, const Ctx &c, con
   if (a.x) tile_task(P, c, c.chunk + static_cast<uint32_t>(a.y), a.z, a.w, b.x, tc_part(c) + c.warp * PART_TASK, b.y, fslot);
 }
 
+// The phases are inlined into the kernel's layer loop.  As functions of their own they cost a call and its register moves (160
+// cycles, ten times a layer) and read every launch parameter through memory; inlined, parameters are constant-bank operands and
+// a phase keeps 128 registers for itself: a step of one fp16 sequence at 64 / 1024 / 4096 tokens 486 / 491 / 518 -> 433 / 446 / 492
+// us, one with FP8 rows at 1024 491 -> 430, two fp16 at 512 568 -> 525, four at 1024 795 -> 748, four FP8 820 -> 781.  (The two call sites of slice_cols and red_wait_norm
+// do not hurt: a phase repeated at once, its code hot, takes as long as the first time.)
 #if QMK_TC_SEQS == 1
 // q|k|v rows of this CTA -> exchange words (megakernel_5090.cu:251-302).
-__device__ __noinline__ uint32_t qkv_phase(const Params &P, Ctx c, uint32_t tag) {
+__device__ __forceinline__ uint32_t qkv_phase(const Params &P, Ctx c, uint32_t tag) {
   const TcTab *t = tctab(c);
   const int nch = t->nq, nkb = t->nkb_qkv;
   QMK_FINE(0);
@@ -336,7 +341,7 @@ __device__ __noinline__ uint32_t qkv_phase(const Params &P, Ctx c, uint32_t tag)
 }
 
 // gate/up rows of this CTA -> silu(gate) * up in shared memory (megakernel_5090.cu:653-685, SiLU in fp32).
-__device__ __noinline__ uint32_t gateup_phase(const Params &P, Ctx c) {
+__device__ __forceinline__ uint32_t gateup_phase(const Params &P, Ctx c) {
   const TcTab *t = tctab(c);
   const int nch = t->ng, nkb = t->nkb_gu;
   QMK_FINE(10);
@@ -398,7 +403,7 @@ __device__ __forceinline__ AttnItem tc_item(const Params &P, const Ctx &c, int p
 // online softmax on the accumulator fragments (log2 domain), then out[128 x 4] += V^T[128 x 16] . p[16 x 4] as 8
 // MMAs with V read through ldmatrix.trans and p split into hi/lo fp16 columns like q: ~75 instructions per 16
 // rows where the CUDA-core loop needs ~480.
-__device__ __noinline__ uint32_t attention_tc(const Params &P, Ctx c, const __half *nv, int layer, int pos, uint32_t tag) {
+__device__ __forceinline__ uint32_t attention_tc(const Params &P, Ctx c, const __half *nv, int layer, int pos, uint32_t tag) {
   const AttnItem it = tc_item(P, c, pos);
   float *s_q = c.f(F_Q), *s_knew = c.f(F_KNEW), *s_vnew = c.f(F_VNEW), *s_wpart = c.f(F_WPART), *s_misc = c.f(F_MISC);
   const float *s_cs = c.f(F_CS);
@@ -667,7 +672,7 @@ __device__ __forceinline__ void store_normalised(const Ctx &c, int n, float v, f
 // to shared memory (which = 0: x1; 1: x, the next input) and RMS-normalises them with `norm_w` (fp16[1024], shared
 // or global) into the hi/lo halves the tile products read.  emit: CTA 0 also writes the reference-signature outputs
 // (final-norm result fp32, last hidden state fp16).  Ends with a consumer barrier.
-__device__ __noinline__ void red_wait_norm(const Params &P, const Ctx c, int which, uint32_t use, const __half *norm_w, int emit) {
+__device__ __forceinline__ void red_wait_norm(const Params &P, const Ctx c, int which, uint32_t use, const __half *norm_w, int emit) {
   constexpr int PT = (H + CONS_THREADS - 1) / CONS_THREADS;
   const unsigned long long *buf = P.red + (which ? RED_X2 : RED_X1);
   float *dst = c.f(which ? F_X : F_X1);
@@ -764,7 +769,7 @@ __device__ __forceinline__ float embed_value(const unsigned char *erow, int n) {
 
 #if QMK_TC_SEQS == 1
 // Embedding row of `token` (megakernel_5090.cu:825-830) -> residual stream, normalised with layer 0's input norm.
-__device__ __noinline__ void embed_norm(const Params &P, const Ctx c, int token, const __half *norm_w) {
+__device__ __forceinline__ void embed_norm(const Params &P, const Ctx c, int token, const __half *norm_w) {
   constexpr int PT = (H + CONS_THREADS - 1) / CONS_THREADS;
   const unsigned char *erow = reinterpret_cast<const unsigned char *>(P.embed) + static_cast<size_t>(token) * ROW_BYTES;
   float v[PT], w[PT], ss = 0.f;
@@ -853,7 +858,7 @@ __device__ __forceinline__ void slice_tiles(const uint32_t (&arow)[2], const uin
 // slice, so a partial is complete when it leaves the warp: after each pair of tiles the 32 sums are spread over
 // the 32 lanes (four shuffles) and every lane adds its one output into the residual sum - no staging in shared
 // memory, no barrier, and the adds of early tiles drain while later tiles are computed.
-__device__ __noinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
+__device__ __forceinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
   const SegTab *t = c.segs();
   const int nrows = which ? tctab(c)->ng * CH_ROWS : t->e1 - t->e0;
   const float *resid = c.f(which ? F_X1 : F_X);
@@ -916,7 +921,7 @@ __device__ __noinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
 // twenty chunks, which leaves sixteen in flight (the stream needs bandwidth x latency = ~130 KB per SM in flight;
 // rounds of three tiles left eight and ran at 3.4 TB/s).  Leaves the per-warp results that argmax_exchange()
 // expects in s_misc[32..43] / s_misc[48..59].
-__device__ __noinline__ uint32_t lm_head_tc(const Params &P, Ctx c, float *dump) {
+__device__ __forceinline__ uint32_t lm_head_tc(const Params &P, Ctx c, float *dump) {
   const TcTab *t = tctab(c);
   const int nch = t->nlm, ntiles = (nch + TILE_CH - 1) / TILE_CH;
   float *part = tc_part(c), *s_misc = c.f(F_MISC);
@@ -1010,7 +1015,14 @@ __device__ __forceinline__ ChunkSrc scale_chunk(const void *base, int rows) {
   return d;
 }
 
-__device__ __noinline__ void producer_main_tc(const Params &P, const Ctx c) {
+// (A function of its own for one sequence, inlined for several: 434 against 442 us per step of one fp16 sequence at 64 tokens, 812
+// against 748 of four at 1024.)
+#if QMK_TC_SEQS == 1
+__device__ __noinline__
+#else
+__device__ __forceinline__
+#endif
+void producer_main_tc(const Params &P, const Ctx c) {
   const uint64_t pol = P.l2_evict_first ? l2_evict_first_policy() : l2_evict_normal_policy();
   const SegTab *t = c.segs();
   const TcTab *tt = tctab(c);

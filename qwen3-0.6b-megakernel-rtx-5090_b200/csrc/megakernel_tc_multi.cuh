@@ -36,7 +36,7 @@ __device__ __forceinline__ float *tc_resid(const Ctx &c, int which, int b) {
 }
 __device__ __forceinline__ int *tc_tokens(const Ctx &c) { return reinterpret_cast<int *>(c.smem + OFF_TOKENS); }
 
-__device__ __noinline__ uint32_t qkv_phase_seqs(const Params &P, Ctx c, uint32_t tag) {
+__device__ __forceinline__ uint32_t qkv_phase_seqs(const Params &P, Ctx c, uint32_t tag) {
   const TcTab *t = tctab(c);
   const int nch = t->nq, nkb = t->nkb_qkv;
   run_tile_task(P, c, t->qkv, 0);
@@ -53,7 +53,7 @@ __device__ __noinline__ uint32_t qkv_phase_seqs(const Params &P, Ctx c, uint32_t
   return c.chunk + static_cast<uint32_t>(nch);
 }
 
-__device__ __noinline__ uint32_t gateup_phase_seqs(const Params &P, Ctx c) {
+__device__ __forceinline__ uint32_t gateup_phase_seqs(const Params &P, Ctx c) {
   const TcTab *t = tctab(c);
   const int nch = t->ng, nkb = t->nkb_gu;
   run_tile_task(P, c, t->gu, 10);
@@ -85,7 +85,7 @@ __device__ __noinline__ uint32_t gateup_phase_seqs(const Params &P, Ctx c) {
 
 // merge_slice (megakernel_fused.cuh) for all sequences at once: lanes LPS * b .. + LPS - 1 of a warp are the splits of
 // sequence b, so a warp still takes elements e0 + warp, + 12, ... and every element's sequences complete together.
-__device__ __noinline__ void merge_seqs(const Params &P, const Ctx c, int step, uint32_t tag) {
+__device__ __forceinline__ void merge_seqs(const Params &P, const Ctx c, int step, uint32_t tag) {
   float *s_wt = reinterpret_cast<float *>(c.smem + OFF_SPLITW);      // [2 heads][32 lanes]
   const int e0 = c.segs()->e0, e1 = c.segs()->e1, h0 = e0 >> 7;
   const int b = c.lane / LPS, sl = c.lane % LPS;
@@ -157,7 +157,7 @@ __device__ __noinline__ void merge_seqs(const Params &P, const Ctx c, int step, 
 
 // slice_cols for all sequences: quad q of a fragment holds sequence q's hi and lo sums of two outputs, which its lanes
 // scale and add into that sequence's residual sum where they are.
-__device__ __noinline__ uint32_t slice_cols_seqs(const Params &P, Ctx c, int which) {
+__device__ __forceinline__ uint32_t slice_cols_seqs(const Params &P, Ctx c, int which) {
   const SegTab *t = c.segs();
   const int nrows = which ? tctab(c)->ng * CH_ROWS : t->e1 - t->e0;
   const int nch = (nrows + CH_ROWS - 1) / CH_ROWS + SCALE_CH;
@@ -257,7 +257,7 @@ __device__ __forceinline__ void normalise_seqs(const Ctx &c, const float (&v)[TC
 // One sequence gains nothing.
 constexpr unsigned long long SUM_SLACK = 48;
 // red_wait_norm for all sequences: which = 0: x1, 1: x2 (kept as the residual of the next layer's O slice, x).
-__device__ __noinline__ void red_wait_norm_seqs(const Params &P, const Ctx c, int which, uint32_t use, const __half *norm_w) {
+__device__ __forceinline__ void red_wait_norm_seqs(const Params &P, const Ctx c, int which, uint32_t use, const __half *norm_w) {
   const unsigned long long base = static_cast<unsigned long long>(use) * static_cast<unsigned long long>(c.ncta);
   const unsigned long long *src = P.red + static_cast<size_t>(which) * TC_SEQS * RED_SUM_WORDS + red_index(c.tid);
   if (c.lane == 0) {   // one lane per warp watches one word (see red_wait_norm)
@@ -308,7 +308,7 @@ __device__ __noinline__ void red_wait_norm_seqs(const Params &P, const Ctx c, in
   normalise_seqs(c, v, which, norm_w);
 }
 
-__device__ __noinline__ void embed_norm_seqs(const Params &P, const Ctx c, const __half *norm_w) {
+__device__ __forceinline__ void embed_norm_seqs(const Params &P, const Ctx c, const __half *norm_w) {
   float v[TC_SEQS][VPT];
 #pragma unroll
   for (int b = 0; b < TC_SEQS; ++b) {
@@ -324,7 +324,7 @@ __device__ __noinline__ void embed_norm_seqs(const Params &P, const Ctx c, const
 
 // lm_head_tc for all sequences: thread 16 b + r finishes row r of every tile for sequence b and keeps its running best;
 // the sixteen lanes of a sequence then agree and publish the CTA's pair.
-__device__ __noinline__ uint32_t lm_head_seqs(const Params &P, Ctx c, int step, uint32_t atag) {
+__device__ __forceinline__ uint32_t lm_head_seqs(const Params &P, Ctx c, int step, uint32_t atag) {
   const TcTab *t = tctab(c);
   const int nch = t->nlm, ntiles = (nch + TILE_CH - 1) / TILE_CH;
   float *part = tc_part(c);
@@ -370,7 +370,7 @@ __device__ __noinline__ uint32_t lm_head_seqs(const Params &P, Ctx c, int step, 
 }
 
 // argmax_exchange for all sequences: the winning rows end up in tc_tokens().
-__device__ __noinline__ void argmax_seqs(const Params &P, const Ctx c, uint32_t atag) {
+__device__ __forceinline__ void argmax_seqs(const Params &P, const Ctx c, uint32_t atag) {
   float *s_amax = c.f(F_WPART);                     // [sequence][2 * MAX_CTAS], free outside the attention phase
   const int b = c.tid / TPS;
   if (b < P.nseq) {
