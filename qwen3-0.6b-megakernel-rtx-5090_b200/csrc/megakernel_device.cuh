@@ -362,6 +362,37 @@ __device__ __forceinline__ void ll_wait_many(const Params &P, const Ctx &c, cons
 #pragma unroll
   for (int j = 0; j < NW; ++j) out[j] = __uint_as_float(static_cast<uint32_t>(w[j]));
 }
+// The same with word offsets from one base: half the address registers.
+template <int NW>
+__device__ __forceinline__ void ll_wait_words(const Params &P, const Ctx &c, const unsigned long long *base, const uint32_t (&p)[NW],
+                                             uint32_t valid, uint32_t tag, float (&out)[NW]) {
+  unsigned long long w[NW];
+#pragma unroll
+  for (int j = 0; j < NW; ++j)
+    if (valid & (1u << j)) w[j] = ll_load(base + p[j]);
+  uint32_t pending = valid;
+  unsigned long long t0 = 0;
+  uint32_t it = 0;
+  for (;;) {
+#pragma unroll
+    for (int j = 0; j < NW; ++j)
+      if ((pending & (1u << j)) && static_cast<uint32_t>(w[j] >> 32) == tag) pending &= ~(1u << j);
+    if (pending == 0u) break;
+    if (P.spin_sleep_ns) __nanosleep(P.spin_sleep_ns);
+#pragma unroll
+    for (int j = 0; j < NW; ++j)
+      if (pending & (1u << j)) w[j] = ll_load(base + p[j]);
+    if ((++it & 255u) == 0u) {
+      if (c.flags()[0]) break;
+      if (ld_relaxed_u32(P.status) != 0u) { c.flags()[0] = 1; break; }
+      const unsigned long long t = now_ns();
+      if (t0 == 0) t0 = t;
+      if (t - t0 > P.timeout_ns) { raise_error(P, c, QMK_ERR_WAIT_TIMEOUT, WHERE_LL); break; }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < NW; ++j) out[j] = __uint_as_float(static_cast<uint32_t>(w[j]));
+}
 
 // Wait on an mbarrier phase with the same bounds.  Returns false after an abort (or, for the
 // producer, after the consumers said stop).

@@ -222,10 +222,8 @@ __device__ __noinline__ uint32_t slice_colgemv(const Params &P, Ctx c, int which
 // heads' splits and turn them into one weight per split, exp2(max_s - max) / sum; meanwhile every warp fetches
 // the unnormalised outputs of its elements (lanes = splits, up to three elements per warp, all words polled
 // together).  After a barrier an element is the weighted sum over its splits.
-// act16 (tensor-core build): also leave the outputs as fp16 hi / scaled-lo halves at act16[i] / act16[ACT16_PITCH + i],
-// zero from the slice's end up to 32.
-constexpr int ACT16_PITCH = 72;                // halves between the hi and the lo row (64 + 8: other banks)
-__device__ __forceinline__ void merge_slice(const Params &P, const Ctx c, int S, uint32_t tag, __half *act16 = nullptr) {
+#ifndef QMK_TC_BUILD
+__device__ __noinline__ void merge_slice(const Params &P, const Ctx c, int S, uint32_t tag) {
   float *s_attn = c.f(FF_ATTN), *s_wt = c.f(FF_SPLITW);
   const int e0 = c.segs()->e0, e1 = c.segs()->e1;
   const int h0 = e0 >> 7;
@@ -242,11 +240,6 @@ __device__ __forceinline__ void merge_slice(const Params &P, const Ctx c, int S,
   }
   float a[NE];
   QMK_FINE(50);
-#ifdef QMK_TC_BUILD
-  // the owner split (the last one) also handles the new row: its words arrive last
-  ll_sentinel(P, c, c.llr + LL_PART + static_cast<size_t>((min(e0 + c.warp, e1 - 1) >> 7) * MAX_SPLITS + S - 1) * PART_STRIDE +
-                        (min(e0 + c.warp, e1 - 1) & (D - 1)), tag);
-#endif
   const int hw = h0 + (c.warp - (CONS_WARPS - 2));                // head whose split weights this warp makes (last two warps)
   if (c.warp >= CONS_WARPS - 2 && hw <= ((e1 - 1) >> 7)) {        // warp-uniform
     // outputs and the head's (max, sum) pairs in ONE round of polls (one after the other costs a second L2 round trip)
@@ -283,19 +276,10 @@ __device__ __forceinline__ void merge_slice(const Params &P, const Ctx c, int S,
 #pragma unroll
   for (int q = 0; q < NE; ++q) {
     const int e = e0 + c.warp + q * CONS_WARPS;
-    if (e < e1 && c.lane == 0) {
-      s_attn[e - e0] = A[q];
-      if (act16) {
-        const __half h = __float2half_rn(A[q]);
-        act16[e - e0] = h;
-        act16[ACT16_PITCH + e - e0] = __float2half_rn((A[q] - __half2float(h)) * 2048.0f);
-      }
-    }
+    if (e < e1 && c.lane == 0) s_attn[e - e0] = A[q];
   }
-  if (act16 && c.tid < 32 && c.tid >= e1 - e0) { act16[c.tid] = __float2half_rn(0.f); act16[ACT16_PITCH + c.tid] = __float2half_rn(0.f); }
 }
 
-#ifndef QMK_TC_BUILD
 __device__ __forceinline__ bool produce_rows(const Params &P, const Ctx &c, uint32_t &idx, uint64_t pol, const unsigned char *src,
                                              int nrows, int row_bytes) {
 #pragma unroll 1

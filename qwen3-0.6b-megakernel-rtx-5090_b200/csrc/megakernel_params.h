@@ -19,6 +19,10 @@ struct __align__(16) LayerW {
 // W_o[:, e], row m of wd_t holds W_down[:, m] (1024 outputs each), so that the rows a CTA needs for ITS slice of
 // the input form one contiguous range.  fp8 format: 1024 e4m3 bytes + 16 unused bytes per row (a
 // conflict-free pitch in shared memory), the per-output fp32 scales of the matrix follow the last row.
+// The tensor-core kernels read wo_t by quarters instead (O_GROUP CTAs share an input slice of the O projection, see
+// megakernel_tc.cuh): [4 quarters of the outputs][2048 rows][256 outputs + 16 unused bytes], the pitch a chunk of rows has in
+// shared memory, so that it is one copy.
+constexpr int O_GROUP = 4, O_COLS = 1024 / O_GROUP, O_PAD = 16;
 struct __align__(16) LayerT {
   const void *wo_t, *wd_t;
 };

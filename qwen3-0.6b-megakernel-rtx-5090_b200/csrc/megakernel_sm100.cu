@@ -96,6 +96,7 @@ struct PrepArgs {
   const qmkp::LayerT *out;        // destinations (device)
   unsigned long long *fp;         // [2][2 * num_layers] hashes of the samples, [2][2 * num_layers] of all bytes, [2 * num_layers] sums being formed
   int num_layers, wfmt, parity, force;
+  int quarters;                   // O rows by quarters of the outputs, as the tensor-core kernels read them (LayerT)
   int all, all_parity;            // compare the hashes of all bytes too (kmajor_hash_kernel ran before)
 };
 __device__ __forceinline__ const unsigned char *prep_matrix(const PrepArgs &a, int m) {
@@ -172,9 +173,13 @@ __global__ void __launch_bounds__(256) kmajor_prepare_kernel(const PrepArgs a) {
   __syncthreads();
   if (!s_redo) return;
   const int tx = t & 31, ty = t >> 5;                 // 32 x 8 threads, four rows each per tile
+  // Output n of row k lies at element k * pitch + n; by quarters (a tile of 32 lies in one): row n / 256 * K + k of 256 outputs.
+  const bool quarters = a.quarters && which == 0;
+  const int pitch = quarters ? (a.wfmt ? qmkp::O_COLS + qmkp::O_PAD : qmkp::O_COLS + qmkp::O_PAD / 2) : a.wfmt ? FP8_PITCH : H;
   const int ntiles = (H / 32) * (K / 32);
   for (int tile = blockIdx.x; tile < ntiles; tile += PREP_SUB) {
     const int tn = tile % (H / 32), tk = tile / (H / 32);
+    const int row0 = tk * 32 + (quarters ? tn * 32 / qmkp::O_COLS * K : 0), col0 = quarters ? tn * 32 % qmkp::O_COLS : tn * 32;
     if (a.wfmt == 0) {
       const unsigned short *in = reinterpret_cast<const unsigned short *>(src);
       unsigned short *out = reinterpret_cast<unsigned short *>(dst);
@@ -182,18 +187,18 @@ __global__ void __launch_bounds__(256) kmajor_prepare_kernel(const PrepArgs a) {
       for (int i = 0; i < 4; ++i) tile16[ty + 8 * i][tx] = in[static_cast<size_t>(tn * 32 + ty + 8 * i) * K + tk * 32 + tx];
       __syncthreads();
 #pragma unroll
-      for (int i = 0; i < 4; ++i) out[static_cast<size_t>(tk * 32 + ty + 8 * i) * H + tn * 32 + tx] = tile16[tx][ty + 8 * i];
+      for (int i = 0; i < 4; ++i) out[static_cast<size_t>(row0 + ty + 8 * i) * pitch + col0 + tx] = tile16[tx][ty + 8 * i];
     } else {
 #pragma unroll
       for (int i = 0; i < 4; ++i) tile8[ty + 8 * i][tx] = src[static_cast<size_t>(tn * 32 + ty + 8 * i) * in_row + tk * 32 + tx];
       __syncthreads();
 #pragma unroll
-      for (int i = 0; i < 4; ++i) dst[static_cast<size_t>(tk * 32 + ty + 8 * i) * FP8_PITCH + tn * 32 + tx] = tile8[tx][ty + 8 * i];
+      for (int i = 0; i < 4; ++i) dst[static_cast<size_t>(row0 + ty + 8 * i) * pitch + col0 + tx] = tile8[tx][ty + 8 * i];
     }
     __syncthreads();
   }
   if (a.wfmt && blockIdx.x == 0) {                    // per-output scales follow the K rows
-    float *sc = reinterpret_cast<float *>(dst + static_cast<size_t>(K) * FP8_PITCH);
+    float *sc = reinterpret_cast<float *>(dst + static_cast<size_t>(quarters ? qmkp::O_GROUP * K : K) * pitch);
     for (int n = t; n < H; n += 256) sc[n] = *reinterpret_cast<const float *>(src + static_cast<size_t>(n) * in_row + K);
   }
 }
@@ -258,6 +263,7 @@ struct Engine {
   struct Prepared {          // K-major copies of W_o / W_down of one caller table
     const void *table = nullptr;
     int num_layers = 0, wfmt = 0, parity = 0, all_parity = 0, force = 1;
+    bool quarters = false;   // O rows by quarters of the outputs
     unsigned char *buf = nullptr;
     qmkp::LayerT *tbl = nullptr;
     unsigned long long *fp = nullptr;
@@ -400,8 +406,9 @@ int ensure_rope(Engine *e, int max_seq_len, cudaStream_t stream) {
 }
 
 // Bytes of the K-major copies of one layer: O rows then down rows (fp8: each followed by 1024 fp32 scales).
-size_t kmajor_o_bytes(int wfmt) {
-  const size_t b = wfmt ? static_cast<size_t>(qmk::QS) * qmk::FP8_PITCH + qmk::H * 4 : static_cast<size_t>(qmk::QS) * qmk::H * 2;
+size_t kmajor_o_bytes(int wfmt, bool quarters) {
+  const size_t row = quarters ? qmkp::O_GROUP * (qmkp::O_COLS * (wfmt ? 1 : 2) + qmkp::O_PAD) : wfmt ? qmk::FP8_PITCH : qmk::H * 2;
+  const size_t b = qmk::QS * row + (wfmt ? qmk::H * 4 : 0);
   return (b + 255) / 256 * 256;
 }
 size_t kmajor_d_bytes(int wfmt) {
@@ -419,10 +426,11 @@ constexpr size_t MAX_PREPARED = 4;   // weight sets kept per device (a 28-layer 
 // Finds or creates the K-major copies for the caller's layer table and enqueues the check-and-rebuild kernel.
 // `several` (sequences): every byte of the matrices is checked, and where the copies do not fit in memory *out stays null
 // instead of an error.
-int ensure_prepared(Engine *e, const Params &P, int wfmt, cudaStream_t stream, Engine::Prepared **out, bool several = false) {
+// `quarters`: the layout of the tensor-core kernels (a set of its own, as each weight format is).
+int ensure_prepared(Engine *e, const Params &P, int wfmt, bool quarters, cudaStream_t stream, Engine::Prepared **out, bool several = false) {
   Engine::Prepared *hit = nullptr;
   for (auto &p : e->prepared)
-    if (p.table == P.layers && p.num_layers == P.num_layers && p.wfmt == wfmt) hit = &p;
+    if (p.table == P.layers && p.num_layers == P.num_layers && p.wfmt == wfmt && p.quarters == quarters) hit = &p;
   if (!hit) {
     if (e->prepared.size() >= MAX_PREPARED) {   // drop the set used longest ago
       size_t victim = 0;
@@ -436,7 +444,8 @@ int ensure_prepared(Engine *e, const Params &P, int wfmt, cudaStream_t stream, E
     p.table = P.layers;
     p.num_layers = P.num_layers;
     p.wfmt = wfmt;
-    const size_t ob = kmajor_o_bytes(wfmt), db = kmajor_d_bytes(wfmt);
+    p.quarters = quarters;
+    const size_t ob = kmajor_o_bytes(wfmt, quarters), db = kmajor_d_bytes(wfmt);
     if (const cudaError_t err = cudaMalloc(&p.buf, (ob + db) * P.num_layers); err != cudaSuccess) {
       cudaGetLastError();
       if (several && err == cudaErrorMemoryAllocation) return QMK_OK;
@@ -462,6 +471,7 @@ int ensure_prepared(Engine *e, const Params &P, int wfmt, cudaStream_t stream, E
   a.fp = hit->fp;
   a.num_layers = P.num_layers;
   a.wfmt = wfmt;
+  a.quarters = quarters ? 1 : 0;
   a.parity = hit->parity;
   a.force = hit->force;
   a.all = several ? 1 : 0;
@@ -570,7 +580,7 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
     const qmk_fused_tc::Build &tc = qmk_fused_tc::build_seqs(e->wfmt, P.nseq);
     Engine::Prepared *prep = nullptr;
     if (P.vocab % tc.rows_per_chunk == 0 && grid >= tc.min_ctas && grid <= tc.max_ctas) {
-      rc = ensure_prepared(e, P, e->wfmt, stream, &prep, true);
+      rc = ensure_prepared(e, P, e->wfmt, true, stream, &prep, true);
       if (rc != QMK_OK) return rc;
     }
     if (prep) {
@@ -587,8 +597,13 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
   if (!batch && e->fused && grid >= qmk::FUSED_MIN_CTAS &&
       kernel == reinterpret_cast<const void *>(qmk::qwen3_decode_megakernel)) {
     // fused kernel: O and down projections as split-K slices of K-major copies, two all-reduced residual sums
+    // Row products on the tensor cores: rows owned in units of one ring chunk (four fp16 rows, eight fp8 rows).  fp8:
+    // 724 -> 493 us per token at 1024-token contexts against the CUDA-core kernel, which stays for the grids and
+    // vocabularies outside these limits.
+    const qmk_fused_tc::Build &tc = qmk_fused_tc::build(e->wfmt);
+    const bool on_tensor_cores = e->fused >= 2 && P.vocab % tc.rows_per_chunk == 0 && grid >= tc.min_ctas && grid <= tc.max_ctas;
     Engine::Prepared *prep = nullptr;
-    rc = ensure_prepared(e, P, e->wfmt, stream, &prep);
+    rc = ensure_prepared(e, P, e->wfmt, on_tensor_cores, stream, &prep);
     if (rc != QMK_OK) return rc;
     QMK_CUDA(e, cudaMemsetAsync(e->red, 0, sizeof(unsigned long long) * qmk::RED_WORDS, stream));
     P.layers_t = prep->tbl;
@@ -596,11 +611,7 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
     P.red_copies = e->red_copies;
     P.spin_sleep_ns = e->fused_sleep_ns;
     kernel = reinterpret_cast<const void *>(qmk::qwen3_decode_megakernel_fused);
-    // row products on the tensor cores: rows owned in units of one ring chunk (four fp16 rows, eight fp8 rows).  fp8:
-    // 724 -> 493 us per token at 1024-token contexts against the CUDA-core kernel, which stays for the grids and
-    // vocabularies outside these limits.
-    const qmk_fused_tc::Build &tc = qmk_fused_tc::build(e->wfmt);
-    if (e->fused >= 2 && P.vocab % tc.rows_per_chunk == 0 && grid >= tc.min_ctas && grid <= tc.max_ctas) {
+    if (on_tensor_cores) {
       rc = encode_cache_maps(e, P);
       if (rc != QMK_OK) return rc;
       kernel = tc.kernel;

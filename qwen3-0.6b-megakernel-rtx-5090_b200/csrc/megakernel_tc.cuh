@@ -61,12 +61,33 @@ constexpr int ODD_SLOT_SKEW = FP8_ROWS ? 0 : 64;
 static_assert(SLOT_BYTES >= ODD_SLOT_SKEW + CH_ROWS * ROW_PITCH, "a slot holds a chunk of padded rows");
 static_assert(ROW_PITCH % 128 == 16, "eight consecutive rows of a chunk fall into different bank groups");
 static_assert(I % CH_ROWS == 0 && QS % CH_ROWS == 0 && KVS % CH_ROWS == 0, "a chunk lies in one matrix");
+// The O projection.  A CTA that merged its own 14 of the 2048 attention outputs multiplied them into all 1024 outputs: 148
+// contributions to every word of the sum x1, which a word's L2 slice adds one after the other, and six tiles of fixed-point
+// conversions a warp.  Here O_GROUP = 4 CTAs (4 g .. 4 g + 3) merge the SAME slice of 52 to 56 attention outputs and each
+// multiplies it into its quarter of the outputs: the bytes of the K-major matrix and the MMAs are what they were, contributions to a
+// word are 37, a CTA's words 256.  What it costs is a merge of four times the words, whose loads take whole 32-byte sectors now.
+// Mean step of five placements of the buffers, us, before / after (with wait_chunks): one fp16 sequence at 64 / 1024 / 4096 tokens 430 / 443 /
+// 488 -> 432 / 443 / 478, one FP8 at 1024 428 -> 411, two fp16 at 512 531 -> 530, four at 1024 747 -> 733, four FP8 801 -> 728.
+// Grids that are no multiple of four leave the last CTAs without a slice.
+using qmkp::O_GROUP;
+using qmkp::O_COLS;
+constexpr int O_TILES = O_COLS / 16;
+constexpr int O_PITCH = (FP8_ROWS ? 1 : 2) * O_COLS + qmkp::O_PAD;   // conflict-free, in memory as in shared memory
+constexpr int O_CH_ROWS = FP8_ROWS ? 32 : 16;                        // rows of a chunk: what one ldmatrix.x4 takes
+constexpr int TILE_STEP = O_CH_ROWS / 16;                            // k-steps of an ldmatrix.x4
+constexpr int O_MAX_QUADS = (QS / 4 + TC_MIN_CTAS / O_GROUP - 1) / (TC_MIN_CTAS / O_GROUP);   // a slice is whole quads of rows
+constexpr int O_KPAIRS = (4 * O_MAX_QUADS + 31) / 32;
+static_assert(TC_MIN_CTAS % O_GROUP == 0 && O_TILES <= 2 * CONS_WARPS, "at most two output tiles per warp");
+static_assert(O_PITCH % 128 == 16, "eight consecutive rows of an O chunk fall into different bank groups");
+static_assert(SLOT_BYTES >= ODD_SLOT_SKEW + O_CH_ROWS * O_PITCH, "a slot holds a chunk of O rows");
+static_assert(O_MAX_QUADS <= 2 * CONS_WARPS - 2, "merge: two quads per warp, one for the last two");
+static_assert(4 * O_MAX_QUADS <= D, "a slice lies in at most two query heads");
 // The norm vectors of layer L go into the buffer of layer L - 2 as soon as the ring has room for layer L's first
 // chunks, i.e. when chunk (last of L - 1) - NSLOTS was handed back.  That must be a gate/up chunk of layer L - 2 or a
 // later one: every warp is past its last use of L - 2's norm vectors (post_ln, before the gate/up rows) by then.  fp16
 // layers have over 18 chunks on every CTA; the short layers of FP8 rows bound the grid.
 constexpr int TC_MAX_CTAS = FP8_ROWS ? 160 : MAX_CTAS;
-constexpr int MIN_QKV_CH = QKV_ROWS / CH_ROWS / TC_MAX_CTAS, MIN_O_CH = (QS / TC_MAX_CTAS + CH_ROWS - 1) / CH_ROWS + SCALE_CH,
+constexpr int MIN_QKV_CH = QKV_ROWS / CH_ROWS / TC_MAX_CTAS, MIN_O_CH = O_GROUP * QS / TC_MAX_CTAS / O_CH_ROWS + SCALE_CH,
               MIN_GU_CH = I / CH_ROWS / TC_MAX_CTAS, MIN_LAYER_CH = MIN_QKV_CH + MIN_O_CH + 3 * MIN_GU_CH + SCALE_CH;
 static_assert(MIN_LAYER_CH > NSLOTS || 2 * MIN_LAYER_CH - 1 - NSLOTS >= MIN_QKV_CH + MIN_O_CH, "norm vectors overwritten in use");
 static_assert(SLOT_BYTES % 128 == 0 && NSLOTS % 2 == 0, "swizzled boxes need 128-byte aligned slots; slot parity = chunk parity");
@@ -81,6 +102,8 @@ static_assert(SLOT_BYTES >= 4 * KV_BOX, "a slot holds the four boxes of a cache 
 constexpr int QKV_CHUNKS = QKV_ROWS / CH_ROWS, GU_CHUNKS = I / CH_ROWS;
 static_assert(CH_ROWS * ((GU_CHUNKS + TC_MIN_CTAS - 1) / TC_MIN_CTAS) <= 32, "slice_cols takes two k-steps");
 constexpr int KPAIRS = H / 32;                 // pairs of 16-input k-steps in a row
+constexpr int ACT16_PITCH = 32 * O_KPAIRS + 8; // halves between the hi and the lo row of a slice's activations (other banks)
+static_assert(32 * O_KPAIRS >= 64, "the gate/up phase writes 64");
 
 // Extra shared memory of this kernel, behind the single-sequence layout.
 // Normalised activations as the B operand of the row products, in MMA fragment order: 128 bytes per pair of
@@ -100,11 +123,13 @@ struct alignas(16) TcTab {
   int q0, nq, g0, ng, lm0, nlm;    // first chunk / chunks of this CTA: q|k|v rows, gate (= up) rows, LM-head rows
   int nkb_qkv, nkb_gu;             // warps per tile in the two row-product phases
   TileTask qkv[12], gu[12];        // each warp's tile task in those phases
+  int e0, ne, no, oq;              // this CTA's slice of the attention outputs, its ring chunks, its quarter of the outputs
+  int n0, n1, groups, pad2;        // outputs whose residuals this CTA adds; groups of CTAs that share a slice
   int s_cap, seq, local, pad;      // several sequences: most splits of one, the sequence of this CTA's attention item, the item
 };
 // Several sequences: previous contributions to the residual sums [x1, x2][sequence][1024] (sequences 0 and 1 where the
 // single-sequence kernel has its fp32 vectors; the pitch puts the four sequences of a fragment into different banks),
-// residuals of the outputs this CTA owns, split weights of the merge, sums of squares, tokens.
+// residuals of the outputs this CTA owns, split weights of the merge, sums of squares, tokens, splits.
 constexpr int PREV_PITCH = H + 8, RESID_PITCH = 12;
 static_assert(4 * PREV_PITCH <= FF_SPLITW, "sequences 0 and 1 fit in front of the weight arrays");
 constexpr size_t OFF_PREV2 = OFF_TCTAB + (sizeof(TcTab) + 15) / 16 * 16;
@@ -112,7 +137,7 @@ constexpr size_t OFF_RESID = OFF_PREV2 + (TC_SEQS > 2 ? 4 * PREV_PITCH * 4 : 0);
 constexpr size_t OFF_SPLITW = OFF_RESID + 2 * TC_SEQS * RESID_PITCH * 4;
 constexpr size_t OFF_REDM = OFF_SPLITW + 2 * 32 * 4;
 constexpr size_t OFF_TOKENS = OFF_REDM + TC_SEQS * CONS_WARPS * 4;
-constexpr size_t TC_SMEM_BYTES = TC_SEQS > 1 ? OFF_TOKENS + TC_SEQS * 4 : OFF_TCTAB + sizeof(TcTab);
+constexpr size_t TC_SMEM_BYTES = TC_SEQS > 1 ? OFF_TOKENS + 2 * TC_SEQS * 4 : OFF_TCTAB + sizeof(TcTab);
 static_assert(TC_SMEM_BYTES <= 232448, "over the 227 KB shared-memory limit of one CTA");
 static_assert(OFF_XF % 128 == 0 && OFF_QF % 16 == 0, "operand rows are 16-byte aligned, a pair's 128 bytes one wavefront");
 // Byte offset in the fragment-order array of input i's hi (lo = 0) or lo (1) half, sequence b.
@@ -203,6 +228,17 @@ __device__ __forceinline__ void e4m3x4_half2x2(uint32_t four, uint32_t &first, u
       : "=r"(first), "=r"(second) : "r"(four));
 }
 
+// Waits for ring chunks [first, first + n), 1 <= n <= 32.  Lanes past the last one ask for it too, so that the warp asks once and
+// votes without branching (a diverging wait took 370 cycles of chunks that were there, of an LM head tile with FP8 rows a sixth:
+// 51.5 -> 44 us).  The vote orders the copied bytes before every lane's loads.
+__device__ __forceinline__ bool wait_chunks(const Params &P, const Ctx &c, uint32_t first, int n) {
+  const uint32_t idx = first + static_cast<uint32_t>(min(c.lane, n - 1));
+  uint64_t *bar = c.full(idx % NSLOTS);
+  const uint32_t parity = (idx / NSLOTS) & 1u;
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait(P, c, bar, parity, WHERE_FULL, false));
+}
+
 // One warp: rows of the 16-row tile that starts at ring chunk `first` (valid rows <= 16), k-step pairs [p0, p1).
 // Operands come in front of the products they feed.  An MMA takes 8.5 cycles of a sub-partition (stand-alone, 4 to 12 warps;
 // 21 from one to the next that depends on it), a ldmatrix 48 cycles until its data can be used and four of the SM's
@@ -216,12 +252,7 @@ __device__ __forceinline__ void e4m3x4_half2x2(uint32_t four, uint32_t &first, u
 __device__ __forceinline__ void tile_task(const Params &P, const Ctx &c, uint32_t first, int valid_rows, int p0, int p1,
                                           float *part, int units, int fslot = 70) {
   const int nch = (valid_rows + CH_ROWS - 1) / CH_ROWS;
-  bool ok = true;
-  if (c.lane < nch) {
-    const uint32_t idx = first + static_cast<uint32_t>(c.lane);
-    ok = mbar_wait(P, c, c.full(idx % NSLOTS), (idx / NSLOTS) & 1u, WHERE_FULL, false);
-  }
-  ok = __all_sync(0xffffffffu, ok);
+  const bool ok = wait_chunks(P, c, first, nch);
   QMK_FINE(fslot + 1);
   int lr = (c.lane & 7) + ((c.lane >> 3) & 1) * 8;      // tile row whose address this lane supplies
   if (lr >= valid_rows) lr = 0;                         // rows past the end repeat row 0 (their sums are not used)
@@ -687,7 +718,7 @@ __device__ __forceinline__ void red_wait_norm(const Params &P, const Ctx c, int 
     if (c.tid + j * CONS_THREADS < H) valid |= 1u << j;
 #pragma unroll 1
   for (int r = 0; r < R; ++r) {
-    const unsigned long long base = static_cast<unsigned long long>(use) * red_contributors(c.ncta, R, r);
+    const unsigned long long base = static_cast<unsigned long long>(use) * red_contributors(which ? c.ncta : tctab(c)->groups, R, r);
     const unsigned long long *src = buf + r * RED_SUM_WORDS + red_index(c.tid);
     {
       // one lane per warp watches one word until it is complete, then the warp fetches its words: 32x fewer polls
@@ -850,31 +881,215 @@ __device__ __forceinline__ void slice_tiles(const uint32_t (&arow)[2], const uin
   }
 }
 
+// What an O slice multiplies: this lane's row address in act16 and in the first four k-steps of 16 weight rows (fp8: two pairs).
+// k-steps past the slice repeat its first row: their activations are zero.
+constexpr int O_LOADS = 4 / TILE_STEP;         // ldmatrix.x4 of four k-steps
+struct OSlice { uint32_t act, row[O_LOADS]; int ne; };
+__device__ __forceinline__ uint32_t o_row(const Ctx &c, int ne, int k) {
+  const int r = FP8_ROWS ? c.lane : (c.lane & 7) + 8 * (c.lane >> 4);
+  const bool in = O_CH_ROWS * k + r < ne;
+  return weight_rows(c, c.chunk + static_cast<uint32_t>(in ? k : 0)) + (in ? r : 0) * O_PITCH + (FP8_ROWS ? 0 : ((c.lane >> 3) & 1) * 16);
+}
+__device__ __forceinline__ OSlice o_slice(const Ctx &c, uint32_t act, int ne) {
+  OSlice o;
+  o.act = act;
+  o.ne = ne;
+#pragma unroll
+  for (int k = 0; k < O_LOADS; ++k) o.row[k] = o_row(c, ne, k);
+  return o;
+}
+// s + e = a + b exactly.
+__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
+  s = a + b;
+  const float z = s - a;
+  e = (a - (s - z)) + (b - z);
+}
+// Products of two k-steps: d0, d1 = their sums.  a0 (fp8: the packed bytes of both), a1: ldmatrix results.
+__device__ __forceinline__ void o_products(uint32_t (&a0)[4], uint32_t (&a1)[4], const uint32_t (&bq)[4], float (&d0)[4], float (&d1)[4]) {
+  if (FP8_ROWS) {
+    uint32_t r[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[i] = __byte_perm(a0[i], 0u, 0x3120);   // as in slice_tiles
+    e4m3x4_half2x2(r[0], a0[0], a0[1]);
+    e4m3x4_half2x2(r[1], a0[2], a0[3]);
+    e4m3x4_half2x2(r[2], a1[0], a1[1]);
+    e4m3x4_half2x2(r[3], a1[2], a1[3]);
+  }
+  mma_16816_zero(d0, a0, bq[0], bq[1]);
+  mma_16816_zero(d1, a1, bq[2], bq[3]);
+}
+// One 16-output tile of an O slice: v[0], v[1] = this lane's two rows of the fragment (quad b: sequence b's hi and lo columns).
+// A k-step's products come out of one MMA; the hi sums of the k-steps are added with their rounding errors kept, so that a
+// contribution is rounded once, as it was with one k-step per CTA.
+__device__ __forceinline__ void slice_o_tile(const Ctx &c, const OSlice &o, int tile, float (&v)[2]) {
+  const uint32_t col = tile * (FP8_ROWS ? 16 : 32);
+  uint32_t a[4][4], bq[2][4];
+  float d[4][4], lo[2], s[2], e[2];
+#pragma unroll
+  for (int k = 0; k < O_LOADS; ++k) ldsm_x4_trans(o.row[k] + col, a[k * TILE_STEP]);
+  ldsm_x4(o.act, bq[0]);
+  ldsm_x4(o.act + 64, bq[1]);
+  o_products(a[0], a[1], bq[0], d[0], d[1]);
+  o_products(a[2], a[3], bq[1], d[2], d[3]);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float s0, s1, e0, e1;
+    two_sum(d[0][2 * h], d[1][2 * h], s0, e0);
+    two_sum(d[2][2 * h], d[3][2 * h], s1, e1);
+    two_sum(s0, s1, s[h], e[h]);
+    e[h] += e0 + e1;
+    lo[h] = (d[0][2 * h + 1] + d[1][2 * h + 1]) + (d[2][2 * h + 1] + d[3][2 * h + 1]);
+  }
+#pragma unroll 1
+  for (int k = 2; 32 * k < o.ne; ++k) {          // grids of up to 124 CTAs: more than 64 rows
+    ldsm_x4_trans(o_row(c, o.ne, k * 2 / TILE_STEP) + col, a[0]);
+    if (!FP8_ROWS) ldsm_x4_trans(o_row(c, o.ne, k * 2 + 1) + col, a[1]);
+    ldsm_x4(o.act + k * 64, bq[0]);
+    o_products(a[0], a[1], bq[0], d[0], d[1]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float s0, e0, e1;
+      two_sum(d[0][2 * h], d[1][2 * h], s0, e0);
+      two_sum(s[h], s0, s[h], e1);
+      e[h] += e0 + e1;
+      lo[h] += d[0][2 * h + 1] + d[1][2 * h + 1];
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) v[h] = s[h] + fmaf(lo[h], LO_INV, e[h]);
+}
+
 #if QMK_TC_SEQS == 1
-// Split-K slice of the O (which = 0) or down (1) projection (see slice_colgemv of megakernel_fused.cuh) on the
+// Merge of the attention partials for this CTA's slice of outputs [e0, e0 + ne): the unnormalised outputs of an element's S
+// splits, weighted with exp2(max_s - max) / sum, go to act16 as the hi / lo halves of the O slice's operand.  A warp takes quads
+// of four consecutive elements (a 32-byte sector of every split's partial): lane 4 k + i holds element i, splits k, k + 8 and k + 16.
+// The last two warps also fetch the (max, sum) pairs of the slice's (at most two) heads, in the same round of polls, and share
+// the weights through a barrier: polled by every warp they cost 2 us a layer.
+constexpr int MERGE_QUADS = 2, MERGE_SPLITS = (MAX_SPLITS + 7) / 8;
+__device__ __forceinline__ void merge_o(const Params &P, const Ctx &c, int S, uint32_t tag) {
+  const TcTab *t = tctab(c);
+  const int e0 = t->e0, ne = t->ne, h0 = e0 >> 7, el = c.lane & 3, sl = c.lane >> 2;
+  float *s_wt = c.f(FF_SPLITW);
+  constexpr int NW = MERGE_QUADS * MERGE_SPLITS;
+  const unsigned long long *words = c.llr + LL_PART;
+  uint32_t wp[NW], valid = 0;
+#pragma unroll
+  for (int i = 0; i < MERGE_QUADS; ++i) {
+    const int q = c.warp + i * CONS_WARPS, e = e0 + (4 * q < ne ? 4 * q : 0) + el;
+    const uint32_t head = (e >> 7) * (MAX_SPLITS * PART_STRIDE) + (e & (D - 1));
+#pragma unroll
+    for (int k = 0; k < MERGE_SPLITS; ++k) {
+      wp[i * MERGE_SPLITS + k] = head + min(sl + 8 * k, S - 1) * PART_STRIDE;
+      if (4 * q < ne && sl + 8 * k < S) valid |= 1u << (i * MERGE_SPLITS + k);
+    }
+  }
+  QMK_FINE(50);
+  float a[NW];
+  if (4 * c.warp < ne) {
+    // the owner split (the last one) also handles the new row: its words arrive last.  (Without this watch where there are one or
+    // two splits, words polled at once: 432 -> 448 us per step at 64 tokens; polls slow the attention CTAs.)
+    const int e = e0 + 4 * c.warp;
+    ll_sentinel(P, c, words + ((e >> 7) * MAX_SPLITS + S - 1) * PART_STRIDE + (e & (D - 1)), tag);
+    const int hw = h0 + (c.warp - (CONS_WARPS - 2));                      // head whose split weights this warp makes
+    if (c.warp >= CONS_WARPS - 2 && hw <= ((e0 + ne - 1) >> 7)) {         // warp-uniform
+      uint32_t wl[MERGE_SPLITS + 2];
+      float v[MERGE_SPLITS + 2];
+#pragma unroll
+      for (int k = 0; k < MERGE_SPLITS; ++k) wl[k] = wp[k];
+      wl[MERGE_SPLITS] = (hw * MAX_SPLITS + min(c.lane, S - 1)) * PART_STRIDE + D;
+      wl[MERGE_SPLITS + 1] = wl[MERGE_SPLITS] + 1;
+      ll_wait_words<MERGE_SPLITS + 2>(P, c, words, wl, (valid & ((1u << MERGE_SPLITS) - 1u)) | (c.lane < S ? 3u << MERGE_SPLITS : 0u), tag, v);
+#pragma unroll
+      for (int k = 0; k < NW; ++k) a[k] = k < MERGE_SPLITS ? v[k] : 0.f;
+      const float m = c.lane < S ? v[MERGE_SPLITS] : -INFINITY, l = c.lane < S ? v[MERGE_SPLITS + 1] : 0.f;
+      const float M = warp_max(m);
+      const float sc = (m == -INFINITY) ? 0.f : exp2f(m - M);
+      const float L = warp_sum(l * sc);
+      s_wt[(hw - h0) * 32 + c.lane] = sc / L;
+    } else {
+      ll_wait_words<NW>(P, c, words, wp, valid, tag, a);
+    }
+    QMK_FINE(51);
+  }
+  cons_sync();
+  QMK_FINE(52);
+  __half *act16 = reinterpret_cast<__half *>(c.smem + OFF_ACT16);
+  float A[MERGE_QUADS];
+#pragma unroll
+  for (int i = 0; i < MERGE_QUADS; ++i) {
+    const int q = c.warp + i * CONS_WARPS, e = e0 + (4 * q < ne ? 4 * q : 0) + el;
+    A[i] = 0.f;
+#pragma unroll
+    for (int k = 0; k < MERGE_SPLITS; ++k)
+      if (valid & (1u << (i * MERGE_SPLITS + k))) A[i] = fmaf(a[i * MERGE_SPLITS + k], s_wt[((e >> 7) - h0) * 32 + sl + 8 * k], A[i]);
+  }
+#pragma unroll
+  for (int o = 16; o > 2; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < MERGE_QUADS; ++i) A[i] += __shfl_xor_sync(0xffffffffu, A[i], o);
+#pragma unroll
+  for (int i = 0; i < MERGE_QUADS; ++i) {
+    const int q = c.warp + i * CONS_WARPS;
+    if (4 * q < ne && sl < 2) act16[sl * ACT16_PITCH + 4 * q + el] = split_half(A[i], sl != 0);
+  }
+  if (c.tid >= ne && c.tid < 32 * O_KPAIRS) { act16[c.tid] = __float2half_rn(0.f); act16[ACT16_PITCH + c.tid] = __float2half_rn(0.f); }
+}
+
+// O slice: this CTA's merged attention outputs times its quarter of the outputs -> sum x1.
+__device__ __forceinline__ uint32_t slice_o(const Params &P, Ctx c) {
+  const TcTab *t = tctab(c);
+  const int ne = t->ne, nch = t->no;
+  if (nch == 0) return c.chunk;
+  const float *resid = c.f(F_X);
+  float *prev = c.f(FF_PREV);
+  unsigned long long *mine = P.red + RED_X1 + ((c.cta / O_GROUP) & (P.red_copies - 1)) * RED_SUM_WORDS;   // one or two copies
+  QMK_FINE(20);
+  const bool ok = wait_chunks(P, c, c.chunk, nch);
+  if (ok) {
+    const OSlice o = o_slice(c, smem_u32(c.smem + OFF_ACT16) + (c.lane & 1) * (ACT16_PITCH * 2) + (c.lane >> 3) * 16, ne);
+    const int n0 = t->n0, n1 = t->n1, out0 = t->oq * O_COLS;
+    const int src = FP8_ROWS ? ((c.lane & 15) >> 1) * 4 : (c.lane & 7) * 4;      // as in slice_cols
+    const bool second = (c.lane & (FP8_ROWS ? 1 : 8)) != 0;
+    float v0[2], v1[2] = {0.f, 0.f};
+    slice_o_tile(c, o, c.warp, v0);
+    if (c.warp + CONS_WARPS < O_TILES) slice_o_tile(c, o, c.warp + CONS_WARPS, v1);
+    const float s0 = __shfl_sync(0xffffffffu, v0[0], src), s1 = __shfl_sync(0xffffffffu, v0[1], src);
+    const float s2 = __shfl_sync(0xffffffffu, v1[0], src), s3 = __shfl_sync(0xffffffffu, v1[1], src);
+    const int tile = c.warp + (c.lane >> 4) * CONS_WARPS;
+    if (tile < O_TILES) {
+      const int j = tile * 16 + (c.lane & 15), n = out0 + j;
+      float v = (c.lane & 16) ? (second ? s3 : s2) : (second ? s1 : s0);
+      if (FP8_ROWS) v *= reinterpret_cast<const float *>(c.smem + (weight_rows(c, c.chunk + static_cast<uint32_t>(nch - 1)) - smem_u32(c.smem)))[j];
+      if (n >= n0 && n < n1) v += resid[n];
+      const long long fx = __float2ll_rn(v * RED_SCALE), fx_prev = __float2ll_rn(prev[j] * RED_SCALE);
+      prev[j] = v;
+      red_add_u64(mine + red_index(n), (static_cast<unsigned long long>(fx - fx_prev) << RED_CNT_BITS) + 1ull);
+    }
+  }
+  __syncwarp();
+  if (c.lane < nch) mbar_arrive_n(c.empty((c.chunk + static_cast<uint32_t>(c.lane)) % NSLOTS), EMPTY_UNITS / CONS_WARPS);
+  QMK_FINE(23);
+  return c.chunk + static_cast<uint32_t>(nch);
+}
+
+// Split-K slice of the down projection (see slice_colgemv of megakernel_fused.cuh) on the
 // tensor cores: partial[n] = sum_i act[i] * Wt[first + i][n] with the K-major rows as the A operand read through
 // ldmatrix.trans (tile = 16 outputs x 16 rows, at most two k-steps: slices of at most 32 rows), the slice's
 // activations as B (hi / lo columns, from act16).  Warp w takes output tiles w, w + 12, ... over ALL rows of the
 // slice, so a partial is complete when it leaves the warp: after each pair of tiles the 32 sums are spread over
 // the 32 lanes (four shuffles) and every lane adds its one output into the residual sum - no staging in shared
 // memory, no barrier, and the adds of early tiles drain while later tiles are computed.
-__device__ __forceinline__ uint32_t slice_cols(const Params &P, Ctx c, int which) {
-  const SegTab *t = c.segs();
-  const int nrows = which ? tctab(c)->ng * CH_ROWS : t->e1 - t->e0;
-  const float *resid = c.f(which ? F_X1 : F_X);
-  float *prev = c.f(FF_PREV) + (which ? H : 0);
-  unsigned long long *mine = P.red + (which ? RED_X2 : RED_X1) + (c.cta % P.red_copies) * RED_SUM_WORDS;
+__device__ __forceinline__ uint32_t slice_cols(const Params &P, Ctx c) {
+  const TcTab *t = tctab(c);
+  const int nrows = t->ng * CH_ROWS;
+  const float *resid = c.f(F_X1);
+  float *prev = c.f(FF_PREV) + H;
+  unsigned long long *mine = P.red + RED_X2 + (c.cta & (P.red_copies - 1)) * RED_SUM_WORDS;   // one or two copies
   const int nch = (nrows + CH_ROWS - 1) / CH_ROWS + SCALE_CH;
   [[maybe_unused]] const float *scales = FP8_ROWS ? reinterpret_cast<const float *>(c.slot(c.chunk + static_cast<uint32_t>(nch - 1))) : nullptr;
   const bool two = nrows > 16;
-  [[maybe_unused]] const int fb = which ? 30 : 20;
-  QMK_FINE(fb + 0);
-  bool ok = true;
-  if (c.lane < nch) {
-    const uint32_t idx = c.chunk + static_cast<uint32_t>(c.lane);
-    ok = mbar_wait(P, c, c.full(idx % NSLOTS), (idx / NSLOTS) & 1u, WHERE_FULL, false);
-  }
-  ok = __all_sync(0xffffffffu, ok);
+  QMK_FINE(30);
+  const bool ok = wait_chunks(P, c, c.chunk, nch);
   if (ok) {
     // B: the slice's activations; row n of B^T = hi (even n) / lo (odd n) vector; one ldmatrix.x4 = two k-steps
     uint32_t bq[4];
@@ -882,7 +1097,7 @@ __device__ __forceinline__ uint32_t slice_cols(const Params &P, Ctx c, int which
     uint32_t arow[2];
     slice_row_addresses(c, nrows, arow);
     const int n0 = t->n0, n1 = t->n1;
-    const float up = which ? c.f(F_MISC)[M_ASCALE] : 1.f;
+    const float up = c.f(F_MISC)[M_ASCALE];
     // lane that holds this lane's output (fragment row = lane / 4), and whether it is its second row
     const int src = FP8_ROWS ? ((c.lane & 15) >> 1) * 4 : (c.lane & 7) * 4;
     const bool second = (c.lane & (FP8_ROWS ? 1 : 8)) != 0;
@@ -911,7 +1126,7 @@ __device__ __forceinline__ uint32_t slice_cols(const Params &P, Ctx c, int which
   }
   __syncwarp();
   if (c.lane < nch) mbar_arrive_n(c.empty((c.chunk + static_cast<uint32_t>(c.lane)) % NSLOTS), EMPTY_UNITS / CONS_WARPS);
-  QMK_FINE(fb + 3);
+  QMK_FINE(33);
   return c.chunk + static_cast<uint32_t>(nch);
 }
 
@@ -1024,7 +1239,6 @@ __device__ __forceinline__
 #endif
 void producer_main_tc(const Params &P, const Ctx c) {
   const uint64_t pol = P.l2_evict_first ? l2_evict_first_policy() : l2_evict_normal_policy();
-  const SegTab *t = c.segs();
   const TcTab *tt = tctab(c);
   const int grp = c.lane >> 2;
   // the caches this CTA attends to
@@ -1036,13 +1250,13 @@ void producer_main_tc(const Params &P, const Ctx c) {
       if (seq == b) { kmap = P.kmaps[b]; vmap = P.vmaps[b]; }
   }
   const int start = TC_SEQS == 1 ? P.start_position : per_seq(P.start_positions, seq);
-  const int nq = tt->nq, ng = tt->ng, ne = t->e1 - t->e0, no = (ne + CH_ROWS - 1) / CH_ROWS;
+  const int nq = tt->nq, ng = tt->ng, ne = tt->ne, no = tt->no;
   uint32_t idx = 0, issued = 0;   // first chunk of the current layer / chunks issued so far
   bool ok = true;
 #pragma unroll 1
   for (int step = 0; ok && step < P.num_steps; ++step) {
     const AttnItem it = tc_item(P, c, start + step);
-    const int s1 = nq, s2 = s1 + it.nchunks, s3 = s2 + no + SCALE_CH, s4 = s3 + ng, s5 = s4 + ng, per_layer = s5 + ng + SCALE_CH;
+    const int s1 = nq, s2 = s1 + it.nchunks, s3 = s2 + no, s4 = s3 + ng, s5 = s4 + ng, per_layer = s5 + ng + SCALE_CH;
 #pragma unroll 1
     for (int l = 0; ok && l < P.num_layers; ++l) {
       const unsigned long long *rec = c.layer_rec(l);
@@ -1070,9 +1284,16 @@ void producer_main_tc(const Params &P, const Ctx c) {
         } else if (j < s2) {     // old K rows (lane 4g) and V rows (lane 4g + 1) of the attention item
           d.kv_row = (l * NKV + it.g) * P.max_seq_len + it.p0 + (j - s1) * it.rpc;
         } else if (j < s3) {
-          const int r = (j - s2) * CH_ROWS;
-          if (r < ne) d = matrix_chunk(reinterpret_cast<const void *>(rect[0]), t->e0 + r, min(CH_ROWS, ne - r));
-          else d = scale_chunk(reinterpret_cast<const void *>(rect[0]), QS);
+          const int r = (j - s2) * O_CH_ROWS;
+          const unsigned char *base = reinterpret_cast<const unsigned char *>(rect[0]);
+          d.rows = 1u;
+          if (r < ne) {
+            d.src = base + static_cast<size_t>(tt->oq * QS + tt->e0 + r) * O_PITCH;
+            d.row_bytes = static_cast<uint32_t>(min(O_CH_ROWS, ne - r) * O_PITCH);
+          } else {               // fp8: the scales of the quarter's outputs
+            d.src = base + static_cast<size_t>(O_GROUP * QS) * O_PITCH + tt->oq * O_COLS * 4;
+            d.row_bytes = 4 * O_COLS;
+          }
         } else if (j < s4) {
           d = matrix_chunk(reinterpret_cast<const void *>(rec[REC_GATE]), (tt->g0 + j - s3) * CH_ROWS, CH_ROWS);
         } else if (j < s5) {
@@ -1118,6 +1339,15 @@ __device__ __forceinline__ void tc_setup(const Params &P, const Ctx &c) {
     split_rows(QKV_CHUNKS, c.ncta, c.cta, a, b); tt->q0 = a; tt->nq = b - a;
     split_rows(GU_CHUNKS, c.ncta, c.cta, a, b); tt->g0 = a; tt->ng = b - a;
     split_rows(P.vocab / CH_ROWS, c.ncta, c.cta, a, b); tt->lm0 = a; tt->nlm = b - a;
+    tt->groups = c.ncta / O_GROUP;
+    const int grp = c.cta / O_GROUP;
+    tt->oq = c.cta % O_GROUP;
+    tt->e0 = tt->ne = tt->no = tt->n0 = tt->n1 = 0;
+    if (grp < tt->groups) {
+      split_rows(QS / 4, tt->groups, grp, a, b); tt->e0 = 4 * a; tt->ne = 4 * (b - a);
+      split_rows(O_COLS, tt->groups, grp, a, b); tt->n0 = tt->oq * O_COLS + a; tt->n1 = tt->oq * O_COLS + b;
+      tt->no = (tt->ne + O_CH_ROWS - 1) / O_CH_ROWS + SCALE_CH;
+    }
     build_tile_tasks(tt->qkv, &tt->nkb_qkv, 1, tt->nq);
     build_tile_tasks(tt->gu, &tt->nkb_gu, GU_ONE_RUN ? 1 : 2, GU_ONE_RUN ? 2 * tt->ng : tt->ng);
   }
@@ -1218,17 +1448,17 @@ __global__ void __launch_bounds__(THREADS, 1) qwen3_decode_megakernel_tc(const _
         QMK_STAMP(layer * 12 + 1);
         c.chunk = attention_tc(P, c, nv, layer, pos, tag);
         QMK_STAMP(layer * 12 + 2);
-        merge_slice(P, c, S_step, tag, reinterpret_cast<__half *>(c.smem + OFF_ACT16));
+        merge_o(P, c, S_step, tag);
         QMK_STAMP(layer * 12 + 3);
         cons_sync();
-        c.chunk = slice_cols(P, c, 0);
+        c.chunk = slice_o(P, c);
         QMK_STAMP(layer * 12 + 4);
         red_wait_norm(P, c, 0, use, nv + NB_POST_LN, 0);
         QMK_STAMP(layer * 12 + 5);
         c.chunk = gateup_phase(P, c);
         QMK_STAMP(layer * 12 + 6);
         cons_sync();
-        c.chunk = slice_cols(P, c, 1);
+        c.chunk = slice_cols(P, c);
         QMK_STAMP(layer * 12 + 7);
         const bool last = layer == P.num_layers - 1;
         if (!last) mbar_wait(P, c, c.nfull((Lg + 1u) & 1u), ((Lg + 1u) >> 1) & 1u, WHERE_FULL, false);

@@ -26,7 +26,7 @@ static_assert(CH_ROWS * ((QKV_CHUNKS + TC_MIN_CTAS - 1) / TC_MIN_CTAS) <= TPS &&
 static_assert(2 * ((GU_CHUNKS + TC_MIN_CTAS - 1) / TC_MIN_CTAS) <= NSLOTS && (QKV_CHUNKS + TC_MIN_CTAS - 1) / TC_MIN_CTAS <= NSLOTS,
               "a phase exceeds the ring");
 static_assert(TC_SEQS * 2 * MAX_CTAS <= CONS_WARPS * 2 * PART_STRIDE, "argmax words alias the attention partials");
-static_assert((H + TC_MIN_CTAS - 1) / TC_MIN_CTAS <= RESID_PITCH, "outputs of a CTA");
+static_assert((O_COLS + TC_MIN_CTAS / O_GROUP - 1) / (TC_MIN_CTAS / O_GROUP) <= RESID_PITCH, "outputs of a CTA");
 
 __device__ __forceinline__ float *tc_prev(const Ctx &c, int which, int b) {
   return (b < 2 ? c.f(F_X) : reinterpret_cast<float *>(c.smem + OFF_PREV2)) + (which * 2 + (b & 1)) * PREV_PITCH;
@@ -35,6 +35,7 @@ __device__ __forceinline__ float *tc_resid(const Ctx &c, int which, int b) {
   return reinterpret_cast<float *>(c.smem + OFF_RESID) + (which * TC_SEQS + b) * RESID_PITCH;
 }
 __device__ __forceinline__ int *tc_tokens(const Ctx &c) { return reinterpret_cast<int *>(c.smem + OFF_TOKENS); }
+__device__ __forceinline__ int *tc_splits(const Ctx &c) { return reinterpret_cast<int *>(c.smem + OFF_TOKENS) + TC_SEQS; }   // of each sequence's attention in this step
 
 __device__ __forceinline__ uint32_t qkv_phase_seqs(const Params &P, Ctx c, uint32_t tag) {
   const TcTab *t = tctab(c);
@@ -83,92 +84,136 @@ __device__ __forceinline__ uint32_t gateup_phase_seqs(const Params &P, Ctx c) {
   return c.chunk + static_cast<uint32_t>(2 * nch);
 }
 
-// merge_slice (megakernel_fused.cuh) for all sequences at once: lanes LPS * b .. + LPS - 1 of a warp are the splits of
-// sequence b, so a warp still takes elements e0 + warp, + 12, ... and every element's sequences complete together.
-__device__ __forceinline__ void merge_seqs(const Params &P, const Ctx c, int step, uint32_t tag) {
-  float *s_wt = reinterpret_cast<float *>(c.smem + OFF_SPLITW);      // [2 heads][32 lanes]
-  const int e0 = c.segs()->e0, e1 = c.segs()->e1, h0 = e0 >> 7;
-  const int b = c.lane / LPS, sl = c.lane % LPS;
-  const int S = max(1, min((per_seq(P.start_positions, min(b, P.nseq - 1)) + step) / max(1, P.split_len), tctab(c)->s_cap));
-  const bool mine = b < P.nseq && sl < S;
-  const unsigned long long *area = P.ll + static_cast<size_t>(min(b, P.nseq - 1)) * LL_WORDS + LL_PART;
-  const int s = min(sl, S - 1);
-  constexpr int NE = 2;
-  static_assert(NE * CONS_WARPS >= (QS + TC_MIN_CTAS - 1) / TC_MIN_CTAS, "elements per CTA exceed two per warp");
-  const unsigned long long *wp[NE];
-  uint32_t valid = 0;
+// merge_o for all sequences at once: a warp takes (quad of elements, sequence) pairs, lane 4 k + i element i and splits k, k + 8.
+constexpr int SEQ_TASKS = (O_MAX_QUADS * TC_SEQS + CONS_WARPS - 1) / CONS_WARPS, SEQ_SPLITS = (LPS + 7) / 8;
+static_assert(O_MAX_QUADS * TC_SEQS <= SEQ_TASKS * CONS_WARPS - 2, "the last two warps have a task less and fetch split weights instead");
+__device__ __forceinline__ void merge_seqs(const Params &P, const Ctx &c, uint32_t tag) {
+  const TcTab *t = tctab(c);
+  float *s_wt = reinterpret_cast<float *>(c.smem + OFF_SPLITW);      // [2 heads][sequence][LPS splits]
+  const int e0 = t->e0, ne = t->ne, h0 = e0 >> 7, el = c.lane & 3, sl = c.lane >> 2;
+  constexpr int NW = SEQ_TASKS * SEQ_SPLITS;
+  const unsigned long long *words = P.ll + LL_PART;
+  uint32_t wp[NW], valid = 0;
 #pragma unroll
-  for (int q = 0; q < NE; ++q) {
-    const int e = min(e0 + c.warp + q * CONS_WARPS, e1 - 1);
-    wp[q] = area + static_cast<size_t>((e >> 7) * MAX_SPLITS + s) * PART_STRIDE + (e & (D - 1));
-    if (mine && e0 + c.warp + q * CONS_WARPS < e1) valid |= 1u << q;
+  for (int i = 0; i < SEQ_TASKS; ++i) {
+    const int task = c.warp + i * CONS_WARPS, q = task / TC_SEQS, b = min(task % TC_SEQS, P.nseq - 1), S = tc_splits(c)[b];
+    const bool mine = task % TC_SEQS < P.nseq && 4 * q < ne;
+    const int e = e0 + (4 * q < ne ? 4 * q : 0) + el;
+    const uint32_t head = b * LL_WORDS + (e >> 7) * (MAX_SPLITS * PART_STRIDE) + (e & (D - 1));
+#pragma unroll
+    for (int k = 0; k < SEQ_SPLITS; ++k) {
+      wp[i * SEQ_SPLITS + k] = head + min(sl + 8 * k, S - 1) * PART_STRIDE;
+      if (mine && sl + 8 * k < S) valid |= 1u << (i * SEQ_SPLITS + k);
+    }
   }
-  {   // one lane per warp watches the last split's word of the last sequence first (see merge_slice)
-    const int Sl = max(1, min((per_seq(P.start_positions, P.nseq - 1) + step) / max(1, P.split_len), tctab(c)->s_cap));
-    const int e = min(e0 + c.warp, e1 - 1);
-    ll_sentinel(P, c, P.ll + static_cast<size_t>(P.nseq - 1) * LL_WORDS + LL_PART + static_cast<size_t>((e >> 7) * MAX_SPLITS + Sl - 1) * PART_STRIDE + (e & (D - 1)), tag);
-  }
-  float a[NE];
-  const int hw = h0 + (c.warp - (CONS_WARPS - 2));                // head whose split weights this warp makes (last two warps)
-  if (c.warp >= CONS_WARPS - 2 && hw <= ((e1 - 1) >> 7)) {        // warp-uniform
-    const unsigned long long *part = area + static_cast<size_t>(hw * MAX_SPLITS + s) * PART_STRIDE;
-    const unsigned long long *wp4[NE + 2] = {wp[0], wp[1], part + D, part + D + 1};
-    float v4[NE + 2];
-    ll_wait_many<NE + 2>(P, c, wp4, valid | (mine ? (3u << NE) : 0u), tag, v4);
+  float a[NW];
+  if (ne > 0) {
+    {   // one lane per warp watches the last split's word of the last sequence first (see merge_o)
+      const int e = e0 + min(4 * c.warp, ne - 1);
+      ll_sentinel(P, c, words + (P.nseq - 1) * LL_WORDS + ((e >> 7) * MAX_SPLITS + tc_splits(c)[P.nseq - 1] - 1) * PART_STRIDE + (e & (D - 1)), tag);
+    }
+    const int hw = h0 + (c.warp - (CONS_WARPS - 2));                // head whose split weights this warp makes (last two warps)
+    if (c.warp >= CONS_WARPS - 2 && hw <= ((e0 + ne - 1) >> 7)) {   // warp-uniform
+      const int b = c.lane / LPS, s = c.lane % LPS, S = tc_splits(c)[min(b, P.nseq - 1)];
+      const bool mine = b < P.nseq && s < S;
+      constexpr int NL = NW - SEQ_SPLITS;
+      uint32_t wl[NL + 2];
+      float v[NL + 2];
 #pragma unroll
-    for (int q = 0; q < NE; ++q) a[q] = v4[q];
-    const float m = mine ? v4[NE] : -INFINITY, l = mine ? v4[NE + 1] : 0.f;
-    float M = m;
+      for (int k = 0; k < NL; ++k) wl[k] = wp[k];
+      wl[NL] = min(b, P.nseq - 1) * LL_WORDS + (hw * MAX_SPLITS + min(s, S - 1)) * PART_STRIDE + D;
+      wl[NL + 1] = wl[NL] + 1;
+      ll_wait_words<NL + 2>(P, c, words, wl, valid | (mine ? 3u << NL : 0u), tag, v);
 #pragma unroll
-    for (int o = LPS / 2; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-    const float sc = (m == -INFINITY) ? 0.f : exp2f(m - M);
-    float L = l * sc;
+      for (int k = 0; k < NW; ++k) a[k] = k < NL ? v[k] : 0.f;
+      const float m = mine ? v[NL] : -INFINITY, l = mine ? v[NL + 1] : 0.f;
+      float M = m;
 #pragma unroll
-    for (int o = LPS / 2; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
-    s_wt[(hw - h0) * 32 + c.lane] = mine ? sc / L : 0.f;
-  } else {
-    ll_wait_many<NE>(P, c, wp, valid, tag, a);
+      for (int o = LPS / 2; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+      const float sc = (m == -INFINITY) ? 0.f : exp2f(m - M);
+      float L = l * sc;
+#pragma unroll
+      for (int o = LPS / 2; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+      s_wt[(hw - h0) * 32 + c.lane] = mine ? sc / L : 0.f;
+    } else {
+      ll_wait_words<NW>(P, c, words, wp, valid, tag, a);
+    }
   }
   cons_sync();
-  float A[NE];
-#pragma unroll
-  for (int q = 0; q < NE; ++q) {
-    const int e = min(e0 + c.warp + q * CONS_WARPS, e1 - 1);
-    const float wgt = s_wt[((e >> 7) - h0) * 32 + c.lane];
-    A[q] = (valid & (1u << q)) ? a[q] * wgt : 0.f;
-  }
-#pragma unroll
-  for (int o = LPS / 2; o > 0; o >>= 1)
-#pragma unroll
-    for (int q = 0; q < NE; ++q) A[q] += __shfl_xor_sync(0xffffffffu, A[q], o);
   __half *act16 = reinterpret_cast<__half *>(c.smem + OFF_ACT16);
+  float A[SEQ_TASKS];
 #pragma unroll
-  for (int q = 0; q < NE; ++q) {
-    const int e = e0 + c.warp + q * CONS_WARPS;
-    if (e < e1 && sl < 2)    // lane 0 of the group stores the hi half, lane 1 the lo half
-      act16[(2 * b + sl) * ACT16_PITCH + e - e0] = split_half(A[q], sl != 0);
+  for (int i = 0; i < SEQ_TASKS; ++i) {
+    const int task = c.warp + i * CONS_WARPS, q = task / TC_SEQS, b = task % TC_SEQS;
+    const int e = e0 + (4 * q < ne ? 4 * q : 0) + el;
+    A[i] = 0.f;
+#pragma unroll
+    for (int k = 0; k < SEQ_SPLITS; ++k)
+      if (valid & (1u << (i * SEQ_SPLITS + k))) A[i] = fmaf(a[i * SEQ_SPLITS + k], s_wt[((e >> 7) - h0) * 32 + b * LPS + sl + 8 * k], A[i]);
   }
-  const int zb = c.tid / TPS, zr = c.tid % TPS;
-  if (zr < 32 && zr >= e1 - e0) {
-    act16[2 * zb * ACT16_PITCH + zr] = __float2half_rn(0.f);
-    act16[(2 * zb + 1) * ACT16_PITCH + zr] = __float2half_rn(0.f);
+#pragma unroll
+  for (int o = 16; o > 2; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < SEQ_TASKS; ++i) A[i] += __shfl_xor_sync(0xffffffffu, A[i], o);
+#pragma unroll
+  for (int i = 0; i < SEQ_TASKS; ++i) {     // (columns of sequences that do not exist: zero)
+    const int task = c.warp + i * CONS_WARPS, q = task / TC_SEQS, b = task % TC_SEQS;
+    if (4 * q < ne && sl < 2) act16[(2 * b + sl) * ACT16_PITCH + 4 * q + el] = split_half(A[i], sl != 0);
   }
+  if (c.tid >= ne && c.tid < 32 * O_KPAIRS) {
+#pragma unroll
+    for (int r = 0; r < 2 * TC_SEQS; ++r) act16[r * ACT16_PITCH + c.tid] = __float2half_rn(0.f);
+  }
+}
+
+// slice_o for all sequences: quad q of a fragment holds sequence q's sums.
+__device__ __forceinline__ uint32_t slice_o_seqs(const Params &P, Ctx c) {
+  const TcTab *t = tctab(c);
+  const int ne = t->ne, nch = t->no;
+  if (nch == 0) return c.chunk;
+  const bool ok = wait_chunks(P, c, c.chunk, nch);
+  if (ok) {
+    const OSlice o = o_slice(c, smem_u32(c.smem + OFF_ACT16) + ((c.lane & 7) % (2 * TC_SEQS)) * (ACT16_PITCH * 2) + (c.lane >> 3) * 16, ne);
+    const int b = c.lane & 3, j = c.lane >> 2;
+    const bool live = b < P.nseq;
+    const int n0 = t->n0, n1 = t->n1, out0 = t->oq * O_COLS;
+    [[maybe_unused]] const float *scales = reinterpret_cast<const float *>(c.smem + (weight_rows(c, c.chunk + static_cast<uint32_t>(nch - 1)) - smem_u32(c.smem)));
+    const float *resid = tc_resid(c, 1, live ? b : 0);
+    float *prev = tc_prev(c, 0, live ? b : 0);
+    unsigned long long *sum = P.red + (live ? b : 0) * RED_SUM_WORDS;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int tile = c.warp + u * CONS_WARPS;
+      if (tile >= O_TILES) break;
+      float v[2];
+      slice_o_tile(c, o, tile, v);
+      if (live) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int i = tile * 16 + (FP8_ROWS ? 2 * j + k : j + 8 * k), n = out0 + i;
+          if (FP8_ROWS) v[k] *= scales[i];
+          if (n >= n0 && n < n1) v[k] += resid[n - n0];
+          const long long fx = __float2ll_rn(v[k] * RED_SCALE), fx_prev = __float2ll_rn(prev[i] * RED_SCALE);
+          prev[i] = v[k];
+          red_add_u64(sum + red_index(n), (static_cast<unsigned long long>(fx - fx_prev) << RED_CNT_BITS) + 1ull);
+        }
+      }
+    }
+  }
+  __syncwarp();
+  if (c.lane < nch) mbar_arrive_n(c.empty((c.chunk + static_cast<uint32_t>(c.lane)) % NSLOTS), EMPTY_UNITS / CONS_WARPS);
+  return c.chunk + static_cast<uint32_t>(nch);
 }
 
 // slice_cols for all sequences: quad q of a fragment holds sequence q's hi and lo sums of two outputs, which its lanes
 // scale and add into that sequence's residual sum where they are.
-__device__ __forceinline__ uint32_t slice_cols_seqs(const Params &P, Ctx c, int which) {
-  const SegTab *t = c.segs();
-  const int nrows = which ? tctab(c)->ng * CH_ROWS : t->e1 - t->e0;
+__device__ __forceinline__ uint32_t slice_cols_seqs(const Params &P, Ctx c) {
+  const TcTab *t = tctab(c);
+  const int nrows = t->ng * CH_ROWS;
   const int nch = (nrows + CH_ROWS - 1) / CH_ROWS + SCALE_CH;
   [[maybe_unused]] const float *scales = FP8_ROWS ? reinterpret_cast<const float *>(c.slot(c.chunk + static_cast<uint32_t>(nch - 1))) : nullptr;
   const bool two = nrows > 16;
-  bool ok = true;
-  if (c.lane < nch) {
-    const uint32_t idx = c.chunk + static_cast<uint32_t>(c.lane);
-    ok = mbar_wait(P, c, c.full(idx % NSLOTS), (idx / NSLOTS) & 1u, WHERE_FULL, false);
-  }
-  ok = __all_sync(0xffffffffu, ok);
+  const bool ok = wait_chunks(P, c, c.chunk, nch);
   if (ok) {
     uint32_t bq[4];
     ldsm_x4(smem_u32(c.smem + OFF_ACT16) + ((c.lane & 7) % (2 * TC_SEQS)) * (ACT16_PITCH * 2) + (c.lane >> 3) * 16, bq);
@@ -177,10 +222,10 @@ __device__ __forceinline__ uint32_t slice_cols_seqs(const Params &P, Ctx c, int 
     const int b = c.lane & 3, j = c.lane >> 2;
     const bool live = b < P.nseq;
     const int n0 = t->n0, n1 = t->n1;
-    const float up = which ? c.f(F_MISC)[M_ASCALE + (live ? b : 0)] : 1.f;
-    const float *resid = tc_resid(c, which ^ 1, live ? b : 0);   // O slice: x, down slice: x1
-    float *prev = tc_prev(c, which, live ? b : 0);
-    unsigned long long *sum = P.red + (which * TC_SEQS + (live ? b : 0)) * RED_SUM_WORDS;
+    const float up = c.f(F_MISC)[M_ASCALE + (live ? b : 0)];
+    const float *resid = tc_resid(c, 0, live ? b : 0);
+    float *prev = tc_prev(c, 1, live ? b : 0);
+    unsigned long long *sum = P.red + (TC_SEQS + (live ? b : 0)) * RED_SUM_WORDS;
     float acc[SLICE_TILES][4];
     slice_tiles(arow, bq, c.warp, two, acc);
 #pragma unroll
@@ -218,7 +263,7 @@ __device__ __forceinline__ void normalise_seqs(const Ctx &c, const float (&v)[TC
     ss = warp_sum(ss);
     if (c.lane == 0) red[b * CONS_WARPS + c.warp] = ss;
   }
-  const int n0 = c.segs()->n0, n1 = c.segs()->n1;
+  const int n0 = tctab(c)->n0, n1 = tctab(c)->n1;
   float w[VPT];
   bool big = false;
 #pragma unroll
@@ -258,7 +303,7 @@ __device__ __forceinline__ void normalise_seqs(const Ctx &c, const float (&v)[TC
 constexpr unsigned long long SUM_SLACK = 48;
 // red_wait_norm for all sequences: which = 0: x1, 1: x2 (kept as the residual of the next layer's O slice, x).
 __device__ __forceinline__ void red_wait_norm_seqs(const Params &P, const Ctx c, int which, uint32_t use, const __half *norm_w) {
-  const unsigned long long base = static_cast<unsigned long long>(use) * static_cast<unsigned long long>(c.ncta);
+  const unsigned long long base = static_cast<unsigned long long>(use) * static_cast<unsigned long long>(which ? c.ncta : tctab(c)->groups);
   const unsigned long long *src = P.red + static_cast<size_t>(which) * TC_SEQS * RED_SUM_WORDS + red_index(c.tid);
   if (c.lane == 0) {   // one lane per warp watches one word (see red_wait_norm)
     const unsigned long long *p = src + static_cast<size_t>(P.nseq - 1) * RED_SUM_WORDS;
@@ -441,6 +486,7 @@ __global__ void __launch_bounds__(THREADS, 1) qwen3_decode_megakernel_tc_seqs(co
       if (c.tid < TC_SEQS) {
         const int token = tc_tokens(c)[c.tid];
         if (token < 0 || token >= P.vocab) { raise_error(P, c, QMK_ERR_BAD_TOKEN, WHERE_TOKEN); tc_tokens(c)[c.tid] = 0; }
+        tc_splits(c)[c.tid] = max(1, min((per_seq(P.start_positions, min(c.tid, P.nseq - 1)) + step) / max(1, P.split_len), tctab(c)->s_cap));
       }
       if (c.tid < D / 2) {
         float cs, sn;
@@ -472,17 +518,17 @@ __global__ void __launch_bounds__(THREADS, 1) qwen3_decode_megakernel_tc_seqs(co
         QMK_STAMP(layer * 12 + 1);
         c.chunk = attention_tc(P, c, nv, layer, pos, tag);
         QMK_STAMP(layer * 12 + 2);
-        merge_seqs(P, c, step, tag);
+        merge_seqs(P, c, tag);
         QMK_STAMP(layer * 12 + 3);
         cons_sync();
-        c.chunk = slice_cols_seqs(P, c, 0);
+        c.chunk = slice_o_seqs(P, c);
         QMK_STAMP(layer * 12 + 4);
         red_wait_norm_seqs(P, c, 0, use, nv + NB_POST_LN);
         QMK_STAMP(layer * 12 + 5);
         c.chunk = gateup_phase_seqs(P, c);
         QMK_STAMP(layer * 12 + 6);
         cons_sync();
-        c.chunk = slice_cols_seqs(P, c, 1);
+        c.chunk = slice_cols_seqs(P, c);
         QMK_STAMP(layer * 12 + 7);
         const bool last = layer == P.num_layers - 1;
         if (!last) mbar_wait(P, c, c.nfull((Lg + 1u) & 1u), ((Lg + 1u) >> 1) & 1u, WHERE_FULL, false);

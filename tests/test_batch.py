@@ -245,3 +245,26 @@ def test_every_in_place_edit_of_the_weights_is_noticed(C, fmt):
         assert not same(last, first) and same(last, fresh())
     finally:
         C.set_weight_format("fp16")
+
+
+@pytest.mark.parametrize("fmt", ["fp16", "fp8"])
+@pytest.mark.parametrize("n,ctas", [(1, 96), (1, 97), (1, 125), (1, 128), (1, 147), (2, 99), (2, 125), (4, 113), (4, 126), (3, 148)])
+def test_attention_slices_of_every_grid(C, fmt, n, ctas):
+    """Groups of four CTAs share a slice of the attention outputs: 88 rows a group on 96 CTAs, 64 on 128, 68 on 125; CTAs past the
+    last whole group have none.  The slices of a grid that were not read, or read twice, would show in every logit: an output
+    is a sum over all of them, and contributions are about 1/24 of it against a bar of 3e-2 of logits of order one."""
+    import quantize as Q
+    w = S.make_weights(seed=17, num_layers=2, vocab_size=2048, norm_std=0.1, max_seq_len=16)
+    engine_w, oracle_w = Q.quantize_weights_fp8(w) if fmt == "fp8" else (w, w)
+    prompts = [S.make_prompt(L, seed=70 + i, vocab_size=2048) for i, L in enumerate([300, 9, 150, 40][:n])]
+    want, logits = _oracle(oracle_w, 320, prompts, 5)
+    eng = _batch_engine(engine_w, n, 320, weight_format=fmt)
+    C.configure(max_ctas=ctas)
+    try:
+        got, dump = _run_with_dump(C, eng, prompts, 5, 2048)
+    finally:
+        C.configure(max_ctas=0)
+        C.set_weight_format("fp16")
+    for b in range(n):
+        assert got[b] == want[b]
+        assert float((dump[b] - logits[b]).abs().max()) < LOGIT_TOL
