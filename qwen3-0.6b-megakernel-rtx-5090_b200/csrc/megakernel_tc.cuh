@@ -124,7 +124,7 @@ struct alignas(16) TcTab {
   int nkb_qkv, nkb_gu;             // warps per tile in the two row-product phases
   TileTask qkv[12], gu[12];        // each warp's tile task in those phases
   int e0, ne, no, oq;              // this CTA's slice of the attention outputs, its ring chunks, its quarter of the outputs
-  int n0, n1, groups, pad2;        // outputs whose residuals this CTA adds; groups of CTAs that share a slice
+  int n0, n1, groups, early;       // outputs whose residuals this CTA adds; groups of CTAs that share a slice; see EARLY_ROWS
   int s_cap, seq, local, pad;      // several sequences: most splits of one, the sequence of this CTA's attention item, the item
 };
 // Several sequences: previous contributions to the residual sums [x1, x2][sequence][1024] (sequences 0 and 1 where the
@@ -249,14 +249,24 @@ __device__ __forceinline__ bool wait_chunks(const Params &P, const Ctx &c, uint3
 // Leaves the 16 row sums of that k range in part[0..15] (sequence b: part[16 b..]) and hands the tile's chunks back with `units` each.
 // Lanes 0..3 each wait for one of the tile's chunks (the vote that follows orders the copied bytes before every
 // lane's loads).
-__device__ __forceinline__ void tile_task(const Params &P, const Ctx &c, uint32_t first, int valid_rows, int p0, int p1,
-                                          float *part, int units, int fslot = 70) {
-  const int nch = (valid_rows + CH_ROWS - 1) / CH_ROWS;
-  const bool ok = wait_chunks(P, c, first, nch);
-  QMK_FINE(fslot + 1);
+struct RowTile { uint32_t first, a_addr; int valid, p0, p1, units; bool ok; };
+__device__ __forceinline__ RowTile prepare_tile(const Params &P, const Ctx &c, uint32_t first, int valid_rows, int p0, int p1, int units) {
+  RowTile r;
+  r.first = first;
+  r.valid = valid_rows;
+  r.p0 = p0;
+  r.p1 = p1;
+  r.units = units;
+  r.ok = wait_chunks(P, c, first, (valid_rows + CH_ROWS - 1) / CH_ROWS);
   int lr = (c.lane & 7) + ((c.lane >> 3) & 1) * 8;      // tile row whose address this lane supplies
   if (lr >= valid_rows) lr = 0;                         // rows past the end repeat row 0 (their sums are not used)
-  const uint32_t a_addr = weight_rows(c, first + static_cast<uint32_t>(lr / CH_ROWS)) + (lr % CH_ROWS) * ROW_PITCH + (c.lane >> 4) * 16;
+  r.a_addr = weight_rows(c, first + static_cast<uint32_t>(lr / CH_ROWS)) + (lr % CH_ROWS) * ROW_PITCH + (c.lane >> 4) * 16;
+  return r;
+}
+__device__ __forceinline__ void run_tile(const Ctx &c, const RowTile &r, float *part, int fslot = 70) {
+  const bool ok = r.ok;
+  const uint32_t first = r.first, a_addr = r.a_addr;
+  const int valid_rows = r.valid, p0 = r.p0, p1 = r.p1, units = r.units, nch = (valid_rows + CH_ROWS - 1) / CH_ROWS;
   float sum[4] = {0.f, 0.f, 0.f, 0.f};
   if (ok && FP8_ROWS) {   // r: rows 0..7 / 8..15 x inputs 0..15, then inputs 16..31; four consecutive inputs per lane
     float odd[4] = {0.f, 0.f, 0.f, 0.f};
@@ -338,10 +348,22 @@ __device__ inline void build_tile_tasks(TileTask *tasks, int *nkb_out, int group
 }
 // Row of the gate/up phase's tiles that holds the up row of gate row r.
 __device__ __forceinline__ int up_row(int nch, int r) { return r + (GU_ONE_RUN ? nch * CH_ROWS : (nch + TILE_CH - 1) / TILE_CH * 16); }
-__device__ __forceinline__ void run_tile_task(const Params &P, const Ctx &c, const TileTask *tasks, int fslot) {
+// FP8 rows, several sequences: what a phase's first MMA waits for besides the activations - the task, the chunks' arrival, addresses -
+// is done in front of the wait for these, which is long there (sums drain for longer): two / three / four sequences at 1024 tokens
+// 560 / 633 / 710 -> 553 / 607 / 680 us per step.  One sequence 412 / 414; fp16 rows, whose phases take most of the ring, lose 4 %.
+// All warps then wait for their chunks before the first one hands any back: the phase and what a group of eight issues
+// with its last chunk must fit into the ring (TcTab::early).  The slots were last used two phases before, so the parity is that
+// of this use (every warp waits for all chunks of an O or down phase, and the row phases end with a barrier).
+constexpr bool EARLY_ROWS = FP8_ROWS && TC_SEQS > 1;
+__device__ __forceinline__ RowTile prepare_rows(const Params &P, const Ctx &c, const TileTask *tasks) {
   const int4 a = reinterpret_cast<const int4 *>(tasks + c.warp)[0], b = reinterpret_cast<const int4 *>(tasks + c.warp)[1];
   // a = {active, first, valid, p0}, b = {p1, units, -, -}
-  if (a.x) tile_task(P, c, c.chunk + static_cast<uint32_t>(a.y), a.z, a.w, b.x, tc_part(c) + c.warp * PART_TASK, b.y, fslot);
+  if (a.x) return prepare_tile(P, c, c.chunk + static_cast<uint32_t>(a.y), a.z, a.w, b.x, b.y);
+  RowTile none = {};
+  return none;
+}
+__device__ __forceinline__ void run_rows(const Ctx &c, const RowTile &rows, int fslot) {
+  if (rows.valid > 0) run_tile(c, rows, tc_part(c) + c.warp * PART_TASK, fslot);
 }
 
 // The phases are inlined into the kernel's layer loop.  As functions of their own they cost a call and its register moves (160
@@ -355,7 +377,7 @@ __device__ __forceinline__ uint32_t qkv_phase(const Params &P, Ctx c, uint32_t t
   const TcTab *t = tctab(c);
   const int nch = t->nq, nkb = t->nkb_qkv;
   QMK_FINE(0);
-  run_tile_task(P, c, t->qkv, 0);
+  run_rows(c, prepare_rows(P, c, t->qkv), 0);
   QMK_FINE(2);
   cons_sync();
   if (c.tid < nch * CH_ROWS) {
@@ -376,7 +398,7 @@ __device__ __forceinline__ uint32_t gateup_phase(const Params &P, Ctx c) {
   const TcTab *t = tctab(c);
   const int nch = t->ng, nkb = t->nkb_gu;
   QMK_FINE(10);
-  run_tile_task(P, c, t->gu, 10);
+  run_rows(c, prepare_rows(P, c, t->gu), 10);
   QMK_FINE(12);
   cons_sync();
   if (c.warp < 2) {          // warp 0 holds the slice; rows past it multiply stale bytes: zero activations
@@ -1147,8 +1169,8 @@ __device__ __forceinline__ uint32_t lm_head_tc(const Params &P, Ctx c, float *du
 #pragma unroll 1
   for (int tile = 0; tile < ntiles; ++tile) {
     float *pr = part + (tile & 1) * (CONS_WARPS * 16);
-    tile_task(P, c, c.chunk + static_cast<uint32_t>(tile * TILE_CH), min(16, (nch - tile * TILE_CH) * CH_ROWS), p0, p1, pr + c.warp * 16,
-              EMPTY_UNITS / CONS_WARPS);
+    run_tile(c, prepare_tile(P, c, c.chunk + static_cast<uint32_t>(tile * TILE_CH), min(16, (nch - tile * TILE_CH) * CH_ROWS), p0, p1,
+                             EMPTY_UNITS / CONS_WARPS), pr + c.warp * 16);
     cons_sync();
     if (c.tid < 16) {
       const int row = tile * 16 + c.tid;
@@ -1339,6 +1361,7 @@ __device__ __forceinline__ void tc_setup(const Params &P, const Ctx &c) {
     split_rows(QKV_CHUNKS, c.ncta, c.cta, a, b); tt->q0 = a; tt->nq = b - a;
     split_rows(GU_CHUNKS, c.ncta, c.cta, a, b); tt->g0 = a; tt->ng = b - a;
     split_rows(P.vocab / CH_ROWS, c.ncta, c.cta, a, b); tt->lm0 = a; tt->nlm = b - a;
+    tt->early = EARLY_ROWS && max(tt->nq, 2 * tt->ng) + 7 <= NSLOTS;
     tt->groups = c.ncta / O_GROUP;
     const int grp = c.cta / O_GROUP;
     tt->oq = c.cta % O_GROUP;

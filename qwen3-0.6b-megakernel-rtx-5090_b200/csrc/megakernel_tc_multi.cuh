@@ -37,10 +37,10 @@ __device__ __forceinline__ float *tc_resid(const Ctx &c, int which, int b) {
 __device__ __forceinline__ int *tc_tokens(const Ctx &c) { return reinterpret_cast<int *>(c.smem + OFF_TOKENS); }
 __device__ __forceinline__ int *tc_splits(const Ctx &c) { return reinterpret_cast<int *>(c.smem + OFF_TOKENS) + TC_SEQS; }   // of each sequence's attention in this step
 
-__device__ __forceinline__ uint32_t qkv_phase_seqs(const Params &P, Ctx c, uint32_t tag) {
+__device__ __forceinline__ uint32_t qkv_phase_seqs(const Params &P, Ctx c, const RowTile &rows, uint32_t tag) {
   const TcTab *t = tctab(c);
   const int nch = t->nq, nkb = t->nkb_qkv;
-  run_tile_task(P, c, t->qkv, 0);
+  run_rows(c, rows, 0);
   cons_sync();
   const int b = c.tid / TPS, r = c.tid % TPS;
   if (b < P.nseq && r < nch * CH_ROWS) {
@@ -54,10 +54,10 @@ __device__ __forceinline__ uint32_t qkv_phase_seqs(const Params &P, Ctx c, uint3
   return c.chunk + static_cast<uint32_t>(nch);
 }
 
-__device__ __forceinline__ uint32_t gateup_phase_seqs(const Params &P, Ctx c) {
+__device__ __forceinline__ uint32_t gateup_phase_seqs(const Params &P, Ctx c, const RowTile &rows) {
   const TcTab *t = tctab(c);
   const int nch = t->ng, nkb = t->nkb_gu;
-  run_tile_task(P, c, t->gu, 10);
+  run_rows(c, rows, 10);
   cons_sync();
   const int b = c.tid / TPS, r = c.tid % TPS;
   __half *act16 = reinterpret_cast<__half *>(c.smem + OFF_ACT16) + 2 * b * ACT16_PITCH;
@@ -382,8 +382,8 @@ __device__ __forceinline__ uint32_t lm_head_seqs(const Params &P, Ctx c, int ste
 #pragma unroll 1
   for (int tile = 0; tile < ntiles; ++tile) {
     float *pr = part + (tile & 1) * (CONS_WARPS * PART_TASK);
-    tile_task(P, c, c.chunk + static_cast<uint32_t>(tile * TILE_CH), min(16, (nch - tile * TILE_CH) * CH_ROWS), p0, p1,
-              pr + c.warp * PART_TASK, EMPTY_UNITS / CONS_WARPS);
+    run_tile(c, prepare_tile(P, c, c.chunk + static_cast<uint32_t>(tile * TILE_CH), min(16, (nch - tile * TILE_CH) * CH_ROWS), p0, p1,
+                             EMPTY_UNITS / CONS_WARPS), pr + c.warp * PART_TASK);
     cons_sync();
     if (b < P.nseq) {
       const int row = tile * 16 + r;
@@ -507,6 +507,8 @@ __global__ void __launch_bounds__(THREADS, 1) qwen3_decode_megakernel_tc_seqs(co
         mbar_wait(P, c, c.nfull(L0 & 1u), (L0 >> 1) & 1u, WHERE_FULL, false);
         embed_norm_seqs(P, c, c.norms(L0 & 1u) + NB_IN_LN);
       }
+      RowTile rows = {};
+      const bool early = EARLY_ROWS && tctab(c)->early;
 #pragma unroll 1
       for (int layer = 0; layer < P.num_layers; ++layer) {
         const uint32_t tag = tag_base + static_cast<uint32_t>(layer) + 1u;
@@ -514,7 +516,8 @@ __global__ void __launch_bounds__(THREADS, 1) qwen3_decode_megakernel_tc_seqs(co
         const __half *nv = c.norms(Lg & 1u);
         const uint32_t use = Lg + 1u;
         QMK_STAMP(layer * 12 + 0);
-        c.chunk = qkv_phase_seqs(P, c, tag);
+        if (!early || layer == 0) rows = prepare_rows(P, c, tctab(c)->qkv);
+        c.chunk = qkv_phase_seqs(P, c, rows, tag);
         QMK_STAMP(layer * 12 + 1);
         c.chunk = attention_tc(P, c, nv, layer, pos, tag);
         QMK_STAMP(layer * 12 + 2);
@@ -523,15 +526,18 @@ __global__ void __launch_bounds__(THREADS, 1) qwen3_decode_megakernel_tc_seqs(co
         cons_sync();
         c.chunk = slice_o_seqs(P, c);
         QMK_STAMP(layer * 12 + 4);
+        if (early) rows = prepare_rows(P, c, tctab(c)->gu);
         red_wait_norm_seqs(P, c, 0, use, nv + NB_POST_LN);
         QMK_STAMP(layer * 12 + 5);
-        c.chunk = gateup_phase_seqs(P, c);
+        if (!early) rows = prepare_rows(P, c, tctab(c)->gu);
+        c.chunk = gateup_phase_seqs(P, c, rows);
         QMK_STAMP(layer * 12 + 6);
         cons_sync();
         c.chunk = slice_cols_seqs(P, c);
         QMK_STAMP(layer * 12 + 7);
         const bool last = layer == P.num_layers - 1;
         if (!last) mbar_wait(P, c, c.nfull((Lg + 1u) & 1u), ((Lg + 1u) >> 1) & 1u, WHERE_FULL, false);
+        if (early && !last) rows = prepare_rows(P, c, tctab(c)->qkv);
         red_wait_norm_seqs(P, c, 1, use, last ? P.final_norm : c.norms((Lg + 1u) & 1u) + NB_IN_LN);
         QMK_STAMP(layer * 12 + 8);
         if (cons_any(c.flags()[0] != 0)) break;
