@@ -357,6 +357,16 @@ int qmk_prefill_packed(
     void *const *k_caches, void *const *v_caches, int num_layers, int max_seq_len,
     float attn_scale, cudaStream_t stream);
 
+/* Any number of passes of qmk_prefill_packed, one behind the other: pass p takes the next seqs_per_pass[p] sequences of the
+ * concatenated arrays, under the limits of one call each.  The same rows as calls of their own leave; the host prepares a
+ * pass while the one before runs and waits once, behind the last.  An argument that a pass refuses is reported when its turn
+ * comes, the passes before it have run then; a device status of any pass is the call's.  Blocks. */
+int qmk_prefill_packed_passes(
+    const int *token_ids_host, int num_passes, const int *seqs_per_pass, const int *seq_lens, const void *embed_weight,
+    const struct LDGLayerWeight *layer_weights, const void *cos_table, const void *sin_table,
+    void *const *k_caches, void *const *v_caches, int num_layers, int max_seq_len,
+    float attn_scale, cudaStream_t stream);
+
 /* Greedy decode of up to 128 sequences on the tensor-core path (the batched configurations): each step runs
  * the seven projections and the LM head as tcgen05 GEMMs over one row tile of sequences (64 or 128 rows), with row kernels
  * for the norms, per-head QK-norm + RoPE + cache write (each sequence at its own position in its own cache),

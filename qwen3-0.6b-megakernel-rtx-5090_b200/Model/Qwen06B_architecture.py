@@ -377,8 +377,8 @@ class BatchDecoder:
                                                    for _ in range(self.num_sequences - 1)]
         self._v_caches = [self._base._v_cache] + [torch.zeros_like(self._base._v_cache)
                                                    for _ in range(self.num_sequences - 1)]
-        self._logs = [torch.full((self.max_seq_len,), -1, dtype=torch.int32, device=dev)
-                      for _ in range(self.num_sequences)]
+        self._all_logs = torch.full((self.num_sequences, self.max_seq_len), -1, dtype=torch.int32, device=dev)
+        self._logs = list(self._all_logs.unbind(0))
         self._logs_cpu = torch.empty(self.num_sequences, self.max_seq_len, dtype=torch.int32).pin_memory()
         self.positions = [0] * self.num_sequences
         self._gen_batch = _require_megakernel_op("generate_batch" if engine == "persistent" else "decode_batched")
@@ -442,53 +442,67 @@ class BatchDecoder:
         """Prefill any number of slots: in packed passes of up to ``packed_prefill_rows`` rows where the engine has
         them, a prompt longer than that (or any prompt of an engine without packed prefill) through ``prefill_slot``."""
         budget = self.packed_prefill_rows
-        group, rows = [], 0
+        passes, group, rows = [], [], 0      # packed passes that go to the device together; the one being filled
 
-        def flush():
+        def close():
             nonlocal group, rows
             if len(group) == 1:
+                send()
                 self.prefill_slot(*group[0])
             elif group:
-                self.prefill_slots([b for b, _ in group], [ids for _, ids in group])
+                passes.append(group)
             group, rows = [], 0
+
+        def send():
+            if passes:
+                self._prefill_passes(passes)
+                passes.clear()
         for b, ids in zip(slots, prompts):
             need = (max(len(ids), 1) + 127) // 128 * 128
             if budget <= 0 or need > budget:
+                send()
                 self.prefill_slot(b, ids)
                 continue
             if group and (rows + need > budget or len(group) == 64):
-                flush()
+                close()
             group.append((b, list(ids)))
             rows += need
-        flush()
+        close()
+        send()
 
     def prefill_slots(self, slots: Sequence[int], prompts: Sequence[Sequence[int]]) -> None:
         """Fill the caches of several slots in ONE tensor-core pass (``qmk_prefill_packed``): weights are read once for all
         of them and a pass's ~200 launches are shared.  Empty prompts are skipped (their slot starts at position 0)."""
-        slots = [int(b) for b in slots]
-        if len(slots) != len(prompts) or len(set(slots)) != len(slots) or not all(0 <= b < self.num_sequences for b in slots):
-            raise ValueError("slots must be distinct, in range, one per prompt")
+        self._prefill_passes([[(int(b), list(ids)) for b, ids in zip(slots, prompts)]] if len(slots) == len(prompts) else [None])
+
+    def _prefill_passes(self, passes) -> None:
+        """``prefill_slots`` passes, each a list of (slot, prompt), one behind the other."""
+        for group in passes:
+            slots = [b for b, _ in group] if group is not None else None
+            if slots is None or len(set(slots)) != len(slots) or not all(0 <= b < self.num_sequences for b in slots):
+                raise ValueError("slots must be distinct, in range, one per prompt")
         base = self._base
         if base.prefill_mode != "tensor":
             raise RuntimeError("prefill_slots needs prefill_mode='tensor'")
-        todo = [(b, list(ids)) for b, ids in zip(slots, prompts) if len(ids) > 0]
-        for _, ids in todo:
-            if len(ids) > self.max_seq_len:
-                raise ValueError("prompt exceeds max_seq_len")
+        todo = [[(b, ids) for b, ids in group if len(ids) > 0] for group in passes]
+        todo = [group for group in todo if group]
+        if any(len(ids) > self.max_seq_len for group in todo for _, ids in group):
+            raise ValueError("prompt exceeds max_seq_len")
         if todo:
             base.apply_options()
-            args = ([ids for _, ids in todo], base._embed_weight, base._layer_weights_packed, base._cos_table, base._sin_table,
-                    [self._k_caches[b] for b, _ in todo], [self._v_caches[b] for b, _ in todo], base.num_layers, self.max_seq_len,
-                    base._attn_scale)
-            op = _require_megakernel_op("prefill_packed")
+            flat = [item for group in todo for item in group]
+            args = ([len(group) for group in todo], [ids for _, ids in flat], base._embed_weight, base._layer_weights_packed, base._cos_table,
+                    base._sin_table, [self._k_caches[b] for b, _ in flat], [self._v_caches[b] for b, _ in flat], base.num_layers,
+                    self.max_seq_len, base._attn_scale)
+            op = _require_megakernel_op("prefill_packed_passes")
             if self._prefill_stream is not None:
                 with torch.cuda.stream(self._prefill_stream):   # the op blocks until its stream is idle
                     op(*args)
             else:
                 op(*args)
-        for b, ids in zip(slots, prompts):
-            self.positions[b] = len(ids)
-
+        for group in passes:
+            for b, ids in group:
+                self.positions[b] = len(ids)
 
     def decode_slots(self, slots: Sequence[int], first_tokens: Sequence[int], steps: int) -> List[List[int]]:
         """One launch: ``steps`` greedy tokens for every slot in ``slots`` (any subset, each from its own
@@ -545,8 +559,7 @@ class BatchDecoder:
             return [[] for _ in range(n)]
         base = self._base
         logs = [self._logs[b][:max_tokens] for b in range(n)]
-        for log in logs:
-            log.fill_(-1)
+        self._all_logs[:n, :max_tokens].fill_(-1)
         base.apply_options()
         self._gen_batch(firsts, self.positions[:n], max_tokens, base._embed_weight, base._layer_weights_packed,
                         base._final_norm_weight, base._lm_head_weight, base._cos_table, base._sin_table,
@@ -554,11 +567,9 @@ class BatchDecoder:
                         base._attn_scale)
         eos = base._eos()
         outs: List[List[int]] = []
-        for b in range(n):
-            host = self._logs_cpu[b, :max_tokens]
-            host.copy_(logs[b])
+        for b, tokens in enumerate(self._all_logs[:n, :max_tokens].cpu().tolist()):
             out: List[int] = []
-            for tok in host.tolist():
+            for tok in tokens:
                 if tok == -1 or tok == eos:
                     break
                 out.append(tok)

@@ -519,6 +519,9 @@ struct Workspace {                  // per device, allocated on first use, never
   __half **k_ptrs = nullptr, **v_ptrs = nullptr;
   CUtensorMap *kv_maps = nullptr;        // [128][2]: tiled-copy descriptors of every sequence's K and V cache (decode_attention_mma)
   unsigned char *packed = nullptr;       // tables of a packed prefill (row info, attention items, per-sequence descriptors and cache pointers)
+  // pinned source of these tables and the pass's tokens, two that passes take in turn: a pass is prepared while the one before runs
+  unsigned char *staging[2] = {nullptr, nullptr};
+  cudaEvent_t staged[2] = {nullptr, nullptr};   // the copies out of it are done
   int **log_ptrs = nullptr;
   float *split_part = nullptr;            // partial attention states of split sequences (both decode attention kernels)
   qmk_pf::DamPlan *attn_plan = nullptr;   // the step's list of attention pieces (decode_attention_mma)
@@ -691,13 +694,28 @@ struct PackedSeqs {
   const int *lens;
   void *const *k_caches, *const *v_caches;
 };
+// One of the passes of a call: the first one reads the layer table and clears the status, the last one waits and reports.
+struct Pass { bool first = true, last = true; int index = 0; };
 constexpr int MAX_PACKED_SEQS = 64;
 constexpr size_t PK_ROWS_OFF = 0, PK_ITEMS_OFF = 32768, PK_MAPS_OFF = 49152, PK_PTRS_OFF = 65536, PK_BYTES = 66560;
+
+// Null where pinned memory is refused: pageable memory serves then, whose copies may hold the host up.
+unsigned char *staging_slot(Workspace &w, int slot) {
+  if (!w.staging[slot]) {
+    void *at = nullptr;
+    cudaEvent_t done = nullptr;
+    if (cudaHostAlloc(&at, PK_BYTES + sizeof(int) * CHUNK, cudaHostAllocDefault) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    if (cudaEventCreateWithFlags(&done, cudaEventDisableTiming) != cudaSuccess) { cudaGetLastError(); cudaFreeHost(at); return nullptr; }
+    w.staging[slot] = static_cast<unsigned char *>(at);
+    w.staged[slot] = done;
+  }
+  return w.staging[slot];
+}
 
 int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_weight, const LDGLayerWeight *layer_weights,
                  const void *cos_table, const void *sin_table, void *k_cache, void *v_cache, int num_layers,
                  int start_position, int max_seq_len, float attn_scale, cudaStream_t stream, const PackedSeqs *pk, bool split,
-                 bool *take_steps = nullptr) {
+                 bool *take_steps = nullptr, const Pass &pass = Pass()) {
   using namespace qmk_pf;
   if (num_tokens <= 0) return QMK_OK;
   qmk_internal::PrefillEnv env;
@@ -735,25 +753,32 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
   std::lock_guard<std::recursive_mutex> lock(g_ws_mu);
   Workspace &w = g_ws[dev];
   rc = ensure_workspace(w, CHUNK, take_steps);
-  if (rc == QMK_OK) rc = ensure_weight_maps(w, layer_weights, num_layers, wq, stream);
+  if (rc == QMK_OK && pass.first) rc = ensure_weight_maps(w, layer_weights, num_layers, wq, stream);
   if (rc != QMK_OK) return rc;
   // ---- packed prompts: rows = the sequences one after the other, each padded to whole 128-row tiles
-  std::vector<int> padded_tokens;
-  std::vector<unsigned char> pk_host;
+  std::vector<unsigned char> pageable;
+  const int slot = pass.index & 1;
   int pk_items = 0;
   if (pk) {
     if (!env.attn_tc) return qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "packed prefill needs the tcgen05 attention kernel");
     if (!w.packed) PF_CUDA(cudaMalloc(&w.packed, PK_BYTES));
-    pk_host.assign(PK_BYTES, 0);
-    int2 *rows = reinterpret_cast<int2 *>(pk_host.data() + PK_ROWS_OFF);
-    int4 *items = reinterpret_cast<int4 *>(pk_host.data() + PK_ITEMS_OFF);
-    CUtensorMap *maps = reinterpret_cast<CUtensorMap *>(pk_host.data() + PK_MAPS_OFF);
-    unsigned long long *ptrs = reinterpret_cast<unsigned long long *>(pk_host.data() + PK_PTRS_OFF);
+    unsigned char *host = staging_slot(w, slot);
+    if (host) {
+      PF_CUDA(cudaEventSynchronize(w.staged[slot]));      // (two passes back)
+    } else {
+      pageable.resize(PK_BYTES + sizeof(int) * CHUNK);
+      host = pageable.data();
+    }
+    memset(host, 0, PK_BYTES);
+    int *const padded_tokens = reinterpret_cast<int *>(host + PK_BYTES);
+    int2 *rows = reinterpret_cast<int2 *>(host + PK_ROWS_OFF);
+    int4 *items = reinterpret_cast<int4 *>(host + PK_ITEMS_OFF);
+    CUtensorMap *maps = reinterpret_cast<CUtensorMap *>(host + PK_MAPS_OFF);
+    unsigned long long *ptrs = reinterpret_cast<unsigned long long *>(host + PK_PTRS_OFF);
     int total_rows = 0;
     for (int s = 0; s < pk->num_seqs; ++s) total_rows += (pk->lens[s] + qmk_gemm::BM - 1) / qmk_gemm::BM * qmk_gemm::BM;
     if (total_rows > CHUNK) return qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "packed prefill: more than 4096 padded rows");
-    padded_tokens.assign(total_rows, 0);
-    for (int i = 0; i < total_rows; ++i) rows[i] = make_int2(0, -1);
+    for (int i = 0; i < total_rows; ++i) { padded_tokens[i] = 0; rows[i] = make_int2(0, -1); }
     std::vector<std::pair<int, int4>> order;   // (key tiles, item)
     std::string merr;
     int row0 = 0, tok0 = 0;
@@ -782,15 +807,15 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     std::stable_sort(order.begin(), order.end(), [](const auto &a, const auto &b) { return a.first > b.first; });   // longest job first
     pk_items = static_cast<int>(order.size());
     for (int i = 0; i < pk_items; ++i) items[i] = order[i].second;
-    PF_CUDA(cudaMemcpyAsync(w.packed, pk_host.data(), PK_BYTES, cudaMemcpyHostToDevice, stream));
-    token_ids_host = padded_tokens.data();
+    PF_CUDA(cudaMemcpyAsync(w.packed, host, PK_BYTES, cudaMemcpyHostToDevice, stream));
+    token_ids_host = padded_tokens;
     num_tokens = total_rows;
   }
   std::vector<unsigned long long> rec(w.table, w.table + static_cast<size_t>(num_layers) * 12);
   const float *rope = env.rope_from_table ? nullptr : env.rope;
   const __half *cosv = static_cast<const __half *>(cos_table), *sinv = static_cast<const __half *>(sin_table);
   const size_t layer_stride = static_cast<size_t>(NKV) * max_seq_len * D;
-  PF_CUDA(cudaMemsetAsync(w.status, 0, 16, stream));
+  if (pass.first) PF_CUDA(cudaMemsetAsync(w.status, 0, 16, stream));
   std::string err;
   // weight matrix j of layer l in boxes of `box_n` rows
   auto wmap_for = [&](int l, int j, int box_n) -> const CUtensorMap & {
@@ -908,6 +933,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
       if (rc != QMK_OK) break;
     }
     PF_CUDA(cudaMemcpyAsync(w.tokens, token_ids_host + c0, sizeof(int) * T, cudaMemcpyHostToDevice, stream));
+    if (pk && pageable.empty()) PF_CUDA(cudaEventRecord(w.staged[slot], stream));
     // Every kernel behind the first launches as a programmatic dependent: its set-up (and a GEMM's first ring fill of WEIGHT
     // tiles) runs under the tail of the kernel before it.  In order are, with each kernel waiting for its predecessor before
     // its first dependent read and any write: the residual rows and sums; the expanded matrices of a packed layer
@@ -1030,6 +1056,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     PF_CUDA(cudaGetLastError());     // (the next chunk's token copy is stream-ordered behind this chunk's kernels)
   }
   if (rc != QMK_OK) return qmk_internal::report(rc, err);
+  if (!pass.last) return QMK_OK;
   unsigned int host_status[4] = {0, 0, 0, 0};
   PF_CUDA(cudaMemcpyAsync(host_status, w.status, 16, cudaMemcpyDeviceToHost, stream));
   PF_CUDA(cudaStreamSynchronize(stream));
@@ -1078,6 +1105,36 @@ extern "C" int qmk_prefill_packed(const int *token_ids_host, int num_seqs, const
   const PackedSeqs pk = {num_seqs, seq_lens, k_caches, v_caches};
   return prefill_impl(token_ids_host, static_cast<int>(total), embed_weight, layer_weights, cos_table, sin_table, nullptr, nullptr,
                       num_layers, 0, max_seq_len, attn_scale, stream, &pk, false);
+}
+
+extern "C" int qmk_prefill_packed_passes(const int *token_ids_host, int num_passes, const int *seqs_per_pass, const int *seq_lens,
+                                         const void *embed_weight, const LDGLayerWeight *layer_weights, const void *cos_table,
+                                         const void *sin_table, void *const *k_caches, void *const *v_caches, int num_layers,
+                                         int max_seq_len, float attn_scale, cudaStream_t stream) {
+  qmk_internal::begin_call();
+  if (num_passes <= 0) return QMK_OK;
+  if (!token_ids_host || !seqs_per_pass || !seq_lens || !k_caches || !v_caches)
+    return qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "packed prefill: null array argument");
+  for (int p = 0; p < num_passes; ++p)
+    if (seqs_per_pass[p] < 1 || seqs_per_pass[p] > MAX_PACKED_SEQS)
+      return qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "packed prefill: 1 to 64 sequences a pass, each from position 0");
+  std::lock_guard<std::recursive_mutex> lock(g_ws_mu);   // (the passes share one workspace and one status)
+  int rc = QMK_OK;
+  for (int p = 0, s0 = 0; p < num_passes && rc == QMK_OK; s0 += seqs_per_pass[p++]) {
+    long total = 0;
+    for (int s = 0; s < seqs_per_pass[p]; ++s) total += seq_lens[s0 + s] > 0 ? seq_lens[s0 + s] : 0;
+    const PackedSeqs pk = {seqs_per_pass[p], seq_lens + s0, k_caches + s0, v_caches + s0};
+    Pass pass;
+    pass.first = p == 0;
+    pass.last = p + 1 == num_passes;
+    pass.index = p;
+    rc = total < 1 ? qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "packed prefill: empty sequence or null cache")
+                   : prefill_impl(token_ids_host, static_cast<int>(total), embed_weight, layer_weights, cos_table, sin_table, nullptr, nullptr,
+                                  num_layers, 0, max_seq_len, attn_scale, stream, &pk, false, nullptr, pass);
+    if (rc != QMK_OK && p > 0) cudaStreamSynchronize(stream);   // the passes before it are done, as behind calls of their own
+    token_ids_host += total;
+  }
+  return rc;
 }
 
 // ----------------------------------------------------------------------------- batched decode on the GEMM path

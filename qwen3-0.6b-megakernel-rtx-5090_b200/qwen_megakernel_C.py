@@ -15,6 +15,7 @@ Additions with no counterpart in the reference are grouped at the bottom
 
 from __future__ import annotations
 
+import array
 import ctypes
 import os
 
@@ -83,6 +84,8 @@ _lib.qmk_prefill_chunked.argtypes = [_P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I,
 _lib.qmk_prefill_chunked.restype = _I
 _lib.qmk_prefill_packed.argtypes = [_P, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _F, _P]
 _lib.qmk_prefill_packed.restype = _I
+_lib.qmk_prefill_packed_passes.argtypes = [_P, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _F, _P]
+_lib.qmk_prefill_packed_passes.restype = _I
 _lib.qmk_gemm_f16_tn.argtypes = [_P, _P, _P, _I, _I, _I, _P]
 _lib.qmk_gemm_f16_tn.restype = _I
 _lib.qmk_gemm_packed_tn.argtypes = [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P]
@@ -124,7 +127,7 @@ _lib.qmk_selftest_gemm_pair_wait_timeout.restype = _I
 EXPORTED_SYMBOLS = (
     "launch_ldg_decode_direct", "launch_ldg_decode_persistent", "launch_ldg_generate_nosync",
     "launch_ldg_prefill", "qmk_abi_version", "qmk_configure", "qmk_set_inv_freq", "qmk_set_logits_dump",
-    "qmk_set_weight_format", "qmk_set_tuning", "qmk_set_tuning2", "qmk_set_profile_buffer", "qmk_set_fused", "qmk_set_step_overlap", "qmk_set_prefill_attention", "qmk_set_decode_attention", "qmk_invalidate_weights", "qmk_release_weights", "qmk_decode", "qmk_generate", "qmk_generate_static", "qmk_generate_batch", "qmk_gemm_f16_tn", "qmk_gemm_packed_tn", "qmk_decode_batched", "qmk_prefill_chunked", "qmk_prefill_packed", "qmk_prefill", "qmk_engine_create", "qmk_engine_destroy", "qmk_engine_apply", "qmk_engine_decode", "qmk_engine_generate", "qmk_engine_prefill", "qmk_sync_status", "qmk_last_error", "qmk_num_ctas",
+    "qmk_set_weight_format", "qmk_set_tuning", "qmk_set_tuning2", "qmk_set_profile_buffer", "qmk_set_fused", "qmk_set_step_overlap", "qmk_set_prefill_attention", "qmk_set_decode_attention", "qmk_invalidate_weights", "qmk_release_weights", "qmk_decode", "qmk_generate", "qmk_generate_static", "qmk_generate_batch", "qmk_gemm_f16_tn", "qmk_gemm_packed_tn", "qmk_decode_batched", "qmk_prefill_chunked", "qmk_prefill_packed", "qmk_prefill_packed_passes", "qmk_prefill", "qmk_engine_create", "qmk_engine_destroy", "qmk_engine_apply", "qmk_engine_decode", "qmk_engine_generate", "qmk_engine_prefill", "qmk_sync_status", "qmk_last_error", "qmk_num_ctas",
     "qmk_scratch_bytes", "qmk_selftest_wait_timeout", "qmk_selftest_gemm_wait_timeout", "qmk_selftest_attention_wait_timeout", "qmk_selftest_gemm_pair_wait_timeout", "qmk_selftest_decode_attention_wait_timeout",
 )
 
@@ -513,22 +516,46 @@ def prefill_chunked(token_ids, embed_weight, layer_weights_packed, cos_table, si
     return None
 
 
+def _c_ints(token_lists):
+    """The lists' integers one after the other, as a C array."""
+    try:
+        flat = array.array("i")
+        for ids in token_lists:
+            flat.extend(ids)
+        return (ctypes.c_int * max(len(flat), 1)).from_buffer(flat if flat else array.array("i", [0]))
+    except (TypeError, OverflowError):     # whatever int() takes
+        flat = [int(t) for ids in token_lists for t in ids]
+        return (ctypes.c_int * max(len(flat), 1))(*flat)
+
+
 def prefill_packed(token_lists, embed_weight, layer_weights_packed, cos_table, sin_table, k_caches, v_caches,
                    num_layers, max_seq_len, attn_scale):
     """Several prompts in one tensor-core prefill pass: ``token_lists[s]`` (ints) fills ``k_caches[s]`` / ``v_caches[s]``
     from position 0.  At most 64 sequences and 4096 rows after padding each prompt to a multiple of 128.  Blocks;
     raises ``RuntimeError`` on any reported error."""
+    return prefill_packed_passes([len(token_lists)], token_lists, embed_weight, layer_weights_packed, cos_table, sin_table, k_caches,
+                                 v_caches, num_layers, max_seq_len, attn_scale)
+
+
+def prefill_packed_passes(seqs_per_pass, token_lists, embed_weight, layer_weights_packed, cos_table, sin_table, k_caches, v_caches,
+                          num_layers, max_seq_len, attn_scale):
+    """``prefill_packed`` passes one behind the other, pass ``p`` with the next ``seqs_per_pass[p]`` prompts; the GPU does not
+    wait for the host between them."""
     _require_cuda()
     n = len(token_lists)
     _check(n >= 1 and n == len(k_caches) == len(v_caches), "prefill_packed: one cache pair per prompt")
+    _check(sum(seqs_per_pass) == n, "prefill_packed: the passes take all prompts")
     _check_table(layer_weights_packed, "prefill_packed")
-    flat = [int(t) for ids in token_lists for t in ids]
-    tok = (ctypes.c_int * max(len(flat), 1))(*flat)
+    tok = _c_ints(token_lists)
     lens = (ctypes.c_int * n)(*[len(ids) for ids in token_lists])
     kp = (ctypes.c_void_p * n)(*[_ptr(c) for c in k_caches])
     vp = (ctypes.c_void_p * n)(*[_ptr(c) for c in v_caches])
-    rc = _lib.qmk_prefill_packed(tok, n, lens, _ptr(embed_weight), _ptr(layer_weights_packed), _ptr(cos_table), _ptr(sin_table),
-                                 kp, vp, int(num_layers), int(max_seq_len), float(attn_scale), _stream())
+    tail = (lens, _ptr(embed_weight), _ptr(layer_weights_packed), _ptr(cos_table), _ptr(sin_table), kp, vp, int(num_layers),
+            int(max_seq_len), float(attn_scale), _stream())
+    if len(seqs_per_pass) == 1:
+        rc = _lib.qmk_prefill_packed(tok, n, *tail)
+    else:
+        rc = _lib.qmk_prefill_packed_passes(tok, len(seqs_per_pass), (ctypes.c_int * len(seqs_per_pass))(*seqs_per_pass), *tail)
     if rc != 0:
         raise RuntimeError(f"prefill_packed: {_lib.qmk_last_error().decode()} (status {rc})")
     return None

@@ -353,3 +353,47 @@ def test_gpu_four_slots_with_tensor_prefill(built_library, overlap):
     sch.run_until_idle()
     sch.stop()
     assert [f.result(timeout=0).tokens for f in futs] == want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt", ["fp16", "fp8"])
+def test_gpu_packed_passes_of_one_call(built_library, fmt):
+    """Four packed passes (4096, 4096, 3968 and 768 rows) sent to the device in one call, each prepared while the one before
+    runs, leave the cache rows of four calls bit for bit: the same kernels on the same rows.  A prompt on its own between
+    two groups still takes the chunked pass.  A pass that is refused is reported, and the next call works."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import qwen_megakernel_C as C
+    import quantize as Q
+    from Model.Qwen06B_architecture import BatchDecoder
+    vocab = 2048
+    w = S.make_weights(seed=9, num_layers=2, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    if fmt == "fp8":
+        w, _ = Q.quantize_weights_fp8(w)
+    lens = [1900, 2100, 4000, 2000, 1, 1900, 60, 1500, 1280, 1000, 0, 700, 60]
+    prompts = [S.make_prompt(n, seed=500 + i, vocab_size=vocab) if n else [] for i, n in enumerate(lens)]
+    eng = BatchDecoder(weights=S.weights_to(w, "cuda"), tokenizer=S.StubTokenizer(-1, vocab), num_sequences=len(lens), max_seq_len=4096,
+                       engine="gemm", prefill_mode="tensor", weight_format=fmt)
+    try:
+        groups = [[0, 1], [2], [3, 4, 5], [6, 7, 8, 9, 10], [11, 12]]
+        for g in groups:
+            if len(g) == 1:
+                eng.prefill_slot(g[0], prompts[g[0]])
+            else:
+                eng.prefill_slots(g, [prompts[b] for b in g])
+        want = [(k.clone(), v.clone()) for k, v in zip(eng._k_caches, eng._v_caches)]
+        for k, v in zip(eng._k_caches, eng._v_caches):
+            k.zero_()
+            v.zero_()
+        for _ in range(2):
+            eng.prefill_many(list(range(len(lens))), prompts)
+            assert eng.positions == lens
+            for b, (k, v) in enumerate(want):
+                assert torch.equal(eng._k_caches[b], k) and torch.equal(eng._v_caches[b], v), b
+        with pytest.raises(RuntimeError, match="vocab"):
+            eng.prefill_many([0, 1, 3, 5, 7], [prompts[0], prompts[1], prompts[3], prompts[5][:-1] + [vocab], prompts[7]])
+        eng.prefill_many([0, 1, 3, 5, 7], [prompts[b] for b in (0, 1, 3, 5, 7)])
+        for b in (0, 1, 3, 5, 7):
+            assert torch.equal(eng._k_caches[b][:, :, :lens[b]], want[b][0][:, :, :lens[b]])
+    finally:
+        C.set_weight_format("fp16")
