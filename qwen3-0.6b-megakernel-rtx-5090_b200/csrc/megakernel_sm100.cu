@@ -33,6 +33,7 @@
 #include <string.h>
 #include <stdlib.h>
 #include <math.h>
+#include <algorithm>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -570,7 +571,7 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
   e->seq += static_cast<uint32_t>(P.num_steps);
 
   void *args[] = {&P};
-  const int grid = grid_for(e);
+  int grid = grid_for(e);
   const void *kernel = batch ? qmk_batch::kernel() : single_sequence_kernel(grid);
   size_t smem = batch ? qmk_batch::smem_bytes() : qmk::SMEM_BYTES;
   int threads = batch ? qmk_batch::threads() : qmk::THREADS;
@@ -592,6 +593,13 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
       kernel = tc.kernel;
       smem = tc.smem_bytes;
       threads = qmk::THREADS;
+      // Two fp16 sequences: 128 CTAs have whole tiles everywhere (32 q|k|v, 48 gate / up rows, slices of 64 attention outputs: a CTA of 148
+      // multiplies as many) and fewer contributions and readers to every sum.  us per step on 148 / 136 / 128 / 124 CTAs, 64 tokens 511 / 491
+      // / 479 / 576, 1024 tokens 541 / 530 / 509 / 593; from about 2200 tokens on (566 / 583 / 566) the attention misses the others.  FP8 rows
+      // (1024 tokens 554 / 543 on 148 / 128, 64 tokens 500 / 508), three (635 / 662) and one (436 / 446) stay on all.
+      int longest = 0;
+      for (int b = 0; b < P.nseq; ++b) longest = std::max(longest, P.start_positions[b] + P.num_steps);
+      if (P.nseq == 2 && e->wfmt == 0 && grid > 128 && longest <= 2048) grid = 128;
     }
   }
   if (!batch && e->fused && grid >= qmk::FUSED_MIN_CTAS &&

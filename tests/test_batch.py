@@ -268,3 +268,17 @@ def test_attention_slices_of_every_grid(C, fmt, n, ctas):
     for b in range(n):
         assert got[b] == want[b]
         assert float((dump[b] - logits[b]).abs().max()) < LOGIT_TOL
+
+
+@pytest.mark.parametrize("length", [2030, 2045])
+def test_two_sequences_either_side_of_the_smaller_grid(C, length):
+    """Two fp16 sequences take 128 CTAs up to 2048 positions and the whole device beyond (18 steps from 2030 end at 2047, from 2045 at
+    2062): the oracle's tokens, logits within the bound of every launch."""
+    w = S.make_weights(seed=31, num_layers=2, vocab_size=2048, norm_std=0.1, max_seq_len=16)
+    prompts = [S.make_prompt(n, seed=80 + n, vocab_size=2048) for n in (length, 700)]
+    want, logits = _oracle(w, 2080, prompts, 18)
+    eng = _batch_engine(w, 2, 2080)
+    got, dump = _run_with_dump(C, eng, prompts, 18, 2048)
+    for b in range(2):
+        assert got[b] == want[b]
+        assert float((dump[b] - logits[b]).abs().max()) < LOGIT_TOL
