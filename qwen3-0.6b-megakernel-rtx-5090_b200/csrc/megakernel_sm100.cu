@@ -99,6 +99,9 @@ struct PrepArgs {
   int num_layers, wfmt, parity, force;
   int quarters;                   // O rows by quarters of the outputs, as the tensor-core kernels read them (LayerT)
   int all, all_parity;            // compare the hashes of all bytes too (kmajor_hash_kernel ran before)
+  unsigned long long *red;        // the launch's residual sums and status words, cleared here: two memory sets less in front of it
+  int red_words;
+  unsigned int *status;
 };
 __device__ __forceinline__ const unsigned char *prep_matrix(const PrepArgs &a, int m) {
   return reinterpret_cast<const unsigned char *>((m & 1) ? a.layers[m >> 1].w_down : a.layers[m >> 1].wo);
@@ -137,6 +140,11 @@ __global__ void __launch_bounds__(256) kmajor_prepare_kernel(const PrepArgs a) {
   const size_t in_row = prep_row_bytes(a, m);
   const size_t n16 = in_row * H / 16;
   const int M = 2 * a.num_layers;
+  {
+    const int first = (m * PREP_SUB + static_cast<int>(blockIdx.x)) * 256 + t;
+    for (int i = first; i < a.red_words; i += M * PREP_SUB * 256) a.red[i] = 0ull;
+    if (first < 4) a.status[first] = 0u;
+  }
   unsigned long long before = 0, all_before = 0, all_now = 0;   // (asked for beside the samples, not behind them)
   if (t == 0) {
     before = a.fp[static_cast<size_t>(a.parity) * M + m];
@@ -428,7 +436,9 @@ constexpr size_t MAX_PREPARED = 4;   // weight sets kept per device (a 28-layer 
 // `several` (sequences): every byte of the matrices is checked, and where the copies do not fit in memory *out stays null
 // instead of an error.
 // `quarters`: the layout of the tensor-core kernels (a set of its own, as each weight format is).
-int ensure_prepared(Engine *e, const Params &P, int wfmt, bool quarters, cudaStream_t stream, Engine::Prepared **out, bool several = false) {
+// The kernel also clears the status and `red_words` words of the residual sums.
+int ensure_prepared(Engine *e, const Params &P, int wfmt, bool quarters, int red_words, cudaStream_t stream, Engine::Prepared **out,
+                    bool several = false) {
   Engine::Prepared *hit = nullptr;
   for (auto &p : e->prepared)
     if (p.table == P.layers && p.num_layers == P.num_layers && p.wfmt == wfmt && p.quarters == quarters) hit = &p;
@@ -477,6 +487,9 @@ int ensure_prepared(Engine *e, const Params &P, int wfmt, bool quarters, cudaStr
   a.force = hit->force;
   a.all = several ? 1 : 0;
   a.all_parity = hit->all_parity;
+  a.red = e->red;
+  a.red_words = red_words;
+  a.status = e->status;
   if (several) {
     QMK_CUDA(e, cudaMemsetAsync(hit->fp + 8 * P.num_layers, 0, sizeof(unsigned long long) * 2 * P.num_layers, stream));
     qmk::kmajor_hash_kernel<<<dim3(qmk::PREP_SUB, 2 * P.num_layers), 256, 0, stream>>>(a);
@@ -553,7 +566,6 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
   rc = ensure_rope(e, P.max_seq_len, stream);
   if (rc != QMK_OK) return rc;
   P.rope = e->rope;
-  QMK_CUDA(e, cudaMemsetAsync(e->status, 0, 16, stream));
   P.ll = e->ll;
   P.status = e->status;
   P.seq_base = e->seq;
@@ -581,13 +593,12 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
     const qmk_fused_tc::Build &tc = qmk_fused_tc::build_seqs(e->wfmt, P.nseq);
     Engine::Prepared *prep = nullptr;
     if (P.vocab % tc.rows_per_chunk == 0 && grid >= tc.min_ctas && grid <= tc.max_ctas) {
-      rc = ensure_prepared(e, P, e->wfmt, true, stream, &prep, true);
+      rc = ensure_prepared(e, P, e->wfmt, true, static_cast<int>(RED_ALLOC_WORDS), stream, &prep, true);
       if (rc != QMK_OK) return rc;
     }
     if (prep) {
       rc = encode_cache_maps(e, P);
       if (rc != QMK_OK) return rc;
-      QMK_CUDA(e, cudaMemsetAsync(e->red, 0, sizeof(unsigned long long) * RED_ALLOC_WORDS, stream));
       P.layers_t = prep->tbl;
       P.red = e->red;
       kernel = tc.kernel;
@@ -611,9 +622,8 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
     const qmk_fused_tc::Build &tc = qmk_fused_tc::build(e->wfmt);
     const bool on_tensor_cores = e->fused >= 2 && P.vocab % tc.rows_per_chunk == 0 && grid >= tc.min_ctas && grid <= tc.max_ctas;
     Engine::Prepared *prep = nullptr;
-    rc = ensure_prepared(e, P, e->wfmt, on_tensor_cores, stream, &prep);
+    rc = ensure_prepared(e, P, e->wfmt, on_tensor_cores, qmk::RED_WORDS, stream, &prep);
     if (rc != QMK_OK) return rc;
-    QMK_CUDA(e, cudaMemsetAsync(e->red, 0, sizeof(unsigned long long) * qmk::RED_WORDS, stream));
     P.layers_t = prep->tbl;
     P.red = e->red;
     P.red_copies = e->red_copies;
@@ -626,6 +636,7 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
       smem = tc.smem_bytes;
     }
   }
+  if (!P.layers_t) QMK_CUDA(e, cudaMemsetAsync(e->status, 0, 16, stream));   // (cleared with the sums otherwise, see ensure_prepared)
   const cudaError_t err = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, smem, stream);
   if (err == cudaErrorCooperativeLaunchTooLarge)
     return fail(e, QMK_ERR_NOT_RESIDENT, "persistent grid cannot be co-resident on this device");
