@@ -17,7 +17,10 @@
 // (.cta_group::2) - the empty and accumulator-full barriers in both (multicast commit).  No multicast loads.
 //
 // MODE 0: C fp32; 1: C fp16; 2: fp16 silu(gate) * up, where the pair's first CTA brings 128 gate rows and the second the 128 up
-// rows of the same columns.  RS: every B row has an fp32 scale (expanded packed matrices).
+// rows of the same columns.  3: fp32, added to C: a pair makes the two parts of K of a tile one after the other and adds each to
+// the matrix with bulk reductions, in order, the first under the main loop of the second. At 4096 rows a product of 1024 columns
+// takes 21 us (19 with two matrices of partial sums, whose row kernel then takes 12 instead of 5).
+// RS: every B row has an fp32 scale (expanded packed matrices).
 // Every wait is bounded (status 4).  After a time-out of whatever role the issuing thread gives up too, or is through: it then waits
 // for the MMAs issued and the copies of both CTAs in flight, which complete on its barriers (`drain`), or its readers wait for the
 // accumulator it has completed, before both CTAs meet at the cluster barrier, free TMEM and leave.  All of it in the roles' cold
@@ -107,13 +110,18 @@ __device__ __forceinline__ void stage_row(uint32_t block, int lane, const uint32
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(block + static_cast<uint32_t>(lane * 128 + ((i ^ (lane & 7)) << 4))),
                  "r"(v[4 * i]), "r"(v[4 * i + 1]), "r"(v[4 * i + 2]), "r"(v[4 * i + 3]) : "memory");
 }
-// The staged block to columns c0 .., rows c1 .. of the matrix (rows past its end are not written).
+// The staged block to (ADD: added to) columns c0 .., rows c1 .. of the matrix (rows past its end are not written).
+template <bool ADD = false>
 __device__ __forceinline__ void store_block(const CUtensorMap *map, uint32_t block, int c0, int c1) {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncwarp();
   if (qmk_gemm::elect_one()) {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
-                 ::"l"(map), "r"(c0), "r"(c1), "r"(block) : "memory");
+    if (ADD)
+      asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%1, %2}], [%3];"
+                   ::"l"(map), "r"(c0), "r"(c1), "r"(block) : "memory");
+    else
+      asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
+                   ::"l"(map), "r"(c0), "r"(c1), "r"(block) : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
   }
 }
@@ -151,6 +159,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int mn_tiles = args.m_tiles * args.n_tiles, tiles = mn_tiles * args.splits;
   const int kblocks = args.kblocks;
+  // the pair's n-th tile, of `count`
+  const int count = MODE == 3 ? (mn_tiles - pair + pairs - 1) / pairs * 2 : (tiles - pair + pairs - 1) / pairs;
+  auto tile_of = [&](int n) { return MODE == 3 ? (n & 1) * mn_tiles + pair + (n >> 1) * pairs : pair + n * pairs; };
 
   if (warp == 0 && elect_one()) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
@@ -190,9 +201,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       int s = 0;
       uint32_t parity = 1;                 // (the first pass over the ring finds it empty)
       bool ok = !(TEST == NO_LOADS || (TEST == SECOND_CTA_NO_LOADS && rank == 1)), waited = false;
-      for (int tile = pair; tile < tiles && ok; tile += pairs) {
+      for (int n = 0; n < count && ok; ++n) {
         int grp, mt, nt, z;
-        locate(tile, grp, mt, nt, z);
+        locate(tile_of(n), grp, mt, nt, z);
         const CUtensorMap *map_b = MODE == 2 ? (rank == 0 ? &map_b0 : &map_b1) : grp == 0 ? &map_b0 : grp == 1 ? &map_b1 : &map_b2;
         const int arow = mt * TM + static_cast<int>(rank) * 128;
         const int brow = MODE == 2 ? nt * 128 : nt * TN + static_cast<int>(rank) * 128;
@@ -226,8 +237,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       int s = 0, n = 0;
       uint32_t parity = 0;
       bool ok = true;
-      auto give_up = [&](int next) { drain(full(0), stopped, next, (tiles - pair + pairs - 1) / pairs * kblocks, budget_ns); };
-      for (int tile = pair; tile < tiles && ok; tile += pairs, ++n) {
+      auto give_up = [&](int next) { drain(full(0), stopped, next, count * kblocks, budget_ns); };
+      for (; n < count && ok; ++n) {
         const int buf = n & 1;
         ok = n < 2 || bar_wait(acc_empty(buf), ((n >> 1) - 1) & 1, abort_flag, status, budget_ns);
         if (TEST == ISSUER_STOPS && n == 1) ok = bar_wait(stopped, 0, abort_flag, status, budget_ns);   // (nothing arrives)
@@ -250,21 +261,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   } else {                                 // ---- epilogue
     const int quarter = warp & 3, half = (warp - 2) >> 2;
     const uint32_t block = base + RING_BYTES + static_cast<uint32_t>(warp - 2) * BLOCK_BYTES;
-    int n = 0;
-    for (int tile = pair; tile < tiles; tile += pairs, ++n) {
+    for (int n = 0; n < count; ++n) {
       const int buf = n & 1;
       int grp, mt, nt, z;
-      locate(tile, grp, mt, nt, z);
+      locate(tile_of(n), grp, mt, nt, z);
       const bool ok = __all_sync(0xffffffffu, bar_wait(acc_full(buf), (n >> 1) & 1, abort_flag, status, budget_ns));
       if (!ok) {
         bar_drain(acc_full(buf), (n >> 1) & 1, budget_ns);
-        if (tile + pairs < tiles) bar_drain(acc_full(buf ^ 1), ((n + 1) >> 1) & 1, budget_ns);
+        if (n + 1 < count) bar_drain(acc_full(buf ^ 1), ((n + 1) >> 1) & 1, budget_ns);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem_base + static_cast<uint32_t>(buf) * TN + (static_cast<uint32_t>(quarter * 32) << 16);
-      const int row = z * args.m_tiles * TM + mt * TM + static_cast<int>(rank) * 128 + quarter * 32;   // first of the warp's 32
-      const bool reused = tile + 2 * pairs < tiles;
+      const int row = (MODE == 3 ? 0 : z * args.m_tiles * TM) + mt * TM + static_cast<int>(rank) * 128 + quarter * 32;   // first of the warp's 32
+      const bool reused = n + 2 < count;
       auto release = [&]() {               // the buffer has been read
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
@@ -299,6 +309,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const int col = nt * TN + half * 128;
         const CUtensorMap *map_c = grp == 0 ? &map_c0 : grp == 1 ? &map_c1 : &map_c2;
         const float *scale = RS ? (grp == 0 ? args.row_scale[0] : grp == 1 ? args.row_scale[1] : args.row_scale[2]) + col : nullptr;
+        // (the part before has been added: this warp's, to the same elements)
+        if (MODE == 3 && z > 0 && elect_one()) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
         uint32_t out[32];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -327,7 +339,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           } else {                         // 32 floats
             block_free();
             stage_row(block, lane, r);
-            store_block(map_c, block, col + c * 32, row);
+            store_block<MODE == 3>(map_c, block, col + c * 32, row);
           }
         }
       }

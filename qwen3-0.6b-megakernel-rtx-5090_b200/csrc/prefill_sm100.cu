@@ -219,7 +219,8 @@ using PairKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensor
 static PairKernel pair_kernel(int mode, bool scaled) {
   if (mode == 0) return scaled ? qmk_pair::gemm_pair_kernel<0, true> : qmk_pair::gemm_pair_kernel<0, false>;
   if (mode == 1) return scaled ? qmk_pair::gemm_pair_kernel<1, true> : qmk_pair::gemm_pair_kernel<1, false>;
-  return scaled ? qmk_pair::gemm_pair_kernel<2, true> : qmk_pair::gemm_pair_kernel<2, false>;
+  if (mode == 2) return scaled ? qmk_pair::gemm_pair_kernel<2, true> : qmk_pair::gemm_pair_kernel<2, false>;
+  return scaled ? qmk_pair::gemm_pair_kernel<3, true> : qmk_pair::gemm_pair_kernel<3, false>;
 }
 
 // Opt-in shared-memory size of every tile variant, once per device (outside any stream capture).
@@ -242,7 +243,7 @@ int ensure_gemm_attrs(std::string *err) {
           if (gemm_kernel_64(bn, fuse != 0, wq))
             e = cudaFuncSetAttribute(reinterpret_cast<const void *>(gemm_kernel_64(bn, fuse != 0, wq)), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(qmk_gemm::smem_bytes_for(fuse ? 2 * bn : bn, wq, 1, 64)));
-    for (int mode = 0; mode < 3 && e == cudaSuccess; ++mode)
+    for (int mode = 0; mode < 4 && e == cudaSuccess; ++mode)
       for (int scaled = 0; scaled < 2 && e == cudaSuccess; ++scaled)
         e = cudaFuncSetAttribute(reinterpret_cast<const void *>(pair_kernel(mode, scaled != 0)), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(qmk_pair::SMEM_BYTES));
@@ -445,13 +446,14 @@ int launch_gemm_splitk(const CUtensorMap &map_a, const CUtensorMap &map_b, float
 }
 
 // The pair kernel: up to three matrices B_g (maps with 128 rows per box) against A, mode 0 fp32 (K split in `splits` parts, the
-// partial matrices M rounded up to 256 rows apart), 1 fp16, 2 SwiGLU of maps_b[0] (gate) and maps_b[1] (up) with N = Ns[0] outputs.
+// partial matrices M rounded up to 256 rows apart), 1 fp16, 2 SwiGLU of maps_b[0] (gate) and maps_b[1] (up) with N = Ns[0] outputs,
+// 3 fp32 added to C (K in two parts, added in order).
 // maps_c: make_map_c.  M a multiple of 128; the last tile may reach 128 rows past it, as far as the C maps go.
 int launch_gemm_pair(int mode, const CUtensorMap &map_a, int ngroups, const CUtensorMap *const *maps_b, const CUtensorMap *const *maps_c,
                      const int *Ns, int M, int K, int splits, unsigned int *status, int timeout_ms, cudaStream_t stream, std::string *err) {
   const int columns = mode == 2 ? qmk_pair::TN / 2 : qmk_pair::TN, matrices = mode == 2 ? 1 : ngroups;
-  bool bad = mode < 0 || mode > 2 || M <= 0 || M % 128 || K <= 0 || splits < 1 || K % (qmk_pair::BK * splits) || ngroups < 1 || ngroups > 3 ||
-             (mode == 2 && ngroups != 2) || (splits > 1 && (mode != 0 || ngroups != 1));
+  bool bad = mode < 0 || mode > 3 || M <= 0 || M % 128 || K <= 0 || splits < 1 || K % (qmk_pair::BK * splits) || ngroups < 1 || ngroups > 3 ||
+             (mode == 2 && ngroups != 2) || (splits > 1 && ((mode != 0 && mode != 3) || ngroups != 1)) || (mode == 3 && splits != 2);
   for (int g = 0; !bad && g < matrices; ++g) bad = Ns[g] <= 0 || Ns[g] % columns;
   for (int g = 0; !bad && g < ngroups; ++g) bad = (t_row_scale[g] == nullptr) != (t_row_scale[0] == nullptr);   // scales for all or for none
   if (bad) { *err = "gemm: bad shape for pairs of CTAs"; return QMK_ERR_BAD_ARGUMENT; }
@@ -467,7 +469,7 @@ int launch_gemm_pair(int mode, const CUtensorMap &map_a, int ngroups, const CUte
   a.m_tiles = (M + qmk_pair::TM - 1) / qmk_pair::TM;
   a.splits = splits;
   a.kblocks = K / qmk_pair::BK / splits;
-  const int tiles = a.m_tiles * a.n_tiles * splits, pairs = std::min(tiles, sm_count() / 2);
+  const int tiles = a.m_tiles * a.n_tiles * (mode == 3 ? 1 : splits), pairs = std::min(tiles, sm_count() / 2);
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
   const cudaError_t e = launch_kernel(pair_kernel(mode, a.row_scale[0] != nullptr), dim3(2 * pairs), dim3(qmk_pair::THREADS), qmk_pair::SMEM_BYTES, stream,
                                       map_a, *maps_b[0], *maps_b[ngroups > 1 ? 1 : 0], *maps_b[ngroups > 2 ? 2 : 0], *maps_c[0], *maps_c[matrices > 1 ? 1 : 0], *maps_c[matrices > 2 ? 2 : 0],
@@ -504,7 +506,7 @@ struct Workspace {                  // per device, allocated on first use, never
   __half *xn = nullptr, *attn = nullptr, *act = nullptr;
   unsigned int *status = nullptr;
   CUtensorMap map_xn, map_attn, map_act, map_qh;
-  CUtensorMap map_cq, map_ck, map_cv, map_cact, map_co, map_cdown;   // outputs of the pair GEMMs
+  CUtensorMap map_cq, map_ck, map_cv, map_cact, map_co, map_cdown, map_cx;   // outputs of the pair GEMMs
   CUtensorMap map_xn2, map_attn2, map_act2;   // split activations: rows of hi and lo halves
   // batched decode: per-sequence state and the logits of one step
   bool decode_ready = false;
@@ -610,6 +612,7 @@ int ensure_workspace(Workspace &w, int rows, bool *no_room = nullptr) {
   if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_cact, w.act, C, I, true, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_co, w.o, 2 * C, H, false, &err);
   if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_cdown, w.down, 2 * C, H, false, &err);
+  if (rc == QMK_OK) rc = qmk_tc::make_map_c(&w.map_cx, w.x, C, H, false, &err);
   if (rc != QMK_OK) {
     qmk_tc::drop_all(buffers, cudaFree);
     cudaGetLastError();
@@ -878,7 +881,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     // 17.6 ms; 500 tokens 1.56 -> 1.61, 250 tokens 1.21 -> 1.40 (a 256 x 256 tile for each pair leaves most pairs idle).
     by_pairs = wq == 0 && !split && M > PAIR_MIN_ROWS;
     // The O and down projections have only 1024 output columns.  K is split so that their tiles fill the SMs; the partial
-    // matrices are added by the residual + RMSNorm kernel that follows anyway.  Four parts below 1024 rows (M = 512: 32 tiles x
+    // matrices are added by the residual + RMSNorm kernel that follows anyway (or by the pairs, below).  Four parts below 1024 rows (M = 512: 32 tiles x
     // 4 = 128 CTAs with K loops of 8 / 12 blocks; unsplit, the narrowest tiles gave 128 CTAs with loops of 32 / 48 blocks of N =
     // 32 MMAs and these two products were 41 % of the pass), two above: the sums, and with them the last bits of every row behind,
     // do not depend on which kernel made them.  (One part where the pairs would fill the SMs without
@@ -889,14 +892,21 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     // Two parts whose 128-wide tiles all find an SM of their own (1024 and 1152 rows) stay with single CTAs: 32 or 40 tiles of
     // 256 x 256 leave half of the pairs idle (1000 tokens, with four parts to fill them, 2.03 ms; here 2.02).
     const bool od_pairs = by_pairs && (M < 1024 || static_cast<long>(M / qmk_gemm::BM) * (H / 128) * od_splits > qmk_tc::gemm_sm_count());
+    // Where the two parts of all tiles are more than one round of the pairs anyway (ten row tiles, 2305 tokens, on 148 SMs), a pair makes
+    // both parts of a tile and adds them to the residual rows itself, in the order in which the RMSNorm kernel added them: the same
+    // bits without writing and reading two matrices of partial sums (32 MB each way at 4096 rows; a row kernel 12 -> 5 us, a product
+    // 19 -> 21).  2400 / 3000 / 3500 / 4096 / 8191 tokens 4.23 / 5.02 / 5.93 / 6.83 / 17.67 -> 4.00 / 4.74 / 5.55 / 6.53 / 17.05 ms, NVFP4
+    // 4096 6.69 -> 6.28.  Below the line half as many pairs work twice as long: 1300 / 1700 / 2048 / 2300 tokens 2.43 / 2.81 / 3.03 /
+    // 3.43 ms with partial sums, 2.73 / 3.10 / 3.27 / 3.54 without.
+    const bool od_adds = od_pairs && od_splits == 2 && static_cast<long>((M + qmk_pair::TM - 1) / qmk_pair::TM) * (H / qmk_pair::TN) * 2 > qmk_tc::gemm_sm_count() / 2;
     const size_t od_stride = static_cast<size_t>(od_pairs ? (M + qmk_pair::TM - 1) / qmk_pair::TM * qmk_pair::TM : M) * H;
     auto gemm_od = [&](const CUtensorMap &a, int l, int j, float *c, int Mrows, int K, int live) {
       row_scales(&j, 1);
       if (od_pairs) {
         const CUtensorMap *const map = &wmap_for(l, j, 128);
-        const CUtensorMap *const out = c == w.o ? &w.map_co : &w.map_cdown;
+        const CUtensorMap *const out = od_adds ? &w.map_cx : c == w.o ? &w.map_co : &w.map_cdown;
         const int n = H;
-        return qmk_tc::launch_gemm_pair(0, a, 1, &map, &out, &n, Mrows, K, od_splits, w.status, env.timeout_ms, stream, &err);
+        return qmk_tc::launch_gemm_pair(od_adds ? 3 : 0, a, 1, &map, &out, &n, Mrows, K, od_splits, w.status, env.timeout_ms, stream, &err);
       }
       if (od_splits == 1) {
         const int box_n = split_box(qmk_tc::gemm_box_n(Mrows, H), 64);
@@ -952,6 +962,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     }
     // residual add (+ split-K partials) and RMSNorm: a warp per row for long chunks, a block per row for short ones
     auto norm_rows = [&](const float *add, const __half *g) {
+      if (od_adds) add = nullptr;
       if (T >= 256 && od_splits <= 2)
         return qmk_tc::launch_kernel(split ? add_rmsnorm_rows_wide<true> : add_rmsnorm_rows_wide<false>, dim3((T + 7) / 8), dim3(256), 0,
                                      stream, w.x, add, od_splits, od_stride, g, w.xn, T, w.status + qmk_gemm::STATUS_BEYOND);

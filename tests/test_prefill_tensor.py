@@ -307,6 +307,15 @@ def test_rows_do_not_depend_on_how_a_prompt_is_cut(C, fmt, cuts):
         assert torch.equal(x[:, :, :cuts[-1]], y[:, :, :cuts[-1]])
 
 
+@pytest.mark.parametrize("fmt,cuts", [("fp16", (1200, 2304)), ("fp16", (1200, 2305)), ("fp16", (1153, 2560)), ("nvfp4", (1300, 3585)),
+                                      ("fp8", (2200, 4095))])
+def test_residual_adds_in_the_epilogue_keep_the_bits(C, fmt, cuts):
+    """From 2305 tokens on (ten row tiles) the O and down products add both parts to the residual rows themselves; the pieces of
+    the prompt stay below and leave the partial matrices to the RMSNorm kernel.  Either side of the line, rows that end with a
+    tile and one behind it, row scales."""
+    test_rows_do_not_depend_on_how_a_prompt_is_cut(C, fmt, cuts)
+
+
 def test_attention_waits_run_out_and_leave_the_device_usable(C):
     """Score products that stop behind the first, with keys and values in flight: status 4 after the budget, copies landed and TMEM
     freed (the prefill behind it allocates all of it on every SM), rows as before."""
