@@ -20,6 +20,7 @@
 // rows of the same columns.  3: fp32, added to C: a pair makes the two parts of K of a tile one after the other and adds each to
 // the matrix with bulk reductions, in order, the first under the main loop of the second. At 4096 rows a product of 1024 columns
 // takes 21 us (19 with two matrices of partial sums, whose row kernel then takes 12 instead of 5).
+// 4: q, k and v with QK norm, rotation and cache write in the epilogue (store_heads): 43 -> 34 us a layer at 4096 rows.
 // RS: every B row has an fp32 scale (expanded packed matrices).
 // Every wait is bounded (status 4).  After a time-out of whatever role the issuing thread gives up too, or is through: it then waits
 // for the MMAs issued and the copies of both CTAs in flight, which complete on its barriers (`drain`), or its readers wait for the
@@ -29,6 +30,7 @@
 #define QMK_GEMM_PAIR_TCGEN05_CUH_
 
 #include "gemm_tcgen05.cuh"
+#include "prefill_kernels.cuh"
 
 namespace qmk_pair {
 
@@ -45,7 +47,21 @@ constexpr size_t SMEM_BYTES = 1024 + OFF_BARS + 256;
 static_assert(SMEM_BYTES <= 232448, "over the 227 KB shared-memory limit of one CTA");
 constexpr uint32_t IDESC = (1u << 4) | (static_cast<uint32_t>(TN >> 3) << 17) | (static_cast<uint32_t>(TM >> 4) << 24);
 
+// MODE 4: where the rows of q, k and v go.
+struct Heads {
+  const __half *q_norm, *k_norm;
+  const float *rope;                          // fp32 rows, or null: the fp16 tables
+  const __half *cos_table, *sin_table;
+  __half *queries;                            // [row][16][128], times q_scale
+  __half *k_cache, *v_cache;                  // one layer's rows [head][max_seq_len][128] (packed prompts: kv_ptrs + layer_off)
+  const int2 *row_info;                       // packed prompts: (sequence, position or < 0) of each row; a prompt begins with a row tile of 128
+  const unsigned long long *kv_ptrs;
+  size_t layer_off;
+  int rows, pos0, max_seq_len;
+  float q_scale;
+};
 struct Args {
+  Heads heads;
   int N[3];                      // columns of the groups' matrices (multiples of 256; MODE 2: of 128, group 0 only)
   const float *row_scale[3];     // RS: scales of the groups' B rows (MODE 2: [0] gate, [1] up)
   int m_tiles, n_tiles, splits;  // tiles of 256 rows / 256 columns (MODE 2: 128 outputs) over all groups, parts of K
@@ -128,6 +144,119 @@ __device__ __forceinline__ void store_block(const CUtensorMap *map, uint32_t blo
 // The block may be written again.
 __device__ __forceinline__ void block_free() {
   if (qmk_gemm::elect_one()) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+  __syncwarp();
+}
+__device__ __forceinline__ float2 as_floats(uint32_t bits) { return __half22float2(*reinterpret_cast<const __half2 *>(&bits)); }
+// MODE 4, a warp's 32 rows of one head (group 0 q, 1 k, 2 v) from row t0, packed halves of row `lane` in `row`: QK norm and rotation with
+// the operations of qk_norm_rope_cache, bit for bit.  The squares are added by the thread that holds the row, in the order of that
+// kernel's shuffles; the rest goes row by row through the warp's 4 KB, 16 rows at a time, so that tables, cache and queries are read
+// and written in whole lines: lane l has dims 2 l, 2 l + 1 and their partners 64 behind, no value crosses lanes.  The tables'
+// rows of the next step are asked for ahead (1500 / 2200 / 4096 tokens 2.456 / 3.14 / 6.28 -> 2.40 / 3.08 / 6.22 ms).  A first form, that
+// kernel's lanes and shuffles as they are, took 51 us a product at 4096 rows; this one 34, the product and the kernel in turn 43.
+// What bounds it there is traffic with L2: without the tables' reads 4096 tokens take 5.87 ms, without the stores 5.55.
+__device__ __forceinline__ void store_heads(const Heads &a, uint32_t block, int lane, const uint32_t (&row)[64], int grp, int head, int t0) {
+  using qmk_pf::D;
+  int live = min(max(a.rows - t0, 0), 32), pos = a.pos0 + t0;
+  __half *kc = a.k_cache, *vc = a.v_cache;
+  if (a.row_info) {
+    const int2 info = lane < live ? a.row_info[t0 + lane] : make_int2(0, -1);
+    live = __popc(__ballot_sync(0xffffffffu, info.y >= 0));      // (rows of one prompt, then padding)
+    const int seq = __shfl_sync(0xffffffffu, info.x, 0);
+    pos = __shfl_sync(0xffffffffu, info.y, 0);
+    kc = reinterpret_cast<__half *>(a.kv_ptrs[2 * seq]) + a.layer_off;
+    vc = reinterpret_cast<__half *>(a.kv_ptrs[2 * seq + 1]) + a.layer_off;
+  }
+  if (live == 0) return;
+  __half *const out = (grp == 0 ? a.queries + (static_cast<size_t>(t0) * qmk_pf::NQ + head) * D
+                                : (grp == 1 ? kc : vc) + (static_cast<size_t>(head) * a.max_seq_len + pos) * D) + 2 * lane;
+  const size_t pitch = grp == 0 ? qmk_pf::QS : D;
+  const bool first = (lane & 1) == 0;      // this lane's first dim is that of a four (see qk_norm_rope_cache)
+  float2 w0 = make_float2(0.f, 0.f), w1 = w0;
+  float rstd = 0.f;
+  if (grp < 2) {
+    const __half *const norm = (grp == 0 ? a.q_norm : a.k_norm) + 2 * lane;
+    w0 = __half22float2(*reinterpret_cast<const __half2 *>(norm));
+    w1 = __half22float2(*reinterpret_cast<const __half2 *>(norm + 64));
+    auto squares4 = [&](int i) {           // dims 4 i .. 4 i + 3
+      const float2 x = as_floats(row[2 * i]), y = as_floats(row[2 * i + 1]);
+      return fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(y.x, y.x, y.y * y.y)));
+    };
+    float t[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) t[i] = squares4(i) + squares4(i + 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < o; ++i) t[i] += t[i + o];
+    rstd = 1.0f / sqrtf(t[0] * (1.0f / D) + qmk_pf::RMS_EPS);
+  }
+  constexpr int ROWS = 4;                  // in flight together
+  float2 cs_next[ROWS], sn_next[ROWS];
+  auto ask = [&](int first) {
+    if (grp == 2) return;
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) {
+      const size_t at = static_cast<size_t>(pos + min(first + j, live - 1)) * D + 2 * lane;
+      if (a.rope) {
+        cs_next[j] = *reinterpret_cast<const float2 *>(a.rope + at);
+        sn_next[j] = *reinterpret_cast<const float2 *>(a.rope + at + 64);
+      } else {
+        cs_next[j] = __half22float2(*reinterpret_cast<const __half2 *>(a.cos_table + at));
+        sn_next[j] = __half22float2(*reinterpret_cast<const __half2 *>(a.sin_table + at));
+      }
+    }
+  };
+  ask(0);
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh) {
+    if (hh * 16 >= live) break;
+    __syncwarp();
+    if ((lane >> 4) == hh) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(block + static_cast<uint32_t>((lane & 15) * 256 + ((i ^ (lane & 7)) << 4))),
+                     "r"(row[4 * i]), "r"(row[4 * i + 1]), "r"(row[4 * i + 2]), "r"(row[4 * i + 3]) : "memory");
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int i0 = 0; i0 < 16 && hh * 16 + i0 < live; i0 += ROWS) {
+      float2 cs[ROWS], sn[ROWS];
+      uint32_t lo[ROWS], hi[ROWS];
+#pragma unroll
+      for (int j = 0; j < ROWS; ++j) { cs[j] = cs_next[j]; sn[j] = sn_next[j]; }
+      ask(hh * 16 + i0 + ROWS);
+#pragma unroll
+      for (int j = 0; j < ROWS; ++j) {
+        const int i = i0 + j;
+        const uint32_t at = block + static_cast<uint32_t>(i * 256 + (((lane >> 2) ^ (i & 7)) << 4) + (lane & 3) * 4);
+        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(lo[j]) : "r"(at));
+        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(hi[j]) : "r"(at + 128));
+      }
+      if (grp < 2) {
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+          const float rs = __shfl_sync(0xffffffffu, rstd, hh * 16 + i0 + j);
+          float2 l = as_floats(lo[j]), h = as_floats(hi[j]);
+          l.x = l.x * rs * w0.x; l.y = l.y * rs * w0.y;
+          h.x = h.x * rs * w1.x; h.y = h.y * rs * w1.y;
+          float2 rl = make_float2(fmaf(l.x, cs[j].x, -__fmul_rn(h.x, sn[j].x)), fmaf(l.y, cs[j].y, -__fmul_rn(h.y, sn[j].y)));
+          float2 rh = make_float2(first ? fmaf(l.x, sn[j].x, __fmul_rn(h.x, cs[j].x)) : fmaf(h.x, cs[j].x, __fmul_rn(l.x, sn[j].x)),
+                                  fmaf(h.y, cs[j].y, __fmul_rn(l.y, sn[j].y)));
+          if (grp == 0) { rl.x *= a.q_scale; rl.y *= a.q_scale; rh.x *= a.q_scale; rh.y *= a.q_scale; }
+          const __half2 pl = __floats2half2_rn(rl.x, rl.y), ph = __floats2half2_rn(rh.x, rh.y);
+          lo[j] = *reinterpret_cast<const uint32_t *>(&pl);
+          hi[j] = *reinterpret_cast<const uint32_t *>(&ph);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < ROWS; ++j)
+        if (hh * 16 + i0 + j < live) {
+          uint32_t *const at = reinterpret_cast<uint32_t *>(out + (hh * 16 + i0 + j) * pitch);
+          at[0] = lo[j];
+          at[32] = hi[j];
+        }
+    }
+  }
   __syncwarp();
 }
 __device__ __forceinline__ uint32_t half2_bits(float a, float b) {
@@ -305,6 +434,26 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         block_free();
         stage_row(block, lane, out);
         store_block(&map_c0, block, col, row);
+      } else if (MODE == 4) {               // a warp's 128 columns are a head
+        const float *scale = RS ? (grp == 0 ? args.row_scale[0] : grp == 1 ? args.row_scale[1] : args.row_scale[2]) + nt * TN + half * 128 : nullptr;
+        uint32_t head[64];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t r[32];
+          tmem_ld32(acc + half * 128 + c * 32, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            float lo = __uint_as_float(r[2 * i]), hi = __uint_as_float(r[2 * i + 1]);
+            if (RS) {
+              const float2 sc = __ldg(reinterpret_cast<const float2 *>(scale + c * 32) + i);
+              lo *= sc.x; hi *= sc.y;
+            }
+            head[c * 16 + i] = half2_bits(lo, hi);
+          }
+        }
+        release();
+        store_heads(args.heads, block, lane, head, grp, nt * 2 + half, row);
       } else {
         const int col = nt * TN + half * 128;
         const CUtensorMap *map_c = grp == 0 ? &map_c0 : grp == 1 ? &map_c1 : &map_c2;

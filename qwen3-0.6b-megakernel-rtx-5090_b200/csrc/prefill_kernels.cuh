@@ -261,11 +261,15 @@ qk_norm_rope_cache(const float *q, const float *k, const float *v, int in_f16, c
     float4 o;   // the partner's normalised values
     o.x = __shfl_xor_sync(0xffffffffu, a.x, 16); o.y = __shfl_xor_sync(0xffffffffu, a.y, 16);
     o.z = __shfl_xor_sync(0xffffffffu, a.z, 16); o.w = __shfl_xor_sync(0xffffffffu, a.w, 16);
+    // (which product is rounded on its own is spelled out: store_heads of gemm_pair_tcgen05.cuh has to do the same; the first of
+    // four high dims is the other way round for no better reason than that the rows have always been so)
     float4 r;
     if (lane < 16) {    // low half: lo * cos - hi * sin
-      r = make_float4(a.x * cs.x - o.x * sn.x, a.y * cs.y - o.y * sn.y, a.z * cs.z - o.z * sn.z, a.w * cs.w - o.w * sn.w);
+      r = make_float4(fmaf(a.x, cs.x, -__fmul_rn(o.x, sn.x)), fmaf(a.y, cs.y, -__fmul_rn(o.y, sn.y)), fmaf(a.z, cs.z, -__fmul_rn(o.z, sn.z)),
+                      fmaf(a.w, cs.w, -__fmul_rn(o.w, sn.w)));
     } else {            // high half: lo * sin + hi * cos
-      r = make_float4(o.x * sn.x + a.x * cs.x, o.y * sn.y + a.y * cs.y, o.z * sn.z + a.z * cs.z, o.w * sn.w + a.w * cs.w);
+      r = make_float4(fmaf(o.x, sn.x, __fmul_rn(a.x, cs.x)), fmaf(a.y, cs.y, __fmul_rn(o.y, sn.y)), fmaf(a.z, cs.z, __fmul_rn(o.z, sn.z)),
+                      fmaf(a.w, cs.w, __fmul_rn(o.w, sn.w)));
     }
     if (h < 2 && q_f16_scale != 0.f)   // fp16 queries, pre-scaled: the tcgen05 attention kernel takes them by TMA as they are
       *reinterpret_cast<uint2 *>(reinterpret_cast<__half *>(qr) + (static_cast<size_t>(t) * NQ + w + 8 * h) * D + d0) =

@@ -220,7 +220,8 @@ static PairKernel pair_kernel(int mode, bool scaled) {
   if (mode == 0) return scaled ? qmk_pair::gemm_pair_kernel<0, true> : qmk_pair::gemm_pair_kernel<0, false>;
   if (mode == 1) return scaled ? qmk_pair::gemm_pair_kernel<1, true> : qmk_pair::gemm_pair_kernel<1, false>;
   if (mode == 2) return scaled ? qmk_pair::gemm_pair_kernel<2, true> : qmk_pair::gemm_pair_kernel<2, false>;
-  return scaled ? qmk_pair::gemm_pair_kernel<3, true> : qmk_pair::gemm_pair_kernel<3, false>;
+  if (mode == 3) return scaled ? qmk_pair::gemm_pair_kernel<3, true> : qmk_pair::gemm_pair_kernel<3, false>;
+  return scaled ? qmk_pair::gemm_pair_kernel<4, true> : qmk_pair::gemm_pair_kernel<4, false>;
 }
 
 // Opt-in shared-memory size of every tile variant, once per device (outside any stream capture).
@@ -243,7 +244,7 @@ int ensure_gemm_attrs(std::string *err) {
           if (gemm_kernel_64(bn, fuse != 0, wq))
             e = cudaFuncSetAttribute(reinterpret_cast<const void *>(gemm_kernel_64(bn, fuse != 0, wq)), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(qmk_gemm::smem_bytes_for(fuse ? 2 * bn : bn, wq, 1, 64)));
-    for (int mode = 0; mode < 4 && e == cudaSuccess; ++mode)
+    for (int mode = 0; mode < 5 && e == cudaSuccess; ++mode)
       for (int scaled = 0; scaled < 2 && e == cudaSuccess; ++scaled)
         e = cudaFuncSetAttribute(reinterpret_cast<const void *>(pair_kernel(mode, scaled != 0)), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(qmk_pair::SMEM_BYTES));
@@ -447,12 +448,13 @@ int launch_gemm_splitk(const CUtensorMap &map_a, const CUtensorMap &map_b, float
 
 // The pair kernel: up to three matrices B_g (maps with 128 rows per box) against A, mode 0 fp32 (K split in `splits` parts, the
 // partial matrices M rounded up to 256 rows apart), 1 fp16, 2 SwiGLU of maps_b[0] (gate) and maps_b[1] (up) with N = Ns[0] outputs,
-// 3 fp32 added to C (K in two parts, added in order).
+// 3 fp32 added to C (K in two parts, added in order), 4 q / k / v heads to where `heads` says (no C maps are read).
 // maps_c: make_map_c.  M a multiple of 128; the last tile may reach 128 rows past it, as far as the C maps go.
 int launch_gemm_pair(int mode, const CUtensorMap &map_a, int ngroups, const CUtensorMap *const *maps_b, const CUtensorMap *const *maps_c,
-                     const int *Ns, int M, int K, int splits, unsigned int *status, int timeout_ms, cudaStream_t stream, std::string *err) {
+                     const int *Ns, int M, int K, int splits, unsigned int *status, int timeout_ms, cudaStream_t stream, std::string *err,
+                     const qmk_pair::Heads *heads = nullptr) {
   const int columns = mode == 2 ? qmk_pair::TN / 2 : qmk_pair::TN, matrices = mode == 2 ? 1 : ngroups;
-  bool bad = mode < 0 || mode > 3 || M <= 0 || M % 128 || K <= 0 || splits < 1 || K % (qmk_pair::BK * splits) || ngroups < 1 || ngroups > 3 ||
+  bool bad = mode < 0 || mode > 4 || (mode == 4) != (heads != nullptr) || M <= 0 || M % 128 || K <= 0 || splits < 1 || K % (qmk_pair::BK * splits) || ngroups < 1 || ngroups > 3 ||
              (mode == 2 && ngroups != 2) || (splits > 1 && ((mode != 0 && mode != 3) || ngroups != 1)) || (mode == 3 && splits != 2);
   for (int g = 0; !bad && g < matrices; ++g) bad = Ns[g] <= 0 || Ns[g] % columns;
   for (int g = 0; !bad && g < ngroups; ++g) bad = (t_row_scale[g] == nullptr) != (t_row_scale[0] == nullptr);   // scales for all or for none
@@ -460,6 +462,7 @@ int launch_gemm_pair(int mode, const CUtensorMap &map_a, int ngroups, const CUte
   const int arc = ensure_gemm_attrs(err);
   if (arc != QMK_OK) return arc;
   qmk_pair::Args a;
+  a.heads = heads ? *heads : qmk_pair::Heads{};
   a.n_tiles = 0;
   for (int g = 0; g < 3; ++g) {
     a.N[g] = g < matrices ? Ns[g] : 0;
@@ -843,7 +846,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
   bool by_pairs = false;   // this chunk's GEMMs run on pairs of CTAs
   // several matrices against the same activations in one launch (q/k/v)
   auto gemm_group = [&](const CUtensorMap &a, int l, int n, const int *js, float *const *cs, const int *ns, int M, int K,
-                        int live) {
+                        int live, const qmk_pair::Heads *heads) {
     int total = 0;
     for (int i = 0; i < n; ++i) total += ns[i];
     if (by_pairs) {
@@ -851,7 +854,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
       for (int i = 0; i < n; ++i) maps[i] = &wmap_for(l, js[i], 128);
       const CUtensorMap *const out[3] = {&w.map_cq, &w.map_ck, &w.map_cv};
       row_scales(js, n);
-      return qmk_tc::launch_gemm_pair(1, a, n, maps, out, ns, M, K, 1, w.status, env.timeout_ms, stream, &err);
+      return qmk_tc::launch_gemm_pair(heads ? 4 : 1, a, n, maps, out, ns, M, K, 1, w.status, env.timeout_ms, stream, &err, heads);
     }
     const int box_n = split_box(qmk_tc::gemm_box_n(M, total), 64);
     const CUtensorMap *maps[3];
@@ -994,7 +997,23 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
                                       dim3(qmk_gemm::EXPAND_THREADS), 0, stream, a));
       }
       PF_CUDA(norm_rows(l > 0 ? w.down : nullptr, reinterpret_cast<const __half *>(r[0])));
+      // On pairs of CTAs the product's epilogue normalises, rotates and stores the heads (fp16 queries, as the tcgen05 attention
+      // kernel reads them).  520 / 777 / 1024 / 1300 / 2200 / 3500 / 6000 / 8191 tokens, with a kernel of its own -> in the epilogue:
+      // 1.697 / 1.922 / 2.046 / 2.43 / 3.21 / 5.55 / 11.4 / 16.95 -> 1.70 / 1.91 / 2.02 / 2.35 / 3.08 / 5.35 / 10.9 / 16.4 ms.  (On single CTAs,
+      // 128 threads walking TMEM eight columns at a time, slower than 2300 x 4 parallel blocks.)
+      const bool heads_in_gemm = by_pairs && env.attn_tc;
       {
+        qmk_pair::Heads heads;
+        heads.q_norm = reinterpret_cast<const __half *>(r[4]);
+        heads.k_norm = reinterpret_cast<const __half *>(r[5]);
+        heads.rope = rope; heads.cos_table = cosv; heads.sin_table = sinv;
+        heads.queries = reinterpret_cast<__half *>(w.qr);
+        heads.k_cache = kc; heads.v_cache = vc;
+        heads.row_info = pk ? reinterpret_cast<const int2 *>(w.packed + PK_ROWS_OFF) : nullptr;
+        heads.kv_ptrs = pk ? reinterpret_cast<const unsigned long long *>(w.packed + PK_PTRS_OFF) : nullptr;
+        heads.layer_off = static_cast<size_t>(l) * layer_stride;
+        heads.rows = T; heads.pos0 = pos0; heads.max_seq_len = max_seq_len;
+        heads.q_scale = attn_scale * 1.4426950408889634f;
         const int js[3] = {0, 1, 2};
         float *const cs[3] = {w.q, w.k, w.v};
         const int ns[3] = {QS, KVS, KVS};
@@ -1003,13 +1022,12 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
         // (split activations: fp32, the operands downstream are not rounded to fp16)
         qmk_tc::set_out_f16(!split);
         const qmk_tc::PrefetchScope ahead(l + 1 < num_layers ? ahead_of(l, {3}) : qmk_tc::PrefetchList());   // (the last layer ends here)
-        rc = gemm_group(map_xn, l, 3, js, cs, ns, M, H, T);
+        rc = gemm_group(map_xn, l, 3, js, cs, ns, M, H, T, heads_in_gemm ? &heads : nullptr);
         qmk_tc::set_out_f16(false);
         if (rc != QMK_OK) break;
       }
-      // (Folding this kernel into the q/k/v GEMM's epilogue - one 128-wide N tile is one head - was built and measured
-      // slower: 128 threads per CTA walking TMEM eight columns at a time lose to 2300 x 4 fully parallel CTAs.)
-      PF_CUDA(qmk_tc::launch_kernel(qk_norm_rope_cache, dim3(T), dim3(256), 0, stream, w.q, w.k, w.v, split ? 0 : 1,
+      if (!heads_in_gemm)
+        PF_CUDA(qmk_tc::launch_kernel(qk_norm_rope_cache, dim3(T), dim3(256), 0, stream, w.q, w.k, w.v, split ? 0 : 1,
                                     reinterpret_cast<const __half *>(r[4]), reinterpret_cast<const __half *>(r[5]), rope, cosv, sinv,
                                     w.qr, kc, vc, pos0, max_seq_len,
                                     pk ? reinterpret_cast<const int2 *>(w.packed + PK_ROWS_OFF) : nullptr,
@@ -1612,6 +1630,7 @@ extern "C" int qmk_selftest_gemm_pair_wait_timeout(int budget_us, int what) {
   if (rc == QMK_OK) rc = qmk_tc::make_map_c(&mc, buf + at_c, M, N, false, &err);
   if (rc == QMK_OK && e == cudaSuccess) {
     qmk_pair::Args a;
+    a.heads = qmk_pair::Heads{};
     for (int g = 0; g < 3; ++g) { a.N[g] = g == 0 ? N : 0; a.row_scale[g] = nullptr; }
     a.m_tiles = 2; a.n_tiles = 1; a.splits = 1;
     a.kblocks = K / qmk_pair::BK;

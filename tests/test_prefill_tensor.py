@@ -316,6 +316,56 @@ def test_residual_adds_in_the_epilogue_keep_the_bits(C, fmt, cuts):
     test_rows_do_not_depend_on_how_a_prompt_is_cut(C, fmt, cuts)
 
 
+@pytest.mark.parametrize("fmt,table_rope,lens", [("fp16", False, (513,)), ("fp16", True, (777,)), ("nvfp4", False, (1025,)), ("fp8", False, (640, 2400)),
+                                                 ("fp16", False, (544, 4095, 1000))])
+def test_heads_stored_by_the_product_keep_the_bits(C, fmt, table_rope, lens):
+    """Chunks on pairs of CTAs normalise, rotate and store q, k and v in the product's epilogue; with the other attention kernel
+    selected a kernel of its own does it.  The first layer's rows do not depend on the attention: equal bit for bit, for rows
+    that end inside a warp's 32, behind a start position, with row scales, and nothing is written behind them."""
+    import quantize as Q
+    vocab, n = 2048, sum(lens)
+    w = S.make_weights(seed=71, num_layers=1, vocab_size=vocab, norm_std=0.1, max_seq_len=n + 40 if table_rope else 16)
+    if fmt != "fp16":
+        w, _ = (Q.quantize_weights_fp8 if fmt == "fp8" else Q.quantize_weights_nvfp4)(w)
+    ids = S.make_prompt(n, seed=8, vocab_size=vocab)
+    rows = []
+    try:
+        eng = _engine(w, n + 40, "tensor", weight_format=fmt, rope_from_table=table_rope)
+        for impl in (1, 0):
+            C.set_prefill_attention(impl)
+            eng.reset()
+            eng._k_cache.zero_(), eng._v_cache.zero_()
+            at = 0
+            for length in lens:
+                eng.prefill_ids(ids[at:at + length])
+                at += length
+            rows.append((eng._k_cache.clone(), eng._v_cache.clone()))
+    finally:
+        C.set_prefill_attention(1)
+        C.configure(rope_from_table=0)
+        C.set_weight_format("fp16")
+    for x, y in zip(*rows):
+        assert float(x[:, :, :n].float().abs().max()) > 0.1 and float(x[:, :, n:].float().abs().max()) == 0
+        assert torch.equal(x, y)
+
+
+def test_heads_of_packed_prompts_keep_the_bits(C):
+    """Packed prompts of 896 rows (the pairs' product stores the heads) and the same prompts on their own (a kernel does)."""
+    from Model.Qwen06B_architecture import BatchDecoder
+    vocab, lens = 2048, [1, 37, 300, 129]
+    w = S.weights_to(S.make_weights(seed=72, num_layers=3, vocab_size=vocab, norm_std=0.1, max_seq_len=16), "cuda")
+    eng = BatchDecoder(weights=w, tokenizer=S.StubTokenizer(-1, vocab), num_sequences=4, max_seq_len=400, engine="gemm", prefill_mode="tensor")
+    prompts = [S.make_prompt(n, seed=80 + n, vocab_size=vocab) for n in lens]
+    for b, ids in enumerate(prompts):
+        eng.prefill_slot(b, ids)
+    want = [(k.clone(), v.clone()) for k, v in zip(eng._k_caches, eng._v_caches)]
+    for k, v in zip(eng._k_caches, eng._v_caches):
+        k.zero_(), v.zero_()
+    eng.prefill_slots(list(range(4)), prompts)
+    for b, (k, v) in enumerate(want):
+        assert torch.equal(eng._k_caches[b], k) and torch.equal(eng._v_caches[b], v), b
+
+
 def test_attention_waits_run_out_and_leave_the_device_usable(C):
     """Score products that stop behind the first, with keys and values in flight: status 4 after the budget, copies landed and TMEM
     freed (the prefill behind it allocates all of it on every SM), rows as before."""
