@@ -617,7 +617,7 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
       kernel == reinterpret_cast<const void *>(qmk::qwen3_decode_megakernel)) {
     // fused kernel: O and down projections as split-K slices of K-major copies, two all-reduced residual sums
     // Row products on the tensor cores: rows owned in units of one ring chunk (four fp16 rows, eight fp8 rows).  fp8:
-    // 724 -> 493 us per token at 1024-token contexts against the CUDA-core kernel, which stays for the grids and
+    // 724 -> 412 us per token at 1024-token contexts against the CUDA-core kernel, which stays for the grids and
     // vocabularies outside these limits.
     const qmk_fused_tc::Build &tc = qmk_fused_tc::build(e->wfmt);
     const bool on_tensor_cores = e->fused >= 2 && P.vocab % tc.rows_per_chunk == 0 && grid >= tc.min_ctas && grid <= tc.max_ctas;

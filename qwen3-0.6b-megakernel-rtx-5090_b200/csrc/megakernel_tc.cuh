@@ -31,7 +31,7 @@
 // (xf_offset).  A packed row is 1040 bytes in memory, which is a conflict-free pitch in shared memory too: a chunk
 // is eight rows and ONE bulk copy (four 2 KB rows: four copies).  Row scales multiply the finished sums (they sit in
 // the rows' trailers); the per-output scales of the K-major O / down copies travel as one more chunk of those phases.
-// Measured after: 493 us per token (128 tokens from a 1024-token context).  Against float64 the cache rows are nearer than the
+// Measured after: 493 us per token (128 tokens from a 1024-token context; 412 with what is described below).  Against float64 the cache rows are nearer than the
 // CUDA-core kernel's (later layers' values that round differently: 0.154 % and 0.167 %).
 
 namespace QMK_NS {

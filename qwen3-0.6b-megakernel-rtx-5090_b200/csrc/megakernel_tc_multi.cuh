@@ -299,7 +299,8 @@ __device__ __forceinline__ void normalise_seqs(const Ctx &c, const float (&v)[TC
 // Contributions that may still be missing from the watched word when a warp goes on to fetch all its words: with several
 // sequences the adds drain for longer, and the fetch's round trip fits into the rest of it (four sequences, us per step at
 // 64 / 1024 / 2048 tokens: 0: 812 / 932 / 1034, 16: 771 / 896 / 981, 48: 725 / 844 / 953, with the watch in front of the merge 712 / 812 / 928; 147: no better; all with full lines of sums, see RED_GROUP).
-// One sequence gains nothing.
+// One sequence gains nothing.  (Those figures are from sums of one contribution per CTA; a word of x1 has a quarter of that now, so that
+// only x2 is watched.)
 constexpr unsigned long long SUM_SLACK = 48;
 // red_wait_norm for all sequences: which = 0: x1, 1: x2 (kept as the residual of the next layer's O slice, x).
 __device__ __forceinline__ void red_wait_norm_seqs(const Params &P, const Ctx c, int which, uint32_t use, const __half *norm_w) {
