@@ -396,12 +396,10 @@ class BatchDecoder:
         """Persistent up to three sequences, gemm from five on (NVFP4 rows: always gemm).  Four: persistent where the launch
         runs on the tensor cores - a grid of at least 112 CTAs, whole ring chunks of vocabulary, room for the K-major
         copies; its group-per-sequence form takes 1.9 ms a step - and the cache has room for 8192 rows at most (FP8 12288).
-        Measured, us per step of four fp16 sequences at 64 / 1024 / 2048 / 4096 / 8000 tokens: 710 / 799 / 913 / 1146 / 1547
-        persistent, 756 / 803 / 870 / 1032 / 1278 gemm; FP8 rows 744 / 822 / 924 / 1118 / 1496 and 900 / 950 / 1009 / 1162 / 1418
-        (one long context among short ones costs either less).  So the GEMM step is the faster one behind about 1100 tokens
-        (FP8 5500); the bound on the rows dates from a GEMM step of 1127 / 1331 / 1583 us at 1024 / 4096 / 8000.  A four-slot
-        serving job, 32 prompts of 64 to 2048 tokens, 128 new ones each, tensor-core prefill: 0.95 s persistent, prefills
-        between the rounds; 0.99 s gemm with prefills beside them."""
+        Measured, us per step of four fp16 sequences at 64 / 1024 / 2048 / 4096 / 8000 tokens: 631 / 726 / 815 / 1001 / 1363
+        persistent, 758 / 804 / 870 / 1034 / 1290 gemm; FP8 rows 576 / 674 / 781 / 975 / 1358 and 904 / 959 / 1019 / 1180 / 1440
+        (one long context among short ones costs either less).  So the GEMM step is the faster one behind about 5000 tokens
+        (FP8 9500), and a cache of that many rows is shorter than that for most of its steps."""
         if weight_format == "nvfp4" or n > cls.MAX_SEQUENCES:
             return "gemm"
         if n < cls.MAX_SEQUENCES or vocab_size % 128:      # (the GEMM step reads vocabularies of whole tiles only)

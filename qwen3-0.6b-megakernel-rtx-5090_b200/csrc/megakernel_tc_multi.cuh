@@ -9,9 +9,9 @@
 // words read back, cache rows.
 // The launch it replaces (megakernel_batch.cuh, which stays for grids outside this kernel's range) gives each sequence a
 // group of warps that convert and multiply every weight for themselves, and has six hand-overs per layer.
-// Measured, us per step at 64 / 1024 / 2048-token contexts: two fp16 sequences 565 / 582 / 614, four 693 / 770 / 904, four
-// with FP8 rows 656 / 740 / 863 (the group launch: two 1137 / 1317 at 64 / 1024; four 1655 / 1942; the GEMM step: four fp16
-// 1080 / 1126 / 1189, four FP8 1230 / 1281 / 1345, with fp16-rounded activations).  Share of later layers' cache values
+// Measured, us per step at 64 / 1024 / 2048-token contexts: two fp16 sequences 494 / 516 / 569, three 632 / 702 / 760, four
+// 631 / 726 / 815, four with FP8 rows 576 / 674 / 781 (the group launch: two 1137 / 1317 at 64 / 1024; four 1655 / 1942; the
+// GEMM step: four fp16 758 / 804 / 870, four FP8 904 / 959 / 1019, with fp16-rounded activations).  Share of later layers' cache values
 // that round to another fp16 than float64's, 1024 tokens: two and four fp16 sequences 0.156 and 0.161 % (group launch 0.147
 // and 0.150), two with FP8 rows 0.152 (0.151).
 
