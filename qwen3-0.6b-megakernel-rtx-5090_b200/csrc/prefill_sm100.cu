@@ -333,9 +333,13 @@ static bool a_box_ok(int a_box_rows, int M, int *rows, uint32_t *a_box_bytes, st
   return true;
 }
 
-// Rows of the MMA for a launch: 64 where its only row tile has a short A box of at most that many and the tile has such a kernel.
+// Rows of the MMA for a launch: 64 where its only row tile has a short A box of at most that many and the tile has such a kernel; fp16
+// weights up to 48: behind that the product issues no faster with half the rows (us per step of 34 / 42 / 50 / 57 / 64 sequences of 64 tokens,
+// 64 rows -> 128: 766 / 837 / 877 / 889 / 897 -> 760 / 833 / 861 / 876 / 884; 44 and 64 of 128 to 1024 tokens 1240 / 1484 -> 1254 / 1470; 5 to 16
+// sequences gain 2 % by 64 rows, packed weights at every size).  A row's sums are the same bit for bit.
 static int mma_rows(const qmk_gemm::Groups &gr, int box_n, bool fuse, int wq) {
-  return gr.a_box_bytes > 0 && gr.a_box_bytes <= 64u * qmk_gemm::BK * 2 && t_ah == 1 && gr.row_scale[0] == nullptr && gemm_kernel_64(box_n, fuse, wq) ? 64 : qmk_gemm::BM;
+  const uint32_t most = wq == 0 ? 48 : 64;
+  return gr.a_box_bytes > 0 && gr.a_box_bytes <= most * qmk_gemm::BK * 2 && t_ah == 1 && gr.row_scale[0] == nullptr && gemm_kernel_64(box_n, fuse, wq) ? 64 : qmk_gemm::BM;
 }
 
 // C_g[M x N_g] fp32 = A[M x K] * B_g[N_g x K]^T for up to three matrices B_g in one launch.  M, N_g multiples of

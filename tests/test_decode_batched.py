@@ -316,6 +316,24 @@ def test_logits_without_a_largest_value_are_an_error(C, fmt, dumped):
         C.set_weight_format("fp16")
 
 
+@pytest.mark.parametrize("more", [49, 56, 64])
+def test_rows_of_the_mma_keep_the_bits(C, more):
+    """Steps of 48 fp16 sequences take 64-row products, of more 128-row ones: the sequences of both end in the same tokens and
+    cache rows bit for bit."""
+    vocab, steps = 2048, 6
+    w = S.make_weights(seed=33, num_layers=3, vocab_size=vocab, norm_std=0.1, max_seq_len=16)
+    prompts = [S.make_prompt(3 + 5 * i, seed=600 + i, vocab_size=vocab) for i in range(more)]
+    ends = []
+    for n in (48, more):
+        eng = _engine(w, n, 400, engine="gemm")
+        tokens = eng.generate_ids(prompts[:n], steps)
+        ends.append((tokens[:48], [(eng._k_caches[b][:, :, :eng.positions[b]].clone(), eng._v_caches[b][:, :, :eng.positions[b]].clone()) for b in range(48)]))
+        del eng
+    (t0, c0), (t1, c1) = ends
+    assert t0 == t1
+    assert all(torch.equal(k, x) and torch.equal(v, y) for (k, v), (x, y) in zip(c0, c1))
+
+
 def test_a_refused_layer_table_changes_no_later_call(C):
     """Layer tables are read back and their matrices' tensor maps kept until another table comes.  A table that is refused half-way
     (its second layer has a null pointer) has replaced the maps of its first: a call on the table before it makes them anew."""
