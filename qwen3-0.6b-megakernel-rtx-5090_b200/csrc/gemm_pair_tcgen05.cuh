@@ -153,8 +153,8 @@ __device__ __forceinline__ float2 as_floats(uint32_t bits) { return __half22floa
 // and written in whole lines: lane l has dims 2 l, 2 l + 1 and their partners 64 behind, no value crosses lanes.  The tables'
 // rows of the next step are asked for ahead (1500 / 2200 / 4096 tokens 2.456 / 3.14 / 6.28 -> 2.40 / 3.08 / 6.22 ms).  A first form, that
 // kernel's lanes and shuffles as they are, took 51 us a product at 4096 rows; this one 34, the product and the kernel in turn 43.
-// Storing plain halves takes 26.6: with heads an epilogue (about 55 instructions a row and warp, two warps on each scheduler) is longer
-// than the main loop it runs under.
+// Storing plain halves takes 26.6: with heads an epilogue (86 instructions a row of a head on average, two warps on each scheduler) is
+// longer than the main loop it runs under.
 __device__ __forceinline__ void store_heads(const Heads &a, uint32_t block, int lane, const uint32_t (&row)[64], int grp, int head, int t0) {
   using qmk_pf::D;
   int live = min(max(a.rows - t0, 0), 32), pos = a.pos0 + t0;
