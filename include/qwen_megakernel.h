@@ -416,6 +416,10 @@ const char *qmk_last_error(void);
 /* Persistent grid size (CTAs) and bytes of library-owned device scratch. */
 int qmk_num_ctas(void);
 long long qmk_scratch_bytes(void);
+/* CTAs that the tensor-core decode kernel for this weight format (0 fp16, 1 FP8) and number of sequences (1 to 4) is launched with
+ * where `ctas` are there (0: another kernel runs), and of CTA `cta` of them counts[0..4]: slots of its ring, chunks of a
+ * layer's q|k|v, O, gate / up and down parts.  Needs no device. */
+int qmk_selftest_decode_ring(int weight_format, int num_seqs, int ctas, int cta, int *counts);
 /* Runs one bounded wait on a word nothing ever sets, with budget_us
  * microseconds; returns QMK_ERR_WAIT_TIMEOUT when the wait gave up as designed. */
 int qmk_selftest_wait_timeout(int budget_us);

@@ -457,7 +457,7 @@ __device__ __forceinline__ bool wait_full(const Params &P, const Ctx &c, uint32_
 }
 
 // Rows [r0, r1) of an n-row matrix owned by CTA `cta` of `ncta` (launch-time only: 64-bit divisions).
-__host__ __device__ __forceinline__ void split_rows(int n, int ncta, int cta, int &r0, int &r1) {
+__host__ __device__ __forceinline__ constexpr void split_rows(int n, int ncta, int cta, int &r0, int &r1) {
   r0 = static_cast<int>((static_cast<long long>(n) * cta) / ncta);
   r1 = static_cast<int>((static_cast<long long>(n) * (cta + 1)) / ncta);
 }

@@ -592,7 +592,8 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
     // for the grids and vocabularies outside the limits, and where the K-major copies do not fit in memory.
     const qmk_fused_tc::Build &tc = qmk_fused_tc::build_seqs(e->wfmt, P.nseq);
     Engine::Prepared *prep = nullptr;
-    if (P.vocab % tc.rows_per_chunk == 0 && grid >= tc.min_ctas && grid <= tc.max_ctas) {
+    const int tc_grid = tc.grid(grid);
+    if (P.vocab % tc.rows_per_chunk == 0 && tc_grid > 0) {
       rc = ensure_prepared(e, P, e->wfmt, true, static_cast<int>(RED_ALLOC_WORDS), stream, &prep, true);
       if (rc != QMK_OK) return rc;
     }
@@ -604,6 +605,7 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
       kernel = tc.kernel;
       smem = tc.smem_bytes;
       threads = qmk::THREADS;
+      grid = tc_grid;
       // Two fp16 sequences: 128 CTAs have whole tiles everywhere (32 q|k|v, 48 gate / up rows, slices of 64 attention outputs: a CTA of 148
       // multiplies as many) and fewer contributions and readers to every sum.  us per step on 148 / 136 / 128 / 124 CTAs, 64 tokens 511 / 491
       // / 479 / 576, 1024 tokens 541 / 530 / 509 / 593; from about 2200 tokens on (566 / 583 / 566) the attention misses the others.  FP8 rows
@@ -620,7 +622,8 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
     // 724 -> 412 us per token at 1024-token contexts against the CUDA-core kernel, which stays for the grids and
     // vocabularies outside these limits.
     const qmk_fused_tc::Build &tc = qmk_fused_tc::build(e->wfmt);
-    const bool on_tensor_cores = e->fused >= 2 && P.vocab % tc.rows_per_chunk == 0 && grid >= tc.min_ctas && grid <= tc.max_ctas;
+    const int tc_grid = tc.grid(grid);
+    const bool on_tensor_cores = e->fused >= 2 && P.vocab % tc.rows_per_chunk == 0 && tc_grid > 0;
     Engine::Prepared *prep = nullptr;
     rc = ensure_prepared(e, P, e->wfmt, on_tensor_cores, qmk::RED_WORDS, stream, &prep);
     if (rc != QMK_OK) return rc;
@@ -634,6 +637,7 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
       if (rc != QMK_OK) return rc;
       kernel = tc.kernel;
       smem = tc.smem_bytes;
+      grid = tc_grid;
     }
   }
   if (!P.layers_t) QMK_CUDA(e, cudaMemsetAsync(e->status, 0, 16, stream));   // (cleared with the sums otherwise, see ensure_prepared)
@@ -1220,6 +1224,16 @@ int qmk_num_ctas(void) {
 
 long long qmk_scratch_bytes(void) {
   return static_cast<long long>(exchange_bytes()) + 16;
+}
+
+int qmk_selftest_decode_ring(int weight_format, int num_seqs, int ctas, int cta, int *counts) {
+  if (weight_format < 0 || weight_format > 1 || num_seqs < 1 || num_seqs > qmkp::MAX_SEQ || !counts) return -1;
+  const qmk_fused_tc::Build &tc = num_seqs == 1 ? qmk_fused_tc::build(weight_format) : qmk_fused_tc::build_seqs(weight_format, num_seqs);
+  const int grid = tc.grid(ctas);
+  int out[5] = {};
+  if (cta >= 0 && cta < grid) tc.ring(grid, cta, out);
+  for (int i = 0; i < 5; ++i) counts[i] = out[i];
+  return grid;
 }
 
 int qmk_selftest_wait_timeout(int budget_us) {

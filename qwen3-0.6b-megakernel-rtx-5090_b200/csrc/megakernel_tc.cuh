@@ -82,14 +82,58 @@ static_assert(O_PITCH % 128 == 16, "eight consecutive rows of an O chunk fall in
 static_assert(SLOT_BYTES >= ODD_SLOT_SKEW + O_CH_ROWS * O_PITCH, "a slot holds a chunk of O rows");
 static_assert(O_MAX_QUADS <= 2 * CONS_WARPS - 2, "merge: two quads per warp, one for the last two");
 static_assert(4 * O_MAX_QUADS <= D, "a slice lies in at most two query heads");
-// The norm vectors of layer L go into the buffer of layer L - 2 as soon as the ring has room for layer L's first
-// chunks, i.e. when chunk (last of L - 1) - NSLOTS was handed back.  That must be a gate/up chunk of layer L - 2 or a
-// later one: every warp is past its last use of L - 2's norm vectors (post_ln, before the gate/up rows) by then.  fp16
-// layers have over 18 chunks on every CTA; the short layers of FP8 rows bound the grid.
+// Chunks that CTA `cta` of `ncta` reads of a layer: of the q|k|v rows, of its slice of the attention outputs (scales included; none
+// past the last whole group), of the gate (= up, down) rows.  The counts of tc_setup, for the host: called there too, this
+// function cost four FP8 sequences 0.7 % of a step (the code around it comes out differently).
+constexpr int QKV_CHUNKS = QKV_ROWS / CH_ROWS, GU_CHUNKS = I / CH_ROWS;
+struct LayerChunks { int nq, no, ng; };
+constexpr LayerChunks layer_chunks(int ncta, int cta) {
+  LayerChunks s = {};
+  int a = 0, b = 0;
+  split_rows(QKV_CHUNKS, ncta, cta, a, b); s.nq = b - a;
+  split_rows(GU_CHUNKS, ncta, cta, a, b); s.ng = b - a;
+  if (cta / O_GROUP < ncta / O_GROUP) {
+    split_rows(QS / 4, ncta / O_GROUP, cta / O_GROUP, a, b);
+    s.no = (4 * (b - a) + O_CH_ROWS - 1) / O_CH_ROWS + SCALE_CH;
+  }
+  return s;
+}
+// The norm vectors of layer L go into the buffer of layer L - 2 as soon as the ring has room for the last chunk of layer L - 1,
+// i.e. when the chunk NSLOTS before it was handed back.  That must be a gate/up chunk of layer L - 2 or a later one: every warp is
+// past its last use of L - 2's norm vectors (post_ln, before the gate/up rows) by then.  So layer L - 1 and what follows the O chunks
+// of L - 2 have to be more chunks than the ring has slots, on every CTA; an attention item only adds to L - 1.  fp16 layers are long
+// enough on all grids.  FP8 layers are not on a CTA without an O slice, and up to 160 CTAs on the others.
+constexpr bool norms_outlive_use(int ncta) {
+  for (int cta = 0; cta < ncta; ++cta) {
+    const LayerChunks s = layer_chunks(ncta, cta);
+    if (s.nq + s.no + 2 * (3 * s.ng + SCALE_CH) <= NSLOTS) return false;
+  }
+  return true;
+}
+// The grid of this kernel where `ctas` CTAs are there: the largest that the norm vectors allow, 0 (another kernel runs) outside
+// [TC_MIN_CTAS, TC_MAX_CTAS].
 constexpr int TC_MAX_CTAS = FP8_ROWS ? 160 : MAX_CTAS;
-constexpr int MIN_QKV_CH = QKV_ROWS / CH_ROWS / TC_MAX_CTAS, MIN_O_CH = O_GROUP * QS / TC_MAX_CTAS / O_CH_ROWS + SCALE_CH,
-              MIN_GU_CH = I / CH_ROWS / TC_MAX_CTAS, MIN_LAYER_CH = MIN_QKV_CH + MIN_O_CH + 3 * MIN_GU_CH + SCALE_CH;
-static_assert(MIN_LAYER_CH > NSLOTS || 2 * MIN_LAYER_CH - 1 - NSLOTS >= MIN_QKV_CH + MIN_O_CH, "norm vectors overwritten in use");
+inline int tc_grid(int ctas) {
+  struct Table { short largest[TC_MAX_CTAS + 1]; };
+  static const Table table = [] {
+    Table t = {};
+    for (int n = TC_MIN_CTAS; n <= TC_MAX_CTAS; ++n) t.largest[n] = norms_outlive_use(n) ? static_cast<short>(n) : t.largest[n - 1];
+    return t;
+  }();
+  return ctas < 0 || ctas > TC_MAX_CTAS ? 0 : table.largest[ctas];
+}
+inline void tc_ring(int ncta, int cta, int (&out)[5]) {
+  const LayerChunks s = layer_chunks(ncta, cta);
+  const int counts[5] = {NSLOTS, s.nq, s.no, 2 * s.ng, s.ng + SCALE_CH};
+  for (int i = 0; i < 5; ++i) out[i] = counts[i];
+}
+// (Grids without a CTA that has no O slice all hold, so that at most three CTAs stay idle.)
+constexpr bool whole_groups_hold() {
+  for (int n = TC_MIN_CTAS; n <= TC_MAX_CTAS; n += O_GROUP)
+    if (!norms_outlive_use(n)) return false;
+  return true;
+}
+static_assert(whole_groups_hold(), "norm vectors overwritten in use");
 static_assert(SLOT_BYTES % 128 == 0 && NSLOTS % 2 == 0, "swizzled boxes need 128-byte aligned slots; slot parity = chunk parity");
 static_assert(EMPTY_UNITS == 12, "1, 2, 3, 4, 6 or 12 warps share a chunk");
 constexpr float LO_SCALE = 2048.0f, LO_INV = 1.0f / 2048.0f;
@@ -99,7 +143,6 @@ constexpr int KV_BOX = KV_ROWS_PER_CHUNK * 128;
 constexpr int KV_V_OFF = 2 * KV_BOX;
 constexpr int KV_PITCH = 2 * D + 16;           // pitch of the four query-operand rows (plain padded rows)
 static_assert(SLOT_BYTES >= 4 * KV_BOX, "a slot holds the four boxes of a cache chunk");
-constexpr int QKV_CHUNKS = QKV_ROWS / CH_ROWS, GU_CHUNKS = I / CH_ROWS;
 static_assert(CH_ROWS * ((GU_CHUNKS + TC_MIN_CTAS - 1) / TC_MIN_CTAS) <= 32, "slice_cols takes two k-steps");
 constexpr int KPAIRS = H / 32;                 // pairs of 16-input k-steps in a row
 constexpr int ACT16_PITCH = 32 * O_KPAIRS + 8; // halves between the hi and the lo row of a slice's activations (other banks)
@@ -1376,7 +1419,7 @@ __device__ __forceinline__ void tc_setup(const Params &P, const Ctx &c) {
     tt->groups = c.ncta / O_GROUP;
     const int grp = c.cta / O_GROUP;
     tt->oq = c.cta % O_GROUP;
-    tt->e0 = tt->ne = tt->no = tt->n0 = tt->n1 = 0;
+    tt->e0 = tt->ne = tt->no = tt->n0 = tt->n1 = 0;   // (chunks as in layer_chunks)
     if (grp < tt->groups) {
       split_rows(QS / 4, tt->groups, grp, a, b); tt->e0 = 4 * a; tt->ne = 4 * (b - a);
       split_rows(O_COLS, tt->groups, grp, a, b); tt->n0 = tt->oq * O_COLS + a; tt->n1 = tt->oq * O_COLS + b;

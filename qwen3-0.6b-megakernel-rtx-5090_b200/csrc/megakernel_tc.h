@@ -9,8 +9,9 @@ namespace qmk_fused_tc {
 struct Build {
   const void *kernel;          // __global__ entry, launched cooperatively with one Params argument
   size_t smem_bytes;           // dynamic shared memory of one CTA
-  int min_ctas, max_ctas;      // grids the kernel's shared-memory slices and its ring are sized for
+  int (*grid)(int ctas);       // the largest grid of at most `ctas` CTAs that its shared-memory slices and its ring are sized for, or 0
   int rows_per_chunk;          // rows are owned in units of this many: the vocabulary is a multiple of it
+  void (*ring)(int ncta, int cta, int (&out)[5]);   // slots of the ring; a layer's q|k|v, O, gate / up and down chunks of a CTA
 };
 const Build &build_f16();
 const Build &build_fp8();

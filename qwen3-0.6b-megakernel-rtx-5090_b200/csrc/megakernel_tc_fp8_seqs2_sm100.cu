@@ -25,8 +25,8 @@
 
 namespace qmk_fused_tc {
 const Build &build_fp8_seqs2() {
-  static const Build b = {reinterpret_cast<const void *>(qmkt8s2::qwen3_decode_megakernel_tc_seqs), qmkt8s2::TC_SMEM_BYTES, qmkt8s2::TC_MIN_CTAS,
-                          qmkt8s2::TC_MAX_CTAS, qmkt8s2::CH_ROWS};
+  static const Build b = {reinterpret_cast<const void *>(qmkt8s2::qwen3_decode_megakernel_tc_seqs), qmkt8s2::TC_SMEM_BYTES, qmkt8s2::tc_grid,
+                          qmkt8s2::CH_ROWS, qmkt8s2::tc_ring};
   return b;
 }
 }  // namespace qmk_fused_tc

@@ -26,8 +26,8 @@
 
 namespace qmk_fused_tc {
 const Build &build_fp8_seqs4() {
-  static const Build b = {reinterpret_cast<const void *>(qmkt8s4::qwen3_decode_megakernel_tc_seqs), qmkt8s4::TC_SMEM_BYTES, qmkt8s4::TC_MIN_CTAS,
-                          qmkt8s4::TC_MAX_CTAS, qmkt8s4::CH_ROWS};
+  static const Build b = {reinterpret_cast<const void *>(qmkt8s4::qwen3_decode_megakernel_tc_seqs), qmkt8s4::TC_SMEM_BYTES, qmkt8s4::tc_grid,
+                          qmkt8s4::CH_ROWS, qmkt8s4::tc_ring};
   return b;
 }
 }  // namespace qmk_fused_tc

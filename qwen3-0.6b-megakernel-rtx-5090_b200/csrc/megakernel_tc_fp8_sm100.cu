@@ -24,8 +24,8 @@
 
 namespace qmk_fused_tc {
 const Build &build_fp8() {
-  static const Build b = {reinterpret_cast<const void *>(qmkt8::qwen3_decode_megakernel_tc), qmkt8::TC_SMEM_BYTES, qmkt8::TC_MIN_CTAS,
-                          qmkt8::TC_MAX_CTAS, qmkt8::CH_ROWS};
+  static const Build b = {reinterpret_cast<const void *>(qmkt8::qwen3_decode_megakernel_tc), qmkt8::TC_SMEM_BYTES, qmkt8::tc_grid,
+                          qmkt8::CH_ROWS, qmkt8::tc_ring};
   return b;
 }
 }  // namespace qmk_fused_tc

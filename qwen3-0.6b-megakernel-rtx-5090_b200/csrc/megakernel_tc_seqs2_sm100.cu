@@ -24,8 +24,8 @@
 
 namespace qmk_fused_tc {
 const Build &build_f16_seqs2() {
-  static const Build b = {reinterpret_cast<const void *>(qmkts2::qwen3_decode_megakernel_tc_seqs), qmkts2::TC_SMEM_BYTES, qmkts2::TC_MIN_CTAS,
-                          qmkts2::TC_MAX_CTAS, qmkts2::CH_ROWS};
+  static const Build b = {reinterpret_cast<const void *>(qmkts2::qwen3_decode_megakernel_tc_seqs), qmkts2::TC_SMEM_BYTES, qmkts2::tc_grid,
+                          qmkts2::CH_ROWS, qmkts2::tc_ring};
   return b;
 }
 }  // namespace qmk_fused_tc

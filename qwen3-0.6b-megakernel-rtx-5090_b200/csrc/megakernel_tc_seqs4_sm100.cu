@@ -25,8 +25,8 @@
 
 namespace qmk_fused_tc {
 const Build &build_f16_seqs4() {
-  static const Build b = {reinterpret_cast<const void *>(qmkts4::qwen3_decode_megakernel_tc_seqs), qmkts4::TC_SMEM_BYTES, qmkts4::TC_MIN_CTAS,
-                          qmkts4::TC_MAX_CTAS, qmkts4::CH_ROWS};
+  static const Build b = {reinterpret_cast<const void *>(qmkts4::qwen3_decode_megakernel_tc_seqs), qmkts4::TC_SMEM_BYTES, qmkts4::tc_grid,
+                          qmkts4::CH_ROWS, qmkts4::tc_ring};
   return b;
 }
 }  // namespace qmk_fused_tc

@@ -24,8 +24,8 @@
 
 namespace qmk_fused_tc {
 const Build &build_f16() {
-  static const Build b = {reinterpret_cast<const void *>(qmkt::qwen3_decode_megakernel_tc), qmkt::TC_SMEM_BYTES, qmkt::TC_MIN_CTAS,
-                          qmkt::TC_MAX_CTAS, qmkt::CH_ROWS};
+  static const Build b = {reinterpret_cast<const void *>(qmkt::qwen3_decode_megakernel_tc), qmkt::TC_SMEM_BYTES, qmkt::tc_grid,
+                          qmkt::CH_ROWS, qmkt::tc_ring};
   return b;
 }
 }  // namespace qmk_fused_tc

@@ -113,6 +113,8 @@ _lib.qmk_sync_status.restype = _I
 _lib.qmk_last_error.restype = ctypes.c_char_p
 _lib.qmk_num_ctas.restype = _I
 _lib.qmk_scratch_bytes.restype = ctypes.c_longlong
+_lib.qmk_selftest_decode_ring.argtypes = [_I, _I, _I, _I, ctypes.POINTER(_I)]
+_lib.qmk_selftest_decode_ring.restype = _I
 _lib.qmk_selftest_wait_timeout.argtypes = [_I]
 _lib.qmk_selftest_wait_timeout.restype = _I
 _lib.qmk_selftest_gemm_wait_timeout.argtypes = [_I]
@@ -128,7 +130,7 @@ EXPORTED_SYMBOLS = (
     "launch_ldg_decode_direct", "launch_ldg_decode_persistent", "launch_ldg_generate_nosync",
     "launch_ldg_prefill", "qmk_abi_version", "qmk_configure", "qmk_set_inv_freq", "qmk_set_logits_dump",
     "qmk_set_weight_format", "qmk_set_tuning", "qmk_set_tuning2", "qmk_set_profile_buffer", "qmk_set_fused", "qmk_set_step_overlap", "qmk_set_prefill_attention", "qmk_set_decode_attention", "qmk_invalidate_weights", "qmk_release_weights", "qmk_decode", "qmk_generate", "qmk_generate_static", "qmk_generate_batch", "qmk_gemm_f16_tn", "qmk_gemm_packed_tn", "qmk_decode_batched", "qmk_prefill_chunked", "qmk_prefill_packed", "qmk_prefill_packed_passes", "qmk_prefill", "qmk_engine_create", "qmk_engine_destroy", "qmk_engine_apply", "qmk_engine_decode", "qmk_engine_generate", "qmk_engine_prefill", "qmk_sync_status", "qmk_last_error", "qmk_num_ctas",
-    "qmk_scratch_bytes", "qmk_selftest_wait_timeout", "qmk_selftest_gemm_wait_timeout", "qmk_selftest_attention_wait_timeout", "qmk_selftest_gemm_pair_wait_timeout", "qmk_selftest_decode_attention_wait_timeout",
+    "qmk_scratch_bytes", "qmk_selftest_decode_ring", "qmk_selftest_wait_timeout", "qmk_selftest_gemm_wait_timeout", "qmk_selftest_attention_wait_timeout", "qmk_selftest_gemm_pair_wait_timeout", "qmk_selftest_decode_attention_wait_timeout",
 )
 
 
@@ -586,7 +588,7 @@ def gemm_packed_tn(a: torch.Tensor, b: torch.Tensor, weight_format, b2: torch.Te
     rows, see ``quantize.pack_rows_fp8`` / ``pack_rows_nvfp4``).  ``mode``: ``"plain"`` -> fp32 ``[m, n]``; ``"splitk"`` ->
     fp32 ``[4, m, n]`` partial matrices; ``"swiglu"`` (``b`` gate, ``b2`` up) -> fp16 ``[m, n]``."""
     _require_cuda()
-    fmt = WEIGHT_FORMATS[weight_format] if isinstance(weight_format, str) else int(weight_format)
+    fmt = WEIGHTWEIGHT_FORMATS[weight_format] if isinstance(weight_format, str) else int(weight_format)
     code = {"plain": 0, "splitk": 1, "swiglu": 2}[mode]
     _check(a.is_cuda and a.dtype == torch.float16 and a.is_contiguous() and a.dim() == 2,
            "gemm_packed_tn: a must be a contiguous fp16 CUDA matrix [m, k]")
@@ -622,6 +624,13 @@ def num_ctas() -> int:
 
 def scratch_bytes() -> int:
     return int(_lib.qmk_scratch_bytes())
+
+
+def selftest_decode_ring(weight_format: str, num_seqs: int, ctas: int, cta: int = 0):
+    """(grid, slots, q|k|v, O, gate / up, down chunks) of the tensor-core decode kernel where ``ctas`` CTAs are there, the chunks those
+    of CTA ``cta`` and one layer; grid 0: another kernel runs.  Needs no device."""
+    counts = (_I * 5)()
+    return (int(_lib.qmk_selftest_decode_ring(WEIGHT_FORMATS[weight_format], int(num_seqs), int(ctas), int(cta), counts)), *counts)
 
 
 def selftest_wait_timeout(budget_us: int = 200) -> int:

@@ -270,6 +270,30 @@ def test_attention_slices_of_every_grid(C, fmt, n, ctas):
         assert float((dump[b] - logits[b]).abs().max()) < LOGIT_TOL
 
 
+@pytest.mark.parametrize("fmt", ["fp16", "fp8"])
+@pytest.mark.parametrize("n,ctas", [(1, 147), (2, 147), (1, 146), (2, 115), (4, 147), (1, 144)])
+def test_norm_vectors_of_every_layer_on_grids_that_are_no_multiple_of_four(C, fmt, n, ctas):
+    """Six layers whose norm vectors differ from one another as much as from one (the two buffers of a CTA alternate by layer, so that
+    two layers with the vectors of each other's predecessors would show nothing), on grids that leave CTAs without an O slice or are
+    rounded down because of them.  One CTA's gate / up rows normalised with another layer's vector are 16 to 24 of 3072 in every layer: with
+    logits of order one about sqrt(24 / 3072) = 0.09 of what the down products add, several times the bar of 3e-2."""
+    import quantize as Q
+    w = S.make_weights(seed=19, num_layers=6, vocab_size=2048, norm_std=0.7, max_seq_len=16)
+    engine_w, oracle_w = Q.quantize_weights_fp8(w) if fmt == "fp8" else (w, w)
+    prompts = [S.make_prompt(L, seed=90 + i, vocab_size=2048) for i, L in enumerate([150, 9, 70, 40][:n])]
+    want, logits = _oracle(oracle_w, 320, prompts, 6)
+    eng = _batch_engine(engine_w, n, 320, weight_format=fmt)
+    C.configure(max_ctas=ctas)
+    try:
+        got, dump = _run_with_dump(C, eng, prompts, 6, 2048)
+    finally:
+        C.configure(max_ctas=0)
+        C.set_weight_format("fp16")
+    for b in range(n):
+        assert got[b] == want[b]
+        assert float((dump[b] - logits[b]).abs().max()) < LOGIT_TOL
+
+
 @pytest.mark.parametrize("length", [2030, 2045])
 def test_two_sequences_either_side_of_the_smaller_grid(C, length):
     """Two fp16 sequences take 128 CTAs up to 2048 positions and the whole device beyond (18 steps from 2030 end at 2047, from 2045 at

@@ -50,6 +50,29 @@ def test_refusals_without_an_engine_have_a_text(built_library):
     assert lib.qmk_engine_destroy(None) == 0
 
 
+@pytest.mark.parametrize("fmt", ["fp16", "fp8"])
+@pytest.mark.parametrize("n", [1, 2, 3, 4])
+def test_norm_vectors_are_not_overwritten_in_use_on_any_grid(built_library, fmt, n):
+    """The persistent tensor-core kernels copy layer L's norm vectors over layer L - 2's when the slot of layer L - 1's last chunk is
+    free, i.e. the chunk `slots` before it was handed back.  With the real chunk counts of every CTA of every grid that
+    a limit on the CTAs leads to, that chunk is a gate / up chunk of L - 2 or a later one (post_ln is read in front of them).  An
+    attention item adds chunks between q|k|v and O."""
+    import qwen_megakernel_C as C
+    launched = {}
+    for ctas in range(1, 270):
+        grid = C.selftest_decode_ring(fmt, n, ctas)[0]
+        assert (grid > 0) == ((112 if n > 2 else 96) <= ctas <= (160 if fmt == "fp8" else 256))
+        assert grid == 0 or ctas - 3 <= grid <= ctas and (ctas % 4 or grid == ctas)
+        launched[grid] = ctas
+    for grid in sorted(launched)[1:]:
+        for cta in range(grid):
+            _, slots, qkv, o, gate_up, down = C.selftest_decode_ring(fmt, n, grid, cta)
+            for attention in (0, 1, 8):
+                layer = [0] * (qkv + attention + o) + [1] * (gate_up + down)       # 1: behind the last use of post_ln
+                handed_back = 2 * len(layer) - 1 - slots                            # counted from layer L - 2's first chunk
+                assert handed_back >= len(layer) or handed_back >= 0 and layer[handed_back], (grid, cta)
+
+
 def test_abi_version_handshake(built_library):
     import qwen_megakernel_C as C
     from Model import Qwen06B_architecture as A
