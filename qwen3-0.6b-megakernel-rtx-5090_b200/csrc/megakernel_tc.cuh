@@ -110,14 +110,17 @@ constexpr bool norms_outlive_use(int ncta) {
   }
   return true;
 }
-// The grid of this kernel where `ctas` CTAs are there: the largest that the norm vectors allow, 0 (another kernel runs) outside
+// One sequence: the last two warps make the split weights of a merge, and take part in it where the slice has a quad for them (merge_o;
+// with the test taken out there, 777 tokens took 0.6 % longer).  That is every slice up to 171 CTAs.
+constexpr bool slices_reach_last_warp(int ncta) { return TC_SEQS > 1 || QS / 4 / (ncta / O_GROUP) >= CONS_WARPS; }
+// The grid of this kernel where `ctas` CTAs are there: the largest that holds in both ways, 0 (another kernel runs) outside
 // [TC_MIN_CTAS, TC_MAX_CTAS].
 constexpr int TC_MAX_CTAS = FP8_ROWS ? 160 : MAX_CTAS;
 inline int tc_grid(int ctas) {
   struct Table { short largest[TC_MAX_CTAS + 1]; };
   static const Table table = [] {
     Table t = {};
-    for (int n = TC_MIN_CTAS; n <= TC_MAX_CTAS; ++n) t.largest[n] = norms_outlive_use(n) ? static_cast<short>(n) : t.largest[n - 1];
+    for (int n = TC_MIN_CTAS; n <= TC_MAX_CTAS; ++n) t.largest[n] = norms_outlive_use(n) && slices_reach_last_warp(n) ? static_cast<short>(n) : t.largest[n - 1];
     return t;
   }();
   return ctas < 0 || ctas > TC_MAX_CTAS ? 0 : table.largest[ctas];
@@ -127,7 +130,7 @@ inline void tc_ring(int ncta, int cta, int (&out)[5]) {
   const int counts[5] = {NSLOTS, s.nq, s.no, 2 * s.ng, s.ng + SCALE_CH};
   for (int i = 0; i < 5; ++i) out[i] = counts[i];
 }
-// (Grids without a CTA that has no O slice all hold, so that at most three CTAs stay idle.)
+// (Grids without a CTA that has no O slice all hold for the norm vectors: at most three CTAs stay idle because of them.)
 constexpr bool whole_groups_hold() {
   for (int n = TC_MIN_CTAS; n <= TC_MAX_CTAS; n += O_GROUP)
     if (!norms_outlive_use(n)) return false;
