@@ -7,6 +7,11 @@
 #include <string>
 
 namespace qmk_internal {
+// What an engine's options say about its weights (they are the device's, and any thread may change them between two calls).
+struct WeightOptions {
+  int vocab, wfmt, rope_from_table;
+  float inv_freq[64];
+};
 struct PrefillEnv {
   const float *rope;      // fp32 [position][cos 64 | sin 64] covering max_seq_len (null in table mode)
   int vocab;
@@ -18,8 +23,9 @@ struct PrefillEnv {
   int attn_tc;            // 1: prefill attention on tcgen05 (causal_attention_tc), 0: on mma.sync (causal_attention_mma)
   int pdl;                // 1: kernels of a decode step / prefill pass are launched as programmatic dependents of one another
 };
-// Engine of the current device, created on first use; clears its last error.
-int prefill_env(int max_seq_len, cudaStream_t stream, PrefillEnv *out);
+// Engine of the current device, created on first use; clears its last error.  `own`, of a call of several passes: the first pass
+// leaves the options here, later ones make them the engine's again under the same hold of the lock.
+int prefill_env(int max_seq_len, cudaStream_t stream, PrefillEnv *out, WeightOptions *own = nullptr, bool first = true);
 // Start of an entry point that returns a status: from here on qmk_last_error on this thread speaks of this call.
 void begin_call();
 // Text for qmk_last_error on this thread, and nothing else.

@@ -260,7 +260,7 @@ struct Engine {
   int repl = 4;              // measured: 835 -> 752 us/token at short context, 1152 -> 1061 at 4096
   int stream_inflight = 0;   // measured: pacing the stream changes nothing
   bool inv_freq_set = false;
-  float inv_freq[qmk::D / 2] = {};   // host copy of what c_inv_freq holds (when inv_freq_set)
+  float inv_freq[qmk::D / 2] = {};   // host copy of what c_inv_freq holds (once ready)
   // fused single-sequence kernel (megakernel_fused.cuh)
   int fused = 2;             // 0: always the unfused kernel; 1: fused, CUDA-core row products; 2: fused, tensor-core row products
   int red_copies = 1;
@@ -373,6 +373,7 @@ int ensure_ready(Engine *e) {
     float inv[qmk::D / 2];
     for (int i = 0; i < qmk::D / 2; ++i) inv[i] = static_cast<float>(1.0 / pow(1.0e6, (2.0 * i) / qmk::D));
     QMK_CUDA(e, cudaMemcpyToSymbol(qmk::c_inv_freq, inv, sizeof(inv)));
+    memcpy(e->inv_freq, inv, sizeof(inv));
   }
   e->seq = 0;
   e->ready = true;
@@ -411,6 +412,17 @@ int ensure_rope(Engine *e, int max_seq_len, cudaStream_t stream) {
   // the table is shared by launches on other streams (overlapped prefill): it is complete before it is published
   QMK_CUDA(e, cudaStreamSynchronize(stream));
   e->rope_cap = cap;
+  return QMK_OK;
+}
+
+// Rotary frequencies; the same again cost nothing (callers re-apply their options before every op).
+int set_inv_freq(Engine *e, const float *inv_freq64) {
+  if (e->inv_freq_set && memcmp(e->inv_freq, inv_freq64, sizeof(e->inv_freq)) == 0) return QMK_OK;
+  QMK_CUDA(e, cudaDeviceSynchronize());   // no launch may still be reading the old table
+  QMK_CUDA(e, cudaMemcpyToSymbol(qmk::c_inv_freq, inv_freq64, sizeof(e->inv_freq)));
+  memcpy(e->inv_freq, inv_freq64, sizeof(e->inv_freq));
+  e->inv_freq_set = true;
+  e->rope_cap = 0;   // rebuilt with the new frequencies at the next launch
   return QMK_OK;
 }
 
@@ -683,12 +695,23 @@ Params base_params(const void *embed, const LDGLayerWeight *layers, const void *
 }  // namespace
 
 namespace qmk_internal {
-int prefill_env(int max_seq_len, cudaStream_t stream, PrefillEnv *out) {
+int prefill_env(int max_seq_len, cudaStream_t stream, PrefillEnv *out, WeightOptions *own, bool first) {
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e) return no_device();
   clear_error(e);
   int rc = ensure_ready(e);
+  if (own && first) {
+    own->vocab = e->vocab;
+    own->wfmt = e->wfmt;
+    own->rope_from_table = e->rope_from_table;
+    memcpy(own->inv_freq, e->inv_freq, sizeof(own->inv_freq));
+  } else if (own) {
+    e->vocab = own->vocab;
+    e->wfmt = own->wfmt;
+    e->rope_from_table = own->rope_from_table;
+    if (rc == QMK_OK && memcmp(e->inv_freq, own->inv_freq, sizeof(e->inv_freq)) != 0) rc = set_inv_freq(e, own->inv_freq);
+  }
   if (rc == QMK_OK) rc = ensure_rope(e, max_seq_len, stream);
   if (rc != QMK_OK) return rc;
   out->rope = e->rope;
@@ -737,14 +760,7 @@ int qmk_set_inv_freq(const float *inv_freq64) {
   std::lock_guard<std::recursive_mutex> lock(g_mutex);
   Engine *e = current_engine_unlocked();
   if (!e || !inv_freq64) return refuse(QMK_ERR_BAD_ARGUMENT, e ? "inv_freq64 is null" : "no CUDA device");
-  // callers re-apply their options before every op: the same frequencies again cost nothing
-  if (e->inv_freq_set && memcmp(e->inv_freq, inv_freq64, sizeof(e->inv_freq)) == 0) return QMK_OK;
-  QMK_CUDA(e, cudaDeviceSynchronize());   // no launch may still be reading the old table
-  QMK_CUDA(e, cudaMemcpyToSymbol(qmk::c_inv_freq, inv_freq64, sizeof(float) * (qmk::D / 2)));
-  memcpy(e->inv_freq, inv_freq64, sizeof(e->inv_freq));
-  e->inv_freq_set = true;
-  e->rope_cap = 0;   // rebuilt with the new frequencies at the next launch
-  return QMK_OK;
+  return set_inv_freq(e, inv_freq64);
 }
 
 int qmk_set_logits_dump(float *logits_out) {
@@ -1059,13 +1075,8 @@ int apply_handle_unlocked(qmk_engine *h, const void *table) {
   if (c.timeout_ms > 0) e->timeout_ms = c.timeout_ms;
   e->wfmt = c.weight_format;
   if (c.fused >= 0) e->fused = c.fused;   // a speed knob, not a property of the weights: negative leaves qmk_set_fused's value
-  if ((!e->inv_freq_set || memcmp(e->inv_freq, h->inv_freq, sizeof(h->inv_freq)) != 0)) {
-    QMK_CUDA(e, cudaDeviceSynchronize());   // no launch may still be reading the old table
-    QMK_CUDA(e, cudaMemcpyToSymbol(qmk::c_inv_freq, h->inv_freq, sizeof(h->inv_freq)));
-    memcpy(e->inv_freq, h->inv_freq, sizeof(h->inv_freq));
-    e->inv_freq_set = true;
-    e->rope_cap = 0;
-  }
+  const int rc = set_inv_freq(e, h->inv_freq);
+  if (rc != QMK_OK) return rc;
   if (table) {
     bool seen = false;
     for (const void *t : h->tables) seen |= (t == table);

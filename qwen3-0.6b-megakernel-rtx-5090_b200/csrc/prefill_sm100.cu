@@ -704,8 +704,9 @@ struct PackedSeqs {
   const int *lens;
   void *const *k_caches, *const *v_caches;
 };
-// One of the passes of a call: the first one reads the layer table and clears the status, the last one waits and reports.
-struct Pass { bool first = true, last = true; int index = 0; };
+// One of the passes of a call: the first one reads the layer table and clears the status, the last one waits and reports.  All run
+// with the options that the first one found: the maps are those of its weight format.
+struct Pass { bool first = true, last = true; int index = 0; qmk_internal::WeightOptions *options = nullptr; };
 constexpr int MAX_PACKED_SEQS = 64;
 constexpr size_t PK_ROWS_OFF = 0, PK_ITEMS_OFF = 32768, PK_MAPS_OFF = 49152, PK_PTRS_OFF = 65536, PK_BYTES = 66560;
 
@@ -729,7 +730,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
   using namespace qmk_pf;
   if (num_tokens <= 0) return QMK_OK;
   qmk_internal::PrefillEnv env;
-  int rc = qmk_internal::prefill_env(max_seq_len, stream, &env);
+  int rc = qmk_internal::prefill_env(max_seq_len, stream, &env, pass.options, pass.first);
   if (rc != QMK_OK) return rc;
   if (split) env.attn_tc = 0;   // (split operands have an attention kernel of their own)
   if (!token_ids_host || !embed_weight || !layer_weights || (!pk && (!k_cache || !v_cache)))
@@ -1152,6 +1153,7 @@ extern "C" int qmk_prefill_packed_passes(const int *token_ids_host, int num_pass
     if (seqs_per_pass[p] < 1 || seqs_per_pass[p] > MAX_PACKED_SEQS)
       return qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "packed prefill: 1 to 64 sequences a pass, each from position 0");
   std::lock_guard<std::recursive_mutex> lock(g_ws_mu);   // (the passes share one workspace and one status)
+  qmk_internal::WeightOptions options;
   int rc = QMK_OK;
   for (int p = 0, s0 = 0; p < num_passes && rc == QMK_OK; s0 += seqs_per_pass[p++]) {
     long total = 0;
@@ -1161,6 +1163,7 @@ extern "C" int qmk_prefill_packed_passes(const int *token_ids_host, int num_pass
     pass.first = p == 0;
     pass.last = p + 1 == num_passes;
     pass.index = p;
+    pass.options = &options;
     rc = total < 1 ? qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "packed prefill: empty sequence or null cache")
                    : prefill_impl(token_ids_host, static_cast<int>(total), embed_weight, layer_weights, cos_table, sin_table, nullptr, nullptr,
                                   num_layers, 0, max_seq_len, attn_scale, stream, &pk, false, nullptr, pass);

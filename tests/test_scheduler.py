@@ -397,3 +397,71 @@ def test_gpu_packed_passes_of_one_call(built_library, fmt):
             assert torch.equal(eng._k_caches[b][:, :, :lens[b]], want[b][0][:, :, :lens[b]])
     finally:
         C.set_weight_format("fp16")
+
+
+def _passes(C, w, vocab, lens, seed, fmt="fp16"):
+    """A batched engine and the arguments that send one packed pass of its own for every prompt in one call."""
+    from Model.Qwen06B_architecture import BatchDecoder
+    eng = BatchDecoder(weights=w, tokenizer=S.StubTokenizer(-1, vocab), num_sequences=len(lens), max_seq_len=max(lens), engine="gemm",
+                       prefill_mode="tensor", weight_format=fmt)
+    base = eng._base
+    prompts = [S.make_prompt(n, seed=seed + i, vocab_size=vocab) for i, n in enumerate(lens)]
+    return eng, ([1] * len(lens), prompts, base._embed_weight, base._layer_weights_packed, base._cos_table, base._sin_table, eng._k_caches,
+                 eng._v_caches, base.num_layers, eng.max_seq_len, base._attn_scale)
+
+
+def _when_rows_appear(cache, do):
+    """A thread that calls `do` as soon as the first pass has written rows of its last layer (its options have been read then)."""
+    import threading
+    stream = torch.cuda.Stream()
+
+    def body():
+        with torch.cuda.stream(stream):
+            while float(cache[-1, :, 0].float().abs().max()) == 0:
+                pass
+        do()
+    t = threading.Thread(target=body)
+    t.start()
+    return t
+
+
+@pytest.mark.gpu
+def test_gpu_options_set_by_another_thread_between_the_passes_of_a_call(built_library):
+    """Options are the device's.  A call of several packed passes runs all of them with those that its first one found: an engine of
+    another format (vocabulary, frequencies) that another thread makes current meanwhile changes no row."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import qwen_megakernel_C as C
+    vocab, lens = 2048, [1500] * 24
+    w = S.weights_to(S.make_weights(seed=12, num_layers=8, vocab_size=vocab, norm_std=0.1, max_seq_len=16), "cuda")
+    eng, args = _passes(C, w, vocab, lens, 700)
+    running, changes = True, 0
+
+    def others():
+        nonlocal changes
+        other = torch.full((64,), 0.25)
+        while running:
+            C.set_weight_format("fp8")
+            C.configure(vocab_size=1024)
+            if changes % 4 == 0:
+                C.set_inv_freq(other)
+            changes += 1
+    try:
+        eng._base.apply_options()
+        C.prefill_packed_passes(*args)
+        want = [(k.clone(), v.clone()) for k, v in zip(eng._k_caches, eng._v_caches)]
+        for k, v in zip(eng._k_caches, eng._v_caches):
+            k.zero_(), v.zero_()
+        torch.cuda.synchronize()
+        eng._base.apply_options()
+        thread = _when_rows_appear(eng._k_caches[0], others)
+        C.prefill_packed_passes(*args)
+        running = False
+        thread.join()
+        assert changes > 0
+        for b, (k, v) in enumerate(want):
+            assert torch.equal(eng._k_caches[b], k) and torch.equal(eng._v_caches[b], v), b
+    finally:
+        running = False
+        eng._base.apply_options()
+        C.set_weight_format("fp16")
