@@ -360,7 +360,8 @@ int qmk_prefill_packed(
 /* Any number of passes of qmk_prefill_packed, one behind the other: pass p takes the next seqs_per_pass[p] sequences of the
  * concatenated arrays, under the limits of one call each.  The same rows as calls of their own leave; the host prepares a
  * pass while the one before runs and waits once, behind the last.  An argument that a pass refuses is reported when its turn
- * comes, the passes before it have run then; a device status of any pass is the call's.  Blocks. */
+ * comes, the passes before it have run then; a device status of any pass is the call's.  A prefill that
+ * another thread starts meanwhile runs behind the pass that is on its way, not behind the call.  Blocks. */
 int qmk_prefill_packed_passes(
     const int *token_ids_host, int num_passes, const int *seqs_per_pass, const int *seq_lens, const void *embed_weight,
     const struct LDGLayerWeight *layer_weights, const void *cos_table, const void *sin_table,

@@ -7,6 +7,9 @@
 #include <stdlib.h>
 #include <string.h>
 #include <mutex>
+#include <atomic>
+#include <chrono>
+#include <thread>
 #include <algorithm>
 #include <string>
 
@@ -562,6 +565,23 @@ struct Workspace {                  // per device, allocated on first use, never
 // stream (and thread) while a decode step of the live sequences runs on another.
 Workspace g_ws[16], g_ws_decode[16];
 std::recursive_mutex g_ws_mu;   // (recursive: qmk_tc::prefill_split's caller holds it already, see prefill_lock)
+std::atomic<int> g_ws_waiting{0};   // threads that wait for it
+std::unique_lock<std::recursive_mutex> lock_workspace() {
+  std::unique_lock<std::recursive_mutex> lock(g_ws_mu, std::try_to_lock);
+  if (!lock) {
+    ++g_ws_waiting;
+    lock.lock();
+    --g_ws_waiting;
+  }
+  return lock;
+}
+// Leaves the workspace to a thread that waits for it (a mutex that is released and taken again at once stays with its thread).
+void let_another_in(std::unique_lock<std::recursive_mutex> &lock) {
+  const int seen = g_ws_waiting.load();
+  lock.unlock();
+  for (int i = 0; i < 200 && seen > 0 && g_ws_waiting.load() >= seen; ++i) std::this_thread::sleep_for(std::chrono::microseconds(10));
+  lock = lock_workspace();
+}
 std::mutex g_ws_decode_mu;
 
 #define PF_CUDA(call)                                                                             \
@@ -704,8 +724,8 @@ struct PackedSeqs {
   const int *lens;
   void *const *k_caches, *const *v_caches;
 };
-// One of the passes of a call: the first one reads the layer table and clears the status, the last one waits and reports.  All run
-// with the options that the first one found: the maps are those of its weight format.
+// One of the passes of a call: the first one under a hold of the workspace reads the layer table and clears the status, the last one
+// waits and reports.  All of a call run with the options that pass 0 found: the maps are those of its weight format.
 struct Pass { bool first = true, last = true; int index = 0; qmk_internal::WeightOptions *options = nullptr; };
 constexpr int MAX_PACKED_SEQS = 64;
 constexpr size_t PK_ROWS_OFF = 0, PK_ITEMS_OFF = 32768, PK_MAPS_OFF = 49152, PK_PTRS_OFF = 65536, PK_BYTES = 66560;
@@ -730,7 +750,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
   using namespace qmk_pf;
   if (num_tokens <= 0) return QMK_OK;
   qmk_internal::PrefillEnv env;
-  int rc = qmk_internal::prefill_env(max_seq_len, stream, &env, pass.options, pass.first);
+  int rc = qmk_internal::prefill_env(max_seq_len, stream, &env, pass.options, pass.index == 0);
   if (rc != QMK_OK) return rc;
   if (split) env.attn_tc = 0;   // (split operands have an attention kernel of their own)
   if (!token_ids_host || !embed_weight || !layer_weights || (!pk && (!k_cache || !v_cache)))
@@ -761,7 +781,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
   int dev = 0;
   PF_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 16) return qmk_internal::report(QMK_ERR_CUDA, "device index out of range");
-  std::lock_guard<std::recursive_mutex> lock(g_ws_mu);
+  const auto lock = lock_workspace();
   Workspace &w = g_ws[dev];
   rc = ensure_workspace(w, CHUNK, take_steps);
   if (rc == QMK_OK && pass.first) rc = ensure_weight_maps(w, layer_weights, num_layers, wq, stream);
@@ -1118,7 +1138,7 @@ namespace qmk_tc {
 // meets them (prefill_impl reports errors to the engine while it holds the workspace).  `take_steps`: set, with
 // nothing reported, where the pass is not the way: the workspace does not fit in memory, or an activation exceeded the range
 // of its halves (65504; the cache rows are then to be written again).
-std::unique_lock<std::recursive_mutex> prefill_lock() { return std::unique_lock<std::recursive_mutex>(g_ws_mu); }
+std::unique_lock<std::recursive_mutex> prefill_lock() { return lock_workspace(); }
 int prefill_split(const int *token_ids_host, int num_tokens, const void *embed_weight, const LDGLayerWeight *layer_weights,
                   const void *cos_table, const void *sin_table, void *k_cache, void *v_cache, int num_layers, int start_position,
                   int max_seq_len, float attn_scale, cudaStream_t stream, bool *take_steps) {
@@ -1152,7 +1172,10 @@ extern "C" int qmk_prefill_packed_passes(const int *token_ids_host, int num_pass
   for (int p = 0; p < num_passes; ++p)
     if (seqs_per_pass[p] < 1 || seqs_per_pass[p] > MAX_PACKED_SEQS)
       return qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "packed prefill: 1 to 64 sequences a pass, each from position 0");
-  std::lock_guard<std::recursive_mutex> lock(g_ws_mu);   // (the passes share one workspace and one status)
+  // The passes share one workspace and one status, so the lock is held over them - until another thread wants it: the pass that is
+  // being sent then ends as the last one of a call does, and the others follow behind that thread's.
+  auto lock = lock_workspace();
+  bool first = true;
   qmk_internal::WeightOptions options;
   int rc = QMK_OK;
   for (int p = 0, s0 = 0; p < num_passes && rc == QMK_OK; s0 += seqs_per_pass[p++]) {
@@ -1160,13 +1183,14 @@ extern "C" int qmk_prefill_packed_passes(const int *token_ids_host, int num_pass
     for (int s = 0; s < seqs_per_pass[p]; ++s) total += seq_lens[s0 + s] > 0 ? seq_lens[s0 + s] : 0;
     const PackedSeqs pk = {seqs_per_pass[p], seq_lens + s0, k_caches + s0, v_caches + s0};
     Pass pass;
-    pass.first = p == 0;
-    pass.last = p + 1 == num_passes;
+    pass.first = first;
+    pass.last = first = p + 1 == num_passes || g_ws_waiting.load() > 0;
     pass.index = p;
     pass.options = &options;
     rc = total < 1 ? qmk_internal::report(QMK_ERR_BAD_ARGUMENT, "packed prefill: empty sequence or null cache")
                    : prefill_impl(token_ids_host, static_cast<int>(total), embed_weight, layer_weights, cos_table, sin_table, nullptr, nullptr,
                                   num_layers, 0, max_seq_len, attn_scale, stream, &pk, false, nullptr, pass);
+    if (rc == QMK_OK && pass.last && p + 1 < num_passes) let_another_in(lock);
     if (rc != QMK_OK && p > 0) cudaStreamSynchronize(stream);   // the passes before it are done, as behind calls of their own
     token_ids_host += total;
   }

@@ -411,17 +411,19 @@ def _passes(C, w, vocab, lens, seed, fmt="fp16"):
 
 
 def _when_rows_appear(cache, do):
-    """A thread that calls `do` as soon as the first pass has written rows of its last layer (its options have been read then)."""
+    """A thread that calls `do` as soon as the first pass has written rows of its last layer (its options have been read then).  Returns
+    when the thread looks."""
     import threading
-    stream = torch.cuda.Stream()
+    stream, looking = torch.cuda.Stream(), threading.Event()
 
     def body():
         with torch.cuda.stream(stream):
             while float(cache[-1, :, 0].float().abs().max()) == 0:
-                pass
+                looking.set()          # (the first look loads its kernels)
         do()
     t = threading.Thread(target=body)
     t.start()
+    assert looking.wait(60)
     return t
 
 
@@ -465,3 +467,37 @@ def test_gpu_options_set_by_another_thread_between_the_passes_of_a_call(built_li
         running = False
         eng._base.apply_options()
         C.set_weight_format("fp16")
+
+
+@pytest.mark.gpu
+def test_gpu_another_prefill_gets_in_between_the_passes_of_a_call(built_library):
+    """A short prompt that another thread prefills while a call of 24 packed passes runs waits for the pass on its way, not for the call,
+    and neither changes the other's rows."""
+    import time
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import qwen_megakernel_C as C
+    from Model.Qwen06B_architecture import Decoder
+    vocab, lens = 2048, [1500] * 24
+    w = S.weights_to(S.make_weights(seed=13, num_layers=8, vocab_size=vocab, norm_std=0.1, max_seq_len=16), "cuda")
+    eng, args = _passes(C, w, vocab, lens, 800)
+    short = Decoder(weights=w, tokenizer=S.StubTokenizer(-1, vocab), verbose=False, max_seq_len=64, prefill_mode="tensor")
+    ids, done = S.make_prompt(60, seed=3, vocab_size=vocab), []
+    C.prefill_packed_passes(*args)
+    short.prefill_ids(ids)
+    want = [x.clone() for x in (*eng._k_caches, *eng._v_caches, short._k_cache, short._v_cache)]
+    for x in (*eng._k_caches, *eng._v_caches, short._k_cache, short._v_cache):
+        x.zero_()
+    short.reset()
+    torch.cuda.synchronize()
+
+    def other():
+        short.prefill_ids(ids)
+        done.append(time.perf_counter())
+    thread = _when_rows_appear(eng._k_caches[0], other)
+    C.prefill_packed_passes(*args)
+    end = time.perf_counter()
+    thread.join()
+    assert done and done[0] < end
+    for x, y in zip((*eng._k_caches, *eng._v_caches, short._k_cache, short._v_cache), want):
+        assert torch.equal(x, y)
