@@ -838,9 +838,12 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
     std::stable_sort(order.begin(), order.end(), [](const auto &a, const auto &b) { return a.first > b.first; });   // longest job first
     pk_items = static_cast<int>(order.size());
     for (int i = 0; i < pk_items; ++i) items[i] = order[i].second;
-    PF_CUDA(cudaMemcpyAsync(w.packed, host, PK_BYTES, cudaMemcpyHostToDevice, stream));
-    token_ids_host = padded_tokens;
-    num_tokens = total_rows;
+    // Both copies out of the staging memory, then its event: whatever fails behind them, the pass that takes the slot next waits.
+    cudaError_t copied = cudaMemcpyAsync(w.packed, host, PK_BYTES, cudaMemcpyHostToDevice, stream);
+    if (copied == cudaSuccess) copied = cudaMemcpyAsync(w.tokens, padded_tokens, sizeof(int) * total_rows, cudaMemcpyHostToDevice, stream);
+    if (pageable.empty()) PF_CUDA(cudaEventRecord(w.staged[slot], stream));
+    PF_CUDA(copied);
+    num_tokens = total_rows;      // (one chunk)
   }
   std::vector<unsigned long long> rec(w.table, w.table + static_cast<size_t>(num_layers) * 12);
   const float *rope = env.rope_from_table ? nullptr : env.rope;
@@ -970,8 +973,7 @@ int prefill_impl(const int *token_ids_host, int num_tokens, const void *embed_we
                                  static_cast<uint64_t>(num_layers) * NKV, &err);
       if (rc != QMK_OK) break;
     }
-    PF_CUDA(cudaMemcpyAsync(w.tokens, token_ids_host + c0, sizeof(int) * T, cudaMemcpyHostToDevice, stream));
-    if (pk && pageable.empty()) PF_CUDA(cudaEventRecord(w.staged[slot], stream));
+    if (!pk) PF_CUDA(cudaMemcpyAsync(w.tokens, token_ids_host + c0, sizeof(int) * T, cudaMemcpyHostToDevice, stream));
     // Every kernel behind the first launches as a programmatic dependent: its set-up (and a GEMM's first ring fill of WEIGHT
     // tiles) runs under the tail of the kernel before it.  In order are, with each kernel waiting for its predecessor before
     // its first dependent read and any write: the residual rows and sums; the expanded matrices of a packed layer
