@@ -438,7 +438,8 @@ class BatchDecoder:
 
     def prefill_many(self, slots: Sequence[int], prompts: Sequence[Sequence[int]]) -> None:
         """Prefill any number of slots: in packed passes of up to ``packed_prefill_rows`` rows where the engine has
-        them, a prompt longer than that (or any prompt of an engine without packed prefill) through ``prefill_slot``."""
+        them, a prompt longer than that (or any prompt of an engine without packed prefill) through ``prefill_slot``.
+        Raises what the first pass that failed did; slots of passes that did not fail hold their prompts then."""
         budget = self.packed_prefill_rows
         passes, group, rows = [], [], 0      # packed passes that go to the device together; the one being filled
 
@@ -493,11 +494,26 @@ class BatchDecoder:
                     base._sin_table, [self._k_caches[b] for b, _ in flat], [self._v_caches[b] for b, _ in flat], base.num_layers,
                     self.max_seq_len, base._attn_scale)
             op = _require_megakernel_op("prefill_packed_passes")
-            if self._prefill_stream is not None:
-                with torch.cuda.stream(self._prefill_stream):   # the op blocks until its stream is idle
+            try:
+                if self._prefill_stream is not None:
+                    with torch.cuda.stream(self._prefill_stream):   # the op blocks until its stream is idle
+                        op(*args)
+                else:
                     op(*args)
-            else:
-                op(*args)
+            except RuntimeError:
+                if len(todo) == 1:
+                    raise
+                # Some passes may have written their rows, some not: each again as a call of its own, so that the position of
+                # every slot speaks of the rows it holds.
+                error = None
+                for group in passes:
+                    try:
+                        self._prefill_passes([group])
+                    except RuntimeError as exc:
+                        error = error or exc
+                if error is not None:
+                    raise error
+                return
         for group in passes:
             for b, ids in group:
                 self.positions[b] = len(ids)

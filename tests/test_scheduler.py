@@ -391,12 +391,54 @@ def test_gpu_packed_passes_of_one_call(built_library, fmt):
             for b, (k, v) in enumerate(want):
                 assert torch.equal(eng._k_caches[b], k) and torch.equal(eng._v_caches[b], v), b
         with pytest.raises(RuntimeError, match="vocab"):
-            eng.prefill_many([0, 1, 3, 5, 7], [prompts[0], prompts[1], prompts[3], prompts[5][:-1] + [vocab], prompts[7]])
+            eng.prefill_many([0, 1, 3, 5, 7], [prompts[0], prompts[1][:-1], prompts[3], prompts[5][:-1] + [vocab], prompts[7]])
+        assert eng.positions[:2] == [lens[0], lens[1] - 1] and eng.positions[3] == lens[3] and eng.positions[5] == lens[5]
         eng.prefill_many([0, 1, 3, 5, 7], [prompts[b] for b in (0, 1, 3, 5, 7)])
         for b in (0, 1, 3, 5, 7):
             assert torch.equal(eng._k_caches[b][:, :, :lens[b]], want[b][0][:, :, :lens[b]])
     finally:
         C.set_weight_format("fp16")
+
+
+@pytest.mark.parametrize("failure", ["refused", "device"])
+def test_positions_after_packed_passes_that_failed(built_library, monkeypatch, failure):
+    """Three packed passes in one call.  One that is refused (the passes in front of it have run then, those behind have not), or a device
+    failure of the call: the position of a slot is that of the prompt whose rows it holds."""
+    from types import SimpleNamespace
+    from Model import Qwen06B_architecture as A
+    rows = {b: 7 for b in range(6)}
+    calls = []
+
+    def op(counts, token_lists, *args):
+        calls.append(counts)
+        at = 0
+        for p, n in enumerate(counts):
+            if any(t >= 100 for ids in token_lists[at:at + n] for t in ids):
+                raise RuntimeError("prompt token outside [0, vocab)")
+            for cache, ids in zip(args[4][at:at + n], token_lists[at:at + n]):
+                rows[cache] = len(ids)
+            at += n
+        if failure == "device" and len(calls) == 1:
+            raise RuntimeError("a bounded device wait ran out")
+    monkeypatch.setattr(A, "_require_megakernel_op", lambda name: op)
+    eng = object.__new__(A.BatchDecoder)
+    eng.num_sequences, eng.max_seq_len, eng.positions, eng._prefill_stream = 6, 4096, [7] * 6, None
+    eng._k_caches = eng._v_caches = list(range(6))
+    eng._base = SimpleNamespace(prefill_mode="tensor", apply_options=lambda: None, _embed_weight=None, _layer_weights_packed=None, _cos_table=None,
+                                _sin_table=None, num_layers=1, _attn_scale=1.0)
+    prompts = [[1] * 2000, [2] * 1900, [3] * 2048, [100 if failure == "refused" else 4] * 2048, [5] * 3000, [6] * 900]
+    if failure == "refused":
+        with pytest.raises(RuntimeError, match="vocab"):
+            eng.prefill_many(range(6), prompts)
+        assert eng.positions[:2] == [2000, 1900] and eng.positions[3] == 7
+    else:
+        eng.prefill_many(range(6), prompts)
+        assert eng.positions == [len(ids) for ids in prompts]
+    assert calls[0] == [2, 2, 2]
+    assert all(eng.positions[b] == rows[b] for b in range(6))
+    with pytest.raises(RuntimeError, match="vocab"):
+        eng.prefill_slots([0, 1], [[1], [100]])          # one pass: as it was
+    assert eng.positions[:2] == ([2000, 1900])
 
 
 def _passes(C, w, vocab, lens, seed, fmt="fp16"):
