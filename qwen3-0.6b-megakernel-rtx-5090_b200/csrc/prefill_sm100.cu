@@ -336,13 +336,15 @@ static bool a_box_ok(int a_box_rows, int M, int *rows, uint32_t *a_box_bytes, st
   return true;
 }
 
-// Rows of the MMA for a launch: 64 where its only row tile has a short A box of at most that many and the tile has such a kernel; fp16
-// weights up to 48: behind that the product issues no faster with half the rows (us per step of 34 / 42 / 50 / 57 / 64 sequences of 64 tokens,
-// 64 rows -> 128: 766 / 837 / 877 / 889 / 897 -> 760 / 833 / 861 / 876 / 884; 44 and 64 of 128 to 1024 tokens 1240 / 1484 -> 1254 / 1470; 5 to 16
-// sequences gain 2 % by 64 rows, packed weights at every size).  A row's sums are the same bit for bit.
-static int mma_rows(const qmk_gemm::Groups &gr, int box_n, bool fuse, int wq) {
-  const uint32_t most = wq == 0 ? 48 : 64;
-  return gr.a_box_bytes > 0 && gr.a_box_bytes <= most * qmk_gemm::BK * 2 && t_ah == 1 && gr.row_scale[0] == nullptr && gemm_kernel_64(box_n, fuse, wq) ? 64 : qmk_gemm::BM;
+// Rows of the MMA for a launch with `live` rows: 64 where its only row tile has a short A box and the tile has such a kernel, with
+// packed weights up to 64, with fp16 weights up to 28 rows.  us per step of fp16 sequences, 64-row -> 128-row products, 48 steps from 64
+// tokens, 16 / 20 / 24 / 28 / 30 / 32 / 36 / 40 / 48 / 64 sequences 778 / 730 / 738 / 749 / 756 / 763 / 779 / 838 / 883 / 917 -> 785 / 737 / 742 / 751 /
+// 752 / 755 / 771 / 836 / 866 / 902; from 128 to 1024 tokens, 16 / 24 / 28 / 30 / 32 / 40 / 48 / 64 sequences 922 / 1011 / 1055 / 1084 / 1108 / 1224 / 1290 /
+// 1475 -> 928 / 1015 / 1059 / 1084 / 1103 / 1206 / 1281 / 1461: the two meet at 29 or 30 (every number from 23 to 42 was timed, three runs
+// of a side within 0.1 %).  Packed weights gain at every size.  A row's sums are the same bit for bit.
+static int mma_rows(const qmk_gemm::Groups &gr, int live, int box_n, bool fuse, int wq) {
+  const bool fits = gr.a_box_bytes > 0 && gr.a_box_bytes <= 64u * qmk_gemm::BK * 2 && t_ah == 1 && gr.row_scale[0] == nullptr && gemm_kernel_64(box_n, fuse, wq);
+  return fits && live <= (wq == 0 ? 28 : 64) ? 64 : qmk_gemm::BM;
 }
 
 // C_g[M x N_g] fp32 = A[M x K] * B_g[N_g x K]^T for up to three matrices B_g in one launch.  M, N_g multiples of
@@ -377,7 +379,7 @@ int launch_gemm_grouped(const CUtensorMap &map_a, int ngroups, const CUtensorMap
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
   int rows = live_rows > 0 ? live_rows : M;   // rows the epilogue stores (the rest of the tile is padding)
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
-  const int am = mma_rows(gr, box_n, false, wq);
+  const int am = mma_rows(gr, rows, box_n, false, wq);
   set_prefetch(&gr, static_cast<long>(grid.x) * grid.y);
   const size_t smem = set_ring(&gr, box_n, wq, static_cast<long>(grid.x) * grid.y, am, K / qmk_gemm::BK);
   cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah, gr.row_scale[0] != nullptr, am), grid, dim3(qmk_gemm::threads_for(wq, t_ah)), smem, stream,
@@ -411,7 +413,7 @@ int launch_gemm_swiglu(const CUtensorMap &map_a, const CUtensorMap &map_gate, co
   int rows = live_rows > 0 ? live_rows : M;
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
-  const int am = mma_rows(gr, box_n, true, wq);
+  const int am = mma_rows(gr, rows, box_n, true, wq);
   set_prefetch(&gr, static_cast<long>(N / box_n) * (M / qmk_gemm::BM));
   const size_t smem = set_ring(&gr, 2 * box_n, wq, static_cast<long>(N / box_n) * (M / qmk_gemm::BM), am, K / qmk_gemm::BK);
   cudaError_t e = launch_kernel(gemm_kernel(box_n, true, wq, t_ah, gr.row_scale[0] != nullptr, am), dim3(N / box_n, M / qmk_gemm::BM), dim3(qmk_gemm::threads_for(wq, t_ah)),
@@ -444,7 +446,7 @@ int launch_gemm_splitk(const CUtensorMap &map_a, const CUtensorMap &map_b, float
   int rows = live_rows > 0 ? live_rows : M;
   if (!a_box_ok(a_box_rows, M, &rows, &gr.a_box_bytes, err)) return QMK_ERR_BAD_ARGUMENT;
   const unsigned long long budget = static_cast<unsigned long long>(timeout_ms) * 1000000ull;
-  const int am = mma_rows(gr, box_n, false, wq);
+  const int am = mma_rows(gr, rows, box_n, false, wq);
   set_prefetch(&gr, static_cast<long>(N / box_n) * (M / qmk_gemm::BM) * splits);
   const size_t smem = set_ring(&gr, box_n, wq, static_cast<long>(N / box_n) * (M / qmk_gemm::BM) * splits, am, gr.kblocks_per_split);
   cudaError_t e = launch_kernel(gemm_kernel(box_n, false, wq, t_ah, gr.row_scale[0] != nullptr, am), dim3(N / box_n, M / qmk_gemm::BM, splits), dim3(qmk_gemm::threads_for(wq, t_ah)),
