@@ -464,7 +464,7 @@ class BatchDecoder:
                 continue
             if group and (rows + need > budget or len(group) == 64):
                 close()
-            group.append((b, list(ids)))
+            group.append((int(b), list(ids)))
             rows += need
         close()
         send()

@@ -400,12 +400,34 @@ def test_gpu_packed_passes_of_one_call(built_library, fmt):
         C.set_weight_format("fp16")
 
 
+def _host_only_engine(monkeypatch, op):
+    """A batched engine of six slots whose packed passes are calls of ``op``; its caches are their slots' numbers."""
+    from types import SimpleNamespace
+    from Model import Qwen06B_architecture as A
+    monkeypatch.setattr(A, "_require_megakernel_op", lambda name: op)
+    eng = object.__new__(A.BatchDecoder)
+    eng.num_sequences, eng.max_seq_len, eng.positions, eng._prefill_stream = 6, 4096, [7] * 6, None
+    eng._k_caches = eng._v_caches = list(range(6))
+    eng._base = SimpleNamespace(prefill_mode="tensor", apply_options=lambda: None, _embed_weight=None, _layer_weights_packed=None, _cos_table=None,
+                                _sin_table=None, num_layers=1, _attn_scale=1.0)
+    return eng
+
+
+def test_slots_of_packed_passes_are_whole_numbers(built_library, monkeypatch):
+    """Whatever int() takes names a slot, and a slot named twice in a pass is refused whatever type its names have."""
+    seen = []
+    eng = _host_only_engine(monkeypatch, lambda counts, lists, *args: seen.extend(args[4]))
+    eng.prefill_many(torch.tensor([1.0, 4.0, 0.0]), [[1, 2], [3], [4, 5, 6]])
+    assert seen == [1, 4, 0] and eng.positions == [3, 2, 7, 7, 1, 7]
+    with pytest.raises(ValueError, match="distinct"):
+        eng.prefill_many(torch.tensor([1, 1]), [[1, 2], [3]])
+    assert seen == [1, 4, 0]
+
+
 @pytest.mark.parametrize("failure", ["refused", "device"])
 def test_positions_after_packed_passes_that_failed(built_library, monkeypatch, failure):
     """Three packed passes in one call.  One that is refused (the passes in front of it have run then, those behind have not), or a device
     failure of the call: the position of a slot is that of the prompt whose rows it holds."""
-    from types import SimpleNamespace
-    from Model import Qwen06B_architecture as A
     rows = {b: 7 for b in range(6)}
     calls = []
 
@@ -420,12 +442,7 @@ def test_positions_after_packed_passes_that_failed(built_library, monkeypatch, f
             at += n
         if failure == "device" and len(calls) == 1:
             raise RuntimeError("a bounded device wait ran out")
-    monkeypatch.setattr(A, "_require_megakernel_op", lambda name: op)
-    eng = object.__new__(A.BatchDecoder)
-    eng.num_sequences, eng.max_seq_len, eng.positions, eng._prefill_stream = 6, 4096, [7] * 6, None
-    eng._k_caches = eng._v_caches = list(range(6))
-    eng._base = SimpleNamespace(prefill_mode="tensor", apply_options=lambda: None, _embed_weight=None, _layer_weights_packed=None, _cos_table=None,
-                                _sin_table=None, num_layers=1, _attn_scale=1.0)
+    eng = _host_only_engine(monkeypatch, op)
     prompts = [[1] * 2000, [2] * 1900, [3] * 2048, [100 if failure == "refused" else 4] * 2048, [5] * 3000, [6] * 900]
     if failure == "refused":
         with pytest.raises(RuntimeError, match="vocab"):
