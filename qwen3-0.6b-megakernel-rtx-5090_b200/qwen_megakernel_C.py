@@ -588,7 +588,7 @@ def gemm_packed_tn(a: torch.Tensor, b: torch.Tensor, weight_format, b2: torch.Te
     rows, see ``quantize.pack_rows_fp8`` / ``pack_rows_nvfp4``).  ``mode``: ``"plain"`` -> fp32 ``[m, n]``; ``"splitk"`` ->
     fp32 ``[4, m, n]`` partial matrices; ``"swiglu"`` (``b`` gate, ``b2`` up) -> fp16 ``[m, n]``."""
     _require_cuda()
-    fmt = WEIGHTWEIGHT_FORMATS[weight_format] if isinstance(weight_format, str) else int(weight_format)
+    fmt = WEIGHT_FORMATS[weight_format] if isinstance(weight_format, str) else int(weight_format)
     code = {"plain": 0, "splitk": 1, "swiglu": 2}[mode]
     _check(a.is_cuda and a.dtype == torch.float16 and a.is_contiguous() and a.dim() == 2,
            "gemm_packed_tn: a must be a contiguous fp16 CUDA matrix [m, k]")
