@@ -414,7 +414,7 @@ int qmk_sync_status(void);
  * theirs in its place.  Every function that returns a status counts as a call, qmk_engine_destroy excepted.  On a thread that has made
  * none: the last error on its device.  The pointer is good until the thread asks again. */
 const char *qmk_last_error(void);
-/* Persistent grid size (CTAs) and bytes of library-owned device scratch. */
+/* Persistent grid size (CTAs; a kernel whose work divides better may launch fewer) and bytes of library-owned device scratch. */
 int qmk_num_ctas(void);
 long long qmk_scratch_bytes(void);
 /* CTAs that the tensor-core decode kernel for this weight format (0 fp16, 1 FP8) and number of sequences (1 to 4) is launched with

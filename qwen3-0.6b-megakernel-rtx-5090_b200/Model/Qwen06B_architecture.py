@@ -396,8 +396,8 @@ class BatchDecoder:
         """Persistent up to three sequences, gemm from five on (NVFP4 rows: always gemm).  Four: persistent where the launch
         runs on the tensor cores - a grid of at least 112 CTAs, whole ring chunks of vocabulary, room for the K-major
         copies; its group-per-sequence form takes 1.9 ms a step - and the cache has room for 8192 rows at most (FP8 12288).
-        Measured, us per step of four fp16 sequences at 64 / 1024 / 2048 / 4096 / 8000 tokens: 631 / 726 / 815 / 1001 / 1363
-        persistent, 758 / 804 / 870 / 1034 / 1290 gemm; FP8 rows 576 / 674 / 781 / 975 / 1358 and 904 / 959 / 1019 / 1180 / 1440
+        Measured, us per step of four fp16 sequences at 64 / 1024 / 2048 / 4096 / 8000 tokens: 642 / 728 / 819 / 1001 / 1363
+        persistent, 758 / 804 / 870 / 1034 / 1290 gemm; FP8 rows 589 / 688 / 793 / 975 / 1358 and 904 / 959 / 1019 / 1180 / 1440
         (one long context among short ones costs either less).  So the GEMM step is the faster one behind about 5000 tokens
         (FP8 9500), and a cache of that many rows is shorter than that for most of its steps."""
         if weight_format == "nvfp4" or n > cls.MAX_SEQUENCES:

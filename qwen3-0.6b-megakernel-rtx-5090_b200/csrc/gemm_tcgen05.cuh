@@ -314,7 +314,7 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 // RS: fp16 B matrices with row scales (Groups::row_scale).  A kernel of its own: a run-time test of the pointers in the
 // epilogues of every fp16 GEMM cost a prefill pass 0.6 to 1 %.
 //
-// AM: rows of the MMA, 128 or, for launches of one row tile with at most 64 live rows (decode steps), 64.  With every operand in
+// AM: rows of the MMA, 128 or, for launches of one row tile with few live rows (decode steps, see mma_rows), 64.  With every operand in
 // place the four products of a K block take 162 cycles against 32 columns at 128 rows and 99 at 64 (the tensor core reads A from
 // shared memory, 4 KB a product against 2 KB), and a stage is 8 KB smaller, so that the ring holds more of the K loop.  Decode
 // steps at 64-token contexts, 128 rows everywhere -> so: 5 / 16 / 64 fp16 sequences 774 / 780 / 878 -> 759 / 773 / 894 us (the last of

@@ -442,7 +442,7 @@ void free_prepared(Engine::Prepared &p) {
   if (p.fp) cudaFree(p.fp);
   p = Engine::Prepared();
 }
-constexpr size_t MAX_PREPARED = 4;   // weight sets kept per device (a 28-layer fp16 set is 294 MB)
+constexpr size_t MAX_PREPARED = 4;   // weight sets kept per device (a 28-layer fp16 set is 294 MB, with O rows by quarters 297)
 
 // Finds or creates the K-major copies for the caller's layer table and enqueues the check-and-rebuild kernel.
 // `several` (sequences): every byte of the matrices is checked, and where the copies do not fit in memory *out stays null
@@ -619,9 +619,10 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
       threads = qmk::THREADS;
       grid = tc_grid;
       // Two fp16 sequences: 128 CTAs have whole tiles everywhere (32 q|k|v, 48 gate / up rows, slices of 64 attention outputs: a CTA of 148
-      // multiplies as many) and fewer contributions and readers to every sum.  us per step on 148 / 136 / 128 / 124 CTAs, 64 tokens 511 / 491
-      // / 479 / 576, 1024 tokens 541 / 530 / 509 / 593; from about 2200 tokens on (566 / 583 / 566) the attention misses the others.  FP8 rows
-      // (1024 tokens 554 / 543 on 148 / 128, 64 tokens 500 / 508), three (635 / 662) and one (436 / 446) stay on all.
+      // multiplies as many) and fewer contributions and readers to every sum.  us per step on 148 / 136 / 128 / 124 CTAs, means of three
+      // placements of the buffers, 64 tokens 513 / 499 / 483 / 575, 1024 tokens 545 / 540 / 517 / 593; at 2200 tokens (570 / 595 / 577 / 665) the
+      // attention misses the others.  FP8 rows (64 tokens 538 / 532 on 148 / 128, 1024 tokens 577 / 558, a placement 7 % either way), three
+      // sequences (635 / 662) and one (440 / 447) stay on all.
       int longest = 0;
       for (int b = 0; b < P.nseq; ++b) longest = std::max(longest, P.start_positions[b] + P.num_steps);
       if (P.nseq == 2 && e->wfmt == 0 && grid > 128 && longest <= 2048) grid = 128;
@@ -631,7 +632,7 @@ int launch(Engine *e, Params &P, cudaStream_t stream, bool synchronize, bool bat
       kernel == reinterpret_cast<const void *>(qmk::qwen3_decode_megakernel)) {
     // fused kernel: O and down projections as split-K slices of K-major copies, two all-reduced residual sums
     // Row products on the tensor cores: rows owned in units of one ring chunk (four fp16 rows, eight fp8 rows).  fp8:
-    // 724 -> 412 us per token at 1024-token contexts against the CUDA-core kernel, which stays for the grids and
+    // 724 -> 416 us per token at 1024-token contexts against the CUDA-core kernel, which stays for the grids and
     // vocabularies outside these limits.
     const qmk_fused_tc::Build &tc = qmk_fused_tc::build(e->wfmt);
     const int tc_grid = tc.grid(grid);

@@ -31,8 +31,8 @@
 // (xf_offset).  A packed row is 1040 bytes in memory, which is a conflict-free pitch in shared memory too: a chunk
 // is eight rows and ONE bulk copy (four 2 KB rows: four copies).  Row scales multiply the finished sums (they sit in
 // the rows' trailers); the per-output scales of the K-major O / down copies travel as one more chunk of those phases.
-// Measured after: 493 us per token (128 tokens from a 1024-token context; 412 with what is described below).  Against float64 the cache rows are nearer than the
-// CUDA-core kernel's (later layers' values that round differently: 0.154 % and 0.167 %).
+// Measured after: 493 us per token (128 tokens from a 1024-token context; 416 with what is described below).  Against float64 the cache rows are nearer than the
+// CUDA-core kernel's (later layers' values that round differently: 0.149 % and 0.167 %).
 
 namespace QMK_NS {
 #if QMK_MAX_SEQ == 1 && defined(QMK_TC_BUILD)
@@ -42,8 +42,8 @@ namespace QMK_NS {
 #endif
 constexpr int TC_SEQS = QMK_TC_SEQS;           // sequences a launch can carry (2 and 4: megakernel_tc_multi.cuh)
 static_assert(TC_SEQS == 1 || TC_SEQS == 2 || TC_SEQS == 4, "two of the eight columns of an MMA per sequence");
-// smallest grid: <= 2 attention outputs per warp to merge, O / down slices of <= 32 rows; four sequences: phases of at
-// most as many chunks as their shorter ring has slots
+// smallest grid: down slices of <= 32 rows, O slices of <= 88 whose merge is two quads of outputs per warp and one for the last two; four
+// sequences: phases of at most as many chunks as their shorter ring has slots
 constexpr int TC_MIN_CTAS = TC_SEQS == 4 ? 112 : 96;
 static_assert(TC_MIN_CTAS >= FUSED_MIN_CTAS, "the tensor-core kernel shares the fused kernel's slice layout");
 #ifdef QMK_TC_FP8
@@ -68,7 +68,7 @@ static_assert(I % CH_ROWS == 0 && QS % CH_ROWS == 0 && KVS % CH_ROWS == 0, "a ch
 // word are 37, a CTA's words 256.  What it costs is a merge of four times the words, whose loads take whole 32-byte sectors now.
 // Mean step of five placements of the buffers, us, before / after (with wait_chunks): one fp16 sequence at 64 / 1024 / 4096 tokens 430 / 443 /
 // 488 -> 432 / 443 / 478, one FP8 at 1024 428 -> 411, two fp16 at 512 531 -> 530, four at 1024 747 -> 733, four FP8 801 -> 728.
-// Grids that are no multiple of four leave the last CTAs without a slice.
+// Grids that are no multiple of four leave the last CTAs without a slice (see tc_grid).
 using qmkp::O_GROUP;
 using qmkp::O_COLS;
 constexpr int O_TILES = O_COLS / 16;

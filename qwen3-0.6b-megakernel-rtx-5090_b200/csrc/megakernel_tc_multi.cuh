@@ -9,11 +9,12 @@
 // words read back, cache rows.
 // The launch it replaces (megakernel_batch.cuh, which stays for grids outside this kernel's range) gives each sequence a
 // group of warps that convert and multiply every weight for themselves, and has six hand-overs per layer.
-// Measured, us per step at 64 / 1024 / 2048-token contexts: two fp16 sequences 494 / 516 / 569, three 632 / 702 / 760, four
-// 631 / 726 / 815, four with FP8 rows 576 / 674 / 781 (the group launch: two 1137 / 1317 at 64 / 1024; four 1655 / 1942; the
-// GEMM step: four fp16 758 / 804 / 870, four FP8 904 / 959 / 1019, with fp16-rounded activations).  Share of later layers' cache values
-// that round to another fp16 than float64's, 1024 tokens: two and four fp16 sequences 0.156 and 0.161 % (group launch 0.147
-// and 0.150), two with FP8 rows 0.152 (0.151).
+// Measured, us per step at 64 / 1024 / 2048-token contexts, means of five placements of the buffers: two fp16 sequences 485 / 514 /
+// 566, three 625 / 694 / 756, four 642 / 728 / 819 (a placement within 1 %; three sequences 3 %), four with FP8 rows 589 / 688 / 793 (5 %),
+// two 516 / 559 at 64 / 1024 (7 %).  (The group launch: two 1137 / 1317 at 64 / 1024; four 1655 / 1942; the GEMM step: four fp16 758 /
+// 804 / 870, four FP8 904 / 959 / 1019, with fp16-rounded activations.)  Share of later layers' cache values
+// that round to another fp16 than float64's, 1024 tokens: two and four fp16 sequences 0.155 and 0.157 % (group launch 0.147
+// and 0.150), two with FP8 rows 0.149 (0.151).
 
 namespace QMK_NS {
 #if QMK_MAX_SEQ == 1 && defined(QMK_TC_BUILD) && QMK_TC_SEQS > 1
